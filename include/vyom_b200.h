@@ -784,8 +784,10 @@ typedef struct VyWinAttn {
   /* row strides of the two pools in elements; 0 = kv_heads * dim and kv_heads * vdim. With explicit strides k_pool and v_pool
    * may be views of ONE pool (latent attention: the value is the leading part of the key row). */
   int64_t k_row, v_row;
-  /* optional scratch of vy_window_attn_workspace_floats(n_seqs, heads, kv_heads, vdim) floats (0: none needed): single-token steps whose query heads share
-   * key / value rows in groups of 8 or more split a sequence's keys over several CTAs and combine the parts from here */
+  /* optional scratch. Single-token steps: vy_window_attn_workspace_floats(n_seqs, heads, kv_heads, vdim) floats (0: none needed); those whose query heads share
+   * key / value rows in groups of 8 or more split a sequence's keys over several CTAs and combine the parts from here. Longer portions:
+   * vy_window_attn_prompt_floats(..) floats, 16-byte aligned (0: none needed); the visible key / value rows are split for the tensor cores once, into it,
+   * instead of by every CTA that reads them */
   float* workspace; int64_t workspace_floats;
   void* stream;
   int32_t chunk;
@@ -801,6 +803,8 @@ typedef struct VyWinAttn {
   const float* head_slope;
 } VyWinAttn;
 VY_API int64_t vy_window_attn_workspace_floats(int32_t n_seqs, int32_t heads, int32_t kv_heads, int32_t vdim);
+VY_API int64_t vy_window_attn_prompt_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t kv_heads, int32_t dim, int32_t vdim,
+                                            int32_t window, int32_t keep_first, int32_t chunk);
 VY_API int vy_window_attn(const VyWinAttn* p);
 
 /* Depthwise causal convolution over time with carried taps, then an activation:

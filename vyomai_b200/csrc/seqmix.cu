@@ -905,6 +905,16 @@ extern "C" int64_t vy_window_attn_workspace_floats(int32_t n_seqs, int32_t heads
   return vy::window_attn_heads_workspace_floats(n_seqs, heads, kv_heads, vdim);
 }
 
+extern "C" int64_t vy_window_attn_prompt_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t kv_heads, int32_t dim, int32_t vdim,
+                                               int32_t window, int32_t keep_first, int32_t chunk) {
+  using namespace vy;
+  if (n_seqs <= 0 || max_new < WA_TILED_MIN || table_width <= 0 || block_size <= 0 || kv_heads <= 0 || dim <= 0 || vdim <= 0) return 0;
+  WinDev d = {};
+  d.tw = table_width; d.bs = block_size; d.kv_heads = kv_heads; d.dim = dim; d.vdim = vdim;
+  d.window = window; d.keep = keep_first; d.chunk = chunk;
+  return window_attn_split_floats(d, n_seqs, max_new);
+}
+
 extern "C" int vy_window_attn(const VyWinAttn* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_window_attn: null params");
@@ -942,8 +952,12 @@ extern "C" int vy_window_attn(const VyWinAttn* p) {
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   VY_CHECK_ARG(p->dim <= 32 * WA_VR, "vy_window_attn: dim %d > %d", p->dim, 32 * WA_VR);
-  if (p->max_new >= WA_TILED_MIN) {   // prompt-sized: 64 x 64 register-tiled form
-    VY_CUDA_OK(launch_window_attn_tiled(d, p->n_seqs, p->max_new, st));
+  if (p->max_new >= WA_TILED_MIN) {   // prompt-sized: tensor-core tiles
+    int launches = 1;
+    VY_CUDA_OK(launch_window_attn_tiled(d, p->n_seqs, p->max_new, p->workspace, p->workspace_floats, st, &launches));
+    VY_LAUNCH_OK();
+    count_launch(launches);
+    return VY_OK;
   } else if (p->max_new == 1 && window_attn_heads_applies(d)) {
     int launches = 1;
     VY_CUDA_OK(launch_window_attn_heads(d, p->n_seqs, p->workspace, p->workspace_floats, st, &launches));

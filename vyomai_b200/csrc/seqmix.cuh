@@ -166,10 +166,11 @@ struct RecDev {
   void* out; long long ld_out; int out_dt;
 };
 
-// Prompt-sized steps: defined in seqmix_tiled.cu.
+// Prompt-sized steps: defined in seqmix_tiled.cu and window_attn_mma.cu.
 cudaError_t launch_linear_attn_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
-cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, cudaStream_t st);
+cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches);
+long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);   // the workspace it makes use of
 // Single tokens whose query heads share key / value rows in groups of 8 or more (latent rows): heads as the rows of a tile.
 bool window_attn_heads_applies(const WinDev& d);
 long long window_attn_heads_workspace_floats(int n_seqs, int heads, int kv_heads, int vdim);

@@ -1,0 +1,414 @@
+// Prompt-sized windowed attention over pages (vy_window_attn, portions of several tokens): scores and weighted values in fp32 precision
+// on the tensor cores, operands split into two fp16 parts (split_mma.cuh), online softmax in registers.
+//
+// A first launch splits every key and value row that some query of the step sees, once, into a workspace in the order the tiles read
+// them ([sequence][key / value head][key]: K hi | K lo | V hi | V lo, the bytes of the fp32 rows). In the second, a CTA owns 16 rows per warp:
+// 2^hl query heads of one key / value head times the rows / 2^hl queries, so that heads that share keys share the key tiles and the window's
+// edges waste little. A warp keeps its scores, weights and outputs in registers from one product to the next; the next tile's rows
+// arrive in the other buffer (cp.async) meanwhile. Without a workspace (a caller of the C ABI that lends none, or one too large to lend) each
+// CTA splits its tiles itself, which costs it about as many instructions as the softmax does.
+//
+// What bounds it: the tensor pipe (three fp16 products per fp32 one on mma.sync), then the instructions of the softmax.
+#include "seqmix.cuh"
+#include "split_mma.cuh"
+
+namespace vy {
+
+// where the split rows of (sequence s, key / value head g) lie, and which keys they are
+struct SplitKv {
+  unsigned char* rows; int* expo;   // expo: [2][n_seqs * kv_heads * cap], keys then values
+  long long cap;                    // key slots per (sequence, key / value head)
+  int row_bytes;                    // 4 (dim16 + vdim16)
+};
+
+// the keys a portion sees, from its first query on: slots [0, nA) are positions [0, nA) (kept first tokens), the others positions from lo on
+__device__ __forceinline__ void portion_keys(const WinDev& d, int p0, int& nA, int& lo) {
+  lo = d.chunk > 0 ? p0 / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p0 - d.window + 1, 0);
+  nA = d.window <= 0 ? 0 : min(d.keep, lo);
+}
+
+constexpr int WS_T = 256, WS_ROWS = WS_T / 8;   // splitting launch: eight lanes per row
+
+// bound by the bytes: every row read once and written once (8000 rows of 2 x (128 + 128) channels: 33 MB)
+template <int MAXD>
+__global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, SplitKv w, int dim16, int vdim16, bool kvvec) {
+  pdl_trigger();
+  pdl_wait();
+  const int s = blockIdx.z, g = blockIdx.y, n = d.cu[s + 1] - d.cu[s], p0 = d.pos0[s];
+  int nA, lo;
+  portion_keys(d, p0, nA, lo);
+  const int count = n > 0 ? nA + p0 + n - lo : 0;
+  const int* tab = d.table + static_cast<long long>(s) * d.tw;
+  const long long slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
+  const long long all = static_cast<long long>(gridDim.z) * d.kv_heads * w.cap;
+  const int r0 = blockIdx.x * WS_ROWS;
+  if (r0 >= count) return;
+  const int rows = min(WS_ROWS, count - r0);
+  const auto row_of = [&](int r) {
+    const int kp = r0 + r < nA ? r0 + r : lo + (r0 + r - nA);
+    return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
+  };
+  unsigned char* out = w.rows + (slot0 + r0) * w.row_bytes;
+  split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, w.expo + slot0 + r0, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
+                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; });
+  out += 4 * dim16;
+  split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, w.expo + all + slot0 + r0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
+                              [&](int r) { return row_of(r) * d.v_row + static_cast<long long>(g) * d.vdim; });
+}
+
+// MAXD: most query / key channels; VT: value channels the accumulators hold; NW: warps (16 rows each); PRE: rows come split from the workspace
+// (two tile buffers), else the CTA splits them itself (one buffer); SIG: sigmoid weights
+template <int MAXD, int VT, int NW, bool PRE, bool SIG>
+__global__ void __launch_bounds__(32 * NW, NW == 4 && VT <= 128 && !PRE ? 2 : 1)
+window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool qvec, bool kvvec, bool ovec) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int R = 16 * NW, N = MAXD > 128 ? 32 : 64, NT = N / 8, KT = N / 16;   // rows of a CTA; keys per tile, as score columns of 8 and value steps of 16
+  constexpr int NC = VT / 32;   // value columns go in blocks of 32
+  extern __shared__ __align__(16) unsigned char wm_smem[];
+  const int kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16;   // bytes between rows: an odd multiple of 16 (ldmatrix without bank conflicts)
+  const int k_lo = N * kb, v_lo = N * vb, buf = 2 * k_lo + 2 * v_lo;   // from a hi plane to its lo plane; bytes of a tile buffer
+  unsigned char* Qh = wm_smem;
+  unsigned char* Ts = Qh + 2 * R * kb;     // [buffers][K hi | K lo | V hi | V lo]
+  int* qe = reinterpret_cast<int*>(Ts + (PRE ? 2 : 1) * buf);   // exponents of the rows of Q, then [buffers][K | V]
+  int* te = qe + R;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+  const int s = blockIdx.z, h0 = blockIdx.y << hl, qn = R >> hl;
+  const int base = d.cu[s], n = d.cu[s + 1] - base;
+  // the last queries see the most keys: they go first
+  const int blk = (n + qn - 1) / qn - 1 - static_cast<int>(blockIdx.x);
+  if (blk < 0) return;
+  const int i0 = blk * qn, nq = min(qn, n - i0), hm = (1 << hl) - 1;
+  const int g = h0 / (d.heads / d.kv_heads);
+  const int p0 = d.pos0[s], p_lo = p0 + i0, p_hi = p_lo + nq - 1;
+  // visible keys of the tile's queries: [0, nA) (kept first tokens outside the band) and [lo, p_hi] (the band); masks are per pair
+  int nA, lo;
+  portion_keys(d, p_lo, nA, lo);
+  const int count = nA + (p_hi - lo + 1);
+  int nA0 = 0, lo0 = 0;   // the same of the portion: where the workspace keeps a key
+  long long slot0 = 0;
+  if constexpr (PRE) {
+    portion_keys(d, p0, nA0, lo0);
+    slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
+  }
+  const int* tab = d.table + static_cast<long long>(s) * d.tw;
+  const auto key_of = [&](int c) { return c < nA ? c : lo + (c - nA); };
+  const auto fetch = [&](int c0, int b) {   // tile of keys c0 .. into buffer b, its exponents beside it
+    unsigned char* T = Ts + b * buf;
+    int* e = te + b * 2 * N;
+    if constexpr (PRE) {
+      const long long all = static_cast<long long>(gridDim.z) * d.kv_heads * w.cap;
+      const int k16 = dim16 >> 3, v16 = vdim16 >> 3, per = 2 * (k16 + v16);   // 16-byte runs of a plane's row, of a row
+      for (int x = threadIdx.x; x < 2 * N; x += 32 * NW) {
+        const int j = x & (N - 1), kp = key_of(c0 + j);
+        e[x] = c0 + j < count ? w.expo[(x >= N ? all : 0) + slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)] : SPLIT_MIN_E;
+      }
+      // a warp copies whole rows
+      for (int j = warp; j < N; j += NW) {
+        const int kp = key_of(min(c0 + j, count - 1));
+        const unsigned char* src = w.rows + (slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)) * w.row_bytes;
+        const unsigned dst = smem_addr(T);
+        for (int x = lane; x < per; x += 32) {
+          int o;   // byte offset in the buffer
+          if (x < 2 * k16) o = x < k16 ? j * kb + 16 * x : k_lo + j * kb + 16 * (x - k16);
+          else o = 2 * k_lo + (x < 2 * k16 + v16 ? j * vb + 16 * (x - 2 * k16) : v_lo + j * vb + 16 * (x - 2 * k16 - v16));
+          cp_async16(dst + o, src + 16 * x, c0 + j < count);
+        }
+      }
+      cp_async_commit();
+    } else {
+      const auto row_of = [&](int j) {
+        if (c0 + j >= count) return -1LL;
+        const int kp = key_of(c0 + j);
+        return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
+      };
+      split_rows<NW, MAXD>(T, T + k_lo, kb, e, N, d.dim, dim16, d.kp, d.pool_dt, kvvec, [&](int j) {
+        const long long r = row_of(j);
+        return r >= 0 ? r * d.k_row + static_cast<long long>(g) * d.dim : -1LL;
+      });
+      split_rows<NW, VT>(T + 2 * k_lo, T + 2 * k_lo + v_lo, vb, e + N, N, d.vdim, vdim16, d.vp, d.pool_dt, kvvec, [&](int j) {
+        const long long r = row_of(j);
+        return r >= 0 ? r * d.v_row + static_cast<long long>(g) * d.vdim : -1LL;
+      });
+    }
+  };
+  if constexpr (PRE) fetch(0, 0);
+  split_rows<NW, MAXD>(Qh, Qh + R * kb, kb, qe, R, d.dim, dim16, d.q, d.q_dt, qvec, [&](int r) {
+    return (r >> hl) < nq ? static_cast<long long>(base + i0 + (r >> hl)) * d.ldq + static_cast<long long>(h0 + (r & hm)) * d.dim : -1LL;
+  });
+  // this lane's two rows: 16 warp + gq and the one 8 below
+  int pos[2];
+  float m[2], l[2], qmul[2], badd[2], slope[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int r = 16 * warp + gq + 8 * e, h = h0 + (r & hm);
+    pos[e] = p_lo + (r >> hl);
+    m[e] = d.sink ? ld_as_float(d.sink, d.sink_dt, h) : -INFINITY;
+    l[e] = d.sink && tq == 0 ? 1.f : 0.f;   // a row's sum is spread over its four lanes
+    badd[e] = head_bias_of(d, h);
+    slope[e] = head_slope_of(d, h);
+    qmul[e] = head_scale_of(d, h);
+  }
+  const float two_over_cap = d.softcap > 0.f ? 2.f / d.softcap : 0.f;
+  const bool shaped = d.softcap > 0.f || d.head_slope != nullptr;
+  float o[NC * 4][4];
+#pragma unroll
+  for (int i = 0; i < NC * 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
+  int E = SPLIT_MIN_E;   // the outputs are kept in units of 2^(E - 2 SPLIT_TOP), E the largest exponent of a value row so far
+  const unsigned qa_h = smem_addr(Qh) + 16 * warp * kb + lane_a(lane, kb), qa_l = qa_h + R * kb;
+  const unsigned kb_0 = smem_addr(Ts) + lane_b(lane, kb), vb_0 = smem_addr(Ts) + 2 * k_lo + lane_bt(lane, vb);
+  int b = 0;
+  for (int c0 = 0; c0 < count; c0 += N) {
+    if constexpr (PRE) {
+      if (c0 + N < count) {
+        fetch(c0 + N, b ^ 1);   // its readers passed the barrier at the end of the previous tile
+        cp_async_wait<1>();
+      } else cp_async_wait<0>();
+    } else {
+      if (c0) __syncthreads();
+      fetch(c0, 0);
+    }
+    __syncthreads();
+    if (c0 == 0) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) qmul[e] *= pow2i(qe[16 * warp + gq + 8 * e] - SPLIT_TOP);
+    }
+    const unsigned kb_h = kb_0 + b * buf, vb_h = vb_0 + b * buf;
+    const int* ke = te + b * 2 * N;
+    const int* ve = ke + N;
+    // ---- scores ----
+    float sc[NT][4], x[NT][4];   // hi hi, and the two small products
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sc[i][e] = x[i][e] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < dim16; k += 16) {
+      unsigned ah[4], al[4];
+      ldsm_x4(ah, qa_h + k * 2);
+      ldsm_x4(al, qa_l + k * 2);
+#pragma unroll
+      for (int j = 0; j < NT / 2; ++j) {
+        unsigned bh[4], bl[4];
+        ldsm_x4(bh, kb_h + 16 * j * kb + k * 2);
+        ldsm_x4(bl, kb_h + k_lo + 16 * j * kb + k * 2);
+        mma_f16(x[2 * j], al, bh[0], bh[1]);
+        mma_f16(x[2 * j + 1], al, bh[2], bh[3]);
+        mma_f16(sc[2 * j], ah, bh[0], bh[1]);
+        mma_f16(sc[2 * j + 1], ah, bh[2], bh[3]);
+        mma_f16(x[2 * j], ah, bl[0], bl[1]);
+        mma_f16(x[2 * j + 1], ah, bl[2], bl[3]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      const int2 ek = *reinterpret_cast<const int2*>(ke + 8 * i + 2 * tq);
+      const float kx[2] = {pow2i(ek.x - SPLIT_TOP), pow2i(ek.y - SPLIT_TOP)};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sc[i][e] = fmaf((sc[i][e] + x[i][e]) * kx[e & 1], qmul[e >> 1], badd[e >> 1]);
+    }
+    // a tile of neighbouring keys (no kept ones) that every query sees needs no mask per pair
+    const int f = lo + (c0 - nA), t = f + N - 1;
+    const bool whole = c0 >= nA && c0 + N <= count && t <= p_lo && (d.window <= 0 || p_hi - f < d.window) && (d.chunk <= 0 || f >= p_hi / d.chunk * d.chunk);
+    if (shaped) {
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          sc[i][e] = shaped_score(d, sc[i][e], two_over_cap, slope[e >> 1], pos[e >> 1] - key_of(c0 + 8 * i + 2 * tq + (e & 1)));
+    }
+    if (!whole) {
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = c0 + 8 * i + 2 * tq + (e & 1), kp = key_of(c), p = pos[e >> 1];
+          const bool vis = c < count && kp <= p && (d.window <= 0 || p - kp < d.window || kp < d.keep) && (d.chunk <= 0 || kp >= p / d.chunk * d.chunk);
+          if (!vis) sc[i][e] = -INFINITY;
+        }
+    }
+    // ---- weights, times 2^SPLIT_TOP and each value row's exponent against the running one ----
+    int ev = ve[lane];
+    if constexpr (N == 64) ev = max(ev, ve[lane + 32]);
+    ev = max(E, __reduce_max_sync(0xffffffffu, ev));
+    float keep_o[2] = {pow2i(E - ev), pow2i(E - ev)};
+    E = ev;
+    if constexpr (!SIG) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float top = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) top = fmaxf(top, fmaxf(sc[i][2 * r], sc[i][2 * r + 1]));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const float mn = fmaxf(m[r], top);
+        const float cr = mn == -INFINITY ? 1.f : expf(m[r] - mn);
+        m[r] = mn;
+        l[r] *= cr;
+        keep_o[r] *= cr;
+      }
+    }
+    const float mm[2] = {m[0] == -INFINITY ? 0.f : m[0], m[1] == -INFINITY ? 0.f : m[1]};   // e^(-inf - 0) = 0 where nothing is visible yet
+    unsigned ph[KT][4], pl[KT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      const int2 ej = *reinterpret_cast<const int2*>(ve + 8 * i + 2 * tq);
+      const float vx[2] = {pow2i(ej.x - E + SPLIT_TOP), pow2i(ej.y - E + SPLIT_TOP)};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if constexpr (SIG) sc[i][e] = sigmoidf_(sc[i][e]);   // of -inf: 0
+        else {
+          sc[i][e] = expf(sc[i][e] - mm[e >> 1]);
+          l[e >> 1] += sc[i][e];
+        }
+        sc[i][e] *= vx[e & 1];
+      }
+      split2(sc[i][0], sc[i][1], ph[i >> 1][(i & 1) * 2], pl[i >> 1][(i & 1) * 2]);
+      split2(sc[i][2], sc[i][3], ph[i >> 1][(i & 1) * 2 + 1], pl[i >> 1][(i & 1) * 2 + 1]);
+    }
+    // ---- weighted values: the tile's own sum first, then one fp32 addition to the running output ----
+#pragma unroll
+    for (int cc = 0; cc < NC; ++cc) {
+      if (32 * cc >= vdim16) break;
+      float y[4][4], z[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[i][e] = z[i][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < KT; ++k) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (32 * cc + 16 * i < vdim16) {
+            unsigned bh[4], bl[4];
+            ldsm_x4_t(bh, vb_h + 16 * k * vb + (32 * cc + 16 * i) * 2);
+            ldsm_x4_t(bl, vb_h + v_lo + 16 * k * vb + (32 * cc + 16 * i) * 2);
+            mma_f16(z[2 * i], pl[k], bh[0], bh[1]);
+            mma_f16(z[2 * i + 1], pl[k], bh[2], bh[3]);
+            mma_f16(y[2 * i], ph[k], bh[0], bh[1]);
+            mma_f16(y[2 * i + 1], ph[k], bh[2], bh[3]);
+            mma_f16(z[2 * i], ph[k], bl[0], bl[1]);
+            mma_f16(z[2 * i + 1], ph[k], bl[2], bl[3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[4 * cc + i][e] = fmaf(o[4 * cc + i][e], keep_o[e >> 1], y[i][e] + z[i][e]);
+    }
+    if constexpr (PRE) {
+      __syncthreads();   // this tile's readers are done
+      b ^= 1;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if constexpr (!SIG) {
+      l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+      l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+    }
+    const int row = 16 * warp + gq + 8 * r, i = row >> hl, h = h0 + (row & hm);
+    if (i >= nq) continue;
+    const long long qrow = base + i0 + i;
+    float og = SIG ? d.out_scale : d.out_scale / l[r];
+    if (d.gate) og *= sigmoidf_(ld_as_float(d.gate, d.gate_dt, qrow * d.ld_gate + h));
+    const float unit = pow2i(E - 2 * SPLIT_TOP);
+    const long long ob = qrow * d.ld_out + static_cast<long long>(h) * d.vdim;
+#pragma unroll
+    for (int t = 0; t < NC * 4; ++t) {
+      const int col = 8 * t + 2 * tq;
+      const float y0 = o[t][2 * r] * unit * og, y1 = o[t][2 * r + 1] * unit * og;
+      if (ovec) {
+        if (col < d.vdim) {
+          if (d.out_dt == VY_BF16) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(d.out) + ob + col) = __floats2bfloat162_rn(y0, y1);
+          else *reinterpret_cast<float2*>(reinterpret_cast<float*>(d.out) + ob + col) = make_float2(y0, y1);
+        }
+      } else {
+        if (col < d.vdim) st_from_float(d.out, d.out_dt, ob + col, y0);
+        if (col + 1 < d.vdim) st_from_float(d.out, d.out_dt, ob + col + 1, y1);
+      }
+    }
+  }
+}
+
+static int round16(int n) { return (n + 15) & ~15; }
+
+// key slots per (sequence, key / value head): what the step's queries can see at most (host-known bounds)
+static long long split_slots(const WinDev& d, int max_new) {
+  const long long all = static_cast<long long>(d.tw) * d.bs;
+  const long long seen = d.chunk > 0 ? static_cast<long long>(d.chunk) + max_new : d.window > 0 ? static_cast<long long>(d.window) + d.keep + max_new : all;
+  return seen < all ? seen : all;
+}
+
+long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new) {
+  return static_cast<long long>(n_seqs) * d.kv_heads * split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 2);
+}
+
+template <int MAXD, int VT, int NW, bool PRE, bool SIG>
+static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, cudaStream_t st) {
+  constexpr int R = 16 * NW, N = MAXD > 128 ? 32 : 64;
+  const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
+  const size_t kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16, bufs = PRE ? 2 : 1;
+  const size_t smem = 2 * R * kb + bufs * 2 * N * (kb + vb) + sizeof(int) * (R + bufs * 2 * N);
+  const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
+  const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q, 16);
+  const bool ovec = d.vdim % 2 == 0 && d.ld_out % 2 == 0 && al(d.out, d.out_dt == VY_BF16 ? 4 : 8);
+  static size_t allowed = 48 * 1024;
+  if (smem > allowed) {
+    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, PRE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    allowed = smem;
+  }
+  const int qn = R >> hl;
+  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, PRE, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, hl,
+                       dim16, vdim16, qvec, kvvec, ovec);
+}
+
+template <int MAXD, int VT>
+static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, bool pre, cudaStream_t st) {
+  const auto go = [&](auto sig) {
+    constexpr bool S = decltype(sig)::value;
+    if (!pre) return launch_wm<MAXD, VT, 4, false, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    if constexpr (MAXD <= 128) {
+      // 128 rows per CTA while that leaves a CTA for every SM, else 64
+      const int qn = 128 >> hl;
+      if (static_cast<long long>((max_new + qn - 1) / qn) * (d.heads >> hl) * n_seqs >= num_sms()) return launch_wm<MAXD, VT, 8, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    }
+    return launch_wm<MAXD, VT, 4, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+  };
+  return d.sigmoid ? go(std::true_type{}) : go(std::false_type{});
+}
+
+cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches) {
+  const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
+  const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && d.k_row % 4 == 0 && d.v_row % 4 == 0 && al(d.kp, 16) && al(d.vp, 16);
+  // heads per tile: the largest power of two, at most 16, that divides the heads of a key / value head
+  const int rep = d.heads / d.kv_heads;
+  int hl = 0;
+  while (hl < 4 && rep % (2 << hl) == 0) ++hl;
+  const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
+  SplitKv w = {};
+  w.cap = split_slots(d, max_new);
+  const long long slots = static_cast<long long>(n_seqs) * d.kv_heads * w.cap;
+  const bool pre = ws && al(ws, 16) && d.kv_heads <= 65535 && ws_floats >= window_attn_split_floats(d, n_seqs, max_new);
+  *launches = 1;
+  if (pre) {
+    w.row_bytes = 4 * (dim16 + vdim16);
+    w.rows = reinterpret_cast<unsigned char*>(ws);
+    w.expo = reinterpret_cast<int*>(w.rows + slots * w.row_bytes);
+    const dim3 grid(static_cast<unsigned>((w.cap + WS_ROWS - 1) / WS_ROWS), d.kv_heads, n_seqs);
+    const int big = d.dim > d.vdim ? d.dim : d.vdim;
+    cudaError_t e = big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, w, dim16, vdim16, kvvec)
+                               : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, w, dim16, vdim16, kvvec);
+    if (e != cudaSuccess) return e;
+    *launches = 2;
+  }
+  if (d.vdim > 128 || d.dim > 128) return launch_wm_pick<256, 256>(d, w, n_seqs, max_new, hl, kvvec, pre, st);   // callers keep both <= 256
+  if (d.vdim > 64) return launch_wm_pick<128, 128>(d, w, n_seqs, max_new, hl, kvvec, pre, st);
+  return d.dim <= 64 ? launch_wm_pick<64, 64>(d, w, n_seqs, max_new, hl, kvvec, pre, st) : launch_wm_pick<128, 64>(d, w, n_seqs, max_new, hl, kvvec, pre, st);
+}
+
+}  // namespace vy

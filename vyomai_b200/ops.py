@@ -1093,6 +1093,10 @@ def kv_page_write(batch: PackedBatch, k: torch.Tensor, v: torch.Tensor, k_pool: 
 ATTN_WEIGHTS = {"softmax": C["VY_ATTN_SOFTMAX"], "sigmoid": C["VY_ATTN_SIGMOID"]}
 
 
+WINDOW_ATTN_WORKSPACE_FLOATS = 1 << 27   # 512 MB: the host only knows the longest portion and table, so a step that mixes one long prompt with many
+#                                          short portions asks for far more than its rows fill; past this the kernel splits rows tile by tile
+
+
 def window_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, *, heads: int, kv_heads: int, dim: int,
                 vdim: int, scale: float, window: int, keep_first: int, sink: Optional[torch.Tensor] = None,
                 gate: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None, k_row: int = 0, v_row: int = 0, chunk: int = 0, out_scale: float = 1.0,
@@ -1115,6 +1119,10 @@ def window_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_poo
     if batch.max_new == 1 and heads // kv_heads >= 8:   # the heads-as-rows form splits keys over CTAs and merges from a scratch buffer
         need = int(_lib.lib().vy_window_attn_workspace_floats(batch.n_seqs, heads, kv_heads, vdim))
         ws = torch.empty(need, device=q.device, dtype=torch.float32) if need > 0 else None
+    elif batch.max_new > 1 and batch.block_table is not None:   # prompts: the visible rows split for the tensor cores, once
+        need = int(_lib.lib().vy_window_attn_prompt_floats(batch.n_seqs, batch.max_new, batch.block_table.shape[1], batch.block_size, kv_heads, dim, vdim,
+                                                           int(window), int(keep_first), int(chunk)))
+        ws = torch.empty(need, device=q.device, dtype=torch.float32) if 0 < need <= WINDOW_ATTN_WORKSPACE_FLOATS else None
     _lib.call("vy_window_attn", "VyWinAttn", workspace=_ptr(ws), workspace_floats=ws.numel() if ws is not None else 0, q=q.data_ptr(), ldq=q.stride(0), q_dtype=_dt(q), k_pool=k_pool.data_ptr(),
               v_pool=v_pool.data_ptr(), pool_dtype=_dt(k_pool), heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=float(scale),
               window=int(window), keep_first=int(keep_first), sink=_ptr(sink), sink_dtype=_dt(sink) if sink is not None else 0,
