@@ -64,11 +64,11 @@ __device__ __forceinline__ unsigned lane_b(int lane, int row_bytes) { return ((l
 __device__ __forceinline__ unsigned lane_bt(int lane, int row_bytes) { return ((lane & 7) + (((lane >> 3) & 1) << 3)) * row_bytes + ((lane >> 4) << 4); }
 
 // Rows [0, rows) of a block of `src` as hi / lo planes (`row_bytes` between rows of a plane, columns zero-filled up to pad16, a
-// multiple of 16 and at most MAXD), with each row's exponent in expo[row]. Row j starts at element off(j) of src or is all zero when
+// multiple of 16 and at most MAXD), with 2^(a row's exponent - drop) in unit[row]. Row j starts at element off(j) of src or is all zero when
 // off(j) < 0. Eight lanes share a row (coalesced 128-byte runs); a thread has the loads of U rows in flight before it uses any. vec: src
 // is fp32, row starts and the width are multiples of 4 elements.
 template <int NW, int MAXD, typename OffFn>
-__device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo, int row_bytes, int* expo, int rows, int width, int pad16, const void* src, int dt,
+__device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo, int row_bytes, float* unit, int drop, int rows, int width, int pad16, const void* src, int dt,
                                            bool vec, OffFn off) {
   constexpr int NI = (MAXD + 31) / 32, U = NI <= 4 ? 4 : 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
@@ -104,7 +104,7 @@ __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo,
       if (r < rows) {
         const int e = split_exponent(m);
         const float sc = split_scale(e);
-        if (l8 == 0) expo[r] = e;
+        if (l8 == 0) unit[r] = pow2i(e - drop);
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
           const int c = l8 * 4 + 32 * i;

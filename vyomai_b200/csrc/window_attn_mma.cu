@@ -8,7 +8,9 @@
 // arrive in the other buffer (cp.async) meanwhile. Without a workspace (a caller of the C ABI that lends none, or one too large to lend) each
 // CTA splits its tiles itself, which costs it about as many instructions as the softmax does.
 //
-// What bounds it: the tensor pipe (three fp16 products per fp32 one on mma.sync), then the instructions of the softmax.
+// What bounds it: the tensor pipe (three fp16 products per fp32 one on mma.sync) and the shared-memory reads that feed it, about alike, then the
+// instructions of the softmax. 4 x 2048 tokens, 8 heads of 128 over 2 key / value heads, window 512, capped: 943 us -> 267 us; 16 heads of 96 / 64
+// channels over the whole context: 2812 us -> 860 us (the fp32-FMA tiles this replaces ran at 15 TFLOP/s).
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 
@@ -16,7 +18,7 @@ namespace vy {
 
 // where the split rows of (sequence s, key / value head g) lie, and which keys they are
 struct SplitKv {
-  unsigned char* rows; int* expo;   // expo: [2][n_seqs * kv_heads * cap], keys then values
+  unsigned char* rows; float* unit;   // unit: [2][n_seqs * kv_heads * cap], 2^(exponent - SPLIT_TOP) of the keys, 2^exponent of the values
   long long cap;                    // key slots per (sequence, key / value head)
   int row_bytes;                    // 4 (dim16 + vdim16)
 };
@@ -49,29 +51,29 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
     return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
   };
   unsigned char* out = w.rows + (slot0 + r0) * w.row_bytes;
-  split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, w.expo + slot0 + r0, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
+  split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, w.unit + slot0 + r0, SPLIT_TOP, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
                               [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; });
   out += 4 * dim16;
-  split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, w.expo + all + slot0 + r0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
+  split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, w.unit + all + slot0 + r0, 0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
                               [&](int r) { return row_of(r) * d.v_row + static_cast<long long>(g) * d.vdim; });
 }
 
 // MAXD: most query / key channels; VT: value channels the accumulators hold; NW: warps (16 rows each); PRE: rows come split from the workspace
 // (two tile buffers), else the CTA splits them itself (one buffer); SIG: sigmoid weights
-template <int MAXD, int VT, int NW, bool PRE, bool SIG>
+template <int MAXD, int VT, int NW, int N, bool PRE, bool SIG>
 __global__ void __launch_bounds__(32 * NW, NW == 4 && VT <= 128 && !PRE ? 2 : 1)
 window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool qvec, bool kvvec, bool ovec) {
   pdl_trigger();
   pdl_wait();
-  constexpr int R = 16 * NW, N = MAXD > 128 ? 32 : 64, NT = N / 8, KT = N / 16;   // rows of a CTA; keys per tile, as score columns of 8 and value steps of 16
+  constexpr int R = 16 * NW, NT = N / 8, KT = N / 16;   // rows of a CTA; the tile's keys as score columns of 8 and value steps of 16
   constexpr int NC = VT / 32;   // value columns go in blocks of 32
   extern __shared__ __align__(16) unsigned char wm_smem[];
   const int kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16;   // bytes between rows: an odd multiple of 16 (ldmatrix without bank conflicts)
   const int k_lo = N * kb, v_lo = N * vb, buf = 2 * k_lo + 2 * v_lo;   // from a hi plane to its lo plane; bytes of a tile buffer
   unsigned char* Qh = wm_smem;
   unsigned char* Ts = Qh + 2 * R * kb;     // [buffers][K hi | K lo | V hi | V lo]
-  int* qe = reinterpret_cast<int*>(Ts + (PRE ? 2 : 1) * buf);   // exponents of the rows of Q, then [buffers][K | V]
-  int* te = qe + R;
+  float* qe = reinterpret_cast<float*>(Ts + (PRE ? 2 : 1) * buf);   // powers of two that undo the scaling of the rows of Q, then [buffers][K | V]
+  float* te = qe + R;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int s = blockIdx.z, h0 = blockIdx.y << hl, qn = R >> hl;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
@@ -95,13 +97,13 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
   const auto key_of = [&](int c) { return c < nA ? c : lo + (c - nA); };
   const auto fetch = [&](int c0, int b) {   // tile of keys c0 .. into buffer b, its exponents beside it
     unsigned char* T = Ts + b * buf;
-    int* e = te + b * 2 * N;
+    float* e = te + b * 2 * N;
     if constexpr (PRE) {
       const long long all = static_cast<long long>(gridDim.z) * d.kv_heads * w.cap;
       const int k16 = dim16 >> 3, v16 = vdim16 >> 3, per = 2 * (k16 + v16);   // 16-byte runs of a plane's row, of a row
       for (int x = threadIdx.x; x < 2 * N; x += 32 * NW) {
         const int j = x & (N - 1), kp = key_of(c0 + j);
-        e[x] = c0 + j < count ? w.expo[(x >= N ? all : 0) + slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)] : SPLIT_MIN_E;
+        e[x] = c0 + j < count ? w.unit[(x >= N ? all : 0) + slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)] : pow2i(SPLIT_MIN_E);
       }
       // a warp copies whole rows
       for (int j = warp; j < N; j += NW) {
@@ -122,18 +124,18 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
         const int kp = key_of(c0 + j);
         return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
       };
-      split_rows<NW, MAXD>(T, T + k_lo, kb, e, N, d.dim, dim16, d.kp, d.pool_dt, kvvec, [&](int j) {
+      split_rows<NW, MAXD>(T, T + k_lo, kb, e, SPLIT_TOP, N, d.dim, dim16, d.kp, d.pool_dt, kvvec, [&](int j) {
         const long long r = row_of(j);
         return r >= 0 ? r * d.k_row + static_cast<long long>(g) * d.dim : -1LL;
       });
-      split_rows<NW, VT>(T + 2 * k_lo, T + 2 * k_lo + v_lo, vb, e + N, N, d.vdim, vdim16, d.vp, d.pool_dt, kvvec, [&](int j) {
+      split_rows<NW, VT>(T + 2 * k_lo, T + 2 * k_lo + v_lo, vb, e + N, 0, N, d.vdim, vdim16, d.vp, d.pool_dt, kvvec, [&](int j) {
         const long long r = row_of(j);
         return r >= 0 ? r * d.v_row + static_cast<long long>(g) * d.vdim : -1LL;
       });
     }
   };
   if constexpr (PRE) fetch(0, 0);
-  split_rows<NW, MAXD>(Qh, Qh + R * kb, kb, qe, R, d.dim, dim16, d.q, d.q_dt, qvec, [&](int r) {
+  split_rows<NW, MAXD>(Qh, Qh + R * kb, kb, qe, SPLIT_TOP, R, d.dim, dim16, d.q, d.q_dt, qvec, [&](int r) {
     return (r >> hl) < nq ? static_cast<long long>(base + i0 + (r >> hl)) * d.ldq + static_cast<long long>(h0 + (r & hm)) * d.dim : -1LL;
   });
   // this lane's two rows: 16 warp + gq and the one 8 below
@@ -150,7 +152,6 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
     qmul[e] = head_scale_of(d, h);
   }
   const float two_over_cap = d.softcap > 0.f ? 2.f / d.softcap : 0.f;
-  const bool shaped = d.softcap > 0.f || d.head_slope != nullptr;
   float o[NC * 4][4];
 #pragma unroll
   for (int i = 0; i < NC * 4; ++i)
@@ -173,11 +174,11 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
     __syncthreads();
     if (c0 == 0) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) qmul[e] *= pow2i(qe[16 * warp + gq + 8 * e] - SPLIT_TOP);
+      for (int e = 0; e < 2; ++e) qmul[e] *= qe[16 * warp + gq + 8 * e];
     }
     const unsigned kb_h = kb_0 + b * buf, vb_h = vb_0 + b * buf;
-    const int* ke = te + b * 2 * N;
-    const int* ve = ke + N;
+    const float* ke = te + b * 2 * N;   // 2^(exponent - SPLIT_TOP) of each key row, 2^exponent of each value row
+    const float* ve = ke + N;
     // ---- scores ----
     float sc[NT][4], x[NT][4];   // hi hi, and the two small products
 #pragma unroll
@@ -204,20 +205,29 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
     }
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      const int2 ek = *reinterpret_cast<const int2*>(ke + 8 * i + 2 * tq);
-      const float kx[2] = {pow2i(ek.x - SPLIT_TOP), pow2i(ek.y - SPLIT_TOP)};
+      const float2 k2 = *reinterpret_cast<const float2*>(ke + 8 * i + 2 * tq);
+      const float kx[2] = {k2.x, k2.y};
 #pragma unroll
       for (int e = 0; e < 4; ++e) sc[i][e] = fmaf((sc[i][e] + x[i][e]) * kx[e & 1], qmul[e >> 1], badd[e >> 1]);
     }
     // a tile of neighbouring keys (no kept ones) that every query sees needs no mask per pair
     const int f = lo + (c0 - nA), t = f + N - 1;
     const bool whole = c0 >= nA && c0 + N <= count && t <= p_lo && (d.window <= 0 || p_hi - f < d.window) && (d.chunk <= 0 || f >= p_hi / d.chunk * d.chunk);
-    if (shaped) {
+    if (d.softcap > 0.f) {
 #pragma unroll
       for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          sc[i][e] = shaped_score(d, sc[i][e], two_over_cap, slope[e >> 1], pos[e >> 1] - key_of(c0 + 8 * i + 2 * tq + (e & 1)));
+        for (int e = 0; e < 4; ++e) sc[i][e] = cap_score(sc[i][e], d.softcap, two_over_cap);
+    }
+    if (d.head_slope) {
+      const float away[2] = {static_cast<float>(pos[0] - f - 2 * tq), static_cast<float>(pos[1] - f - 2 * tq)};   // distance to the tile's first key of this lane
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = 8 * i + (e & 1), r = e >> 1, c = c0 + j + 2 * tq;
+          sc[i][e] = fmaf(-slope[r], c0 >= nA || c >= nA ? away[r] - static_cast<float>(j) : static_cast<float>(pos[r] - c), sc[i][e]);
+        }
     }
     if (!whole) {
 #pragma unroll
@@ -230,11 +240,12 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
         }
     }
     // ---- weights, times 2^SPLIT_TOP and each value row's exponent against the running one ----
-    int ev = ve[lane];
-    if constexpr (N == 64) ev = max(ev, ve[lane + 32]);
-    ev = max(E, __reduce_max_sync(0xffffffffu, ev));
-    float keep_o[2] = {pow2i(E - ev), pow2i(E - ev)};
-    E = ev;
+    unsigned ev = __float_as_uint(ve[lane]);   // positive numbers order like their bits
+    if constexpr (N == 64) ev = max(ev, __float_as_uint(ve[lane + 32]));
+    const int e_new = max(E, static_cast<int>(__reduce_max_sync(0xffffffffu, ev) >> 23) - 127);
+    float keep_o[2] = {pow2i(E - e_new), pow2i(E - e_new)};
+    E = e_new;
+    const float v_unit = pow2i(SPLIT_TOP - E);
     if constexpr (!SIG) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -254,8 +265,8 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
     unsigned ph[KT][4], pl[KT][4];
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      const int2 ej = *reinterpret_cast<const int2*>(ve + 8 * i + 2 * tq);
-      const float vx[2] = {pow2i(ej.x - E + SPLIT_TOP), pow2i(ej.y - E + SPLIT_TOP)};
+      const float2 v2 = *reinterpret_cast<const float2*>(ve + 8 * i + 2 * tq);
+      const float vx[2] = {v2.x * v_unit, v2.y * v_unit};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if constexpr (SIG) sc[i][e] = sigmoidf_(sc[i][e]);   // of -inf: 0
@@ -347,9 +358,9 @@ long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new) {
   return static_cast<long long>(n_seqs) * d.kv_heads * split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 2);
 }
 
-template <int MAXD, int VT, int NW, bool PRE, bool SIG>
+template <int MAXD, int VT, int NW, int N, bool PRE, bool SIG>
 static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, cudaStream_t st) {
-  constexpr int R = 16 * NW, N = MAXD > 128 ? 32 : 64;
+  constexpr int R = 16 * NW;
   const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
   const size_t kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16, bufs = PRE ? 2 : 1;
   const size_t smem = 2 * R * kb + bufs * 2 * N * (kb + vb) + sizeof(int) * (R + bufs * 2 * N);
@@ -358,12 +369,12 @@ static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int 
   const bool ovec = d.vdim % 2 == 0 && d.ld_out % 2 == 0 && al(d.out, d.out_dt == VY_BF16 ? 4 : 8);
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, PRE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, N, PRE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
   const int qn = R >> hl;
-  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, PRE, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, hl,
+  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, N, PRE, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, hl,
                        dim16, vdim16, qvec, kvvec, ovec);
 }
 
@@ -371,13 +382,19 @@ template <int MAXD, int VT>
 static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, bool pre, cudaStream_t st) {
   const auto go = [&](auto sig) {
     constexpr bool S = decltype(sig)::value;
-    if (!pre) return launch_wm<MAXD, VT, 4, false, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    constexpr int N = MAXD > 128 ? 32 : 64;
+    if (!pre) return launch_wm<MAXD, VT, 4, N, false, S>(d, w, n_seqs, max_new, hl, kvvec, st);
     if constexpr (MAXD <= 128) {
-      // 128 rows per CTA while that leaves a CTA for every SM, else 64
-      const int qn = 128 >> hl;
-      if (static_cast<long long>((max_new + qn - 1) / qn) * (d.heads >> hl) * n_seqs >= num_sms()) return launch_wm<MAXD, VT, 8, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+      const auto ctas = [&](int rows) { const int qn = rows >> hl; return static_cast<long long>((max_new + qn - 1) / qn) * (d.heads >> hl) * n_seqs; };
+      // rows of a CTA: 192 on narrow key tiles (three warps per scheduler; wide values leave room for no more than two otherwise) where that is
+      // two CTAs or more per SM, 128 where that is a CTA for every SM, else 64. 8 heads of 128 over 2, 4 x 2048 tokens, window 512: 192 rows
+      // 267 us, 128 rows 285 us, 64 rows 321 us; two portions of 1000 and 37 tokens: 137, 74, 82 us; 96 / 64 channels, whole context: 885, 860 us
+      if constexpr (VT == 128) {
+        if (ctas(192) >= 2 * num_sms()) return launch_wm<MAXD, VT, 12, 32, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+      }
+      if (ctas(128) >= num_sms()) return launch_wm<MAXD, VT, 8, 64, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
     }
-    return launch_wm<MAXD, VT, 4, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    return launch_wm<MAXD, VT, 4, N, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
   };
   return d.sigmoid ? go(std::true_type{}) : go(std::false_type{});
 }
@@ -398,7 +415,7 @@ cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, f
   if (pre) {
     w.row_bytes = 4 * (dim16 + vdim16);
     w.rows = reinterpret_cast<unsigned char*>(ws);
-    w.expo = reinterpret_cast<int*>(w.rows + slots * w.row_bytes);
+    w.unit = reinterpret_cast<float*>(w.rows + slots * w.row_bytes);
     const dim3 grid(static_cast<unsigned>((w.cap + WS_ROWS - 1) / WS_ROWS), d.kv_heads, n_seqs);
     const int big = d.dim > d.vdim ? d.dim : d.vdim;
     cudaError_t e = big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, w, dim16, vdim16, kvvec)
