@@ -201,13 +201,33 @@ def _timed(fn_name: str, kw: dict, thunk):
     return rc
 
 
+def fill(struct_name: str, kw: dict):
+    """`struct_name` with the given fields set (None: left zero)."""
+    try:
+        return STRUCTS[struct_name](**kw)   # pointers take None; one call into ctypes instead of one per field
+    except TypeError:
+        return STRUCTS[struct_name](**{k: v for k, v in kw.items() if v is not None})
+
+
+_ENTRY: Dict[str, object] = {}   # entry points of the loaded library by name
+
+
+def run(fn_name: str, st) -> None:
+    """Calls `fn_name(&st)`."""
+    fn = _ENTRY.get(fn_name)
+    if fn is None:
+        fn = _ENTRY[fn_name] = getattr(lib(), fn_name)
+    rc = fn(ctypes.byref(st))
+    if rc != 0:
+        check(rc, fn_name)
+
+
 def call(fn_name: str, struct_name: str, **kw) -> None:
     """Fills `struct_name` from keyword arguments and calls `fn_name(&struct)`."""
-    st = STRUCTS[struct_name]()
-    for k, v in kw.items():
-        if v is None:
-            continue
-        setattr(st, k, v)
+    st = fill(struct_name, kw)
+    if TIMER is None:
+        run(fn_name, st)
+        return
     fn = getattr(lib(), fn_name)
     rc = _timed(fn_name, kw, lambda: fn(ctypes.byref(st)))
     check(rc, fn_name)

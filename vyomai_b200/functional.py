@@ -88,7 +88,7 @@ def pack_linears(linears) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     Parameters keep their identity (`.data` is re-pointed into the packed buffer), so state_dict
     keys, optimizers and `.grad` are unaffected. Re-packs lazily after `.to()` moved them."""
     ws = [l.weight for l in linears]
-    if not _adjacent([w.data for w in ws]):
+    if not _adjacent(ws):
         flat = torch.empty((sum(w.shape[0] for w in ws), ws[0].shape[1]), device=ws[0].device, dtype=ws[0].dtype)
         r = 0
         for w in ws:
@@ -100,7 +100,7 @@ def pack_linears(linears) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     bs = [l.bias for l in linears]
     Bv = None
     if bs[0] is not None:
-        if not _adjacent([b.data for b in bs]):
+        if not _adjacent(bs):
             flatb = torch.empty(sum(b.shape[0] for b in bs), device=bs[0].device, dtype=bs[0].dtype)
             r = 0
             for b in bs:

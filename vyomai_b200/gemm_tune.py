@@ -35,7 +35,24 @@ MAX_SCRATCH_BYTES = 4 << 30
 LOG: List[tuple] = []  # (key, winner, us, model_us) of every signature tuned in this process
 
 
+# argument blocks of vy_gemm calls by everything about them but addresses and stream (ops.gemm), made once their tiling is settled
+PLANS: Dict[tuple, bytes] = {}
+MAX_PLANS = 4096   # ragged prompts bring new row counts for ever: start over when this many have been seen
+
+
+def keep_plan(key: tuple, block: bytes) -> None:
+    if len(PLANS) >= MAX_PLANS:
+        PLANS.clear()
+    PLANS[key] = block
+
+
+def settled(key: tuple) -> bool:
+    """Has `hints` answered for good (not just for now, as while a graph is captured)?"""
+    return key in _CACHE
+
+
 def clear() -> None:
+    PLANS.clear()
     _CACHE.clear()
     LOG.clear()
 
