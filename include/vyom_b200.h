@@ -837,7 +837,12 @@ typedef struct VyLinAttn {
   float* state;
   void* out; int64_t ld_out; int32_t out_dtype;
   void* stream;
+  /* optional scratch, 16-byte aligned, of vy_linear_attn_workspace_floats(rows, ..) floats (0: none needed), and the step's packed rows: long portions
+   * then run all their chunks at once instead of one after the other */
+  int64_t rows;
+  float* workspace; int64_t workspace_floats;
 } VyLinAttn;
+VY_API int64_t vy_linear_attn_workspace_floats(int64_t rows, int32_t n_seqs, int32_t max_new, int32_t heads, int32_t dim, int32_t vdim);
 VY_API int vy_linear_attn(const VyLinAttn* p);
 
 /* Gated delta rule, state carried per sequence. Per head h (q / k head h / (heads / kv_heads)) and token:

@@ -108,6 +108,11 @@ def _ln_bwd(dy: torch.Tensor, s: torch.Tensor, gamma: torch.Tensor, beta: torch.
         if bias is not None:
             _ready(bias)
         return ds, None, None, None
+    if gamma.dtype == beta.dtype and (bias is None or bias.dtype == gamma.dtype):   # written in the parameters' type by the reduce kernel, no casts
+        new = lambda: torch.empty(gamma.shape[0], device=dy.device, dtype=gamma.dtype)  # noqa: E731
+        dgamma, dbeta, dbias = new(), new(), None if bias is None else new()
+        ds = ops.add_layernorm_bwd(dy, s, gamma, mean, rstd, dgamma_out=dgamma, dbeta_out=dbeta, dbias_out=dbias, accumulate=False, dropout=dropout)[0]
+        return ds, dgamma, dbeta, dbias
     if bias is not None:
         ds, dgamma, dbeta, dbias = ops.add_layernorm_bwd(dy, s, gamma, mean, rstd, want_dbias=True, dropout=dropout)
         return ds, dgamma.to(gamma.dtype), dbeta.to(beta.dtype), dbias.to(bias.dtype)

@@ -1,0 +1,579 @@
+// Prompt-sized linear attention with a decay per head (fixed, or per token as in the state-space recurrence), all chunks of 64 tokens at
+// once, fp32 precision on the tensor cores (split_mma.cuh). Three launches:
+//
+//   la_states   U_c = sum_j decay(j .. end of chunk c) w_j k_j v_j^T of every chunk, and the chunk's whole decay D_c
+//   la_scan     S <- D_c S + U_c chunk after chunk, element by element; the state BEFORE each chunk takes the place of U_c
+//   la_outputs  O = (Q K^T . D) V + diag(decay to i) Q S_before
+//
+// The walk this replaces for long portions (linear_attn_chunk_kernel: one CTA per sequence, head and slice of columns goes through the chunks in
+// order, on fp32 FMAs) is as long as the sequence and leaves SMs idle for few sequences; here only the scan is serial, and it is bound by the bytes
+// of the states (dim x vdim x 4 per chunk and head, written twice, read twice). q and k shared by a group of heads (state space: b and c) are
+// split, and their scores computed, once per group.
+#include "seqmix.cuh"
+#include "split_mma.cuh"
+
+namespace vy {
+
+constexpr int LM_C = 64;   // tokens per chunk
+
+// The chunks' states in the workspace: chunk c of sequence s is slot cu[s] / 64 + s + c (never more than rows / 64 + n_seqs in all)
+struct LaChunks {
+  float* U;          // [slots][heads][dim][vdim]
+  float* D;          // [slots][heads]
+  unsigned* top;     // [slots][heads] largest |S| before the chunk, as bits
+};
+__device__ __forceinline__ long long la_slot(const RecDev& d, int s, int c) { return d.cu[s] / LM_C + s + c; }
+
+// One warp: tokens 2 lane, 2 lane + 1 of a chunk of nt: log decays summed (two floats each: their differences are what counts) and write
+// strengths, as in linear_attn_chunk_kernel
+struct TokenDecay { float Lh[2], Ll[2], w[2], eL[2], es[2], whole; };
+__device__ __forceinline__ TokenDecay token_decays(const RecDev& d, long long r0, int nt, int h, int lane) {
+  const float rate = expf(ld_as_float(d.a_log, d.a_log_dt, h)), dt_b = ld_as_float(d.dt_bias, d.a_log_dt, h);
+  TokenDecay o;
+  double la[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int tt = 2 * lane + e;
+    o.w[e] = tt < nt ? softplusf_(d.dt[(r0 + tt) * d.ld_dt + h] + dt_b) : 0.f;
+    la[e] = fmaxf(-rate * o.w[e], MIN_LOG_DECAY);
+  }
+  double run = la[0] + la[1];
+#pragma unroll
+  for (int k = 1; k < 32; k <<= 1) {
+    const double x = __shfl_up_sync(0xffffffffu, run, k);
+    if (lane >= k) run += x;
+  }
+  const double end = __shfl_sync(0xffffffffu, run, 31);
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const double L = e ? run : run - la[1];
+    o.Lh[e] = static_cast<float>(L);
+    o.Ll[e] = static_cast<float>(L - static_cast<double>(o.Lh[e]));
+    o.eL[e] = expf(static_cast<float>(L));
+    o.es[e] = expf(static_cast<float>(end - L)) * o.w[e];
+  }
+  o.whole = expf(static_cast<float>(end));
+  return o;
+}
+
+// a^n, n < 128, in seven steps of repeated squaring (double: rounded once, to the fp32 result)
+__device__ __forceinline__ float power(float a, int n) {
+  double x = a, r = 1.0;
+#pragma unroll
+  for (int b = 0; b < 7; ++b) {
+    if (n >> b & 1) r *= x;
+    x *= x;
+  }
+  return static_cast<float>(r);
+}
+
+// four entries of row `row` (element offset o of src) from column c on, zero past `width`
+__device__ __forceinline__ float4 load4(const void* src, int dt, bool vec, long long o, int c, int width) {
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c >= width) return x;
+  if (vec) return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(src) + o + c);
+  return load4_any(src, dt, o, c, width);
+}
+static __device__ __noinline__ float uact_any(float x, int act) { return apply_uact(x, act); }
+// ACT: VY_UACT_NONE or VY_UACT_SILU at compile time, any other activation by a call
+template <int ACT>
+__device__ __forceinline__ float act_of(float x, int act) {
+  if constexpr (ACT == VY_UACT_NONE) return x;
+  else return act == VY_UACT_SILU ? siluf_(x) : uact_any(x, act);
+}
+template <int ACT>
+__device__ __forceinline__ float4 act4(float4 x, int act) {
+  return make_float4(act_of<ACT>(x.x, act), act_of<ACT>(x.y, act), act_of<ACT>(x.z, act), act_of<ACT>(x.w, act));
+}
+__device__ __forceinline__ float abs4(float4 x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); }
+__device__ __forceinline__ void store_split4(unsigned char* hi, unsigned char* lo, int at, float4 x, float sc) {
+  uint2 h, l;
+  split2(x.x * sc, x.y * sc, h.x, l.x);
+  split2(x.z * sc, x.w * sc, h.y, l.y);
+  *reinterpret_cast<uint2*>(hi + at) = h;
+  *reinterpret_cast<uint2*>(lo + at) = l;
+}
+// the CTA's largest value, in every thread (T threads; red: one float per warp, free before and after)
+template <int T>
+__device__ __forceinline__ float block_max(float m, float* red) {
+  m = warp_max(m);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  float x = red[0];
+#pragma unroll
+  for (int i = 1; i < T / 32; ++i) x = fmaxf(x, red[i]);
+  __syncthreads();
+  return x;
+}
+
+constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows of 64 value columns
+
+// CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w ..; tokens are the summed index, so k and the
+// weighted v are each scaled by one power of two for the whole chunk. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: see la_outputs
+// ACT: see act_of
+template <bool TD, int ACT>
+__global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
+  pdl_trigger();
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char lu_smem[];
+  const int kb = dim16 * 2 + 16;
+  unsigned char* Kh = lu_smem;
+  unsigned char* Kl = Kh + LM_C * kb;
+  unsigned char* Wh = Kl + LM_C * kb;
+  unsigned char* Wl = Wh + LM_C * LU_VB;
+  float* es = reinterpret_cast<float*>(Wl + LM_C * LU_VB);   // [64] decay to the chunk's end times write strength
+  float* red = es + LM_C;
+  const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
+  const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LM_C;
+  if (t0 >= n) return;
+  const int nt = min(LM_C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
+  const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
+  const long long r0 = base + t0, slot = la_slot(d, s, c);
+  const int row = t >> 2, c4 = (t & 3) * 4;   // loads: four threads per token row
+  float4 x[8];
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    x[i] = row < nt ? load4(d.k, d.in_dt, vec, (r0 + row) * d.ldk + static_cast<long long>(hq) * d.dim, c4 + 16 * i, d.dim) : make_float4(0.f, 0.f, 0.f, 0.f);
+    x[i] = act4<ACT>(x[i], d.in_act);
+    m = fmaxf(m, abs4(x[i]));
+  }
+  const int ek = split_exponent(block_max<LU_T>(m, red));
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (c4 + 16 * i < dim16) store_split4(Kh, Kl, row * kb + (c4 + 16 * i) * 2, x[i], split_scale(ek));
+  const unsigned ka = smem_addr(Kh) + lane_b(lane, kb) + 16 * warp * 2, wb = smem_addr(Wh) + lane_bt(lane, LU_VB);
+  float4 next[4];
+  const auto fetch = [&](int h) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) next[i] = row < nt ? load4(d.v, d.in_dt, vec, (r0 + row) * d.ldv + static_cast<long long>(h) * d.vdim + v0, c4 + 16 * i, vw) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  fetch(h0);
+  for (int h = h0; h < h0 + hp; ++h) {
+    __syncthreads();   // the previous head's readers of es and W are done
+    if constexpr (TD) {
+      if (warp == 0) {
+        const TokenDecay q = token_decays(d, r0, nt, h, lane);
+        es[2 * lane] = q.es[0];
+        es[2 * lane + 1] = q.es[1];
+        if (lane == 0 && v0 == 0) w.D[slot * d.heads + h] = q.whole;
+      }
+    } else if (t <= LM_C) {
+      if (t < LM_C) es[t] = t < nt ? power(d.decay[h], nt - 1 - t) : 0.f;
+      else if (v0 == 0) w.D[slot * d.heads + h] = power(d.decay[h], nt);
+    }
+    if (t == 0 && v0 == 0) w.top[slot * d.heads + h] = 0u;
+    float4 y[4] = {next[0], next[1], next[2], next[3]};
+    if (h + 1 < h0 + hp) fetch(h + 1);   // in flight during this head's products
+    __syncthreads();
+    float mv = 0.f;
+    const float e = es[row];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      y[i] = act4<ACT>(y[i], d.in_act);
+      y[i] = make_float4(y[i].x * e, y[i].y * e, y[i].z * e, y[i].w * e);
+      mv = fmaxf(mv, abs4(y[i]));
+    }
+    const int ew = split_exponent(block_max<LU_T>(mv, red));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) store_split4(Wh, Wl, row * LU_VB + (c4 + 16 * i) * 2, y[i], split_scale(ew));
+    __syncthreads();
+    if (16 * warp < dim16) {
+      float a[8][4], b[8][4];   // hi hi, and the two small products
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[i][k] = b[i][k] = 0.f;
+#pragma unroll
+      for (int k = 0; k < LM_C / 16; ++k) {
+        unsigned ah[4], al[4];   // k^T: stored [token][channel], read transposed (lane_b's order is what .trans turns into an A operand)
+        ldsm_x4_t(ah, ka + 16 * k * kb);
+        ldsm_x4_t(al, ka + LM_C * kb + 16 * k * kb);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          unsigned bh[4], bl[4];
+          ldsm_x4_t(bh, wb + 16 * k * LU_VB + 32 * j);
+          ldsm_x4_t(bl, wb + LM_C * LU_VB + 16 * k * LU_VB + 32 * j);
+          mma_f16(b[2 * j], al, bh[0], bh[1]);
+          mma_f16(b[2 * j + 1], al, bh[2], bh[3]);
+          mma_f16(a[2 * j], ah, bh[0], bh[1]);
+          mma_f16(a[2 * j + 1], ah, bh[2], bh[3]);
+          mma_f16(b[2 * j], ah, bl[0], bl[1]);
+          mma_f16(b[2 * j + 1], ah, bl[2], bl[3]);
+        }
+      }
+      const float u1 = pow2i(ek - SPLIT_TOP), u2 = pow2i(ew - SPLIT_TOP);
+      float* U = w.U + (slot * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int i = 16 * warp + gq + 8 * r;
+        if (i >= d.dim) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int col = 8 * j + 2 * tq;
+          const float p = (a[j][2 * r] + b[j][2 * r]) * u1 * u2, q = (a[j][2 * r + 1] + b[j][2 * r + 1]) * u1 * u2;
+          float* at = U + static_cast<long long>(i) * d.vdim + col;
+          if (col + 1 < vw && d.vdim % 2 == 0) *reinterpret_cast<float2*>(at) = make_float2(p, q);
+          else {
+            if (col < vw) at[0] = p;
+            if (col + 1 < vw) at[1] = q;
+          }
+        }
+      }
+    }
+  }
+}
+
+// V elements per thread. Bound by the bytes: every chunk's state read once and written once; eight chunks' worth is in flight per thread
+template <int V>
+__global__ void __launch_bounds__(256) la_scan_kernel(RecDev d, LaChunks w) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int P = 8;
+  const int s = blockIdx.z, h = blockIdx.y, n = d.cu[s + 1] - d.cu[s];
+  if (n <= 0) return;
+  const int e = (blockIdx.x * 256 + threadIdx.x) * V, each = d.dim * d.vdim, chunks = (n + LM_C - 1) / LM_C;
+  const bool on = e < each;
+  const long long first = la_slot(d, s, 0) * d.heads + h;
+  float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * each + e;
+  float* U = w.U + first * each + e;
+  const long long step = static_cast<long long>(d.heads) * each;
+  float S[V], u[P][V], D[P];
+  const auto get = [&](const float* p, float (&x)[V]) {
+    if constexpr (V == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p);
+      x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
+    } else x[0] = *p;
+  };
+  const auto put = [&](float* p, const float (&x)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+    else *p = x[0];
+  };
+#pragma unroll
+  for (int k = 0; k < V; ++k) S[k] = 0.f;
+  if (on && d.pos0[s] > 0) get(sp, S);
+  for (int c0 = 0; c0 < chunks; c0 += P) {
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+      if (on && c0 + p < chunks) {
+        get(U + (c0 + p) * step, u[p]);
+        D[p] = w.D[first + static_cast<long long>(c0 + p) * d.heads];
+      }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      if (c0 + p >= chunks) break;
+      const long long at = first + static_cast<long long>(c0 + p) * d.heads;
+      float m = 0.f;
+      if (on) {
+        put(U + (c0 + p) * step, S);
+#pragma unroll
+        for (int k = 0; k < V; ++k) m = fmaxf(m, fabsf(S[k]));
+      }
+      const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+      if ((threadIdx.x & 31) == 0 && mb) atomicMax(w.top + at, mb);
+      if (on) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) S[k] = fmaf(D[p], S[k], u[p][k]);
+      }
+    }
+  }
+  if (on) put(sp, S);
+}
+
+constexpr int LO_T = 128, LO_W = 4;
+
+// CTA: (chunk, 64 value columns) x (hp heads that share q and k) x sequence; warp w owns tokens 16 w .. 16 w + 15 and keeps their scores in registers
+// for all its heads. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8
+template <bool TD, int ACT>
+__global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec, bool svec) {
+  pdl_trigger();
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char lo_smem[];
+  const int kb = dim16 * 2 + 16, q_lo = LM_C * kb, v_lo = LM_C * LU_VB, s_lo = dim16 * LU_VB;
+  unsigned char* Qh = lo_smem;
+  unsigned char* Kh = Qh + 2 * q_lo;   // k until the scores are done, then V and the state of one head after the other
+  unsigned char* Vh = Kh;
+  unsigned char* Sh = Vh + 2 * v_lo;
+  float* sc = reinterpret_cast<float*>(Kh + max(2 * q_lo, 2 * v_lo + 2 * s_lo));
+  float *qu = sc, *ku = qu + LM_C, *vu = ku + LM_C, *Lh = vu + LM_C, *Ll = Lh + LM_C, *wr = Ll + LM_C, *eL = wr + LM_C;   // [64] each (eL: decay up to and with token i)
+  const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
+  const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LM_C;
+  if (t0 >= n) return;
+  const int nt = min(LM_C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
+  const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
+  const long long r0 = base + t0, slot = la_slot(d, s, c);
+  const int act = d.in_act;
+  const auto map = [act](float x) { return act_of<ACT>(x, act); };
+  split_rows<LO_W, 128>(Qh, Qh + q_lo, kb, qu, SPLIT_TOP, LM_C, d.dim, dim16, d.q, d.in_dt, vec,
+                        [&](int r) { return r < nt ? (r0 + r) * d.ldq + static_cast<long long>(hq) * d.dim : -1LL; }, map);
+  split_rows<LO_W, 128>(Kh, Kh + q_lo, kb, ku, SPLIT_TOP, LM_C, d.dim, dim16, d.k, d.in_dt, vec,
+                        [&](int r) { return r < nt ? (r0 + r) * d.ldk + static_cast<long long>(hq) * d.dim : -1LL; }, map);
+  __syncthreads();
+  const unsigned qa = smem_addr(Qh) + 16 * warp * kb + lane_a(lane, kb), kk = smem_addr(Kh) + lane_b(lane, kb);
+  const unsigned va = smem_addr(Vh) + lane_bt(lane, LU_VB), sa = smem_addr(Sh) + lane_bt(lane, LU_VB);
+  const int i0 = 16 * warp + gq;   // this lane's rows: i0 and i0 + 8
+  const float qunit[2] = {qu[i0], qu[i0 + 8]};
+  float p[8][4];   // scores q_i . k_j; a warp's tokens only see keys j < 16 (warp + 1)
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a[2][4], b[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i][e] = b[i][e] = 0.f;
+    if (j <= warp) {
+      for (int k = 0; k < dim16; k += 16) {
+        unsigned ah[4], al[4], bh[4], bl[4];
+        ldsm_x4(ah, qa + 2 * k);
+        ldsm_x4(al, qa + q_lo + 2 * k);
+        ldsm_x4(bh, kk + 16 * j * kb + 2 * k);
+        ldsm_x4(bl, kk + q_lo + 16 * j * kb + 2 * k);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          mma_f16(b[i], al, bh[2 * i], bh[2 * i + 1]);
+          mma_f16(a[i], ah, bh[2 * i], bh[2 * i + 1]);
+          mma_f16(b[i], ah, bl[2 * i], bl[2 * i + 1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[2 * j + i][e] = (a[i][e] + b[i][e]) * qunit[e >> 1] * ku[16 * j + 8 * i + 2 * tq + (e & 1)];
+  }
+  for (int h = h0; h < h0 + hp; ++h) {
+    __syncthreads();   // the readers of k, or of the previous head's values and state, are done
+    float skip = 0.f;
+    if constexpr (TD) {
+      skip = ld_as_float(d.skip, d.a_log_dt, h);
+      if (warp == 0) {
+        const TokenDecay q = token_decays(d, r0, nt, h, lane);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          Lh[2 * lane + e] = q.Lh[e];
+          Ll[2 * lane + e] = q.Ll[e];
+          wr[2 * lane + e] = q.w[e];
+          eL[2 * lane + e] = q.eL[e];
+        }
+      }
+    } else if (t <= LM_C) {   // decay^t: wr, shifted by one: eL
+      const float x = power(d.decay[h], t);
+      if (t < LM_C) wr[t] = x;
+      if (t > 0) eL[t - 1] = x;
+    }
+    const int es = split_exponent(__uint_as_float(w.top[slot * d.heads + h]));
+    const float* U = w.U + (slot * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0;
+    float4 x[8];   // sixteen threads per state row, eight rows in flight (beside the values')
+    const auto get = [&](int i) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = i + k * (LO_T / 16);
+        x[k] = r < d.dim ? load4(U, VY_F32, svec, static_cast<long long>(r) * d.vdim, (t & 15) * 4, vw) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    get(t >> 4);
+    split_rows<LO_W, 64>(Vh, Vh + v_lo, LU_VB, vu, 0, LM_C, vw, 64, d.v, d.in_dt, vec,
+                         [&](int r) { return r < nt ? (r0 + r) * d.ldv + static_cast<long long>(h) * d.vdim + v0 : -1LL; }, map);
+    for (int i = t >> 4; i < dim16; i += 8 * (LO_T / 16)) {
+      if (i >= 8 * (LO_T / 16)) get(i);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = i + k * (LO_T / 16);
+        if (r < dim16) store_split4(Sh, Sh + s_lo, r * LU_VB + (t & 15) * 8, x[k], split_scale(es));
+      }
+    }
+    __syncthreads();
+    // what the earlier chunks left: Q S
+    float o[8][4];
+    {
+      float b[8][4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][e] = b[i][e] = 0.f;
+      for (int k = 0; k < dim16; k += 16) {
+        unsigned ah[4], al[4];
+        ldsm_x4(ah, qa + 2 * k);
+        ldsm_x4(al, qa + q_lo + 2 * k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          unsigned bh[4], bl[4];
+          ldsm_x4_t(bh, sa + k * LU_VB + 32 * j);
+          ldsm_x4_t(bl, sa + s_lo + k * LU_VB + 32 * j);
+          mma_f16(b[2 * j], al, bh[0], bh[1]);
+          mma_f16(b[2 * j + 1], al, bh[2], bh[3]);
+          mma_f16(o[2 * j], ah, bh[0], bh[1]);
+          mma_f16(o[2 * j + 1], ah, bh[2], bh[3]);
+          mma_f16(b[2 * j], ah, bl[0], bl[1]);
+          mma_f16(b[2 * j + 1], ah, bl[2], bl[3]);
+        }
+      }
+      const float su = pow2i(es - SPLIT_TOP);
+      const float f[2] = {qunit[0] * eL[i0], qunit[1] * eL[i0 + 8]};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][e] = (o[i][e] + b[i][e]) * su * f[e >> 1];
+    }
+    // the weights inside the chunk, times the exponent of each value row, then scaled row by row
+    unsigned ph[4][4], pl[4][4];
+    float pu[2];
+    {
+      float x[8][4], top[2] = {0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = i0 + 8 * (e >> 1), k = 8 * j + 2 * tq + (e & 1);
+          float y = 0.f;
+          if (k <= i && j < 2 * (warp + 1)) {
+            if constexpr (TD) {
+              y = p[j][e] * (expf((Lh[i] - Lh[k]) + (Ll[i] - Ll[k])) * wr[k]);
+              if (k == i) y += skip;
+            } else y = p[j][e] * wr[i - k];
+            y *= vu[k];
+          }
+          x[j][e] = y;
+          top[e >> 1] = fmaxf(top[e >> 1], fabsf(y));
+        }
+      float f[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
+        top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
+        const int e = split_exponent(top[r]);
+        f[r] = split_scale(e);
+        pu[r] = pow2i(e - SPLIT_TOP);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        split2(x[j][0] * f[0], x[j][1] * f[0], ph[j >> 1][(j & 1) * 2], pl[j >> 1][(j & 1) * 2]);
+        split2(x[j][2] * f[1], x[j][3] * f[1], ph[j >> 1][(j & 1) * 2 + 1], pl[j >> 1][(j & 1) * 2 + 1]);
+      }
+    }
+    const float v_unit = pow2i(-SPLIT_TOP);
+    const bool pairs = svec && d.out_dt == VY_F32 && vw % 2 == 0;   // svec: vdim, strides and bases also suit pairs
+    float2 gate[2][8];   // in flight during the products below
+    if constexpr (TD) {
+      if (pairs && d.gate) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int i = i0 + 8 * r, col = 8 * j + 2 * tq;
+            if (i < nt && col < vw) gate[r][j] = *reinterpret_cast<const float2*>(d.gate + (r0 + i) * d.ld_gate + static_cast<long long>(h) * d.vdim + v0 + col);
+          }
+      }
+    }
+#pragma unroll
+    for (int cb = 0; cb < 2; ++cb) {
+      float a[4][4], b[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a[i][e] = b[i][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k > warp) break;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          unsigned bh[4], bl[4];
+          ldsm_x4_t(bh, va + 16 * k * LU_VB + 64 * cb + 32 * j);
+          ldsm_x4_t(bl, va + v_lo + 16 * k * LU_VB + 64 * cb + 32 * j);
+          mma_f16(b[2 * j], pl[k], bh[0], bh[1]);
+          mma_f16(b[2 * j + 1], pl[k], bh[2], bh[3]);
+          mma_f16(a[2 * j], ph[k], bh[0], bh[1]);
+          mma_f16(a[2 * j + 1], ph[k], bh[2], bh[3]);
+          mma_f16(b[2 * j], ph[k], bl[0], bl[1]);
+          mma_f16(b[2 * j + 1], ph[k], bl[2], bl[3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[4 * cb + i][e] = fmaf(a[i][e] + b[i][e], pu[e >> 1] * v_unit, o[4 * cb + i][e]);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = i0 + 8 * r;
+      if (i >= nt) continue;
+      const long long ob = (r0 + i) * d.ld_out + static_cast<long long>(h) * d.vdim + v0, gb = (r0 + i) * d.ld_gate + static_cast<long long>(h) * d.vdim + v0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int col = 8 * j + 2 * tq;
+        float y0 = o[j][2 * r], y1 = o[j][2 * r + 1];
+        if (pairs) {
+          if (col >= vw) continue;
+          if constexpr (TD) {
+            if (d.gate) {
+              y0 *= act_of<VY_UACT_SILU>(gate[r][j].x, d.gate_act);
+              y1 *= act_of<VY_UACT_SILU>(gate[r][j].y, d.gate_act);
+            }
+          }
+          *reinterpret_cast<float2*>(reinterpret_cast<float*>(d.out) + ob + col) = make_float2(y0, y1);
+        } else {
+          if constexpr (TD) {
+            if (d.gate && col < vw) y0 *= uact_any(d.gate[gb + col], d.gate_act);
+            if (d.gate && col + 1 < vw) y1 *= uact_any(d.gate[gb + col + 1], d.gate_act);
+          }
+          store2_any(d.out, d.out_dt, ob + col, y0, y1, vw - col);
+        }
+      }
+    }
+  }
+}
+
+// from two chunks on the three launches beat the walk
+long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim) {
+  if (max_new <= LM_C || dim > 128 || rows <= 0) return 0;
+  const long long slots = rows / LM_C + n_seqs, floats = slots * heads * (static_cast<long long>(dim) * vdim + 2) + 4;
+  return floats <= (1LL << 28) ? floats : 0;   // 1 GB: past it the walk, which keeps its state on the chip
+}
+
+template <bool TD, int ACT>
+static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st) {
+  const auto al = [](const void* p, long long ld, int a) { return reinterpret_cast<uintptr_t>(p) % (4 * a) == 0 && ld % a == 0; };
+  const bool vec = d.in_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && al(d.q, d.ldq, 4) && al(d.k, d.ldk, 4) && al(d.v, d.ldv, 4);
+  const bool svec = d.vdim % 4 == 0 && (d.out_dt != VY_F32 || al(d.out, d.ld_out, 2)) && (!d.gate || al(d.gate, d.ld_gate, 2));
+  const long long slots = rows / LM_C + n_seqs;
+  LaChunks w;
+  w.U = ws;
+  w.D = ws + slots * d.heads * static_cast<long long>(d.dim) * d.vdim;
+  w.top = reinterpret_cast<unsigned*>(w.D + slots * d.heads);
+  const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, vslices = (d.vdim + 63) / 64, chunks = (max_new + LM_C - 1) / LM_C;
+  // heads per CTA: those that share q and k, fewer while that leaves less than two CTAs per SM
+  int hp = TD ? d.heads / d.kv_heads : 1;
+  while (hp % 2 == 0 && static_cast<long long>(chunks) * vslices * (d.heads / hp) * n_seqs < 2LL * num_sms()) hp /= 2;
+  const dim3 grid(static_cast<unsigned>(chunks) * vslices, d.heads / hp, n_seqs);
+  const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + LU_T / 32);
+  const size_t q2 = 2 * LM_C * static_cast<size_t>(kb), vs = 2 * LM_C * LU_VB + 2 * static_cast<size_t>(dim16) * LU_VB;
+  const size_t smem_o = q2 + (q2 > vs ? q2 : vs) + sizeof(float) * 7 * LM_C;
+  static bool once = false;
+  if (!once) {
+    cudaError_t e = cudaFuncSetAttribute(la_states_kernel<TD, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(la_outputs_kernel<TD, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+    if (e != cudaSuccess) return e;
+    once = true;
+  }
+  cudaError_t e = launch_kernel(la_states_kernel<TD, ACT>, grid, dim3(LU_T), smem_u, st, d, w, hp, vslices, dim16, vec);
+  if (e != cudaSuccess) return e;
+  const int each = d.dim * d.vdim;
+  const bool quad = d.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(d.state) % 16 == 0 && reinterpret_cast<uintptr_t>(ws) % 16 == 0;
+  const int per = 256 * (quad ? 4 : 1);
+  const dim3 sgrid((each + per - 1) / per, d.heads, n_seqs);
+  e = quad ? launch_kernel(la_scan_kernel<4>, sgrid, dim3(256), 0, st, d, w) : launch_kernel(la_scan_kernel<1>, sgrid, dim3(256), 0, st, d, w);
+  if (e != cudaSuccess) return e;
+  return launch_kernel(la_outputs_kernel<TD, ACT>, grid, dim3(LO_T), smem_o, st, d, w, hp, vslices, dim16, vec, svec && quad);
+}
+
+template <bool TD>
+cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st) {
+  if constexpr (!TD) {
+    if (d.in_act != VY_UACT_NONE) return launch_la_mma<TD, VY_UACT_SILU>(d, n_seqs, max_new, rows, ws, st);
+  }
+  return launch_la_mma<TD, VY_UACT_NONE>(d, n_seqs, max_new, rows, ws, st);
+}
+template cudaError_t launch_linear_attn_mma<false>(const RecDev&, int, int, long long, float*, cudaStream_t);
+template cudaError_t launch_linear_attn_mma<true>(const RecDev&, int, int, long long, float*, cudaStream_t);
+
+}  // namespace vy

@@ -1047,6 +1047,11 @@ static cudaError_t launch_delta_rule(const RecDev& d, int n_seqs, cudaStream_t s
 }
 }  // namespace vy
 
+extern "C" int64_t vy_linear_attn_workspace_floats(int64_t rows, int32_t n_seqs, int32_t max_new, int32_t heads, int32_t dim, int32_t vdim) {
+  if (rows <= 0 || n_seqs <= 0 || max_new <= 0 || heads <= 0 || dim <= 0 || vdim <= 0) return 0;
+  return vy::linear_attn_mma_floats(rows, n_seqs, max_new, heads, dim, vdim);
+}
+
 extern "C" int vy_linear_attn(const VyLinAttn* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_linear_attn: null params");
@@ -1066,6 +1071,13 @@ extern "C" int vy_linear_attn(const VyLinAttn* p) {
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   cudaError_t e;
+  const long long ws_need = linear_attn_mma_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->dim, p->vdim);
+  if (ws_need > 0 && p->workspace && reinterpret_cast<uintptr_t>(p->workspace) % 16 == 0 && p->workspace_floats >= ws_need) {
+    VY_CUDA_OK(launch_linear_attn_mma<false>(d, p->n_seqs, p->max_new, p->rows, p->workspace, st));
+    VY_LAUNCH_OK();
+    count_launch(3);
+    return VY_OK;
+  }
   if (p->max_new >= LA_CHUNKED_MIN && p->dim <= 128) {
     e = launch_linear_attn_chunked(d, p->n_seqs, st);
   } else switch (pad_dim(p->dim)) {

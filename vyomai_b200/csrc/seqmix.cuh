@@ -166,9 +166,13 @@ struct RecDev {
   void* out; long long ld_out; int out_dt;
 };
 
-// Prompt-sized steps: defined in seqmix_tiled.cu and window_attn_mma.cu.
+// Prompt-sized steps: defined in seqmix_tiled.cu, window_attn_mma.cu and linear_attn_mma.cu.
 cudaError_t launch_linear_attn_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
+// All chunks at once (linear_attn_mma.cu), given linear_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); three launches
+long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
+template <bool TD>
+cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
 cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches);
 long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);   // the workspace it makes use of
 // Single tokens whose query heads share key / value rows in groups of 8 or more (latent rows): heads as the rows of a tile.

@@ -63,13 +63,33 @@ __device__ __forceinline__ unsigned lane_b(int lane, int row_bytes) { return ((l
 // B operand stored [k][n] (ldmatrix.trans), 16 k x 16 n: same registers
 __device__ __forceinline__ unsigned lane_bt(int lane, int row_bytes) { return ((lane & 7) + (((lane >> 3) & 1) << 3)) * row_bytes + ((lane >> 4) << 4); }
 
+// Rare forms as calls of their own: unrolled into every place that needs them they would push the kernels' loops out of the instruction cache
+// (la_outputs_kernel: 4.8 of 9 stall cycles per instruction were instruction fetches)
+// entries c .. c + 3 of a row of any type and alignment, zero past `width`
+static __device__ __noinline__ float4 load4_any(const void* src, int dt, long long o, int c, int width) {
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  x.x = ld_as_float(src, dt, o + c);
+  if (c + 1 < width) x.y = ld_as_float(src, dt, o + c + 1);
+  if (c + 2 < width) x.z = ld_as_float(src, dt, o + c + 2);
+  if (c + 3 < width) x.w = ld_as_float(src, dt, o + c + 3);
+  return x;
+}
+// the first `n` (of 2) values to entries at, at + 1
+static __device__ __noinline__ void store2_any(void* dst, int dt, long long at, float a, float b, int n) {
+  if (n > 0) st_from_float(dst, dt, at, a);
+  if (n > 1) st_from_float(dst, dt, at + 1, b);
+}
+
 // Rows [0, rows) of a block of `src` as hi / lo planes (`row_bytes` between rows of a plane, columns zero-filled up to pad16, a
 // multiple of 16 and at most MAXD), with 2^(a row's exponent - drop) in unit[row]. Row j starts at element off(j) of src or is all zero when
 // off(j) < 0. Eight lanes share a row (coalesced 128-byte runs); a thread has the loads of U rows in flight before it uses any. vec: src
-// is fp32, row starts and the width are multiples of 4 elements.
-template <int NW, int MAXD, typename OffFn>
+// is fp32, row starts and the width are multiples of 4 elements. map: applied to every entry read (map(0) = 0).
+struct SameValue {
+  __device__ __forceinline__ float operator()(float x) const { return x; }
+};
+template <int NW, int MAXD, typename OffFn, typename MapFn = SameValue>
 __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo, int row_bytes, float* unit, int drop, int rows, int width, int pad16, const void* src, int dt,
-                                           bool vec, OffFn off) {
+                                           bool vec, OffFn off, MapFn map = MapFn()) {
   constexpr int NI = (MAXD + 31) / 32, U = NI <= 4 ? 4 : 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
   for (int r0 = warp * 4 + (lane >> 3); r0 - (lane >> 3) < rows; r0 += NW * 4 * U) {
@@ -84,12 +104,7 @@ __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo,
         x[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (o >= 0 && c < width) {
           if (vec) x[u][i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(src) + o + c);
-          else {
-            x[u][i].x = ld_as_float(src, dt, o + c);
-            if (c + 1 < width) x[u][i].y = ld_as_float(src, dt, o + c + 1);
-            if (c + 2 < width) x[u][i].z = ld_as_float(src, dt, o + c + 2);
-            if (c + 3 < width) x[u][i].w = ld_as_float(src, dt, o + c + 3);
-          }
+          else x[u][i] = load4_any(src, dt, o, c, width);
         }
       }
     }
@@ -97,6 +112,8 @@ __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo,
     for (int u = 0; u < U; ++u) {
       const int r = r0 + u * NW * 4;
       float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < NI; ++i) x[u][i] = make_float4(map(x[u][i].x), map(x[u][i].y), map(x[u][i].z), map(x[u][i].w));
 #pragma unroll
       for (int i = 0; i < NI; ++i) m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u][i].x), fabsf(x[u][i].y)), fmaxf(fabsf(x[u][i].z), fabsf(x[u][i].w))));
 #pragma unroll

@@ -413,7 +413,7 @@ static int64_t up4(int64_t n) { return (n + 3) / 4 * 4; }
 extern "C" int64_t vy_ssd_workspace_floats(int64_t rows, int32_t n_seqs, int32_t max_new, int32_t heads, int32_t groups, int32_t dim, int32_t vdim) {
   if (rows <= 0 || n_seqs <= 0 || max_new <= 0 || heads <= 0 || groups <= 0 || dim <= 0 || vdim <= 0) return 0;
   const int64_t inner = static_cast<int64_t>(heads) * vdim, channels = inner + 2LL * groups * dim;
-  return up4(rows * inner) + (max_new > 1 ? rows * up4(channels) : 0);
+  return up4(rows * inner) + (max_new > 1 ? rows * up4(channels) : 0) + vy::linear_attn_mma_floats(rows, n_seqs, max_new, heads, dim, vdim);
 }
 
 extern "C" int vy_ssd(const VySsd* p) {
@@ -429,7 +429,8 @@ extern "C" int vy_ssd(const VySsd* p) {
   VY_CHECK_ARG(p->x && p->b && p->c && p->dt && p->conv_w && p->conv_state && p->dt_bias && p->a_log && p->skip && p->norm && p->state && p->tickets && p->out &&
                    dtype_ok(p->w_dtype) && dtype_ok(p->out_dtype), "vy_ssd: bad tensors");
   VY_CHECK_ARG(p->workspace && reinterpret_cast<uintptr_t>(p->workspace) % 16 == 0 && reinterpret_cast<uintptr_t>(p->state) % 16 == 0 &&
-                   p->workspace_floats >= vy_ssd_workspace_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->groups, p->dim, p->vdim),
+                   p->workspace_floats >= vy_ssd_workspace_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->groups, p->dim, p->vdim) -
+                                              linear_attn_mma_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->dim, p->vdim),
                "vy_ssd: the workspace is 16-byte aligned and holds vy_ssd_workspace_floats(...) floats");
   SsdDev d;
   memset(&d, 0, sizeof(d));
@@ -483,9 +484,16 @@ extern "C" int vy_ssd(const VySsd* p) {
   r.heads = p->heads; r.kv_heads = p->groups; r.dim = p->dim; r.vdim = p->vdim;
   r.state = d.state;
   r.out = d.u; r.ld_out = inner; r.out_dt = VY_F32;
-  VY_CUDA_OK(launch_ssd_chunked(r, p->n_seqs, st));
-  VY_LAUNCH_OK();
-  count_launch();
+  const long long chunk_floats = linear_attn_mma_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->dim, p->vdim);
+  if (chunk_floats > 0 && p->workspace_floats >= vy_ssd_workspace_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->groups, p->dim, p->vdim)) {
+    VY_CUDA_OK(launch_linear_attn_mma<true>(r, p->n_seqs, p->max_new, p->rows, d.xc + p->rows * d.ld_xc, st));
+    VY_LAUNCH_OK();
+    count_launch(3);
+  } else {
+    VY_CUDA_OK(launch_ssd_chunked(r, p->n_seqs, st));
+    VY_LAUNCH_OK();
+    count_launch();
+  }
   VyRmsNorm nm;
   memset(&nm, 0, sizeof(nm));
   nm.tokens = p->rows; nm.groups = p->norm_groups; nm.width = static_cast<int32_t>(inner / p->norm_groups);

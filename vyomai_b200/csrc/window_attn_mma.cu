@@ -338,8 +338,7 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
           else *reinterpret_cast<float2*>(reinterpret_cast<float*>(d.out) + ob + col) = make_float2(y0, y1);
         }
       } else {
-        if (col < d.vdim) st_from_float(d.out, d.out_dt, ob + col, y0);
-        if (col + 1 < d.vdim) st_from_float(d.out, d.out_dt, ob + col + 1, y1);
+        store2_any(d.out, d.out_dt, ob + col, y0, y1, d.vdim - col);
       }
     }
   }

@@ -1434,7 +1434,11 @@ def linear_attn(batch: PackedBatch, q: torch.Tensor, k: torch.Tensor, v: torch.T
     if decay.dtype != torch.float32 or state.dtype != torch.float32 or not state.is_contiguous():
         raise _lib.VyomError("linear_attn: decay and state are fp32")
     out = torch.empty((q.shape[0], heads * vdim), device=q.device, dtype=out_dtype or torch.float32)
-    _lib.call("vy_linear_attn", "VyLinAttn", q=q.data_ptr(), ldq=q.stride(0), k=k.data_ptr(), ldk=k.stride(0), v=v.data_ptr(), ldv=v.stride(0),
+    need = 0
+    if batch.max_new > 1:
+        need = int(_lib.lib().vy_linear_attn_workspace_floats(q.shape[0], batch.n_seqs, batch.max_new, heads, dim, vdim))
+    ws = torch.empty(need, device=q.device, dtype=torch.float32) if need > 0 else None
+    _lib.call("vy_linear_attn", "VyLinAttn", rows=q.shape[0], workspace=_ptr(ws), workspace_floats=need, q=q.data_ptr(), ldq=q.stride(0), k=k.data_ptr(), ldk=k.stride(0), v=v.data_ptr(), ldv=v.stride(0),
               in_dtype=_dt(q), in_act=UACT[in_act], heads=heads, dim=dim, vdim=vdim, decay=decay.data_ptr(), state=state.data_ptr(),
               out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out), stream=_stream(), **batch._kw())
     return out
