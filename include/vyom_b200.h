@@ -1169,6 +1169,9 @@ typedef struct VyTalkAttn {
   int32_t force_form; /* 0 = chosen by the step's shape; 1 = one query per CTA; 2 = tiled (an error if the sizes do not fit it) */
   void* stream;
 } VyTalkAttn;
+/* prompts (portions of several tokens): the scratch with which 8, 16 or 32 heads of at most 64 channels run on the tensor cores (0: none) */
+VY_API int64_t vy_talk_attn_prompt_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t heads, int32_t kv_heads, int32_t dim,
+                                          int32_t vdim, int32_t window);
 VY_API int64_t vy_talk_attn_workspace_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t heads, int32_t vdim);
 VY_API int vy_talk_attn(const VyTalkAttn* p);
 

@@ -173,6 +173,14 @@ cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 template <bool TD>
 cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
+// where the split rows of (sequence s, key / value head g) lie, and which keys they are
+struct SplitKv {
+  unsigned char* rows; float* unit;   // unit: [2][n_seqs * kv_heads * cap], 2^(exponent - SPLIT_TOP) of the keys, 2^exponent of the values
+  long long cap;                    // key slots per (sequence, key / value head)
+  int row_bytes;                    // 4 (dim16 + vdim16)
+};
+// splits the rows that some query of the step sees into ws (window_attn_split_floats(..) floats, 16-byte aligned) and says where they are
+cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st);
 cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches);
 long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);   // the workspace it makes use of
 // Single tokens whose query heads share key / value rows in groups of 8 or more (latent rows): heads as the rows of a tile.

@@ -17,27 +17,9 @@
 #include <stdlib.h>
 
 #include "seqmix.cuh"
+#include "talk_attn.cuh"
 
 namespace vy {
-
-struct TalkDev {
-  const int* cu; const int* pos0; const int* table; int tw, bs;
-  const void* q; long long ldq; int q_dt;
-  const void* kp; const void* vp; int pool_dt;
-  int heads, kv_heads, dim, vdim;
-  float scale, softcap; int window;
-  const void* talk; int talk_dt;
-  const void* sink; int sink_dt; int zero_sink;
-  const void* gate; long long ld_gate; int gate_dt; int gate_ch;
-  void* out; long long ld_out; int out_dt;
-};
-
-// the extra softmax term of head h as (score, present)
-__device__ __forceinline__ bool sink_of(const TalkDev& d, int h, float& s) {
-  if (d.sink) { s = ld_as_float(d.sink, d.sink_dt, h); return true; }
-  s = 0.f;
-  return d.zero_sink != 0;
-}
 
 // talk[h, b] -> T_s[b * Hp + h], zero for the padding heads; identity without a matrix
 template <int T>
@@ -49,11 +31,6 @@ __device__ __forceinline__ void load_talk(const TalkDev& d, float* T_s, int H, i
 }
 
 __device__ __forceinline__ int pow2_shift(int n) { return n > 0 && (n & (n - 1)) == 0 ? 31 - __clz(n) : -1; }
-
-__device__ __forceinline__ float gate_of(const TalkDev& d, long long row, int h, int c) {
-  if (!d.gate) return 1.f;
-  return sigmoidf_(ld_as_float(d.gate, d.gate_dt, row * d.ld_gate + (d.gate_ch ? static_cast<long long>(h) * d.vdim + c : h)));
-}
 
 // Stages the rows krow[j] (j < 2^kn_shift; -1 = zero row) of ALL key/value heads into dst[(g * kn + j) * ld + c] (zero-filled up to
 // width4 columns): pool rows are [G][width]. Index arithmetic by shifts when width4 / 4 is a power of two (w4_shift >= 0); global
@@ -598,6 +575,16 @@ extern "C" int64_t vy_talk_attn_workspace_floats(int32_t n_seqs, int32_t max_new
   return static_cast<int64_t>(n_seqs) * max_new * splits * heads * (vdim + 2);
 }
 
+constexpr int TALK_MMA_MIN = 16;
+
+extern "C" int64_t vy_talk_attn_prompt_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t heads, int32_t kv_heads, int32_t dim,
+                                             int32_t vdim, int32_t window) {
+  if (n_seqs <= 0 || max_new < TALK_MMA_MIN || table_width <= 0 || block_size <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || dim <= 0 || vdim <= 0) return 0;
+  vy::TalkDev d = {};
+  d.tw = table_width; d.bs = block_size; d.heads = heads; d.kv_heads = kv_heads; d.dim = dim; d.vdim = vdim; d.window = window;
+  return vy::talk_attn_mma_floats(d, n_seqs, max_new);
+}
+
 extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_talk_attn: null params");
@@ -625,6 +612,16 @@ extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q);
   const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && al(d.kp) && al(d.vp);
   const TiledPlan pl = tiled_plan(d, dim4, vdim4);
+  // prompts: the tensor-core form where the geometry suits it and the scratch is lent (16 tokens fill its 16-row products)
+  if (p->max_new >= TALK_MMA_MIN && p->force_form != 1 && p->workspace && al(p->workspace)) {
+    const long long need = talk_attn_mma_floats(d, p->n_seqs, p->max_new);
+    if (need > 0 && p->workspace_floats >= need) {
+      VY_CUDA_OK(launch_talk_attn_mma(d, p->n_seqs, p->max_new, p->workspace, st));
+      VY_LAUNCH_OK();
+      count_launch(2);
+      return VY_OK;
+    }
+  }
   VY_CHECK_ARG(p->force_form != 2 || pl.ok, "vy_talk_attn: the tiled form takes heads <= 64 and vdim <= 128 within 200 KB of shared memory");
   const bool tiled = p->force_form == 2 || (p->force_form == 0 && pl.ok && p->max_new >= 8);
   if (tiled) {

@@ -16,13 +16,6 @@
 
 namespace vy {
 
-// where the split rows of (sequence s, key / value head g) lie, and which keys they are
-struct SplitKv {
-  unsigned char* rows; float* unit;   // unit: [2][n_seqs * kv_heads * cap], 2^(exponent - SPLIT_TOP) of the keys, 2^exponent of the values
-  long long cap;                    // key slots per (sequence, key / value head)
-  int row_bytes;                    // 4 (dim16 + vdim16)
-};
-
 // the keys a portion sees, from its first query on: slots [0, nA) are positions [0, nA) (kept first tokens), the others positions from lo on
 __device__ __forceinline__ void portion_keys(const WinDev& d, int p0, int& nA, int& lo) {
   lo = d.chunk > 0 ? p0 / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p0 - d.window + 1, 0);
@@ -357,6 +350,22 @@ long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new) {
   return static_cast<long long>(n_seqs) * d.kv_heads * split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 2);
 }
 
+static bool kv_quads(const WinDev& d) {
+  const auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  return d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && d.k_row % 4 == 0 && d.v_row % 4 == 0 && al(d.kp) && al(d.vp);
+}
+
+cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st) {
+  const int dim16 = round16(d.dim), vdim16 = round16(d.vdim), big = d.dim > d.vdim ? d.dim : d.vdim;
+  w->cap = split_slots(d, max_new);
+  w->row_bytes = 4 * (dim16 + vdim16);
+  w->rows = reinterpret_cast<unsigned char*>(ws);
+  w->unit = reinterpret_cast<float*>(w->rows + static_cast<long long>(n_seqs) * d.kv_heads * w->cap * w->row_bytes);
+  const dim3 grid(static_cast<unsigned>((w->cap + WS_ROWS - 1) / WS_ROWS), d.kv_heads, n_seqs);
+  return big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d))
+                    : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d));
+}
+
 template <int MAXD, int VT, int NW, int N, bool PRE, bool SIG>
 static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, cudaStream_t st) {
   constexpr int R = 16 * NW;
@@ -400,25 +409,16 @@ static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs,
 
 cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches) {
   const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
-  const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && d.k_row % 4 == 0 && d.v_row % 4 == 0 && al(d.kp, 16) && al(d.vp, 16);
+  const bool kvvec = kv_quads(d);
   // heads per tile: the largest power of two, at most 16, that divides the heads of a key / value head
   const int rep = d.heads / d.kv_heads;
   int hl = 0;
   while (hl < 4 && rep % (2 << hl) == 0) ++hl;
-  const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
   SplitKv w = {};
-  w.cap = split_slots(d, max_new);
-  const long long slots = static_cast<long long>(n_seqs) * d.kv_heads * w.cap;
   const bool pre = ws && al(ws, 16) && d.kv_heads <= 65535 && ws_floats >= window_attn_split_floats(d, n_seqs, max_new);
   *launches = 1;
   if (pre) {
-    w.row_bytes = 4 * (dim16 + vdim16);
-    w.rows = reinterpret_cast<unsigned char*>(ws);
-    w.unit = reinterpret_cast<float*>(w.rows + slots * w.row_bytes);
-    const dim3 grid(static_cast<unsigned>((w.cap + WS_ROWS - 1) / WS_ROWS), d.kv_heads, n_seqs);
-    const int big = d.dim > d.vdim ? d.dim : d.vdim;
-    cudaError_t e = big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, w, dim16, vdim16, kvvec)
-                               : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, w, dim16, vdim16, kvvec);
+    cudaError_t e = launch_window_attn_split(d, n_seqs, max_new, ws, &w, st);
     if (e != cudaSuccess) return e;
     *launches = 2;
   }

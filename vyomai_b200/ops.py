@@ -1345,6 +1345,9 @@ def talk_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_pool:
     out = torch.empty((q.shape[0], heads * vdim), device=q.device, dtype=out_dtype or q.dtype)
     tw = batch.block_table.shape[1] if batch.block_table is not None else 0
     need = int(_lib.lib().vy_talk_attn_workspace_floats(batch.n_seqs, batch.max_new, tw, batch.block_size, heads, vdim)) if form != "tiled" else 0
+    if form is None and batch.max_new > 1:   # prompts: the visible rows split for the tensor cores
+        more = int(_lib.lib().vy_talk_attn_prompt_floats(batch.n_seqs, batch.max_new, tw, batch.block_size, heads, kv_heads, dim, vdim, int(window)))
+        need = max(need, more if more <= WINDOW_ATTN_WORKSPACE_FLOATS else 0)
     ws = torch.empty(need, device=q.device, dtype=torch.float32) if need > 0 else None
     _lib.call("vy_talk_attn", "VyTalkAttn", q=q.data_ptr(), ldq=q.stride(0), q_dtype=_dt(q), k_pool=k_pool.data_ptr(), v_pool=v_pool.data_ptr(),
               pool_dtype=_dt(k_pool), heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=float(scale), softcap=float(softcap), window=int(window),
