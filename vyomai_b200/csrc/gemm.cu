@@ -202,6 +202,13 @@ static PoisonSlot* poison_slot() {
   return &s;
 }
 static std::atomic<int> g_gemm_launch_id{0};
+bool poison_ref(PoisonRef* r) {
+  PoisonSlot* ps = poison_slot();
+  if (!ps) return false;
+  const int lid = g_gemm_launch_id.fetch_add(1, std::memory_order_relaxed) + 1;
+  *r = {ps->dev, ps->host_dev, lid & 0x7fffffff ? lid & 0x7fffffff : 1};
+  return true;
+}
 
 }  // namespace vy
 
@@ -277,10 +284,7 @@ extern "C" int vy_gemm(const VyGemm* p) {
               *reinterpret_cast<volatile int*>(ps->host));
     return VY_ERR_CUDA;
   }
-  g.poison.flag = ps->dev;
-  g.poison.host = ps->host_dev;
-  int lid = g_gemm_launch_id.fetch_add(1, std::memory_order_relaxed) + 1;
-  g.poison.id = lid & 0x7fffffff ? lid & 0x7fffffff : 1;
+  poison_ref(&g.poison);
   g.M = p->M; g.N = p->N; g.K = p->K;
   g.epi = p->epi; g.act = p->act; g.transposed_out = p->transposed_out;
   g.gate_act = gate_act;

@@ -4,6 +4,7 @@
 #include <math.h>
 
 #include "vy_common.cuh"
+#include "vy_ptx.cuh"   // warp_sum, warp_max
 
 namespace vy {
 
@@ -20,17 +21,6 @@ __device__ __forceinline__ float apply_uact(float x, int act) {
   }
 }
 constexpr float MIN_LOG_DECAY = -1e4f;   // exp of it is 0 in fp32; keeps sums and differences of log decays finite
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // cap * tanh(s / cap) as cap * (1 - 2 / (1 + e^(2 s / cap))): expf and a fast reciprocal, absolute error a few 1e-7 * cap (the softmax
 // that follows depends on score differences, i.e. on absolute error); e^x overflowing to inf gives exactly cap, underflow exactly -cap
 __device__ __forceinline__ float cap_score(float s, float cap, float two_over_cap) {
@@ -173,11 +163,13 @@ cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 template <bool TD>
 cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
-// where the split rows of (sequence s, key / value head g) lie, and which keys they are
+// Where the split rows of (sequence s, key / value head g) lie: slot (s * kv_heads + g) * cap + i holds the i-th key, K hi | K lo | V hi | V lo and 16 bytes
+// with the numbers that undo the scaling, 2^(exponent - SPLIT_TOP) of the key row and 2^exponent of the value row. The 16 bytes also make the
+// distance between rows an odd multiple of 16, as ldmatrix wants it in shared memory: a run of rows is one copy.
 struct SplitKv {
-  unsigned char* rows; float* unit;   // unit: [2][n_seqs * kv_heads * cap], 2^(exponent - SPLIT_TOP) of the keys, 2^exponent of the values
-  long long cap;                    // key slots per (sequence, key / value head)
-  int row_bytes;                    // 4 (dim16 + vdim16)
+  unsigned char* rows;
+  long long cap;   // key slots per (sequence, key / value head)
+  int row_bytes;   // 4 (dim16 + vdim16) + 16
 };
 // splits the rows that some query of the step sees into ws (window_attn_split_floats(..) floats, 16-byte aligned) and says where they are
 cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st);

@@ -57,7 +57,6 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
   const int p0 = d.pos0[s], p_lo = p0 + i0, p_hi = p_lo + nq - 1;
   const int lo = d.window > 0 ? max(p_lo - d.window + 1, 0) : 0, lo0 = d.window > 0 ? max(p0 - d.window + 1, 0) : 0;
   const int count = p_hi - lo + 1;
-  const long long all = static_cast<long long>(gridDim.y) * G * w.cap;
   // one tile's K (part 0) or V (part 1) rows of every key / value head; past the end: zeros
   const auto fetch = [&](int c0, int part) {
     const int w16 = (part ? vdim16 : dim16) >> 3, each = 2 * w16, rb = part ? vb : kb, pl = part ? v_lo : k_lo;
@@ -66,7 +65,7 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
     for (int x = t; x < G * N; x += TM_T) {
       const int g = x / N, j = x & (N - 1);
       const long long at = (static_cast<long long>(s) * G + g) * w.cap + (lo - lo0) + min(c0 + j, count - 1);
-      un[x] = c0 + j < count ? w.unit[(part ? all : 0) + at] : pow2i(SPLIT_MIN_E);
+      un[x] = c0 + j < count ? reinterpret_cast<const float*>(w.rows + at * w.row_bytes + 4 * (dim16 + vdim16))[part] : pow2i(SPLIT_MIN_E);
     }
     for (int x = t; x < G * N * each; x += TM_T) {
       const int r = x / each, c = x - r * each, g = r / N, j = r & (N - 1);

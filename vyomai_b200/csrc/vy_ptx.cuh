@@ -86,6 +86,7 @@ struct PoisonRef {
   int* host;  // mapped pinned host memory, one per device
   int id;     // id of this launch (never 0)
 };
+bool poison_ref(PoisonRef* r);  // gemm.cu: the flags of the current device, a fresh launch id
 template <bool CLUSTER_SCOPE = false>
 VY_DEVINL void mbar_wait_soft(uint64_t* bar, uint32_t parity, const PoisonRef& poison) {
   uint32_t spins = 0;

@@ -4,15 +4,17 @@
 // A first launch splits every key and value row that some query of the step sees, once, into a workspace in the order the tiles read
 // them ([sequence][key / value head][key]: K hi | K lo | V hi | V lo, the bytes of the fp32 rows). In the second, a CTA owns 16 rows per warp:
 // 2^hl query heads of one key / value head times the rows / 2^hl queries, so that heads that share keys share the key tiles and the window's
-// edges waste little. A warp keeps its scores, weights and outputs in registers from one product to the next; the next tile's rows
-// arrive in the other buffer (cp.async) meanwhile. Without a workspace (a caller of the C ABI that lends none, or one too large to lend) each
-// CTA splits its tiles itself, which costs it about as many instructions as the softmax does.
+// edges waste little. A warp keeps its scores, weights and outputs in registers from one product to the next. Tiles of keys arrive by bulk copies
+// into a ring of buffers; a warp waits for a tile, never for another warp, and the warp that is through with a buffer last refills it. (With CTA
+// barriers per tile all warps are in the same phase: 267 and 854 us instead of the 235 and 548 below.) Without a workspace (a caller of the C
+// ABI that lends none, or one too large to lend) each CTA splits its tiles itself, which costs it about as many instructions as the softmax does.
 //
 // What bounds it: the tensor pipe (three fp16 products per fp32 one on mma.sync) and the shared-memory reads that feed it, about alike, then the
-// instructions of the softmax. 4 x 2048 tokens, 8 heads of 128 over 2 key / value heads, window 512, capped: 943 us -> 267 us; 16 heads of 96 / 64
-// channels over the whole context: 2812 us -> 860 us (the fp32-FMA tiles this replaces ran at 15 TFLOP/s).
+// instructions of the softmax. 4 x 2048 tokens, 8 heads of 128 over 2 key / value heads, window 512, capped: 943 us -> 235 us; 16 heads of 96 / 64
+// channels over the whole context: 2812 us -> 548 us (the fp32-FMA tiles this replaces ran at 15 TFLOP/s).
 #include "seqmix.cuh"
 #include "split_mma.cuh"
+#include "vy_ptx.cuh"
 
 namespace vy {
 
@@ -20,6 +22,11 @@ namespace vy {
 __device__ __forceinline__ void portion_keys(const WinDev& d, int p0, int& nA, int& lo) {
   lo = d.chunk > 0 ? p0 / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p0 - d.window + 1, 0);
   nA = d.window <= 0 ? 0 : min(d.keep, lo);
+}
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 constexpr int WS_T = 256, WS_ROWS = WS_T / 8;   // splitting launch: eight lanes per row
@@ -35,7 +42,6 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
   const int count = n > 0 ? nA + p0 + n - lo : 0;
   const int* tab = d.table + static_cast<long long>(s) * d.tw;
   const long long slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
-  const long long all = static_cast<long long>(gridDim.z) * d.kv_heads * w.cap;
   const int r0 = blockIdx.x * WS_ROWS;
   if (r0 >= count) return;
   const int rows = min(WS_ROWS, count - r0);
@@ -44,29 +50,33 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
     return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
   };
   unsigned char* out = w.rows + (slot0 + r0) * w.row_bytes;
-  split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, w.unit + slot0 + r0, SPLIT_TOP, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
-                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; });
+  float* unit = reinterpret_cast<float*>(out + 4 * (dim16 + vdim16));
+  split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, unit, SPLIT_TOP, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
+                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; }, SameValue(), w.row_bytes / 4);
   out += 4 * dim16;
-  split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, w.unit + all + slot0 + r0, 0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
-                              [&](int r) { return row_of(r) * d.v_row + static_cast<long long>(g) * d.vdim; });
+  split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, unit + 1, 0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
+                              [&](int r) { return row_of(r) * d.v_row + static_cast<long long>(g) * d.vdim; }, SameValue(), w.row_bytes / 4);
 }
 
-// MAXD: most query / key channels; VT: value channels the accumulators hold; NW: warps (16 rows each); PRE: rows come split from the workspace
-// (two tile buffers), else the CTA splits them itself (one buffer); SIG: sigmoid weights
-template <int MAXD, int VT, int NW, int N, bool PRE, bool SIG>
+// MAXD: most query / key channels; VT: value channels the accumulators hold; NW: warps (16 rows each); N: keys per tile; NS: tile buffers; PRE: rows
+// come split from the workspace, else the CTA splits them itself (one buffer); SIG: sigmoid weights
+template <int MAXD, int VT, int NW, int N, int NS, bool PRE, bool SIG>
 __global__ void __launch_bounds__(32 * NW, NW == 4 && VT <= 128 && !PRE ? 2 : 1)
-window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool qvec, bool kvvec, bool ovec) {
+window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16, int vdim16, bool qvec, bool kvvec, bool ovec) {
   pdl_trigger();
   pdl_wait();
   constexpr int R = 16 * NW, NT = N / 8, KT = N / 16;   // rows of a CTA; the tile's keys as score columns of 8 and value steps of 16
   constexpr int NC = VT / 32;   // value columns go in blocks of 32
   extern __shared__ __align__(16) unsigned char wm_smem[];
-  const int kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16;   // bytes between rows: an odd multiple of 16 (ldmatrix without bank conflicts)
-  const int k_lo = N * kb, v_lo = N * vb, buf = 2 * k_lo + 2 * v_lo;   // from a hi plane to its lo plane; bytes of a tile buffer
+  // bytes between rows (odd multiples of 16: ldmatrix without bank conflicts), from a hi entry to its lo entry, to the values, of a tile buffer
+  const int qb = dim16 * 2 + 16, kb = PRE ? w.row_bytes : qb, vb = PRE ? w.row_bytes : vdim16 * 2 + 16;
+  const int k_lo = PRE ? 2 * dim16 : N * kb, v_lo = PRE ? 2 * vdim16 : N * vb, v_at = 2 * k_lo, buf = PRE ? N * kb : 2 * N * (kb + vb);
   unsigned char* Qh = wm_smem;
-  unsigned char* Ts = Qh + 2 * R * kb;     // [buffers][K hi | K lo | V hi | V lo]
-  float* qe = reinterpret_cast<float*>(Ts + (PRE ? 2 : 1) * buf);   // powers of two that undo the scaling of the rows of Q, then [buffers][K | V]
+  unsigned char* Ts = Qh + 2 * R * qb;     // [buffers]: rows of the workspace, or K hi | K lo | V hi | V lo
+  float* qe = reinterpret_cast<float*>(Ts + NS * buf);   // powers of two that undo the scaling of the rows of Q, then (!PRE) [K | V]
   float* te = qe + R;
+  uint64_t* full = reinterpret_cast<uint64_t*>(te + (PRE ? 0 : 2 * N));   // PRE: a buffer's tile has arrived
+  int* done = reinterpret_cast<int*>(full + NS);                     // PRE: warps that are through with a buffer, counted up for ever
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int s = blockIdx.z, h0 = blockIdx.y << hl, qn = R >> hl;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
@@ -90,45 +100,46 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
   const auto key_of = [&](int c) { return c < nA ? c : lo + (c - nA); };
   const auto fetch = [&](int c0, int b) {   // tile of keys c0 .. into buffer b, its exponents beside it
     unsigned char* T = Ts + b * buf;
-    float* e = te + b * 2 * N;
-    if constexpr (PRE) {
-      const long long all = static_cast<long long>(gridDim.z) * d.kv_heads * w.cap;
-      const int k16 = dim16 >> 3, v16 = vdim16 >> 3, per = 2 * (k16 + v16);   // 16-byte runs of a plane's row, of a row
-      for (int x = threadIdx.x; x < 2 * N; x += 32 * NW) {
-        const int j = x & (N - 1), kp = key_of(c0 + j);
-        e[x] = c0 + j < count ? w.unit[(x >= N ? all : 0) + slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)] : pow2i(SPLIT_MIN_E);
-      }
-      // a warp copies whole rows
-      for (int j = warp; j < N; j += NW) {
-        const int kp = key_of(min(c0 + j, count - 1));
-        const unsigned char* src = w.rows + (slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)) * w.row_bytes;
-        const unsigned dst = smem_addr(T);
-        for (int x = lane; x < per; x += 32) {
-          int o;   // byte offset in the buffer
-          if (x < 2 * k16) o = x < k16 ? j * kb + 16 * x : k_lo + j * kb + 16 * (x - k16);
-          else o = 2 * k_lo + (x < 2 * k16 + v16 ? j * vb + 16 * (x - 2 * k16) : v_lo + j * vb + 16 * (x - 2 * k16 - v16));
-          cp_async16(dst + o, src + 16 * x, c0 + j < count);
+    if constexpr (PRE) {   // by one warp: runs of neighbouring slots, one copy each; rows past the end are zeros
+      const int nk = min(N, count - c0);
+      for (int x = lane; x < (N - nk) * (kb / 16); x += 32) *reinterpret_cast<uint4*>(T + nk * kb + 16 * x) = make_uint4(0, 0, 0, 0);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&full[b], static_cast<unsigned>(nk) * w.row_bytes);
+        for (int j = 0; j < nk;) {   // kept tokens and the band are a run each; kept tokens beyond the portion's own lie at the band's start
+          const int c = c0 + j, kp = key_of(c);
+          const int run = min(nk - j, c >= nA ? nk : (kp < nA0 ? nA0 - c : nA - c));
+          bulk_load(T + j * kb, w.rows + (slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)) * w.row_bytes, static_cast<unsigned>(run) * w.row_bytes, &full[b]);
+          j += run;
         }
       }
-      cp_async_commit();
     } else {
       const auto row_of = [&](int j) {
         if (c0 + j >= count) return -1LL;
         const int kp = key_of(c0 + j);
         return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
       };
-      split_rows<NW, MAXD>(T, T + k_lo, kb, e, SPLIT_TOP, N, d.dim, dim16, d.kp, d.pool_dt, kvvec, [&](int j) {
+      split_rows<NW, MAXD>(T, T + k_lo, kb, te, SPLIT_TOP, N, d.dim, dim16, d.kp, d.pool_dt, kvvec, [&](int j) {
         const long long r = row_of(j);
         return r >= 0 ? r * d.k_row + static_cast<long long>(g) * d.dim : -1LL;
       });
-      split_rows<NW, VT>(T + 2 * k_lo, T + 2 * k_lo + v_lo, vb, e + N, 0, N, d.vdim, vdim16, d.vp, d.pool_dt, kvvec, [&](int j) {
+      split_rows<NW, VT>(T + v_at, T + v_at + v_lo, vb, te + N, 0, N, d.vdim, vdim16, d.vp, d.pool_dt, kvvec, [&](int j) {
         const long long r = row_of(j);
         return r >= 0 ? r * d.v_row + static_cast<long long>(g) * d.vdim : -1LL;
       });
     }
   };
-  if constexpr (PRE) fetch(0, 0);
-  split_rows<NW, MAXD>(Qh, Qh + R * kb, kb, qe, SPLIT_TOP, R, d.dim, dim16, d.q, d.q_dt, qvec, [&](int r) {
+  const int tiles = (count + N - 1) / N;
+  if constexpr (PRE) {
+    if (threadIdx.x < NS) {
+      mbar_init(&full[threadIdx.x], 1);
+      done[threadIdx.x] = 0;
+    }
+    fence_mbar_init();
+    __syncthreads();
+    if (warp < min(NS, tiles)) fetch(warp * N, warp);
+  }
+  split_rows<NW, MAXD>(Qh, Qh + R * qb, qb, qe, SPLIT_TOP, R, d.dim, dim16, d.q, d.q_dt, qvec, [&](int r) {
     return (r >> hl) < nq ? static_cast<long long>(base + i0 + (r >> hl)) * d.ldq + static_cast<long long>(h0 + (r & hm)) * d.dim : -1LL;
   });
   // this lane's two rows: 16 warp + gq and the one 8 below
@@ -151,27 +162,27 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
   int E = SPLIT_MIN_E;   // the outputs are kept in units of 2^(E - 2 SPLIT_TOP), E the largest exponent of a value row so far
-  const unsigned qa_h = smem_addr(Qh) + 16 * warp * kb + lane_a(lane, kb), qa_l = qa_h + R * kb;
-  const unsigned kb_0 = smem_addr(Ts) + lane_b(lane, kb), vb_0 = smem_addr(Ts) + 2 * k_lo + lane_bt(lane, vb);
-  int b = 0;
-  for (int c0 = 0; c0 < count; c0 += N) {
+  const unsigned qa_h = smem_addr(Qh) + 16 * warp * qb + lane_a(lane, qb), qa_l = qa_h + R * qb;
+  const unsigned kb_0 = smem_addr(Ts) + lane_b(lane, kb), vb_0 = smem_addr(Ts) + v_at + lane_bt(lane, vb);
+  if constexpr (PRE) __syncthreads();   // Q is there; from here on the warps wait for tiles, not for one another, so that one's softmax meets another's products
+  for (int it = 0; it < tiles; ++it) {
+    const int c0 = it * N, b = it % NS;
     if constexpr (PRE) {
-      if (c0 + N < count) {
-        fetch(c0 + N, b ^ 1);   // its readers passed the barrier at the end of the previous tile
-        cp_async_wait<1>();
-      } else cp_async_wait<0>();
+      mbar_wait_soft(&full[b], (it / NS) & 1, poison);
     } else {
       if (c0) __syncthreads();
       fetch(c0, 0);
+      __syncthreads();
     }
-    __syncthreads();
     if (c0 == 0) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) qmul[e] *= qe[16 * warp + gq + 8 * e];
     }
     const unsigned kb_h = kb_0 + b * buf, vb_h = vb_0 + b * buf;
-    const float* ke = te + b * 2 * N;   // 2^(exponent - SPLIT_TOP) of each key row, 2^exponent of each value row
-    const float* ve = ke + N;
+    // 2^(exponent - SPLIT_TOP) of each key row, 2^exponent of each value row
+    const int ustep = PRE ? w.row_bytes / 4 : 1;
+    const float* ke = PRE ? reinterpret_cast<const float*>(Ts + b * buf + 4 * (dim16 + vdim16)) : te;
+    const float* ve = PRE ? ke + 1 : te + N;
     // ---- scores ----
     float sc[NT][4], x[NT][4];   // hi hi, and the two small products
 #pragma unroll
@@ -198,8 +209,7 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
     }
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      const float2 k2 = *reinterpret_cast<const float2*>(ke + 8 * i + 2 * tq);
-      const float kx[2] = {k2.x, k2.y};
+      const float kx[2] = {ke[(8 * i + 2 * tq) * ustep], ke[(8 * i + 2 * tq + 1) * ustep]};
 #pragma unroll
       for (int e = 0; e < 4; ++e) sc[i][e] = fmaf((sc[i][e] + x[i][e]) * kx[e & 1], qmul[e >> 1], badd[e >> 1]);
     }
@@ -233,8 +243,8 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
         }
     }
     // ---- weights, times 2^SPLIT_TOP and each value row's exponent against the running one ----
-    unsigned ev = __float_as_uint(ve[lane]);   // positive numbers order like their bits
-    if constexpr (N == 64) ev = max(ev, __float_as_uint(ve[lane + 32]));
+    unsigned ev = __float_as_uint(ve[lane * ustep]);   // positive numbers order like their bits
+    if constexpr (N == 64) ev = max(ev, __float_as_uint(ve[(lane + 32) * ustep]));
     const int e_new = max(E, static_cast<int>(__reduce_max_sync(0xffffffffu, ev) >> 23) - 127);
     float keep_o[2] = {pow2i(E - e_new), pow2i(E - e_new)};
     E = e_new;
@@ -258,8 +268,7 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
     unsigned ph[KT][4], pl[KT][4];
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      const float2 v2 = *reinterpret_cast<const float2*>(ve + 8 * i + 2 * tq);
-      const float vx[2] = {v2.x * v_unit, v2.y * v_unit};
+      const float vx[2] = {ve[(8 * i + 2 * tq) * ustep] * v_unit, ve[(8 * i + 2 * tq + 1) * ustep] * v_unit};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if constexpr (SIG) sc[i][e] = sigmoidf_(sc[i][e]);   // of -inf: 0
@@ -303,9 +312,15 @@ window_attn_mma_kernel(WinDev d, SplitKv w, int hl, int dim16, int vdim16, bool 
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[4 * cc + i][e] = fmaf(o[4 * cc + i][e], keep_o[e >> 1], y[i][e] + z[i][e]);
     }
-    if constexpr (PRE) {
-      __syncthreads();   // this tile's readers are done
-      b ^= 1;
+    if constexpr (PRE) {   // the warp that is through with a buffer last refills it
+      __syncwarp();
+      int last = 0;
+      if (lane == 0) {
+        __threadfence_block();
+        last = atomicAdd(&done[b], 1) % NW == NW - 1;
+        __threadfence_block();
+      }
+      if (__shfl_sync(0xffffffffu, last, 0) && it + NS < tiles) fetch((it + NS) * N, b);
     }
   }
 #pragma unroll
@@ -347,7 +362,7 @@ static long long split_slots(const WinDev& d, int max_new) {
 }
 
 long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new) {
-  return static_cast<long long>(n_seqs) * d.kv_heads * split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 2);
+  return static_cast<long long>(n_seqs) * d.kv_heads * split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 4);
 }
 
 static bool kv_quads(const WinDev& d) {
@@ -358,31 +373,32 @@ static bool kv_quads(const WinDev& d) {
 cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st) {
   const int dim16 = round16(d.dim), vdim16 = round16(d.vdim), big = d.dim > d.vdim ? d.dim : d.vdim;
   w->cap = split_slots(d, max_new);
-  w->row_bytes = 4 * (dim16 + vdim16);
+  w->row_bytes = 4 * (dim16 + vdim16) + 16;
   w->rows = reinterpret_cast<unsigned char*>(ws);
-  w->unit = reinterpret_cast<float*>(w->rows + static_cast<long long>(n_seqs) * d.kv_heads * w->cap * w->row_bytes);
   const dim3 grid(static_cast<unsigned>((w->cap + WS_ROWS - 1) / WS_ROWS), d.kv_heads, n_seqs);
   return big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d))
                     : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d));
 }
 
-template <int MAXD, int VT, int NW, int N, bool PRE, bool SIG>
+template <int MAXD, int VT, int NW, int N, int NS, bool PRE, bool SIG>
 static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, cudaStream_t st) {
   constexpr int R = 16 * NW;
   const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
-  const size_t kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16, bufs = PRE ? 2 : 1;
-  const size_t smem = 2 * R * kb + bufs * 2 * N * (kb + vb) + sizeof(int) * (R + bufs * 2 * N);
+  const size_t kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16, bufs = NS;
+  const size_t smem = 2 * R * kb + (PRE ? bufs * N * (2 * (kb + vb) - 48) : 2 * N * (kb + vb)) + sizeof(float) * (R + (PRE ? 0 : 2 * N)) + 12 * NS;
   const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q, 16);
   const bool ovec = d.vdim % 2 == 0 && d.ld_out % 2 == 0 && al(d.out, d.out_dt == VY_BF16 ? 4 : 8);
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, N, PRE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, N, NS, PRE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
+  PoisonRef poison = {};
+  if (PRE && !poison_ref(&poison)) return cudaErrorMemoryAllocation;
   const int qn = R >> hl;
-  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, N, PRE, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, hl,
+  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, N, NS, PRE, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, poison, hl,
                        dim16, vdim16, qvec, kvvec, ovec);
 }
 
@@ -390,19 +406,18 @@ template <int MAXD, int VT>
 static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, bool pre, cudaStream_t st) {
   const auto go = [&](auto sig) {
     constexpr bool S = decltype(sig)::value;
-    constexpr int N = MAXD > 128 ? 32 : 64;
-    if (!pre) return launch_wm<MAXD, VT, 4, N, false, S>(d, w, n_seqs, max_new, hl, kvvec, st);
-    if constexpr (MAXD <= 128) {
-      const auto ctas = [&](int rows) { const int qn = rows >> hl; return static_cast<long long>((max_new + qn - 1) / qn) * (d.heads >> hl) * n_seqs; };
-      // rows of a CTA: 192 on narrow key tiles (three warps per scheduler; wide values leave room for no more than two otherwise) where that is
-      // two CTAs or more per SM, 128 where that is a CTA for every SM, else 64. 8 heads of 128 over 2, 4 x 2048 tokens, window 512: 192 rows
-      // 267 us, 128 rows 285 us, 64 rows 321 us; two portions of 1000 and 37 tokens: 137, 74, 82 us; 96 / 64 channels, whole context: 885, 860 us
-      if constexpr (VT == 128) {
-        if (ctas(192) >= 2 * num_sms()) return launch_wm<MAXD, VT, 12, 32, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
-      }
-      if (ctas(128) >= num_sms()) return launch_wm<MAXD, VT, 8, 64, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    constexpr int N_OWN = MAXD <= 128 ? 64 : 32, N = VT <= 64 ? 64 : 32;
+    if (!pre) return launch_wm<MAXD, VT, 4, N_OWN, 1, false, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    // CTAs of 64 rows, two per SM (key tiles as wide as that allows), so that one's softmax runs beside the other's products; wide values on
+    // long prompts take one CTA of 192 rows with three warps per scheduler instead, where that still is two rounds of CTAs over the SMs.
+    // 8 heads of 128 over 2, 4 x 2048 tokens, window 512, capped / sigmoid: 192 rows 235 / 237 us, 64 rows 240 / 262 us, 128 rows 236 / 270 us;
+    // portions of 1000 and 37 tokens: 123, 56, 62 us; 96 / 64 channels, whole context, 64 / 128 / 192 rows: 548, 590, 656 us
+    if constexpr (VT == 128) {
+      const int qn = 192 >> hl;
+      if (static_cast<long long>((max_new + qn - 1) / qn) * (d.heads >> hl) * n_seqs >= 2 * num_sms())
+        return launch_wm<MAXD, VT, 12, 32, 3, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
     }
-    return launch_wm<MAXD, VT, 4, N, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    return launch_wm<MAXD, VT, 4, N, 2, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
   };
   return d.sigmoid ? go(std::true_type{}) : go(std::false_type{});
 }
