@@ -867,6 +867,9 @@ typedef struct VyDeltaRule {
   int64_t rows; float* workspace; int64_t workspace_floats;
   void* stream;
 } VyDeltaRule;
+/* floats with which (16-byte aligned) a step walks its tokens 16 at a time on the tensor cores; 0: not for this step (max_new < 32, or 64 for
+ * dim <= 32; dim > 128; more than 1 GB), which then takes the form above */
+VY_API int64_t vy_delta_rule_prompt_floats(int64_t rows, int32_t n_seqs, int32_t max_new, int32_t heads, int32_t dim, int32_t vdim);
 VY_API int64_t vy_delta_rule_workspace_floats(int64_t rows, int32_t heads, int32_t kv_heads, int32_t dim);
 VY_API int vy_delta_rule(const VyDeltaRule* p);
 

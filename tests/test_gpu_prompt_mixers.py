@@ -1,0 +1,198 @@
+"""The prompt-sized forms of the packed decoders' mixers (csrc/window_attn_mma.cu, talk_attn_mma.cu, linear_attn_mma.cu, delta_rule_mma.cu) at
+the edges of their tiles and of the rules that choose them, against the float64 oracles and against the form that the same call takes
+without the lent workspace. Bound: an fp32 result off by a few units in the last place of its row's largest term per contraction, 16 * 2^-24 of the
+output's 2-norm (about 1e-6; the kernels measure 1e-7 to 3e-7)."""
+import pytest
+import torch
+
+from oracle import hybrid_oracle as OH
+from oracle import vazepel_oracle as OV
+from oracle import zaparax_oracle as OZ
+from tests.hybrid_util import shuffled_batch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BOUND = 16 * 2.0 ** -24
+
+
+def _err(got, want):
+    return float((got.detach().double().cpu() - want.double()).norm() / want.double().norm())
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+def _both(monkeypatch, rule, call):
+    """call() as it is, and with the rule that lends the workspace saying that this step needs none."""
+    from vyomai_b200 import ops
+    first = call()
+    monkeypatch.setattr(ops._lib.lib(), rule, lambda *a: 0)
+    second = call()
+    monkeypatch.undo()
+    return first, second
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 1, 20, 24), (2, 2, 33, 33), (4, 2, 64, 72), (2, 1, 128, 8), (1, 1, 100, 130), (1, 1, 1, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_delta_rule_sixteen_tokens_at_a_time(monkeypatch, H, G, dk, dv, dtype):
+    """Sequences that end on, before and after a chunk's edge, one of them carried on from a state; then their continuation. Strided inputs."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(dk)
+    lengths, more = [1, 15, 16, 17, 65], [64, 2, 16, 5, 1]
+    T = [a + b for a, b in zip(lengths, more)]
+    mk = lambda w: [torch.randn(t, w, generator=g).to(dtype) for t in T]  # noqa: E731
+    q, k, v, a, b = mk(G * dk), mk(G * dk), mk(H * dv), mk(H * dk), mk(H)
+    a_log = torch.randn(H, generator=g) - 1.0
+    want = []
+    for s, t in enumerate(T):
+        unit = lambda x: OH.unit(x.double().view(t, G, dk))  # noqa: E731
+        decay = torch.exp(-torch.exp(a_log.double())[None, :, None] * torch.nn.functional.softplus(a[s].double(), threshold=1e9).view(t, H, dk))
+        want.append(OH.gated_delta_rule(unit(q[s]) * dk ** -0.5, unit(k[s]), v[s].double().view(t, H, dv), decay, torch.sigmoid(b[s].double())).reshape(t, -1))
+
+    def walk():
+        state = torch.full((7, H, dk, dv), float("nan"), device=DEV)
+        slots, out = [3, 0, 6, 2, 5], []
+        for at, take in (([0] * 5, lengths), (lengths, more)):
+            wide = lambda src: torch.cat([torch.cat([src[s][at[s]:at[s] + take[s]] for s in range(5)]).to(DEV), torch.zeros(sum(take), 3, dtype=dtype, device=DEV)], 1)[:, :-3]  # noqa: E731
+            batch = ops.PackedBatch(_i32([sum(take[:i]) for i in range(6)]), _i32(at), _i32(slots), max(take))
+            out.append(ops.delta_rule(batch, wide(q), wide(k), wide(v), wide(a), wide(b), a_log.to(DEV), state, heads=H, kv_heads=G, dim=dk, vdim=dv, out_dtype=torch.float32).split(take))
+        assert bool(torch.isnan(state[[1, 4]]).all())   # other slots untouched
+        return [torch.cat([x, y]) for x, y in zip(*out)]
+
+    for form in _both(monkeypatch, "vy_delta_rule_prompt_floats", walk):
+        for s in range(5):
+            assert _err(form[s], want[s]) < 4 * BOUND, s   # a recurrence: each of the up to 66 steps carries its rounding on
+
+
+def test_delta_rule_keeps_a_bad_value_to_its_column_and_later_tokens():
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(1)
+    T, H, dk, dv, at, col = 40, 1, 48, 40, 21, 5
+    q, k, v, a, b = (torch.randn(T, w, generator=g, device=DEV) for w in (dk, dk, dv, dk, H))
+    batch = ops.PackedBatch(_i32([0, T]), _i32([0]), _i32([0]), T)
+    run = lambda vv: ops.delta_rule(batch, q, k, vv, a, b, torch.zeros(1, device=DEV), torch.zeros(1, H, dk, dv, device=DEV), heads=H, kv_heads=H, dim=dk, vdim=dv)  # noqa: E731
+    clean = run(v)
+    for bad in (float("inf"), float("nan")):
+        vv = v.clone()
+        vv[at, col] = bad
+        got = run(vv)
+        hit = torch.zeros(T, dv, dtype=torch.bool, device=DEV)
+        hit[at:, col] = True
+        assert torch.equal(torch.isfinite(got), ~hit)
+        assert float((got - clean)[~hit].abs().max()) < 1e-6
+
+
+@pytest.mark.parametrize("H,dk,dv", [(2, 20, 24), (1, 128, 64), (3, 64, 65), (2, 100, 130), (1, 8, 7)])
+def test_linear_attention_all_chunks_at_once(monkeypatch, H, dk, dv):
+    """Chunks of 64 tokens: portions of 64 (the walk), 65, 128, 130 and 1 token side by side, then a continuation of 66."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(dk)
+    lengths, more = [64, 65, 128, 130, 1], [66, 1, 3, 64, 66]
+    T = [a + b for a, b in zip(lengths, more)]
+    q, k, v = ([torch.randn(t, H * w, generator=g) for t in T] for w in (dk, dk, dv))
+    decay = torch.tensor([0.999, 0.5, 0.9][:H]).double().tolist()   # as fp32 holds them: 0.999 itself is 1.3e-8 off, 130 steps of it 1e-6
+    want = [OH.lightning_attention(q[s].double().view(t, H, dk), k[s].double().view(t, H, dk), v[s].double().view(t, H, dv), decay).reshape(t, -1) for s, t in enumerate(T)]
+
+    def walk():
+        state = torch.full((6, H, dk, dv), float("nan"), device=DEV)
+        out = []
+        for at, take in (([0] * 5, lengths), (lengths, more)):
+            cat = lambda src: torch.cat([src[s][at[s]:at[s] + take[s]] for s in range(5)]).to(DEV)  # noqa: E731
+            batch = ops.PackedBatch(_i32([sum(take[:i]) for i in range(6)]), _i32(at), _i32([4, 1, 0, 5, 2]), max(take))
+            out.append(ops.linear_attn(batch, cat(q), cat(k), cat(v), torch.tensor(decay, device=DEV), state, heads=H, dim=dk, vdim=dv).split(take))
+        return [torch.cat([x, y]) for x, y in zip(*out)]
+
+    for form in _both(monkeypatch, "vy_linear_attn_workspace_floats", walk):
+        for s in range(5):
+            assert _err(form[s], want[s]) < BOUND, s
+
+
+@pytest.mark.parametrize("pool", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,d,dv,window,cap,sinks", [(4, 2, 20, 10, 0, 0.0, True), (8, 1, 64, 64, 31, 20.0, False), (2, 2, 96, 130, 65, 0.0, True), (16, 2, 128, 128, 0, 0.0, False),
+                                                       (4, 4, 192, 192, 100, 0.0, False), (6, 2, 33, 256, 7, 5.0, True)])
+def test_prompt_attention_on_the_tensor_cores(monkeypatch, pool, H, G, d, dv, window, cap, sinks):
+    """Portions of 1 to 200 queries on contexts that end on and off the key tiles; pages that no query may read hold large numbers."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(d)
+    new, pos0 = [200, 64, 17, 1], [0, 65, 130, 33]
+    T = [n + p for n, p in zip(new, pos0)]
+    q, k, v = ([(torch.randn(t, n, w, generator=g) / d ** (0.25 if i < 2 else 0)).to(pool).float() for t in T] for i, (n, w) in enumerate(((H, d), (G, d), (G, dv))))
+    sink = torch.randn(H, generator=g) if sinks else None
+    slopes = OZ.head_slopes(H)
+    want = torch.cat([OZ.biased_attention(q[s].double(), k[s].double(), v[s].double(), scale=1.3, softcap=cap, window=window, slopes=slopes,
+                                          sink=None if sink is None else sink.double())[pos0[s]:].reshape(new[s], -1) for s in range(4)])
+    bs = 16
+    batch, table, _, n_blocks, _ = shuffled_batch(new, pos0, bs, DEV, seed=d)
+    kp, vp = torch.full((n_blocks, bs, G, d), 1e3, dtype=pool, device=DEV), torch.full((n_blocks, bs, G, dv), 1e3, dtype=pool, device=DEV)
+    for s in range(4):
+        for p in range(T[s]):
+            kp[table[s][p // bs], p % bs], vp[table[s][p // bs], p % bs] = k[s][p].to(DEV, pool), v[s][p].to(DEV, pool)
+    qq = torch.cat([q[s][pos0[s]:].reshape(new[s], -1) for s in range(4)]).to(DEV)
+    call = lambda: ops.window_attn(batch, qq, kp, vp, heads=H, kv_heads=G, dim=d, vdim=dv, scale=1.3, window=window, keep_first=0, softcap=cap,  # noqa: E731
+                                   head_slope=torch.tensor(slopes, device=DEV), sink=None if sink is None else sink.to(DEV), out_dtype=torch.float32)
+    for got in _both(monkeypatch, "vy_window_attn_prompt_floats", call):
+        assert _err(got, want) < BOUND
+
+
+@pytest.mark.parametrize("H,G,d,dv,window", [(8, 2, 64, 64, 0), (16, 4, 20, 33, 37), (32, 8, 48, 16, 0), (8, 8, 7, 5, 16)])
+def test_score_exchanging_prompts_on_the_tensor_cores(monkeypatch, H, G, d, dv, window):
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(H)
+    new, pos0, scale, bs = [130, 17, 16], [0, 48, 1], 0.3, 4
+    T = [n + p for n, p in zip(new, pos0)]
+    q, k, v = ([torch.randn(t, n, w, generator=g) for t in T] for n, w in ((H, d), (G, d), (G, dv)))
+    talk = torch.eye(H) + 0.3 * torch.randn(H, H, generator=g) / H ** 0.5
+    want = []
+    for s, t in enumerate(T):
+        sc = torch.stack([q[s][:, a].double() @ k[s][:, a // (H // G)].double().T for a in range(H)]) * scale
+        back = torch.arange(t)[:, None] - torch.arange(t)[None, :]
+        p = OV.plus_one_softmax(OV.mix_heads(OV.capped(sc, 9.0), talk.double()), (back >= 0) & (back < window) if window else back >= 0)
+        want.append(torch.stack([p[a] @ v[s][:, a // (H // G)].double() for a in range(H)], 1).reshape(t, -1)[pos0[s]:])
+    batch, table, _, n_blocks, _ = shuffled_batch(new, pos0, bs, DEV, seed=H)
+    kp, vp = torch.full((n_blocks, bs, G, d), 1e3, device=DEV), torch.full((n_blocks, bs, G, dv), 1e3, device=DEV)
+    for s in range(3):
+        for p in range(T[s]):
+            kp[table[s][p // bs], p % bs], vp[table[s][p // bs], p % bs] = k[s][p].to(DEV), v[s][p].to(DEV)
+    qq = torch.cat([q[s][pos0[s]:].reshape(new[s], -1) for s in range(3)]).to(DEV)
+    call = lambda: ops.talk_attn(batch, qq, kp, vp, heads=H, kv_heads=G, dim=d, vdim=dv, scale=scale, softcap=9.0, talk=talk.to(DEV), zero_sink=True, window=window)  # noqa: E731
+    for got in _both(monkeypatch, "vy_talk_attn_prompt_floats", call):
+        assert _err(got, torch.cat(want)) < 4 * BOUND   # mixed scores: each is a sum over H capped ones, and the softmax takes its absolute error
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_repeated_product_reads_its_own_operands(dtype):
+    """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(2)
+    xs = [torch.randn(96, 264, generator=g, device=DEV).to(dtype) for _ in range(6)]
+    ws = [torch.randn(128, 256, generator=g, device=DEV).to(dtype) for _ in range(6)]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for i, (x, w) in enumerate(zip(xs, ws)):
+        x = x[:, :256] if i % 2 else x[:, :256].contiguous()
+        with torch.cuda.stream(side if i % 3 == 2 else torch.cuda.current_stream()):
+            y = ops.gemm(x, w)
+        torch.cuda.synchronize()
+        want = x.double() @ w.double().T
+        assert float((y.double() - want).norm() / want.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -9)   # the output's or the operands' rounding
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_norm_gradients_in_the_parameters_type(dtype):
+    from vyomai_b200 import ops
+    from vyomai_b200.autograd_train import _ln_bwd
+    g = torch.Generator(device=DEV).manual_seed(3)
+    W, rows = 264, 77
+    s, dy = (torch.randn(rows, W, generator=g, device=DEV).to(dtype) for _ in range(2))
+    gamma, beta, bias = (torch.nn.Parameter(torch.randn(W, generator=g, device=DEV).to(dtype)) for _ in range(3))
+    mean = s.float().mean(1)
+    rstd = torch.rsqrt(s.float().var(1, unbiased=False) + 1e-5)
+    ds, dg, db, dbias = _ln_bwd(dy, s, gamma, beta, mean, rstd, bias)
+    xhat = (s.double() - mean.double()[:, None]) * rstd.double()[:, None]
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else BOUND
+    assert dg.dtype == db.dtype == dbias.dtype == dtype
+    assert _err(dg, (dy.double() * xhat).sum(0).cpu()) < tol and _err(db, dy.double().sum(0).cpu()) < tol
+    dx = gamma.double() * dy.double()
+    dx = (dx - dx.mean(1, keepdim=True) - xhat * (dx * xhat).mean(1, keepdim=True)) * rstd.double()[:, None]
+    assert _err(ds, dx.cpu()) < 2 * tol and _err(dbias, dx.sum(0).cpu()) < 32 * tol   # columns of dx nearly cancel

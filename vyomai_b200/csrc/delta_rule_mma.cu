@@ -1,0 +1,551 @@
+// Gated delta rule with a decay per channel, prompts: 16 tokens per step of the serial walk, on the tensor cores in fp32 precision
+// (split_mma.cuh). Per head, with the state S [dim, vdim] before a chunk of 16 tokens, the products G_t of the chunk's decays up to token t
+// and k / q the unit vectors, the 16 writes u_t and read-outs o_t solve
+//   u_t + beta_t sum_{s < t} A_ts u_s = beta_t (v_t - S^T (G_t k_t)),      A_ts = k_t . (G_t / G_s k_s)
+//   o_t = S^T (G_t q_t) + sum_{s <= t} B_ts u_s,                           B_ts = q_t . (G_t / G_s k_s)
+//   S <- G_15 S + sum_s (G_15 / G_s k_s) u_s^T
+// The quotients are products of the decays between s and t or exponentials of sums: nothing is divided, no underflow matters. With W the inverse of the
+// triangular 16 x 16 system times diag(beta), u = W v - (W G k) S. Two launches:
+//   delta_chunk_kernel   all chunks in parallel: W, then W v, P = W G k, G q, G_15 / G_s k, B, split into fp16 pairs and stored in the
+//                        register layout of the second launch's operands
+//   delta_scan_kernel    the walk. It is transposed (S^T: a warp owns 16 value columns and all channels), so that the state in accumulator
+//                        registers is the next product's A operand, the writes likewise, and no warp waits for another one
+// The walk token by token (delta_rule_kernel) is bound by its chain of two reductions per token: 46 + 1013 us with its preparation for 4 x 2048
+// tokens, 8 heads of 128 x 128; here 166 + 217 us. The first launch is bound by instructions (decays, exponentials, sums of pairs of tokens), the
+// second by the latency of one warp's chain, 1.7 us per chunk. Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
+#include "seqmix.cuh"
+#include "split_mma.cuh"
+
+namespace vy {
+namespace {
+
+constexpr int DC_T = 16;            // tokens per chunk
+constexpr int DC_KTOP = 15;         // the decayed unit keys are split in units of 2^-15: their entries are at most 1
+constexpr int DC_NW = 2;            // warps of the walk's CTA: 32 value columns
+constexpr int DC_NS = 3;            // chunks in flight per CTA of the walk
+// A tensor-core accumulation cuts off where fp32 rounds: a result is this share too small on average (measured: read-outs -5.8e-8 without it,
+// -0.4e-8 with it, the serial walk +0.5e-8). A sum of n accumulations loses (n + 1) / 2 such shares of its end value on average
+constexpr float DC_CUT = 0x1p-25f;
+
+// One chunk and head in the workspace. An operand entry is 16 bytes per lane: (b0, b1) of mma.m16n8k16, hi then lo
+template <int DP>
+struct DcBlob {
+  static constexpr int q_at = 64 * DP, k_at = 128 * DP, b_at = 192 * DP, g_at = b_at + 1024, unit_at = g_at + 4 * DP, bytes = unit_at + 3 * 64;
+};
+
+struct DeltaChunks {
+  unsigned char* blobs;   // [slot][head] DcBlob
+  float* wv;              // [slot][head][vpad / 16][32 lanes][8]: W v as accumulator registers
+  int vpad;
+};
+
+// a sequence's first chunk slot: cu[s] / 16 + s, so that sequences never overlap and rows / 16 + n_seqs slots suffice
+__device__ __forceinline__ long long chunk_slot0(int base, int s) { return base / DC_T + s; }
+
+template <int DP>
+__global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks w) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int LD = DP + 8, NP = DC_T * DP / 256, PER = DP / 16;
+  using Blob = DcBlob<DP>;
+  __shared__ __align__(16) float ks[DC_T][LD], qs[DC_T][LD], gs[DC_T][LD], xs[DC_T][LD], kb[DC_T][LD];
+  __shared__ float A[DC_T][DC_T + 1], B[DC_T][DC_T + 1], W[DC_T][DC_T + 1], beta[DC_T], scale[3][DC_T];
+  const int s = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * DC_T;
+  const int base = d.cu[s], n = d.cu[s + 1] - base;
+  if (t0 >= n) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = min(DC_T, n - t0);
+  const int gq = h / (d.heads / d.kv_heads);
+  const long long row0 = base + t0, at = (chunk_slot0(base, s) + blockIdx.x) * d.heads + h;
+  unsigned char* blob = w.blobs + at * Blob::bytes;
+  {
+    float rq[NP], rk[NP], ra[NP];
+#pragma unroll
+    for (int u = 0; u < NP; ++u) {
+      const int e = tid + 256 * u, tt = e / DP, i = e % DP;
+      const bool ok = tt < nt && i < d.dim;
+      rq[u] = ok ? ld_as_float(d.q, d.in_dt, (row0 + tt) * d.ldq + static_cast<long long>(gq) * d.dim + i) : 0.f;
+      rk[u] = ok ? ld_as_float(d.k, d.in_dt, (row0 + tt) * d.ldk + static_cast<long long>(gq) * d.dim + i) : 0.f;
+      ra[u] = ok ? ld_as_float(d.a, d.a_dt, (row0 + tt) * d.ld_a + static_cast<long long>(h) * d.dim + i) : 0.f;
+    }
+    const float neg_rate = -expf(ld_as_float(d.a_log, d.a_log_dt, h));
+    if (tid < DC_T) beta[tid] = tid < nt ? sigmoidf_(ld_as_float(d.b, d.b_dt, (row0 + tid) * d.ld_b + h)) : 0.f;
+#pragma unroll
+    for (int u = 0; u < NP; ++u) {
+      const int e = tid + 256 * u, tt = e / DP, i = e % DP;
+      qs[tt][i] = rq[u];
+      ks[tt][i] = rk[u];
+      const float x = tt < nt && i < d.dim ? neg_rate * softplusf_(ra[u]) : 0.f;
+      xs[tt][i] = x;
+      gs[tt][i] = expf(x);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {   // unit vectors, two tokens per warp
+    const int tt = 2 * warp + r;
+    float xq[DP / 32], xk[DP / 32], sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int m = 0; m < DP / 32; ++m) {
+      xq[m] = qs[tt][lane + 32 * m];
+      xk[m] = ks[tt][lane + 32 * m];
+      sq = fmaf(xq[m], xq[m], sq);
+      sk = fmaf(xk[m], xk[m], sk);
+    }
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    const float qn = tt < nt ? 1.f / sqrtf(static_cast<float>(d.dim)) / sqrtf(sq + d.unit_eps) : 0.f, kn = tt < nt ? 1.f / sqrtf(sk + d.unit_eps) : 0.f;
+#pragma unroll
+    for (int m = 0; m < DP / 32; ++m) {
+      qs[tt][lane + 32 * m] = xq[m] * qn;
+      ks[tt][lane + 32 * m] = xk[m] * kn;
+    }
+  }
+  __syncthreads();
+  {   // G_t and G_15 / G_s k_s, a channel per thread, from sums of the decays' logarithms: an fp32 decay near 1 is off by a share of its distance
+      // from 1 that a product over a long memory multiplies
+    const int i = tid & 127;
+    float G[DC_T], x = 0.f;
+    if (i < DP) {
+      if (tid < 128) {
+#pragma unroll
+        for (int t = 0; t < DC_T; ++t) G[t] = expf(x += xs[t][i]);
+      } else {
+#pragma unroll
+        for (int t = DC_T - 1; t >= 0; --t) {
+          kb[t][i] = ks[t][i] * expf(x);
+          x += xs[t][i];
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < DP) {
+#pragma unroll
+      for (int t = 0; t < DC_T; ++t) xs[t][i] = G[t];
+      reinterpret_cast<float*>(blob + Blob::g_at)[i] = G[DC_T - 1];
+    }
+  }
+  {   // A and B: 16 lanes per token s carry G_t / G_s k_s through the tokens t after it
+    const int sl = tid & 15, c = tid >> 4;
+    const auto lane_channels = [&](const float* p, float (&x)[PER]) {
+      if constexpr (PER == 2) {
+        const float2 v = *reinterpret_cast<const float2*>(p + 2 * sl);
+        x[0] = v.x; x[1] = v.y;
+      } else {
+#pragma unroll
+        for (int m = 0; m < PER / 4; ++m) {
+          const float4 v = f4(p + 64 * m + 4 * sl);
+          x[4 * m] = v.x; x[4 * m + 1] = v.y; x[4 * m + 2] = v.z; x[4 * m + 3] = v.w;
+        }
+      }
+    };
+    float D[PER];
+#pragma unroll
+    for (int e = 0; e < PER; ++e) D[e] = 0.f;
+    for (int t = 2 * warp; t < DC_T; ++t) {
+      float kt[PER], qt[PER], gt[PER], a = 0.f, b = 0.f;
+      lane_channels(ks[t], kt);
+      lane_channels(qs[t], qt);
+      lane_channels(gs[t], gt);
+#pragma unroll
+      for (int e = 0; e < PER; ++e) {
+        D[e] = t == c ? kt[e] : (t > c ? D[e] * gt[e] : 0.f);
+        a = fmaf(D[e], kt[e], a);
+        b = fmaf(D[e], qt[e], b);
+      }
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      if (sl == 0 && t >= c) {
+        A[t][c] = a;
+        B[t][c] = b;
+      }
+    }
+  }
+  __syncthreads();
+  if (tid < DC_T) {   // W, a column per lane
+    float x[DC_T];
+#pragma unroll
+    for (int t = 0; t < DC_T; ++t) {
+      float r = 0.f;
+#pragma unroll
+      for (int c = 0; c < t; ++c)
+        if (c >= tid) r = fmaf(A[t][c], x[c], r);
+      x[t] = t < tid ? 0.f : (t == tid ? beta[t] : -beta[t] * r);
+      W[t][tid] = x[t];
+    }
+  }
+  __syncthreads();
+  {   // P = W G k, and G q in place; a later token never enters an earlier one's sum, not even times zero
+    const int i = tid % DP, tp = tid / DP * NP;
+    float kc[DC_T], p[NP];
+#pragma unroll
+    for (int t = 0; t < DC_T; ++t) kc[t] = ks[t][i] * xs[t][i];
+#pragma unroll
+    for (int r = 0; r < NP; ++r) {
+      p[r] = 0.f;
+#pragma unroll
+      for (int c = 0; c < DC_T; ++c)
+        if (c <= tp + r) p[r] = fmaf(W[tp + r][c], kc[c], p[r]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < NP; ++r) {
+      ks[tp + r][i] = p[r];
+      qs[tp + r][i] *= xs[tp + r][i];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {   // a scale per token for each of P, G q and B
+    const int tt = 2 * warp + r;
+    float mp = 0.f, mq = 0.f, mb = lane <= tt ? fabsf(B[tt][min(lane, DC_T - 1)]) : 0.f;
+#pragma unroll
+    for (int m = 0; m < DP / 32; ++m) {
+      mp = fmaxf(mp, fabsf(ks[tt][lane + 32 * m]));
+      mq = fmaxf(mq, fabsf(qs[tt][lane + 32 * m]));
+    }
+    const int ep = split_exponent(warp_max(mp)), eq = split_exponent(warp_max(mq)), eb = split_exponent(warp_max(mb));
+    if (lane == 0) {
+      scale[0][tt] = split_scale(ep);
+      scale[1][tt] = split_scale(eq);
+      scale[2][tt] = split_scale(eb);
+      float* unit = reinterpret_cast<float*>(blob + Blob::unit_at);
+      unit[tt] = pow2i(ep - SPLIT_TOP);
+      unit[DC_T + tt] = pow2i(eq - SPLIT_TOP);
+      unit[2 * DC_T + tt] = pow2i(eb - SPLIT_TOP);
+    }
+  }
+  __syncthreads();
+  const int l4 = lane >> 2, tq = 2 * (lane & 3);
+  uint4* out = reinterpret_cast<uint4*>(blob);
+#pragma unroll
+  for (int u = 0; u < DP / 64 + (DP < 64); ++u) {
+    const int e = tid + 256 * u;
+    if (e < 4 * DP) {   // P and G q: 16 channels (k) x 8 tokens (n) per 32 entries
+      const int t = 8 * ((e >> 5) & 1) + l4, i = 16 * (e >> 6) + tq;
+      uint4 x;
+      const float sp = scale[0][t], sq = scale[1][t];
+      const float2 p0 = *reinterpret_cast<const float2*>(&ks[t][i]), p1 = *reinterpret_cast<const float2*>(&ks[t][i + 8]);
+      split2(p0.x * sp, p0.y * sp, x.x, x.z);
+      split2(p1.x * sp, p1.y * sp, x.y, x.w);
+      out[e] = x;
+      const float2 q0 = *reinterpret_cast<const float2*>(&qs[t][i]), q1 = *reinterpret_cast<const float2*>(&qs[t][i + 8]);
+      split2(q0.x * sq, q0.y * sq, x.x, x.z);
+      split2(q1.x * sq, q1.y * sq, x.y, x.w);
+      out[Blob::q_at / 16 + e] = x;
+      const int j = 8 * (e >> 5) + l4;   // G_15 / G_s k_s: 16 tokens (k) x 8 channels (n)
+      constexpr float one = 1 << DC_KTOP;
+      split2(kb[tq][j] * one, kb[tq + 1][j] * one, x.x, x.z);
+      split2(kb[tq + 8][j] * one, kb[tq + 9][j] * one, x.y, x.w);
+      out[Blob::k_at / 16 + e] = x;
+    }
+  }
+  if (tid < 64) {   // B: tokens s (k) x tokens t (n)
+    const int t = 8 * warp + l4;
+    const float sb = scale[2][t];
+    const auto b = [&](int c) { return c <= t ? B[t][c] * sb : 0.f; };
+    uint4 x;
+    split2(b(tq), b(tq + 1), x.x, x.z);
+    split2(b(tq + 8), b(tq + 9), x.y, x.w);
+    out[Blob::b_at / 16 + tid] = x;
+  }
+  for (int e = tid; e < w.vpad * 2; e += 256) {   // W v: entry lane of 16 columns holds columns l4, l4 + 8 of tokens tq, tq + 1, tq + 8, tq + 9
+    const int c0 = 16 * (e >> 5) + l4;
+    const bool ok0 = c0 < d.vdim, ok1 = c0 + 8 < d.vdim;
+    float v[2][DC_T], x[8];
+#pragma unroll
+    for (int c = 0; c < DC_T; ++c) {
+      const long long o = (row0 + c) * d.ldv + static_cast<long long>(h) * d.vdim + c0;
+      v[0][c] = c < nt && ok0 ? ld_as_float(d.v, d.in_dt, o) : 0.f;
+      v[1][c] = c < nt && ok1 ? ld_as_float(d.v, d.in_dt, o + 8) : 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {   // register r: token half r / 4, column half r / 2 % 2, token r % 2
+      const int t = tq + 8 * (r >> 2) + (r & 1);
+      x[r] = 0.f;
+#pragma unroll
+      for (int c = 0; c < DC_T; ++c)
+        if (c <= t) x[r] = fmaf(W[t][c], v[(r >> 1) & 1][c], x[r]);
+    }
+    float4* o = reinterpret_cast<float4*>(w.wv + (at * (w.vpad / 16) + (e >> 5)) * 256 + lane * 8);
+    o[0] = make_float4(x[0], x[1], x[2], x[3]);
+    o[1] = make_float4(x[4], x[5], x[6], x[7]);
+  }
+}
+
+__device__ __forceinline__ void dc_bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// The writes' share of the read-outs when a write is infinite or NaN: the product's zeros would carry it to the tokens before it
+static __device__ __noinline__ void dc_read_finite(float (&o)[2][4], const float (&u)[2][4], const unsigned char* b, const float* unit, int lane) {
+  const int tq = 2 * (lane & 3);
+#pragma unroll
+  for (int s = 0; s < DC_T; ++s) {
+    const int src = (lane & ~3) | ((s & 7) >> 1);
+    const float u0 = __shfl_sync(0xffffffffu, u[s >> 3][s & 1], src), u1 = __shfl_sync(0xffffffffu, u[s >> 3][2 + (s & 1)], src);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int t = 8 * (r >> 1) + tq + (r & 1);
+      if (s > t) continue;
+      const __half* e = reinterpret_cast<const __half*>(b + 16 * (32 * (t >> 3) + 4 * (t & 7) + ((s & 7) >> 1))) + 2 * (s >> 3) + (s & 1);
+      const float x = (__half2float(e[0]) + __half2float(e[4])) * unit[t];
+      o[r >> 1][r & 1] = fmaf(x, u0, o[r >> 1][r & 1]);
+      o[r >> 1][2 + (r & 1)] = fmaf(x, u1, o[r >> 1][2 + (r & 1)]);
+    }
+  }
+}
+
+template <int DP>
+__global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaChunks w, PoisonRef poison) {
+  pdl_trigger();
+  pdl_wait();
+  using Blob = DcBlob<DP>;
+  constexpr int KS = DP / 16, NT = DP / 8, STAGE = Blob::bytes + DC_NW * 1024;
+  extern __shared__ __align__(128) unsigned char dc_smem[];
+  __shared__ __align__(8) uint64_t full[DC_NS];
+  __shared__ int done[DC_NS];   // warps that are through with a stage, counted up for ever
+  const int s = blockIdx.z, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l4 = lane >> 2, tq = 2 * (lane & 3);
+  const int base = d.cu[s], n = d.cu[s + 1] - base;
+  if (n <= 0) return;
+  const int chunks = (n + DC_T - 1) / DC_T;
+  const long long slot0 = chunk_slot0(base, s);
+  const auto fetch = [&](int c, int b) {
+    const long long at = (slot0 + c) * d.heads + h;
+    unsigned char* st = dc_smem + b * STAGE;
+    mbar_arrive_expect_tx(&full[b], STAGE);
+    dc_bulk_load(st, w.blobs + at * Blob::bytes, Blob::bytes, &full[b]);
+    dc_bulk_load(st + Blob::bytes, w.wv + (at * (w.vpad / 16) + blockIdx.x * DC_NW) * 256, DC_NW * 1024, &full[b]);
+  };
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < DC_NS; ++b) {
+      mbar_init(&full[b], 1);
+      done[b] = 0;
+    }
+    fence_mbar_init();
+    for (int b = 0; b < min(DC_NS, chunks); ++b) fetch(b, b);
+  }
+  // S^T as accumulators: S[j][e] is column l4 + 8 (e / 2), channel 8 j + tq + e % 2
+  const int col = 32 * blockIdx.x + 16 * warp + l4;
+  const bool ok0 = col < d.vdim, ok1 = col + 8 < d.vdim;
+  float* sp = d.state + ((static_cast<long long>(d.slot[s]) * d.heads + h) * d.dim) * d.vdim + col;
+  const bool carried = d.pos0[s] > 0;
+  float S[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = 8 * j + tq + (e & 1);
+      S[j][e] = carried && i < d.dim && (e < 2 ? ok0 : ok1) ? sp[static_cast<long long>(i) * d.vdim + 8 * (e >> 1)] : 0.f;
+    }
+  __syncthreads();
+  for (int c = 0; c < chunks; ++c) {
+    const int b = c % DC_NS;
+    const unsigned char* st = dc_smem + b * STAGE;
+    float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      m0 = fmaxf(m0, fmaxf(fabsf(S[j][0]), fabsf(S[j][1])));
+      m1 = fmaxf(m1, fmaxf(fabsf(S[j][2]), fabsf(S[j][3])));
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+      m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    }
+    const int e0 = split_exponent(m0), e1 = split_exponent(m1);
+    const float s0 = split_scale(e0), s1 = split_scale(e1), n0 = pow2i(e0 - SPLIT_TOP), n1 = pow2i(e1 - SPLIT_TOP);
+    mbar_wait_soft(&full[b], (c / DC_NS) & 1, poison);
+    const uint4* ops = reinterpret_cast<const uint4*>(st) + lane;
+    float r[4][4], x[4][4], half[4][4];   // S^T P and S^T G q: 8 tokens each
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) r[j][e] = x[j][e] = half[j][e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      unsigned ah[4], al[4];
+      split2(S[2 * k][0] * s0, S[2 * k][1] * s0, ah[0], al[0]);
+      split2(S[2 * k][2] * s1, S[2 * k][3] * s1, ah[1], al[1]);
+      split2(S[2 * k + 1][0] * s0, S[2 * k + 1][1] * s0, ah[2], al[2]);
+      split2(S[2 * k + 1][2] * s1, S[2 * k + 1][3] * s1, ah[3], al[3]);
+      uint4 f[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = ops[(j >= 2 ? Blob::q_at / 16 : 0) + 32 * (2 * k + (j & 1))];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_f16(x[j], al, f[j].x, f[j].y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_f16(r[j], ah, f[j].x, f[j].y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_f16(x[j], ah, f[j].z, f[j].w);
+      if (KS >= 4 && k == KS / 2 - 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            half[j][e] = r[j][e];
+            r[j][e] = 0.f;
+          }
+      }
+    }
+    // the writes, then as A operand
+    constexpr float cut = ((KS >= 4 ? KS / 2 : KS) + 1) * 0.5f * DC_CUT;
+    const float* unit = reinterpret_cast<const float*>(st + Blob::unit_at);
+    const float4* wv = reinterpret_cast<const float4*>(st + Blob::bytes + 1024 * warp + 32 * lane);
+    float u[2][4];
+    m0 = m1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float4 y = wv[j];
+      const float2 p = *reinterpret_cast<const float2*>(unit + 8 * j + tq);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float y0 = r[j][e] + half[j][e], z = (y0 + fmaf(y0, cut, x[j][e])) * (e < 2 ? n0 : n1);
+        u[j][e] = fmaf(-z, e & 1 ? p.y : p.x, e == 0 ? y.x : e == 1 ? y.y : e == 2 ? y.z : y.w);
+      }
+      m0 = fmaxf(m0, fmaxf(fabsf(u[j][0]), fabsf(u[j][1])));
+      m1 = fmaxf(m1, fmaxf(fabsf(u[j][2]), fabsf(u[j][3])));
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+      m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    }
+    const int f0 = split_exponent(m0), f1 = split_exponent(m1);
+    const float t0 = split_scale(f0), t1 = split_scale(f1), w0 = pow2i(f0 - SPLIT_TOP), w1 = pow2i(f1 - SPLIT_TOP);
+    unsigned uh[4], ul[4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      split2(u[j][0] * t0, u[j][1] * t0, uh[2 * j], ul[2 * j]);
+      split2(u[j][2] * t1, u[j][3] * t1, uh[2 * j + 1], ul[2 * j + 1]);
+    }
+    // the state
+    const float k0 = w0 * (1.f / (1 << DC_KTOP)), k1 = w1 * (1.f / (1 << DC_KTOP));
+    const float* G = reinterpret_cast<const float*>(st + Blob::g_at) + tq;
+#pragma unroll
+    for (int j = 0; j < NT; j += 2) {
+      float y[2][4], z[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[i][e] = z[i][e] = 0.f;
+      const uint4 f[2] = {ops[Blob::k_at / 16 + 32 * j], ops[Blob::k_at / 16 + 32 * j + 32]};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mma_f16(z[i], ul, f[i].x, f[i].y);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mma_f16(y[i], uh, f[i].x, f[i].y);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mma_f16(z[i], uh, f[i].z, f[i].w);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float2 g = *reinterpret_cast<const float2*>(G + 8 * (j + i));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j + i][e] = fmaf(S[j + i][e], e & 1 ? g.y : g.x, (y[i][e] + fmaf(y[i][e], DC_CUT, z[i][e])) * (e < 2 ? k0 : k1));
+      }
+    }
+    // the read-outs
+    float o[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float2 q = *reinterpret_cast<const float2*>(unit + DC_T + 8 * j + tq);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float y0 = r[2 + j][e] + half[2 + j][e];
+        o[j][e] = (y0 + fmaf(y0, cut, x[2 + j][e])) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
+      }
+    }
+    bool finite = true;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) finite = finite && fabsf(u[j][e]) < INFINITY;
+    if (__all_sync(0xffffffffu, finite)) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint4 f = ops[Blob::b_at / 16 + 32 * j];
+        const float2 p = *reinterpret_cast<const float2*>(unit + 2 * DC_T + 8 * j + tq);
+        mma_f16(z, ul, f.x, f.y);
+        mma_f16(y, uh, f.x, f.y);
+        mma_f16(z, uh, f.z, f.w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] = fmaf((y[e] + fmaf(y[e], DC_CUT, z[e])) * (e < 2 ? w0 : w1), e & 1 ? p.y : p.x, o[j][e]);
+      }
+    } else {
+      dc_read_finite(o, u, st + Blob::b_at, unit + 2 * DC_T, lane);
+    }
+    // through with the stage: the last warp refills it
+    __syncwarp();
+    if (lane == 0 && c + DC_NS < chunks) {
+      __threadfence_block();
+      if (atomicAdd(&done[b], 1) % DC_NW == DC_NW - 1) {
+        __threadfence_block();
+        fence_proxy_async_smem();
+        fetch(c + DC_NS, b);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = DC_T * c + 8 * j + tq + (e & 1);
+        if (t < n && (e < 2 ? ok0 : ok1))
+          st_from_float(d.out, d.out_dt, static_cast<long long>(base + t) * d.ld_out + static_cast<long long>(h) * d.vdim + col + 8 * (e >> 1), o[j][e]);
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = 8 * j + tq + (e & 1);
+      if (i < d.dim && (e < 2 ? ok0 : ok1)) sp[static_cast<long long>(i) * d.vdim + 8 * (e >> 1)] = S[j][e];
+    }
+}
+
+int blob_bytes(int dim) { return dim <= 32 ? DcBlob<32>::bytes : dim <= 64 ? DcBlob<64>::bytes : DcBlob<128>::bytes; }
+int round32(int x) { return (x + 31) / 32 * 32; }
+
+template <int DP>
+cudaError_t launch(const RecDev& d, int n_seqs, int max_new, const DeltaChunks& w, cudaStream_t st) {
+  const size_t smem = DC_NS * (DcBlob<DP>::bytes + DC_NW * 1024);
+  static bool once = false;
+  if (!once) {
+    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    once = true;
+  }
+  PoisonRef poison = {};
+  if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
+  cudaError_t e = launch_kernel(delta_chunk_kernel<DP>, dim3((max_new + DC_T - 1) / DC_T, d.heads, n_seqs), dim3(256), 0, st, d, w);
+  if (e != cudaSuccess) return e;
+  count_launch();
+  return launch_kernel(delta_scan_kernel<DP>, dim3(w.vpad / 32, d.heads, n_seqs), dim3(32 * DC_NW), smem, st, d, w, poison);
+}
+
+}  // namespace
+
+// From 32 tokens on (64 for heads of up to 32 channels): two launches and a chunk's preparation cost more than a short walk. In us, chunks / tokens:
+// 1 sequence, 8 heads of 128 x 128: 20.3 / 19.9 at 24 tokens, 20.5 / 23.2 at 32, 30 / 71 at 128; 32 sequences, 4 heads of 64 x 64: 19.2 / 18.4,
+// 19.3 / 22.0, 44 / 72; 4 sequences, 4 heads of 16 x 16: 16.2 / 15.4 at 48, 17.3 / 18.6 at 64. Past 128 channels a warp's share of the state
+// (16 columns) does not fit its registers.
+long long delta_rule_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim) {
+  if (max_new < (dim > 32 ? 32 : 64) || dim > 128 || rows <= 0) return 0;
+  const long long f = (rows / DC_T + n_seqs) * heads * (blob_bytes(dim) / 4 + 16LL * round32(vdim));
+  return f <= (1LL << 28) ? f : 0;
+}
+
+cudaError_t launch_delta_rule_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st) {
+  DeltaChunks w;
+  w.blobs = reinterpret_cast<unsigned char*>(ws);
+  w.wv = ws + (rows / DC_T + n_seqs) * d.heads * (blob_bytes(d.dim) / 4);
+  w.vpad = round32(d.vdim);
+  if (d.dim <= 32) return launch<32>(d, n_seqs, max_new, w, st);
+  if (d.dim <= 64) return launch<64>(d, n_seqs, max_new, w, st);
+  return launch<128>(d, n_seqs, max_new, w, st);
+}
+
+}  // namespace vy

@@ -1097,6 +1097,10 @@ extern "C" int64_t vy_delta_rule_workspace_floats(int64_t rows, int32_t heads, i
   return rows * (2LL * kv_heads * dim + static_cast<int64_t>(heads) * dim + heads);
 }
 
+extern "C" int64_t vy_delta_rule_prompt_floats(int64_t rows, int32_t n_seqs, int32_t max_new, int32_t heads, int32_t dim, int32_t vdim) {
+  return vy::delta_rule_mma_floats(rows, n_seqs, max_new, heads, dim, vdim);
+}
+
 extern "C" int vy_delta_rule(const VyDeltaRule* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_delta_rule: null params");
@@ -1117,6 +1121,14 @@ extern "C" int vy_delta_rule(const VyDeltaRule* p) {
   d.unit_eps = p->unit_eps;
   d.state = p->state;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
+  d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
+  const long long prompt_floats = p->workspace ? delta_rule_mma_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->dim, p->vdim) : 0;
+  if (prompt_floats > 0 && p->workspace_floats >= prompt_floats && reinterpret_cast<uintptr_t>(p->workspace) % 16 == 0) {
+    VY_CUDA_OK(launch_delta_rule_mma(d, p->n_seqs, p->max_new, p->rows, p->workspace, st));
+    VY_LAUNCH_OK();
+    count_launch();
+    return VY_OK;
+  }
   if (p->workspace && p->rows > 0 && p->in_dtype == VY_F32 && p->workspace_floats >= vy_delta_rule_workspace_floats(p->rows, p->heads, p->kv_heads, p->dim)) {
     DeltaPrepDev pd;
     pd.rows = p->rows;
@@ -1137,7 +1149,6 @@ extern "C" int vy_delta_rule(const VyDeltaRule* p) {
     d.b = pd.beta; d.ld_b = p->heads; d.b_dt = VY_F32;
     d.prepared = 1;
   }
-  d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaError_t e;
   switch (pad_dim(p->dim)) {
     case 16: e = launch_delta_rule<16>(d, p->n_seqs, st); break;

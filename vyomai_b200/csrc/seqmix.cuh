@@ -159,6 +159,9 @@ struct RecDev {
 // Prompt-sized steps: defined in seqmix_tiled.cu, window_attn_mma.cu and linear_attn_mma.cu.
 cudaError_t launch_linear_attn_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
+// 16 tokens per step of the walk (delta_rule_mma.cu), given delta_rule_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); two launches
+long long delta_rule_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
+cudaError_t launch_delta_rule_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
 // All chunks at once (linear_attn_mma.cu), given linear_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); three launches
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 template <bool TD>
