@@ -160,6 +160,26 @@ def test_score_exchanging_prompts_on_the_tensor_cores(monkeypatch, H, G, d, dv, 
         assert _err(got, torch.cat(want)) < 4 * BOUND   # mixed scores: each is a sum over H capped ones, and the softmax takes its absolute error
 
 
+@pytest.mark.parametrize("taps", [1, 3, 4, 5, 16])
+def test_causal_conv_over_portions_of_every_length(taps):
+    """Portions shorter and longer than the taps and the kernel's token block, carried on; the taps that stay behind are the last inputs."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(taps)
+    C, lengths, more = 130, [1, 15, 16, 17, 70], [33, 2, 16, 1, 15]
+    x = [torch.randn(a + b, C, generator=g) for a, b in zip(lengths, more)]
+    w = torch.randn(C, taps, generator=g)
+    state = torch.full((6, C, max(taps - 1, 1)), float("nan"), device=DEV)
+    slots, out = [4, 1, 0, 5, 2], []
+    for at, take in (([0] * 5, lengths), (lengths, more)):
+        batch = ops.PackedBatch(_i32([sum(take[:i]) for i in range(6)]), _i32(at), _i32(slots), max(take))
+        out.append(ops.causal_conv(batch, torch.cat([x[s][at[s]:at[s] + take[s]] for s in range(5)]).to(DEV), w.to(DEV), state, act="silu").split(take))
+    for s in range(5):
+        assert _err(torch.cat([out[0][s], out[1][s]]), OH.causal_conv(x[s].double(), w.double())) < BOUND
+        if taps > 1:
+            last = torch.cat([torch.zeros(taps, C), x[s]])[-(taps - 1):]
+            assert torch.equal(state[slots[s]].cpu(), last.T)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

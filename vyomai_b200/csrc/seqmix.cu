@@ -495,10 +495,9 @@ struct ConvDev {
   float* state;
   int act;
   void* out; long long ld_out; int out_dt;
-  int fuse_state;   // every sequence's tokens fit one CTA row: the thread that read a channel's taps also writes the new ones
 };
 constexpr int CONV_MAX_TAPS = 16;
-constexpr int CONV_TOK = 32;
+constexpr int CONV_TOK = 16;   // at least CONV_MAX_TAPS - 1: only the first CTA row of a sequence reaches back to the slot's taps
 
 // the last taps - 1 inputs of channel c after the step's n tokens (older ones come from the taps the slot held)
 __device__ __forceinline__ void conv_new_taps(const ConvDev& d, int c, int base, int n, bool carried, float* stp) {
@@ -515,44 +514,43 @@ __device__ __forceinline__ void conv_new_taps(const ConvDev& d, int c, int base,
     if (t < d.taps - 1) stp[t] = tmp[t];
 }
 
+// A thread makes CONV_TOK outputs of one channel from a register window: its CONV_TOK + TAPS - 1 inputs are loaded at once and each serves `taps`
+// outputs. Bound by memory latency, one round trip per thread. fp32, 4 taps, the walk of 32 tokens that loaded an input per tap and output / this:
+// 8192 tokens x 1024 channels 65.5 / 31.8 us, x 512 40.4 / 17.4 us, 80 tokens x 512 31.1 / 7.3 us. The first CTA column of a sequence, the only
+// one that reads the slot's old taps, writes the new ones (a launch of its own before, 2.2 us). TAPS >= taps
+template <int TAPS>
 __global__ void __launch_bounds__(128) causal_conv_kernel(ConvDev d) {
   pdl_trigger();
   pdl_wait();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = blockIdx.z;
+  const int c = blockIdx.y * blockDim.x + threadIdx.x;
+  const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (c >= d.channels) return;
-  float w[CONV_MAX_TAPS];
-#pragma unroll
-  for (int t = 0; t < CONV_MAX_TAPS; ++t) w[t] = t < d.taps ? ld_as_float(d.w, d.w_dt, static_cast<long long>(c) * d.taps + t) : 0.f;
+  if (c >= d.channels || i0 >= n) return;
   const bool carried = d.pos0[s] > 0;
-  const float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
-  for (int i = blockIdx.y * CONV_TOK; i < n && i < (blockIdx.y + 1) * CONV_TOK; ++i) {
+  float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
+  float x[CONV_TOK + TAPS - 1], w[TAPS];
+#pragma unroll
+  for (int u = 0; u < CONV_TOK + TAPS - 1; ++u) {
+    const int j = i0 + u - (TAPS - 1);
+    x[u] = 0.f;
+    if (j >= 0) {
+      if (j < n && j > i0 - d.taps) x[u] = ld_as_float(d.x, d.x_dt, static_cast<long long>(base + j) * d.ldx + c);
+    } else if (carried && j > -d.taps) {
+      x[u] = stp[d.taps - 1 + j];
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < TAPS; ++t) w[t] = t < d.taps ? ld_as_float(d.w, d.w_dt, static_cast<long long>(c) * d.taps + d.taps - 1 - t) : 0.f;   // w[0]: the current token's
+#pragma unroll
+  for (int u = 0; u < CONV_TOK; ++u) {
+    if (i0 + u >= n) break;
     float y = 0.f;
 #pragma unroll
-    for (int dd = 0; dd < CONV_MAX_TAPS; ++dd) {
-      if (dd < d.taps) {
-        const int j = i - dd;
-        float xv = 0.f;
-        if (j >= 0) xv = ld_as_float(d.x, d.x_dt, static_cast<long long>(base + j) * d.ldx + c);
-        else if (carried) xv = stp[d.taps - 1 + j];
-        y = fmaf(w[d.taps - 1 - dd], xv, y);
-      }
-    }
-    st_from_float(d.out, d.out_dt, static_cast<long long>(base + i) * d.ld_out + c, apply_uact(y, d.act));
+    for (int t = 0; t < TAPS; ++t)
+      if (t < d.taps) y = fmaf(w[t], x[u + TAPS - 1 - t], y);
+    st_from_float(d.out, d.out_dt, static_cast<long long>(base + i0 + u) * d.ld_out + c, apply_uact(y, d.act));
   }
-  if (d.fuse_state && d.taps > 1 && n > 0)
-    conv_new_taps(d, c, base, n, carried, d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1));
-}
-
-__global__ void __launch_bounds__(128) causal_conv_state_kernel(ConvDev d) {
-  pdl_trigger();
-  pdl_wait();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = blockIdx.y;
-  const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (c >= d.channels || n <= 0) return;
-  conv_new_taps(d, c, base, n, d.pos0[s] > 0, d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1));
+  if (i0 == 0 && d.taps > 1) conv_new_taps(d, c, base, n, carried, stp);
 }
 
 // ---- recurrences: one thread owns one column of the dim x vdim state in registers ---------------------------------------
@@ -1001,25 +999,21 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
                p->taps, CONV_MAX_TAPS);
   VY_CHECK_ARG(p->x && p->w && p->out && p->x != p->out && (p->state || p->taps == 1) && dtype_ok(p->x_dtype) && dtype_ok(p->w_dtype) &&
                    dtype_ok(p->out_dtype), "vy_causal_conv: bad tensors");
-  VY_CHECK_ARG((p->max_new + CONV_TOK - 1) / CONV_TOK <= 65535, "vy_causal_conv: too many tokens per sequence");
+  VY_CHECK_ARG((p->max_new + 31) / 32 <= 65535, "vy_causal_conv: too many tokens per sequence");
+  VY_CHECK_ARG((p->channels + 127) / 128 <= 65535, "vy_causal_conv: too many channels");
   ConvDev d;
   d.cu = p->cu_tokens; d.pos0 = p->pos0; d.slot = p->slot;
   d.channels = p->channels; d.taps = p->taps;
   d.x = p->x; d.ldx = p->ldx; d.x_dt = p->x_dtype;
   d.w = p->w; d.w_dt = p->w_dtype;
   d.state = p->state; d.act = p->act;
-  d.fuse_state = p->max_new <= CONV_TOK ? 1 : 0;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   const int cb = (p->channels + 127) / 128;
-  VY_CUDA_OK(launch_kernel(causal_conv_kernel, dim3(cb, (p->max_new + CONV_TOK - 1) / CONV_TOK, p->n_seqs), dim3(128), 0, st, d));
+  const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, cb, p->n_seqs);
+  VY_CUDA_OK(p->taps <= 4 ? launch_kernel(causal_conv_kernel<4>, grid, dim3(128), 0, st, d) : launch_kernel(causal_conv_kernel<CONV_MAX_TAPS>, grid, dim3(128), 0, st, d));
   VY_LAUNCH_OK();
   count_launch();
-  if (p->taps > 1 && !d.fuse_state) {
-    VY_CUDA_OK(launch_kernel(causal_conv_state_kernel, dim3(cb, p->n_seqs), dim3(128), 0, st, d));
-    VY_LAUNCH_OK();
-    count_launch();
-  }
   return VY_OK;
 }
 
