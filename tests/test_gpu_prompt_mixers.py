@@ -180,6 +180,30 @@ def test_causal_conv_over_portions_of_every_length(taps):
             assert torch.equal(state[slots[s]].cpu(), last.T)
 
 
+@pytest.mark.parametrize("M,N,K", [(33, 1, 256), (64, 64, 256), (65, 63, 260), (130, 200, 516), (40, 65, 1000)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_fp32_products_on_the_tensor_cores(M, N, K, aligned):
+    """Edges of the 64 x 64 x 64 tiles and the shortest K of the rule, with epilogue; unaligned rows take the FMA form; infinities and NaN stay
+    where a chain of FMAs has them, and rows of very large and very small numbers keep their precision."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(K)
+    pad = 4 if aligned else 3
+    x, w = (torch.randn(r, K + pad, generator=g, device=DEV)[:, :K] for r in (M, N))
+    bias, addend = torch.randn(N, generator=g, device=DEV), torch.randn(M, N, generator=g, device=DEV)
+    x[1] *= 1e30
+    x[2] *= 1e-30
+    want = torch.nn.functional.silu(x.double() @ w.double().T + bias.double()) * 0.5 + addend.double()
+    got = ops.linear_plain(x, w, bias=bias, act="silu", scale=0.5, addend=addend)
+    plain, exact = ops.linear_plain(x, w), x.double() @ w.double().T
+    for a, b in ((got, want), (plain, exact)):
+        for rows in (slice(0, 1), slice(1, 2), slice(2, 3), slice(3, M)):
+            assert _err(a[rows], b[rows].cpu()) < 2 * BOUND   # a few rows of K terms: the sum may be smaller than its terms
+    x[5, K - 1], x[6, 0], w[0, 3] = float("inf"), float("nan"), 0.0
+    bad = ops.linear_plain(x, w)
+    ref = x.double() @ w.double().T
+    assert torch.equal(torch.isnan(bad), torch.isnan(ref)) and torch.equal(torch.isinf(bad), torch.isinf(ref))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -1,10 +1,12 @@
-// vy_linear_plain: out = act(A W^T + bias) * scale + addend for any M, N, K and any alignment, fp32 FMA accumulation.
-// Three kernels: 64 x 64 x 16 shared-memory tiles (4 x 4 outputs per thread) for many rows, a weight-streaming kernel
+// vy_linear_plain: out = act(A W^T + bias) * scale + addend for any M, N, K and any alignment, fp32 accumulation.
+// Four kernels: for many rows 64 x 64 tiles on the tensor cores in fp32 precision where both operands are fp32, aligned and K is long, else
+// 64 x 64 x 16 shared-memory tiles of FMAs (4 x 4 outputs per thread); a weight-streaming kernel
 // (one warp per output feature, lanes over K) for at most 8 rows, and a 32-feature tile for 9 .. 32 rows. A call may hold a batch
 // of independent products of one shape (blockIdx z / y picks the product). This is the exact-fp32 arm of every projection of the
 // sequence-mixer models and the bf16 arm of the shapes the tensor-core GEMM does not take (a contraction over a
 // low rank, a handful of output features, strides that are not 16-byte multiples). vy_unary and vy_embed_rows live
 // here as well.
+#include "split_mma.cuh"
 #include "vy_common.cuh"
 
 namespace vy {
@@ -88,6 +90,135 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(LinDev d) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (m0 + tm + i < d.M && n0 + tn + j < d.N) lin_store(d, m0 + tm + i, n0 + tn + j, acc[i][j]);
+}
+
+// One product in fp32 FMAs: what an infinity or NaN among the operands makes of it (the halves of an infinity would all be NaN)
+static __device__ __noinline__ float lin_dot(const float* a, const float* w, int K) {
+  float acc = 0.f;
+  for (int k = 0; k < K; ++k) acc = fmaf(a[k], w[k], acc);
+  return acc;
+}
+
+// fp32 operands with 16-byte aligned rows: fp32 precision on the tensor cores (split_mma.cuh). 64 rows x 64 features per CTA, a warp 32 x 16.
+// Tiles of 64 k: loaded into registers while the tile before is multiplied, then split, with a scale per row and tile, into one of two buffers; a
+// tile's sums (chains of 4 steps) are added to fp32 registers. 8 warps and two CTAs per SM hide the loads and the splitting behind the products.
+// The FMA form / this, us: 1600 x 3072, K 1024 459 / 173; 8192 x 1024, K 1024 695 / 263; 512 x 1024, K 1024 82 / 26; 8192 x 16, K 1024 77 / 25.
+// Bound by the instructions that split the tiles (three products take a third of the time)
+constexpr int LS_KT = 64, LS_KB = LS_KT * 2 + 16, LS_PLANE = LT * LS_KB, LS_BUF = 4 * LS_PLANE + 2 * LT * 4;
+
+__global__ void __launch_bounds__(256, 2) linear_split_kernel(const LinDev d0) {
+  pdl_trigger();
+  pdl_wait();
+  LinDev d = d0;
+  lin_select(d, blockIdx.z);
+  extern __shared__ __align__(16) unsigned char lin_smem[];
+  const int m0 = blockIdx.y * LT, n0 = blockIdx.x * LT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+  const int lr = 4 * warp + (lane >> 3), lc = (lane & 7) * 4;   // loader: rows lr, lr + 32 of A and of W, columns lc .., lc + 32 ..
+  const float* src[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int r = lr + 32 * (u & 1);
+    src[u] = nullptr;
+    if (u < 2 && m0 + r < d.M) src[u] = static_cast<const float*>(d.A) + static_cast<long long>(m0 + r) * d.lda + lc;
+    if (u >= 2 && n0 + r < d.N) src[u] = static_cast<const float*>(d.W) + static_cast<long long>(n0 + r) * d.ldw + lc;
+  }
+  float4 x[4][2];
+  const auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        x[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (src[u] && k0 + lc + 32 * i < d.K) x[u][i] = *reinterpret_cast<const float4*>(src[u] + k0 + 32 * i);
+      }
+  };
+  float acc[2][2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+  load(0);
+  for (int k0 = 0, b = 0; k0 < d.K; k0 += LS_KT, b ^= 1) {
+    unsigned char* buf = lin_smem + b * LS_BUF;   // A hi | A lo | W hi | W lo | units of A and W rows
+    float* unit = reinterpret_cast<float*>(buf + 4 * LS_PLANE);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u][i].x), fabsf(x[u][i].y)), fmaxf(fabsf(x[u][i].z), fabsf(x[u][i].w))));
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const int ex = split_exponent(m), r = lr + 32 * (u & 1);
+      const float sc = split_scale(ex);
+      if (lc == 0) unit[LT * (u >> 1) + r] = pow2i(ex - SPLIT_TOP);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint2 h, l;
+        split2(x[u][i].x * sc, x[u][i].y * sc, h.x, l.x);
+        split2(x[u][i].z * sc, x[u][i].w * sc, h.y, l.y);
+        unsigned char* o = buf + (u & 2) * LS_PLANE + r * LS_KB + 2 * (lc + 32 * i);
+        *reinterpret_cast<uint2*>(o) = h;
+        *reinterpret_cast<uint2*>(o + LS_PLANE) = l;
+      }
+    }
+    if (k0 + LS_KT < d.K) load(k0 + LS_KT);
+    __syncthreads();   // the only one per tile: the buffer written next was read before this barrier
+    float y[2][2][4], z[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[i][j][e] = z[i][j][e] = 0.f;
+    const unsigned aa = smem_addr(buf) + wm * LS_KB + lane_a(lane, LS_KB), wa = smem_addr(buf) + 2 * LS_PLANE + wn * LS_KB + lane_b(lane, LS_KB);
+#pragma unroll
+    for (int k = 0; k < LS_KT; k += 16) {
+      unsigned ah[2][4], al[2][4], bh[4], bl[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        ldsm_x4(ah[i], aa + 16 * i * LS_KB + 2 * k);
+        ldsm_x4(al[i], aa + LS_PLANE + 16 * i * LS_KB + 2 * k);
+      }
+      ldsm_x4(bh, wa + 2 * k);
+      ldsm_x4(bl, wa + LS_PLANE + 2 * k);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_f16(z[i][j], al[i], bh[2 * j], bh[2 * j + 1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_f16(y[i][j], ah[i], bh[2 * j], bh[2 * j + 1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_f16(z[i][j], ah[i], bl[2 * j], bl[2 * j + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float u0 = unit[wm + 16 * i + (lane >> 2)], u1 = unit[wm + 16 * i + 8 + (lane >> 2)];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 w = *reinterpret_cast<const float2*>(unit + LT + wn + 8 * j + 2 * (lane & 3));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = fmaf((y[i][j][e] + z[i][j][e]) * (e < 2 ? u0 : u1), e & 1 ? w.y : w.x, acc[i][j][e]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int m = m0 + wm + 16 * i + (lane >> 2) + 8 * (e >> 1), n = n0 + wn + 8 * j + 2 * (lane & 3) + (e & 1);
+        if (m >= d.M || n >= d.N) continue;
+        if (!(fabsf(acc[i][j][e]) < INFINITY)) acc[i][j][e] = lin_dot(static_cast<const float*>(d.A) + m * d.lda, static_cast<const float*>(d.W) + n * d.ldw, d.K);
+        lin_store(d, m, n, acc[i][j][e]);
+      }
 }
 
 // at most 8 rows: one warp per output feature, lanes stride over K (coalesced weight rows), shuffle reduction
@@ -289,6 +420,20 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
     VY_CUDA_OK(launch_kernel(linear_small_kernel, dim3((p->N + LS_N - 1) / LS_N, batch), dim3(256), 0, st, d));
   } else {
     VY_CHECK_ARG((p->M + LT - 1) / LT <= 65535, "vy_linear_plain: too many rows (%d)", p->M);
+    const auto rows16 = [](const void* q, int dt, long long ld, long long step) { return dt == VY_F32 && reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0 && step % 4 == 0; };
+    // from K = 256 on: below, a chain of FMAs is at least as exact (all terms positive, K 256: 2.5e-7 by FMAs, 2.1e-7 split; K 64: 1.2e-7, 2.1e-7), and the
+    // two cost the same at 64 (9 us for 33 x 64)
+    if (p->K >= 256 && p->K % 4 == 0 && rows16(d.A, d.a_dt, d.lda, batch > 1 ? d.a_batch : 0) && rows16(d.W, d.w_dt, d.ldw, batch > 1 ? d.w_batch : 0)) {
+      static bool once = false;
+      if (!once) {
+        VY_CUDA_OK(cudaFuncSetAttribute(linear_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * LS_BUF));
+        once = true;
+      }
+      VY_CUDA_OK(launch_kernel(linear_split_kernel, dim3((p->N + LT - 1) / LT, (p->M + LT - 1) / LT, batch), dim3(256), 2 * LS_BUF, st, d));
+      VY_LAUNCH_OK();
+      count_launch();
+      return VY_OK;
+    }
     VY_CUDA_OK(launch_kernel(linear_tile_kernel, dim3((p->N + LT - 1) / LT, (p->M + LT - 1) / LT, batch), dim3(256), 0, st, d));
   }
   VY_LAUNCH_OK();
