@@ -907,7 +907,7 @@ def run_ours(args):
 # ------------------------------------------------------------------------------------------------
 # --workload hybrid: the Gelutar hybrid decoder beside DecoderModel at equal width / depth / vocabulary
 # ------------------------------------------------------------------------------------------------
-HYBRID_KERNELS = ("linear_attn_chunk", "linear_attn", "delta_rule", "window_attn", "causal_conv", "rms_norm", "kv_page_write", "qk_norm_write",
+HYBRID_KERNELS = ("la_states", "la_scan", "la_outputs", "delta_chunk", "delta_scan", "window_attn_mma", "window_attn_split", "linear_split", "linear_attn_chunk", "linear_attn", "delta_rule", "window_attn", "causal_conv", "rms_norm", "kv_page_write", "qk_norm_write",
                   "linear_plain", "unary", "embed_rows", "gemm_skinny", "gemm_kernel", "attn_fwd", "attn_decode", "add_layernorm", "argmax")
 
 
@@ -977,7 +977,7 @@ def measure_hybrid(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, de
     pre_ms = sorted(times)[len(times) // 2]
     out["prefill"] = {"batch": batch_prefill, "prompt": prompt, "ms": round(pre_ms, 3), "tok_per_s": round(batch_prefill * prompt / pre_ms * 1e3)}
     out["prefill_kernels"] = _kernel_table(lambda: prefill(batch_prefill))
-    # the three sequence mixers are fp32 by definition (scores, weights, state): their roofline is the FMA rate, not the tensor cores'
+    # the three sequence mixers are fp32 by definition (scores, weights, state): rates beside the FMA rate, which three 16-bit products per fp32 one may pass
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     fp32_tflops = sms * 128 * 2 * 1.965e9 / 1e12          # nominal: 128 FMA lanes per SM at the maximum SM clock
     tokens, lin, par = batch_prefill * prompt, cfgd["layers"][0]["mixer"], cfgd["layers"][3]["mixer"]
@@ -990,7 +990,9 @@ def measure_hybrid(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, de
              "delta_rule": n_par * tokens * par["right"]["heads"] * 3 * par["right"]["dim"] * par["right"]["vdim"] * 2}
     out["prefill_fp32_roofline"] = {"fp32_tflops_nominal": round(fp32_tflops, 1)}
     for name, f in flops.items():
-        ms = out["prefill_kernels"].get(name, {}).get("ms")
+        forms = {"linear_attn_chunk": ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), "window_attn": ("window_attn_mma", "window_attn_split", "window_attn"),
+                 "delta_rule": ("delta_chunk", "delta_scan", "delta_rule")}[name]
+        ms = sum(out["prefill_kernels"].get(k, {}).get("ms", 0.0) for k in forms)
         if ms:
             out["prefill_fp32_roofline"][name] = {"gflop": round(f / 1e9, 1), "tflops": round(f / ms / 1e9, 2), "frac": round(f / ms / 1e9 / fp32_tflops, 3)}
     eng.release(range(batch_prefill))
@@ -1083,7 +1085,7 @@ def run_hybrid(args):
 # --workload latent: the Zugunex latent-attention / mixture-of-experts decoder beside the Gelutar hybrid decoder at equal
 # width / depth / vocabulary (both run on HybridBatchEngine's packed step)
 # ------------------------------------------------------------------------------------------------
-LATENT_KERNELS = ("window_attn_tiled", "window_attn_decode", "window_attn_heads_merge", "window_attn_heads", "window_attn", "latent_kv_write", "rope_split", "moe_route", "moe_scale", "moe_sort",
+LATENT_KERNELS = ("window_attn_mma", "window_attn_split", "la_states", "la_scan", "la_outputs", "delta_chunk", "delta_scan", "linear_split", "window_attn_decode", "window_attn_heads_merge", "window_attn_heads", "window_attn", "latent_kv_write", "rope_split", "moe_route", "moe_scale", "moe_sort",
                   "moe_gather", "moe_combine", "linear_tile", "linear_rows", "linear_attn_chunk", "linear_attn", "delta_rule", "delta_prep",
                   "causal_conv", "rms_norm", "kv_page_write", "unary", "embed_rows", "gemm_skinny", "gemm_kernel", "argmax")
 
@@ -1178,9 +1180,9 @@ def measure_latent(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, de
     row = m["kv_rank"] + m["rot_dim"]
     # whole prompts attend over per-head expanded keys / values: dim + rot_dim and vdim channels per (query, key, head)
     fl = len(cfgd["layers"]) * tokens * m["heads"] * visible * (m["dim"] + m["rot_dim"] + m["vdim"]) * 2
-    ms = z["prefill_kernels"].get("window_attn_tiled", {}).get("ms")
+    ms = z["prefill_kernels"].get("window_attn_mma", {}).get("ms")
     if ms:
-        z["window_attn_tiled_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        z["window_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     # single-token attention: the bytes of the visible latent rows, read once per (sequence, layer) if the heads share them through L2
     dk = z["decode_kernels_eager"]   # 8 or more heads per latent row: the heads-as-rows kernel and its merge; else the key-parallel kernel
     ms = sum(dk.get(k, {}).get("ms", 0.0) for k in ("window_attn_heads", "window_attn_heads_merge", "window_attn_decode"))
@@ -1206,9 +1208,9 @@ def measure_latent(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, de
     Wg, K = par["mask"]["size"], par["mask"]["keep_first"]
     vis = sum(min(p + 1, Wg) + (min(K, p + 1 - Wg) if p + 1 > Wg else 0) for p in range(prompt)) / prompt
     fl = n_par * tokens * par["heads"] * vis * (par["dim"] + par["vdim"]) * 2
-    ms = gz["prefill_kernels"].get("window_attn_tiled", {}).get("ms")
+    ms = gz["prefill_kernels"].get("window_attn_mma", {}).get("ms")
     if ms:
-        gz["window_attn_tiled_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        gz["window_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     ms = gz["decode_kernels_eager"].get("window_attn_decode", {}).get("ms")
     if ms:
         by = n_par * batch_decode * (Wg + K) * par["kv_heads"] * (par["dim"] + par["vdim"]) * 4
@@ -1257,7 +1259,7 @@ def run_latent(args):
 # --workload talking: the Vazepel parallel-layer decoder (score-exchanging attention, gated experts) beside the Zugunex
 # latent-attention decoder at equal width / depth / vocabulary (both run on HybridBatchEngine's packed step)
 # ------------------------------------------------------------------------------------------------
-TALKING_KERNELS = ("talk_attn_tiled", "talk_attn_rows", "talk_attn_merge", "depth_mix_norm", "moe_glu", "rope_kv_write") + LATENT_KERNELS
+TALKING_KERNELS = ("talk_attn_mma", "talk_attn_tiled", "talk_attn_rows", "talk_attn_merge", "depth_mix_norm", "moe_glu", "rope_kv_write") + LATENT_KERNELS
 
 
 def talking_config(width, layers=8, vocab=32768):
@@ -1299,9 +1301,9 @@ def measure_talking(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     visible = (prompt + 1) / 2.0
     # prompts: the two contractions (dim + vdim channels per query, key, head) plus the exchange (heads multiply-adds per query, key, head)
     fl = n_layers * tokens * H * visible * (m["dim"] + m["vdim"] + H) * 2
-    ms = z["prefill_kernels"].get("talk_attn_tiled", {}).get("ms")
+    ms = z["prefill_kernels"].get("talk_attn_mma", {}).get("ms")
     if ms:
-        z["talk_attn_tiled_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        z["talk_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     dk = z["decode_kernels_eager"]
     ms = sum(dk.get(k, {}).get("ms", 0.0) for k in ("talk_attn_rows", "talk_attn_merge"))
     if ms:
@@ -1326,9 +1328,9 @@ def measure_talking(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     Wn = lm["mask"]["size"]
     vis = sum(min(p + 1, Wn) for p in range(prompt)) / prompt
     fl = len(ld["layers"]) * tokens * lm["heads"] * vis * (lm["dim"] + lm["rot_dim"] + lm["vdim"]) * 2
-    ms = lz["prefill_kernels"].get("window_attn_tiled", {}).get("ms")
+    ms = lz["prefill_kernels"].get("window_attn_mma", {}).get("ms")
     if ms:
-        lz["window_attn_tiled_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        lz["window_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     dk = lz["decode_kernels_eager"]
     ms = sum(dk.get(k, {}).get("ms", 0.0) for k in ("window_attn_heads", "window_attn_heads_merge", "window_attn_decode"))
     if ms:
@@ -1437,9 +1439,9 @@ def measure_fubinex(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     # recurrences: per (token, head) and state element, gated linear attention does a decay multiply and two multiply-adds (5 flop), the
     # chunked fixed-decay kernel is counted as in --workload hybrid
     z["prefill_roofline"] = {
-        "window_attn_tiled": _roof(pk, ("window_attn_tiled",), flop=fl_attn, **rf),
+        "window_attn_mma": _roof(pk, ("window_attn_mma",), flop=fl_attn, **rf),
         "gated_linear_attn (delta_rule kernel, no correction)": _roof(pk, ("delta_rule",), flop=n_par * tokens * rt["heads"] * rt["dim"] * rt["vdim"] * 5, **rf),
-        "linear_attn_chunk": _roof(pk, ("linear_attn_chunk",), flop=n_ret * tokens * ret["heads"] * (2 * ret["dim"] * ret["vdim"] + 32 * (ret["dim"] + ret["vdim"])) * 2, **rf),
+        "linear_attn_chunk": _roof(pk, ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), flop=n_ret * tokens * ret["heads"] * (2 * ret["dim"] * ret["vdim"] + 32 * (ret["dim"] + ret["vdim"])) * 2, **rf),
         # row kernels against the copy bandwidth: fp32 in, bf16 out (poly_norm); q / k read and written in fp32, v copied (rotation)
         "poly_norm": _roof(pk, ("poly_norm",), byts=n_all * tokens * ff * 6, **rf),
         "rope_heads": _roof(pk, ("rope_heads",), byts=tokens * (n_par * (lf["heads"] + 2 * lf["kv_heads"]) * lf["dim"] + n_ret * 2 * ret["heads"] * ret["dim"]) * 8, **rf),
@@ -1481,10 +1483,10 @@ def measure_fubinex(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     vis = sum(min(p + 1, Wg) + (min(K, p + 1 - Wg) if p + 1 > Wg else 0) for p in range(prompt)) / prompt
     gpk, gdk = gz["prefill_kernels"], gz["decode_kernels_eager"]
     gz["prefill_roofline"] = {
-        "window_attn_tiled": _roof(gpk, ("window_attn_tiled",), flop=g_par * tokens * gl["heads"] * vis * (gl["dim"] + gl["vdim"]) * 2, **rf),
+        "window_attn_mma": _roof(gpk, ("window_attn_mma",), flop=g_par * tokens * gl["heads"] * vis * (gl["dim"] + gl["vdim"]) * 2, **rf),
         # the delta rule adds the correction's contraction: a decay multiply and three multiply-adds per state element (7 flop)
-        "delta_rule": _roof(gpk, ("delta_rule",), flop=g_par * tokens * gr["heads"] * gr["dim"] * gr["vdim"] * 7, **rf),
-        "linear_attn_chunk": _roof(gpk, ("linear_attn_chunk",), flop=g_lin * tokens * glin["heads"] * (2 * glin["dim"] * glin["vdim"] + 32 * (glin["dim"] + glin["vdim"])) * 2, **rf),
+        "delta_rule": _roof(gpk, ("delta_rule", "delta_chunk", "delta_scan"), flop=g_par * tokens * gr["heads"] * gr["dim"] * gr["vdim"] * 7, **rf),
+        "linear_attn_chunk": _roof(gpk, ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), flop=g_lin * tokens * glin["heads"] * (2 * glin["dim"] * glin["vdim"] + 32 * (glin["dim"] + glin["vdim"])) * 2, **rf),
         "unary (relu^2 between the feed-forward products, fp32 in / bf16 out)": _roof(gpk, ("unary",), byts=len(gd["layers"]) * tokens * ff * 6, **rf),
     }
     gz["decode_roofline"] = {
@@ -1574,7 +1576,7 @@ def measure_kifetar(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     chan = 2 * dl["kv_heads"] * dl["dim"] + dl["heads"] * dl["vdim"]
     vis = sum(min(p + 1, W) for p in range(prompt)) / prompt
     z["prefill_roofline"] = {
-        "window_attn_tiled": _roof(pk, ("window_attn_tiled",), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
+        "window_attn_mma": _roof(pk, ("window_attn_mma",), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
         # a decay multiply and three multiply-adds per state element and token, as Gelutar's delta rule is counted
         "gd_scan (gated delta rule)": _roof(pk, ("gd_scan",), flop=n_d * tokens * state * 7, **rf),
         # row kernels against the copy bandwidth. gd_prep: projections in, unit vectors / values / records out (fp32)
@@ -1614,8 +1616,8 @@ def measure_kifetar(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     gstate, gchan = gr["heads"] * gr["dim"] * gr["vdim"], 2 * gr["kv_heads"] * gr["dim"] + gr["heads"] * gr["vdim"]
     glin = gd["layers"][0]["mixer"]
     gz["prefill_roofline"] = {
-        "window_attn_tiled": _roof(gpk, ("window_attn_tiled",), flop=g_par * tokens * gl["heads"] * gvis * (gl["dim"] + gl["vdim"]) * 2, **rf),
-        "delta_rule (+ its preparing launch)": _roof(gpk, ("delta_rule",), flop=g_par * tokens * gstate * 7, **rf),
+        "window_attn_mma": _roof(gpk, ("window_attn_mma",), flop=g_par * tokens * gl["heads"] * gvis * (gl["dim"] + gl["vdim"]) * 2, **rf),
+        "delta_rule (+ its preparing launch)": _roof(gpk, ("delta_rule", "delta_chunk", "delta_scan"), flop=g_par * tokens * gstate * 7, **rf),
         "causal_conv": _roof(gpk, ("causal_conv",), byts=g_par * tokens * gchan * 8, **rf),
         # layer norms (bf16 out), the parallel layer's q / k norms and its two output norms added into the residual, the recurrences' gated read-outs
         "rms_norm": _roof(gpk, ("rms_norm",), byts=tokens * ((2 * len(gd["layers"]) + g_lin) * width * 6 + g_lin * glin["heads"] * glin["vdim"] * 4 +
@@ -1710,9 +1712,9 @@ def measure_zaparax(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     chosen = top * moe["router"]["experts"] / (moe["router"]["experts"] + moe["router"]["identity"])
     vis = sum(min(p + 1, W) for p in range(prompt)) / prompt
     z["prefill_roofline"] = {
-        "window_attn_tiled": _roof(pk, ("window_attn_tiled",), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
+        "window_attn_mma": _roof(pk, ("window_attn_mma",), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
         # per token and head: carried state read and updated (dim x vdim each), half a chunk of 64 inside it; counted as the fixed-decay form is
-        "linear_attn_chunk (state-space recurrence)": _roof(pk, ("linear_attn_chunk",), flop=n_s * tokens * sm["heads"] *
+        "linear_attn_chunk (state-space recurrence)": _roof(pk, ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), flop=n_s * tokens * sm["heads"] *
                                                             (2 * sm["state"] * sm["vdim"] + 32 * (sm["state"] + sm["vdim"])) * 2, **rf),
         "ssd_conv": _roof(pk, ("ssd_conv",), byts=n_s * tokens * chan * 8, **rf),
         # a close reads residual and result, writes residual and the next norm (bf16); behind experts it also reads some bf16 input rows
@@ -1751,7 +1753,7 @@ def measure_zaparax(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     kpk, kdk = kz["prefill_kernels"], kz["decode_kernels_eager"]
     kstate, kchan = dl["heads"] * dl["dim"] * dl["vdim"], 2 * dl["kv_heads"] * dl["dim"] + dl["heads"] * dl["vdim"]
     kz["prefill_roofline"] = {
-        "window_attn_tiled": _roof(kpk, ("window_attn_tiled",), flop=n_a * tokens * ka["heads"] * vis * (ka["dim"] + ka["vdim"]) * 2, **rf),
+        "window_attn_mma": _roof(kpk, ("window_attn_mma",), flop=n_a * tokens * ka["heads"] * vis * (ka["dim"] + ka["vdim"]) * 2, **rf),
         "gd_scan (gated delta rule)": _roof(kpk, ("gd_scan",), flop=n_s * tokens * kstate * 7, **rf),
         "gd_prep": _roof(kpk, ("gd_prep",), byts=n_s * tokens * (2 * kchan + 18 * dl["heads"]) * 4, **rf),
         "sandwich_norm": _roof(kpk, ("sandwich_norm",), byts=2 * n_all * tokens * width * 14, **rf),

@@ -109,7 +109,8 @@ __device__ __forceinline__ float block_max(float m, float* red) {
 constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows of 64 value columns
 
 // CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w ..; tokens are the summed index, so k and the
-// weighted v are each scaled by one power of two for the whole chunk. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: see la_outputs
+// weighted v are each scaled by one power of two for the whole chunk. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 84 us, bound by
+// writing the states (268 MB) and by the latency of each chunk's few steps
 // ACT: see act_of
 template <bool TD, int ACT>
 __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
@@ -283,7 +284,8 @@ __global__ void __launch_bounds__(256) la_scan_kernel(RecDev d, LaChunks w) {
 constexpr int LO_T = 128, LO_W = 4;
 
 // CTA: (chunk, 64 value columns) x (hp heads that share q and k) x sequence; warp w owns tokens 16 w .. 16 w + 15 and keeps their scores in registers
-// for all its heads. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8
+// for all its heads. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 277 us (la_scan 83; the walk over the chunks was 737 us for everything). Bound by
+// fixed latencies at two warps per scheduler (255 registers): the tensor pipe is 13 % active; twice the warps with half the columns: 301 us
 template <bool TD, int ACT>
 __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec, bool svec) {
   pdl_trigger();

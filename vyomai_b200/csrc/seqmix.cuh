@@ -1,5 +1,5 @@
 // Shared by the sequence-mixer kernels (seqmix.cu: token-serial forms used for single tokens and short portions;
-// seqmix_tiled.cu: tiled forms used for prompts): activation helpers, the kernels' argument blocks and the tiled launchers.
+// seqmix_tiled.cu, window_attn_mma.cu, linear_attn_mma.cu, delta_rule_mma.cu: forms used for prompts): activation helpers, the kernels' argument blocks and the tiled launchers.
 #pragma once
 #include <math.h>
 
@@ -156,7 +156,7 @@ struct RecDev {
   void* out; long long ld_out; int out_dt;
 };
 
-// Prompt-sized steps: defined in seqmix_tiled.cu, window_attn_mma.cu and linear_attn_mma.cu.
+// Prompt-sized steps: defined in the files named above.
 cudaError_t launch_linear_attn_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 // 16 tokens per step of the walk (delta_rule_mma.cu), given delta_rule_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); two launches

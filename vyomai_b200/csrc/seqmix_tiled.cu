@@ -1,16 +1,14 @@
-// Prompt-sized forms of two sequence mixers, in fp32 on register tiles (scores, softmax weights, decays and recurrent state
-// are 32-bit by the models' definition, so the contractions run on the FMA pipes, not on the 16-bit tensor-core path):
+// Linear attention with a fixed decay and the state-space recurrence, chunk by chunk, in fp32 on register tiles: the form for portions of up to 64
+// tokens, for heads of more than 128 channels and for calls without a workspace (linear_attn_mma.cu takes the other ones, all chunks at once):
 //
 //   * linear attention with a fixed decay, chunk by chunk: for a chunk of C tokens with the state S0 before it,
 //       O = (Q K^T . D) V + diag(decay^(i+1)) Q S0,   D[i][j] = decay^(i-j) for j <= i, else 0
 //       S = decay^C S0 + sum_j decay^(C-1-j) k_j v_j^T
 //     one CTA owns (sequence, head, 64 value columns) and walks the chunks in order with its slice of S in shared memory.
 //     The state-space recurrence runs on the same kernel with a decay and a write strength per token: decay^(i-j) becomes
-//     exp(L_i - L_j) w_j with L the summed log decays of the chunk (kept as two floats: their differences are what counts);
-//   * windowed softmax attention with kept first tokens and a sink over pages: one CTA owns 64 queries of one head, walks
-//     the visible keys in tiles of 64 (the kept prefix first, then the window band) with an online softmax.
+//     exp(L_i - L_j) w_j with L the summed log decays of the chunk (kept as two floats: their differences are what counts).
 //
-// Both give the same values as the token-serial kernels of seqmix.cu up to fp32 rounding, whatever the portion sizes.
+// It gives the same values as the token-serial kernels of seqmix.cu up to fp32 rounding, whatever the portion sizes.
 #include <stdlib.h>
 
 #include "seqmix.cuh"
