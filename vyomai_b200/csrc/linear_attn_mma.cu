@@ -110,7 +110,7 @@ constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows 
 
 // CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w ..; tokens are the summed index, so k and the
 // weighted v are each scaled by one power of two for the whole chunk. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 84 us, bound by
-// writing the states (268 MB) and by the latency of each chunk's few steps
+// writing the states (134 MB) and by the latency of each chunk's few steps
 // ACT: see act_of
 template <bool TD, int ACT>
 __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
