@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define VY_ABI_VERSION 13
+#define VY_ABI_VERSION 14
 
 #if defined(__GNUC__)
 #define VY_API __attribute__((visibility("default")))
