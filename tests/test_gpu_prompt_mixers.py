@@ -204,6 +204,21 @@ def test_fp32_products_on_the_tensor_cores(M, N, K, aligned):
     assert torch.equal(torch.isnan(bad), torch.isnan(ref)) and torch.equal(torch.isinf(bad), torch.isinf(ref))
 
 
+@pytest.mark.parametrize("ratio", [2.0 ** 16, 2.0 ** 20, 2.0 ** 24])
+def test_fp32_products_of_entries_far_below_their_row_s_largest(ratio):
+    """One entry per row is `ratio` times the others and meets a zero: the sums consist of the small ones alone."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, w = torch.randn(65, 320, generator=g, device=DEV), torch.randn(70, 320, generator=g, device=DEV)
+    x[:, 7::64] = ratio
+    w[:, 7::64] = 0.0
+    assert _err(ops.linear_plain(x, w), (x.double() @ w.double().T).cpu()) < BOUND
+    w, x = torch.randn(70, 320, generator=g, device=DEV), torch.randn(65, 320, generator=g, device=DEV)
+    w[:, 7::64] = ratio
+    x[:, 7::64] = 0.0
+    assert _err(ops.linear_plain(x, w), (x.double() @ w.double().T).cpu()) < BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -25,7 +25,7 @@ constexpr int DC_NW = 2;            // warps of the walk's CTA: 32 value columns
 constexpr int DC_NS = 3;            // chunks in flight per CTA of the walk
 // A tensor-core accumulation cuts off where fp32 rounds: a result is this share too small on average (measured: read-outs -5.8e-8 without it,
 // -0.4e-8 with it, the serial walk +0.5e-8). A sum of n accumulations loses (n + 1) / 2 such shares of its end value on average
-constexpr float DC_CUT = 0x1p-25f;
+constexpr float DC_CUT = 0x1p-25f / LO_UNIT;   // in the unit of the small products' sums, to which it is added
 
 // One chunk and head in the workspace. An operand entry is 16 bytes per lane: (b0, b1) of mma.m16n8k16, hi then lo
 template <int DP>
@@ -292,7 +292,7 @@ static __device__ __noinline__ void dc_read_finite(float (&o)[2][4], const float
       const int t = 8 * (r >> 1) + tq + (r & 1);
       if (s > t) continue;
       const __half* e = reinterpret_cast<const __half*>(b + 16 * (32 * (t >> 3) + 4 * (t & 7) + ((s & 7) >> 1))) + 2 * (s >> 3) + (s & 1);
-      const float x = (__half2float(e[0]) + __half2float(e[4])) * unit[t];
+      const float x = fmaf(__half2float(e[4]), LO_UNIT, __half2float(e[0])) * unit[t];
       o[r >> 1][r & 1] = fmaf(x, u0, o[r >> 1][r & 1]);
       o[r >> 1][2 + (r & 1)] = fmaf(x, u1, o[r >> 1][2 + (r & 1)]);
     }
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       const float2 p = *reinterpret_cast<const float2*>(unit + 8 * j + tq);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float y0 = r[j][e] + half[j][e], z = (y0 + fmaf(y0, cut, x[j][e])) * (e < 2 ? n0 : n1);
+        const float y0 = r[j][e] + half[j][e], z = fmaf(fmaf(y0, cut, x[j][e]), LO_UNIT, y0) * (e < 2 ? n0 : n1);
         u[j][e] = fmaf(-z, e & 1 ? p.y : p.x, e == 0 ? y.x : e == 1 ? y.y : e == 2 ? y.z : y.w);
       }
       m0 = fmaxf(m0, fmaxf(fabsf(u[j][0]), fabsf(u[j][1])));
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       for (int i = 0; i < 2; ++i) {
         const float2 g = *reinterpret_cast<const float2*>(G + 8 * (j + i));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[j + i][e] = fmaf(S[j + i][e], e & 1 ? g.y : g.x, (y[i][e] + fmaf(y[i][e], DC_CUT, z[i][e])) * (e < 2 ? k0 : k1));
+        for (int e = 0; e < 4; ++e) S[j + i][e] = fmaf(S[j + i][e], e & 1 ? g.y : g.x, fmaf(fmaf(y[i][e], DC_CUT, z[i][e]), LO_UNIT, y[i][e]) * (e < 2 ? k0 : k1));
       }
     }
     // the read-outs
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float y0 = r[2 + j][e] + half[2 + j][e];
-        o[j][e] = (y0 + fmaf(y0, cut, x[2 + j][e])) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
+        o[j][e] = fmaf(fmaf(y0, cut, x[2 + j][e]), LO_UNIT, y0) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
       }
     }
     bool finite = true;
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
         mma_f16(y, uh, f.x, f.y);
         mma_f16(z, uh, f.z, f.w);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[j][e] = fmaf((y[e] + fmaf(y[e], DC_CUT, z[e])) * (e < 2 ? w0 : w1), e & 1 ? p.y : p.x, o[j][e]);
+        for (int e = 0; e < 4; ++e) o[j][e] = fmaf(fmaf(fmaf(y[e], DC_CUT, z[e]), LO_UNIT, y[e]) * (e < 2 ? w0 : w1), e & 1 ? p.y : p.x, o[j][e]);
       }
     } else {
       dc_read_finite(o, u, st + Blob::b_at, unit + 2 * DC_T, lane);

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, i
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int col = 8 * j + 2 * tq;
-          const float p = (a[j][2 * r] + b[j][2 * r]) * u1 * u2, q = (a[j][2 * r + 1] + b[j][2 * r + 1]) * u1 * u2;
+          const float p = fmaf(b[j][2 * r], LO_UNIT, a[j][2 * r]) * u1 * u2, q = fmaf(b[j][2 * r + 1], LO_UNIT, a[j][2 * r + 1]) * u1 * u2;
           float* at = U + static_cast<long long>(i) * d.vdim + col;
           if (col + 1 < vw && d.vdim % 2 == 0) *reinterpret_cast<float2*>(at) = make_float2(p, q);
           else {
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) p[2 * j + i][e] = (a[i][e] + b[i][e]) * qunit[e >> 1] * ku[16 * j + 8 * i + 2 * tq + (e & 1)];
+      for (int e = 0; e < 4; ++e) p[2 * j + i][e] = fmaf(b[i][e], LO_UNIT, a[i][e]) * qunit[e >> 1] * ku[16 * j + 8 * i + 2 * tq + (e & 1)];
   }
   for (int h = h0; h < h0 + hp; ++h) {
     __syncthreads();   // the readers of k, or of the previous head's values and state, are done
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][e] = (o[i][e] + b[i][e]) * su * f[e >> 1];
+        for (int e = 0; e < 4; ++e) o[i][e] = fmaf(b[i][e], LO_UNIT, o[i][e]) * su * f[e >> 1];
     }
     // the weights inside the chunk, times the exponent of each value row, then scaled row by row
     unsigned ph[4][4], pl[4][4];
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[4 * cb + i][e] = fmaf(a[i][e] + b[i][e], pu[e >> 1] * v_unit, o[4 * cb + i][e]);
+        for (int e = 0; e < 4; ++e) o[4 * cb + i][e] = fmaf(fmaf(b[i][e], LO_UNIT, a[i][e]), pu[e >> 1] * v_unit, o[4 * cb + i][e]);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256, 2) linear_split_kernel(const LinDev d0) {
       for (int j = 0; j < 2; ++j) {
         const float2 w = *reinterpret_cast<const float2*>(unit + LT + wn + 8 * j + 2 * (lane & 3));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[i][j][e] = fmaf((y[i][j][e] + z[i][j][e]) * (e < 2 ? u0 : u1), e & 1 ? w.y : w.x, acc[i][j][e]);
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = fmaf(fmaf(z[i][j][e], LO_UNIT, y[i][j][e]) * (e < 2 ? u0 : u1), e & 1 ? w.y : w.x, acc[i][j][e]);
       }
     }
   }

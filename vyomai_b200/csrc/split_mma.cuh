@@ -1,10 +1,11 @@
 // fp32 contractions on the tensor cores: every operand row is scaled by a power of two (exact) so that its largest entry lies in
-// [2^12, 2^13), and each entry becomes the sum of two fp16 numbers, x = hi + lo. hi carries 11 significant bits and lo the next 11
-// or 12, so hi + lo is off by at most 2^-23 |x| (entries more than 2^27 below their row's largest: by 2^-38 of that largest one), about
-// what fp32 itself resolves. A product of two such rows is lo hi + hi lo + hi hi with fp32 accumulation; the dropped lo lo term is below
-// 2^-22 of a product and random in sign. The two small products get an accumulator of their own, and an accumulator takes few steps before
-// it is added to a longer sum in fp32 registers: a tensor-core accumulation does not round to nearest, and this keeps its share of the
-// error below that of a serial fp32 FMA chain. Three 16-bit products run at a third of the 16-bit rate where fp32 FMAs run at an eighth
+// [2^12, 2^13), and each entry becomes two fp16 numbers, x = hi + 2^-11 lo. hi carries 11 significant bits and lo the next 11 or 12; kept 2^11
+// times larger, lo stays a normal fp16 number as long as hi does. So the pair is off by at most 2^-23 |x| down to 2^24 below the row's largest
+// entry, by 2^-22 |x| down to 2^27 below it, and by 2^-49 of that largest entry further down (lo itself stored instead: 2^-23 |x| only down to 2^14
+// below, then 2^-38 of the largest). A product of two such rows is hi hi + 2^-11 (lo hi + hi lo) with fp32 accumulation; the dropped lo lo term is
+// below 2^-22 of a product and random in sign. The two small products get an accumulator of their own (LO_UNIT undoes the 2^11), and an accumulator
+// takes few steps before it is added to a longer sum in fp32 registers: a tensor-core accumulation does not round to nearest, and this keeps its
+// share of the error below that of a serial fp32 FMA chain. Three 16-bit products run at a third of the 16-bit rate where fp32 FMAs run at an eighth
 // of it (and need a shared-memory operand read per FMA).
 #pragma once
 #include <cuda_fp16.h>
@@ -14,6 +15,7 @@
 namespace vy {
 
 constexpr int SPLIT_TOP = 12;     // scaled rows have their largest entry in [2^SPLIT_TOP, 2^(SPLIT_TOP + 1))
+constexpr float LO_UNIT = 0x1p-11f;   // a lo half is stored in this unit
 constexpr int SPLIT_MIN_E = -100; // rows whose largest entry is below 2^-100 (all zero, for one) keep this exponent: scales stay finite
 
 // exponent of a row's largest absolute value
@@ -31,7 +33,7 @@ __device__ __forceinline__ void split2(float a, float b, unsigned& hi, unsigned&
   const __half2 h = __floats2half2_rn(a, b);
   const float2 f = __half22float2(h);
   hi = pack_h2(h);
-  lo = pack_h2(__floats2half2_rn(a - f.x, b - f.y));
+  lo = pack_h2(__floats2half2_rn((a - f.x) * (1.f / LO_UNIT), (b - f.y) * (1.f / LO_UNIT)));
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }

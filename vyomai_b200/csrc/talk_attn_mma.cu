@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
       const float2 k2 = *reinterpret_cast<const float2*>(ku + g * N + 8 * i + 2 * tq);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        sc[i][e] = cap_score((sc[i][e] + x[i][e]) * (e & 1 ? k2.y : k2.x) * qm[e >> 1], d.softcap, two_over_cap);
+        sc[i][e] = cap_score(fmaf(x[i][e], LO_UNIT, sc[i][e]) * (e & 1 ? k2.y : k2.x) * qm[e >> 1], d.softcap, two_over_cap);
         largest = fmaxf(largest, fabsf(sc[i][e]));
       }
     }
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
 #pragma unroll
             for (int i = 0; i < 2; ++i)
               *reinterpret_cast<float2*>(X + h * C::XH + q * C::XQ + 16 * j + 8 * i + 2 * tq) =
-                  make_float2((y[a][i][2 * r] + z[a][i][2 * r]) * f, (y[a][i][2 * r + 1] + z[a][i][2 * r + 1]) * f);
+                  make_float2(fmaf(z[a][i][2 * r], LO_UNIT, y[a][i][2 * r]) * f, fmaf(z[a][i][2 * r + 1], LO_UNIT, y[a][i][2 * r + 1]) * f);
           }
         }
     }
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[2 * cc + i][e] = fmaf(o[2 * cc + i][e], keep_o[e >> 1], y[i][e] + z[i][e]);
+        for (int e = 0; e < 4; ++e) o[2 * cc + i][e] = fmaf(o[2 * cc + i][e], keep_o[e >> 1], fmaf(z[i][e], LO_UNIT, y[i][e]));
     }
   }
   cp_async_wait<0>();

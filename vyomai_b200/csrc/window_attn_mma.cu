@@ -211,7 +211,7 @@ window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16,
     for (int i = 0; i < NT; ++i) {
       const float kx[2] = {ke[(8 * i + 2 * tq) * ustep], ke[(8 * i + 2 * tq + 1) * ustep]};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) sc[i][e] = fmaf((sc[i][e] + x[i][e]) * kx[e & 1], qmul[e >> 1], badd[e >> 1]);
+      for (int e = 0; e < 4; ++e) sc[i][e] = fmaf(fmaf(x[i][e], LO_UNIT, sc[i][e]) * kx[e & 1], qmul[e >> 1], badd[e >> 1]);
     }
     // a tile of neighbouring keys (no kept ones) that every query sees needs no mask per pair
     const int f = lo + (c0 - nA), t = f + N - 1;
@@ -310,7 +310,7 @@ window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16,
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[4 * cc + i][e] = fmaf(o[4 * cc + i][e], keep_o[e >> 1], y[i][e] + z[i][e]);
+        for (int e = 0; e < 4; ++e) o[4 * cc + i][e] = fmaf(o[4 * cc + i][e], keep_o[e >> 1], fmaf(z[i][e], LO_UNIT, y[i][e]));
     }
     if constexpr (PRE) {   // the warp that is through with a buffer last refills it
       __syncwarp();
