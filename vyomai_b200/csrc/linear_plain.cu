@@ -8,6 +8,7 @@
 // here as well.
 #include "split_mma.cuh"
 #include "vy_common.cuh"
+#include "vy_ptx.cuh"   // warp_sum
 
 namespace vy {
 
@@ -92,17 +93,29 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(LinDev d) {
       if (m0 + tm + i < d.M && n0 + tn + j < d.N) lin_store(d, m0 + tm + i, n0 + tn + j, acc[i][j]);
 }
 
-// One product in fp32 FMAs: what an infinity or NaN among the operands makes of it (the halves of an infinity would all be NaN)
+// One product in fp32 FMAs by a warp (16-byte aligned rows, K a multiple of 4), the sum in every lane
 static __device__ __noinline__ float lin_dot(const float* a, const float* w, int K) {
   float acc = 0.f;
-  for (int k = 0; k < K; ++k) acc = fmaf(a[k], w[k], acc);
-  return acc;
+  for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
+    const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+    acc = fmaf(x.x, y.x, acc);
+    acc = fmaf(x.y, y.y, acc);
+    acc = fmaf(x.z, y.z, acc);
+    acc = fmaf(x.w, y.w, acc);
+  }
+  return warp_sum(acc);
 }
+
+// An entry's halves are off by at most 2^-48 of the largest entry of its row and tile (split_mma.cuh), so a product is as good as an fp32 one unless it is
+// this small beside its rows' largest entries: then, as where an infinity or NaN went in (the halves of an infinity would all be NaN), it is computed again
+// in FMAs. At 2^-16 the halves' share is below 2^-25 of the product; of normal numbers' products 2 to 6 in a million are that small
+constexpr float LS_SMALL = 0x1p-16f * (1 << SPLIT_TOP) * (1 << SPLIT_TOP);
 
 // fp32 operands with 16-byte aligned rows: fp32 precision on the tensor cores (split_mma.cuh). 64 rows x 64 features per CTA, a warp 32 x 16.
 // Tiles of 64 k: loaded into registers while the tile before is multiplied, then split, with a scale per row and tile, into one of two buffers; a
 // tile's sums (chains of 4 steps) are added to fp32 registers. 8 warps and two CTAs per SM hide the loads and the splitting behind the products.
-// The FMA form / this, us: 1600 x 3072, K 1024 459 / 173; 8192 x 1024, K 1024 695 / 263; 512 x 1024, K 1024 82 / 26; 8192 x 16, K 1024 77 / 25.
+// The FMA form / this, us: 1600 x 3072, K 1024 460 / 178; 8192 x 1024, K 1024 696 / 275; 512 x 1024, K 1024 82 / 28; 8192 x 16, K 1024 77 / 27 (error
+// against 64 bits 5.7e-7 / 1.6e-7; without the second look at small products 173, 264, 26, 25 us).
 // Bound by the instructions that split the tiles (three products take a third of the time)
 constexpr int LS_KT = 64, LS_KB = LS_KT * 2 + 16, LS_PLANE = LT * LS_KB, LS_BUF = 4 * LS_PLANE + 2 * LT * 4;
 
@@ -140,6 +153,7 @@ __global__ void __launch_bounds__(256, 2) linear_split_kernel(const LinDev d0) {
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+  float top_a[2][2] = {}, top_w[2][2] = {};   // the largest units of this lane's rows of A (and of 8 below) and of W
   load(0);
   for (int k0 = 0, b = 0; k0 < d.K; k0 += LS_KT, b ^= 1) {
     unsigned char* buf = lin_smem + b * LS_BUF;   // A hi | A lo | W hi | W lo | units of A and W rows
@@ -153,7 +167,7 @@ __global__ void __launch_bounds__(256, 2) linear_split_kernel(const LinDev d0) {
       for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       const int ex = split_exponent(m), r = lr + 32 * (u & 1);
       const float sc = split_scale(ex);
-      if (lc == 0) unit[LT * (u >> 1) + r] = pow2i(ex - SPLIT_TOP);
+      if (lc == 0) unit[LT * (u >> 1) + r] = m > 0.f ? pow2i(ex - SPLIT_TOP) : 0.f;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         uint2 h, l;
@@ -200,9 +214,15 @@ __global__ void __launch_bounds__(256, 2) linear_split_kernel(const LinDev d0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const float u0 = unit[wm + 16 * i + (lane >> 2)], u1 = unit[wm + 16 * i + 8 + (lane >> 2)];
+      top_a[i][0] = fmaxf(top_a[i][0], u0);
+      top_a[i][1] = fmaxf(top_a[i][1], u1);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float2 w = *reinterpret_cast<const float2*>(unit + LT + wn + 8 * j + 2 * (lane & 3));
+        if (i == 0) {
+          top_w[j][0] = fmaxf(top_w[j][0], w.x);
+          top_w[j][1] = fmaxf(top_w[j][1], w.y);
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[i][j][e] = fmaf(fmaf(z[i][j][e], LO_UNIT, y[i][j][e]) * (e < 2 ? u0 : u1), e & 1 ? w.y : w.x, acc[i][j][e]);
       }
@@ -215,9 +235,14 @@ __global__ void __launch_bounds__(256, 2) linear_split_kernel(const LinDev d0) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int m = m0 + wm + 16 * i + (lane >> 2) + 8 * (e >> 1), n = n0 + wn + 8 * j + 2 * (lane & 3) + (e & 1);
-        if (m >= d.M || n >= d.N) continue;
-        if (!(fabsf(acc[i][j][e]) < INFINITY)) acc[i][j][e] = lin_dot(static_cast<const float*>(d.A) + m * d.lda, static_cast<const float*>(d.W) + n * d.ldw, d.K);
-        lin_store(d, m, n, acc[i][j][e]);
+        const bool in = m < d.M && n < d.N;
+        const float y = fabsf(acc[i][j][e]);
+        for (unsigned again = __ballot_sync(0xffffffffu, in && !(y >= LS_SMALL * top_a[i][e >> 1] * top_w[j][e & 1] && y < INFINITY)); again; again &= again - 1) {
+          const int src = __ffs(again) - 1, ms = __shfl_sync(0xffffffffu, m, src), ns = __shfl_sync(0xffffffffu, n, src);
+          const float x = lin_dot(static_cast<const float*>(d.A) + ms * d.lda, static_cast<const float*>(d.W) + ns * d.ldw, d.K);
+          if (lane == src) acc[i][j][e] = x;
+        }
+        if (in) lin_store(d, m, n, acc[i][j][e]);
       }
 }
 
