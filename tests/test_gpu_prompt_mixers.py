@@ -219,6 +219,54 @@ def test_fp32_products_of_entries_far_below_their_row_s_largest(ratio):
     assert _err(ops.linear_plain(x, w), (x.double() @ w.double().T).cpu()) < BOUND
 
 
+def _wide_case(g, T, H, G, d, dv, bad, what):
+    """q, k, v of one sequence: one channel of one value row, or one channel of every key (and zeros there in the queries), far outside the others' range."""
+    q, k, v = (torch.randn(T, n, w, generator=g) / d ** (0.25 if i < 2 else 0) for i, (n, w) in enumerate(((H, d), (G, d), (G, dv))))
+    clean = v.clone()
+    if what == "value":
+        v[40, :, 5] = bad
+    elif what == "row":
+        v[40] *= bad
+    else:
+        k[:, :, 3] = bad
+        q[:, :, 3] = 0.0
+    return q, k, v, clean
+
+
+@pytest.mark.parametrize("form", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("window", [0, 20])
+@pytest.mark.parametrize("what,bad", [("value", 1e5), ("value", 1e9), ("value", float("inf")), ("value", float("nan")), ("row", 1e6), ("row", 1e12), ("key", 1e9), ("key", 1e15)])
+def test_prompt_attention_keeps_large_numbers_to_where_they_are_seen(form, window, what, bad):
+    """A value that a query does not see changes nothing for it, and one that it sees nothing in the other columns; large key channels that meet zeros
+    change nothing. (An infinity or NaN may reach its own column of the queries that share a tile with it: a weight of zero times it.)"""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(7)
+    T, H, G, d, dv, bs = 70, 4, 2, 64, 40, 16
+    q, k, v, clean = _wide_case(g, T, H, G, d, dv, bad, what)
+    back = torch.arange(T)[:, None] - torch.arange(T)[None, :]
+    seen = (back >= 0) & (back < window) if window else back >= 0
+    want = torch.empty(T, H, dv, dtype=torch.float64)
+    for h in range(H):
+        sc = q[:, h].double() @ k[:, h // 2].double().T
+        p = torch.softmax(sc.masked_fill(~seen, -torch.inf), 1) if form == "softmax" else torch.sigmoid(sc) * seen
+        for c in range(dv):   # a column of its own: infinity times zero stays out of the others
+            x = v[:, h // 2, c].double()
+            want[:, h, c] = p @ (x if bool(torch.isfinite(x).all()) else clean[:, h // 2, c].double())
+    batch, table, _, n_blocks, _ = shuffled_batch([T], [0], bs, DEV, seed=d)
+    kp, vp = torch.zeros(n_blocks, bs, G, d, device=DEV), torch.zeros(n_blocks, bs, G, dv, device=DEV)
+    for p in range(T):
+        kp[table[0][p // bs], p % bs], vp[table[0][p // bs], p % bs] = k[p].to(DEV), v[p].to(DEV)
+    got = ops.window_attn(batch, q.reshape(T, -1).to(DEV), kp, vp, heads=H, kv_heads=G, dim=d, vdim=dv, scale=1.0, window=window, keep_first=0, weights=form,
+                          out_dtype=torch.float32).view(T, H, dv).cpu()
+    sees = seen[:, 40]
+    other = torch.arange(dv) != 5
+    finite = bad == bad and abs(bad) < float("inf")
+    for rows in (sees, ~sees):
+        assert _err(got[rows][..., other], want[rows][..., other]) < BOUND
+        if finite:
+            assert _err(got[rows][..., 5], want[rows][..., 5]) < BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -952,7 +952,7 @@ extern "C" int vy_window_attn(const VyWinAttn* p) {
   VY_CHECK_ARG(p->dim <= 32 * WA_VR, "vy_window_attn: dim %d > %d", p->dim, 32 * WA_VR);
   if (p->max_new >= WA_TILED_MIN) {   // prompt-sized: tensor-core tiles
     int launches = 1;
-    VY_CUDA_OK(launch_window_attn_tiled(d, p->n_seqs, p->max_new, p->workspace, p->workspace_floats, st, &launches));
+    VY_CUDA_OK(launch_window_attn_prompt(d, p->n_seqs, p->max_new, p->workspace, p->workspace_floats, st, &launches));
     VY_LAUNCH_OK();
     count_launch(launches);
     return VY_OK;

@@ -173,11 +173,38 @@ struct SplitKv {
   unsigned char* rows;
   long long cap;   // key slots per (sequence, key / value head)
   int row_bytes;   // 4 (dim16 + vdim16) + 16
+  uint4* range;    // [sequence, key / value head][blocks]: of a block of SPLIT_ROWS rows the largest key entry, the largest value entry and the smallest of its value
+                   // rows' and columns' largest ones (zeros aside), as bits of floats
+  int blocks;
+  int* odd;        // [sequence, key / value head]: 1 where the keys or values are not for fp16 halves (split_odd) and the fp32 form has to do the work
 };
-// splits the rows that some query of the step sees into ws (window_attn_split_floats(..) floats, 16-byte aligned) and says where they are
+constexpr int SPLIT_ROWS = 32;
+// Are the values of list sg (all its visible rows) not for fp16 halves? A value row's halves are off by at most 2^-49 of its largest entry, and the weights' by as
+// much of the largest row's in the tile, seen or not (they carry the rows' exponents). With every row's and every column's largest within 2^20 of the
+// list's largest this stays below 2^-26 of what a column sums; rows or columns further apart, infinities and NaN are the fp32 form's. Read by a whole warp.
+constexpr float SPLIT_RANGE = 0x1p-20f;
+// Scores: a softmax or sigmoid takes a score's absolute error. With |q k scale| per channel up to 2^18 (units of q are 2^-13 of a row's largest or more) the
+// halves' share is below 2^-30 a channel; larger ones are the fp32 form's
+constexpr float SPLIT_SCORE = 0x1p5f;   // of units of q times largest entries of k
+__device__ __forceinline__ bool split_odd(const SplitKv& w, int sg, int keys, float& top_k) {
+  unsigned k = 0u, v = 0u, low = 0x7f800000u;
+  for (int b = threadIdx.x & 31; b < (keys + SPLIT_ROWS - 1) / SPLIT_ROWS; b += 32) {
+    const uint4 r = w.range[static_cast<long long>(sg) * w.blocks + b];
+    k = max(k, r.x);
+    v = max(v, r.y);
+    low = min(low, r.z);
+  }
+  top_k = __uint_as_float(__reduce_max_sync(0xffffffffu, k));
+  const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, v));
+  return !(top < INFINITY) || __uint_as_float(__reduce_min_sync(0xffffffffu, low)) < SPLIT_RANGE * top;
+}
+// splits the rows that some query of the step sees into ws (window_attn_split_floats(..) floats, 16-byte aligned), says where they are, sets `odd` to 0
 cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st);
-cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches);
-long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);   // the workspace it makes use of
+long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);
+// on the tensor cores, as many sequences at a time as the workspace holds; in fp32 where it holds none
+cudaError_t launch_window_attn_prompt(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches);
+// in fp32 (seqmix_tiled.cu); odd: null, or what the tensor-core form leaves to do
+cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, const int* odd, cudaStream_t st);
 // Single tokens whose query heads share key / value rows in groups of 8 or more (latent rows): heads as the rows of a tile.
 bool window_attn_heads_applies(const WinDev& d);
 long long window_attn_heads_workspace_floats(int n_seqs, int heads, int kv_heads, int vdim);

@@ -1,14 +1,16 @@
-// Linear attention with a fixed decay and the state-space recurrence, chunk by chunk, in fp32 on register tiles: the form for portions of up to 64
-// tokens, for heads of more than 128 channels and for calls without a workspace (linear_attn_mma.cu takes the other ones, all chunks at once):
+// Prompt-sized forms of two sequence mixers, in fp32 on register tiles: for what the tensor-core forms (linear_attn_mma.cu, window_attn_mma.cu) do not take.
 //
-//   * linear attention with a fixed decay, chunk by chunk: for a chunk of C tokens with the state S0 before it,
+//   * linear attention with a fixed decay, chunk by chunk (portions of up to 64 tokens, heads of more than 128 channels, calls without a workspace): for a chunk of C tokens with the state S0 before it,
 //       O = (Q K^T . D) V + diag(decay^(i+1)) Q S0,   D[i][j] = decay^(i-j) for j <= i, else 0
 //       S = decay^C S0 + sum_j decay^(C-1-j) k_j v_j^T
 //     one CTA owns (sequence, head, 64 value columns) and walks the chunks in order with its slice of S in shared memory.
 //     The state-space recurrence runs on the same kernel with a decay and a write strength per token: decay^(i-j) becomes
-//     exp(L_i - L_j) w_j with L the summed log decays of the chunk (kept as two floats: their differences are what counts).
+//     exp(L_i - L_j) w_j with L the summed log decays of the chunk (kept as two floats: their differences are what counts);
+//   * windowed softmax or sigmoid attention with kept first tokens and a sink over pages (calls without a workspace, and keys or values whose range the fp16
+//     halves of the other form do not cover): one CTA owns 64 queries of one head, walks the visible keys in tiles (the kept prefix first, then the
+//     window band) with an online softmax.
 //
-// It gives the same values as the token-serial kernels of seqmix.cu up to fp32 rounding, whatever the portion sizes.
+// Both give the same values as the token-serial kernels of seqmix.cu up to fp32 rounding, whatever the portion sizes.
 #include <stdlib.h>
 
 #include "seqmix.cuh"
@@ -302,6 +304,172 @@ cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st) {
   return launch_la_dp<256, true>(d, n_seqs, st);   // callers keep dim <= 256
 }
 
+// ---- tiled windowed attention --------------------------------------------------------------------------------------------
+constexpr int WT_M = 64;            // queries per CTA
+constexpr int WT_T = 256;           // threads: 16 x 16, each 4 query rows (ti + 16 r) by BN / 16 key columns (tj + 16 c)
+// BN: keys per tile. 64 halves the barriers per key; 32 lets two CTAs share an SM at 128-wide heads (the kernel is bound by
+// shared-memory and FMA latency with 8 warps, so a second CTA is what fills the issue slots)
+
+// SIG: sigmoid weights, written with the scores (no row statistics, one barrier less per key tile). odd: null, or where window_attn_mma_kernel left its word
+// per (sequence, key / value head): what it did is not done again
+template <int MV, int BN, bool SIG>
+__global__ void __launch_bounds__(WT_T, BN == 32 ? 2 : 1) window_attn_tiled_kernel(WinDev d, const int* odd, int ldq_s, int ldv_s, int dim4, int vdim4, bool qvec, bool kvvec) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int WT_N = BN, WT_LDP = BN + 4, NCB = BN / 16;
+  extern __shared__ __align__(16) float wt_smem[];
+  float* Qs = wt_smem;                       // [WT_M][ldq_s]
+  float* Ks = Qs + WT_M * ldq_s;             // [WT_N][ldq_s]
+  float* Vs = Ks + WT_N * ldq_s;             // [WT_N][ldv_s]
+  float* Ps = Vs + WT_N * ldv_s;             // [WT_M][WT_LDP]
+  float* corr_s = Ps + WT_M * WT_LDP;        // [WT_M]
+  float* l_s = corr_s + WT_M;                // [WT_M]
+  int* kpos_s = reinterpret_cast<int*>(l_s + WT_M);   // [WT_N] key position, -1 past the end
+  int* krow_s = kpos_s + WT_N;                        // [WT_N] its row in the pools
+  const int s = blockIdx.z, h = blockIdx.y;
+  const int t = threadIdx.x, ti = t >> 4, tj = t & 15, warp = t >> 5, lane = t & 31;
+  const int base = d.cu[s], n = d.cu[s + 1] - base;
+  const int g = h / (d.heads / d.kv_heads);
+  if (odd && !odd[s * d.kv_heads + g]) return;
+  for (int i0 = blockIdx.x * WT_M; i0 < n; i0 += gridDim.x * WT_M) {
+  __syncthreads();   // the readers of the previous queries are done
+  const int rows = min(WT_M, n - i0);
+  rows_to_smem<WT_T>(Qs, ldq_s, WT_M, d.dim, dim4, d.q, d.q_dt, qvec, VY_UACT_NONE,
+               [&](int i) { return i < rows ? static_cast<long long>(base + i0 + i) * d.ldq + static_cast<long long>(h) * d.dim : -1LL; });
+  const int p_lo = d.pos0[s] + i0, p_hi = p_lo + rows - 1;
+  // visible keys of the tile's queries: [0, nA) (kept first tokens outside the band) and [lo, p_hi] (the band); masks are per pair
+  const int lo = d.chunk > 0 ? p_lo / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p_lo - d.window + 1, 0);
+  const int nA = d.window <= 0 ? 0 : min(d.keep, lo);
+  const int count = nA + (p_hi - lo + 1);
+  const int* tab = d.table + static_cast<long long>(s) * d.tw;
+  float m[8], l[8];   // softmax statistics of rows 8 warp .. 8 warp + 7, the same in every lane
+#pragma unroll
+  for (int rr = 0; rr < 8; ++rr) {
+    m[rr] = d.sink ? ld_as_float(d.sink, d.sink_dt, h) : -INFINITY;
+    l[rr] = d.sink ? 1.f : 0.f;
+  }
+  float acc[4][MV][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int mm = 0; mm < MV; ++mm)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[r][mm][e] = 0.f;
+  const long long kstride = d.k_row, vstride = d.v_row;
+  const float sc_mul = head_scale_of(d, h), sc_add = head_bias_of(d, h);
+  const float slope = head_slope_of(d, h), two_over_cap = d.softcap > 0.f ? 2.f / d.softcap : 0.f;
+  for (int c0 = 0; c0 < count; c0 += WT_N) {
+    __syncthreads();
+    if (t < WT_N) {
+      const int c = c0 + t;
+      const int kp = c < count ? (c < nA ? c : lo + (c - nA)) : -1;
+      kpos_s[t] = kp;
+      krow_s[t] = kp >= 0 ? tab[kp / d.bs] * d.bs + kp % d.bs : 0;
+    }
+    __syncthreads();
+    rows_to_smem<WT_T>(Ks, ldq_s, WT_N, d.dim, dim4, d.kp, d.pool_dt, kvvec, VY_UACT_NONE,
+                 [&](int j) { return kpos_s[j] >= 0 ? static_cast<long long>(krow_s[j]) * kstride + static_cast<long long>(g) * d.dim : -1LL; });
+    rows_to_smem<WT_T>(Vs, ldv_s, WT_N, d.vdim, vdim4, d.vp, d.pool_dt, kvvec, VY_UACT_NONE,
+                 [&](int j) { return kpos_s[j] >= 0 ? static_cast<long long>(krow_s[j]) * vstride + static_cast<long long>(g) * d.vdim : -1LL; });
+    __syncthreads();
+    float sc[4][NCB];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < NCB; ++c) sc[r][c] = 0.f;
+#pragma unroll 2
+    for (int d4 = 0; d4 < dim4; d4 += 4) {
+      float4 kv[NCB];
+#pragma unroll
+      for (int c = 0; c < NCB; ++c) kv[c] = f4(Ks + (tj + 16 * c) * ldq_s + d4);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float4 qv = f4(Qs + (ti + 16 * r) * ldq_s + d4);
+#pragma unroll
+        for (int c = 0; c < NCB; ++c) sc[r][c] = dot4(qv, kv[c], sc[r][c]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < NCB; ++c) {
+        const int i = ti + 16 * r, j = tj + 16 * c;
+        const int p = p_lo + i, kp = kpos_s[j];
+        const bool vis = i < rows && kp >= 0 && kp <= p && (d.window <= 0 || p - kp < d.window || kp < d.keep) && (d.chunk <= 0 || kp >= p / d.chunk * d.chunk);
+        const float z = shaped_score(d, fmaf(sc[r][c], sc_mul, sc_add), two_over_cap, slope, p - kp);
+        if constexpr (SIG) Ps[i * WT_LDP + j] = vis ? sigmoidf_(z) : 0.f;
+        else Ps[i * WT_LDP + j] = vis ? z : -INFINITY;
+      }
+    __syncthreads();
+    if constexpr (!SIG) {
+#pragma unroll
+    for (int rr = 0; rr < 8; ++rr) {
+      float* pr = Ps + (8 * warp + rr) * WT_LDP;
+      const float a = pr[lane], b = BN == 64 ? pr[lane + 32] : -INFINITY;
+      const float mn = fmaxf(m[rr], warp_max(fmaxf(a, b)));
+      const float cr = mn == -INFINITY ? 1.f : expf(m[rr] - mn);
+      const float pa = a == -INFINITY ? 0.f : expf(a - mn), pb = b == -INFINITY ? 0.f : expf(b - mn);
+      pr[lane] = pa;
+      if (BN == 64) pr[lane + 32] = pb;
+      l[rr] = fmaf(l[rr], cr, warp_sum(pa + pb));
+      m[rr] = mn;
+      if (lane == 0) corr_s[8 * warp + rr] = cr;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float cr = corr_s[ti + 16 * r];
+#pragma unroll
+      for (int mm = 0; mm < MV; ++mm)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[r][mm][e] *= cr;
+    }
+    }
+    const int nv = min(WT_N, (count - c0 + 3) & ~3);
+    for (int j4 = 0; j4 < nv; j4 += 4) {
+      float4 pv[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) pv[r] = f4(Ps + (ti + 16 * r) * WT_LDP + j4);
+#pragma unroll
+      for (int mm = 0; mm < MV; ++mm) {
+        const int col = 4 * (tj + 16 * mm);
+        if (col < vdim4) {
+          const float4 x0 = f4(Vs + (j4 + 0) * ldv_s + col), x1 = f4(Vs + (j4 + 1) * ldv_s + col);
+          const float4 x2 = f4(Vs + (j4 + 2) * ldv_s + col), x3 = f4(Vs + (j4 + 3) * ldv_s + col);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            axpy4(acc[r][mm], pv[r].x, x0);
+            axpy4(acc[r][mm], pv[r].y, x1);
+            axpy4(acc[r][mm], pv[r].z, x2);
+            axpy4(acc[r][mm], pv[r].w, x3);
+          }
+        }
+      }
+    }
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int rr = 0; rr < 8; ++rr) l_s[8 * warp + rr] = l[rr];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = ti + 16 * r;
+    if (i >= rows) continue;
+    const long long qrow = base + i0 + i;
+    float og = SIG ? d.out_scale : d.out_scale / l_s[i];
+    if (d.gate) og *= sigmoidf_(ld_as_float(d.gate, d.gate_dt, qrow * d.ld_gate + h));
+#pragma unroll
+    for (int mm = 0; mm < MV; ++mm)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int col = 4 * (tj + 16 * mm) + e;
+        if (col < d.vdim) st_from_float(d.out, d.out_dt, qrow * d.ld_out + static_cast<long long>(h) * d.vdim + col, acc[r][mm][e] * og);
+      }
+  }
+  }
+}
+
 // ---- single tokens, many query heads per key / value head ---------------------------------------------------------------------
 // Latent rows (one key / value head for all query heads) and wide head groups: the heads of ONE token are the query rows of a tile.
 // A CTA owns (sequence, 16 heads of one key / value head, one split of the visible keys) and walks its keys 64 at a time: the key
@@ -554,6 +722,42 @@ cudaError_t launch_window_attn_heads(const WinDev& d, int n_seqs, float* ws, lon
   if (e != cudaSuccess || splits == 1) return e;
   *launches = 2;
   return launch_kernel(window_attn_heads_merge_kernel, dim3(d.heads, n_seqs), dim3(64), 0, st, d, static_cast<int>(splits), static_cast<const float*>(ws));
+}
+
+template <int MV, int BN, bool SIG>
+static cudaError_t launch_wt(const WinDev& d, int n_seqs, int max_new, const int* odd, cudaStream_t st) {
+  constexpr int WT_N = BN, WT_LDP = BN + 4;
+  const int dim4 = (d.dim + 3) & ~3, vdim4 = (d.vdim + 3) & ~3;
+  const int ldq_s = ((dim4 >> 2) & 1) ? dim4 + 8 : dim4 + 4;   // (row stride / 4) odd: rows 1 apart start in distinct 16-byte bank groups
+  const int ldv_s = vdim4 + 4;
+  const size_t smem = sizeof(float) * (static_cast<size_t>(WT_M + WT_N) * ldq_s + static_cast<size_t>(WT_N) * ldv_s + WT_M * WT_LDP + 2 * WT_M) +
+                      sizeof(int) * 2 * WT_N;
+  const auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q);
+  const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && d.k_row % 4 == 0 && d.v_row % 4 == 0 && al(d.kp) && al(d.vp);
+  static size_t allowed = 48 * 1024;
+  if (smem > allowed) {
+    cudaError_t e = cudaFuncSetAttribute(window_attn_tiled_kernel<MV, BN, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    allowed = smem;
+  }
+  // behind the tensor-core form mostly nothing is left to do: two CTAs per SM, which walk the blocks of queries, cost less to launch than one per block
+  const long long tiles = (max_new + WT_M - 1) / WT_M, most = (2LL * num_sms() + static_cast<long long>(d.heads) * n_seqs - 1) / (static_cast<long long>(d.heads) * n_seqs);
+  return launch_kernel(window_attn_tiled_kernel<MV, BN, SIG>, dim3(static_cast<unsigned>(odd && most < tiles ? most : tiles), d.heads, n_seqs), dim3(WT_T), smem, st, d, odd,
+                       ldq_s, ldv_s, dim4, vdim4, qvec, kvvec);
+}
+
+template <bool SIG>
+static cudaError_t launch_wt_any(const WinDev& d, int n_seqs, int max_new, const int* odd, cudaStream_t st) {
+  static const int bn_env = getenv("VY_WINDOW_ATTN_BN") ? atoi(getenv("VY_WINDOW_ATTN_BN")) : 0;   // development: 32 or 64
+  const bool narrow = bn_env ? bn_env == 32 : (d.dim > 64 || d.vdim > 64);   // wide heads: 64-key tiles would take the SM for one CTA
+  if (d.vdim <= 64) return narrow ? launch_wt<1, 32, SIG>(d, n_seqs, max_new, odd, st) : launch_wt<1, 64, SIG>(d, n_seqs, max_new, odd, st);
+  if (d.vdim <= 128) return narrow ? launch_wt<2, 32, SIG>(d, n_seqs, max_new, odd, st) : launch_wt<2, 64, SIG>(d, n_seqs, max_new, odd, st);
+  return launch_wt<4, 64, SIG>(d, n_seqs, max_new, odd, st);   // vdim <= 256 (checked by the caller): the accumulators leave no room for two CTAs
+}
+
+cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, const int* odd, cudaStream_t st) {
+  return d.sigmoid ? launch_wt_any<true>(d, n_seqs, max_new, odd, st) : launch_wt_any<false>(d, n_seqs, max_new, odd, st);
 }
 
 }  // namespace vy

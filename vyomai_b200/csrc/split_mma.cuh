@@ -85,13 +85,16 @@ static __device__ __noinline__ void store2_any(void* dst, int dt, long long at, 
 // Rows [0, rows) of a block of `src` as hi / lo planes (`row_bytes` between rows of a plane, columns zero-filled up to pad16, a
 // multiple of 16 and at most MAXD), with 2^(a row's exponent - drop) in unit[row * ustep]. Row j starts at element off(j) of src or is all zero when
 // off(j) < 0. Eight lanes share a row (coalesced 128-byte runs); a thread has the loads of U rows in flight before it uses any. vec: src
-// is fp32, row starts and the width are multiples of 4 elements. map: applied to every entry read (map(0) = 0).
+// is fp32, row starts and the width are multiples of 4 elements. map: applied to every entry read (map(0) = 0). seen: given each row's largest entry.
 struct SameValue {
   __device__ __forceinline__ float operator()(float x) const { return x; }
 };
-template <int NW, int MAXD, typename OffFn, typename MapFn = SameValue>
+struct NotSeen {
+  __device__ __forceinline__ void operator()(float) const {}
+};
+template <int NW, int MAXD, typename OffFn, typename MapFn = SameValue, typename SeenFn = NotSeen>
 __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo, int row_bytes, float* unit, int drop, int rows, int width, int pad16, const void* src, int dt,
-                                           bool vec, OffFn off, MapFn map = MapFn(), int ustep = 1) {
+                                           bool vec, OffFn off, MapFn map = MapFn(), int ustep = 1, SeenFn seen = SeenFn()) {
   constexpr int NI = (MAXD + 31) / 32, U = NI <= 4 ? 4 : 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
   for (int r0 = warp * 4 + (lane >> 3); r0 - (lane >> 3) < rows; r0 += NW * 4 * U) {
@@ -123,7 +126,10 @@ __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo,
       if (r < rows) {
         const int e = split_exponent(m);
         const float sc = split_scale(e);
-        if (l8 == 0) unit[r * ustep] = pow2i(e - drop);
+        if (l8 == 0) {
+          unit[r * ustep] = pow2i(e - drop);
+          seen(m);
+        }
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
           const int c = l8 * 4 + 32 * i;

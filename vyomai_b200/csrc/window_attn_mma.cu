@@ -29,7 +29,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                : "memory");
 }
 
-constexpr int WS_T = 256, WS_ROWS = WS_T / 8;   // splitting launch: eight lanes per row
+constexpr int WS_T = 8 * SPLIT_ROWS;   // splitting launch: eight lanes per row
 
 // bound by the bytes: every row read once and written once (8000 rows of 2 x (128 + 128) channels: 33 MB)
 template <int MAXD>
@@ -42,41 +42,64 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
   const int count = n > 0 ? nA + p0 + n - lo : 0;
   const int* tab = d.table + static_cast<long long>(s) * d.tw;
   const long long slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
-  const int r0 = blockIdx.x * WS_ROWS;
+  const int r0 = blockIdx.x * SPLIT_ROWS, sg = s * d.kv_heads + g;
+  if (blockIdx.x == 0 && threadIdx.x == 0) w.odd[sg] = 0;
   if (r0 >= count) return;
-  const int rows = min(WS_ROWS, count - r0);
+  __shared__ unsigned top_k, top_v, low_v;   // positive numbers order like their bits (and NaN after infinity)
+  __shared__ long long row_s[SPLIT_ROWS];
+  const int rows = min(SPLIT_ROWS, count - r0);
   const auto row_of = [&](int r) {
     const int kp = r0 + r < nA ? r0 + r : lo + (r0 + r - nA);
     return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
   };
+  if (threadIdx.x < rows) row_s[threadIdx.x] = row_of(threadIdx.x) * d.v_row + static_cast<long long>(g) * d.vdim;
+  if (threadIdx.x == 0) {
+    top_k = top_v = 0u;
+    low_v = 0x7f800000u;
+  }
+  __syncthreads();
   unsigned char* out = w.rows + (slot0 + r0) * w.row_bytes;
   float* unit = reinterpret_cast<float*>(out + 4 * (dim16 + vdim16));
   split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, unit, SPLIT_TOP, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
-                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; }, SameValue(), w.row_bytes / 4);
+                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; }, SameValue(), w.row_bytes / 4,
+                              [&](float m) { atomicMax(&top_k, __float_as_uint(m)); });
   out += 4 * dim16;
   split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, unit + 1, 0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
-                              [&](int r) { return row_of(r) * d.v_row + static_cast<long long>(g) * d.vdim; }, SameValue(), w.row_bytes / 4);
+                              [&](int r) { return row_s[r]; }, SameValue(), w.row_bytes / 4, [&](float m) {
+                                if (m > 0.f) atomicMin(&low_v, __float_as_uint(m));
+                              });
+  for (int c0 = 0; c0 < d.vdim; c0 += WS_T) {   // columns, from the L1 cache
+    const int c = c0 + threadIdx.x;
+    unsigned m = 0u;
+    if (c < d.vdim) {
+#pragma unroll 8
+      for (int r = 0; r < rows; ++r) m = max(m, __float_as_uint(fabsf(ld_as_float(d.vp, d.pool_dt, row_s[r] + c))));
+    }
+    const unsigned top = __reduce_max_sync(0xffffffffu, m), low = __reduce_min_sync(0xffffffffu, m && rows >= 8 ? m : 0x7f800000u);   // of fewer rows the largest may be small by chance
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&top_v, top);
+      atomicMin(&low_v, low);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) w.range[static_cast<long long>(sg) * w.blocks + blockIdx.x] = make_uint4(top_k, top_v, low_v, 0u);
 }
 
-// MAXD: most query / key channels; VT: value channels the accumulators hold; NW: warps (16 rows each); N: keys per tile; NS: tile buffers; PRE: rows
-// come split from the workspace, else the CTA splits them itself (one buffer); SIG: sigmoid weights
-template <int MAXD, int VT, int NW, int N, int NS, bool PRE, bool SIG>
-__global__ void __launch_bounds__(32 * NW, NW == 4 && VT <= 128 && !PRE ? 2 : 1)
-window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16, int vdim16, bool qvec, bool kvvec, bool ovec) {
+// MAXD: most query / key channels; VT: value channels the accumulators hold; NW: warps (16 rows each); N: keys per tile; NS: tile buffers; SIG: sigmoid weights
+template <int MAXD, int VT, int NW, int N, int NS, bool SIG>
+__global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16, int vdim16, bool qvec, bool ovec) {
   pdl_trigger();
   pdl_wait();
   constexpr int R = 16 * NW, NT = N / 8, KT = N / 16;   // rows of a CTA; the tile's keys as score columns of 8 and value steps of 16
   constexpr int NC = VT / 32;   // value columns go in blocks of 32
   extern __shared__ __align__(16) unsigned char wm_smem[];
   // bytes between rows (odd multiples of 16: ldmatrix without bank conflicts), from a hi entry to its lo entry, to the values, of a tile buffer
-  const int qb = dim16 * 2 + 16, kb = PRE ? w.row_bytes : qb, vb = PRE ? w.row_bytes : vdim16 * 2 + 16;
-  const int k_lo = PRE ? 2 * dim16 : N * kb, v_lo = PRE ? 2 * vdim16 : N * vb, v_at = 2 * k_lo, buf = PRE ? N * kb : 2 * N * (kb + vb);
+  const int qb = dim16 * 2 + 16, kb = w.row_bytes, k_lo = 2 * dim16, v_lo = 2 * vdim16, v_at = 2 * k_lo, buf = N * kb;
   unsigned char* Qh = wm_smem;
-  unsigned char* Ts = Qh + 2 * R * qb;     // [buffers]: rows of the workspace, or K hi | K lo | V hi | V lo
-  float* qe = reinterpret_cast<float*>(Ts + NS * buf);   // powers of two that undo the scaling of the rows of Q, then (!PRE) [K | V]
-  float* te = qe + R;
-  uint64_t* full = reinterpret_cast<uint64_t*>(te + (PRE ? 0 : 2 * N));   // PRE: a buffer's tile has arrived
-  int* done = reinterpret_cast<int*>(full + NS);                     // PRE: warps that are through with a buffer, counted up for ever
+  unsigned char* Ts = Qh + 2 * R * qb;     // [buffers]: rows of the workspace
+  float* qe = reinterpret_cast<float*>(Ts + NS * buf);   // powers of two that undo the scaling of the rows of Q
+  uint64_t* full = reinterpret_cast<uint64_t*>(qe + R);  // a buffer's tile has arrived
+  int* done = reinterpret_cast<int*>(full + NS);         // warps that are through with a buffer, counted up for ever
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int s = blockIdx.z, h0 = blockIdx.y << hl, qn = R >> hl;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
@@ -90,55 +113,33 @@ window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16,
   int nA, lo;
   portion_keys(d, p_lo, nA, lo);
   const int count = nA + (p_hi - lo + 1);
-  int nA0 = 0, lo0 = 0;   // the same of the portion: where the workspace keeps a key
-  long long slot0 = 0;
-  if constexpr (PRE) {
-    portion_keys(d, p0, nA0, lo0);
-    slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
-  }
-  const int* tab = d.table + static_cast<long long>(s) * d.tw;
+  int nA0, lo0;   // the same of the portion: where the workspace keeps a key
+  portion_keys(d, p0, nA0, lo0);
+  const long long slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
   const auto key_of = [&](int c) { return c < nA ? c : lo + (c - nA); };
-  const auto fetch = [&](int c0, int b) {   // tile of keys c0 .. into buffer b, its exponents beside it
+  const auto fetch = [&](int c0, int b) {   // tile of keys c0 .. into buffer b, by one warp: runs of neighbouring slots, one copy each; rows past the end are zeros
     unsigned char* T = Ts + b * buf;
-    if constexpr (PRE) {   // by one warp: runs of neighbouring slots, one copy each; rows past the end are zeros
-      const int nk = min(N, count - c0);
-      for (int x = lane; x < (N - nk) * (kb / 16); x += 32) *reinterpret_cast<uint4*>(T + nk * kb + 16 * x) = make_uint4(0, 0, 0, 0);
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&full[b], static_cast<unsigned>(nk) * w.row_bytes);
-        for (int j = 0; j < nk;) {   // kept tokens and the band are a run each; kept tokens beyond the portion's own lie at the band's start
-          const int c = c0 + j, kp = key_of(c);
-          const int run = min(nk - j, c >= nA ? nk : (kp < nA0 ? nA0 - c : nA - c));
-          bulk_load(T + j * kb, w.rows + (slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)) * w.row_bytes, static_cast<unsigned>(run) * w.row_bytes, &full[b]);
-          j += run;
-        }
+    const int nk = min(N, count - c0);
+    for (int x = lane; x < (N - nk) * (kb / 16); x += 32) *reinterpret_cast<uint4*>(T + nk * kb + 16 * x) = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive_expect_tx(&full[b], static_cast<unsigned>(nk) * w.row_bytes);
+      for (int j = 0; j < nk;) {   // kept tokens and the band are a run each; kept tokens beyond the portion's own lie at the band's start
+        const int c = c0 + j, kp = key_of(c);
+        const int run = min(nk - j, c >= nA ? nk : (kp < nA0 ? nA0 - c : nA - c));
+        bulk_load(T + j * kb, w.rows + (slot0 + (kp >= lo0 ? nA0 + kp - lo0 : kp)) * w.row_bytes, static_cast<unsigned>(run) * w.row_bytes, &full[b]);
+        j += run;
       }
-    } else {
-      const auto row_of = [&](int j) {
-        if (c0 + j >= count) return -1LL;
-        const int kp = key_of(c0 + j);
-        return static_cast<long long>(tab[kp / d.bs] * d.bs + kp % d.bs);
-      };
-      split_rows<NW, MAXD>(T, T + k_lo, kb, te, SPLIT_TOP, N, d.dim, dim16, d.kp, d.pool_dt, kvvec, [&](int j) {
-        const long long r = row_of(j);
-        return r >= 0 ? r * d.k_row + static_cast<long long>(g) * d.dim : -1LL;
-      });
-      split_rows<NW, VT>(T + v_at, T + v_at + v_lo, vb, te + N, 0, N, d.vdim, vdim16, d.vp, d.pool_dt, kvvec, [&](int j) {
-        const long long r = row_of(j);
-        return r >= 0 ? r * d.v_row + static_cast<long long>(g) * d.vdim : -1LL;
-      });
     }
   };
   const int tiles = (count + N - 1) / N;
-  if constexpr (PRE) {
-    if (threadIdx.x < NS) {
-      mbar_init(&full[threadIdx.x], 1);
-      done[threadIdx.x] = 0;
-    }
-    fence_mbar_init();
-    __syncthreads();
-    if (warp < min(NS, tiles)) fetch(warp * N, warp);
+  if (threadIdx.x < NS) {
+    mbar_init(&full[threadIdx.x], 1);
+    done[threadIdx.x] = 0;
   }
+  fence_mbar_init();
+  __syncthreads();
+  if (warp < min(NS, tiles)) fetch(warp * N, warp);
   split_rows<NW, MAXD>(Qh, Qh + R * qb, qb, qe, SPLIT_TOP, R, d.dim, dim16, d.q, d.q_dt, qvec, [&](int r) {
     return (r >> hl) < nq ? static_cast<long long>(base + i0 + (r >> hl)) * d.ldq + static_cast<long long>(h0 + (r & hm)) * d.dim : -1LL;
   });
@@ -163,26 +164,30 @@ window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16,
     for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
   int E = SPLIT_MIN_E;   // the outputs are kept in units of 2^(E - 2 SPLIT_TOP), E the largest exponent of a value row so far
   const unsigned qa_h = smem_addr(Qh) + 16 * warp * qb + lane_a(lane, qb), qa_l = qa_h + R * qb;
-  const unsigned kb_0 = smem_addr(Ts) + lane_b(lane, kb), vb_0 = smem_addr(Ts) + v_at + lane_bt(lane, vb);
-  if constexpr (PRE) __syncthreads();   // Q is there; from here on the warps wait for tiles, not for one another, so that one's softmax meets another's products
+  const unsigned kb_0 = smem_addr(Ts) + lane_b(lane, kb), vb_0 = smem_addr(Ts) + v_at + lane_bt(lane, kb);
+  float top_k;
+  const bool odd = split_odd(w, s * d.kv_heads + g, nA0 + p0 + n - lo0, top_k);
+  __syncthreads();   // Q is there
+  bool big = false;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    qmul[e] *= qe[16 * warp + gq + 8 * e];
+    big = big || !(fabsf(qmul[e]) * top_k <= SPLIT_SCORE);
+  }
+  if (__syncthreads_or(odd || big)) {   // not for fp16 halves: the fp32 form's
+    for (int b = 0; b < min(NS, tiles); ++b) mbar_wait_soft(&full[b], 0, poison);   // the copies in flight write to this CTA's memory
+    if (threadIdx.x == 0) w.odd[s * d.kv_heads + g] = 1;
+    return;
+  }
+  // from here on the warps wait for tiles, not for one another, so that one's softmax meets another's products
   for (int it = 0; it < tiles; ++it) {
     const int c0 = it * N, b = it % NS;
-    if constexpr (PRE) {
-      mbar_wait_soft(&full[b], (it / NS) & 1, poison);
-    } else {
-      if (c0) __syncthreads();
-      fetch(c0, 0);
-      __syncthreads();
-    }
-    if (c0 == 0) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) qmul[e] *= qe[16 * warp + gq + 8 * e];
-    }
+    mbar_wait_soft(&full[b], (it / NS) & 1, poison);
     const unsigned kb_h = kb_0 + b * buf, vb_h = vb_0 + b * buf;
     // 2^(exponent - SPLIT_TOP) of each key row, 2^exponent of each value row
-    const int ustep = PRE ? w.row_bytes / 4 : 1;
-    const float* ke = PRE ? reinterpret_cast<const float*>(Ts + b * buf + 4 * (dim16 + vdim16)) : te;
-    const float* ve = PRE ? ke + 1 : te + N;
+    const int ustep = kb / 4;
+    const float* ke = reinterpret_cast<const float*>(Ts + b * buf + 4 * (dim16 + vdim16));
+    const float* ve = ke + 1;
     // ---- scores ----
     float sc[NT][4], x[NT][4];   // hi hi, and the two small products
 #pragma unroll
@@ -296,8 +301,8 @@ window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16,
         for (int i = 0; i < 2; ++i) {
           if (32 * cc + 16 * i < vdim16) {
             unsigned bh[4], bl[4];
-            ldsm_x4_t(bh, vb_h + 16 * k * vb + (32 * cc + 16 * i) * 2);
-            ldsm_x4_t(bl, vb_h + v_lo + 16 * k * vb + (32 * cc + 16 * i) * 2);
+            ldsm_x4_t(bh, vb_h + 16 * k * kb + (32 * cc + 16 * i) * 2);
+            ldsm_x4_t(bl, vb_h + v_lo + 16 * k * kb + (32 * cc + 16 * i) * 2);
             mma_f16(z[2 * i], pl[k], bh[0], bh[1]);
             mma_f16(z[2 * i + 1], pl[k], bh[2], bh[3]);
             mma_f16(y[2 * i], ph[k], bh[0], bh[1]);
@@ -312,16 +317,15 @@ window_attn_mma_kernel(WinDev d, SplitKv w, PoisonRef poison, int hl, int dim16,
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[4 * cc + i][e] = fmaf(o[4 * cc + i][e], keep_o[e >> 1], fmaf(z[i][e], LO_UNIT, y[i][e]));
     }
-    if constexpr (PRE) {   // the warp that is through with a buffer last refills it
-      __syncwarp();
-      int last = 0;
-      if (lane == 0) {
-        __threadfence_block();
-        last = atomicAdd(&done[b], 1) % NW == NW - 1;
-        __threadfence_block();
-      }
-      if (__shfl_sync(0xffffffffu, last, 0) && it + NS < tiles) fetch((it + NS) * N, b);
+    // the warp that is through with a buffer last refills it
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) {
+      __threadfence_block();
+      last = atomicAdd(&done[b], 1) % NW == NW - 1;
+      __threadfence_block();
     }
+    if (__shfl_sync(0xffffffffu, last, 0) && it + NS < tiles) fetch((it + NS) * N, b);
   }
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -361,8 +365,11 @@ static long long split_slots(const WinDev& d, int max_new) {
   return seen < all ? seen : all;
 }
 
+static long long split_blocks(const WinDev& d, int max_new) { return (split_slots(d, max_new) + SPLIT_ROWS - 1) / SPLIT_ROWS; }
+
+// rows, ranges of blocks, and `odd` (in fours: whole 16 bytes)
 long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new) {
-  return static_cast<long long>(n_seqs) * d.kv_heads * split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 4);
+  return static_cast<long long>(n_seqs) * d.kv_heads * (split_slots(d, max_new) * (round16(d.dim) + round16(d.vdim) + 4) + 4 * split_blocks(d, max_new) + 4);
 }
 
 static bool kv_quads(const WinDev& d) {
@@ -374,40 +381,42 @@ cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, f
   const int dim16 = round16(d.dim), vdim16 = round16(d.vdim), big = d.dim > d.vdim ? d.dim : d.vdim;
   w->cap = split_slots(d, max_new);
   w->row_bytes = 4 * (dim16 + vdim16) + 16;
+  w->blocks = static_cast<int>(split_blocks(d, max_new));
+  const long long lists = static_cast<long long>(n_seqs) * d.kv_heads;
   w->rows = reinterpret_cast<unsigned char*>(ws);
-  const dim3 grid(static_cast<unsigned>((w->cap + WS_ROWS - 1) / WS_ROWS), d.kv_heads, n_seqs);
+  w->range = reinterpret_cast<uint4*>(w->rows + lists * w->cap * w->row_bytes);
+  w->odd = reinterpret_cast<int*>(w->range + lists * w->blocks);
+  const dim3 grid(w->blocks, d.kv_heads, n_seqs);
   return big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d))
                     : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d));
 }
 
-template <int MAXD, int VT, int NW, int N, int NS, bool PRE, bool SIG>
-static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, cudaStream_t st) {
+template <int MAXD, int VT, int NW, int N, int NS, bool SIG>
+static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, cudaStream_t st) {
   constexpr int R = 16 * NW;
   const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
-  const size_t kb = dim16 * 2 + 16, vb = vdim16 * 2 + 16, bufs = NS;
-  const size_t smem = 2 * R * kb + (PRE ? bufs * N * (2 * (kb + vb) - 48) : 2 * N * (kb + vb)) + sizeof(float) * (R + (PRE ? 0 : 2 * N)) + 12 * NS;
+  const size_t smem = 2 * R * (dim16 * 2 + 16) + static_cast<size_t>(NS) * N * w.row_bytes + sizeof(float) * R + 12 * NS;
   const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q, 16);
   const bool ovec = d.vdim % 2 == 0 && d.ld_out % 2 == 0 && al(d.out, d.out_dt == VY_BF16 ? 4 : 8);
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, N, NS, PRE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, N, NS, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
   PoisonRef poison = {};
-  if (PRE && !poison_ref(&poison)) return cudaErrorMemoryAllocation;
+  if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
   const int qn = R >> hl;
-  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, N, NS, PRE, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, poison, hl,
-                       dim16, vdim16, qvec, kvvec, ovec);
+  return launch_kernel(window_attn_mma_kernel<MAXD, VT, NW, N, NS, SIG>, dim3((max_new + qn - 1) / qn, d.heads >> hl, n_seqs), dim3(32 * NW), smem, st, d, w, poison, hl,
+                       dim16, vdim16, qvec, ovec);
 }
 
 template <int MAXD, int VT>
-static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, bool kvvec, bool pre, cudaStream_t st) {
+static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, cudaStream_t st) {
   const auto go = [&](auto sig) {
     constexpr bool S = decltype(sig)::value;
-    constexpr int N_OWN = MAXD <= 128 ? 64 : 32, N = VT <= 64 ? 64 : 32;
-    if (!pre) return launch_wm<MAXD, VT, 4, N_OWN, 1, false, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    constexpr int N = VT <= 64 ? 64 : 32;
     // CTAs of 64 rows, two per SM (key tiles as wide as that allows), so that one's softmax runs beside the other's products; wide values on
     // long prompts take one CTA of 192 rows with three warps per scheduler instead, where that still is two rounds of CTAs over the SMs.
     // 8 heads of 128 over 2, 4 x 2048 tokens, window 512, capped / sigmoid: 192 rows 235 / 237 us, 64 rows 240 / 262 us, 128 rows 236 / 270 us;
@@ -415,31 +424,42 @@ static cudaError_t launch_wm_pick(const WinDev& d, const SplitKv& w, int n_seqs,
     if constexpr (VT == 128) {
       const int qn = 192 >> hl;
       if (static_cast<long long>((max_new + qn - 1) / qn) * (d.heads >> hl) * n_seqs >= 2 * num_sms())
-        return launch_wm<MAXD, VT, 12, 32, 3, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+        return launch_wm<MAXD, VT, 12, 32, 3, S>(d, w, n_seqs, max_new, hl, st);
     }
-    return launch_wm<MAXD, VT, 4, N, 2, true, S>(d, w, n_seqs, max_new, hl, kvvec, st);
+    return launch_wm<MAXD, VT, 4, N, 2, S>(d, w, n_seqs, max_new, hl, st);
   };
   return d.sigmoid ? go(std::true_type{}) : go(std::false_type{});
 }
 
-cudaError_t launch_window_attn_tiled(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches) {
-  const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
-  const bool kvvec = kv_quads(d);
+static cudaError_t launch_window_attn_mma(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, cudaStream_t st) {
   // heads per tile: the largest power of two, at most 16, that divides the heads of a key / value head
   const int rep = d.heads / d.kv_heads;
   int hl = 0;
   while (hl < 4 && rep % (2 << hl) == 0) ++hl;
-  SplitKv w = {};
-  const bool pre = ws && al(ws, 16) && d.kv_heads <= 65535 && ws_floats >= window_attn_split_floats(d, n_seqs, max_new);
+  if (d.vdim > 128 || d.dim > 128) return launch_wm_pick<256, 256>(d, w, n_seqs, max_new, hl, st);   // callers keep both <= 256
+  if (d.vdim > 64) return launch_wm_pick<128, 128>(d, w, n_seqs, max_new, hl, st);
+  return d.dim <= 64 ? launch_wm_pick<64, 64>(d, w, n_seqs, max_new, hl, st) : launch_wm_pick<128, 64>(d, w, n_seqs, max_new, hl, st);
+}
+
+cudaError_t launch_window_attn_prompt(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches) {
   *launches = 1;
-  if (pre) {
-    cudaError_t e = launch_window_attn_split(d, n_seqs, max_new, ws, &w, st);
-    if (e != cudaSuccess) return e;
-    *launches = 2;
+  const long long fit = ws && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && d.kv_heads <= 65535 ? ws_floats / window_attn_split_floats(d, 1, max_new) : 0;
+  if (fit < 1) return launch_window_attn_tiled(d, n_seqs, max_new, nullptr, st);
+  *launches = 0;
+  for (int s = 0; s < n_seqs; s += static_cast<int>(fit < n_seqs ? fit : n_seqs)) {   // as many sequences at a time as the workspace holds
+    const int ns = static_cast<int>(fit < n_seqs - s ? fit : n_seqs - s);
+    WinDev e = d;
+    e.cu += s;
+    e.pos0 += s;
+    e.table += static_cast<long long>(s) * d.tw;
+    SplitKv w = {};
+    cudaError_t err = launch_window_attn_split(e, ns, max_new, ws, &w, st);
+    if (err == cudaSuccess) err = launch_window_attn_mma(e, w, ns, max_new, st);
+    if (err == cudaSuccess) err = launch_window_attn_tiled(e, ns, max_new, w.odd, st);
+    if (err != cudaSuccess) return err;
+    *launches += 3;
   }
-  if (d.vdim > 128 || d.dim > 128) return launch_wm_pick<256, 256>(d, w, n_seqs, max_new, hl, kvvec, pre, st);   // callers keep both <= 256
-  if (d.vdim > 64) return launch_wm_pick<128, 128>(d, w, n_seqs, max_new, hl, kvvec, pre, st);
-  return d.dim <= 64 ? launch_wm_pick<64, 64>(d, w, n_seqs, max_new, hl, kvvec, pre, st) : launch_wm_pick<128, 64>(d, w, n_seqs, max_new, hl, kvvec, pre, st);
+  return cudaSuccess;
 }
 
 }  // namespace vy
