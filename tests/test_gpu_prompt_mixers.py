@@ -267,6 +267,36 @@ def test_prompt_attention_keeps_large_numbers_to_where_they_are_seen(form, windo
             assert _err(got[rows][..., 5], want[rows][..., 5]) < BOUND
 
 
+@pytest.mark.parametrize("window", [0, 20])
+@pytest.mark.parametrize("what,bad", [("value", 1e5), ("value", 1e9), ("value", float("inf")), ("value", float("nan")), ("row", 1e12), ("key", 1e9), ("talk", 1e9)])
+def test_score_exchanging_prompts_keep_large_numbers_to_where_they_are_seen(window, what, bad):
+    """As above. "talk": an exchange weight that meets a head whose scores are all zero."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(8)
+    T, H, G, d, dv, bs = 70, 8, 2, 32, 24, 16
+    q, k, v, clean = _wide_case(g, T, H, G, d, dv, bad, what)
+    talk = torch.eye(H) + 0.3 * torch.randn(H, H, generator=g) / H ** 0.5
+    if what == "talk":
+        q[:, 6] = 0.0
+        talk[:, 6] = bad
+    back = torch.arange(T)[:, None] - torch.arange(T)[None, :]
+    seen = (back >= 0) & (back < window) if window else back >= 0
+    p = OV.plus_one_softmax(OV.mix_heads(OV.capped(torch.stack([q[:, a].double() @ k[:, a // 4].double().T for a in range(H)]) * 0.3, 9.0), talk.double()), seen)
+    x = torch.where(torch.isfinite(v), v, clean).double()
+    want = torch.stack([p[a] @ x[:, a // 4] for a in range(H)], 1)
+    batch, table, _, n_blocks, _ = shuffled_batch([T], [0], bs, DEV, seed=H)
+    kp, vp = torch.zeros(n_blocks, bs, G, d, device=DEV), torch.zeros(n_blocks, bs, G, dv, device=DEV)
+    for t in range(T):
+        kp[table[0][t // bs], t % bs], vp[table[0][t // bs], t % bs] = k[t].to(DEV), v[t].to(DEV)
+    got = ops.talk_attn(batch, q.reshape(T, -1).to(DEV), kp, vp, heads=H, kv_heads=G, dim=d, vdim=dv, scale=0.3, softcap=9.0, talk=talk.to(DEV), zero_sink=True,
+                        window=window).view(T, H, dv).cpu()
+    other = torch.arange(dv) != 5
+    for rows in (seen[:, 40], ~seen[:, 40]):
+        assert _err(got[rows][..., other], want[rows][..., other]) < 4 * BOUND
+        if bad == bad and abs(bad) < float("inf"):
+            assert _err(got[rows][..., 5], want[rows][..., 5]) < 4 * BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -14,6 +14,7 @@ struct TalkDev {
   const void* sink; int sink_dt; int zero_sink;
   const void* gate; long long ld_gate; int gate_dt; int gate_ch;
   void* out; long long ld_out; int out_dt;
+  const int* odd;   // null, or [sequence][key / value head]: sequences without a 1 are done (by talk_attn_mma_kernel)
 };
 
 // the extra softmax term of head h as (score, present)
@@ -30,6 +31,6 @@ __device__ __forceinline__ float gate_of(const TalkDev& d, long long row, int h,
 
 // Prompts on the tensor cores (talk_attn_mma.cu), given talk_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this geometry); two launches
 long long talk_attn_mma_floats(const TalkDev& d, int n_seqs, int max_new);
-cudaError_t launch_talk_attn_mma(const TalkDev& d, int n_seqs, int max_new, float* ws, cudaStream_t st);
+cudaError_t launch_talk_attn_mma(const TalkDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st);   // odd: what the fp32 tiles have to do
 
 }  // namespace vy

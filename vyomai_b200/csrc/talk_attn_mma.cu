@@ -17,6 +17,9 @@
 namespace vy {
 
 constexpr int TM_T = 512, TM_W = 16, TM_R = 256;
+// As SPLIT_SCORE (seqmix.cuh), for scores that are mixed: |q k scale| per channel, and an exchange weight times the largest score. A tile's scores share one scale,
+// so a mixed score is off by 2^-48 of TM_MIXED per head at most
+constexpr float TM_SCORE = 0x1p14f, TM_MIXED = 0x1p20f;
 
 // sizes in bytes or elements that the kernel and its launcher share
 template <int HL, int N>
@@ -81,6 +84,7 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
     return i < nq ? static_cast<long long>(base + i0 + i) * d.ldq + static_cast<long long>(h) * d.dim : -1LL;
   });
   // talk: two lanes' worth of loads per row would not pay: a thread scales and splits a row
+  bool odd = false;   // numbers that are not for fp16 halves (seqmix.cuh): the fp32 tiles' sequence
   if (t < 16 * MT) {
     float x[16 * MT], m = 0.f;
 #pragma unroll
@@ -90,6 +94,7 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
     }
     const int e = split_exponent(m);
     tu[t] = pow2i(e - SPLIT_TOP);
+    odd = !(m * (d.softcap > 0.f ? fminf(d.softcap, TM_SCORE) : TM_SCORE) <= TM_MIXED);
 #pragma unroll
     for (int b = 0; b < 16 * MT; b += 2) {
       unsigned h, l;
@@ -100,6 +105,16 @@ __global__ void __launch_bounds__(TM_T, 1) talk_attn_mma_kernel(TalkDev d, Split
   }
   if (t < 4) reinterpret_cast<unsigned*>(zero)[t] = 0u;
   const int rw = 16 * warp, hw = rw / TQ, g = hw / per;   // this warp's rows; they all read key / value head g
+  float top_k;
+  odd = split_odd(w, s * G + g, p0 + n - lo0, top_k) || odd;
+  __syncthreads();   // qu
+#pragma unroll
+  for (int e = 0; e < 2; ++e) odd = odd || !(fabsf(qu[rw + gq + 8 * e] * d.scale) * top_k <= TM_SCORE * 0x1p-13f);
+  if (__syncthreads_or(odd)) {
+    cp_async_wait<0>();
+    if (t == 0) w.odd[s * G] = 1;
+    return;
+  }
   const float two_over_cap = d.softcap > 0.f ? 2.f / d.softcap : 0.f;
   float m[2], l[2];
   int pos[2], hr[2], qr[2];
@@ -381,10 +396,11 @@ static cudaError_t launch_talk_mma(const TalkDev& d, const SplitKv& w, int n_seq
                        qvec, ovec);
 }
 
-cudaError_t launch_talk_attn_mma(const TalkDev& d, int n_seqs, int max_new, float* ws, cudaStream_t st) {
+cudaError_t launch_talk_attn_mma(const TalkDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st) {
   SplitKv w;
   cudaError_t e = launch_window_attn_split(talk_keys(d), n_seqs, max_new, ws, &w, st);
   if (e != cudaSuccess) return e;
+  *odd = w.odd;
   const int N = talk_mma_keys(d);
   if (d.heads == 8) return launch_talk_mma<3, 32>(d, w, n_seqs, max_new, st);
   if (d.heads == 16) return N == 32 ? launch_talk_mma<4, 32>(d, w, n_seqs, max_new, st) : launch_talk_mma<4, 16>(d, w, n_seqs, max_new, st);

@@ -291,7 +291,7 @@ talk_attn_tiled_kernel(TalkDev d, int TQ, int dim4, int vdim4, int ldq_s, int ld
   const int s = blockIdx.y, i0 = blockIdx.x * TQ;
   const int t = threadIdx.x, ti = t >> 4, tj = t & 15, warp = t >> 5, lane = t & 31;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (i0 >= n) return;
+  if (i0 >= n || (d.odd && !d.odd[s * G])) return;
   const int nq = min(TQ, n - i0);
   const int rows = H * TQ;   // <= R
   rows_to_smem<TT_T>(Q_s, ldq_s, R, d.dim, dim4, d.q, d.q_dt, qvec, VY_UACT_NONE, [&](int r) {
@@ -582,7 +582,7 @@ extern "C" int64_t vy_talk_attn_prompt_floats(int32_t n_seqs, int32_t max_new, i
   if (n_seqs <= 0 || max_new < TALK_MMA_MIN || table_width <= 0 || block_size <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || dim <= 0 || vdim <= 0) return 0;
   vy::TalkDev d = {};
   d.tw = table_width; d.bs = block_size; d.heads = heads; d.kv_heads = kv_heads; d.dim = dim; d.vdim = vdim; d.window = window;
-  return vy::talk_attn_mma_floats(d, n_seqs, max_new);
+  return vy::tiled_plan(d, (dim + 3) & ~3, (vdim + 3) & ~3).ok ? vy::talk_attn_mma_floats(d, n_seqs, max_new) : 0;
 }
 
 extern "C" int vy_talk_attn(const VyTalkAttn* p) {
@@ -596,7 +596,7 @@ extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   VY_CHECK_ARG(p->q && p->k_pool && p->v_pool && p->out && dtype_ok(p->q_dtype) && dtype_ok(p->pool_dtype) && dtype_ok(p->out_dtype) &&
                    (!p->talk || dtype_ok(p->talk_dtype)) && (!p->sink || dtype_ok(p->sink_dtype)) && (!p->gate || dtype_ok(p->gate_dtype)),
                "vy_talk_attn: bad tensors");
-  TalkDev d;
+  TalkDev d = {};
   d.cu = p->cu_tokens; d.pos0 = p->pos0; d.table = p->block_table; d.tw = p->table_width; d.bs = p->block_size;
   d.q = p->q; d.ldq = p->ldq; d.q_dt = p->q_dtype;
   d.kp = p->k_pool; d.vp = p->v_pool; d.pool_dt = p->pool_dtype;
@@ -612,14 +612,13 @@ extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q);
   const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && al(d.kp) && al(d.vp);
   const TiledPlan pl = tiled_plan(d, dim4, vdim4);
-  // prompts: the tensor-core form where the geometry suits it and the scratch is lent (16 tokens fill its 16-row products)
-  if (p->max_new >= TALK_MMA_MIN && p->force_form != 1 && p->workspace && al(p->workspace)) {
+  // prompts: the tensor-core form where the geometry suits it and the scratch is lent (16 tokens fill its 16-row products), the tiles behind it for what it leaves
+  if (p->max_new >= TALK_MMA_MIN && p->force_form != 1 && pl.ok && p->workspace && al(p->workspace)) {
     const long long need = talk_attn_mma_floats(d, p->n_seqs, p->max_new);
     if (need > 0 && p->workspace_floats >= need) {
-      VY_CUDA_OK(launch_talk_attn_mma(d, p->n_seqs, p->max_new, p->workspace, st));
+      VY_CUDA_OK(launch_talk_attn_mma(d, p->n_seqs, p->max_new, p->workspace, &d.odd, st));
       VY_LAUNCH_OK();
       count_launch(2);
-      return VY_OK;
     }
   }
   VY_CHECK_ARG(p->force_form != 2 || pl.ok, "vy_talk_attn: the tiled form takes heads <= 64 and vdim <= 128 within 200 KB of shared memory");
