@@ -297,6 +297,72 @@ def test_score_exchanging_prompts_keep_large_numbers_to_where_they_are_seen(wind
             assert _err(got[rows][..., 5], want[rows][..., 5]) < 4 * BOUND
 
 
+@pytest.mark.parametrize("bad", [1e5, 1e12, float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["value", "state"])
+def test_linear_attention_keeps_large_numbers_to_their_column(bad, where):
+    """All chunks at once, then a continuation: a value, or an entry of the state that is carried in, changes its own column and nothing else."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(4)
+    T, more, H, dk, dv, at, col = 200, 70, 2, 48, 80, 112, 5
+    q, k, v = (torch.randn(T + more, H * w, generator=g, device=DEV) for w in (dk, dk, dv))
+    S0 = torch.randn(1, H, dk, dv, generator=g, device=DEV)
+    decay = torch.tensor([0.99, 0.9], device=DEV)
+
+    def walk(v, S):
+        S, out = S.clone(), []
+        for a, n in ((0, T), (T, more)):
+            batch = ops.PackedBatch(_i32([0, n]), _i32([a + 1]), _i32([0]), n)
+            out.append(ops.linear_attn(batch, q[a:a + n], k[a:a + n], v[a:a + n], decay, S, heads=H, dim=dk, vdim=dv))
+        return torch.cat(out).view(-1, H, dv), S
+
+    clean, S_clean = walk(v, S0)
+    vb, Sb = v.clone(), S0.clone()
+    if where == "value":
+        vb[at, col] = bad
+    else:
+        Sb[0, 0, 7, col] = bad
+    got, S = walk(vb, Sb)
+    hit = torch.zeros_like(got, dtype=torch.bool)
+    hit[at if where == "value" else 0:, 0, col] = True
+    hit_S = torch.zeros_like(S, dtype=torch.bool)
+    hit_S[0, 0, :, col] = True
+    assert float((got - clean)[~hit].norm() / clean[~hit].norm()) < BOUND and float((S - S_clean)[~hit_S].norm() / S_clean[~hit_S].norm()) < BOUND
+    if not bad == bad or abs(bad) == float("inf"):
+        assert not bool(torch.isfinite(got[hit][64:]).any())
+    else:
+        want = OH.lightning_attention(q.double().view(-1, H, dk).cpu(), k.double().view(-1, H, dk).cpu(), vb.double().view(-1, H, dv).cpu(), decay.double().tolist())
+        if where == "value":   # from a state of zero: the column's own numbers
+            got0, _ = walk(vb, torch.zeros_like(S0))
+            assert _err(got0[:, 0, col], want[:, 0, col].cpu()) < BOUND
+
+
+@pytest.mark.parametrize("bad", [1e6, 1e12, float("inf")])
+def test_state_space_keeps_large_numbers_to_their_column(bad):
+    """The same recurrence with a decay per token (vy_ssd): a large input channel of one head stays in its column of the state and out of the other heads."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(5)
+    T, H, G, N, dv, taps, at, col = 200, 4, 2, 48, 32, 3, 112, 5
+    inner, gn = H * dv, G * N
+    x, b, c, dt, z = (torch.randn(T, w, generator=g, device=DEV) for w in (inner, gn, gn, H, inner))
+    cw = torch.randn(inner + 2 * gn, taps, generator=g, device=DEV).abs() * 0.5
+
+    def run(x):
+        state, conv = torch.zeros(1, H, N, dv, device=DEV), torch.zeros(1, taps, inner + 2 * gn, device=DEV)
+        out = ops.ssd(ops.PackedBatch(_i32([0, T]), _i32([0]), _i32([0]), T), x, b, c, dt, z, cw, None, conv, torch.zeros(H, device=DEV), torch.full((H,), -2.0, device=DEV),
+                      torch.ones(H, device=DEV), torch.ones(inner, device=DEV), state, torch.zeros(1, 1, dtype=torch.int32, device=DEV), heads=H, groups=G, dim=N, vdim=dv,
+                      taps=taps, norm_groups=H, norm_eps=1e-5)
+        return out.view(T, H, dv), state
+
+    clean, S_clean = run(x)
+    xb = x.clone()
+    xb[at, col] = bad
+    got, S = run(xb)
+    hit = torch.zeros_like(S, dtype=torch.bool)
+    hit[0, 0, :, col] = True
+    assert float((S - S_clean)[~hit].norm() / S_clean[~hit].norm()) < BOUND
+    assert float((got - clean)[:, 1:].norm() / clean[:, 1:].norm()) < BOUND and float((got - clean)[:at].norm() / clean[:at].norm()) < BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -9,6 +9,11 @@
 // order, on fp32 FMAs) is as long as the sequence and leaves SMs idle for few sequences; here only the scan is serial, and it is bound by the bytes
 // of the states (dim x vdim x 4 per chunk and head, written twice, read twice). q and k shared by a group of heads (state space: b and c) are
 // split, and their scores computed, once per group.
+//
+// The fp16 halves are off by at most 2^-49 of the largest entry under their unit, a row of q, k or v or a whole state. la_states looks at the rows (tokens) and
+// columns (channels) of every chunk's q, k and v and of the state that is carried in: where the largest entry of one is below 2^-20 of the largest of all
+// (a column of fewer than 8 tokens, whose entries may all be small by chance: 2^-24; zeros aside), and where an infinity or NaN is among them, the
+// heads of the CTA are left to the walk, which runs behind the three launches and starts from the state that la_scan kept as the one before the first chunk.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 
@@ -21,6 +26,7 @@ struct LaChunks {
   float* U;          // [slots][heads][dim][vdim]
   float* D;          // [slots][heads]
   unsigned* top;     // [slots][heads] largest |S| before the chunk, as bits
+  int* odd;          // [slots][heads / hp][vslices] 1: not for fp16 halves
 };
 __device__ __forceinline__ long long la_slot(const RecDev& d, int s, int c) { return d.cu[s] / LM_C + s + c; }
 
@@ -85,35 +91,74 @@ template <int ACT>
 __device__ __forceinline__ float4 act4(float4 x, int act) {
   return make_float4(act_of<ACT>(x.x, act), act_of<ACT>(x.y, act), act_of<ACT>(x.z, act), act_of<ACT>(x.w, act));
 }
-__device__ __forceinline__ float abs4(float4 x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); }
-__device__ __forceinline__ void store_split4(unsigned char* hi, unsigned char* lo, int at, float4 x, float sc) {
+__device__ __forceinline__ void store_split4(unsigned char* hi, unsigned char* lo, int at, float4 x, float4 sc) {
   uint2 h, l;
-  split2(x.x * sc, x.y * sc, h.x, l.x);
-  split2(x.z * sc, x.w * sc, h.y, l.y);
+  split2(x.x * sc.x, x.y * sc.y, h.x, l.x);
+  split2(x.z * sc.z, x.w * sc.w, h.y, l.y);
   *reinterpret_cast<uint2*>(hi + at) = h;
   *reinterpret_cast<uint2*>(lo + at) = l;
 }
-// the CTA's largest value, in every thread (T threads; red: one float per warp, free before and after)
-template <int T>
-__device__ __forceinline__ float block_max(float m, float* red) {
-  m = warp_max(m);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  float x = red[0];
+// Largest and smallest (but not zero) of rows' and columns' largest entries, as bits: positive numbers order like them, NaN after infinity
+constexpr unsigned RANGE_NONE = 0x7f800000u;   // infinity: no entry yet
+struct Range { unsigned top, low; };
+__device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ void note(Range& r, unsigned m, bool few = false) {
+  r.top = max(r.top, m);
+  if (m) r.low = min(r.low, few ? __float_as_uint(16.f * __uint_as_float(m)) : m);
+}
+__device__ __forceinline__ void note_warp(Range* to, Range r) {   // to: shared memory, read after a barrier
+  r.top = __reduce_max_sync(0xffffffffu, r.top);
+  r.low = __reduce_min_sync(0xffffffffu, r.low);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&to->top, r.top);
+    atomicMin(&to->low, r.low);
+  }
+}
+__device__ __forceinline__ bool too_wide(Range r) { return r.top >= 0x7f800000u || __uint_as_float(r.low) < 0x1p-20f * __uint_as_float(r.top); }
+
+// A thread's N quads of four columns, of rows STEP apart: each column's largest over all rows (lanes that share the columns differ in bits FROM and above), noted;
+// each row's largest into rows_s (bits; zero before)
+template <int N, int STEP, int FROM>
+__device__ __forceinline__ uint4 look(const float4 (&x)[N], unsigned* rows_s, bool few, Range& r) {
+  uint4 m = make_uint4(0u, 0u, 0u, 0u);
+  const int lane = threadIdx.x & 31, row = lane / FROM;
 #pragma unroll
-  for (int i = 1; i < T / 32; ++i) x = fmaxf(x, red[i]);
-  __syncthreads();
-  return x;
+  for (int i = 0; i < N; ++i) {
+    const uint4 a = make_uint4(abs_bits(x[i].x), abs_bits(x[i].y), abs_bits(x[i].z), abs_bits(x[i].w));
+    m = make_uint4(max(m.x, a.x), max(m.y, a.y), max(m.z, a.z), max(m.w, a.w));
+    unsigned most = max(max(a.x, a.y), max(a.z, a.w));
+#pragma unroll
+    for (int k = 1; k < FROM; k <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, k));
+    if ((lane & (FROM - 1)) == 0) atomicMax(rows_s + row + STEP * i, most);
+  }
+#pragma unroll
+  for (int k = FROM; k < 32; k <<= 1)
+    m = make_uint4(max(m.x, __shfl_xor_sync(0xffffffffu, m.x, k)), max(m.y, __shfl_xor_sync(0xffffffffu, m.y, k)), max(m.z, __shfl_xor_sync(0xffffffffu, m.z, k)),
+                   max(m.w, __shfl_xor_sync(0xffffffffu, m.w, k)));
+  note(r, m.x, few);
+  note(r, m.y, few);
+  note(r, m.z, few);
+  note(r, m.w, few);
+  return m;
+}
+__device__ __forceinline__ float4 column_units(uint4 m) {   // 2^(exponent - SPLIT_TOP) of each column
+  const auto u = [](unsigned b) { return pow2i(split_exponent(__uint_as_float(b)) - SPLIT_TOP); };
+  return make_float4(u(m.x), u(m.y), u(m.z), u(m.w));
+}
+__device__ __forceinline__ float4 column_scales(uint4 m) {
+  const auto u = [](unsigned b) { return split_scale(split_exponent(__uint_as_float(b))); };
+  return make_float4(u(m.x), u(m.y), u(m.z), u(m.w));
 }
 
 constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows of 64 value columns
 
-// CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w ..; tokens are the summed index, so k and the
-// weighted v are each scaled by one power of two for the whole chunk. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 84 us, bound by
+// CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w .., and it reads and splits those channels of k (eight
+// tokens at a time) and value columns 8 w .. (sixteen at a time), all tokens of them: tokens are the summed index, so a channel and a column have one unit
+// each, and their largest entries need no other warp. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 84 us, bound by
 // writing the states (134 MB) and by the latency of each chunk's few steps
 // ACT: see act_of
 template <bool TD, int ACT>
-__global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
+__global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) unsigned char lu_smem[];
@@ -123,31 +168,57 @@ __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, i
   unsigned char* Wh = Kl + LM_C * kb;
   unsigned char* Wl = Wh + LM_C * LU_VB;
   float* es = reinterpret_cast<float*>(Wl + LM_C * LU_VB);   // [64] decay to the chunk's end times write strength
-  float* red = es + LM_C;
+  float* ku = es + LM_C;                                     // [128], [64]: units of k's channels and of w's columns
+  float* wu = ku + 128;
+  unsigned* rows_s = reinterpret_cast<unsigned*>(wu + 64);   // [4][64] rows' largest: k, q, v of even and of odd heads; [128] of the state
+  Range* range = reinterpret_cast<Range*>(rows_s + 4 * LM_C + 128);   // [4]: k, q, v, state
   const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
   const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LM_C;
   if (t0 >= n) return;
   const int nt = min(LM_C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
   const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
   const long long r0 = base + t0, slot = la_slot(d, s, c);
-  const int row = t >> 2, c4 = (t & 3) * 4;   // loads: four threads per token row
-  float4 x[8];
-  float m = 0.f;
+  for (int i = t; i < 4 * LM_C + 128; i += LU_T) rows_s[i] = 0u;
+  if (t < 4) range[t] = {0u, RANGE_NONE};
+  __syncthreads();
+  const bool few = nt < 8;
+  {
+    const int row = lane >> 2, ch = 16 * warp + 4 * (lane & 3);
+    float4 x[8];
+    const auto read = [&](const void* p, long long ld) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    x[i] = row < nt ? load4(d.k, d.in_dt, vec, (r0 + row) * d.ldk + static_cast<long long>(hq) * d.dim, c4 + 16 * i, d.dim) : make_float4(0.f, 0.f, 0.f, 0.f);
-    x[i] = act4<ACT>(x[i], d.in_act);
-    m = fmaxf(m, abs4(x[i]));
+      for (int i = 0; i < 8; ++i) {
+        const int r = row + 8 * i;
+        x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < nt && ch < d.dim) x[i] = act4<ACT>(load4(p, d.in_dt, vec, (r0 + r) * ld + static_cast<long long>(hq) * d.dim, ch, d.dim), d.in_act);
+      }
+    };
+    Range rk = {0u, RANGE_NONE}, rq = rk;
+    if (v0 == 0) {
+      read(d.q, d.ldq);
+      look<8, 8, 4>(x, rows_s + LM_C, few, rq);
+      note_warp(range + 1, rq);
+    }
+    read(d.k, d.ldk);
+    const uint4 m = look<8, 8, 4>(x, rows_s, few, rk);
+    note_warp(range, rk);
+    const float4 sc = column_scales(m);
+    if (row == 0) *reinterpret_cast<float4*>(ku + ch) = column_units(m);
+    if (ch < dim16) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) store_split4(Kh, Kl, (row + 8 * i) * kb + ch * 2, x[i], sc);
+    }
   }
-  const int ek = split_exponent(block_max<LU_T>(m, red));
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    if (c4 + 16 * i < dim16) store_split4(Kh, Kl, row * kb + (c4 + 16 * i) * 2, x[i], split_scale(ek));
   const unsigned ka = smem_addr(Kh) + lane_b(lane, kb) + 16 * warp * 2, wb = smem_addr(Wh) + lane_bt(lane, LU_VB);
+  const int row = lane >> 1, vc = 8 * warp + 4 * (lane & 1);
+  Range rv = {0u, RANGE_NONE}, rs = rv;   // this thread's share
   float4 next[4];
   const auto fetch = [&](int h) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) next[i] = row < nt ? load4(d.v, d.in_dt, vec, (r0 + row) * d.ldv + static_cast<long long>(h) * d.vdim + v0, c4 + 16 * i, vw) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < 4; ++i) {
+      const int r = row + 16 * i;
+      next[i] = r < nt ? load4(d.v, d.in_dt, vec, (r0 + r) * d.ldv + static_cast<long long>(h) * d.vdim + v0, vc, vw) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   };
   fetch(h0);
   for (int h = h0; h < h0 + hp; ++h) {
@@ -167,18 +238,48 @@ __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, i
     float4 y[4] = {next[0], next[1], next[2], next[3]};
     if (h + 1 < h0 + hp) fetch(h + 1);   // in flight during this head's products
     __syncthreads();
-    float mv = 0.f;
-    const float e = es[row];
+    unsigned* vrows = rows_s + (2 + ((h - h0) & 1)) * LM_C;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      y[i] = act4<ACT>(y[i], d.in_act);
-      y[i] = make_float4(y[i].x * e, y[i].y * e, y[i].z * e, y[i].w * e);
-      mv = fmaxf(mv, abs4(y[i]));
+      if (row + 16 * i < nt) y[i] = act4<ACT>(y[i], d.in_act);
     }
-    const int ew = split_exponent(block_max<LU_T>(mv, red));
+    look<4, 16, 2>(y, vrows, few, rv);
+    uint4 m = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) store_split4(Wh, Wl, row * LU_VB + (c4 + 16 * i) * 2, y[i], split_scale(ew));
+    for (int i = 0; i < 4; ++i) {
+      const float e = es[row + 16 * i];
+      y[i] = make_float4(y[i].x * e, y[i].y * e, y[i].z * e, y[i].w * e);
+      m = make_uint4(max(m.x, abs_bits(y[i].x)), max(m.y, abs_bits(y[i].y)), max(m.z, abs_bits(y[i].z)), max(m.w, abs_bits(y[i].w)));
+    }
+#pragma unroll
+    for (int k = 2; k < 32; k <<= 1)
+      m = make_uint4(max(m.x, __shfl_xor_sync(0xffffffffu, m.x, k)), max(m.y, __shfl_xor_sync(0xffffffffu, m.y, k)), max(m.z, __shfl_xor_sync(0xffffffffu, m.z, k)),
+                     max(m.w, __shfl_xor_sync(0xffffffffu, m.w, k)));
+    const float4 sv = column_scales(m);
+    if (row == 0) *reinterpret_cast<float4*>(wu + vc) = column_units(m);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) store_split4(Wh, Wl, (row + 16 * i) * LU_VB + vc * 2, y[i], sv);
+    if (c == 0 && d.pos0[s] > 0) {   // the state that is carried in: a thread reads every fourth entry of a column
+      const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 + (t & 63);
+      unsigned* srows = rows_s + 4 * LM_C;
+      unsigned top = 0u;
+#pragma unroll 4
+      for (int i = t >> 6; i < d.dim; i += 4) {
+        const unsigned a = (t & 63) < vw ? abs_bits(sp[static_cast<long long>(i) * d.vdim]) : 0u, most = __reduce_max_sync(0xffffffffu, a);
+        top = max(top, a);
+        if (lane == 0) atomicMax(srows + i, most);
+      }
+      note(rs, top, true);
+    }
     __syncthreads();
+    if (t < LM_C) {   // cleared for the head after the next, two barriers away
+      note(rv, vrows[t]);
+      vrows[t] = 0u;
+    }
+    if (c == 0 && t < 128) {
+      note(rs, rows_s[4 * LM_C + t]);
+      rows_s[4 * LM_C + t] = 0u;
+    }
     if (16 * warp < dim16) {
       float a[8][4], b[8][4];   // hi hi, and the two small products
 #pragma unroll
@@ -203,16 +304,17 @@ __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, i
           mma_f16(b[2 * j + 1], ah, bl[2], bl[3]);
         }
       }
-      const float u1 = pow2i(ek - SPLIT_TOP), u2 = pow2i(ew - SPLIT_TOP);
       float* U = w.U + (slot * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int i = 16 * warp + gq + 8 * r;
         if (i >= d.dim) continue;
+        const float u1 = ku[i];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int col = 8 * j + 2 * tq;
-          const float p = fmaf(b[j][2 * r], LO_UNIT, a[j][2 * r]) * u1 * u2, q = fmaf(b[j][2 * r + 1], LO_UNIT, a[j][2 * r + 1]) * u1 * u2;
+          const float2 u2 = *reinterpret_cast<const float2*>(wu + col);
+          const float p = fmaf(b[j][2 * r], LO_UNIT, a[j][2 * r]) * u1 * u2.x, q = fmaf(b[j][2 * r + 1], LO_UNIT, a[j][2 * r + 1]) * u1 * u2.y;
           float* at = U + static_cast<long long>(i) * d.vdim + col;
           if (col + 1 < vw && d.vdim % 2 == 0) *reinterpret_cast<float2*>(at) = make_float2(p, q);
           else {
@@ -223,6 +325,18 @@ __global__ void __launch_bounds__(LU_T) la_states_kernel(RecDev d, LaChunks w, i
       }
     }
   }
+  if (t < LM_C) {
+    Range r = {0u, RANGE_NONE};
+    note(r, rows_s[t]);
+    note_warp(range, r);
+    r = {0u, RANGE_NONE};
+    note(r, rows_s[LM_C + t]);
+    note_warp(range + 1, r);
+  }
+  note_warp(range + 2, rv);
+  note_warp(range + 3, rs);
+  __syncthreads();
+  if (t == 0) w.odd[(slot * gridDim.y + blockIdx.y) * vslices + blockIdx.x % vslices] = too_wide(range[0]) || too_wide(range[1]) || too_wide(range[2]) || too_wide(range[3]);
 }
 
 // V elements per thread. Bound by the bytes: every chunk's state read once and written once; eight chunks' worth is in flight per thread
@@ -381,7 +495,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const int r = i + k * (LO_T / 16);
-        if (r < dim16) store_split4(Sh, Sh + s_lo, r * LU_VB + (t & 15) * 8, x[k], split_scale(es));
+        if (r < dim16) store_split4(Sh, Sh + s_lo, r * LU_VB + (t & 15) * 8, x[k], make_float4(split_scale(es), split_scale(es), split_scale(es), split_scale(es)));
       }
     }
     __syncthreads();
@@ -528,7 +642,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 // from two chunks on the three launches beat the walk
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim) {
   if (max_new <= LM_C || dim > 128 || rows <= 0) return 0;
-  const long long slots = rows / LM_C + n_seqs, floats = slots * heads * (static_cast<long long>(dim) * vdim + 2) + 4;
+  const long long slots = rows / LM_C + n_seqs, floats = slots * heads * (static_cast<long long>(dim) * vdim + 2 + (vdim + 63) / 64) + 4;
   return floats <= (1LL << 28) ? floats : 0;   // 1 GB: past it the walk, which keeps its state on the chip
 }
 
@@ -542,12 +656,13 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   w.U = ws;
   w.D = ws + slots * d.heads * static_cast<long long>(d.dim) * d.vdim;
   w.top = reinterpret_cast<unsigned*>(w.D + slots * d.heads);
+  w.odd = reinterpret_cast<int*>(w.top + slots * d.heads);
   const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, vslices = (d.vdim + 63) / 64, chunks = (max_new + LM_C - 1) / LM_C;
   // heads per CTA: those that share q and k, fewer while that leaves less than two CTAs per SM
   int hp = TD ? d.heads / d.kv_heads : 1;
   while (hp % 2 == 0 && static_cast<long long>(chunks) * vslices * (d.heads / hp) * n_seqs < 2LL * num_sms()) hp /= 2;
   const dim3 grid(static_cast<unsigned>(chunks) * vslices, d.heads / hp, n_seqs);
-  const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + LU_T / 32);
+  const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + 128 + 64 + 4 * LM_C + 128) + 4 * sizeof(Range);
   const size_t q2 = 2 * LM_C * static_cast<size_t>(kb), vs = 2 * LM_C * LU_VB + 2 * static_cast<size_t>(dim16) * LU_VB;
   const size_t smem_o = q2 + (q2 > vs ? q2 : vs) + sizeof(float) * 7 * LM_C;
   static bool once = false;
@@ -565,7 +680,14 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   const dim3 sgrid((each + per - 1) / per, d.heads, n_seqs);
   e = quad ? launch_kernel(la_scan_kernel<4>, sgrid, dim3(256), 0, st, d, w) : launch_kernel(la_scan_kernel<1>, sgrid, dim3(256), 0, st, d, w);
   if (e != cudaSuccess) return e;
-  return launch_kernel(la_outputs_kernel<TD, ACT>, grid, dim3(LO_T), smem_o, st, d, w, hp, vslices, dim16, vec, svec && quad);
+  e = launch_kernel(la_outputs_kernel<TD, ACT>, grid, dim3(LO_T), smem_o, st, d, w, hp, vslices, dim16, vec, svec && quad);
+  if (e != cudaSuccess) return e;
+  RecDev r = d;   // the walk, for what is left to it
+  r.odd = w.odd;
+  r.odd_heads = hp;
+  r.odd_each = vslices;
+  r.first = w.U;
+  return TD ? launch_ssd_chunked(r, n_seqs, st) : launch_linear_attn_chunked(r, n_seqs, st);
 }
 
 template <bool TD>

@@ -1069,7 +1069,7 @@ extern "C" int vy_linear_attn(const VyLinAttn* p) {
   if (ws_need > 0 && p->workspace && reinterpret_cast<uintptr_t>(p->workspace) % 16 == 0 && p->workspace_floats >= ws_need) {
     VY_CUDA_OK(launch_linear_attn_mma<false>(d, p->n_seqs, p->max_new, p->rows, p->workspace, st));
     VY_LAUNCH_OK();
-    count_launch(3);
+    count_launch(4);
     return VY_OK;
   }
   if (p->max_new >= LA_CHUNKED_MIN && p->dim <= 128) {

@@ -154,6 +154,9 @@ struct RecDev {
   float q_scale;  // gated linear attention (the delta kernel without its correction term): multiplies q as it is read
   float* state;
   void* out; long long ld_out; int out_dt;
+  // chunked walk behind linear_attn_mma.cu: null, or [cu / 64 + sequence + chunk][heads / odd_heads][odd_each] with a 1 where the sequence and head are left to
+  // it, and their state before each chunk, [cu / 64 + sequence + chunk][heads][dim][vdim]
+  const int* odd; int odd_heads, odd_each; const float* first;
 };
 
 // Prompt-sized steps: defined in the files named above.
@@ -162,7 +165,7 @@ cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 // 16 tokens per step of the walk (delta_rule_mma.cu), given delta_rule_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); two launches
 long long delta_rule_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 cudaError_t launch_delta_rule_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
-// All chunks at once (linear_attn_mma.cu), given linear_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); three launches
+// All chunks at once (linear_attn_mma.cu), given linear_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); four launches
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 template <bool TD>
 cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);

@@ -70,6 +70,15 @@ __global__ void __launch_bounds__(LA_T, OCC) linear_attn_chunk_kernel(RecDev d, 
   const int t = threadIdx.x, ti = t >> 4, tj = t & 15;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
   if (n <= 0) return;
+  const float* sp_in = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * d.dim * d.vdim;
+  if (d.odd) {
+    const long long slot0 = base / LA_C + s, groups = d.heads / d.odd_heads;
+    bool odd = false;
+    for (int i = t; i < (n + LA_C - 1) / LA_C * d.odd_each; i += LA_T)
+      odd = odd || d.odd[((slot0 + i / d.odd_each) * groups + h / d.odd_heads) * d.odd_each + i % d.odd_each];
+    if (!__syncthreads_or(odd)) return;
+    sp_in = d.first + (slot0 * d.heads + h) * static_cast<long long>(d.dim) * d.vdim;
+  }
   const int hq = TD ? h / (d.heads / d.kv_heads) : h;
   float rate = 0.f, dt_b = 0.f, skip = 0.f;
   if constexpr (TD) {
@@ -81,7 +90,7 @@ __global__ void __launch_bounds__(LA_T, OCC) linear_attn_chunk_kernel(RecDev d, 
   const bool carried = d.pos0[s] > 0;
   for (int e = t; e < DP * VS; e += LA_T) {
     const int i = e / VS, c = e % VS;
-    Ss[i * LDV + c] = (carried && i < d.dim && v0 + c < d.vdim) ? sp[static_cast<long long>(i) * d.vdim + v0 + c] : 0.f;
+    Ss[i * LDV + c] = (carried && i < d.dim && v0 + c < d.vdim) ? sp_in[static_cast<long long>(i) * d.vdim + v0 + c] : 0.f;
   }
   for (int t0 = 0; t0 < n; t0 += LA_C) {
     const int nt = min(LA_C, n - t0);

@@ -488,7 +488,7 @@ extern "C" int vy_ssd(const VySsd* p) {
   if (chunk_floats > 0 && p->workspace_floats >= vy_ssd_workspace_floats(p->rows, p->n_seqs, p->max_new, p->heads, p->groups, p->dim, p->vdim)) {
     VY_CUDA_OK(launch_linear_attn_mma<true>(r, p->n_seqs, p->max_new, p->rows, d.xc + p->rows * d.ld_xc, st));
     VY_LAUNCH_OK();
-    count_launch(3);
+    count_launch(4);
   } else {
     VY_CUDA_OK(launch_ssd_chunked(r, p->n_seqs, st));
     VY_LAUNCH_OK();
