@@ -363,6 +363,29 @@ def test_state_space_keeps_large_numbers_to_their_column(bad):
     assert float((got - clean)[:, 1:].norm() / clean[:, 1:].norm()) < BOUND and float((got - clean)[:at].norm() / clean[:at].norm()) < BOUND
 
 
+@pytest.mark.parametrize("bad", [1e6, 1e12, 1e30])
+def test_delta_rule_keeps_a_large_value_to_later_tokens(bad):
+    """The tokens before a large value that share its 16-token step read what they read without it."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(1)
+    T, H, dk, dv, at, col = 40, 1, 48, 40, 29, 5
+    q, k, v, a, b = (torch.randn(T, w, generator=g, device=DEV) for w in (dk, dk, dv, dk, H))
+    batch = ops.PackedBatch(_i32([0, T]), _i32([0]), _i32([0]), T)
+    run = lambda vv: ops.delta_rule(batch, q, k, vv, a, b, torch.zeros(1, device=DEV), torch.zeros(1, H, dk, dv, device=DEV), heads=H, kv_heads=H, dim=dk, vdim=dv)  # noqa: E731
+    clean = run(v)
+    vv = v.clone()
+    vv[at, col] = bad
+    got = run(vv)
+    hit = torch.zeros(T, dv, dtype=torch.bool, device=DEV)
+    hit[at:, col] = True
+    assert float((got - clean)[16:at, col].norm() / clean[16:at, col].norm()) < BOUND
+    assert float((got - clean)[~hit].norm() / clean[~hit].norm()) < BOUND
+    unit = lambda x: OH.unit(x.double().cpu().view(T, 1, dk))  # noqa: E731
+    decay = torch.exp(-torch.nn.functional.softplus(a.double().cpu(), threshold=1e9).view(T, 1, dk))
+    want = OH.gated_delta_rule(unit(q) * dk ** -0.5, unit(k), vv.double().cpu().view(T, 1, dv), decay, torch.sigmoid(b.double().cpu()))[:, 0, col]
+    assert _err(got[at:, col], want[at:]) < 4 * BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -280,8 +280,10 @@ __device__ __forceinline__ void dc_bulk_load(void* dst, const void* src, unsigne
                : "memory");
 }
 
-// The writes' share of the read-outs when a write is infinite or NaN: the product's zeros would carry it to the tokens before it
-static __device__ __noinline__ void dc_read_finite(float (&o)[2][4], const float (&u)[2][4], const unsigned char* b, const float* unit, int lane) {
+// The writes' share of the read-outs in FMAs, a token at a time: where a write is infinite or NaN, the product's zeros would carry it to the tokens before it, and
+// where the writes of a column lie far apart, the larger ones' unit would cost the smaller ones, which earlier tokens read, their bits
+constexpr float DC_APART = 0x1p-20f;   // the halves are off by at most 2^-49 of the column's largest write; 3 in 10000 chunks of normal numbers come here
+static __device__ __noinline__ void dc_read_serial(float (&o)[2][4], const float (&u)[2][4], const unsigned char* b, const float* unit, int lane) {
   const int tq = 2 * (lane & 3);
 #pragma unroll
   for (int s = 0; s < DC_T; ++s) {
@@ -458,12 +460,12 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
         o[j][e] = fmaf(fmaf(y0, cut, x[2 + j][e]), LO_UNIT, y0) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
       }
     }
-    bool finite = true;
+    bool together = true;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) finite = finite && fabsf(u[j][e]) < INFINITY;
-    if (__all_sync(0xffffffffu, finite)) {
+      for (int e = 0; e < 4; ++e) together = together && fabsf(u[j][e]) < INFINITY && (fabsf(u[j][e]) >= DC_APART * (e < 2 ? m0 : m1) || u[j][e] == 0.f);
+    if (__all_sync(0xffffffffu, together)) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         float y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
         for (int e = 0; e < 4; ++e) o[j][e] = fmaf(fmaf(fmaf(y[e], DC_CUT, z[e]), LO_UNIT, y[e]) * (e < 2 ? w0 : w1), e & 1 ? p.y : p.x, o[j][e]);
       }
     } else {
-      dc_read_finite(o, u, st + Blob::b_at, unit + 2 * DC_T, lane);
+      dc_read_serial(o, u, st + Blob::b_at, unit + 2 * DC_T, lane);
     }
     // through with the stage: the last warp refills it
     __syncwarp();
