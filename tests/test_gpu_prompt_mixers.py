@@ -386,6 +386,21 @@ def test_delta_rule_keeps_a_large_value_to_later_tokens(bad):
     assert _err(got[at:, col], want[at:]) < 4 * BOUND
 
 
+@pytest.mark.parametrize("dim", [20, 48, 100])
+@pytest.mark.parametrize("act", ["sigmoid", "silu", "relu2", "gelu_tanh"])
+@pytest.mark.parametrize("T", [40, 150])
+def test_linear_attention_activations_leave_padding_alone(dim, act, T):
+    """Channel counts that no tile divides, with activations whose value at zero is not zero, chunk by chunk and all chunks at once."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    q, k, v = (torch.randn(T, w, generator=g, device=DEV) for w in (dim, dim, 20))
+    state = torch.zeros(1, 1, dim, 20, device=DEV)
+    got = ops.linear_attn(ops.PackedBatch(_i32([0, T]), _i32([0]), _i32([0]), T), q, k, v, torch.tensor([0.9], device=DEV), state, heads=1, dim=dim, vdim=20, in_act=act)
+    f = {"sigmoid": torch.sigmoid, "silu": torch.nn.functional.silu, "relu2": lambda x: torch.relu(x) ** 2, "gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh")}[act]
+    x = [f(t.double().cpu()).view(T, 1, -1) for t in (q, k, v)]
+    assert _err(got, OH.lightning_attention(*x, [float(torch.tensor(0.9))]).reshape(T, -1)) < 2 * BOUND   # activations in fp32
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

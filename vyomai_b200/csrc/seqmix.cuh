@@ -68,7 +68,7 @@ __device__ __forceinline__ void rows_to_smem(float* dst, int ld, int rows, int w
         const int e = e0 + u * T;
         if (e < total) {
           const int j = e / w4, c = (e - j * w4) << 2;
-          if (act != VY_UACT_NONE) {
+          if (act != VY_UACT_NONE && c < width) {   // not the channels that fill up rows: act(0) may not be 0
             v[u].x = apply_uact(v[u].x, act); v[u].y = apply_uact(v[u].y, act);
             v[u].z = apply_uact(v[u].z, act); v[u].w = apply_uact(v[u].w, act);
           }
@@ -95,7 +95,7 @@ __device__ __forceinline__ void rows_to_smem(float* dst, int ld, int rows, int w
         const int e = e0 + u * T;
         if (e < total) {
           const int j = e / width4, c = e - j * width4;
-          dst[j * ld + c] = act != VY_UACT_NONE ? apply_uact(v[u], act) : v[u];
+          dst[j * ld + c] = act != VY_UACT_NONE && c < width ? apply_uact(v[u], act) : v[u];
         }
       }
     }

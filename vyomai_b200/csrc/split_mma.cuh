@@ -85,7 +85,7 @@ static __device__ __noinline__ void store2_any(void* dst, int dt, long long at, 
 // Rows [0, rows) of a block of `src` as hi / lo planes (`row_bytes` between rows of a plane, columns zero-filled up to pad16, a
 // multiple of 16 and at most MAXD), with 2^(a row's exponent - drop) in unit[row * ustep]. Row j starts at element off(j) of src or is all zero when
 // off(j) < 0. Eight lanes share a row (coalesced 128-byte runs); a thread has the loads of U rows in flight before it uses any. vec: src
-// is fp32, row starts and the width are multiples of 4 elements. map: applied to every entry read (map(0) = 0). seen: given each row's largest entry.
+// is fp32, row starts and the width are multiples of 4 elements. map: applied to every entry read, not to the zeros that fill up rows. seen: given each row's largest entry.
 struct SameValue {
   __device__ __forceinline__ float operator()(float x) const { return x; }
 };
@@ -118,7 +118,10 @@ __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo,
       const int r = r0 + u * NW * 4;
       float m = 0.f;
 #pragma unroll
-      for (int i = 0; i < NI; ++i) x[u][i] = make_float4(map(x[u][i].x), map(x[u][i].y), map(x[u][i].z), map(x[u][i].w));
+      for (int i = 0; i < NI; ++i) {
+        const int c = l8 * 4 + 32 * i;
+        x[u][i] = make_float4(c < width ? map(x[u][i].x) : 0.f, c + 1 < width ? map(x[u][i].y) : 0.f, c + 2 < width ? map(x[u][i].z) : 0.f, c + 3 < width ? map(x[u][i].w) : 0.f);
+      }
 #pragma unroll
       for (int i = 0; i < NI; ++i) m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u][i].x), fabsf(x[u][i].y)), fmaxf(fabsf(x[u][i].z), fabsf(x[u][i].w))));
 #pragma unroll
