@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
       __threadfence_block();
       last = atomicAdd(&done[b], 1) % NW == NW - 1;
       __threadfence_block();
+      if (last) fence_proxy_async_smem();   // the reads of the buffer come before the copy that refills it
     }
     if (__shfl_sync(0xffffffffu, last, 0) && it + NS < tiles) fetch((it + NS) * N, b);
   }
