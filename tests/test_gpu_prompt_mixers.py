@@ -401,6 +401,35 @@ def test_linear_attention_activations_leave_padding_alone(dim, act, T):
     assert _err(got, OH.lightning_attention(*x, [float(torch.tensor(0.9))]).reshape(T, -1)) < 2 * BOUND   # activations in fp32
 
 
+def test_a_wait_that_timed_out_stops_what_would_use_its_results():
+    """The flag such a wait raises (here from the host): attention, delta rule, product and a serving step refuse until it is acknowledged, in fp32 models too."""
+    from tests import hybrid_util as HU
+    from vyomai_b200 import ops
+    from vyomai_b200._lib import VyomError, lib
+    model, _ = HU.build(HU.small_config())   # fp32: no vy_gemm
+    engine, _ = HU.engine_for(model)
+    for _ in range(3):
+        engine.feed([("a", [3], [0])])   # from the third on a replayed step
+    x = torch.randn(64, 64, device=DEV)
+    batch = ops.PackedBatch(_i32([0, 64]), _i32([0]), _i32([0]), 64, _i32([[0]]), 64)
+    calls = [lambda: ops.window_attn(batch, x, x.view(1, 64, 1, 64), x.view(1, 64, 1, 64), heads=1, kv_heads=1, dim=64, vdim=64, scale=1.0, window=0, keep_first=0),
+             lambda: ops.delta_rule(batch, x, x, x, x, x[:, :1], torch.zeros(1, device=DEV), torch.zeros(1, 1, 64, 64, device=DEV), heads=1, kv_heads=1, dim=64, vdim=64),
+             lambda: ops.gemm(x, x), lambda: engine.feed([("a", [3], [0])])]
+    for call in calls:
+        call()
+    assert lib().vy_gemm_poison_raise() == 0
+    try:
+        for call in calls:
+            with pytest.raises(VyomError, match="timed out"):
+                call()
+    finally:
+        assert lib().vy_gemm_poisoned() == 1
+    for call in calls:
+        call()
+    torch.cuda.synchronize()
+    assert lib().vy_gemm_poison_peek() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

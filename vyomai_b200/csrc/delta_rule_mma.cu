@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
   constexpr int KS = DP / 16, NT = DP / 8, STAGE = Blob::bytes + DC_NW * 1024;
   extern __shared__ __align__(128) unsigned char dc_smem[];
   __shared__ __align__(8) uint64_t full[DC_NS];
-  __shared__ int done[DC_NS];   // warps that are through with a stage, counted up for ever
+  __shared__ int done[DC_NS], issued[DC_NS];   // warps that are through with a stage, counted up for ever; chunks sent for into it
   const int s = blockIdx.z, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l4 = lane >> 2, tq = 2 * (lane & 3);
   const int base = d.cu[s], n = d.cu[s + 1] - base;
@@ -319,6 +319,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
   const auto fetch = [&](int c, int b) {
     const long long at = (slot0 + c) * d.heads + h;
     unsigned char* st = dc_smem + b * STAGE;
+    ++issued[b];
     mbar_arrive_expect_tx(&full[b], STAGE);
     dc_bulk_load(st, w.blobs + at * Blob::bytes, Blob::bytes, &full[b]);
     dc_bulk_load(st + Blob::bytes, w.wv + (at * (w.vpad / 16) + blockIdx.x * DC_NW) * 256, DC_NW * 1024, &full[b]);
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
   if (threadIdx.x == 0) {
     for (int b = 0; b < DC_NS; ++b) {
       mbar_init(&full[b], 1);
-      done[b] = 0;
+      done[b] = issued[b] = 0;
     }
     fence_mbar_init();
     for (int b = 0; b < min(DC_NS, chunks); ++b) fetch(b, b);
@@ -345,6 +346,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       S[j][e] = carried && i < d.dim && (e < 2 ? ok0 : ok1) ? sp[static_cast<long long>(i) * d.vdim + 8 * (e >> 1)] : 0.f;
     }
   __syncthreads();
+  bool alive = true;   // no wait of this thread has timed out; lane 0 sends for chunks
   for (int c = 0; c < chunks; ++c) {
     const int b = c % DC_NS;
     const unsigned char* st = dc_smem + b * STAGE;
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
     }
     const int e0 = split_exponent(m0), e1 = split_exponent(m1);
     const float s0 = split_scale(e0), s1 = split_scale(e1), n0 = pow2i(e0 - SPLIT_TOP), n1 = pow2i(e1 - SPLIT_TOP);
-    mbar_wait_soft(&full[b], (c / DC_NS) & 1, poison);
+    alive = mbar_wait_soft(&full[b], (c / DC_NS) & 1, poison) && alive;
     const uint4* ops = reinterpret_cast<const uint4*>(st) + lane;
     float r[4][4], x[4][4], half[4][4];   // S^T P and S^T G q: 8 tokens each
 #pragma unroll
@@ -482,7 +484,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
     }
     // through with the stage: the last warp refills it
     __syncwarp();
-    if (lane == 0 && c + DC_NS < chunks) {
+    if (lane == 0 && alive && c + DC_NS < chunks) {
       __threadfence_block();
       if (atomicAdd(&done[b], 1) % DC_NW == DC_NW - 1) {
         __threadfence_block();
@@ -506,6 +508,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       const int i = 8 * j + tq + (e & 1);
       if (i < d.dim && (e < 2 ? ok0 : ok1)) sp[static_cast<long long>(i) * d.vdim + 8 * (e >> 1)] = S[j][e];
     }
+  if (__syncthreads_or(!alive)) mbar_drain(full, issued, DC_NS);
 }
 
 int blob_bytes(int dim) { return dim <= 32 ? DcBlob<32>::bytes : dim <= 64 ? DcBlob<64>::bytes : DcBlob<128>::bytes; }

@@ -172,7 +172,7 @@ splitk_reduce_kernel(int M, int N, int splits, const float* __restrict__ ws, con
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Per-device pair of flags that a timed-out wait inside a GEMM kernel raises (mbar_wait_soft): one int of device memory
+// Per-device pair of flags that a timed-out wait inside a kernel raises (mbar_wait_soft): one int of device memory
 // (what the other waits of the same launch poll) and one int of mapped pinned host memory (what the host reads without
 // synchronising). Allocated on first use on whichever device is current, so a process that drives several GPUs never
 // hands one device's flag to another device's kernels.
@@ -192,11 +192,13 @@ static PoisonSlot* poison_slot() {
     int* dv = nullptr;
     int* h = nullptr;
     int* hd = nullptr;
-    if (cudaMalloc(&dv, sizeof(int)) != cudaSuccess) return nullptr;
-    if (cudaMemset(dv, 0, sizeof(int)) != cudaSuccess) return nullptr;
-    if (cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the first call may come while a stream is captured: these are no part of the capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool ok = cudaMalloc(&dv, sizeof(int)) == cudaSuccess && cudaMemset(dv, 0, sizeof(int)) == cudaSuccess &&
+                    cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess && cudaHostGetDevicePointer(&hd, h, 0) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) return nullptr;
     *h = 0;
-    if (cudaHostGetDevicePointer(&hd, h, 0) != cudaSuccess) return nullptr;
     s.dev = dv; s.host = h; s.host_dev = hd;
   }
   return &s;
@@ -207,6 +209,14 @@ bool poison_ref(PoisonRef* r) {
   if (!ps) return false;
   const int lid = g_gemm_launch_id.fetch_add(1, std::memory_order_relaxed) + 1;
   *r = {ps->dev, ps->host_dev, lid & 0x7fffffff ? lid & 0x7fffffff : 1};
+  return true;
+}
+bool poison_raised(const char* who) {
+  const PoisonSlot* ps = poison_slot();
+  const int id = ps ? *reinterpret_cast<volatile int*>(ps->host) : 0;
+  if (id == 0) return false;
+  set_error("%s: a barrier wait inside an earlier kernel on this device timed out (launch id %d) — its results "
+            "and everything computed from them are invalid; vy_gemm_poisoned() acknowledges and lowers the flag", who, id);
   return true;
 }
 
@@ -236,6 +246,14 @@ extern "C" int vy_gemm_poisoned(void) {
     *reinterpret_cast<volatile int*>(f->host) = 0;
     return 1;
   }
+  return 0;
+}
+
+extern "C" int vy_gemm_poison_raise(void) {
+  using namespace vy;
+  PoisonSlot* f = poison_slot();
+  if (!f) return -1;
+  *reinterpret_cast<volatile int*>(f->host) = 1;
   return 0;
 }
 
@@ -278,12 +296,7 @@ extern "C" int vy_gemm(const VyGemm* p) {
   g.debug = dbg;
   PoisonSlot* ps = poison_slot();
   VY_CHECK_ARG(ps != nullptr, "vy_gemm: could not allocate the poison flags of this device");
-  if (*reinterpret_cast<volatile int*>(ps->host) != 0) {
-    set_error("vy_gemm: a barrier wait inside an earlier GEMM kernel on this device timed out (launch id %d) — its results "
-              "and everything computed from them are invalid; vy_gemm_poisoned() acknowledges and lowers the flag",
-              *reinterpret_cast<volatile int*>(ps->host));
-    return VY_ERR_CUDA;
-  }
+  if (poison_raised("vy_gemm")) return VY_ERR_CUDA;
   poison_ref(&g.poison);
   g.M = p->M; g.N = p->N; g.K = p->K;
   g.epi = p->epi; g.act = p->act; g.transposed_out = p->transposed_out;

@@ -916,6 +916,7 @@ extern "C" int64_t vy_window_attn_prompt_floats(int32_t n_seqs, int32_t max_new,
 extern "C" int vy_window_attn(const VyWinAttn* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_window_attn: null params");
+  if (vy_device_ok() && poison_raised("vy_window_attn")) return VY_ERR_CUDA;
   VY_NEED_DEVICE("vy_window_attn");
   VY_CHECK_ARG(p->n_seqs > 0 && p->n_seqs <= 65535 && p->max_new > 0 && p->cu_tokens && p->pos0 && p->block_table && p->block_size > 0 &&
                    p->table_width > 0, "vy_window_attn: bad batch");
@@ -1098,6 +1099,7 @@ extern "C" int64_t vy_delta_rule_prompt_floats(int64_t rows, int32_t n_seqs, int
 extern "C" int vy_delta_rule(const VyDeltaRule* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_delta_rule: null params");
+  if (vy_device_ok() && poison_raised("vy_delta_rule")) return VY_ERR_CUDA;
   VY_NEED_DEVICE("vy_delta_rule");
   VY_CHECK_ARG(p->n_seqs > 0 && p->n_seqs <= 65535 && p->cu_tokens && p->pos0 && p->slot, "vy_delta_rule: bad batch");
   VY_CHECK_ARG(p->heads > 0 && p->heads <= 65535 && p->kv_heads > 0 && p->heads % p->kv_heads == 0 && p->dim > 0 && p->dim <= 256 && p->vdim > 0,

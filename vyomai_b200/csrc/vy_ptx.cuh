@@ -75,31 +75,40 @@ VY_DEVINL void mbar_wait(uint64_t* bar, uint32_t parity) {
   }
 }
 
-// GEMM flavour of the bounded wait: instead of trapping, a wait that times out raises a flag and returns; every other
+// Flavour of the bounded wait that does not trap: a wait that times out raises a flag and returns false; every other
 // wait of the SAME launch notices the flag within 64 attempts and returns too, so a protocol bug ends that kernel with
 // wrong results and a raised flag rather than with a fault or a hang. The flag holds the id of the launch that timed
 // out: waits of later launches compare it with their own id, so a stale flag never makes a healthy GEMM bail out.
-// `host` is the device address of a pinned host mirror the library reads without synchronising (every vy_gemm call
-// and vy_gemm_poison_peek() fail loudly once it is non-zero; vy_gemm_poisoned() lowers both).
+// `host` is the device address of a pinned host mirror the library reads without synchronising (the entry points whose kernels
+// wait like this and vy_gemm_poison_peek() fail loudly once it is non-zero; vy_gemm_poisoned() lowers both).
 struct PoisonRef {
   int* flag;  // device memory, one per device
   int* host;  // mapped pinned host memory, one per device
   int id;     // id of this launch (never 0)
 };
 bool poison_ref(PoisonRef* r);  // gemm.cu: the flags of the current device, a fresh launch id
+bool poison_raised(const char* who);  // gemm.cu: a wait on the current device has timed out and nobody has acknowledged it: sets the error message of `who`
 template <bool CLUSTER_SCOPE = false>
-VY_DEVINL void mbar_wait_soft(uint64_t* bar, uint32_t parity, const PoisonRef& poison) {
+VY_DEVINL bool mbar_wait_soft(uint64_t* bar, uint32_t parity, const PoisonRef& poison) {
   uint32_t spins = 0;
   while (!(CLUSTER_SCOPE ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity))) {
     if ((++spins & 63u) == 0) {
-      if (*reinterpret_cast<volatile int*>(poison.flag) == poison.id) return;
+      if (*reinterpret_cast<volatile int*>(poison.flag) == poison.id) return false;
       if (spins > (1u << 21)) {
         atomicExch(poison.flag, poison.id);
         *reinterpret_cast<volatile int*>(poison.host) = poison.id;
         __threadfence_system();
-        return;
+        return false;
       }
     }
+  }
+  return true;
+}
+// Behind a wait that timed out: the copies in flight to this CTA's `n` buffers are waited for (with a limit) before it leaves. issued: copies per buffer so far
+VY_DEVINL void mbar_drain(uint64_t* bars, const int* issued, int n) {
+  for (int b = 0; b < n; ++b) {
+    const int k = *reinterpret_cast<const volatile int*>(issued + b);
+    for (uint32_t spins = 0; k > 0 && spins < (1u << 20) && !mbar_try_wait(bars + b, (k - 1) & 1); ++spins) {}
   }
 }
 

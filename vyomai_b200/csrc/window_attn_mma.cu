@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
   float* qe = reinterpret_cast<float*>(Ts + NS * buf);   // powers of two that undo the scaling of the rows of Q
   uint64_t* full = reinterpret_cast<uint64_t*>(qe + R);  // a buffer's tile has arrived
   int* done = reinterpret_cast<int*>(full + NS);         // warps that are through with a buffer, counted up for ever
+  int* issued = done + NS;                               // tiles sent for into a buffer
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int s = blockIdx.z, h0 = blockIdx.y << hl, qn = R >> hl;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
     for (int x = lane; x < (N - nk) * (kb / 16); x += 32) *reinterpret_cast<uint4*>(T + nk * kb + 16 * x) = make_uint4(0, 0, 0, 0);
     __syncwarp();
     if (lane == 0) {
+      ++issued[b];
       mbar_arrive_expect_tx(&full[b], static_cast<unsigned>(nk) * w.row_bytes);
       for (int j = 0; j < nk;) {   // kept tokens and the band are a run each; kept tokens beyond the portion's own lie at the band's start
         const int c = c0 + j, kp = key_of(c);
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
   const int tiles = (count + N - 1) / N;
   if (threadIdx.x < NS) {
     mbar_init(&full[threadIdx.x], 1);
-    done[threadIdx.x] = 0;
+    done[threadIdx.x] = issued[threadIdx.x] = 0;
   }
   fence_mbar_init();
   __syncthreads();
@@ -175,14 +177,16 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
     big = big || !(fabsf(qmul[e]) * top_k <= SPLIT_SCORE);
   }
   if (__syncthreads_or(odd || big)) {   // not for fp16 halves: the fp32 form's
-    for (int b = 0; b < min(NS, tiles); ++b) mbar_wait_soft(&full[b], 0, poison);   // the copies in flight write to this CTA's memory
+    for (int b = 0; b < min(NS, tiles); ++b)   // the copies in flight write to this CTA's memory
+      if (!mbar_wait_soft(&full[b], 0, poison)) mbar_drain(full, issued, NS);
     if (threadIdx.x == 0) w.odd[s * d.kv_heads + g] = 1;
     return;
   }
   // from here on the warps wait for tiles, not for one another, so that one's softmax meets another's products
+  bool alive = true;   // no wait of this thread has timed out; lane 0 sends for tiles
   for (int it = 0; it < tiles; ++it) {
     const int c0 = it * N, b = it % NS;
-    mbar_wait_soft(&full[b], (it / NS) & 1, poison);
+    alive = mbar_wait_soft(&full[b], (it / NS) & 1, poison) && alive;
     const unsigned kb_h = kb_0 + b * buf, vb_h = vb_0 + b * buf;
     // 2^(exponent - SPLIT_TOP) of each key row, 2^exponent of each value row
     const int ustep = kb / 4;
@@ -322,7 +326,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
     int last = 0;
     if (lane == 0) {
       __threadfence_block();
-      last = atomicAdd(&done[b], 1) % NW == NW - 1;
+      last = atomicAdd(&done[b], 1) % NW == NW - 1 && alive;
       __threadfence_block();
       if (last) fence_proxy_async_smem();   // the reads of the buffer come before the copy that refills it
     }
@@ -355,6 +359,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
       }
     }
   }
+  if (__syncthreads_or(!alive)) mbar_drain(full, issued, NS);
 }
 
 static int round16(int n) { return (n + 15) & ~15; }
@@ -396,7 +401,7 @@ template <int MAXD, int VT, int NW, int N, int NS, bool SIG>
 static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int max_new, int hl, cudaStream_t st) {
   constexpr int R = 16 * NW;
   const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
-  const size_t smem = 2 * R * (dim16 * 2 + 16) + static_cast<size_t>(NS) * N * w.row_bytes + sizeof(float) * R + 12 * NS;
+  const size_t smem = 2 * R * (dim16 * 2 + 16) + static_cast<size_t>(NS) * N * w.row_bytes + sizeof(float) * R + 16 * NS;
   const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q, 16);
   const bool ovec = d.vdim % 2 == 0 && d.ld_out % 2 == 0 && al(d.out, d.out_dt == VY_BF16 ? 4 : 8);

@@ -58,6 +58,14 @@ def _stream() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
+def check_waits() -> None:
+    """Raises when a barrier wait inside an earlier kernel on this device has timed out: results since then are invalid. No synchronisation; for callers
+    that replay captured launches (a direct call of an op whose kernels wait checks by itself)."""
+    if _lib.lib().vy_gemm_poison_peek() == 1:
+        raise _lib.VyomError("a barrier wait inside an earlier kernel on this device timed out: results since then are invalid "
+                             "(vy_gemm_poisoned() acknowledges the flag)")
+
+
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 

@@ -415,6 +415,8 @@ class HybridBatchEngine:
         """work: [(sequence, new tokens)]; want[i]: offsets among sequence i's new tokens whose logits are returned
         (in order). Extends the sequences' pages, runs the model step, advances `num_cached`."""
         mgr = self.cache
+        if self.device.type == "cuda":
+            ops.check_waits()   # replayed steps call no op that would
         n = len(work)
         cu, pos0, slot, ids, rows = [0], [], [], [], []
         for (seq, toks), w in zip(work, want):
@@ -528,6 +530,8 @@ class HybridBatchEngine:
         work = [(s, s.tokens[s.num_cached:]) for s in seqs]
         logits = self._run(work, [[len(t) - 1] for _, t in work])
         nxt = ops.argmax_rows(logits).tolist()
+        if self.device.type == "cuda":
+            ops.check_waits()   # this step's, before its tokens count
         finished: Dict[int, List[int]] = {}
         for s, t in zip(seqs, nxt):
             s.tokens.append(int(t))
