@@ -430,6 +430,17 @@ def test_a_wait_that_timed_out_stops_what_would_use_its_results():
     assert lib().vy_gemm_poison_peek() == 0
 
 
+def test_causal_conv_over_very_many_channels():
+    """More channels than a launch has blocks of 128 for."""
+    from vyomai_b200 import ops
+    C = 65535 * 128 + 130
+    g = torch.Generator(device=DEV).manual_seed(2)
+    x, w, state = torch.randn(2, C, generator=g, device=DEV), torch.randn(C, 2, generator=g, device=DEV), torch.zeros(1, C, 1, device=DEV)
+    out = ops.causal_conv(ops.PackedBatch(_i32([0, 2]), _i32([0]), _i32([0]), 2), x, w, state, act=None)
+    assert torch.equal(state[0, :, 0], x[1]) and torch.equal(out[0], x[0] * w[:, 1])
+    assert float((out[1] - (x[1] * w[:, 1] + x[0] * w[:, 0])).abs().max()) < 1e-5
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

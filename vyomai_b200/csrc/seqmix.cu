@@ -495,6 +495,7 @@ struct ConvDev {
   float* state;
   int act;
   void* out; long long ld_out; int out_dt;
+  int first;   // first channel of the launch
 };
 constexpr int CONV_MAX_TAPS = 16;
 constexpr int CONV_TOK = 16;   // at least CONV_MAX_TAPS - 1: only the first CTA row of a sequence reaches back to the slot's taps
@@ -522,7 +523,7 @@ template <int TAPS>
 __global__ void __launch_bounds__(128) causal_conv_kernel(ConvDev d) {
   pdl_trigger();
   pdl_wait();
-  const int c = blockIdx.y * blockDim.x + threadIdx.x;
+  const int c = d.first + blockIdx.y * blockDim.x + threadIdx.x;
   const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
   if (c >= d.channels || i0 >= n) return;
@@ -1001,7 +1002,6 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   VY_CHECK_ARG(p->x && p->w && p->out && p->x != p->out && (p->state || p->taps == 1) && dtype_ok(p->x_dtype) && dtype_ok(p->w_dtype) &&
                    dtype_ok(p->out_dtype), "vy_causal_conv: bad tensors");
   VY_CHECK_ARG((p->max_new + 31) / 32 <= 65535, "vy_causal_conv: too many tokens per sequence");
-  VY_CHECK_ARG((p->channels + 127) / 128 <= 65535, "vy_causal_conv: too many channels");
   ConvDev d;
   d.cu = p->cu_tokens; d.pos0 = p->pos0; d.slot = p->slot;
   d.channels = p->channels; d.taps = p->taps;
@@ -1010,11 +1010,14 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   d.state = p->state; d.act = p->act;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
-  const int cb = (p->channels + 127) / 128;
-  const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, cb, p->n_seqs);
-  VY_CUDA_OK(p->taps <= 4 ? launch_kernel(causal_conv_kernel<4>, grid, dim3(128), 0, st, d) : launch_kernel(causal_conv_kernel<CONV_MAX_TAPS>, grid, dim3(128), 0, st, d));
-  VY_LAUNCH_OK();
-  count_launch();
+  const long long blocks = (p->channels + 127LL) / 128;
+  for (long long b = 0; b < blocks; b += 65535) {   // one launch, up to 8 million channels
+    d.first = static_cast<int>(128 * b);
+    const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, static_cast<unsigned>(blocks - b < 65535 ? blocks - b : 65535), p->n_seqs);
+    VY_CUDA_OK(p->taps <= 4 ? launch_kernel(causal_conv_kernel<4>, grid, dim3(128), 0, st, d) : launch_kernel(causal_conv_kernel<CONV_MAX_TAPS>, grid, dim3(128), 0, st, d));
+    VY_LAUNCH_OK();
+    count_launch();
+  }
   return VY_OK;
 }
 
