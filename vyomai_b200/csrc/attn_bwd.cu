@@ -624,12 +624,9 @@ extern "C" int vy_attn_bwd(const VyAttnBwd* p) {
   g.scale = 0.125f;
   g.scale_log2 = 1.4426950408889634f * 0.125f;
 
-  static bool attr_set = false;
-  if (!attr_set) {
-    VY_CUDA_OK(cudaFuncSetAttribute(attn_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AB_SMEM_DKDV));
-    VY_CUDA_OK(cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AB_SMEM_DQ));
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> allowed_dkdv{0}, allowed_dq{0};
+  VY_CUDA_OK(allow_smem(attn_bwd_dkdv_kernel, allowed_dkdv));
+  VY_CUDA_OK(allow_smem(attn_bwd_dq_kernel, allowed_dq));
   dim3 grid_kv((p->Skv + AB_T - 1) / AB_T, p->n_kv_heads, p->B);
   VY_CUDA_OK(launch_kernel(attn_bwd_dkdv_kernel, dim3(grid_kv), dim3(256), AB_SMEM_DKDV, st, tq, tk, tv, tdo, g));
   VY_LAUNCH_OK();

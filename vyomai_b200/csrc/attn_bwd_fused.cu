@@ -444,11 +444,8 @@ int attn_bwd_fused_launch(const VyAttnBwd* p) {
   g.scale = 0.125f;
   g.scale_log2 = 1.4426950408889634f * 0.125f;
 
-  static bool attr_set = false;
-  if (!attr_set) {
-    VY_CUDA_OK(cudaFuncSetAttribute(attn_bwd_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AF_SMEM));
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> allowed{0};
+  VY_CUDA_OK(allow_smem(attn_bwd_fused_kernel, allowed));
   dim3 grid(p->n_kv_heads, p->B);
   VY_CUDA_OK(launch_kernel(attn_bwd_fused_kernel, dim3(grid), dim3(AF_THREADS), AF_SMEM, static_cast<cudaStream_t>(p->stream), tq, tk, tv, tdo, g));
   VY_LAUNCH_OK();

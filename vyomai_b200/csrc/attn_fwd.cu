@@ -428,11 +428,8 @@ extern "C" int vy_attn_fwd(const VyAttn* p) {
   g.lse = p->lse;
   g.scale_log2 = 1.4426950408889634f / 8.0f;
 
-  static bool attr_set = false;
-  if (!attr_set) {
-    VY_CUDA_OK(cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM));
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> allowed{0};
+  VY_CUDA_OK(allow_smem(attn_fwd_kernel, allowed));
   dim3 grid((p->Sq + AT_BM - 1) / AT_BM, p->n_q_heads, p->B);
   VY_CUDA_OK(launch_kernel(attn_fwd_kernel, dim3(grid), dim3(256), AT_SMEM, static_cast<cudaStream_t>(p->stream), tq, tk, tv, g));
   VY_LAUNCH_OK();

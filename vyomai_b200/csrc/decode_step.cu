@@ -1100,10 +1100,8 @@ extern "C" int vy_decode_step(const VyDecodeStep* q) {
 #define DS_LAUNCH(NR)                                                                                        \
   do {                                                                                                       \
     auto kern = decode_step_kernel<NR>;                                                                      \
-    static std::once_flag once;                                                                              \
-    static cudaError_t attr_rc = cudaSuccess;                                                                \
-    std::call_once(once, [&] { attr_rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); }); \
-    VY_CUDA_OK(attr_rc);                                                                                     \
+    static std::atomic<unsigned long long> allowed{0};                                                       \
+    VY_CUDA_OK(allow_smem(kern, allowed));                                                                   \
     cudaLaunchConfig_t cfg;                                                                                  \
     memset(&cfg, 0, sizeof(cfg));                                                                            \
     cfg.gridDim = dim3(grid);                                                                                \

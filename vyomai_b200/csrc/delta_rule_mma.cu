@@ -517,12 +517,9 @@ int round32(int x) { return (x + 31) / 32 * 32; }
 template <int DP>
 cudaError_t launch(const RecDev& d, int n_seqs, int max_new, const DeltaChunks& w, cudaStream_t st) {
   const size_t smem = DC_NS * (DcBlob<DP>::bytes + DC_NW * 1024);
-  static bool once = false;
-  if (!once) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    once = true;
-  }
+  static std::atomic<unsigned long long> allowed{0};
+  cudaError_t ea = allow_smem(delta_scan_kernel<DP>, allowed);
+  if (ea != cudaSuccess) return ea;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
   cudaError_t e = launch_kernel(delta_chunk_kernel<DP>, dim3((max_new + DC_T - 1) / DC_T, d.heads, n_seqs), dim3(256), 0, st, d, w);

@@ -541,12 +541,9 @@ template <int RPL>
 static cudaError_t launch_gd_scan(const GdDev& d, int n_seqs, cudaStream_t st) {
   constexpr size_t smem = sizeof(float) * 2 * GdStage<RPL>::floats;
   if (smem > 48 * 1024) {
-    static bool once = false;
-    if (!once) {
-      cudaError_t e = cudaFuncSetAttribute(gd_scan_kernel<RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return e;
-      once = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t ea = allow_smem(gd_scan_kernel<RPL>, allowed);
+    if (ea != cudaSuccess) return ea;
   }
   return launch_kernel(gd_scan_kernel<RPL>, dim3((d.vdim + 31) / 32, d.heads, n_seqs), dim3(GD_T), smem, st, d);
 }

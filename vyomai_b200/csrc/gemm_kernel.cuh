@@ -1162,11 +1162,8 @@ int launch_gemm(const VyGemm* p, const GemmDev& g) {
   }
   auto kern = gemm_kernel<TIn, BN, A_MN, B_MN, PAIR, GATED>;
   constexpr int smem_bytes = PAIR ? Cfg::PAIR_SMEM_BYTES : Cfg::SMEM_BYTES;
-  static bool attr_set = false;  // per instantiation
-  if (!attr_set) {
-    VY_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> allowed{0};  // per instantiation
+  VY_CUDA_OK(allow_smem(kern, allowed));
   const int m_tiles = (p->M + Cfg::BM - 1) / Cfg::BM;
   const int n_tiles = (p->N + BN - 1) / BN;
   const int m_slots = PAIR ? (m_tiles + 1) / 2 : m_tiles;

@@ -665,14 +665,11 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + 128 + 64 + 4 * LM_C + 128) + 4 * sizeof(Range);
   const size_t q2 = 2 * LM_C * static_cast<size_t>(kb), vs = 2 * LM_C * LU_VB + 2 * static_cast<size_t>(dim16) * LU_VB;
   const size_t smem_o = q2 + (q2 > vs ? q2 : vs) + sizeof(float) * 7 * LM_C;
-  static bool once = false;
-  if (!once) {
-    cudaError_t e = cudaFuncSetAttribute(la_states_kernel<TD, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(la_outputs_kernel<TD, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
-    if (e != cudaSuccess) return e;
-    once = true;
-  }
-  cudaError_t e = launch_kernel(la_states_kernel<TD, ACT>, grid, dim3(LU_T), smem_u, st, d, w, hp, vslices, dim16, vec);
+  static std::atomic<unsigned long long> allowed_u{0}, allowed_o{0};
+  cudaError_t e = allow_smem(la_states_kernel<TD, ACT>, allowed_u);
+  if (e == cudaSuccess) e = allow_smem(la_outputs_kernel<TD, ACT>, allowed_o);
+  if (e != cudaSuccess) return e;
+  e = launch_kernel(la_states_kernel<TD, ACT>, grid, dim3(LU_T), smem_u, st, d, w, hp, vslices, dim16, vec);
   if (e != cudaSuccess) return e;
   const int each = d.dim * d.vdim;
   const bool quad = d.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(d.state) % 16 == 0 && reinterpret_cast<uintptr_t>(ws) % 16 == 0;

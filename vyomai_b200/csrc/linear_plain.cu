@@ -449,11 +449,8 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
     // from K = 256 on: below, a chain of FMAs is at least as exact (all terms positive, K 256: 2.5e-7 by FMAs, 2.1e-7 split; K 64: 1.2e-7, 2.1e-7), and the
     // two cost the same at 64 (9 us for 33 x 64)
     if (p->K >= 256 && p->K % 4 == 0 && rows16(d.A, d.a_dt, d.lda, batch > 1 ? d.a_batch : 0) && rows16(d.W, d.w_dt, d.ldw, batch > 1 ? d.w_batch : 0)) {
-      static bool once = false;
-      if (!once) {
-        VY_CUDA_OK(cudaFuncSetAttribute(linear_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * LS_BUF));
-        once = true;
-      }
+      static std::atomic<unsigned long long> allowed{0};
+      VY_CUDA_OK(allow_smem(linear_split_kernel, allowed));
       VY_CUDA_OK(launch_kernel(linear_split_kernel, dim3((p->N + LT - 1) / LT, (p->M + LT - 1) / LT, batch), dim3(256), 2 * LS_BUF, st, d));
       VY_LAUNCH_OK();
       count_launch();

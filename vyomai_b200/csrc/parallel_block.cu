@@ -361,12 +361,9 @@ static unsigned mix_threads(int width) {
 }
 
 static cudaError_t mix_smem_ok(size_t smem, bool mix) {
-  static size_t allowed[2] = {48 * 1024, 48 * 1024};
-  if (smem <= allowed[mix]) return cudaSuccess;
-  cudaError_t e = mix ? cudaFuncSetAttribute(vy::depth_mix_norm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))
-                      : cudaFuncSetAttribute(vy::depth_mix_norm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e == cudaSuccess) allowed[mix] = smem;
-  return e;
+  static std::atomic<unsigned long long> allowed[2];
+  if (smem <= 48 * 1024) return cudaSuccess;
+  return mix ? vy::allow_smem(vy::depth_mix_norm_kernel<true>, allowed[1]) : vy::allow_smem(vy::depth_mix_norm_kernel<false>, allowed[0]);
 }
 
 extern "C" int vy_layer_norm(const VyLayerNorm* p) {

@@ -276,11 +276,8 @@ extern "C" int vy_poly_norm(const VyPolyNorm* p) {
   if (p->width <= 1024) {
     VY_CUDA_OK(launch_kernel(poly_norm_kernel<128>, dim3(blocks), dim3(128), smem, st, d));
   } else {
-    static size_t allowed = 48 * 1024;
-    if (smem > allowed) {
-      VY_CUDA_OK(cudaFuncSetAttribute(poly_norm_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      allowed = smem;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    if (smem > 48 * 1024) VY_CUDA_OK(allow_smem(poly_norm_kernel<512>, allowed));
     VY_CUDA_OK(launch_kernel(poly_norm_kernel<512>, dim3(blocks), dim3(512), smem, st, d));
   }
   VY_LAUNCH_OK();

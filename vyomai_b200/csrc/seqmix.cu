@@ -1034,12 +1034,9 @@ static cudaError_t launch_delta_rule(const RecDev& d, int n_seqs, cudaStream_t s
   const size_t smem = sizeof(float) * (3 * CT * DP + CT + CT * 32);
   const int cols = 32;
   if (DP >= 256) {
-    static bool once = false;
-    if (!once) {
-      cudaError_t e = cudaFuncSetAttribute(delta_rule_kernel<DP, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-      if (e != cudaSuccess) return e;
-      once = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t ea = allow_smem(delta_rule_kernel<DP, PLAIN>, allowed);
+    if (ea != cudaSuccess) return ea;
   }
   return launch_kernel(delta_rule_kernel<DP, PLAIN>, dim3((d.vdim + cols - 1) / cols, d.heads, n_seqs), dim3(threads), smem, st, d);
 }

@@ -274,12 +274,9 @@ __global__ void __launch_bounds__(LA_T, OCC) linear_attn_chunk_kernel(RecDev d, 
 template <int DP, int VS, int OCC, bool TD = false>
 static cudaError_t launch_la(const RecDev& d, int n_seqs, cudaStream_t st) {
   constexpr size_t smem = sizeof(float) * LaSmem<DP, VS, TD>::floats;
-  static bool once = false;
-  if (!once) {
-    cudaError_t e = cudaFuncSetAttribute(linear_attn_chunk_kernel<DP, VS, OCC, TD>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    once = true;
-  }
+  static std::atomic<unsigned long long> allowed{0};
+  cudaError_t ea = allow_smem(linear_attn_chunk_kernel<DP, VS, OCC, TD>, allowed);
+  if (ea != cudaSuccess) return ea;
   const auto al = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
   const bool vec = d.in_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && al(d.q, d.ldq) && al(d.k, d.ldk) && al(d.v, d.ldv);
   return launch_kernel(linear_attn_chunk_kernel<DP, VS, OCC, TD>, dim3((d.vdim + VS - 1) / VS, d.heads, n_seqs), dim3(LA_T), smem, st, d, vec);
@@ -712,11 +709,10 @@ cudaError_t launch_window_attn_heads(const WinDev& d, int n_seqs, float* ws, lon
   const auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q);
   const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && d.k_row % 4 == 0 && d.v_row % 4 == 0 && al(d.kp) && al(d.vp);
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(window_attn_heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  static std::atomic<unsigned long long> allowed{0};
+  if (smem > 48 * 1024) {
+    cudaError_t e = allow_smem(window_attn_heads_kernel, allowed);
     if (e != cudaSuccess) return e;
-    allowed = smem;
   }
   const int per_kv = d.heads / d.kv_heads, tiles = (per_kv + WH_H - 1) / WH_H;
   // splits: enough CTAs for two per SM, at most one per 64 keys of the longest possible context, at most 16 and what the workspace holds
@@ -744,11 +740,10 @@ static cudaError_t launch_wt(const WinDev& d, int n_seqs, int max_new, const int
   const auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q);
   const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && d.k_row % 4 == 0 && d.v_row % 4 == 0 && al(d.kp) && al(d.vp);
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(window_attn_tiled_kernel<MV, BN, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  static std::atomic<unsigned long long> allowed{0};
+  if (smem > 48 * 1024) {
+    cudaError_t e = allow_smem(window_attn_tiled_kernel<MV, BN, SIG>, allowed);
     if (e != cudaSuccess) return e;
-    allowed = smem;
   }
   // behind the tensor-core form mostly nothing is left to do: two CTAs per SM, which walk the blocks of queries, cost less to launch than one per block
   const long long tiles = (max_new + WT_M - 1) / WT_M, most = (2LL * num_sms() + static_cast<long long>(d.heads) * n_seqs - 1) / (static_cast<long long>(d.heads) * n_seqs);

@@ -382,11 +382,10 @@ long long talk_attn_mma_floats(const TalkDev& d, int n_seqs, int max_new) {
 template <int HL, int N>
 static cudaError_t launch_talk_mma(const TalkDev& d, const SplitKv& w, int n_seqs, int max_new, cudaStream_t st) {
   const size_t smem = talk_mma_smem<HL, N>(d);
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(talk_attn_mma_kernel<HL, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  static std::atomic<unsigned long long> allowed{0};
+  if (smem > 48 * 1024) {
+    cudaError_t e = allow_smem(talk_attn_mma_kernel<HL, N>, allowed);
     if (e != cudaSuccess) return e;
-    allowed = smem;
   }
   const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q, 16);

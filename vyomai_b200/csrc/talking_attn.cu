@@ -545,11 +545,10 @@ static TiledPlan tiled_plan(const TalkDev& d, int dim4, int vdim4) {
 
 template <int NT, int RB, int MV, int KN>
 static cudaError_t launch_tiled_kn(const TalkDev& d, const TiledPlan& pl, int n_seqs, int max_new, int dim4, int vdim4, bool qvec, bool kvvec, cudaStream_t st) {
-  static size_t allowed = 48 * 1024;
-  if (pl.smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(talk_attn_tiled_kernel<NT, RB, MV, KN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pl.smem));
+  static std::atomic<unsigned long long> allowed{0};
+  if (pl.smem > 48 * 1024) {
+    cudaError_t e = allow_smem(talk_attn_tiled_kernel<NT, RB, MV, KN>, allowed);
     if (e != cudaSuccess) return e;
-    allowed = pl.smem;
   }
   return launch_kernel(talk_attn_tiled_kernel<NT, RB, MV, KN>, dim3((max_new + pl.TQ - 1) / pl.TQ, n_seqs), dim3(NT), pl.smem, st, d, pl.TQ, dim4, vdim4,
                        pl.ldq_s, pl.ldkv, qvec, kvvec);
@@ -651,11 +650,8 @@ extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   const int per = d.heads / d.kv_heads;
   const int hb = per % 4 == 0 ? 4 : per % 2 == 0 ? 2 : 1;
   auto kern = hb == 4 ? talk_attn_rows_kernel<4> : hb == 2 ? talk_attn_rows_kernel<2> : talk_attn_rows_kernel<1>;
-  static size_t allowed[3] = {48 * 1024, 48 * 1024, 48 * 1024};
-  if (smem > allowed[hb >> 1]) {
-    VY_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    allowed[hb >> 1] = smem;
-  }
+  static std::atomic<unsigned long long> allowed[3];
+  if (smem > 48 * 1024) VY_CUDA_OK(allow_smem(kern, allowed[hb >> 1]));
   int splits = rows_splits(p->n_seqs, p->max_new, p->table_width, p->block_size);
   const long long rows_bound = static_cast<long long>(p->n_seqs) * p->max_new;
   if (splits > 1) {

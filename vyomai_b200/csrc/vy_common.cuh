@@ -104,6 +104,22 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 }
 
 // ---- device: dtype-generic element access ---------------------------------------------------
+// More than 48 KB of dynamic shared memory has to be allowed per kernel AND per device. Allows `kern` all that the current device has beside its static share,
+// the first time on each device; `done`: a bit per device, one such word per kernel (both threads of a race set the same limit)
+template <typename... KArgs>
+inline cudaError_t allow_smem(void (*kern)(KArgs...), std::atomic<unsigned long long>& done) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  cudaFuncAttributes a;
+  if ((e = cudaFuncGetAttributes(&a, kern)) != cudaSuccess || (e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - static_cast<int>(a.sharedSizeBytes))) != cudaSuccess) return e;
+  done.fetch_or(bit, std::memory_order_release);
+  return cudaSuccess;
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

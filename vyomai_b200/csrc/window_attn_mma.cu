@@ -405,11 +405,10 @@ static cudaError_t launch_wm(const WinDev& d, const SplitKv& w, int n_seqs, int 
   const auto al = [](const void* p, int a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
   const bool qvec = d.q_dt == VY_F32 && d.dim % 4 == 0 && d.ldq % 4 == 0 && al(d.q, 16);
   const bool ovec = d.vdim % 2 == 0 && d.ld_out % 2 == 0 && al(d.out, d.out_dt == VY_BF16 ? 4 : 8);
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(window_attn_mma_kernel<MAXD, VT, NW, N, NS, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  static std::atomic<unsigned long long> allowed{0};
+  if (smem > 48 * 1024) {
+    cudaError_t e = allow_smem(window_attn_mma_kernel<MAXD, VT, NW, N, NS, SIG>, allowed);
     if (e != cudaSuccess) return e;
-    allowed = smem;
   }
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
