@@ -441,6 +441,34 @@ def test_causal_conv_over_very_many_channels():
     assert float((out[1] - (x[1] * w[:, 1] + x[0] * w[:, 0])).abs().max()) < 1e-5
 
 
+def test_scratch_that_cannot_be_had_is_done_without(monkeypatch):
+    """A device without room for a prompt form's scratch: the step takes the form that needs none. Attention in a smaller scratch: a few sequences at a time."""
+    from vyomai_b200 import ops
+    assert ops._lend(1 << 50, torch.device(DEV)) is None and ops._lend(0, torch.device(DEV)) is None
+    g = torch.Generator(device=DEV).manual_seed(6)
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    new, bs, H = [70, 33, 130, 5], 16, 8
+    cu = [sum(new[:i]) for i in range(5)]
+    q, k, v, a, b = (R(cu[4], w) for w in (H * 32, H * 32, H * 32, H * 32, H))
+    kp, vp = R(40, bs, 2, 32), R(40, bs, 2, 32)
+    batch = ops.PackedBatch(_i32(cu), _i32([0, 20, 0, 30]), _i32([0, 1, 2, 3]), 130, torch.arange(40, dtype=torch.int32, device=DEV).view(4, 10), bs)
+    x = {n: R(cu[4], w) for n, w in (("x", H * 32), ("b", 64), ("c", 64), ("dt", H), ("gate", H * 32))}
+    ssd = dict(conv_w=R(H * 32 + 128, 3), conv_b=None, dt_bias=R(H), a_log=R(H), skip=R(H), norm=R(H * 32), heads=H, groups=2, dim=32, vdim=32, taps=3, norm_groups=H, norm_eps=1e-5)
+    calls = [lambda: ops.window_attn(batch, q, kp, vp, heads=H, kv_heads=2, dim=32, vdim=32, scale=0.2, window=40, keep_first=3),
+             lambda: ops.talk_attn(batch, q, kp, vp, heads=H, kv_heads=2, dim=32, vdim=32, scale=0.2, softcap=9.0, zero_sink=True),
+             lambda: ops.linear_attn(batch, q, k, v, torch.full((H,), 0.9, device=DEV), torch.zeros(4, H, 32, 32, device=DEV), heads=H, dim=32, vdim=32),
+             lambda: ops.delta_rule(batch, q, k, v, a, b, torch.zeros(H, device=DEV), torch.zeros(4, H, 32, 32, device=DEV), heads=H, kv_heads=H, dim=32, vdim=32),
+             lambda: ops.ssd(batch, **x, **ssd, conv_state=torch.zeros(4, 3, H * 32 + 128, device=DEV), state=torch.zeros(4, H, 32, 32, device=DEV),
+                             tickets=torch.zeros(4, 1, dtype=torch.int32, device=DEV))]
+    whole = [c() for c in calls]
+    monkeypatch.setattr(ops, "_prompt_attn_floats", lambda one, n_seqs: one)   # one sequence at a time
+    for c, want in zip(calls[:2], whole):
+        assert torch.equal(c(), want)
+    monkeypatch.setattr(ops, "_lend", lambda floats, device: None)
+    for c, want in zip(calls, whole):
+        assert float((c() - want).norm() / want.norm()) < 4 * BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -612,25 +612,33 @@ extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   const bool kvvec = d.pool_dt == VY_F32 && d.dim % 4 == 0 && d.vdim % 4 == 0 && al(d.kp) && al(d.vp);
   const TiledPlan pl = tiled_plan(d, dim4, vdim4);
   // prompts: the tensor-core form where the geometry suits it and the scratch is lent (16 tokens fill its 16-row products), the tiles behind it for what it leaves
+  const auto tiles = [&](const TalkDev& e, int n_seqs) {
+    if (pl.NT == 512) return pl.MV == 1 ? launch_tiled<512, 2, 1>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
+                                        : launch_tiled<512, 2, 2>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
+    if (pl.RB == 1) return pl.MV == 1 ? launch_tiled<256, 1, 1>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
+                                      : launch_tiled<256, 1, 2>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
+    return pl.MV == 1 ? launch_tiled<256, 2, 1>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
+                      : launch_tiled<256, 2, 2>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
+  };
   if (p->max_new >= TALK_MMA_MIN && p->force_form != 1 && pl.ok && p->workspace && al(p->workspace)) {
-    const long long need = talk_attn_mma_floats(d, p->n_seqs, p->max_new);
-    if (need > 0 && p->workspace_floats >= need) {
-      VY_CUDA_OK(launch_talk_attn_mma(d, p->n_seqs, p->max_new, p->workspace, &d.odd, st));
+    const long long one = talk_attn_mma_floats(d, 1, p->max_new), fit = one > 0 ? p->workspace_floats / one : 0;
+    for (int s = 0; fit > 0 && s < p->n_seqs;) {   // as many sequences at a time as the workspace holds
+      const int ns = static_cast<int>(fit < p->n_seqs - s ? fit : p->n_seqs - s);
+      TalkDev e = d;
+      e.cu += s;
+      e.pos0 += s;
+      e.table += static_cast<long long>(s) * d.tw;
+      VY_CUDA_OK(launch_talk_attn_mma(e, ns, p->max_new, p->workspace, &e.odd, st));
+      VY_CUDA_OK(tiles(e, ns));
       VY_LAUNCH_OK();
-      count_launch(2);
+      count_launch(3);
+      s += ns;
     }
+    if (fit > 0) return VY_OK;
   }
   VY_CHECK_ARG(p->force_form != 2 || pl.ok, "vy_talk_attn: the tiled form takes heads <= 64 and vdim <= 128 within 200 KB of shared memory");
-  const bool tiled = p->force_form == 2 || (p->force_form == 0 && pl.ok && p->max_new >= 8);
-  if (tiled) {
-    cudaError_t e;
-    if (pl.NT == 512) e = pl.MV == 1 ? launch_tiled<512, 2, 1>(d, pl, p->n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
-                                     : launch_tiled<512, 2, 2>(d, pl, p->n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
-    else if (pl.RB == 1) e = pl.MV == 1 ? launch_tiled<256, 1, 1>(d, pl, p->n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
-                                        : launch_tiled<256, 1, 2>(d, pl, p->n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
-    else e = pl.MV == 1 ? launch_tiled<256, 2, 1>(d, pl, p->n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
-                        : launch_tiled<256, 2, 2>(d, pl, p->n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
-    VY_CUDA_OK(e);
+  if (p->force_form == 2 || (p->force_form == 0 && pl.ok && p->max_new >= 8)) {
+    VY_CUDA_OK(tiles(d, p->n_seqs));
     VY_LAUNCH_OK();
     count_launch();
     return VY_OK;

@@ -1124,8 +1124,26 @@ def kv_page_write(batch: PackedBatch, k: torch.Tensor, v: torch.Tensor, k_pool: 
 ATTN_WEIGHTS = {"softmax": C["VY_ATTN_SOFTMAX"], "sigmoid": C["VY_ATTN_SIGMOID"]}
 
 
-WINDOW_ATTN_WORKSPACE_FLOATS = 1 << 27   # 512 MB: the host only knows the longest portion and table, so a step that mixes one long prompt with many
-#                                          short portions asks for far more than its rows fill; past this the kernel splits rows tile by tile
+def _lend(floats: int, device) -> Optional[torch.Tensor]:
+    """Scratch for a form that a step can do without: None where none is asked for, or where the device has no room for it (the step then takes the form
+    that needs none, instead of failing for want of memory)."""
+    if floats <= 0:
+        return None
+    try:
+        return torch.empty(floats, device=device, dtype=torch.float32)
+    except torch.OutOfMemoryError:
+        return None
+
+
+# What a step lends its prompt attention at most (512 MB): the host only knows the longest portion and table, so a step that mixes one long prompt with many short
+# portions asks for far more than its rows fill. Past it the kernels go through the sequences a few at a time (32 sequences, 31 of them with one token on 2000 cached
+# ones: 216 us at once, 385 in two goes)
+PROMPT_ATTN_FLOATS = 1 << 27
+
+
+def _prompt_attn_floats(one: int, n_seqs: int) -> int:
+    """one: what one sequence of the step asks for."""
+    return one * min(n_seqs, PROMPT_ATTN_FLOATS // one) if one > 0 else 0
 
 
 def window_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, *, heads: int, kv_heads: int, dim: int,
@@ -1151,9 +1169,9 @@ def window_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_poo
         need = int(_lib.lib().vy_window_attn_workspace_floats(batch.n_seqs, heads, kv_heads, vdim))
         ws = torch.empty(need, device=q.device, dtype=torch.float32) if need > 0 else None
     elif batch.max_new > 1 and batch.block_table is not None:   # prompts: the visible rows split for the tensor cores, once
-        need = int(_lib.lib().vy_window_attn_prompt_floats(batch.n_seqs, batch.max_new, batch.block_table.shape[1], batch.block_size, kv_heads, dim, vdim,
-                                                           int(window), int(keep_first), int(chunk)))
-        ws = torch.empty(need, device=q.device, dtype=torch.float32) if 0 < need <= WINDOW_ATTN_WORKSPACE_FLOATS else None
+        one = int(_lib.lib().vy_window_attn_prompt_floats(1, batch.max_new, batch.block_table.shape[1], batch.block_size, kv_heads, dim, vdim,
+                                                          int(window), int(keep_first), int(chunk)))
+        ws = _lend(_prompt_attn_floats(one, batch.n_seqs), q.device)
     _lib.call("vy_window_attn", "VyWinAttn", workspace=_ptr(ws), workspace_floats=ws.numel() if ws is not None else 0, q=q.data_ptr(), ldq=q.stride(0), q_dtype=_dt(q), k_pool=k_pool.data_ptr(),
               v_pool=v_pool.data_ptr(), pool_dtype=_dt(k_pool), heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=float(scale),
               window=int(window), keep_first=int(keep_first), sink=_ptr(sink), sink_dtype=_dt(sink) if sink is not None else 0,
@@ -1354,9 +1372,10 @@ def talk_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_pool:
     tw = batch.block_table.shape[1] if batch.block_table is not None else 0
     need = int(_lib.lib().vy_talk_attn_workspace_floats(batch.n_seqs, batch.max_new, tw, batch.block_size, heads, vdim)) if form != "tiled" else 0
     if form is None and batch.max_new > 1:   # prompts: the visible rows split for the tensor cores
-        more = int(_lib.lib().vy_talk_attn_prompt_floats(batch.n_seqs, batch.max_new, tw, batch.block_size, heads, kv_heads, dim, vdim, int(window)))
-        need = max(need, more if more <= WINDOW_ATTN_WORKSPACE_FLOATS else 0)
-    ws = torch.empty(need, device=q.device, dtype=torch.float32) if need > 0 else None
+        one = int(_lib.lib().vy_talk_attn_prompt_floats(1, batch.max_new, tw, batch.block_size, heads, kv_heads, dim, vdim, int(window)))
+        need = max(need, _prompt_attn_floats(one, batch.n_seqs))
+    ws = _lend(need, q.device)
+    need = ws.numel() if ws is not None else 0
     _lib.call("vy_talk_attn", "VyTalkAttn", q=q.data_ptr(), ldq=q.stride(0), q_dtype=_dt(q), k_pool=k_pool.data_ptr(), v_pool=v_pool.data_ptr(),
               pool_dtype=_dt(k_pool), heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=float(scale), softcap=float(softcap), window=int(window),
               talk=_ptr(talk), talk_dtype=_dt(talk) if talk is not None else 0, sink=_ptr(sink), sink_dtype=_dt(sink) if sink is not None else 0,
@@ -1448,8 +1467,8 @@ def linear_attn(batch: PackedBatch, q: torch.Tensor, k: torch.Tensor, v: torch.T
     need = 0
     if batch.max_new > 1:
         need = int(_lib.lib().vy_linear_attn_workspace_floats(q.shape[0], batch.n_seqs, batch.max_new, heads, dim, vdim))
-    ws = torch.empty(need, device=q.device, dtype=torch.float32) if need > 0 else None
-    _lib.call("vy_linear_attn", "VyLinAttn", rows=q.shape[0], workspace=_ptr(ws), workspace_floats=need, q=q.data_ptr(), ldq=q.stride(0), k=k.data_ptr(), ldk=k.stride(0), v=v.data_ptr(), ldv=v.stride(0),
+    ws = _lend(need, q.device)
+    _lib.call("vy_linear_attn", "VyLinAttn", rows=q.shape[0], workspace=_ptr(ws), workspace_floats=need if ws is not None else 0, q=q.data_ptr(), ldq=q.stride(0), k=k.data_ptr(), ldk=k.stride(0), v=v.data_ptr(), ldv=v.stride(0),
               in_dtype=_dt(q), in_act=UACT[in_act], heads=heads, dim=dim, vdim=vdim, decay=decay.data_ptr(), state=state.data_ptr(),
               out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out), stream=_stream(), **batch._kw())
     return out
@@ -1469,7 +1488,9 @@ def delta_rule(batch: PackedBatch, q: torch.Tensor, k: torch.Tensor, v: torch.Te
     need = 0
     if batch.max_new > 1:
         need = int(_lib.lib().vy_delta_rule_prompt_floats(rows, batch.n_seqs, batch.max_new, heads, dim, vdim))
-    ws = torch.empty(need or rows * (2 * kv_heads * dim + heads * dim + heads), device=q.device, dtype=torch.float32)   # unit q / k, decays, strengths
+    ws = _lend(need, q.device)
+    if ws is None:
+        ws = torch.empty(rows * (2 * kv_heads * dim + heads * dim + heads), device=q.device, dtype=torch.float32)   # unit q / k, decays, strengths
     _lib.call("vy_delta_rule", "VyDeltaRule", rows=rows, workspace=ws.data_ptr(), workspace_floats=ws.numel(), q=q.data_ptr(), ldq=q.stride(0), k=k.data_ptr(), ldk=k.stride(0), v=v.data_ptr(), ldv=v.stride(0),
               in_dtype=_dt(q), a=a.data_ptr(), ld_a=a.stride(0), a_dtype=_dt(a), b=b.data_ptr(), ld_b=b.stride(0), b_dtype=_dt(b),
               a_log=a_log.data_ptr(), a_log_dtype=_dt(a_log), heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, unit_eps=float(unit_eps),
@@ -1561,7 +1582,10 @@ def ssd(batch: PackedBatch, x: torch.Tensor, b: torch.Tensor, c: torch.Tensor, d
     rows = x.shape[0]
     out = torch.empty((rows, _round_up(inner, 8)), device=x.device, dtype=out_dtype or torch.float32)[:, :inner]
     need = int(_lib.lib().vy_ssd_workspace_floats(rows, batch.n_seqs, batch.max_new, heads, groups, dim, vdim))
-    ws = torch.empty(need, device=x.device, dtype=torch.float32)
+    ws = _lend(need, x.device)
+    if ws is None:   # without the chunks' states
+        need -= int(_lib.lib().vy_linear_attn_workspace_floats(rows, batch.n_seqs, batch.max_new, heads, dim, vdim))
+        ws = torch.empty(need, device=x.device, dtype=torch.float32)
     _lib.call("vy_ssd", "VySsd", rows=rows, x=x.data_ptr(), ldx=x.stride(0), b=b.data_ptr(), ldb=b.stride(0), c=c.data_ptr(), ldc=c.stride(0), dt=dt.data_ptr(),
               ld_dt=dt.stride(0), gate=_ptr(gate), ld_gate=gate.stride(0) if gate is not None else 0, gate_act=UACT[gate_act], conv_w=conv_w.data_ptr(),
               conv_b=_ptr(conv_b), taps=taps, conv_state=conv_state.data_ptr(), dt_bias=dt_bias.data_ptr(), a_log=a_log.data_ptr(), skip=skip.data_ptr(),
