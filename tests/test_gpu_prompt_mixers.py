@@ -469,6 +469,18 @@ def test_scratch_that_cannot_be_had_is_done_without(monkeypatch):
         assert float((c() - want).norm() / want.norm()) < 4 * BOUND
 
 
+def test_a_forced_form_is_taken_with_scratch_too(monkeypatch):
+    """A caller that forces the tiled form of the score-exchanging attention and lends scratch gets the tiled form."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(9)
+    q, kp, vp = torch.randn(64, 8 * 32, generator=g, device=DEV), torch.randn(4, 16, 2, 32, generator=g, device=DEV), torch.randn(4, 16, 2, 32, generator=g, device=DEV)
+    batch = ops.PackedBatch(_i32([0, 64]), _i32([0]), _i32([0]), 64, _i32([[0, 1, 2, 3]]), 16)
+    call = lambda: ops.talk_attn(batch, q, kp, vp, heads=8, kv_heads=2, dim=32, vdim=32, scale=0.2, softcap=9.0, form="tiled")  # noqa: E731
+    want, real, ws = call(), ops._lib.call, torch.empty(1 << 22, device=DEV)
+    monkeypatch.setattr(ops._lib, "call", lambda fn, st, **kw: real(fn, st, **{**kw, "workspace": ws.data_ptr(), "workspace_floats": ws.numel()}))
+    assert torch.equal(call(), want)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -620,7 +620,7 @@ extern "C" int vy_talk_attn(const VyTalkAttn* p) {
     return pl.MV == 1 ? launch_tiled<256, 2, 1>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st)
                       : launch_tiled<256, 2, 2>(e, pl, n_seqs, p->max_new, dim4, vdim4, qvec, kvvec, st);
   };
-  if (p->max_new >= TALK_MMA_MIN && p->force_form != 1 && pl.ok && p->workspace && al(p->workspace)) {
+  if (p->max_new >= TALK_MMA_MIN && p->force_form == 0 && pl.ok && p->workspace && al(p->workspace)) {
     const long long one = talk_attn_mma_floats(d, 1, p->max_new), fit = one > 0 ? p->workspace_floats / one : 0;
     for (int s = 0; fit > 0 && s < p->n_seqs;) {   // as many sequences at a time as the workspace holds
       const int ns = static_cast<int>(fit < p->n_seqs - s ? fit : p->n_seqs - s);
