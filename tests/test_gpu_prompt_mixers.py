@@ -481,6 +481,19 @@ def test_a_forced_form_is_taken_with_scratch_too(monkeypatch):
     assert torch.equal(call(), want)
 
 
+@pytest.mark.parametrize("width,ff,experts,top,form,rows,want", [(1024, 256, 28, 3, "swiglu", 1024, False), (1024, 256, 28, 3, "swiglu", 4096, True), (512, 128, 28, 3, "swiglu", 4096, False),
+                                                                 (1024, 512, 8, 2, "glu", 768, False), (1024, 512, 8, 2, "glu", 2048, True), (1024, 256, 16, 2, "plain", 1024, False),
+                                                                 (1024, 256, 16, 2, "plain", 4096, True)])
+def test_fp32_experts_are_sorted_where_that_is_faster(width, ff, experts, top, form, rows, want):
+    """The estimate against what was measured (both forms at these sizes, the slower one at least a fifth behind)."""
+    from vyomai_b200.layers.mixers import MoEFeedForward
+    w = {"router": torch.zeros(experts, width, device=DEV)}
+    for e in range(experts):
+        w.update({f"e{e}.{k}": torch.zeros(ff, width, device=DEV) for k in (("up",) if form == "plain" else ("up", "gate"))})
+        w[f"e{e}.down"] = torch.zeros(width, ff, device=DEV)
+    assert MoEFeedForward(w, experts, top, 1.0, torch.float32, True, router="softmax", form=form)._sorted_is_faster(rows) is want
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -776,8 +776,10 @@ class MoEFeedForward:
     the multiply-adds: a step of at least `sorted_min_rows` rows takes the sorted form when its estimated time is the smaller one
     (`force_sorted` skips the estimate)."""
 
-    TC_RATE, FMA_RATE = 1.0e15, 2.0e13   # multiply-add rates the estimate assumes for bf16 tensor-core and fp32 FMA products (FLOP/s)
-    LAUNCH_COST = 15e-6                   # host time of one product issued from Python (s): what bounds many small launches
+    # multiply-add rates the estimate assumes for bf16 tensor-core products, fp32 ones on the tensor cores (vy_linear_plain, contractions of 256 and more) and FMA
+    # ones (FLOP/s)
+    TC_RATE, SPLIT_RATE, FMA_RATE = 1.0e15, 6.3e13, 2.0e13
+    LAUNCH_COST = 15e-6                   # host time of one launch issued from Python (s): what bounds many small launches
 
     def __init__(self, w: Dict[str, torch.Tensor], experts: int, top: int, route_scale: float, act_dtype: torch.dtype, tensor_cores: bool,
                  act: str = "relu2", shared: bool = False, sorted_min_rows: int = 128, force_sorted: bool = False, router: str = "sigmoid",
@@ -828,10 +830,14 @@ class MoEFeedForward:
 
     def _sorted_is_faster(self, rows: int) -> bool:
         width = self.down_all.out_features
-        rate = self.TC_RATE if self.up_all.tensor_cores and self.act_dtype == torch.bfloat16 else self.FMA_RATE
+        fp32 = self.act_dtype == torch.float32
+        rate = self.TC_RATE if self.up_all.tensor_cores and not fp32 else self.SPLIT_RATE if fp32 and width >= 256 else self.FMA_RATE
+        # fp32, us, sorted / all experts (28 experts of 256, top 3, width 1024): 512 rows 1367 / 474, 1024 1381 / 797, 1536 1391 / 1183, 2048 1401 / 1522; 8 of 512, top 2:
+        # 768 rows 510 / 422, 1024 512 / 482, 1536 529 / 701
+        launches = self.experts * (3 if fp32 and self.glu else 2)   # an fp32 gate has a launch of its own
         per_choice = (6.0 if self.glu else 4.0) * rows * self.ff * width / rate   # up (+ gate) + down multiply-adds of one expert-sized slice over all rows
         moved = 3.0 * rows * self.top * width * 4 / 2.0e12   # gather, per-pair results, combine
-        return self.top * per_choice + 2 * self.experts * self.LAUNCH_COST + moved < self.experts * per_choice
+        return self.top * per_choice + launches * self.LAUNCH_COST + moved < self.experts * per_choice
 
     def _hidden(self, proj: Projection, x: torch.Tensor, dense: Optional[torch.Tensor], experts: int, shared_ff: int, sg, wide: bool) -> torch.Tensor:
         """The activated (and, with `dense`, weighted) hidden rows of `experts` experts and / or the shared expert, in the activation dtype."""
