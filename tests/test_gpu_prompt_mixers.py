@@ -494,6 +494,38 @@ def test_fp32_experts_are_sorted_where_that_is_faster(width, ff, experts, top, f
     assert MoEFeedForward(w, experts, top, 1.0, torch.float32, True, router="softmax", form=form)._sorted_is_faster(rows) is want
 
 
+@pytest.mark.parametrize("form,H,G,d,dv,window,keep", [("softmax", 4, 4, 96, 128, 33, 5), ("sigmoid", 4, 4, 128, 72, 0, 0), ("softmax", 8, 2, 128, 128, 70, 0), ("sigmoid", 8, 2, 40, 100, 33, 5)])
+def test_prompt_attention_in_blocks_of_192_rows(form, H, G, d, dv, window, keep):
+    """Enough sequences of odd length for the wide form (window_attn_mma.cu: two rounds of its CTAs over the SMs), from position 0 and carried on."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(d)
+    new = [193, 47, 49, 16, 97, 1] * 7
+    pos0 = [(29 * i) % 90 for i in range(len(new))]
+    rep = H // G
+    hl = min(4, rep.bit_length() - 1)
+    qn = 192 >> hl
+    assert (max(new) + qn - 1) // qn * (H >> hl) * len(new) >= 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    T = [n + p for n, p in zip(new, pos0)]
+    q, k, v = ([torch.randn(t, n, w, generator=g) / d ** (0.25 if i < 2 else 0) for t in T] for i, (n, w) in enumerate(((H, d), (G, d), (G, dv))))
+    want, bs = [], 16
+    for s, t in enumerate(T):
+        i, j = torch.arange(pos0[s], t)[:, None], torch.arange(t)[None, :]
+        seen = (j <= i) & ((i - j < window) | (j < keep)) if window else j <= i
+        kk, vv = (x[s].double().repeat_interleave(rep, 1) for x in (k, v))
+        sc = torch.einsum("ihd,jhd->hij", q[s][pos0[s]:].double(), kk)
+        p = torch.softmax(sc.masked_fill(~seen, -torch.inf), 2) if form == "softmax" else torch.sigmoid(sc) * seen
+        want.append(torch.einsum("hij,jhd->ihd", p, vv).reshape(new[s], -1))
+    batch, table, _, n_blocks, _ = shuffled_batch(new, pos0, bs, DEV, seed=d)
+    kp, vp = torch.full((n_blocks, bs, G, d), 1e3), torch.full((n_blocks, bs, G, dv), 1e3)
+    for s, t in enumerate(T):
+        at = torch.arange(t)
+        rows = torch.tensor([table[s][p // bs] for p in range(t)])
+        kp[rows, at % bs], vp[rows, at % bs] = k[s], v[s]
+    got = ops.window_attn(batch, torch.cat([q[s][pos0[s]:].reshape(new[s], -1) for s in range(len(new))]).to(DEV), kp.to(DEV), vp.to(DEV), heads=H, kv_heads=G, dim=d, vdim=dv,
+                          scale=1.0, window=window, keep_first=keep, weights=form, out_dtype=torch.float32)
+    assert _err(got, torch.cat(want)) < BOUND
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""
