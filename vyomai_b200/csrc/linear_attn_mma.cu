@@ -11,8 +11,8 @@
 // split, and their scores computed, once per group.
 //
 // The fp16 halves are off by at most 2^-49 of the largest entry under their unit, a row of q, k or v or a whole state. la_states looks at the rows (tokens) and
-// columns (channels) of every chunk's q, k and v and of the state that is carried in: where the largest entry of one is below 2^-20 of the largest of all
-// (a column of fewer than 8 tokens, whose entries may all be small by chance: 2^-24; zeros aside), and where an infinity or NaN is among them, the
+// columns (channels) of every chunk's q, k and v, as each warp has them, and of the state that is carried in: where the largest entry of one is below 2^-20 of the
+// largest of all (rows and columns of few entries, which may all be small by chance: 2^-24; zeros aside), and where an infinity or NaN is among them, the
 // heads of the CTA are left to the walk, which runs behind the three launches and starts from the state that la_scan kept as the one before the first chunk.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
@@ -116,12 +116,11 @@ __device__ __forceinline__ void note_warp(Range* to, Range r) {   // to: shared 
 }
 __device__ __forceinline__ bool too_wide(Range r) { return r.top >= 0x7f800000u || __uint_as_float(r.low) < 0x1p-20f * __uint_as_float(r.top); }
 
-// A thread's N quads of four columns, of rows STEP apart: each column's largest over all rows (lanes that share the columns differ in bits FROM and above), noted;
-// each row's largest into rows_s (bits; zero before)
-template <int N, int STEP, int FROM>
-__device__ __forceinline__ uint4 look(const float4 (&x)[N], unsigned* rows_s, bool few, Range& r) {
+// A warp's tile, a thread's N quads of it: FROM lanes share a row, 4 FROM columns. Notes the largest entry of each row and of each column (few_rows, few_columns: all
+// may be small by chance) and returns the columns'
+template <int N, int FROM>
+__device__ __forceinline__ uint4 look(const float4 (&x)[N], bool few_rows, bool few_columns, Range& r) {
   uint4 m = make_uint4(0u, 0u, 0u, 0u);
-  const int lane = threadIdx.x & 31, row = lane / FROM;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const uint4 a = make_uint4(abs_bits(x[i].x), abs_bits(x[i].y), abs_bits(x[i].z), abs_bits(x[i].w));
@@ -129,16 +128,16 @@ __device__ __forceinline__ uint4 look(const float4 (&x)[N], unsigned* rows_s, bo
     unsigned most = max(max(a.x, a.y), max(a.z, a.w));
 #pragma unroll
     for (int k = 1; k < FROM; k <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, k));
-    if ((lane & (FROM - 1)) == 0) atomicMax(rows_s + row + STEP * i, most);
+    note(r, most, few_columns);
   }
 #pragma unroll
   for (int k = FROM; k < 32; k <<= 1)
     m = make_uint4(max(m.x, __shfl_xor_sync(0xffffffffu, m.x, k)), max(m.y, __shfl_xor_sync(0xffffffffu, m.y, k)), max(m.z, __shfl_xor_sync(0xffffffffu, m.z, k)),
                    max(m.w, __shfl_xor_sync(0xffffffffu, m.w, k)));
-  note(r, m.x, few);
-  note(r, m.y, few);
-  note(r, m.z, few);
-  note(r, m.w, few);
+  note(r, m.x, few_rows);
+  note(r, m.y, few_rows);
+  note(r, m.z, few_rows);
+  note(r, m.w, few_rows);
   return m;
 }
 __device__ __forceinline__ float4 column_units(uint4 m) {   // 2^(exponent - SPLIT_TOP) of each column
@@ -170,15 +169,13 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
   float* es = reinterpret_cast<float*>(Wl + LM_C * LU_VB);   // [64] decay to the chunk's end times write strength
   float* ku = es + LM_C;                                     // [128], [64]: units of k's channels and of w's columns
   float* wu = ku + 128;
-  unsigned* rows_s = reinterpret_cast<unsigned*>(wu + 64);   // [4][64] rows' largest: k, q, v of even and of odd heads; [128] of the state
-  Range* range = reinterpret_cast<Range*>(rows_s + 4 * LM_C + 128);   // [4]: k, q, v, state
+  Range* range = reinterpret_cast<Range*>(wu + 64);          // [4]: k, q, v, state
   const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
   const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LM_C;
   if (t0 >= n) return;
   const int nt = min(LM_C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
   const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
   const long long r0 = base + t0, slot = la_slot(d, s, c);
-  for (int i = t; i < 4 * LM_C + 128; i += LU_T) rows_s[i] = 0u;
   if (t < 4) range[t] = {0u, RANGE_NONE};
   __syncthreads();
   const bool few = nt < 8;
@@ -196,11 +193,11 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
     Range rk = {0u, RANGE_NONE}, rq = rk;
     if (v0 == 0) {
       read(d.q, d.ldq);
-      look<8, 8, 4>(x, rows_s + LM_C, few, rq);
+      look<8, 4>(x, few, d.dim - 16 * warp < 4, rq);
       note_warp(range + 1, rq);
     }
     read(d.k, d.ldk);
-    const uint4 m = look<8, 8, 4>(x, rows_s, few, rk);
+    const uint4 m = look<8, 4>(x, few, d.dim - 16 * warp < 4, rk);
     note_warp(range, rk);
     const float4 sc = column_scales(m);
     if (row == 0) *reinterpret_cast<float4*>(ku + ch) = column_units(m);
@@ -238,48 +235,37 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
     float4 y[4] = {next[0], next[1], next[2], next[3]};
     if (h + 1 < h0 + hp) fetch(h + 1);   // in flight during this head's products
     __syncthreads();
-    unsigned* vrows = rows_s + (2 + ((h - h0) & 1)) * LM_C;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (row + 16 * i < nt) y[i] = act4<ACT>(y[i], d.in_act);
     }
-    look<4, 16, 2>(y, vrows, few, rv);
-    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+    uint4 m = look<4, 2>(y, few, vw - 8 * warp < 4, rv);
+    {   // the weighted columns' units from a bound, the columns' largest times the largest weight: rows are within 2^20 of one another, and the halves good to 2^24
+      const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, max(abs_bits(es[lane]), abs_bits(es[lane + 32]))));
+      const auto times = [most](unsigned b) { return __float_as_uint(__uint_as_float(b) * most); };
+      m = make_uint4(times(m.x), times(m.y), times(m.z), times(m.w));
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float e = es[row + 16 * i];
       y[i] = make_float4(y[i].x * e, y[i].y * e, y[i].z * e, y[i].w * e);
-      m = make_uint4(max(m.x, abs_bits(y[i].x)), max(m.y, abs_bits(y[i].y)), max(m.z, abs_bits(y[i].z)), max(m.w, abs_bits(y[i].w)));
     }
-#pragma unroll
-    for (int k = 2; k < 32; k <<= 1)
-      m = make_uint4(max(m.x, __shfl_xor_sync(0xffffffffu, m.x, k)), max(m.y, __shfl_xor_sync(0xffffffffu, m.y, k)), max(m.z, __shfl_xor_sync(0xffffffffu, m.z, k)),
-                     max(m.w, __shfl_xor_sync(0xffffffffu, m.w, k)));
     const float4 sv = column_scales(m);
     if (row == 0) *reinterpret_cast<float4*>(wu + vc) = column_units(m);
 #pragma unroll
     for (int i = 0; i < 4; ++i) store_split4(Wh, Wl, (row + 16 * i) * LU_VB + vc * 2, y[i], sv);
     if (c == 0 && d.pos0[s] > 0) {   // the state that is carried in: a thread reads every fourth entry of a column
       const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 + (t & 63);
-      unsigned* srows = rows_s + 4 * LM_C;
       unsigned top = 0u;
 #pragma unroll 4
       for (int i = t >> 6; i < d.dim; i += 4) {
         const unsigned a = (t & 63) < vw ? abs_bits(sp[static_cast<long long>(i) * d.vdim]) : 0u, most = __reduce_max_sync(0xffffffffu, a);
         top = max(top, a);
-        if (lane == 0) atomicMax(srows + i, most);
+        note(rs, most, true);
       }
       note(rs, top, true);
     }
     __syncthreads();
-    if (t < LM_C) {   // cleared for the head after the next, two barriers away
-      note(rv, vrows[t]);
-      vrows[t] = 0u;
-    }
-    if (c == 0 && t < 128) {
-      note(rs, rows_s[4 * LM_C + t]);
-      rows_s[4 * LM_C + t] = 0u;
-    }
     if (16 * warp < dim16) {
       float a[8][4], b[8][4];   // hi hi, and the two small products
 #pragma unroll
@@ -324,14 +310,6 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
         }
       }
     }
-  }
-  if (t < LM_C) {
-    Range r = {0u, RANGE_NONE};
-    note(r, rows_s[t]);
-    note_warp(range, r);
-    r = {0u, RANGE_NONE};
-    note(r, rows_s[LM_C + t]);
-    note_warp(range + 1, r);
   }
   note_warp(range + 2, rv);
   note_warp(range + 3, rs);
@@ -419,7 +397,10 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
   const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
   const long long r0 = base + t0, slot = la_slot(d, s, c);
   const int act = d.in_act;
-  const auto map = [act](float x) { return act_of<ACT>(x, act); };
+  const auto map = [act] {
+    if constexpr (ACT == VY_UACT_NONE) return SameValue();
+    else return [act](float x) { return act_of<ACT>(x, act); };
+  }();
   split_rows<LO_W, 128>(Qh, Qh + q_lo, kb, qu, SPLIT_TOP, LM_C, d.dim, dim16, d.q, d.in_dt, vec,
                         [&](int r) { return r < nt ? (r0 + r) * d.ldq + static_cast<long long>(hq) * d.dim : -1LL; }, map);
   split_rows<LO_W, 128>(Kh, Kh + q_lo, kb, ku, SPLIT_TOP, LM_C, d.dim, dim16, d.k, d.in_dt, vec,
@@ -662,7 +643,7 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   int hp = TD ? d.heads / d.kv_heads : 1;
   while (hp % 2 == 0 && static_cast<long long>(chunks) * vslices * (d.heads / hp) * n_seqs < 2LL * num_sms()) hp /= 2;
   const dim3 grid(static_cast<unsigned>(chunks) * vslices, d.heads / hp, n_seqs);
-  const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + 128 + 64 + 4 * LM_C + 128) + 4 * sizeof(Range);
+  const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + 128 + 64) + 4 * sizeof(Range);
   const size_t q2 = 2 * LM_C * static_cast<size_t>(kb), vs = 2 * LM_C * LU_VB + 2 * static_cast<size_t>(dim16) * LU_VB;
   const size_t smem_o = q2 + (q2 > vs ? q2 : vs) + sizeof(float) * 7 * LM_C;
   static std::atomic<unsigned long long> allowed_u{0}, allowed_o{0};

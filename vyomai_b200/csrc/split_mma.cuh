@@ -10,6 +10,8 @@
 #pragma once
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "vy_common.cuh"
 
 namespace vy {
@@ -118,7 +120,7 @@ __device__ __forceinline__ void split_rows(unsigned char* hi, unsigned char* lo,
       const int r = r0 + u * NW * 4;
       float m = 0.f;
 #pragma unroll
-      for (int i = 0; i < NI; ++i) {
+      for (int i = 0; i < NI && !std::is_same<MapFn, SameValue>::value; ++i) {
         const int c = l8 * 4 + 32 * i;
         x[u][i] = make_float4(c < width ? map(x[u][i].x) : 0.f, c + 1 < width ? map(x[u][i].y) : 0.f, c + 2 < width ? map(x[u][i].z) : 0.f, c + 3 < width ? map(x[u][i].w) : 0.f);
       }
