@@ -282,7 +282,8 @@ __device__ __forceinline__ void dc_bulk_load(void* dst, const void* src, unsigne
 
 // The writes' share of the read-outs in FMAs, a token at a time: where a write is infinite or NaN, the product's zeros would carry it to the tokens before it, and
 // where the writes of a column lie far apart, the larger ones' unit would cost the smaller ones, which earlier tokens read, their bits
-constexpr float DC_APART = 0x1p-20f;   // the halves are off by at most 2^-49 of the column's largest write; 3 in 10000 chunks of normal numbers come here
+constexpr float DC_APART = 0x1p-20f;   // the halves are off by at most 2^-49 of the column's largest write; 3 in 10000 chunks of normal numbers come here, and a
+                                       // sequence's last chunk where it has fewer than 16 tokens (writes of zero beside others: the test has no instruction for them)
 static __device__ __noinline__ void dc_read_serial(float (&o)[2][4], const float (&u)[2][4], const unsigned char* b, const float* unit, int lane) {
   const int tq = 2 * (lane & 3);
 #pragma unroll
@@ -462,11 +463,12 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
         o[j][e] = fmaf(fmaf(y0, cut, x[2 + j][e]), LO_UNIT, y0) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
       }
     }
-    bool together = true;
+    const float a0 = DC_APART * m0, a1 = DC_APART * m1;
+    bool together = m0 < INFINITY && m1 < INFINITY;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) together = together && fabsf(u[j][e]) < INFINITY && (fabsf(u[j][e]) >= DC_APART * (e < 2 ? m0 : m1) || u[j][e] == 0.f);
+      for (int e = 0; e < 4; ++e) together = together && fabsf(u[j][e]) >= (e < 2 ? a0 : a1);   // false for NaN
     if (__all_sync(0xffffffffu, together)) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
