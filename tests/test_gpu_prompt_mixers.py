@@ -526,6 +526,15 @@ def test_prompt_attention_in_blocks_of_192_rows(form, H, G, d, dv, window, keep)
     assert _err(got, torch.cat(want)) < BOUND
 
 
+def test_delta_rule_form_for_one_prompt_beside_many_tokens():
+    """One long portion beside many short ones takes the walk up to a length that grows with the rounds of CTAs; portions that are alike do not."""
+    from vyomai_b200._lib import lib
+    floats = lambda lengths, H, d: int(lib().vy_delta_rule_prompt_floats(sum(lengths), len(lengths), max(lengths), H, d, d))  # noqa: E731
+    assert floats([32] + [1] * 31, 8, 128) == 0 and floats([100] + [1] * 31, 8, 128) > 0
+    assert floats([70] + [1] * 63, 8, 128) == 0 and floats([200] + [1] * 63, 8, 128) > 0
+    assert floats([32] * 32, 8, 128) > 0 and floats([32] + [1] * 7, 8, 128) > 0 and floats([48] + [1] * 31, 4, 64) > 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_repeated_product_reads_its_own_operands(dtype):
     """Products of one shape share a prepared argument block: other addresses, strides and streams give what a first call gives."""

@@ -534,10 +534,14 @@ cudaError_t launch(const RecDev& d, int n_seqs, int max_new, const DeltaChunks& 
 
 // From 32 tokens on (64 for heads of up to 32 channels): two launches and a chunk's preparation cost more than a short walk. In us, chunks / tokens:
 // 1 sequence, 8 heads of 128 x 128: 20.3 / 19.9 at 24 tokens, 20.5 / 23.2 at 32, 30 / 71 at 128; 32 sequences, 4 heads of 64 x 64: 19.2 / 18.4,
-// 19.3 / 22.0, 44 / 72; 4 sequences, 4 heads of 16 x 16: 16.2 / 15.4 at 48, 17.3 / 18.6 at 64. Past 128 channels a warp's share of the state
-// (16 columns) does not fit its registers.
+// 19.3 / 22.0, 44 / 72; 4 sequences, 4 heads of 16 x 16: 16.2 / 15.4 at 48, 17.3 / 18.6 at 64. Where a long portion stands beside many short ones the walk is
+// through with those at once, but here each of their CTAs fills its buffers: 8 heads of 128 x 128, 31 single tokens and one portion of 32, 64, 100: 46 / 27, 47 / 43,
+// 48 / 62; 63 single tokens and 70, 200: 71 / 51, 83 / 115; 4 heads of 64 x 64, 31 and 48: 21 / 24. So 20 tokens per round of CTAs (two per SM).
+// Past 128 channels a warp's share of the state (16 columns) does not fit its registers.
 long long delta_rule_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim) {
   if (max_new < (dim > 32 ? 32 : 64) || dim > 128 || rows <= 0) return 0;
+  const long long ctas = static_cast<long long>(n_seqs) * heads * (round32(vdim) / 32);
+  if (4 * rows < static_cast<long long>(n_seqs) * max_new && max_new < 20 * ctas / (2 * num_sms())) return 0;
   const long long f = (rows / DC_T + n_seqs) * heads * (blob_bytes(dim) / 4 + 16LL * round32(vdim));
   return f <= (1LL << 28) ? f : 0;
 }
