@@ -23,9 +23,7 @@ constexpr int DC_T = 16;            // tokens per chunk
 constexpr int DC_KTOP = 15;         // the decayed unit keys are split in units of 2^-15: their entries are at most 1
 constexpr int DC_NW = 2;            // warps of the walk's CTA: 32 value columns
 constexpr int DC_NS = 3;            // chunks in flight per CTA of the walk
-// A tensor-core accumulation cuts off where fp32 rounds: a result is this share too small on average (measured: read-outs -5.8e-8 without it,
-// -0.4e-8 with it, the serial walk +0.5e-8). A sum of n accumulations loses (n + 1) / 2 such shares of its end value on average
-constexpr float DC_CUT = 0x1p-25f / LO_UNIT;   // in the unit of the small products' sums, to which it is added
+// What the accumulations cut off (split_mma.cuh) is added back: read-outs are off by -5.8e-8 on average without it, -0.4e-8 with it, in the serial walk +0.5e-8
 
 // One chunk and head in the workspace. An operand entry is 16 bytes per lane: (b0, b1) of mma.m16n8k16, hi then lo
 template <int DP>
@@ -398,7 +396,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       }
     }
     // the writes, then as A operand
-    constexpr float cut = ((KS >= 4 ? KS / 2 : KS) + 1) * 0.5f * DC_CUT;
+    constexpr float cut = ((KS >= 4 ? KS / 2 : KS) + 1) * 0.5f * SPLIT_CUT;
     const float* unit = reinterpret_cast<const float*>(st + Blob::unit_at);
     const float4* wv = reinterpret_cast<const float4*>(st + Blob::bytes + 1024 * warp + 32 * lane);
     float u[2][4];
@@ -409,7 +407,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       const float2 p = *reinterpret_cast<const float2*>(unit + 8 * j + tq);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float y0 = r[j][e] + half[j][e], z = fmaf(fmaf(y0, cut, x[j][e]), LO_UNIT, y0) * (e < 2 ? n0 : n1);
+        const float y0 = r[j][e] + half[j][e], z = split_sum(y0, x[j][e], cut) * (e < 2 ? n0 : n1);
         u[j][e] = fmaf(-z, e & 1 ? p.y : p.x, e == 0 ? y.x : e == 1 ? y.y : e == 2 ? y.z : y.w);
       }
       m0 = fmaxf(m0, fmaxf(fabsf(u[j][0]), fabsf(u[j][1])));
@@ -449,7 +447,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
       for (int i = 0; i < 2; ++i) {
         const float2 g = *reinterpret_cast<const float2*>(G + 8 * (j + i));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[j + i][e] = fmaf(S[j + i][e], e & 1 ? g.y : g.x, fmaf(fmaf(y[i][e], DC_CUT, z[i][e]), LO_UNIT, y[i][e]) * (e < 2 ? k0 : k1));
+        for (int e = 0; e < 4; ++e) S[j + i][e] = fmaf(S[j + i][e], e & 1 ? g.y : g.x, split_sum(y[i][e], z[i][e], SPLIT_CUT) * (e < 2 ? k0 : k1));
       }
     }
     // the read-outs
@@ -460,7 +458,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float y0 = r[2 + j][e] + half[2 + j][e];
-        o[j][e] = fmaf(fmaf(y0, cut, x[2 + j][e]), LO_UNIT, y0) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
+        o[j][e] = split_sum(y0, x[2 + j][e], cut) * ((e < 2 ? n0 : n1) * (e & 1 ? q.y : q.x));
       }
     }
     const float a0 = DC_APART * m0, a1 = DC_APART * m1;
@@ -479,7 +477,7 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
         mma_f16(y, uh, f.x, f.y);
         mma_f16(z, uh, f.z, f.w);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[j][e] = fmaf(fmaf(fmaf(y[e], DC_CUT, z[e]), LO_UNIT, y[e]) * (e < 2 ? w0 : w1), e & 1 ? p.y : p.x, o[j][e]);
+        for (int e = 0; e < 4; ++e) o[j][e] = fmaf(split_sum(y[e], z[e], SPLIT_CUT) * (e < 2 ? w0 : w1), e & 1 ? p.y : p.x, o[j][e]);
       }
     } else {
       dc_read_serial(o, u, st + Blob::b_at, unit + 2 * DC_T, lane);

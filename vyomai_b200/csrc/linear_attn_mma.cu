@@ -296,11 +296,12 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
         const int i = 16 * warp + gq + 8 * r;
         if (i >= d.dim) continue;
         const float u1 = ku[i];
+        constexpr float cut = (LM_C / 16 + 1) * 0.5f * SPLIT_CUT;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int col = 8 * j + 2 * tq;
           const float2 u2 = *reinterpret_cast<const float2*>(wu + col);
-          const float p = fmaf(b[j][2 * r], LO_UNIT, a[j][2 * r]) * u1 * u2.x, q = fmaf(b[j][2 * r + 1], LO_UNIT, a[j][2 * r + 1]) * u1 * u2.y;
+          const float p = split_sum(a[j][2 * r], b[j][2 * r], cut) * u1 * u2.x, q = split_sum(a[j][2 * r + 1], b[j][2 * r + 1], cut) * u1 * u2.y;
           float* at = U + static_cast<long long>(i) * d.vdim + col;
           if (col + 1 < vw && d.vdim % 2 == 0) *reinterpret_cast<float2*>(at) = make_float2(p, q);
           else {
@@ -410,6 +411,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
   const unsigned va = smem_addr(Vh) + lane_bt(lane, LU_VB), sa = smem_addr(Sh) + lane_bt(lane, LU_VB);
   const int i0 = 16 * warp + gq;   // this lane's rows: i0 and i0 + 8
   const float qunit[2] = {qu[i0], qu[i0 + 8]};
+  const float cut = (dim16 / 16 + 1) * 0.5f * SPLIT_CUT, vcut = (warp + 2) * 0.5f * SPLIT_CUT;   // sums over the channels, over the tokens this warp sees
   float p[8][4];   // scores q_i . k_j; a warp's tokens only see keys j < 16 (warp + 1)
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -436,7 +438,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) p[2 * j + i][e] = fmaf(b[i][e], LO_UNIT, a[i][e]) * qunit[e >> 1] * ku[16 * j + 8 * i + 2 * tq + (e & 1)];
+      for (int e = 0; e < 4; ++e) p[2 * j + i][e] = split_sum(a[i][e], b[i][e], cut) * qunit[e >> 1] * ku[16 * j + 8 * i + 2 * tq + (e & 1)];
   }
   for (int h = h0; h < h0 + hp; ++h) {
     __syncthreads();   // the readers of k, or of the previous head's values and state, are done
@@ -510,7 +512,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][e] = fmaf(b[i][e], LO_UNIT, o[i][e]) * su * f[e >> 1];
+        for (int e = 0; e < 4; ++e) o[i][e] = split_sum(o[i][e], b[i][e], cut) * su * f[e >> 1];
     }
     // the weights inside the chunk, times the exponent of each value row, then scaled row by row
     unsigned ph[4][4], pl[4][4];
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[4 * cb + i][e] = fmaf(fmaf(b[i][e], LO_UNIT, a[i][e]), pu[e >> 1] * v_unit, o[4 * cb + i][e]);
+        for (int e = 0; e < 4; ++e) o[4 * cb + i][e] = fmaf(split_sum(a[i][e], b[i][e], vcut), pu[e >> 1] * v_unit, o[4 * cb + i][e]);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {

@@ -18,6 +18,10 @@ namespace vy {
 
 constexpr int SPLIT_TOP = 12;     // scaled rows have their largest entry in [2^SPLIT_TOP, 2^(SPLIT_TOP + 1))
 constexpr float LO_UNIT = 0x1p-11f;   // a lo half is stored in this unit
+// A tensor-core accumulation cuts off where fp32 rounds: a result is this share too small on average (in the unit of the small products' sums, to which it can be
+// added: sum = (small + hi * cut) * LO_UNIT + hi). A sum of n accumulations loses (n + 1) / 2 such shares of its end value on average
+constexpr float SPLIT_CUT = 0x1p-25f / LO_UNIT;
+__device__ __forceinline__ float split_sum(float hi, float small, float cut) { return fmaf(fmaf(hi, cut, small), LO_UNIT, hi); }
 constexpr int SPLIT_MIN_E = -100; // rows whose largest entry is below 2^-100 (all zero, for one) keep this exponent: scales stay finite
 
 // exponent of a row's largest absolute value
