@@ -303,7 +303,7 @@ def test_linear_attention_keeps_large_numbers_to_their_column(bad, where):
     """All chunks at once, then a continuation: a value, or an entry of the state that is carried in, changes its own column and nothing else."""
     from vyomai_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(4)
-    T, more, H, dk, dv, at, col = 200, 70, 2, 48, 80, 112, 5
+    T, more, H, dk, dv, at, col = 200, 140, 2, 48, 80, 112, 5
     q, k, v = (torch.randn(T + more, H * w, generator=g, device=DEV) for w in (dk, dk, dv))
     S0 = torch.randn(1, H, dk, dv, generator=g, device=DEV)
     decay = torch.tensor([0.99, 0.9], device=DEV)
@@ -562,6 +562,15 @@ def test_linear_attention_sums_are_not_cut_short():
     got = ops.linear_attn(ops.PackedBatch(_i32([0, T]), _i32([0]), _i32([0]), T), q.to(DEV), k.to(DEV), v.to(DEV), torch.full((H,), decay, device=DEV),
                           torch.zeros(1, H, d, d, device=DEV), heads=H, dim=d, vdim=d).double().cpu()
     assert abs(float(((got - want) * want).sum() / (want * want).sum())) < 4e-8
+
+
+def test_linear_attention_form_for_one_prompt_beside_many_tokens():
+    """One long portion beside many short ones takes the walk up to a length that grows with the chunks; portions that are alike do from three chunks on."""
+    from vyomai_b200._lib import lib
+    floats = lambda lengths, H, d, dv: int(lib().vy_linear_attn_workspace_floats(sum(lengths), len(lengths), max(lengths), H, d, dv))  # noqa: E731
+    assert floats([128], 16, 128, 64) == 0 and floats([130], 16, 128, 64) > 0 and floats([130] * 32, 16, 128, 64) > 0
+    assert floats([200] + [1] * 31, 16, 128, 64) == 0 and floats([512] + [1] * 31, 16, 128, 64) > 0 and floats([200] + [1] * 7, 16, 128, 64) > 0
+    assert floats([400] + [1] * 31, 32, 128, 64) == 0 and floats([2000] + [1] * 31, 32, 128, 64) > 0
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])

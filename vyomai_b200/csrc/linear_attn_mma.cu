@@ -622,10 +622,15 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
   }
 }
 
-// from two chunks on the three launches beat the walk
+// From three chunks on: us, here / walk, 16 heads of 128 x 64, one portion of 70, 130, 300 tokens 27 / 24, 28 / 35, 28 / 60; 32 of 130, 300: 195 / 187, 311 / 330. Every
+// sequence has a chunk at least, which here costs two passes over its state more than in the walk, while the walk takes about 10 us per chunk of the longest portion. So
+// where portions are uneven these launches pay from about 2 / 3 token per chunk and head on: one of 200, 400, 512 beside 31 single tokens 88 / 62, 103 / 107, 105 / 125, one of
+// 200 beside 7 41 / 53; state space, 32 heads of 128 x 64, one of 130, 400 beside 31 312 / 156, 328 / 173
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim) {
-  if (max_new <= LM_C || dim > 128 || rows <= 0) return 0;
-  const long long slots = rows / LM_C + n_seqs, floats = slots * heads * (static_cast<long long>(dim) * vdim + 2 + (vdim + 63) / 64) + 4;
+  if (max_new <= 2 * LM_C || dim > 128 || rows <= 0) return 0;
+  const long long slots = rows / LM_C + n_seqs;
+  if (2 * rows < static_cast<long long>(n_seqs) * max_new && 3LL * max_new < 2 * slots * heads * ((vdim + 63) / 64) * (dim + 64) / 192) return 0;
+  const long long floats = slots * heads * (static_cast<long long>(dim) * vdim + 2 + (vdim + 63) / 64) + 4;
   return floats <= (1LL << 28) ? floats : 0;   // 1 GB: past it the walk, which keeps its state on the chip
 }
 
@@ -643,7 +648,7 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, vslices = (d.vdim + 63) / 64, chunks = (max_new + LM_C - 1) / LM_C;
   // heads per CTA: those that share q and k, fewer while that leaves less than two CTAs per SM
   int hp = TD ? d.heads / d.kv_heads : 1;
-  while (hp % 2 == 0 && static_cast<long long>(chunks) * vslices * (d.heads / hp) * n_seqs < 2LL * num_sms()) hp /= 2;
+  while (hp % 2 == 0 && slots * vslices * (d.heads / hp) < 2LL * num_sms()) hp /= 2;
   const dim3 grid(static_cast<unsigned>(chunks) * vslices, d.heads / hp, n_seqs);
   const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + 128 + 64) + 4 * sizeof(Range);
   const size_t q2 = 2 * LM_C * static_cast<size_t>(kb), vs = 2 * LM_C * LU_VB + 2 * static_cast<size_t>(dim16) * LU_VB;
