@@ -273,11 +273,6 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks 
   }
 }
 
-__device__ __forceinline__ void dc_bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
 // The writes' share of the read-outs in FMAs, a token at a time: where a write is infinite or NaN, the product's zeros would carry it to the tokens before it, and
 // where the writes of a column lie far apart, the larger ones' unit would cost the smaller ones, which earlier tokens read, their bits
 constexpr float DC_APART = 0x1p-20f;   // the halves are off by at most 2^-49 of the column's largest write; 3 in 10000 chunks of normal numbers come here, and a
@@ -320,8 +315,8 @@ __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaC
     unsigned char* st = dc_smem + b * STAGE;
     ++issued[b];
     mbar_arrive_expect_tx(&full[b], STAGE);
-    dc_bulk_load(st, w.blobs + at * Blob::bytes, Blob::bytes, &full[b]);
-    dc_bulk_load(st + Blob::bytes, w.wv + (at * (w.vpad / 16) + blockIdx.x * DC_NW) * 256, DC_NW * 1024, &full[b]);
+    bulk_load(st, w.blobs + at * Blob::bytes, Blob::bytes, &full[b]);
+    bulk_load(st + Blob::bytes, w.wv + (at * (w.vpad / 16) + blockIdx.x * DC_NW) * 256, DC_NW * 1024, &full[b]);
   };
   if (threadIdx.x == 0) {
     for (int b = 0; b < DC_NS; ++b) {

@@ -104,6 +104,11 @@ VY_DEVINL bool mbar_wait_soft(uint64_t* bar, uint32_t parity, const PoisonRef& p
   }
   return true;
 }
+// untiled bulk copy global -> shared (both addresses 16-byte aligned, a multiple of 16 bytes), counted by `bar`
+VY_DEVINL void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
 // Behind a wait that timed out: the copies in flight to this CTA's `n` buffers are waited for (with a limit) before it leaves. issued: copies per buffer so far
 VY_DEVINL void mbar_drain(uint64_t* bars, const int* issued, int n) {
   for (int b = 0; b < n; ++b) {

@@ -6,8 +6,10 @@
 // 2^hl query heads of one key / value head times the rows / 2^hl queries, so that heads that share keys share the key tiles and the window's
 // edges waste little. A warp keeps its scores, weights and outputs in registers from one product to the next. Tiles of keys arrive by bulk copies
 // into a ring of buffers; a warp waits for a tile, never for another warp, and the warp that is through with a buffer last refills it. (With CTA
-// barriers per tile all warps are in the same phase: 267 and 854 us instead of the 235 and 548 below.) Without a workspace (a caller of the C
-// ABI that lends none, or one too large to lend) each CTA splits its tiles itself, which costs it about as many instructions as the softmax does.
+// barriers per tile all warps are in the same phase: 267 and 854 us where the ring takes 228 and 548.)
+//
+// Halves suit keys and values of a moderate range: where a list's (one sequence, one key / value head) is too wide, or its scores too large, the kernel leaves it
+// to the fp32 tiles (seqmix_tiled.cu), which are launched behind it and serve calls without a workspace too. 2.3 us where they find nothing to do.
 //
 // What bounds it: the tensor pipe (three fp16 products per fp32 one on mma.sync) and the shared-memory reads that feed it, about alike, then the
 // instructions of the softmax. 4 x 2048 tokens, 8 heads of 128 over 2 key / value heads, window 512, capped: 943 us -> 235 us; 16 heads of 96 / 64
@@ -22,11 +24,6 @@ namespace vy {
 __device__ __forceinline__ void portion_keys(const WinDev& d, int p0, int& nA, int& lo) {
   lo = d.chunk > 0 ? p0 / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p0 - d.window + 1, 0);
   nA = d.window <= 0 ? 0 : min(d.keep, lo);
-}
-
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
 }
 
 constexpr int WS_T = 8 * SPLIT_ROWS;   // splitting launch: eight lanes per row
