@@ -11,8 +11,8 @@
 //   delta_scan_kernel    the walk. It is transposed (S^T: a warp owns 16 value columns and all channels), so that the state in accumulator
 //                        registers is the next product's A operand, the writes likewise, and no warp waits for another one
 // The walk token by token (delta_rule_kernel) is bound by its chain of two reductions per token: 46 + 1013 us with its preparation for 4 x 2048
-// tokens, 8 heads of 128 x 128; here 166 + 217 us. The first launch is bound by instructions (decays, exponentials, sums of pairs of tokens), the
-// second by the latency of one warp's chain, 1.7 us per chunk. Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
+// tokens, 8 heads of 128 x 128; here 164 + 236 us. The first launch is bound by instructions (decays, exponentials, sums of pairs of tokens), the
+// second by the latency of one warp's chain, 1.8 us per chunk. Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 

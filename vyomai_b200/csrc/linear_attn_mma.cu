@@ -153,7 +153,7 @@ constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows 
 
 // CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w .., and it reads and splits those channels of k (eight
 // tokens at a time) and value columns 8 w .. (sixteen at a time), all tokens of them: tokens are the summed index, so a channel and a column have one unit
-// each, and their largest entries need no other warp. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 84 us, bound by
+// each, and their largest entries need no other warp. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 101 us, bound by
 // writing the states (134 MB) and by the latency of each chunk's few steps
 // ACT: see act_of
 template <bool TD, int ACT>
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(256) la_scan_kernel(RecDev d, LaChunks w) {
 constexpr int LO_T = 128, LO_W = 4;
 
 // CTA: (chunk, 64 value columns) x (hp heads that share q and k) x sequence; warp w owns tokens 16 w .. 16 w + 15 and keeps their scores in registers
-// for all its heads. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 277 us (la_scan 83; the walk over the chunks was 737 us for everything). Bound by
+// for all its heads. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 292 us (la_scan 83; the walk over the chunks was 737 us for everything). Bound by
 // fixed latencies at two warps per scheduler (255 registers): the tensor pipe is 13 % active; twice the warps with half the columns: 301 us
 template <bool TD, int ACT>
 __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec, bool svec) {

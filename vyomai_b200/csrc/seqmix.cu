@@ -516,7 +516,7 @@ __device__ __forceinline__ void conv_new_taps(const ConvDev& d, int c, int base,
 }
 
 // A thread makes CONV_TOK outputs of one channel from a register window: its CONV_TOK + TAPS - 1 inputs are loaded at once and each serves `taps`
-// outputs. Bound by memory latency, one round trip per thread. fp32, 4 taps, the walk of 32 tokens that loaded an input per tap and output / this:
+// outputs. Bound by instructions (71 to 75 % of the issue slots). fp32, 4 taps, the walk of 32 tokens that loaded an input per tap and output / this:
 // 8192 tokens x 1024 channels 65.5 / 31.8 us, x 512 40.4 / 17.4 us, 80 tokens x 512 31.1 / 7.3 us. The first CTA column of a sequence, the only
 // one that reads the slot's old taps, writes the new ones (a launch of its own before, 2.2 us). TAPS >= taps
 template <int TAPS>

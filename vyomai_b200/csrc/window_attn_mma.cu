@@ -12,8 +12,8 @@
 // to the fp32 tiles (seqmix_tiled.cu), which are launched behind it and serve calls without a workspace too. 2.3 us where they find nothing to do.
 //
 // What bounds it: the tensor pipe (three fp16 products per fp32 one on mma.sync) and the shared-memory reads that feed it, about alike, then the
-// instructions of the softmax. 4 x 2048 tokens, 8 heads of 128 over 2 key / value heads, window 512, capped: 943 us -> 235 us; 16 heads of 96 / 64
-// channels over the whole context: 2812 us -> 548 us (the fp32-FMA tiles this replaces ran at 15 TFLOP/s).
+// instructions of the softmax. 4 x 2048 tokens, 8 heads of 128 over 2 key / value heads, window 512, capped: 236 us and 8 for the splitting (fp32 tiles, at 15 TFLOP/s: 943);
+// 16 heads of 96 / 64 channels over the whole context: 545 and 41 us (2812).
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 #include "vy_ptx.cuh"

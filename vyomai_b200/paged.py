@@ -373,7 +373,7 @@ class HybridBatchEngine:
     """Continuous batching for hybrid models, the counterpart of ContinuousBatchEngine for models with a packed `step`
     (models/gelutar.py): every engine iteration is ONE model step over the concatenated new tokens of all live
     sequences — whole prompts of the sequences that start, one token of those that decode — so nothing is padded and
-    a sequence's logits do not depend on its neighbours. `step()` is the greedy generation loop (waiting room, eos /
+    a sequence's logits do not depend on its neighbours (but for rounding: kernel forms and tile sizes follow the step's shape). `step()` is the greedy generation loop (waiting room, eos /
     length retirement as above); `feed()` / `release()` advance named sequences by GIVEN tokens and return the logits of
     chosen rows (replaying a recorded trace, scoring, teacher forcing) through the same step and manager."""
 
