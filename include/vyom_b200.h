@@ -788,8 +788,8 @@ typedef struct VyWinAttn {
   int64_t k_row, v_row;
   /* optional scratch. Single-token steps: vy_window_attn_workspace_floats(n_seqs, heads, kv_heads, vdim) floats (0: none needed); those whose query heads share
    * key / value rows in groups of 8 or more split a sequence's keys over several CTAs and combine the parts from here. Longer portions:
-   * vy_window_attn_prompt_floats(..) floats, 16-byte aligned (0: none needed); the visible key / value rows are split for the tensor cores once, into it,
-   * instead of by every CTA that reads them */
+   * vy_window_attn_prompt_floats(..) floats, 16-byte aligned (0: none needed): the visible key / value rows are split for the tensor cores into it. With less, but
+   * enough for one sequence (n_seqs = 1), the sequences go a few at a time; without, in fp32 tiles */
   float* workspace; int64_t workspace_floats;
   void* stream;
   int32_t chunk;
@@ -840,7 +840,7 @@ typedef struct VyLinAttn {
   void* out; int64_t ld_out; int32_t out_dtype;
   void* stream;
   /* optional scratch, 16-byte aligned, of vy_linear_attn_workspace_floats(rows, ..) floats (0: none needed), and the step's packed rows: long portions
-   * then run all their chunks at once instead of one after the other */
+   * then run all their chunks at once instead of one after the other (not: up to 128 tokens, one prompt beside many short portions, dim > 128, more than 1 GB) */
   int64_t rows;
   float* workspace; int64_t workspace_floats;
 } VyLinAttn;
@@ -870,7 +870,7 @@ typedef struct VyDeltaRule {
   void* stream;
 } VyDeltaRule;
 /* floats with which (16-byte aligned) a step walks its tokens 16 at a time on the tensor cores; 0: not for this step (max_new < 32, or 64 for
- * dim <= 32; dim > 128; more than 1 GB), which then takes the form above */
+ * dim <= 32; one prompt of few tokens beside many short portions; dim > 128; more than 1 GB), which then takes the form above */
 VY_API int64_t vy_delta_rule_prompt_floats(int64_t rows, int32_t n_seqs, int32_t max_new, int32_t heads, int32_t dim, int32_t vdim);
 VY_API int64_t vy_delta_rule_workspace_floats(int64_t rows, int32_t heads, int32_t kv_heads, int32_t dim);
 VY_API int vy_delta_rule(const VyDeltaRule* p);
@@ -1174,7 +1174,8 @@ typedef struct VyTalkAttn {
   int32_t force_form; /* 0 = chosen by the step's shape; 1 = one query per CTA; 2 = tiled (an error if the sizes do not fit it) */
   void* stream;
 } VyTalkAttn;
-/* prompts (portions of several tokens): the scratch with which 8, 16 or 32 heads of at most 64 channels run on the tensor cores (0: none) */
+/* prompts (portions of several tokens): the scratch with which 8, 16 or 32 heads of at most 64 channels run on the tensor cores (0: none); with less, but enough for
+ * one sequence (n_seqs = 1), the sequences go a few at a time. Not with a forced form */
 VY_API int64_t vy_talk_attn_prompt_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t heads, int32_t kv_heads, int32_t dim,
                                           int32_t vdim, int32_t window);
 VY_API int64_t vy_talk_attn_workspace_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t heads, int32_t vdim);
