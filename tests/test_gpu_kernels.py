@@ -314,6 +314,43 @@ def test_gemm_pinned_flavours_vs_oracle(pair, bn, splits):
     assert L.vy_gemm_poisoned() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("pair,bn", [(0, 32), (0, 64), (0, 128), (0, 192), (0, 256), (1, 128), (1, 192), (1, 256)])
+def test_gemm_fp32_write_back(pair, bn, dtype):
+    """fp32 results leave through bulk tensor stores: remainders of the tile in rows and columns, every activation, addends of both types
+    (one of them the output itself), a scale, padded output rows whose padding stays as it was. bf16 inputs: fp32 sums of exact products;
+    fp32 inputs run in tf32 (2e-3, as above)."""
+    from vyomai_b200 import _lib, ops
+    if pair and dtype == torch.float32:
+        pytest.skip("pairs of CTAs take bf16 operands")
+    L, tol = _lib.lib(), 1e-5 if dtype == torch.bfloat16 else 2e-3
+    acts = {None: lambda z: z, "gelu": O.gelu_erf, "gelu_tanh": O.gelu_tanh, "relu2": lambda z: torch.relu(z) ** 2}
+    try:
+        for i, (M, N, K) in enumerate(((33, 132, 72), (129, 320, 64), (300, 264, 200), (257, 137, 40))):
+            a, b, bias, res = _randn((M, K), 40 + i, dtype), _randn((N, K), 50 + i, dtype, K ** -0.5), _randn((N,), 60 + i, dtype), _randn((M, N), 70 + i)
+            ad, bd, biasd = (t.to(dtype).to(DEV) for t in (a, b, bias))
+            z, ld = a.double() @ b.double().t() + bias.double(), (N + 7) // 8 * 8 + 8
+            L.vy_gemm_tune_override(pair, bn, 0)
+            for act, f in acts.items():
+                buf = torch.full((M, ld), 7.0, device=DEV)
+                ops.gemm(ad, bd, bias=biasd, act=act, out=buf[:, :N])
+                assert rel_l2(buf[:, :N].cpu(), f(z.float()).double() if act else z) <= tol + (2e-6 if act else 0), (M, N, K, act)
+                assert bool((buf[:, N:] == 7.0).all())
+            for add in (res.to(DEV), res.bfloat16().to(DEV)):
+                if add.dtype == torch.bfloat16 and N % 8:
+                    continue
+                out = ops.gemm(ad, bd, bias=biasd, addend=add, out_scale=0.5, out=torch.empty(M, ld, device=DEV)[:, :N])
+                assert rel_l2(out.cpu(), 0.5 * (z + add.double().cpu())) <= tol, (M, N, K, add.dtype)
+            buf = torch.zeros(M, ld, device=DEV)
+            buf[:, :N] = res.to(DEV)
+            out = buf[:, :N]
+            ops.gemm(ad, bd, bias=biasd, addend=out, out=out)
+            assert rel_l2(out.cpu(), z + res.double()) <= tol
+    finally:
+        L.vy_gemm_tune_override(-1, 0, 0)
+    assert L.vy_gemm_poisoned() == 0
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 6e-3), (torch.float32, 2e-3)])
 def test_gemm_epilogues_vs_oracle(dtype, tol):
     """bias + exact-erf GELU (+ saved pre-activation), tanh GELU, residual addend, dGELU (the dgrad epilogue), swap-AB

@@ -25,14 +25,35 @@ VY_GEMM_EXTERN_PAIR(false, true, 128) VY_GEMM_EXTERN_PAIR(false, true, 256)
 VY_GEMM_EXTERN_PAIR(true, true, 128) VY_GEMM_EXTERN_PAIR(true, true, 256)
 
 // staged SwiGLU epilogue (inference form): bf16, both operands K-major, BN 128 | 256, either flavour
-extern template int launch_gemm<__nv_bfloat16, 128, false, false, false, true>(const VyGemm*, const GemmDev&);
-extern template int launch_gemm<__nv_bfloat16, 256, false, false, false, true>(const VyGemm*, const GemmDev&);
-extern template int launch_gemm<__nv_bfloat16, 128, false, false, true, true>(const VyGemm*, const GemmDev&);
-extern template int launch_gemm<__nv_bfloat16, 256, false, false, true, true>(const VyGemm*, const GemmDev&);
+extern template int launch_gemm<__nv_bfloat16, 128, false, false, false, WB_GATED>(const VyGemm*, const GemmDev&);
+extern template int launch_gemm<__nv_bfloat16, 256, false, false, false, WB_GATED>(const VyGemm*, const GemmDev&);
+extern template int launch_gemm<__nv_bfloat16, 128, false, false, true, WB_GATED>(const VyGemm*, const GemmDev&);
+extern template int launch_gemm<__nv_bfloat16, 256, false, false, true, WB_GATED>(const VyGemm*, const GemmDev&);
+// staged fp32 write-back: both operands K-major
+#define VY_GEMM_EXTERN_F32(T, BN, P) extern template int launch_gemm<T, BN, false, false, P, WB_F32>(const VyGemm*, const GemmDev&);
+VY_GEMM_EXTERN_F32(__nv_bfloat16, 32, false) VY_GEMM_EXTERN_F32(__nv_bfloat16, 64, false) VY_GEMM_EXTERN_F32(__nv_bfloat16, 128, false)
+VY_GEMM_EXTERN_F32(__nv_bfloat16, 192, false) VY_GEMM_EXTERN_F32(__nv_bfloat16, 256, false)
+VY_GEMM_EXTERN_F32(__nv_bfloat16, 128, true) VY_GEMM_EXTERN_F32(__nv_bfloat16, 192, true) VY_GEMM_EXTERN_F32(__nv_bfloat16, 256, true)
+VY_GEMM_EXTERN_F32(float, 32, false) VY_GEMM_EXTERN_F32(float, 64, false) VY_GEMM_EXTERN_F32(float, 128, false)
+VY_GEMM_EXTERN_F32(float, 192, false) VY_GEMM_EXTERN_F32(float, 256, false)
+template <typename T>
+static int dispatch_gemm_f32(const VyGemm* p, const GemmDev& g, int bn, bool pair) {
+  if constexpr (sizeof(T) == 2) {
+    if (pair) return bn == 128 ? launch_gemm<T, 128, false, false, true, WB_F32>(p, g) : bn == 192 ? launch_gemm<T, 192, false, false, true, WB_F32>(p, g)
+                               : launch_gemm<T, 256, false, false, true, WB_F32>(p, g);
+  }
+  switch (bn) {
+    case 32: return launch_gemm<T, 32, false, false, false, WB_F32>(p, g);
+    case 64: return launch_gemm<T, 64, false, false, false, WB_F32>(p, g);
+    case 128: return launch_gemm<T, 128, false, false, false, WB_F32>(p, g);
+    case 192: return launch_gemm<T, 192, false, false, false, WB_F32>(p, g);
+    default: return launch_gemm<T, 256, false, false, false, WB_F32>(p, g);
+  }
+}
 static int dispatch_gemm_gated(const VyGemm* p, const GemmDev& g, int bn, bool pair) {
   using T = __nv_bfloat16;
-  if (pair) return bn == 128 ? launch_gemm<T, 128, false, false, true, true>(p, g) : launch_gemm<T, 256, false, false, true, true>(p, g);
-  return bn == 128 ? launch_gemm<T, 128, false, false, false, true>(p, g) : launch_gemm<T, 256, false, false, false, true>(p, g);
+  if (pair) return bn == 128 ? launch_gemm<T, 128, false, false, true, WB_GATED>(p, g) : launch_gemm<T, 256, false, false, true, WB_GATED>(p, g);
+  return bn == 128 ? launch_gemm<T, 128, false, false, false, WB_GATED>(p, g) : launch_gemm<T, 256, false, false, false, WB_GATED>(p, g);
 }
 
 static int dispatch_gemm_pair(const VyGemm* p, const GemmDev& g, int bn) {
@@ -382,6 +403,12 @@ extern "C" int vy_gemm(const VyGemm* p) {
   if (tma_store_on && p->epi == VY_EPI_LINEAR && (p->act != VY_ACT_SWIGLU || gated_fast) && !p->transposed_out && g.vec_ok && p->out_dtype == VY_BF16 && !p->addend2 &&
       p->out_row_group == 0 && (!p->aux || p->aux_dtype == VY_BF16) && (!p->addend || p->addend_dtype == VY_BF16))
     g.tma_store = 1;
+  // the staged fp32 write-back: like the fast bf16 epilogues it loads the bias in vectors and keeps no pre-activation. A bulk store is cut off at
+  // whole 16 bytes, so rows that end elsewhere (N no multiple of 4) would spill over into what lies beside the result
+  const bool f32_fast = tma_store_on && p->epi == VY_EPI_LINEAR && p->out_dtype == VY_F32 && p->N % 4 == 0 && !p->transposed_out && g.vec_ok && !p->a_mn_major && !p->b_mn_major &&
+                        !p->addend2 && !p->aux && p->out_row_group == 0 && aligned16(p->bias) &&
+                        (p->act == VY_ACT_NONE || p->act == VY_ACT_GELU_ERF || p->act == VY_ACT_GELU_TANH || p->act == VY_ACT_RELU2);
+  if (f32_fast) g.tma_store = 1;
   const int bk = p->in_dtype == VY_BF16 ? 64 : 32;
   const int num_kb = (p->K + bk - 1) / bk;
   // split-K is offered for plain linear epilogues (what the weight gradients use) when the caller lent scratch space
@@ -454,6 +481,11 @@ extern "C" int vy_gemm(const VyGemm* p) {
   }
 
   if (p->act == VY_ACT_SWIGLU && g.tma_store) return dispatch_gemm_gated(p, g, bn, pair);
+  if (f32_fast) {
+    const int rc = p->in_dtype == VY_BF16 ? dispatch_gemm_f32<__nv_bfloat16>(p, g, bn, pair) : dispatch_gemm_f32<float>(p, g, bn, false);
+    if (rc != NO_OUT_MAP) return rc;
+    g.tma_store = 0;
+  }
   if (pair) return dispatch_gemm_pair(p, g, bn);
   if (p->in_dtype == VY_BF16) return dispatch_gemm<__nv_bfloat16>(p, g, bn);
   return dispatch_gemm<float>(p, g, bn);

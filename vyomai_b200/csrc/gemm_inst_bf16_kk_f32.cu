@@ -1,0 +1,9 @@
+// explicit instantiations of the vy_gemm kernels whose epilogue is the staged fp32 one (see gemm_kernel.cuh)
+#include "gemm_kernel.cuh"
+namespace vy {
+template int launch_gemm<__nv_bfloat16, 32, false, false, false, WB_F32>(const VyGemm*, const GemmDev&);
+template int launch_gemm<__nv_bfloat16, 64, false, false, false, WB_F32>(const VyGemm*, const GemmDev&);
+template int launch_gemm<__nv_bfloat16, 128, false, false, false, WB_F32>(const VyGemm*, const GemmDev&);
+template int launch_gemm<__nv_bfloat16, 192, false, false, false, WB_F32>(const VyGemm*, const GemmDev&);
+template int launch_gemm<__nv_bfloat16, 256, false, false, false, WB_F32>(const VyGemm*, const GemmDev&);
+}  // namespace vy

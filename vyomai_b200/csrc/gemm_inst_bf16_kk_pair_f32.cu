@@ -1,0 +1,7 @@
+// explicit instantiations of the vy_gemm kernels whose epilogue is the staged fp32 one (see gemm_kernel.cuh)
+#include "gemm_kernel.cuh"
+namespace vy {
+template int launch_gemm<__nv_bfloat16, 128, false, false, true, WB_F32>(const VyGemm*, const GemmDev&);
+template int launch_gemm<__nv_bfloat16, 192, false, false, true, WB_F32>(const VyGemm*, const GemmDev&);
+template int launch_gemm<__nv_bfloat16, 256, false, false, true, WB_F32>(const VyGemm*, const GemmDev&);
+}  // namespace vy

@@ -597,6 +597,90 @@ __device__ __forceinline__ void epilogue_swiglu_fast(const GemmDev& g, uint32_t 
   __syncwarp();
 }
 
+// Write-back of fp32 results (what the packed-step decoders' projections and the fp32 layers give): bias, activation and addend in registers,
+// then boxes of [32 rows x 16 columns] (64-byte rows, the staging geometry of the bf16 epilogues) by bulk tensor stores, two buffers in turn.
+// One row per lane straight to global memory (epilogue_linear_general) is 32 pieces of 32 bytes an instruction, and that, not the mainloop, set the
+// pace of these products: bf16 7970 x 5152, K 1024: 183.7 us, so 70.7 (1189 TFLOP/s, result 2.3 TB/s); 7970 x 1536, K 512: 63.4, 17.5; tf32 1576 x 3072, K 768: 39.2, 18.9.
+template <int BN>
+__device__ __forceinline__ void epilogue_f32_fast(const GemmDev& g, uint32_t tmem_acc, int m0, int n0, int q, int half, int lane,
+                                                  uint64_t* tfull_bar, uint32_t tfull_phase, uint32_t tmem_empty_bar, uint8_t* stage,
+                                                  const CUtensorMap* tma_out) {
+  constexpr int WC = BN >= 64 ? BN / 2 : BN;
+  constexpr int NCH = WC / 32;
+  if (BN < 64 && half) {  // as in epilogue_linear_general: an idle warp arrives once per tile, once the tile exists
+    mbar_wait_soft(tfull_bar, tfull_phase, g.poison);
+    release_acc(tmem_empty_bar, lane);
+    return;
+  }
+  const int wcol0 = BN >= 64 ? half * WC : 0;
+  const int grow = m0 + q * 32 + lane;
+  const int gc0 = n0 + wcol0;
+  const float scale = g.out_scale == 0.f ? 1.f : g.out_scale;
+  const int sw = (lane >> 1) & 3;
+  const long long arow = g.addend && grow < g.M ? remap_add_row(g, grow) * g.ld_addend + gc0 : -1;
+  float add[32];
+  const auto fetch = [&](int c) {  // the row operand of chunk c; a row's last columns one by one
+    if (arow < 0 || c >= NCH) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = gc0 + c * 32 + j * 8;
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (col + 8 <= g.N) {
+        ld8_as_float(g.addend, g.addend_dtype, arow + c * 32 + j * 8, v);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (col + k < g.N) v[k] = ld_as_float(g.addend, g.addend_dtype, arow + c * 32 + j * 8 + k);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) add[j * 8 + k] = v[k];
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < 32; ++j) add[j] = 0.f;
+  fetch(0);
+  mbar_wait_soft(tfull_bar, tfull_phase, g.poison);
+  tc_fence_after();
+#pragma unroll 1
+  for (int c = 0; c < NCH; ++c) {
+    uint32_t raw[32];
+    tmem_ld_x32(tmem_acc + wcol0 + c * 32, raw);
+    tmem_ld_wait();
+    if (c == NCH - 1) release_acc(tmem_empty_bar, lane);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int col0 = gc0 + c * 32 + h * 16;
+      if (col0 >= g.N) continue;
+      uint8_t* srow = stage + h * GEMM_STAGE_OUT + lane * 64;
+      if (elect_one_sync()) tma_store_wait_read<1>();  // the store before the last, out of this buffer, has been read
+      __syncwarp();
+#pragma unroll
+      for (int j8 = 0; j8 < 2; ++j8) {
+        float x[8], bb[8];
+        load_bias8(g, col0 + j8 * 8, bb);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(raw[h * 16 + j8 * 8 + j]) + bb[j];
+        if (g.act != VY_ACT_NONE) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[j] = apply_act(g.act, x[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = (x[j] + add[h * 16 + j8 * 8 + j]) * scale;
+        *reinterpret_cast<float4*>(srow + (((2 * j8) ^ sw) << 4)) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4*>(srow + (((2 * j8 + 1) ^ sw) << 4)) = make_float4(x[4], x[5], x[6], x[7]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (elect_one_sync()) {
+        tma_store_2d(tma_out, stage + h * GEMM_STAGE_OUT, col0, m0 + q * 32);
+        tma_store_commit();
+      }
+    }
+    fetch(c + 1);
+  }
+  __syncwarp();
+}
+
 // split-K epilogue: the raw fp32 accumulators of this (tile, split) unit go to the workspace slab of the split;
 // vy_gemm's reduce kernel sums the slabs and applies bias / addend / scale.
 template <int BN>
@@ -797,10 +881,11 @@ __device__ __forceinline__ void epilogue_qkv_rope(const GemmDev& g, uint32_t tme
 // --------------------------------------------------------------------------------------------
 // kernel
 // --------------------------------------------------------------------------------------------
-// GATED: the kernel's only epilogue is the staged SwiGLU one (epilogue_swiglu_fast). It is a separate instantiation so that
-// the register allocation of the other epilogues does not change with it (inlined next to them it cost the split-K /
-// plain paths a few spills and ~5 % on the weight-gradient GEMMs).
-template <typename TIn, int BN, bool A_MN, bool B_MN, bool PAIR, bool GATED = false>
+// WB: the write-backs that the kernel holds: WB_ANY all but the two that follow, WB_GATED the staged SwiGLU one alone (epilogue_swiglu_fast),
+// WB_F32 the staged fp32 one alone (epilogue_f32_fast). They are instantiations of their own so that the register allocation of the other
+// epilogues does not change with them (inlined next to them SwiGLU cost the split-K / plain paths a few spills and ~5 % on the weight-gradient GEMMs).
+enum { WB_ANY = 0, WB_GATED = 1, WB_F32 = 2 };
+template <typename TIn, int BN, bool A_MN, bool B_MN, bool PAIR, int WB = WB_ANY>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
             const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_aux,
@@ -1041,7 +1126,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       // where this warp announces that it has drained the accumulator: the (leader's) MMA thread waits there
       const uint32_t tempty_addr = PAIR ? mapa_u32(smem_u32(&tempty_bar[acc]), 0) : smem_u32(&tempty_bar[acc]);
       VY_TRACE(2 + e, local, 0);
-      if (!GATED && !g.transposed_out && g.k_splits <= 1 && fast_mode < 0) {  // the fast epilogues read the bias straight from global
+      if (WB == WB_ANY && !g.transposed_out && g.k_splits <= 1 && fast_mode < 0) {  // the fast epilogues read the bias straight from global
         for (int j = et; j < BN; j += GEMM_EPI_WARPS * 32) {
           const int col = n0 + j;
           bs[j] = (g.bias && col < g.N) ? ld_as_float(g.bias, g.bias_dtype, col) : 0.f;
@@ -1049,8 +1134,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         named_bar_sync(1, GEMM_EPI_WARPS * 32);
       }
       const uint32_t tmem_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      if constexpr (GATED) {
+      if constexpr (WB == WB_GATED) {
         epilogue_swiglu_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, &tma_out);
+        continue;
+      }
+      if constexpr (WB == WB_F32) {
+        epilogue_f32_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, &tma_out);
         continue;
       }
       if (g.debug & 1) {
@@ -1133,7 +1222,8 @@ static inline int get_tmap_2d(CUtensorMap* out, int dtype, const void* base, uin
   return get_tensor_map_cached(out, dtype, 2, base, dims, strides, box, swz);
 }
 
-template <typename TIn, int BN, bool A_MN, bool B_MN, bool PAIR, bool GATED = false>
+constexpr int NO_OUT_MAP = -1000;   // launch_gemm with WB_F32: the output has no tensor map; nothing was launched
+template <typename TIn, int BN, bool A_MN, bool B_MN, bool PAIR, int WB = WB_ANY>
 int launch_gemm(const VyGemm* p, const GemmDev& g) {
   using Cfg = GemmCfg<TIn, BN>;
   const int dt = p->in_dtype;
@@ -1154,13 +1244,15 @@ int launch_gemm(const VyGemm* p, const GemmDev& g) {
   // write-back tensor maps of the fast epilogues: [32 cols x 32 rows] bf16 boxes, SWIZZLE_64B (the staging layout)
   CUtensorMap tout = ta, taux = ta;
   GemmDev gl = g;
-  if (g.tma_store) {
+  if constexpr (WB == WB_F32) {   // [16 cols x 32 rows] fp32 boxes
+    if (get_tmap_2d(&tout, VY_F32, p->out, p->N, p->M, p->ld_out * 4, 16, 32, 3) != VY_OK) return NO_OUT_MAP;
+  } else if (g.tma_store) {
     rc = get_tmap_2d(&tout, VY_BF16, p->out, p->act == VY_ACT_SWIGLU ? p->N / 2 : p->N, p->M, p->ld_out * 2, 32, 32, 3);
     if (rc == VY_OK && p->aux && (p->act == VY_ACT_GELU_ERF))
       rc = get_tmap_2d(&taux, VY_BF16, p->aux, p->N, p->M, p->ld_aux * 2, 32, 32, 3);
     if (rc != VY_OK) gl.tma_store = 0;  // fall back to the staged st.global write-back
   }
-  auto kern = gemm_kernel<TIn, BN, A_MN, B_MN, PAIR, GATED>;
+  auto kern = gemm_kernel<TIn, BN, A_MN, B_MN, PAIR, WB>;
   constexpr int smem_bytes = PAIR ? Cfg::PAIR_SMEM_BYTES : Cfg::SMEM_BYTES;
   static std::atomic<unsigned long long> allowed{0};  // per instantiation
   VY_CUDA_OK(allow_smem(kern, allowed));
