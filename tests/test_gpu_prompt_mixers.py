@@ -1,4 +1,4 @@
-"""The prompt-sized forms of the packed decoders' mixers (csrc/window_attn_mma.cu, talk_attn_mma.cu, linear_attn_mma.cu, delta_rule_mma.cu) at
+"""The prompt-sized forms of the packed decoders' mixers (csrc/window_attn_tc.cu, window_attn_mma.cu, talk_attn_mma.cu, linear_attn_mma.cu, delta_rule_mma.cu) at
 the edges of their tiles and of the rules that choose them, against the float64 oracles and against the form that the same call takes
 without the lent workspace. Bound: an fp32 result off by a few units in the last place of its row's largest term per contraction, 16 * 2^-24 of the
 output's 2-norm (about 1e-6; the kernels measure 1e-7 to 3e-7)."""
@@ -524,6 +524,51 @@ def test_prompt_attention_in_blocks_of_192_rows(form, H, G, d, dv, window, keep)
     got = ops.window_attn(batch, torch.cat([q[s][pos0[s]:].reshape(new[s], -1) for s in range(len(new))]).to(DEV), kp.to(DEV), vp.to(DEV), heads=H, kv_heads=G, dim=d, vdim=dv,
                           scale=1.0, window=window, keep_first=keep, weights=form, out_dtype=torch.float32)
     assert _err(got, torch.cat(want)) < BOUND
+
+
+@pytest.mark.parametrize("form,H,G,d,dv,window,keep,chunk,cap,new,pos0", [
+    ("softmax", 2, 2, 64, 64, 0, 0, 0, 0.0, [128, 127, 64, 1, 65], [0, 64, 65, 200, 63]),          # one tile, whole tiles, an odd number of them
+    ("softmax", 8, 2, 128, 128, 70, 0, 0, 30.0, [193, 33, 130, 1], [0, 100, 31, 190]),              # bands that start inside a tile
+    ("sigmoid", 8, 2, 128, 96, 0, 0, 0, 0.0, [131, 40, 257], [0, 90, 3]),
+    ("softmax", 16, 1, 96, 64, 50, 70, 0, 0.0, [140, 9, 300], [0, 200, 77]),                         # kept tokens: two tiles of them, one of them inside the band
+    ("sigmoid", 4, 1, 33, 7, 20, 5, 0, 0.0, [150, 16], [10, 300]),
+    ("softmax", 3, 3, 112, 128, 0, 0, 48, 0.0, [200, 47, 96], [0, 50, 144]),                         # blocks of 48 positions
+    ("softmax", 6, 3, 16, 24, 129, 0, 0, 5.0, [385, 66], [0, 130]),
+    ("sigmoid", 4, 4, 128, 128, 0, 0, 0, 0.0, [100, 37, 64] * 25, [0, 3, 40] * 25),                  # fewer rows than a tile, many sequences: 192 rows on mma.sync
+])
+def test_prompt_attention_on_tcgen05(form, H, G, d, dv, window, keep, chunk, cap, new, pos0):
+    """The edges of 64-key tiles, of pairs of them and of 128-row blocks, in every form of the scores, with sinks, gates and slopes; padded query rows."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(d + dv)
+    rep, bs, T = H // G, 16, [n + p for n, p in zip(new, pos0)]
+    q, k, v = ([torch.randn(t, n, w, generator=g) / d ** (0.25 if i < 2 else 0) for t in T] for i, (n, w) in enumerate(((H, d), (G, d), (G, dv))))
+    sink, gate, slopes = torch.randn(H, generator=g), [torch.randn(n, H, generator=g) for n in new], torch.tensor(OZ.head_slopes(H), dtype=torch.float32)
+    want = []
+    for s, t in enumerate(T):
+        i, j = torch.arange(pos0[s], t)[:, None], torch.arange(t)[None, :]
+        seen = (j <= i) & ((i - j < window) | (j < keep)) if window else (j <= i) & (j >= i // chunk * chunk) if chunk else j <= i
+        kk, vv = (x[s].double().repeat_interleave(rep, 1) for x in (k, v))
+        sc = torch.einsum("ihd,jhd->hij", q[s][pos0[s]:].double(), kk) * 1.5
+        if cap:
+            sc = cap * torch.tanh(sc / cap) - slopes.double()[:, None, None] * (i - j)
+        if form == "softmax":
+            p = torch.softmax(torch.cat([sc.masked_fill(~seen, -torch.inf), sink.double()[:, None, None].expand(H, new[s], 1)], 2), 2)[:, :, :t]
+        else:
+            p = torch.sigmoid(sc) * seen
+        want.append((torch.einsum("hij,jhd->ihd", p, vv) * torch.sigmoid(gate[s].double())[:, :, None]).reshape(new[s], -1))
+    batch, table, _, n_blocks, _ = shuffled_batch(new, pos0, bs, DEV, seed=d)
+    kp, vp = torch.full((n_blocks, bs, G, d), 1e3), torch.full((n_blocks, bs, G, dv), 1e3)
+    for s, t in enumerate(T):
+        rows = torch.tensor([table[s][p // bs] for p in range(t)])
+        kp[rows, torch.arange(t) % bs], vp[rows, torch.arange(t) % bs] = k[s], v[s]
+    wide = torch.cat([torch.cat([q[s][pos0[s]:].reshape(new[s], -1) for s in range(len(new))]), torch.zeros(sum(new), 3)], 1).to(DEV)[:, :-3]
+    call = lambda: ops.window_attn(batch, wide, kp.to(DEV), vp.to(DEV), heads=H, kv_heads=G, dim=d, vdim=dv, scale=1.5, window=window, keep_first=keep, chunk=chunk,  # noqa: E731
+                                   weights=form, softcap=cap, head_slope=slopes.to(DEV) if cap else None, sink=sink.to(DEV) if form == "softmax" else None,
+                                   gate=torch.cat(gate).to(DEV), out_dtype=torch.float32)
+    got = call()
+    # a capped score is cap (1 - 2 r) with r in [0, 1] off by a unit in its last place: cap 2^-24 as an exponent, as much as that of the weight
+    assert _err(got, torch.cat(want)) < BOUND + cap * 2.0 ** -24
+    assert torch.equal(call(), got)
 
 
 def test_delta_rule_form_for_one_prompt_beside_many_tokens():

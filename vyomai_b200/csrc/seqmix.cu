@@ -911,7 +911,8 @@ extern "C" int64_t vy_window_attn_prompt_floats(int32_t n_seqs, int32_t max_new,
   WinDev d = {};
   d.tw = table_width; d.bs = block_size; d.kv_heads = kv_heads; d.dim = dim; d.vdim = vdim;
   d.window = window; d.keep = keep_first; d.chunk = chunk;
-  return window_attn_split_floats(d, n_seqs, max_new);
+  const long long mma = window_attn_split_floats(d, n_seqs, max_new), tc = window_attn_tc_floats(d, n_seqs, max_new);
+  return mma > tc ? mma : tc;
 }
 
 extern "C" int vy_window_attn(const VyWinAttn* p) {

@@ -136,6 +136,12 @@ __device__ __forceinline__ void visible_keys(const WinDev& d, int pos, int& nA, 
   else { nA = min(d.keep, pos + 1); lowB = max(pos - d.window + 1, nA); }
 }
 
+// the keys a portion sees, from its first query on: slots [0, nA) are positions [0, nA) (kept first tokens), the others positions from lo on
+__device__ __forceinline__ void portion_keys(const WinDev& d, int p0, int& nA, int& lo) {
+  lo = d.chunk > 0 ? p0 / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p0 - d.window + 1, 0);
+  nA = d.window <= 0 ? 0 : min(d.keep, lo);
+}
+
 // recurrences (linear attention with a fixed decay, gated delta rule): state [slots, heads, dim, vdim] fp32
 struct RecDev {
   const int* cu; const int* pos0; const int* slot;
@@ -169,13 +175,20 @@ cudaError_t launch_delta_rule_mma(const RecDev& d, int n_seqs, int max_new, long
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 template <bool TD>
 cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
-// Where the split rows of (sequence s, key / value head g) lie: slot (s * kv_heads + g) * cap + i holds the i-th key, K hi | K lo | V hi | V lo and 16 bytes
-// with the numbers that undo the scaling, 2^(exponent - SPLIT_TOP) of the key row and 2^exponent of the value row. The 16 bytes also make the
-// distance between rows an odd multiple of 16, as ldmatrix wants it in shared memory: a run of rows is one copy.
+// Where the split rows of (sequence s, key / value head g) lie: slot (s * kv_heads + g) * cap + i holds the i-th key, K hi | K lo | V hi | V lo, and the numbers
+// that undo the scaling, 2^(exponent - SPLIT_TOP) of the key row and 2^exponent of the value row. Two layouts:
+// - for mma.sync, channels filled up to 16, the two numbers in 16 bytes behind the row. The 16 bytes also make the distance between rows an odd multiple
+//   of 16, as ldmatrix wants it in shared memory: a run of rows is one copy;
+// - for tcgen05 (tail > 0), K hi | K lo filled up to a multiple of 64 entries together, V hi and V lo each, since a tensor map's box takes 128 bytes of a row;
+//   the numbers in an array of their own, and `tail` rows of zeros behind a list's last, which the last tile's box may take in.
 struct SplitKv {
   unsigned char* rows;
   long long cap;   // key slots per (sequence, key / value head)
-  int row_bytes;   // 4 (dim16 + vdim16) + 16
+  int row_bytes;
+  int k_lo, v_at, v_lo;   // bytes from a key's hi halves to its lo ones, to its values, from those to their lo halves
+  int vpad;        // channels that a value row's halves are filled up to
+  float* unit;     // a slot's two numbers, `ustep` floats between slots
+  int ustep, tail;
   uint4* range;    // [sequence, key / value head][blocks]: of a block of SPLIT_ROWS rows the largest key entry, the largest value entry and the smallest of its value
                    // rows' and columns' largest ones (zeros aside), as bits of floats
   int blocks;
@@ -204,6 +217,13 @@ __device__ __forceinline__ bool split_odd(const SplitKv& w, int sg, int keys, fl
 // splits the rows that some query of the step sees into ws (window_attn_split_floats(..) floats, 16-byte aligned), says where they are, sets `odd` to 0
 cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st);
 long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);
+// window_attn_tc.cu: the same rows for tcgen05, and the kernel that reads them (dim, vdim <= 128)
+bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new);
+long long window_attn_tc_floats(const WinDev& d, int n_seqs, int max_new);
+cudaError_t launch_window_attn_tc(const WinDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st);
+// key slots per (sequence, key / value head) that the step's queries can see at most (host-known bounds)
+long long split_slots(const WinDev& d, int max_new);
+cudaError_t launch_split_rows(const WinDev& d, int n_seqs, const SplitKv& w, cudaStream_t st);
 // on the tensor cores, as many sequences at a time as the workspace holds; in fp32 where it holds none
 cudaError_t launch_window_attn_prompt(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches);
 // in fp32 (seqmix_tiled.cu); odd: null, or what the tensor-core form leaves to do

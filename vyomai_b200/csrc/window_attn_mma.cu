@@ -1,4 +1,5 @@
-// Prompt-sized windowed attention over pages (vy_window_attn, portions of several tokens): scores and weighted values in fp32 precision
+// Prompt-sized windowed attention over pages (vy_window_attn, portions of several tokens) where window_attn_tc.cu does not apply - short portions, more
+// than 128 channels, little scratch - and the splitting of keys and values for both: scores and weighted values in fp32 precision
 // on the tensor cores, operands split into two fp16 parts (split_mma.cuh), online softmax in registers.
 //
 // A first launch splits every key and value row that some query of the step sees, once, into a workspace in the order the tiles read
@@ -20,17 +21,11 @@
 
 namespace vy {
 
-// the keys a portion sees, from its first query on: slots [0, nA) are positions [0, nA) (kept first tokens), the others positions from lo on
-__device__ __forceinline__ void portion_keys(const WinDev& d, int p0, int& nA, int& lo) {
-  lo = d.chunk > 0 ? p0 / d.chunk * d.chunk : d.window <= 0 ? 0 : max(p0 - d.window + 1, 0);
-  nA = d.window <= 0 ? 0 : min(d.keep, lo);
-}
-
 constexpr int WS_T = 8 * SPLIT_ROWS;   // splitting launch: eight lanes per row
 
 // bound by the bytes: every row read once and written once (8000 rows of 2 x (128 + 128) channels: 33 MB)
 template <int MAXD>
-__global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, SplitKv w, int dim16, int vdim16, bool kvvec) {
+__global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, SplitKv w, int dim16, bool kvvec) {
   pdl_trigger();
   pdl_wait();
   const int s = blockIdx.z, g = blockIdx.y, n = d.cu[s + 1] - d.cu[s], p0 = d.pos0[s];
@@ -41,6 +36,11 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
   const long long slot0 = (static_cast<long long>(s) * d.kv_heads + g) * w.cap;
   const int r0 = blockIdx.x * SPLIT_ROWS, sg = s * d.kv_heads + g;
   if (blockIdx.x == 0 && threadIdx.x == 0) w.odd[sg] = 0;
+  // zeros behind the list, units too (rows the last tile's box takes in must not hold what their bits happen to say)
+  for (int r = max(r0, count); w.tail > 0 && r < min(r0 + SPLIT_ROWS, count + w.tail) && slot0 + r < (static_cast<long long>(s) * d.kv_heads + g + 1) * w.cap; ++r) {
+    for (int x = threadIdx.x; x < w.row_bytes / 16; x += WS_T) *reinterpret_cast<uint4*>(w.rows + (slot0 + r) * w.row_bytes + 16 * x) = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < 2) w.unit[(slot0 + r) * w.ustep + threadIdx.x] = 0.f;
+  }
   if (r0 >= count) return;
   __shared__ unsigned top_k, top_v, low_v;   // positive numbers order like their bits (and NaN after infinity)
   __shared__ long long row_s[SPLIT_ROWS];
@@ -56,13 +56,13 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
   }
   __syncthreads();
   unsigned char* out = w.rows + (slot0 + r0) * w.row_bytes;
-  float* unit = reinterpret_cast<float*>(out + 4 * (dim16 + vdim16));
-  split_rows<WS_T / 32, MAXD>(out, out + 2 * dim16, w.row_bytes, unit, SPLIT_TOP, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
-                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; }, SameValue(), w.row_bytes / 4,
+  float* unit = w.unit + (slot0 + r0) * w.ustep;
+  split_rows<WS_T / 32, MAXD>(out, out + w.k_lo, w.row_bytes, unit, SPLIT_TOP, rows, d.dim, dim16, d.kp, d.pool_dt, kvvec,
+                              [&](int r) { return row_of(r) * d.k_row + static_cast<long long>(g) * d.dim; }, SameValue(), w.ustep,
                               [&](float m) { atomicMax(&top_k, __float_as_uint(m)); });
-  out += 4 * dim16;
-  split_rows<WS_T / 32, MAXD>(out, out + 2 * vdim16, w.row_bytes, unit + 1, 0, rows, d.vdim, vdim16, d.vp, d.pool_dt, kvvec,
-                              [&](int r) { return row_s[r]; }, SameValue(), w.row_bytes / 4, [&](float m) {
+  out += w.v_at;
+  split_rows<WS_T / 32, MAXD>(out, out + w.v_lo, w.row_bytes, unit + 1, 0, rows, d.vdim, w.vpad, d.vp, d.pool_dt, kvvec,
+                              [&](int r) { return row_s[r]; }, SameValue(), w.ustep, [&](float m) {
                                 if (m > 0.f) atomicMin(&low_v, __float_as_uint(m));
                               });
   for (int c0 = 0; c0 < d.vdim; c0 += WS_T) {   // columns, from the L1 cache
@@ -361,8 +361,7 @@ __global__ void __launch_bounds__(32 * NW, 1) window_attn_mma_kernel(WinDev d, S
 
 static int round16(int n) { return (n + 15) & ~15; }
 
-// key slots per (sequence, key / value head): what the step's queries can see at most (host-known bounds)
-static long long split_slots(const WinDev& d, int max_new) {
+long long split_slots(const WinDev& d, int max_new) {
   const long long all = static_cast<long long>(d.tw) * d.bs;
   const long long seen = d.chunk > 0 ? static_cast<long long>(d.chunk) + max_new : d.window > 0 ? static_cast<long long>(d.window) + d.keep + max_new : all;
   return seen < all ? seen : all;
@@ -381,17 +380,28 @@ static bool kv_quads(const WinDev& d) {
 }
 
 cudaError_t launch_window_attn_split(const WinDev& d, int n_seqs, int max_new, float* ws, SplitKv* w, cudaStream_t st) {
-  const int dim16 = round16(d.dim), vdim16 = round16(d.vdim), big = d.dim > d.vdim ? d.dim : d.vdim;
+  const int dim16 = round16(d.dim), vdim16 = round16(d.vdim);
   w->cap = split_slots(d, max_new);
   w->row_bytes = 4 * (dim16 + vdim16) + 16;
+  w->k_lo = 2 * dim16;
+  w->v_at = 4 * dim16;
+  w->v_lo = 2 * vdim16;
+  w->vpad = vdim16;
+  w->ustep = w->row_bytes / 4;
+  w->tail = 0;
   w->blocks = static_cast<int>(split_blocks(d, max_new));
   const long long lists = static_cast<long long>(n_seqs) * d.kv_heads;
   w->rows = reinterpret_cast<unsigned char*>(ws);
   w->range = reinterpret_cast<uint4*>(w->rows + lists * w->cap * w->row_bytes);
   w->odd = reinterpret_cast<int*>(w->range + lists * w->blocks);
-  const dim3 grid(w->blocks, d.kv_heads, n_seqs);
-  return big <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d))
-                    : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, *w, dim16, vdim16, kv_quads(d));
+  w->unit = reinterpret_cast<float*>(w->rows + 4 * (dim16 + vdim16));
+  return launch_split_rows(d, n_seqs, *w, st);
+}
+
+cudaError_t launch_split_rows(const WinDev& d, int n_seqs, const SplitKv& w, cudaStream_t st) {
+  const dim3 grid(w.blocks, d.kv_heads, n_seqs);
+  return d.dim <= 128 && d.vdim <= 128 ? launch_kernel(window_attn_split_kernel<128>, grid, dim3(WS_T), 0, st, d, w, round16(d.dim), kv_quads(d))
+                                       : launch_kernel(window_attn_split_kernel<256>, grid, dim3(WS_T), 0, st, d, w, round16(d.dim), kv_quads(d));
 }
 
 template <int MAXD, int VT, int NW, int N, int NS, bool SIG>
@@ -443,17 +453,37 @@ static cudaError_t launch_window_attn_mma(const WinDev& d, const SplitKv& w, int
   return d.dim <= 64 ? launch_wm_pick<64, 64>(d, w, n_seqs, max_new, hl, st) : launch_wm_pick<128, 64>(d, w, n_seqs, max_new, hl, st);
 }
 
+static WinDev from_sequence(const WinDev& d, int s) {
+  WinDev e = d;
+  e.cu += s;
+  e.pos0 += s;
+  e.table += static_cast<long long>(s) * d.tw;
+  return e;
+}
+
 cudaError_t launch_window_attn_prompt(const WinDev& d, int n_seqs, int max_new, float* ws, long long ws_floats, cudaStream_t st, int* launches) {
   *launches = 1;
-  const long long fit = ws && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && d.kv_heads <= 65535 ? ws_floats / window_attn_split_floats(d, 1, max_new) : 0;
+  const bool aligned = ws && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && d.kv_heads <= 65535;
+  if (aligned && window_attn_tc_applies(d, n_seqs, max_new) && window_attn_tc_floats(d, 1, max_new) <= ws_floats) {
+    const long long fit = ws_floats / window_attn_tc_floats(d, 1, max_new);
+    *launches = 0;
+    for (int s = 0; s < n_seqs; s += static_cast<int>(fit < n_seqs ? fit : n_seqs)) {
+      const int ns = static_cast<int>(fit < n_seqs - s ? fit : n_seqs - s);
+      const WinDev e = from_sequence(d, s);
+      const int* odd = nullptr;
+      cudaError_t err = launch_window_attn_tc(e, ns, max_new, ws, &odd, st);
+      if (err == cudaSuccess) err = launch_window_attn_tiled(e, ns, max_new, odd, st);
+      if (err != cudaSuccess) return err;
+      *launches += 3;
+    }
+    return cudaSuccess;
+  }
+  const long long fit = aligned ? ws_floats / window_attn_split_floats(d, 1, max_new) : 0;
   if (fit < 1) return launch_window_attn_tiled(d, n_seqs, max_new, nullptr, st);
   *launches = 0;
   for (int s = 0; s < n_seqs; s += static_cast<int>(fit < n_seqs ? fit : n_seqs)) {   // as many sequences at a time as the workspace holds
     const int ns = static_cast<int>(fit < n_seqs - s ? fit : n_seqs - s);
-    WinDev e = d;
-    e.cu += s;
-    e.pos0 += s;
-    e.table += static_cast<long long>(s) * d.tw;
+    const WinDev e = from_sequence(d, s);
     SplitKv w = {};
     cudaError_t err = launch_window_attn_split(e, ns, max_new, ws, &w, st);
     if (err == cudaSuccess) err = launch_window_attn_mma(e, w, ns, max_new, st);
