@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define VY_ABI_VERSION 14
+#define VY_ABI_VERSION 15
 
 #if defined(__GNUC__)
 #define VY_API __attribute__((visibility("default")))
@@ -1339,6 +1339,65 @@ typedef struct VyDpAdamW {
 VY_API int vy_dp_barrier(const VyDpGroup* g, void* stream);
 VY_API int vy_dp_reduce_shard(const VyDpGroup* g, const VyDpReduce* p);
 VY_API int vy_dp_adamw_shard(const VyDpGroup* g, const VyDpAdamW* p);
+
+/* ---- whole sublayers of a transformer layer in one call ----
+ * The launches of the attention block (VyomAI/layers/attention.py:57-133, 190-215; VyomAI/models/decoder.py:87-111) and of the feed-forward block
+ * (VyomAI/layers/ffn.py:32-40), forward and backward, each exactly as the single entry points above make it. All tensors are contiguous, of one dtype and on one
+ * device; head_dim is 64; no dropout. `scratch` (vy_*_block_bytes) holds what lies between the launches; with `save` it is what the backward call reads, and
+ * must then be handed to it unchanged. `work` (vy_*_block_work_bytes) is the backward call's own. hint_*: tilings, VyGemm's hint_flavour | hint_bn << 4 |
+ * hint_splits << 16 (0: the library's choice). Products of at most VY_BLOCK_SWAP_ROWS rows are computed transposed (VyGemm.transposed_out). */
+#define VY_BLOCK_SWAP_ROWS 64
+typedef struct VyAttnBlock {
+  int32_t seqs, tokens, width, heads, kv_heads, dtype; /* rows = seqs * tokens */
+  const void* x;                                       /* [rows, width]; y = LayerNorm(attention(x) W_out^T + b_out + x) */
+  const void *w_qkv, *b_qkv, *w_out, *b_out, *gamma, *beta; /* w_qkv [(heads + 2 kv_heads) * 64, width], w_out [width, heads * 64]; biases may be NULL */
+  float eps;
+  const float *rope_cos, *rope_sin; /* or NULL */
+  int32_t rope_rows, rope_pos;      /* table row of the first token */
+  const uint8_t* key_padding;       /* or NULL */
+  int64_t kpm_stride;
+  int32_t causal, q_pos0;
+  void *k_cache, *v_cache; /* [>= seqs, kv_heads, cache_len, 64] or NULL; keys and values go to slots start .. start + tokens, slots [0, start + tokens) are attended */
+  int64_t c_sb, c_sh, c_sl;
+  int32_t cache_dtype, cache_len, start;
+  int32_t decode;     /* one token per sequence, no mask: vy_attn_decode on a cache of either dtype (else a cache is bf16) */
+  uint32_t* tickets;  /* decode: >= seqs * kv_heads zeros */
+  int32_t weights_static, save;
+  void *y, *scratch;
+  int64_t scratch_bytes;
+  /* backward */
+  const void* dy;
+  void *dx, *dw_qkv, *db_qkv, *dw_out, *db_out, *dgamma, *dbeta; /* db_qkv, db_out: NULL without the bias */
+  void *work, *split_ws;                                          /* split_ws: VyGemm.workspace */
+  int64_t work_bytes, split_bytes;
+  int32_t hint_qkv, hint_out, hint_dw_out, hint_d_out, hint_d_qkv, hint_dw_qkv;
+  void* stream;
+} VyAttnBlock;
+
+typedef struct VyFfnBlock {
+  int32_t rows, width, inner, dtype, act, dact; /* VY_ACT_* of the first product and of its gradient */
+  const void *h, *input;                        /* y = LayerNorm(act(h W1^T + b1) W2^T + b2 + input) */
+  const void *w1, *b1, *w2, *b2, *gamma, *beta; /* w1 [inner, width], w2 [width, inner] */
+  float eps;
+  int32_t weights_static, save;
+  void *y, *scratch;
+  int64_t scratch_bytes;
+  const void* dy;
+  void *dh, *d_input, *dw1, *db1, *dw2, *db2, *dgamma, *dbeta;
+  void *work, *split_ws;
+  int64_t work_bytes, split_bytes;
+  int32_t hint_1, hint_2, hint_dw2, hint_d2, hint_dw1, hint_d1;
+  void* stream;
+} VyFfnBlock;
+
+VY_API int64_t vy_attn_block_bytes(const VyAttnBlock* p);
+VY_API int64_t vy_attn_block_work_bytes(const VyAttnBlock* p);
+VY_API int vy_attn_block_fwd(const VyAttnBlock* p);
+VY_API int vy_attn_block_bwd(const VyAttnBlock* p);
+VY_API int64_t vy_ffn_block_bytes(const VyFfnBlock* p);
+VY_API int64_t vy_ffn_block_work_bytes(const VyFfnBlock* p);
+VY_API int vy_ffn_block_fwd(const VyFfnBlock* p);
+VY_API int vy_ffn_block_bwd(const VyFfnBlock* p);
 
 #ifdef __cplusplus
 }

@@ -11,7 +11,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from . import _lib, ops
+from . import _lib, block, gemm_tune, ops
 from . import functional as F
 from .functional import KVTarget, MaskSpec
 
@@ -20,30 +20,30 @@ def _needs_grad(*ts) -> bool:
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ts)
 
 
-def _qkv_params(mod):
-    lin = mod._packed()
-    ws = [l.weight for l in lin]
-    bs = [l.bias for l in lin if l.bias is not None]
-    return lin, ws, bs
-
-
 # ----------------------------------------------------------------------------------------------
 # attention block: qkv projection + RoPE + attention + output projection + residual + LayerNorm
 # ----------------------------------------------------------------------------------------------
 def attention_block_fn(mod, x2d: torch.Tensor, B: int, S: int, mask: MaskSpec, rope, kv: Optional[KVTarget],
                        start_pos: int, decode_no_mask: bool) -> torch.Tensor:
-    lin, ws, bs = _qkv_params(mod)
-    dense, ln = mod.out.dense, mod.out.layernorm
-    if _needs_grad(x2d, *ws, dense.weight, ln.weight):
+    a = block.AttentionParts(mod)
+    if _needs_grad(x2d, *a.ws, a.wo, a.gamma):
         if kv is not None:
             raise _lib.VyomError("gradients through a kv-cache forward are not supported (use_cache=True is an inference path)")
         from .autograd_train import AttentionBlockFn
-        flat = [x2d] + ws + bs + [dense.weight] + ([dense.bias] if dense.bias is not None else []) + [ln.weight, ln.bias]
+        flat = [x2d] + a.ws + [b for b in a.bs if b is not None] + [a.wo] + ([a.bo] if a.bo is not None else []) + [a.gamma, a.beta]
         return AttentionBlockFn.apply(mod, B, S, mask, rope, start_pos, *flat)
-    w_qkv, b_qkv = F.pack_linears(lin)
-    attn, _ = F.attention_core(x2d, B, S, w_qkv, b_qkv, mod.num_attention_heads, mod._kv_heads, mask, rope, kv,
-                               decode_no_mask, pos0=start_pos)
-    y, _ = F.self_output(attn, x2d, dense, ln, dropout=F.dropout_state(mod.out, mod.out.dropout.p))
+    key = block.attention_key(a, x2d, B, S, mask, rope, kv, decode_no_mask, False)
+    hints = gemm_tune.LAYERS.get(key)
+    if hints is not None:
+        return block.attention_forward(a, x2d, B, S, mask, rope, kv, start_pos, key, hints)[0]
+    lin, dense, ln = a.lin, a.dense, a.ln
+    with gemm_tune.collecting() as got:
+        w_qkv, b_qkv = F.pack_linears(lin)
+        attn, _ = F.attention_core(x2d, B, S, w_qkv, b_qkv, mod.num_attention_heads, mod._kv_heads, mask, rope, kv,
+                                   decode_no_mask, pos0=start_pos)
+        y, _ = F.self_output(attn, x2d, dense, ln, dropout=F.dropout_state(mod.out, mod.out.dropout.p))
+    if key is not None:
+        gemm_tune.keep_layer(key, got, 2)
     return y
 
 
@@ -80,12 +80,21 @@ def self_output_fn(attn2d: torch.Tensor, residual2d: torch.Tensor, dense: nn.Lin
 
 
 def feed_forward_fn(mod, h2d: torch.Tensor, input2d: torch.Tensor) -> torch.Tensor:
-    inter, out, ln = mod.intermediate, mod.out, mod.layernorm
-    if _needs_grad(h2d, input2d, inter.weight, out.weight, ln.weight):
+    m = mod._modules
+    inter, out, ln, param = m["intermediate"], m["out"], m["layernorm"], block._param
+    w1, b1, w2, b2, gamma, beta = param(inter, "weight"), param(inter, "bias"), param(out, "weight"), param(out, "bias"), param(ln, "weight"), param(ln, "bias")
+    train = _needs_grad(h2d, input2d, w1, w2, gamma)
+    key = block.ffn_key(mod._act_name, h2d, input2d, w1, b1, w2, b2, ln, gamma, beta, mod.training and m["dropout"].p > 0.0, train)
+    if train:
         from .autograd_train import FeedForwardFn
-        return FeedForwardFn.apply(mod._act_name, ln.eps, F.dropout_state(mod, mod.dropout.p), h2d, input2d, inter.weight,
-                                   inter.bias, out.weight, out.bias, ln.weight, ln.bias)
-    y, _ = F.feed_forward(h2d, input2d, inter, out, ln, act=mod._act_name, dropout=F.dropout_state(mod, mod.dropout.p))
+        return FeedForwardFn.apply(mod._act_name, ln.eps, F.dropout_state(mod, mod.dropout.p), key, h2d, input2d, w1, b1, w2, b2, gamma, beta)
+    hints = gemm_tune.LAYERS.get(key)
+    if hints is not None:
+        return block.ffn_forward(mod._act_name, h2d, input2d, w1, b1, w2, b2, gamma, beta, ln.eps, hints)[0]
+    with gemm_tune.collecting() as got:
+        y, _ = F.feed_forward(h2d, input2d, inter, out, ln, act=mod._act_name, dropout=F.dropout_state(mod, mod.dropout.p))
+    if key is not None:
+        gemm_tune.keep_layer(key, got, 2)
     return y
 
 

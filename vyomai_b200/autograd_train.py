@@ -15,7 +15,7 @@ from typing import Optional
 
 import torch
 
-from . import ops
+from . import block, gemm_tune, ops
 from . import functional as F
 from .functional import MaskSpec
 
@@ -145,15 +145,25 @@ class AttentionBlockFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, mod, B, S, mask: MaskSpec, rope, start_pos, x2d, *params):
-        lin = mod._packed()
-        dense, ln = mod.out.dense, mod.out.layernorm
-        w_qkv, b_qkv = F.pack_linears(lin)
-        attn, saved = F.attention_core(x2d, B, S, w_qkv, b_qkv, mod.num_attention_heads, mod._kv_heads, mask, rope,
-                                       None, False, need_lse=True, pos0=start_pos)
-        q, k, v, lse = saved
-        ctx.drop = F.dropout_state(mod.out, mod.out.dropout.p)
-        y, (s, mean, rstd) = F.self_output(attn, x2d, dense, ln, save=True, dropout=ctx.drop)
         ctx.mod, ctx.B, ctx.S, ctx.mask, ctx.rope, ctx.start_pos = mod, B, S, mask, rope, start_pos
+        parts = block.AttentionParts(mod)
+        ctx.key = key = block.attention_key(parts, x2d, B, S, mask, rope, None, False, True)
+        hints = gemm_tune.LAYERS.get(key)
+        ctx.whole = hints is not None and ("backward", key) in gemm_tune.LAYERS   # both directions as one call each, or neither
+        if ctx.whole:
+            y, scratch = block.attention_forward(parts, x2d, B, S, mask, rope, None, start_pos, key, hints, save=True)
+            ctx.save_for_backward(x2d, scratch)
+            return y
+        lin, dense, ln = parts.lin, parts.dense, parts.ln
+        with gemm_tune.collecting() as got:
+            w_qkv, b_qkv = F.pack_linears(lin)
+            attn, saved = F.attention_core(x2d, B, S, w_qkv, b_qkv, mod.num_attention_heads, mod._kv_heads, mask, rope,
+                                           None, False, need_lse=True, pos0=start_pos)
+            q, k, v, lse = saved
+            ctx.drop = F.dropout_state(mod.out, mod.out.dropout.p)
+            y, (s, mean, rstd) = F.self_output(attn, x2d, dense, ln, save=True, dropout=ctx.drop)
+        if key is not None:
+            gemm_tune.keep_layer(key, got, 2)
         ctx.n_w = len(lin)
         ctx.has_qkv_bias = lin[0].bias is not None
         ctx.has_dense_bias = dense.bias is not None
@@ -162,6 +172,18 @@ class AttentionBlockFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
+        if ctx.whole:
+            x2d, scratch = ctx.saved_tensors
+            return (None, None, None, None, None, None, *block.attention_backward(block.AttentionParts(ctx.mod), x2d, scratch, dy.contiguous(), ctx.B, ctx.S, ctx.mask,
+                                                                                  ctx.rope, ctx.start_pos, gemm_tune.LAYERS.get(("backward", ctx.key), (0, 0, 0, 0))))
+        with gemm_tune.collecting() as got:
+            grads = AttentionBlockFn._launches(ctx, dy)
+        if ctx.key is not None:
+            gemm_tune.keep_layer(("backward", ctx.key), got, 4)
+        return grads
+
+    @staticmethod
+    def _launches(ctx, dy):
         x2d, q, k, v, attn, lse, s, mean, rstd = ctx.saved_tensors
         mod, B, S, mask, rope = ctx.mod, ctx.B, ctx.S, ctx.mask, ctx.rope
         lin = mod._packed()
@@ -315,23 +337,44 @@ class FeedForwardFn(torch.autograd.Function):
     """y = LN(W2 act(W1 h + b1) + b2 + input)."""
 
     @staticmethod
-    def forward(ctx, act, eps, dropout, h2d, input2d, w1, b1, w2, b2, gamma, beta):
-        z = torch.empty((h2d.shape[0], w1.shape[0]), device=h2d.device, dtype=h2d.dtype)
-        a = F._lin(h2d, w1, b1, act=act, aux=z)
-        if dropout is None:
-            s = F._lin(a, w2, b2, addend=input2d)
-            y, _, mean, rstd = ops.add_layernorm(s, None, gamma, beta, eps, save_stats=True)
-        else:
-            y, s, mean, rstd = ops.add_layernorm(F._lin(a, w2, b2), input2d.contiguous(), gamma, beta, eps, save_stats=True,
-                                                 save_sum=True, dropout=dropout)
+    def forward(ctx, act, eps, dropout, key, h2d, input2d, w1, b1, w2, b2, gamma, beta):
         ctx.drop = dropout
-        ctx.act = act
+        ctx.act, ctx.eps, ctx.key = act, eps, key
         ctx.params = (w1, b1, w2, b2, gamma, beta)  # the Parameter objects (direct-gradient attributes live on them)
+        hints = gemm_tune.LAYERS.get(key)
+        ctx.whole = hints is not None and ("backward", key) in gemm_tune.LAYERS
+        if ctx.whole:
+            y, scratch = block.ffn_forward(act, h2d, input2d, w1, b1, w2, b2, gamma, beta, eps, hints, save=True)
+            ctx.save_for_backward(h2d, scratch)
+            return y
+        with gemm_tune.collecting() as got:
+            z = torch.empty((h2d.shape[0], w1.shape[0]), device=h2d.device, dtype=h2d.dtype)
+            a = F._lin(h2d, w1, b1, act=act, aux=z)
+            if dropout is None:
+                s = F._lin(a, w2, b2, addend=input2d)
+                y, _, mean, rstd = ops.add_layernorm(s, None, gamma, beta, eps, save_stats=True)
+            else:
+                y, s, mean, rstd = ops.add_layernorm(F._lin(a, w2, b2), input2d.contiguous(), gamma, beta, eps, save_stats=True,
+                                                     save_sum=True, dropout=dropout)
+        if key is not None:
+            gemm_tune.keep_layer(key, got, 2)
         ctx.save_for_backward(h2d, z, a, s, mean, rstd)
         return y
 
     @staticmethod
     def backward(ctx, dy):
+        if ctx.whole:
+            h2d, scratch = ctx.saved_tensors
+            dh, ds, *grads = block.ffn_backward(ctx.act, h2d, scratch, dy.contiguous(), *ctx.params, ctx.eps, gemm_tune.LAYERS.get(("backward", ctx.key), (0, 0, 0, 0)))
+            return None, None, None, None, dh, ds, *grads
+        with gemm_tune.collecting() as got:
+            grads = FeedForwardFn._launches(ctx, dy)
+        if ctx.key is not None:
+            gemm_tune.keep_layer(("backward", ctx.key), got, 4)
+        return grads
+
+    @staticmethod
+    def _launches(ctx, dy):
         h2d, z, a, s, mean, rstd = ctx.saved_tensors
         w1, b1, w2, b2, gamma, beta = ctx.params
         ds, dgamma, dbeta, d_b2 = _ln_bwd(dy.contiguous(), s, gamma, beta, mean, rstd, bias=b2, dropout=ctx.drop)
@@ -343,7 +386,7 @@ class FeedForwardFn(torch.autograd.Function):
         d_b1 = _emit_bgrad(b1, dz, after=fork)  # column sums of dz under the weight-gradient GEMM
         dh = _dgrad(dz, w1)
         ops.side_join()
-        return None, None, None, dh, ds, d_w1, d_b1, d_w2, d_b2, dgamma, dbeta
+        return None, None, None, None, dh, ds, d_w1, d_b1, d_w2, d_b2, dgamma, dbeta
 
 
 def _padded_logits(rows: int, V: int, like: torch.Tensor):

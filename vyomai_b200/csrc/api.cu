@@ -183,6 +183,8 @@ int vy_abi_sizeof(const char* name) {
 #define VY_SZ(T) if (strcmp(name, #T) == 0) return static_cast<int>(sizeof(T))
   VY_SZ(VyGemm);
   VY_SZ(VyNorm);
+  VY_SZ(VyAttnBlock);
+  VY_SZ(VyFfnBlock);
   VY_SZ(VyAttn);
   VY_SZ(VyAttnBwd);
   VY_SZ(VyDecode);

@@ -16,7 +16,7 @@ from . import _lib, ops
 HEAD_DIM = 64  # the tcgen05 attention / QKV-RoPE epilogues are specialised for head_dim 64
 
 # decode-shaped GEMMs (few tokens, many output features) run swap-AB
-SWAP_AB_MAX_ROWS = 64
+SWAP_AB_MAX_ROWS = _lib.CONSTS["VY_BLOCK_SWAP_ROWS"]
 
 
 @dataclass

@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import json
 import os
+import threading
 from typing import Dict, List, Optional, Tuple
 
 import torch
@@ -46,6 +47,42 @@ def keep_plan(key: tuple, block: bytes) -> None:
     PLANS[key] = block
 
 
+# the tilings of whole sublayers (block.py): by everything that the hints of their products depend on, the products' hints in the order they are made in, packed
+LAYERS: Dict[tuple, tuple] = {}
+_LISTENING = threading.local()
+
+
+class collecting:
+    """While it is open, the products of this thread leave their hints in the list it gives (None for one that is not settled yet)."""
+
+    def __enter__(self) -> list:
+        self.before = getattr(_LISTENING, "got", None)
+        _LISTENING.got = got = []
+        return got
+
+    def __exit__(self, *exc):
+        _LISTENING.got = self.before
+
+
+def heard(settled_: bool, hint: Dict[str, int]) -> None:
+    got = getattr(_LISTENING, "got", None)
+    if got is not None:
+        got.append((hint.get("hint_flavour", 0) | hint.get("hint_bn", 0) << 4 | hint.get("hint_splits", 0) << 16) if settled_ else None)
+
+
+def listening() -> bool:
+    return getattr(_LISTENING, "got", None) is not None
+
+
+def keep_layer(key: tuple, got: list, products: int) -> None:
+    """What was collected, if it is the sublayer's `products` products and all are settled."""
+    if len(got) != products or any(h is None for h in got):
+        return
+    if len(LAYERS) >= MAX_PLANS:
+        LAYERS.clear()
+    LAYERS[key] = tuple(got)
+
+
 def settled(key: tuple) -> bool:
     """Has `hints` answered for good (not just for now, as while a graph is captured)?"""
     return key in _CACHE
@@ -53,6 +90,7 @@ def settled(key: tuple) -> bool:
 
 def clear() -> None:
     PLANS.clear()
+    LAYERS.clear()
     _CACHE.clear()
     LOG.clear()
 
