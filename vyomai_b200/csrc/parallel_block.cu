@@ -346,6 +346,112 @@ __global__ void __launch_bounds__(256, 4) rope_heads_kernel(RopeHeadsDev d) {
   }
 }
 
+// Prompts with fp32 rows on 16-byte boundaries and dim <= 128: one warp per token, which goes through the heads with the next one's entries on their way, four
+// neighbouring entries per lane, the angles taken once per token. Bound by the bytes (q read and written, k and v copied): 7970 tokens, 8 + 2 heads of 128: no rotation, unit RMS
+// 40.5 us with a warp per head and scattered entries, 17.0 here; half rotated, weighted norm 56.6, 20.8.
+__global__ void __launch_bounds__(256) rope_heads_rows_kernel(RopeHeadsDev d) {
+  pdl_trigger();
+  pdl_wait();
+  const RopeKvDev& b = d.b;
+  const int s = blockIdx.y, base = b.cu[s], n = b.cu[s + 1] - base, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 8 + warp;
+  if (i >= n) return;
+  const int pos = b.pos0[s] + i, half = b.rot_dims / 2, c = 4 * lane, units = b.heads + b.kv_heads;
+  const bool on = c < b.dim;
+  const long long row = base + i;
+  long long prow = 0;
+  if (b.kp) prow = static_cast<long long>(b.table[static_cast<long long>(s) * b.tw + pos / b.bs]) * b.bs + pos % b.bs;
+  const float* q = static_cast<float*>(b.q) + row * b.ldq + c;
+  const float* k = static_cast<const float*>(b.k) + row * b.ldk + c;
+  const auto fetch = [&](int u) {
+    return u < units && on ? *reinterpret_cast<const float4*>(u < b.heads ? q + u * b.dim : k + (u - b.heads) * b.dim) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  float4 next = fetch(0);
+  // cosine and signed sine of this lane's entries: y = x cos + partner sin. Lane l has taken the angles of pairs l and l + 32
+  float cs[4] = {1.f, 1.f, 1.f, 1.f}, sn[4] = {0.f, 0.f, 0.f, 0.f};
+  const int from = d.half_layout && half > 0 ? (c < half ? lane + half / 4 : lane - half / 4) & 31 : lane;   // the lane that holds the partners of a half layout
+  if (half > 0) {
+    float a[2] = {0.f, 0.f}, z[2] = {0.f, 0.f};
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (lane + 32 * r < half) sincosf(static_cast<float>(pos) * b.inv_freq[lane + 32 * r], &z[r], &a[r]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int p = d.half_layout ? (c + e) % half : (c + e) / 2;
+      const float c0 = __shfl_sync(0xffffffffu, a[0], p & 31), c1 = __shfl_sync(0xffffffffu, a[1], p & 31);
+      const float s0 = __shfl_sync(0xffffffffu, z[0], p & 31), s1 = __shfl_sync(0xffffffffu, z[1], p & 31);
+      if (c + e < b.rot_dims) {
+        const bool second = d.half_layout ? c + e >= half : e & 1;
+        cs[e] = (p < 32 ? c0 : c1) * d.rot_scale;
+        sn[e] = (p < 32 ? s0 : s1) * (second ? d.rot_scale : -d.rot_scale);
+      }
+    }
+  }
+  float wq[4], wk[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    wq[e] = d.q_norm && on ? ld_as_float(d.q_norm, d.norm_dt, c + e) : 1.f;
+    wk[e] = d.k_norm && on ? ld_as_float(d.k_norm, d.norm_dt, c + e) : 1.f;
+  }
+  float temp = d.q_scale;
+  if (d.q_temp_every > 0) temp *= fmaf(d.q_temp, logf(static_cast<float>((pos + 1) / d.q_temp_every) + 1.f), 1.f);
+  for (int u = 0; u < units; ++u) {
+    const float4 v = next;
+    next = fetch(u + 1);
+    const bool is_q = u < b.heads;
+    float x[4] = {v.x, v.y, v.z, v.w};
+    if (is_q ? d.q_norm != nullptr : d.k_norm != nullptr) {   // norm with a weight, then the rotation
+      float sr = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sr = fmaf(x[e], x[e], sr);
+      const float inv = 1.f / sqrtf(warp_sum(sr) / static_cast<float>(b.dim) + d.eps);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] *= inv * (is_q ? wq[e] : wk[e]);
+    }
+    if (half > 0) {
+      float p[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[e] = d.half_layout ? __shfl_sync(0xffffffffu, x[e], from) : x[e ^ 1];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (c + e < b.rot_dims) x[e] = x[e] * cs[e] + p[e] * sn[e];
+    }
+    float f = is_q ? temp : d.k_scale;
+    if (d.unit_rms) {
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ss = fmaf(x[e], x[e], ss);
+      f /= sqrtf(warp_sum(ss) / static_cast<float>(b.dim) + d.eps);
+    }
+    if (!on) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[e] *= f;
+    const int h = is_q ? u : u - b.heads;
+    if (!is_q && b.kp && b.pool_dt != VY_F32) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) st_from_float(b.kp, b.pool_dt, (prow * b.kv_heads + h) * b.dim + c + e, x[e]);
+      continue;
+    }
+    float* dst = is_q ? static_cast<float*>(b.q) + row * b.ldq + h * b.dim
+                      : b.kp ? static_cast<float*>(b.kp) + (prow * b.kv_heads + h) * b.dim : static_cast<float*>(d.k_out) + row * d.ld_k_out + h * b.dim;
+    *reinterpret_cast<float4*>(dst + c) = make_float4(x[0], x[1], x[2], x[3]);
+  }
+  if (b.vp) {
+    const float* vo = static_cast<const float*>(b.v) + row * b.ldv;
+    const long long vpo = prow * b.kv_heads * b.vdim;
+    for (int e = c; e < b.kv_heads * b.vdim; e += 128) {
+      const float4 v = *reinterpret_cast<const float4*>(vo + e);
+      if (b.pool_dt == VY_F32) *reinterpret_cast<float4*>(static_cast<float*>(b.vp) + vpo + e) = v;
+      else {
+        st_from_float(b.vp, b.pool_dt, vpo + e, v.x);
+        st_from_float(b.vp, b.pool_dt, vpo + e + 1, v.y);
+        st_from_float(b.vp, b.pool_dt, vpo + e + 2, v.z);
+        st_from_float(b.vp, b.pool_dt, vpo + e + 3, v.w);
+      }
+    }
+  }
+}
+
 }  // namespace vy
 
 #define VY_NEED_DEVICE(name)                                                   \
@@ -485,6 +591,17 @@ extern "C" int vy_rope_kv_write(const VyRopeKvWrite* p) {
     // single tokens: a warp per head in flight (up to 8), few CTAs; prompts: 4 warps per token, more CTAs per SM (measured: 8 warps cost
     // prompts 0.23 -> 0.34 ms over 4 launches of 8192 tokens and saved single-token steps 29 -> 21 us)
     const int units = p->heads + p->kv_heads;
+    const auto quads = [](const void* t, long long ld) { return t == nullptr || (reinterpret_cast<uintptr_t>(t) % 16 == 0 && ld % 4 == 0); };
+    // rows of four: in a half layout the halves are whole lanes. From some hundred tokens on: few tokens' heads go to several warps each above (80 tokens 5.8 / 6.8 us)
+    const bool rows = p->max_new >= 16 && static_cast<long long>(p->n_seqs) * p->max_new >= 512 && (p->max_new + 7) / 8 <= 65535 * 1024 && d.in_dt == VY_F32 && d.dim <= 128 && d.dim % 4 == 0 && (!g.half_layout || d.rot_dims % 8 == 0) &&
+                      (d.heads == 0 || quads(d.q, d.ldq)) && (d.kv_heads == 0 || (quads(d.k, d.ldk) && (paged || quads(g.k_out, g.ld_k_out)))) &&
+                      (!paged || (quads(d.v, d.ldv) && d.vdim % 4 == 0 && (d.pool_dt != VY_F32 || (quads(d.kp, 0) && quads(d.vp, 0)))));
+    if (rows) {
+      VY_CUDA_OK(launch_kernel(rope_heads_rows_kernel, dim3((p->max_new + 7) / 8, p->n_seqs), dim3(256), 0, static_cast<cudaStream_t>(p->stream), g));
+      VY_LAUNCH_OK();
+      count_launch();
+      return VY_OK;
+    }
     const unsigned threads = p->max_new > 1 ? 128u : 32u * static_cast<unsigned>(units < 4 ? 4 : units > 8 ? 8 : units);
     VY_CUDA_OK(launch_kernel(rope_heads_kernel, dim3(gx, p->n_seqs), dim3(threads), 0, static_cast<cudaStream_t>(p->stream), g));
   } else {
