@@ -25,6 +25,24 @@ def _off(t):
     return v
 
 
+@pytest.mark.parametrize("taps", [1, 2, 4])
+@pytest.mark.parametrize("act", ["silu", "sigmoid", None])
+def test_convolution_of_four_channels_per_thread(taps, act):
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(taps)
+    C, pos0 = 8196, [0, 3, 0, 40, 2]   # enough channels for a CTA per SM
+    batch = ops.PackedBatch(torch.tensor([0, 1, 16, 32, 49, 119], dtype=torch.int32, device=DEV), torch.tensor(pos0, dtype=torch.int32, device=DEV),
+                            torch.tensor([4, 1, 0, 5, 2], dtype=torch.int32, device=DEV), 70)
+    x, w, state = torch.randn(119, C, generator=g, device=DEV) * 3, torch.randn(C, taps, generator=g, device=DEV), torch.randn(6, C, max(taps - 1, 1), generator=g, device=DEV)
+    x[5, 7], x[6, 9], x[7, 11], w[11] = 200.0, -200.0, -1e30, w[11].abs()   # the exponentials there overflow or vanish
+    if taps == 1:
+        state = state[:, :, :0].contiguous()
+    states = [state.clone(), state.clone()]
+    a, b = (ops.causal_conv(batch, t, w, s, act=act) for t, s in zip((x, _off(x)), states))
+    _close(a, b)
+    assert torch.equal(*states)
+
+
 @pytest.mark.parametrize("layout,rot,dim", [("half", 64, 128), ("half", 24, 48), ("pairs", 6, 20), ("pairs", 128, 128), ("pairs", 0, 128), ("half", 128, 128)])
 @pytest.mark.parametrize("norm,pool", [("weight", torch.float32), ("unit", torch.float32), (None, torch.bfloat16), ("unit", None)])
 def test_rotation_of_four_entries_per_lane(layout, rot, dim, norm, pool):

@@ -94,6 +94,18 @@ __global__ void __launch_bounds__(256) rms_norm_cached_kernel(NormDev d) {
       ss = fmaf(xv[i], xv[i], ss);
     }
   }
+  // the gate is on its way while the row's sum goes round
+  float4 gv[VEC ? NC / 4 : 1];
+  if constexpr (VEC) {
+    if (d.gate) {
+      const float* gp = reinterpret_cast<const float*>(d.gate) + st * d.ld_gate + static_cast<long long>(grp) * d.width;
+#pragma unroll
+      for (int i = 0; i < NC / 4; ++i) {
+        const int c = 4 * lt + i * 4 * TPR;
+        if (live && c < d.width) gv[i] = *reinterpret_cast<const float4*>(gp + c);
+      }
+    }
+  }
   ss = warp_sum(ss);
   if (TPR > 32) {
     if ((threadIdx.x & 31) == 0) part[lr][lt >> 5] = ss;
@@ -106,7 +118,6 @@ __global__ void __launch_bounds__(256) rms_norm_cached_kernel(NormDev d) {
   const float inv = d.coef / sqrtf(ss / static_cast<float>(d.width) + d.eps);
   const int wo = d.w_full ? grp * d.width : 0;
   if constexpr (VEC) {
-    const long long go = st * d.ld_gate + static_cast<long long>(grp) * d.width;
     const long long oo = static_cast<long long>(tok) * d.ld_out + static_cast<long long>(grp) * d.width;
 #pragma unroll
     for (int i = 0; i < NC / 4; ++i) {
@@ -120,9 +131,8 @@ __global__ void __launch_bounds__(256) rms_norm_cached_kernel(NormDev d) {
         else if (d.w_mode == 2) y[e] *= 1.f + ld_as_float(d.w, d.w_dt, wo + c + e);
       }
       if (d.gate) {
-        const float4 g = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.gate) + go + c);
-        y[0] *= apply_uact(g.x, d.gate_act); y[1] *= apply_uact(g.y, d.gate_act);
-        y[2] *= apply_uact(g.z, d.gate_act); y[3] *= apply_uact(g.w, d.gate_act);
+        y[0] *= uact_near(gv[i].x, d.gate_act); y[1] *= uact_near(gv[i].y, d.gate_act);
+        y[2] *= uact_near(gv[i].z, d.gate_act); y[3] *= uact_near(gv[i].w, d.gate_act);
       }
       if (d.out_dt == VY_F32) {
         float4* op = reinterpret_cast<float4*>(reinterpret_cast<float*>(d.out) + oo + c);
@@ -552,6 +562,52 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(ConvDev d) {
     st_from_float(d.out, d.out_dt, static_cast<long long>(base + i0 + u) * d.ld_out + c, apply_uact(y, d.act));
   }
   if (i0 == 0 && d.taps > 1) conv_new_taps(d, c, base, n, carried, stp);
+}
+
+// The same for four neighbouring channels per thread (fp32 rows on 16-byte boundaries, up to 4 taps): a quarter of the loads, stores and addresses per output,
+// and the SiLU without a division. Bound by the bytes and the exponentials: 7970 tokens x 1024 channels 30.1 us with one channel per thread, 17.0 here; x 512 16.7, 11.1.
+__global__ void __launch_bounds__(128) causal_conv_quads_kernel(ConvDev d) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int TAPS = 4;
+  const int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+  const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
+  const int base = d.cu[s], n = d.cu[s + 1] - base;
+  if (c >= d.channels || i0 >= n) return;
+  const bool carried = d.pos0[s] > 0;
+  float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
+  const float* xp = reinterpret_cast<const float*>(d.x) + static_cast<long long>(base) * d.ldx + c;
+  float4 x[CONV_TOK + TAPS - 1], w[TAPS];
+#pragma unroll
+  for (int u = 0; u < CONV_TOK + TAPS - 1; ++u) {
+    const int j = i0 + u - (TAPS - 1);
+    x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j >= 0) {
+      if (j < n && j > i0 - d.taps) x[u] = *reinterpret_cast<const float4*>(xp + j * d.ldx);
+    } else if (carried && j > -d.taps) {
+      const float* t = stp + d.taps - 1 + j;
+      x[u] = make_float4(t[0], t[d.taps - 1], t[2 * (d.taps - 1)], t[3 * (d.taps - 1)]);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < TAPS; ++t) {   // w[0]: the current token's
+    const auto at = [&](int e) { return t < d.taps ? ld_as_float(d.w, d.w_dt, static_cast<long long>(c + e) * d.taps + d.taps - 1 - t) : 0.f; };
+    w[t] = make_float4(at(0), at(1), at(2), at(3));
+  }
+#pragma unroll
+  for (int u = 0; u < CONV_TOK; ++u) {
+    if (i0 + u >= n) break;
+    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < TAPS; ++t) {
+      const float4 v = x[u + TAPS - 1 - t];
+      y = make_float4(fmaf(w[t].x, v.x, y.x), fmaf(w[t].y, v.y, y.y), fmaf(w[t].z, v.z, y.z), fmaf(w[t].w, v.w, y.w));
+    }
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(d.out) + static_cast<long long>(base + i0 + u) * d.ld_out + c) =
+        make_float4(uact_near(y.x, d.act), uact_near(y.y, d.act), uact_near(y.z, d.act), uact_near(y.w, d.act));
+  }
+  if (i0 == 0 && d.taps > 1)
+    for (int e = 0; e < 4; ++e) conv_new_taps(d, c + e, base, n, carried, stp + e * (d.taps - 1));
 }
 
 // ---- recurrences: one thread owns one column of the dim x vdim state in registers ---------------------------------------
@@ -1011,6 +1067,17 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   d.state = p->state; d.act = p->act;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
+  const auto quads = [](const void* q, int dt, long long ld) { return dt == VY_F32 && reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0; };
+  // from a CTA per SM on: 80 tokens x 512 channels are 7.2 us with a channel per thread, 8.2 with four
+  if (static_cast<long long>(p->n_seqs) * ((p->max_new + CONV_TOK - 1) / CONV_TOK) * ((p->channels + 511) / 512) >= num_sms() && p->taps <= 4 && p->channels % 4 == 0 &&
+      p->channels <= 65535 * 512 && quads(d.x, d.x_dt, d.ldx) && quads(d.out, d.out_dt, d.ld_out)) {
+    d.first = 0;
+    const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, (p->channels + 511) / 512, p->n_seqs);
+    VY_CUDA_OK(launch_kernel(causal_conv_quads_kernel, grid, dim3(128), 0, st, d));
+    VY_LAUNCH_OK();
+    count_launch();
+    return VY_OK;
+  }
   const long long blocks = (p->channels + 127LL) / 128;
   for (long long b = 0; b < blocks; b += 65535) {   // one launch, up to 8 million channels
     d.first = static_cast<int>(128 * b);

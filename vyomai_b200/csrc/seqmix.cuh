@@ -20,6 +20,16 @@ __device__ __forceinline__ float apply_uact(float x, int act) {
     default: return x;
   }
 }
+// 1 / y for y >= 1, an ulp at most off: the approximate reciprocal and a Newton step (1 / infinity = 0; a NaN stays one). A division with its rounding and its
+// range checks is three times as many instructions
+__device__ __forceinline__ float recip_near(float y) {
+  const float r = vy_rcp_approx(y), n = fmaf(r, fmaf(-y, r, 1.f), r);
+  return y < INFINITY ? n : r;
+}
+__device__ __forceinline__ float sigmoid_near(float x) { return recip_near(1.f + expf(-x)); }
+__device__ __forceinline__ float uact_near(float x, int act) {
+  return act == VY_UACT_SILU ? x * sigmoid_near(x) : act == VY_UACT_SIGMOID ? sigmoid_near(x) : apply_uact(x, act);
+}
 constexpr float MIN_LOG_DECAY = -1e4f;   // exp of it is 0 in fp32; keeps sums and differences of log decays finite
 // cap * tanh(s / cap) as cap * (1 - 2 / (1 + e^(2 s / cap))): expf and a fast reciprocal, absolute error a few 1e-7 * cap (the softmax
 // that follows depends on score differences, i.e. on absolute error); e^x overflowing to inf gives exactly cap, underflow exactly -cap
