@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(ConvDev d) {
 }
 
 // The same for four neighbouring channels per thread (fp32 rows on 16-byte boundaries, up to 4 taps): a quarter of the loads, stores and addresses per output,
-// and the SiLU without a division. Bound by the bytes and the exponentials: 7970 tokens x 1024 channels 30.1 us with one channel per thread, 17.0 here; x 512 16.7, 11.1.
+// and the SiLU without a division. Bound by the bytes and the exponentials: 7970 tokens x 1024 channels 30.1 us with one channel per thread, 18.1 here; x 512 16.7, 11.6.
 __global__ void __launch_bounds__(128) causal_conv_quads_kernel(ConvDev d) {
   pdl_trigger();
   pdl_wait();

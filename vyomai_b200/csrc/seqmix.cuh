@@ -20,15 +20,20 @@ __device__ __forceinline__ float apply_uact(float x, int act) {
     default: return x;
   }
 }
-// 1 / y for y >= 1, an ulp at most off: the approximate reciprocal and a Newton step (1 / infinity = 0; a NaN stays one). A division with its rounding and its
-// range checks is three times as many instructions
+// 1 / y for y >= 1 in two Newton steps from the approximate reciprocal (1 / infinity = 0; a NaN stays one), and x / (1 + e^-x) with its quotient corrected once: rounded as a
+// division but for a hair, which with its range checks is twice as many instructions
 __device__ __forceinline__ float recip_near(float y) {
-  const float r = vy_rcp_approx(y), n = fmaf(r, fmaf(-y, r, 1.f), r);
+  float r = vy_rcp_approx(y), n = fmaf(r, fmaf(-y, r, 1.f), r);
+  n = fmaf(n, fmaf(-y, n, 1.f), n);
   return y < INFINITY ? n : r;
 }
 __device__ __forceinline__ float sigmoid_near(float x) { return recip_near(1.f + expf(-x)); }
+__device__ __forceinline__ float silu_near(float x) {
+  const float y = 1.f + expf(-x), r0 = vy_rcp_approx(y), r = fmaf(r0, fmaf(-y, r0, 1.f), r0), q = x * r, a = fmaf(fmaf(-y, q, x), r, q);
+  return a == a ? a : x * r0;   // infinities
+}
 __device__ __forceinline__ float uact_near(float x, int act) {
-  return act == VY_UACT_SILU ? x * sigmoid_near(x) : act == VY_UACT_SIGMOID ? sigmoid_near(x) : apply_uact(x, act);
+  return act == VY_UACT_SILU ? silu_near(x) : act == VY_UACT_SIGMOID ? sigmoid_near(x) : apply_uact(x, act);
 }
 constexpr float MIN_LOG_DECAY = -1e4f;   // exp of it is 0 in fp32; keeps sums and differences of log decays finite
 // cap * tanh(s / cap) as cap * (1 - 2 / (1 + e^(2 s / cap))): expf and a fast reciprocal, absolute error a few 1e-7 * cap (the softmax

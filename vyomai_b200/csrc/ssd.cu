@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(SC_T) ssd_conv_kernel(SsdDev d, int run) {
         float a = bias[e];
 #pragma unroll
         for (int lag = 0; lag < TP; ++lag) a = fmaf(w[lag][e], xs[t + TP - 1 - lag][e], a);
-        y[e] = a * sigmoid_near(a);
+        y[e] = silu_near(a);
       }
       if (i + t < i1) st_run<V>(d.xc + static_cast<long long>(base + i + t) * d.ld_xc + ch, y);
     }
