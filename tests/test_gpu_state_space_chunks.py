@@ -1,0 +1,72 @@
+"""-m gpu: state-space prompts in chunks of 128 tokens (csrc/linear_attn_tc.cu) against the form in chunks of 64 that the same call takes where the gate is one element
+off a 16-byte boundary. Either is within about 2^-22 of the result's 2-norm of 64-bit arithmetic: 8 * 2^-24 between them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BOUND = 8 * 2.0 ** -24
+
+
+def _i32(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+def _inputs(lengths, H, G, dim, vdim, seed, dt_scale=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    T, n, inner = sum(lengths), len(lengths), H * vdim
+    C = inner + 2 * G * dim
+    x = dict(x=R(T, inner), b=R(T, G * dim), c=R(T, G * dim), dt=R(T, H) * dt_scale, gate=R(T, inner))
+    w = dict(conv_w=R(C, 3) * 0.5, conv_b=R(C), dt_bias=R(H) - 1, a_log=R(H) * 0.3, skip=R(H), norm=torch.ones(inner, device=DEV), heads=H, groups=G, dim=dim, vdim=vdim, taps=3,
+             norm_groups=H, norm_eps=1e-6, out_dtype=torch.float32)
+    return x, w, R(n, 3, C), R(n, H, dim, vdim)
+
+
+def _run(lengths, pos0, x, w, conv, state, off):
+    from vyomai_b200 import ops
+    cu = [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    x = dict(x)
+    if off:
+        buf = torch.zeros(cu[-1], x["gate"].shape[1] + 4, device=DEV)
+        buf[:, 1:-3] = x["gate"]
+        x["gate"] = buf[:, 1:-3]
+    conv, state = conv.clone(), state.clone()
+    out = ops.ssd(ops.PackedBatch(_i32(cu), _i32(pos0), _i32(list(range(len(lengths)))), max(lengths)), **x, **w, conv_state=conv, state=state,
+                  tickets=torch.zeros(len(lengths), 1, dtype=torch.int32, device=DEV))
+    return out, state
+
+
+def _close(a, b):
+    assert a.shape == b.shape and float((a.double() - b.double()).norm()) <= BOUND * float(b.double().norm())
+
+
+@pytest.mark.parametrize("H,G,dim,vdim", [(8, 1, 128, 64), (6, 2, 96, 40), (5, 5, 16, 64), (24, 2, 64, 132), (4, 1, 128, 32), (22, 2, 20, 68)])
+@pytest.mark.parametrize("lengths,pos0", [([129], [0]), ([1, 127, 128, 129, 300], [7, 0, 3, 0, 1]), ([256, 5, 640], [0, 2, 9])])
+def test_chunks_of_128_tokens(H, G, dim, vdim, lengths, pos0):
+    args = _inputs(lengths, H, G, dim, vdim, H + dim)
+    a, b = (_run(lengths, pos0, *args, off) for off in (False, True))
+    _close(a[0], b[0])
+    _close(a[1], b[1])
+
+
+@pytest.mark.parametrize("what", ["steep decays", "flat decays", "wide rows", "infinite value", "infinite gates"])
+def test_chunks_of_128_tokens_at_the_ends_of_their_range(what):
+    """Decays that vanish within a chunk or never start; rows too far apart for fp16 halves and infinities, which leave their heads to the walk in either form."""
+    lengths, pos0 = [400, 260], [0, 4]
+    x, w, conv, state = _inputs(lengths, 8, 2, 64, 64, 3, dt_scale=30.0 if what == "steep decays" else 1.0)
+    if what == "flat decays":
+        w["dt_bias"] = torch.full_like(w["dt_bias"], -40.0)
+    if what == "wide rows":
+        x["x"][130:140] *= 1e9
+        x["c"][50] *= 1e-12
+    if what == "infinite value":
+        x["x"][300, 70] = float("inf")
+    if what == "infinite gates":
+        x["gate"][5, 3], x["gate"][200, 65], x["gate"][7, 9], x["gate"][8, 9], x["gate"][9, 9] = float("inf"), float("-inf"), float("nan"), 200.0, -200.0
+    a, b = (_run(lengths, pos0, x, w, conv, state, off) for off in (False, True))
+    for p, q in zip(a, b):
+        assert torch.equal(p.isfinite(), q.isfinite())
+        _close(p.nan_to_num(0, 0, 0), q.nan_to_num(0, 0, 0))

@@ -14,53 +14,11 @@
 // columns (channels) of every chunk's q, k and v, as each warp has them, and of the state that is carried in: where the largest entry of one is below 2^-20 of the
 // largest of all (rows and columns of few entries, which may all be small by chance: 2^-24; zeros aside), and where an infinity or NaN is among them, the
 // heads of the CTA are left to the walk, which runs behind the three launches and starts from the state that la_scan kept as the one before the first chunk.
+#include "linear_attn.cuh"
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 
 namespace vy {
-
-constexpr int LM_C = 64;   // tokens per chunk
-
-// The chunks' states in the workspace: chunk c of sequence s is slot cu[s] / 64 + s + c (never more than rows / 64 + n_seqs in all)
-struct LaChunks {
-  float* U;          // [slots][heads][dim][vdim]
-  float* D;          // [slots][heads]
-  unsigned* top;     // [slots][heads] largest |S| before the chunk, as bits
-  int* odd;          // [slots][heads / hp][vslices] 1: not for fp16 halves
-};
-__device__ __forceinline__ long long la_slot(const RecDev& d, int s, int c) { return d.cu[s] / LM_C + s + c; }
-
-// One warp: tokens 2 lane, 2 lane + 1 of a chunk of nt: log decays summed (two floats each: their differences are what counts) and write
-// strengths, as in linear_attn_chunk_kernel
-struct TokenDecay { float Lh[2], Ll[2], w[2], eL[2], es[2], whole; };
-__device__ __forceinline__ TokenDecay token_decays(const RecDev& d, long long r0, int nt, int h, int lane) {
-  const float rate = expf(ld_as_float(d.a_log, d.a_log_dt, h)), dt_b = ld_as_float(d.dt_bias, d.a_log_dt, h);
-  TokenDecay o;
-  double la[2];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const int tt = 2 * lane + e;
-    o.w[e] = tt < nt ? softplusf_(d.dt[(r0 + tt) * d.ld_dt + h] + dt_b) : 0.f;
-    la[e] = fmaxf(-rate * o.w[e], MIN_LOG_DECAY);
-  }
-  double run = la[0] + la[1];
-#pragma unroll
-  for (int k = 1; k < 32; k <<= 1) {
-    const double x = __shfl_up_sync(0xffffffffu, run, k);
-    if (lane >= k) run += x;
-  }
-  const double end = __shfl_sync(0xffffffffu, run, 31);
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const double L = e ? run : run - la[1];
-    o.Lh[e] = static_cast<float>(L);
-    o.Ll[e] = static_cast<float>(L - static_cast<double>(o.Lh[e]));
-    o.eL[e] = expf(static_cast<float>(L));
-    o.es[e] = expf(static_cast<float>(end - L)) * o.w[e];
-  }
-  o.whole = expf(static_cast<float>(end));
-  return o;
-}
 
 // a^n, n < 128, in seven steps of repeated squaring (double: rounded once, to the fp32 result)
 __device__ __forceinline__ float power(float a, int n) {
@@ -91,64 +49,6 @@ template <int ACT>
 __device__ __forceinline__ float4 act4(float4 x, int act) {
   return make_float4(act_of<ACT>(x.x, act), act_of<ACT>(x.y, act), act_of<ACT>(x.z, act), act_of<ACT>(x.w, act));
 }
-__device__ __forceinline__ void store_split4(unsigned char* hi, unsigned char* lo, int at, float4 x, float4 sc) {
-  uint2 h, l;
-  split2(x.x * sc.x, x.y * sc.y, h.x, l.x);
-  split2(x.z * sc.z, x.w * sc.w, h.y, l.y);
-  *reinterpret_cast<uint2*>(hi + at) = h;
-  *reinterpret_cast<uint2*>(lo + at) = l;
-}
-// Largest and smallest (but not zero) of rows' and columns' largest entries, as bits: positive numbers order like them, NaN after infinity
-constexpr unsigned RANGE_NONE = 0x7f800000u;   // infinity: no entry yet
-struct Range { unsigned top, low; };
-__device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
-__device__ __forceinline__ void note(Range& r, unsigned m, bool few = false) {
-  r.top = max(r.top, m);
-  if (m) r.low = min(r.low, few ? __float_as_uint(16.f * __uint_as_float(m)) : m);
-}
-__device__ __forceinline__ void note_warp(Range* to, Range r) {   // to: shared memory, read after a barrier
-  r.top = __reduce_max_sync(0xffffffffu, r.top);
-  r.low = __reduce_min_sync(0xffffffffu, r.low);
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(&to->top, r.top);
-    atomicMin(&to->low, r.low);
-  }
-}
-__device__ __forceinline__ bool too_wide(Range r) { return r.top >= 0x7f800000u || __uint_as_float(r.low) < 0x1p-20f * __uint_as_float(r.top); }
-
-// A warp's tile, a thread's N quads of it: FROM lanes share a row, 4 FROM columns. Notes the largest entry of each row and of each column (few_rows, few_columns: all
-// may be small by chance) and returns the columns'
-template <int N, int FROM>
-__device__ __forceinline__ uint4 look(const float4 (&x)[N], bool few_rows, bool few_columns, Range& r) {
-  uint4 m = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const uint4 a = make_uint4(abs_bits(x[i].x), abs_bits(x[i].y), abs_bits(x[i].z), abs_bits(x[i].w));
-    m = make_uint4(max(m.x, a.x), max(m.y, a.y), max(m.z, a.z), max(m.w, a.w));
-    unsigned most = max(max(a.x, a.y), max(a.z, a.w));
-#pragma unroll
-    for (int k = 1; k < FROM; k <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, k));
-    note(r, most, few_columns);
-  }
-#pragma unroll
-  for (int k = FROM; k < 32; k <<= 1)
-    m = make_uint4(max(m.x, __shfl_xor_sync(0xffffffffu, m.x, k)), max(m.y, __shfl_xor_sync(0xffffffffu, m.y, k)), max(m.z, __shfl_xor_sync(0xffffffffu, m.z, k)),
-                   max(m.w, __shfl_xor_sync(0xffffffffu, m.w, k)));
-  note(r, m.x, few_rows);
-  note(r, m.y, few_rows);
-  note(r, m.z, few_rows);
-  note(r, m.w, few_rows);
-  return m;
-}
-__device__ __forceinline__ float4 column_units(uint4 m) {   // 2^(exponent - SPLIT_TOP) of each column
-  const auto u = [](unsigned b) { return pow2i(split_exponent(__uint_as_float(b)) - SPLIT_TOP); };
-  return make_float4(u(m.x), u(m.y), u(m.z), u(m.w));
-}
-__device__ __forceinline__ float4 column_scales(uint4 m) {
-  const auto u = [](unsigned b) { return split_scale(split_exponent(__uint_as_float(b))); };
-  return make_float4(u(m.x), u(m.y), u(m.z), u(m.w));
-}
-
 constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows of 64 value columns
 
 // CTA: (chunk, 64 value columns) x (hp heads that share k) x sequence. Warp w owns state rows 16 w .., and it reads and splits those channels of k (eight
@@ -158,22 +58,23 @@ constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows 
 // ACT: see act_of
 template <bool TD, int ACT>
 __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
+  constexpr int C = LM_C;
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) unsigned char lu_smem[];
   const int kb = dim16 * 2 + 16;
   unsigned char* Kh = lu_smem;
-  unsigned char* Kl = Kh + LM_C * kb;
-  unsigned char* Wh = Kl + LM_C * kb;
-  unsigned char* Wl = Wh + LM_C * LU_VB;
-  float* es = reinterpret_cast<float*>(Wl + LM_C * LU_VB);   // [64] decay to the chunk's end times write strength
-  float* ku = es + LM_C;                                     // [128], [64]: units of k's channels and of w's columns
+  unsigned char* Kl = Kh + C * kb;
+  unsigned char* Wh = Kl + C * kb;
+  unsigned char* Wl = Wh + C * LU_VB;
+  float* es = reinterpret_cast<float*>(Wl + C * LU_VB);   // [64] decay to the chunk's end times write strength
+  float* ku = es + C;                                     // [128], [64]: units of k's channels and of w's columns
   float* wu = ku + 128;
   Range* range = reinterpret_cast<Range*>(wu + 64);          // [4]: k, q, v, state
   const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
-  const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LM_C;
+  const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * C;
   if (t0 >= n) return;
-  const int nt = min(LM_C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
+  const int nt = min(C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
   const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
   const long long r0 = base + t0, slot = la_slot(d, s, c);
   if (t < 4) range[t] = {0u, RANGE_NONE};
@@ -181,10 +82,10 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
   const bool few = nt < 8;
   {
     const int row = lane >> 2, ch = 16 * warp + 4 * (lane & 3);
-    float4 x[8];
+    float4 x[C / 8];
     const auto read = [&](const void* p, long long ld) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < C / 8; ++i) {
         const int r = row + 8 * i;
         x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < nt && ch < d.dim) x[i] = act4<ACT>(load4(p, d.in_dt, vec, (r0 + r) * ld + static_cast<long long>(hq) * d.dim, ch, d.dim), d.in_act);
@@ -193,26 +94,26 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
     Range rk = {0u, RANGE_NONE}, rq = rk;
     if (v0 == 0) {
       read(d.q, d.ldq);
-      look<8, 4>(x, few, d.dim - 16 * warp < 4, rq);
+      look<C / 8, 4>(x, few, d.dim - 16 * warp < 4, rq);
       note_warp(range + 1, rq);
     }
     read(d.k, d.ldk);
-    const uint4 m = look<8, 4>(x, few, d.dim - 16 * warp < 4, rk);
+    const uint4 m = look<C / 8, 4>(x, few, d.dim - 16 * warp < 4, rk);
     note_warp(range, rk);
     const float4 sc = column_scales(m);
     if (row == 0) *reinterpret_cast<float4*>(ku + ch) = column_units(m);
     if (ch < dim16) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) store_split4(Kh, Kl, (row + 8 * i) * kb + ch * 2, x[i], sc);
+      for (int i = 0; i < C / 8; ++i) store_split4(Kh, Kl, (row + 8 * i) * kb + ch * 2, x[i], sc);
     }
   }
   const unsigned ka = smem_addr(Kh) + lane_b(lane, kb) + 16 * warp * 2, wb = smem_addr(Wh) + lane_bt(lane, LU_VB);
   const int row = lane >> 1, vc = 8 * warp + 4 * (lane & 1);
   Range rv = {0u, RANGE_NONE}, rs = rv;   // this thread's share
-  float4 next[4];
+  float4 next[C / 16];
   const auto fetch = [&](int h) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < C / 16; ++i) {
       const int r = row + 16 * i;
       next[i] = r < nt ? load4(d.v, d.in_dt, vec, (r0 + r) * d.ldv + static_cast<long long>(h) * d.vdim + v0, vc, vw) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -222,38 +123,41 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
     __syncthreads();   // the previous head's readers of es and W are done
     if constexpr (TD) {
       if (warp == 0) {
-        const TokenDecay q = token_decays(d, r0, nt, h, lane);
-        es[2 * lane] = q.es[0];
-        es[2 * lane + 1] = q.es[1];
-        if (lane == 0 && v0 == 0) w.D[slot * d.heads + h] = q.whole;
+        const float whole = token_decays<C / 32>(d, r0, nt, h, lane, [&](int i, double L, float strength, double end) { es[i] = expf(static_cast<float>(end - L)) * strength; });
+        if (lane == 0 && v0 == 0) w.D[slot * d.heads + h] = whole;
       }
-    } else if (t <= LM_C) {
-      if (t < LM_C) es[t] = t < nt ? power(d.decay[h], nt - 1 - t) : 0.f;
+    } else if (t <= C) {
+      if (t < C) es[t] = t < nt ? power(d.decay[h], nt - 1 - t) : 0.f;
       else if (v0 == 0) w.D[slot * d.heads + h] = power(d.decay[h], nt);
     }
     if (t == 0 && v0 == 0) w.top[slot * d.heads + h] = 0u;
-    float4 y[4] = {next[0], next[1], next[2], next[3]};
+    float4 y[C / 16];
+#pragma unroll
+    for (int i = 0; i < C / 16; ++i) y[i] = next[i];
     if (h + 1 < h0 + hp) fetch(h + 1);   // in flight during this head's products
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < C / 16; ++i) {
       if (row + 16 * i < nt) y[i] = act4<ACT>(y[i], d.in_act);
     }
-    uint4 m = look<4, 2>(y, few, vw - 8 * warp < 4, rv);
+    uint4 m = look<C / 16, 2>(y, few, vw - 8 * warp < 4, rv);
     {   // the weighted columns' units from a bound, the columns' largest times the largest weight: rows are within 2^20 of one another, and the halves good to 2^24
-      const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, max(abs_bits(es[lane]), abs_bits(es[lane + 32]))));
+      unsigned top = 0u;
+#pragma unroll
+      for (int i = lane; i < C; i += 32) top = max(top, abs_bits(es[i]));
+      const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, top));
       const auto times = [most](unsigned b) { return __float_as_uint(__uint_as_float(b) * most); };
       m = make_uint4(times(m.x), times(m.y), times(m.z), times(m.w));
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < C / 16; ++i) {
       const float e = es[row + 16 * i];
       y[i] = make_float4(y[i].x * e, y[i].y * e, y[i].z * e, y[i].w * e);
     }
     const float4 sv = column_scales(m);
     if (row == 0) *reinterpret_cast<float4*>(wu + vc) = column_units(m);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) store_split4(Wh, Wl, (row + 16 * i) * LU_VB + vc * 2, y[i], sv);
+    for (int i = 0; i < C / 16; ++i) store_split4(Wh, Wl, (row + 16 * i) * LU_VB + vc * 2, y[i], sv);
     if (c == 0 && d.pos0[s] > 0) {   // the state that is carried in: a thread reads every fourth entry of a column
       const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 + (t & 63);
       unsigned top = 0u;
@@ -273,15 +177,15 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
 #pragma unroll
         for (int k = 0; k < 4; ++k) a[i][k] = b[i][k] = 0.f;
 #pragma unroll
-      for (int k = 0; k < LM_C / 16; ++k) {
+      for (int k = 0; k < C / 16; ++k) {
         unsigned ah[4], al[4];   // k^T: stored [token][channel], read transposed (lane_b's order is what .trans turns into an A operand)
         ldsm_x4_t(ah, ka + 16 * k * kb);
-        ldsm_x4_t(al, ka + LM_C * kb + 16 * k * kb);
+        ldsm_x4_t(al, ka + C * kb + 16 * k * kb);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           unsigned bh[4], bl[4];
           ldsm_x4_t(bh, wb + 16 * k * LU_VB + 32 * j);
-          ldsm_x4_t(bl, wb + LM_C * LU_VB + 16 * k * LU_VB + 32 * j);
+          ldsm_x4_t(bl, wb + C * LU_VB + 16 * k * LU_VB + 32 * j);
           mma_f16(b[2 * j], al, bh[0], bh[1]);
           mma_f16(b[2 * j + 1], al, bh[2], bh[3]);
           mma_f16(a[2 * j], ah, bh[0], bh[1]);
@@ -296,7 +200,7 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
         const int i = 16 * warp + gq + 8 * r;
         if (i >= d.dim) continue;
         const float u1 = ku[i];
-        constexpr float cut = (LM_C / 16 + 1) * 0.5f * SPLIT_CUT;
+        constexpr float cut = (C / 16 + 1) * 0.5f * SPLIT_CUT;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int col = 8 * j + 2 * tq;
@@ -326,7 +230,7 @@ __global__ void __launch_bounds__(256) la_scan_kernel(RecDev d, LaChunks w) {
   constexpr int P = 8;
   const int s = blockIdx.z, h = blockIdx.y, n = d.cu[s + 1] - d.cu[s];
   if (n <= 0) return;
-  const int e = (blockIdx.x * 256 + threadIdx.x) * V, each = d.dim * d.vdim, chunks = (n + LM_C - 1) / LM_C;
+  const int e = (blockIdx.x * 256 + threadIdx.x) * V, each = d.dim * d.vdim, chunks = (n + w.chunk - 1) / w.chunk;
   const bool on = e < each;
   const long long first = la_slot(d, s, 0) * d.heads + h;
   float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * each + e;
@@ -446,14 +350,12 @@ __global__ void __launch_bounds__(LO_T, 2) la_outputs_kernel(RecDev d, LaChunks 
     if constexpr (TD) {
       skip = ld_as_float(d.skip, d.a_log_dt, h);
       if (warp == 0) {
-        const TokenDecay q = token_decays(d, r0, nt, h, lane);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          Lh[2 * lane + e] = q.Lh[e];
-          Ll[2 * lane + e] = q.Ll[e];
-          wr[2 * lane + e] = q.w[e];
-          eL[2 * lane + e] = q.eL[e];
-        }
+        token_decays<LM_C / 32>(d, r0, nt, h, lane, [&](int i, double L, float strength, double) {   // two floats: the sums' differences are what counts
+          Lh[i] = static_cast<float>(L);
+          Ll[i] = static_cast<float>(L - static_cast<double>(Lh[i]));
+          wr[i] = strength;
+          eL[i] = expf(Lh[i]);
+        });
       }
     } else if (t <= LM_C) {   // decay^t: wr, shifted by one: eL
       const float x = power(d.decay[h], t);
@@ -645,32 +547,43 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   w.D = ws + slots * d.heads * static_cast<long long>(d.dim) * d.vdim;
   w.top = reinterpret_cast<unsigned*>(w.D + slots * d.heads);
   w.odd = reinterpret_cast<int*>(w.top + slots * d.heads);
-  const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, vslices = (d.vdim + 63) / 64, chunks = (max_new + LM_C - 1) / LM_C;
+  const bool quad = d.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(d.state) % 16 == 0 && reinterpret_cast<uintptr_t>(ws) % 16 == 0;
+  const bool tc = TD && vec && quad && linear_attn_tc_applies(d);
+  const int C = w.chunk = tc ? LT_C : LM_C;
+  const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, vslices = (d.vdim + 63) / 64, chunks = (max_new + C - 1) / C;
   // heads per CTA: those that share q and k, fewer while that leaves less than two CTAs per SM
   int hp = TD ? d.heads / d.kv_heads : 1;
-  while (hp % 2 == 0 && slots * vslices * (d.heads / hp) < 2LL * num_sms()) hp /= 2;
+  if (tc) hp = linear_attn_tc_heads(d, n_seqs, max_new, rows, vslices);
+  else
+    while (hp % 2 == 0 && slots * vslices * (d.heads / hp) < 2LL * num_sms()) hp /= 2;
   const dim3 grid(static_cast<unsigned>(chunks) * vslices, d.heads / hp, n_seqs);
   const size_t smem_u = 2 * LM_C * static_cast<size_t>(kb) + 2 * LM_C * LU_VB + sizeof(float) * (LM_C + 128 + 64) + 4 * sizeof(Range);
   const size_t q2 = 2 * LM_C * static_cast<size_t>(kb), vs = 2 * LM_C * LU_VB + 2 * static_cast<size_t>(dim16) * LU_VB;
   const size_t smem_o = q2 + (q2 > vs ? q2 : vs) + sizeof(float) * 7 * LM_C;
   static std::atomic<unsigned long long> allowed_u{0}, allowed_o{0};
-  cudaError_t e = allow_smem(la_states_kernel<TD, ACT>, allowed_u);
-  if (e == cudaSuccess) e = allow_smem(la_outputs_kernel<TD, ACT>, allowed_o);
-  if (e != cudaSuccess) return e;
-  e = launch_kernel(la_states_kernel<TD, ACT>, grid, dim3(LU_T), smem_u, st, d, w, hp, vslices, dim16, vec);
+  cudaError_t e;
+  if (tc) e = launch_la_states_tc(d, w, hp, n_seqs, max_new, rows, st);
+  else {
+    e = allow_smem(la_states_kernel<TD, ACT>, allowed_u);
+    if (e == cudaSuccess) e = launch_kernel(la_states_kernel<TD, ACT>, grid, dim3(LU_T), smem_u, st, d, w, hp, vslices, dim16, vec);
+  }
   if (e != cudaSuccess) return e;
   const int each = d.dim * d.vdim;
-  const bool quad = d.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(d.state) % 16 == 0 && reinterpret_cast<uintptr_t>(ws) % 16 == 0;
   const int per = 256 * (quad ? 4 : 1);
   const dim3 sgrid((each + per - 1) / per, d.heads, n_seqs);
   e = quad ? launch_kernel(la_scan_kernel<4>, sgrid, dim3(256), 0, st, d, w) : launch_kernel(la_scan_kernel<1>, sgrid, dim3(256), 0, st, d, w);
   if (e != cudaSuccess) return e;
-  e = launch_kernel(la_outputs_kernel<TD, ACT>, grid, dim3(LO_T), smem_o, st, d, w, hp, vslices, dim16, vec, svec && quad);
+  if (tc) e = launch_la_outputs_tc(d, w, hp, n_seqs, max_new, rows, st);
+  else {
+    e = allow_smem(la_outputs_kernel<TD, ACT>, allowed_o);
+    if (e == cudaSuccess) e = launch_kernel(la_outputs_kernel<TD, ACT>, grid, dim3(LO_T), smem_o, st, d, w, hp, vslices, dim16, vec, svec && quad);
+  }
   if (e != cudaSuccess) return e;
   RecDev r = d;   // the walk, for what is left to it
   r.odd = w.odd;
   r.odd_heads = hp;
   r.odd_each = vslices;
+  r.odd_chunk = C;
   r.first = w.U;
   return TD ? launch_ssd_chunked(r, n_seqs, st) : launch_linear_attn_chunked(r, n_seqs, st);
 }

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(128) kv_page_write_kernel(KvwDev d) {
 
 constexpr int WA_WARPS = 4;
 constexpr int WA_VR = 8;  // value columns per lane: vdim <= 256
-constexpr int WA_TILED_MIN = 16;   // longest portion of a step from which the prompt kernel (window_attn_mma.cu) takes over
+constexpr int WA_TILED_MIN = 16;   // longest portion of a step from which the prompt kernels (window_attn_tc.cu, window_attn_mma.cu) take over
 constexpr int LA_CHUNKED_MIN = 8;  // same for the chunked linear attention
 
 __device__ __forceinline__ float dot_row(const void* base, int dt, long long off, int n, const float* __restrict__ qs) {

@@ -1,5 +1,5 @@
 // Shared by the sequence-mixer kernels (seqmix.cu: token-serial forms used for single tokens and short portions;
-// seqmix_tiled.cu, window_attn_mma.cu, linear_attn_mma.cu, delta_rule_mma.cu: forms used for prompts): activation helpers, the kernels' argument blocks and the tiled launchers.
+// seqmix_tiled.cu, window_attn_tc.cu, window_attn_mma.cu, linear_attn_tc.cu, linear_attn_mma.cu, delta_rule_mma.cu: forms used for prompts): activation helpers, the kernels' argument blocks and the tiled launchers.
 #pragma once
 #include <math.h>
 
@@ -175,9 +175,9 @@ struct RecDev {
   float q_scale;  // gated linear attention (the delta kernel without its correction term): multiplies q as it is read
   float* state;
   void* out; long long ld_out; int out_dt;
-  // chunked walk behind linear_attn_mma.cu: null, or [cu / 64 + sequence + chunk][heads / odd_heads][odd_each] with a 1 where the sequence and head are left to
-  // it, and their state before each chunk, [cu / 64 + sequence + chunk][heads][dim][vdim]
-  const int* odd; int odd_heads, odd_each; const float* first;
+  // chunked walk behind linear_attn_mma.cu and linear_attn_tc.cu: null, or [cu / 64 + sequence + chunk][heads / odd_heads][odd_each] with a 1 where the sequence and head are left to
+  // it, and their state before each chunk, [cu / 64 + sequence + chunk][heads][dim][vdim]; odd_chunk: tokens per chunk
+  const int* odd; int odd_heads, odd_each, odd_chunk; const float* first;
 };
 
 // Prompt-sized steps: defined in the files named above.
@@ -186,7 +186,7 @@ cudaError_t launch_ssd_chunked(const RecDev& d, int n_seqs, cudaStream_t st);
 // 16 tokens per step of the walk (delta_rule_mma.cu), given delta_rule_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); two launches
 long long delta_rule_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 cudaError_t launch_delta_rule_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);
-// All chunks at once (linear_attn_mma.cu), given linear_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); four launches
+// All chunks at once (linear_attn_mma.cu, linear_attn_tc.cu), given linear_attn_mma_floats(..) floats of 16-byte aligned scratch (0: not for this step); four launches
 long long linear_attn_mma_floats(long long rows, int n_seqs, int max_new, int heads, int dim, int vdim);
 template <bool TD>
 cudaError_t launch_linear_attn_mma(const RecDev& d, int n_seqs, int max_new, long long rows, float* ws, cudaStream_t st);

@@ -1,4 +1,4 @@
-// Prompt-sized forms of two sequence mixers, in fp32 on register tiles: for what the tensor-core forms (linear_attn_mma.cu, window_attn_mma.cu) do not take.
+// Prompt-sized forms of two sequence mixers, in fp32 on register tiles: for what the tensor-core forms (linear_attn_tc.cu, linear_attn_mma.cu, window_attn_tc.cu, window_attn_mma.cu) do not take.
 //
 //   * linear attention with a fixed decay, chunk by chunk (portions of up to 64 tokens, heads of more than 128 channels, calls without a workspace): for a chunk of C tokens with the state S0 before it,
 //       O = (Q K^T . D) V + diag(decay^(i+1)) Q S0,   D[i][j] = decay^(i-j) for j <= i, else 0
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(LA_T, OCC) linear_attn_chunk_kernel(RecDev d, 
   if (d.odd) {
     const long long slot0 = base / LA_C + s, groups = d.heads / d.odd_heads;
     bool odd = false;
-    for (int i = t; i < (n + LA_C - 1) / LA_C * d.odd_each; i += LA_T)
+    for (int i = t; i < (n + d.odd_chunk - 1) / d.odd_chunk * d.odd_each; i += LA_T)
       odd = odd || d.odd[((slot0 + i / d.odd_each) * groups + h / d.odd_heads) * d.odd_each + i % d.odd_each];
     if (!__syncthreads_or(odd)) return;
     sp_in = d.first + (slot0 * d.heads + h) * static_cast<long long>(d.dim) * d.vdim;
@@ -316,7 +316,7 @@ constexpr int WT_T = 256;           // threads: 16 x 16, each 4 query rows (ti +
 // BN: keys per tile. 64 halves the barriers per key; 32 lets two CTAs share an SM at 128-wide heads (the kernel is bound by
 // shared-memory and FMA latency with 8 warps, so a second CTA is what fills the issue slots)
 
-// SIG: sigmoid weights, written with the scores (no row statistics, one barrier less per key tile). odd: null, or where window_attn_mma_kernel left its word
+// SIG: sigmoid weights, written with the scores (no row statistics, one barrier less per key tile). odd: null, or where the tensor-core form left its word
 // per (sequence, key / value head): what it did is not done again
 template <int MV, int BN, bool SIG>
 __global__ void __launch_bounds__(WT_T, BN == 32 ? 2 : 1) window_attn_tiled_kernel(WinDev d, const int* odd, int ldq_s, int ldv_s, int dim4, int vdim4, bool qvec, bool kvvec) {

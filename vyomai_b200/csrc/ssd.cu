@@ -421,6 +421,7 @@ extern "C" int vy_ssd(const VySsd* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_ssd: null params");
   VY_NEED_DEVICE("vy_ssd");
+  if (poison_raised("vy_ssd")) return VY_ERR_CUDA;
   VY_CHECK_ARG(p->n_seqs > 0 && p->n_seqs <= 65535 && p->max_new > 0 && p->rows > 0 && p->cu_tokens && p->pos0 && p->slot, "vy_ssd: bad batch");
   VY_CHECK_ARG(p->heads > 0 && p->heads <= 65535 && p->groups > 0 && p->heads % p->groups == 0 && p->dim > 0 && p->dim <= 256 && p->vdim > 0 && p->vdim <= 1024 &&
                    p->taps >= 1 && p->taps <= 16, "vy_ssd: heads %d, groups %d, dim %d (<= 256), vdim %d (<= 1024), taps %d (1..16)", p->heads, p->groups, p->dim,
