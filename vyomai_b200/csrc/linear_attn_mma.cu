@@ -8,7 +8,7 @@
 // The walk this replaces for long portions (linear_attn_chunk_kernel: one CTA per sequence, head and slice of columns goes through the chunks in
 // order, on fp32 FMAs) is as long as the sequence and leaves SMs idle for few sequences; here only the scan is serial, and it is bound by the bytes
 // of the states (dim x vdim x 4 per chunk and head, written twice, read twice). q and k shared by a group of heads (state space: b and c) are
-// split, and their scores computed, once per group.
+// split, and their scores computed, once per group. A state-space prompt whose rows come in quads has the first and the third launch on tcgen05 (linear_attn_tc.cu).
 //
 // The fp16 halves are off by at most 2^-49 of the largest entry under their unit, a row of q, k or v or a whole state. la_states looks at the rows (tokens) and
 // columns (channels) of every chunk's q, k and v, as each warp has them, and of the state that is carried in: where the largest entry of one is below 2^-20 of the
