@@ -351,6 +351,47 @@ def test_gemm_fp32_write_back(pair, bn, dtype):
     assert L.vy_gemm_poisoned() == 0
 
 
+@pytest.mark.parametrize("kind", ["fp32", "fp32_of_fp32", "bf16", "add", "swiglu"])
+@pytest.mark.parametrize("pair,bn", [(0, 64), (0, 128), (0, 192), (0, 256), (1, 128), (1, 192), (1, 256)])
+def test_gemm_write_back_from_tile_to_tile(pair, bn, kind):
+    """Results that leave through bulk tensor stores when a CTA goes through many tiles one after the other (few k-blocks, so that the write-back is the slower side): a
+    staging buffer is written again only once its store has been read. Tiles that end with an odd number of stores, by their width or by N (its last columns mod 32: 4, 8,
+    12, 16, 24), are where the turn of the two buffers counts. Every entry against float64 (fp32 sums of 64 exact products, or tf32 operands; then the rounding to
+    bf16), the repeats against the first to the bit."""
+    from vyomai_b200 import _lib, ops
+    bf = torch.bfloat16
+    src = torch.float32 if kind == "fp32_of_fp32" else bf
+    if (pair and src == torch.float32) or (kind == "swiglu" and bn in (64, 192)):
+        pytest.skip("not a form of this kind")
+    L, K = _lib.lib(), 64
+    try:
+        for i, (M, N) in enumerate(((8000, 2088), (6100, 1552), (9001, 1164), (8000, 900), (8000, 1560))):
+            if kind in ("bf16", "add", "swiglu") and N % 8:   # rows of bf16 on 16-byte boundaries
+                continue
+            a, b, res = _randn((M, K), 80 + i, src).to(DEV, src), _randn((N, K), 90 + i, src, K ** -0.5).to(DEV, src), _randn((M, N), 100 + i, bf).to(DEV, bf)
+            z, room = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+            err = room * (K * 2.0 ** -24 if src == bf else 2.0 ** -9)
+            kw = dict(out_dtype=torch.float32 if kind.startswith("fp32") else bf)
+            if kind == "add":
+                kw["addend"], z = res, z + res.double()
+            if kind == "swiglu":
+                kw["act"] = "swiglu"
+                g, u = z[:, 0::2], z[:, 1::2]
+                err = 1.2 * err[:, 0::2] * u.abs() + g.abs() * err[:, 1::2] + 1e-6 * (g * u).abs()   # |silu'| < 1.1; e^x and the division
+                z = g * torch.sigmoid(g) * u
+            if kw["out_dtype"] == bf:
+                err = err + 2.0 ** -8 * z.abs()
+            L.vy_gemm_tune_override(pair, bn, 0)
+            first = ops.gemm(a, b, **kw)
+            wrong = (first.double() - z).abs() > err + 1e-30
+            assert not bool(wrong.any()), (M, N, int(wrong.sum()), wrong.nonzero()[:4].tolist())
+            for _ in range(8):
+                assert torch.equal(first, ops.gemm(a, b, **kw)), (M, N)
+    finally:
+        L.vy_gemm_tune_override(-1, 0, 0)
+    assert L.vy_gemm_poisoned() == 0
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 6e-3), (torch.float32, 2e-3)])
 def test_gemm_epilogues_vs_oracle(dtype, tol):
     """bias + exact-erf GELU (+ saved pre-activation), tanh GELU, residual addend, dGELU (the dgrad epilogue), swap-AB

@@ -327,6 +327,11 @@ enum { EPI_PLAIN = 0, EPI_ADD = 1, EPI_GELU = 2, EPI_DGELU = 3 };
 // row operand (addend / aux) of the first two chunks is fetched before the accumulator is awaited and
 // each later chunk's while its predecessor is processed; the two staging buffers alternate so one
 // __syncwarp per chunk suffices. (With EPI_GELU + aux both buffers are used by every chunk.)
+// With bulk stores, waiting for all but the last one covers the buffer that is written next only while the stores of a warp alternate, from one tile of a persistent CTA
+// to the next as well: a tile that begins with the first buffer behind one that ended with it (an odd number of chunks, or of chunks before N) could write over what is still
+// being read. So widths with an odd number of chunks per warp, SwiGLU and fp32 results go on with the buffer whose turn it is (`turn`, its offset; between tiles it rests in
+// shared memory, since a register held through all epilogues spills), and widths with an even number, whose loop has its two buffers at fixed offsets (with variable ones
+// 8192 x 4096, K 768 in pairs of 256 columns: dGELU 75.4 -> 79.6 us, residual 57.8 -> 61.2), wait for all stores behind a tile that N cut to an odd number.
 __device__ __forceinline__ void store_ragged8(__nv_bfloat16* dst, const uint4& v, int n) {
   const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
 #pragma unroll
@@ -359,7 +364,7 @@ __device__ __forceinline__ void load_bias8(const GemmDev& g, int col, float (&bb
 template <int BN, int MODE, bool TMA>
 __device__ __forceinline__ void epilogue_linear_fast(const GemmDev& g, uint32_t tmem_acc, int m0, int n0, int q, int half,
                                                      int lane, const float* bias_s, uint64_t* tfull_bar, uint32_t tfull_phase,
-                                                     uint32_t tmem_empty_bar, uint8_t* stage, int trace_tile,
+                                                     uint32_t tmem_empty_bar, uint8_t* stage, uint32_t* turn_at, int trace_tile,
                                                      const CUtensorMap* tma_out, const CUtensorMap* tma_aux) {
   constexpr int WC = BN >= 64 ? BN / 2 : BN;
   constexpr int NCH = WC / 32;
@@ -376,6 +381,12 @@ __device__ __forceinline__ void epilogue_linear_fast(const GemmDev& g, uint32_t 
   const int gc0 = n0 + wcol0;  // first global column of this warp
   const float scale = g.out_scale == 0.f ? 1.f : g.out_scale;
   const bool save_aux = MODE == EPI_GELU && g.aux != nullptr;
+  constexpr bool TURNS = TMA && NCH % 2 != 0;
+  uint32_t turn = TURNS ? *turn_at : 0;
+  if (TMA && !TURNS && *turn_at) {   // the last store went out of the first buffer
+    if (elect_one_sync()) tma_store_wait_read<0>();
+    __syncwarp();
+  }
 
   const __nv_bfloat16* pf_src = nullptr;
   if (row_ok) {
@@ -437,9 +448,10 @@ __device__ __forceinline__ void epilogue_linear_fast(const GemmDev& g, uint32_t 
     prefetch_bias(c + 1);
     const int nvalid = g.N - (gc0 + c * 32);
     if (nvalid <= 0) return;
+    if (TURNS && !save_aux) stg = stage + turn;
     uint8_t* srow = stg + lane * 64;
     if (TMA) {
-      // the buffer about to be overwritten must have been read by its bulk store: the out buffers alternate per chunk,
+      // the buffer about to be overwritten must have been read by its bulk store: the out buffers alternate per store,
       // so only the store before the last has to be done — except with GELU + aux, where both buffers are used every chunk
       if (elect_one_sync()) {  // the lane that issued (and committed) the bulk stores: the same one is elected every time
         if (save_aux) tma_store_wait_read<0>();
@@ -499,6 +511,7 @@ __device__ __forceinline__ void epilogue_linear_fast(const GemmDev& g, uint32_t 
         if (save_aux) tma_store_2d(tma_aux, stage + GEMM_STAGE_OUT, gc0 + c * 32, m0 + q * 32);
         tma_store_commit();
       }
+      if (TURNS) turn ^= GEMM_STAGE_OUT;
       return;
     }
     __syncwarp();
@@ -565,7 +578,8 @@ __device__ __forceinline__ void epilogue_linear_fast(const GemmDev& g, uint32_t 
       process(NCH - 1, raw, pf[0], stage);
     }
   }
-  __syncwarp();  // the next tile's first chunk reuses stage buffer 0
+  if (TMA && !save_aux && lane == 0) *turn_at = TURNS ? turn : gc0 < g.N && gc0 + WC > g.N ? (g.N - gc0 + 31) / 32 & 1 : 0;
+  __syncwarp();  // the next tile's first chunk writes a staging buffer
 }
 
 
@@ -575,7 +589,7 @@ __device__ __forceinline__ void epilogue_linear_fast(const GemmDev& g, uint32_t 
 template <int BN>
 __device__ __forceinline__ void epilogue_swiglu_fast(const GemmDev& g, uint32_t tmem_acc, int m0, int n0, int q, int half, int lane,
                                                      uint64_t* tfull_bar, uint32_t tfull_phase, uint32_t tmem_empty_bar,
-                                                     uint8_t* stage, const CUtensorMap* tma_out) {
+                                                     uint8_t* stage, uint32_t* turn_at, const CUtensorMap* tma_out) {
   static_assert(BN % 128 == 0, "SwiGLU fast epilogue: an even number of 32-column chunks per warp");
   constexpr int WC = BN / 2;
   constexpr int NCH = WC / 32;
@@ -583,16 +597,17 @@ __device__ __forceinline__ void epilogue_swiglu_fast(const GemmDev& g, uint32_t 
   const int gc0 = n0 + wcol0;
   const float scale = g.out_scale == 0.f ? 1.f : g.out_scale;
   const int sw = (lane >> 1) & 3;
+  uint32_t turn = *turn_at;
   mbar_wait_soft(tfull_bar, tfull_phase, g.poison);
   tc_fence_after();
   const uint32_t taddr = tmem_acc + wcol0;
 #pragma unroll 1
   for (int c = 0; c < NCH; c += 2) {
     const bool live = gc0 + c * 32 < g.N;
-    uint8_t* stg = (c & 2) ? stage + GEMM_STAGE_OUT : stage;
+    uint8_t* stg = stage + turn;   // see above: per store sent off
     uint8_t* srow = stg + lane * 64;
     if (live) {
-      if (elect_one_sync()) tma_store_wait_read<1>();  // the bulk store that last read this buffer (two pairs ago) is done
+      if (elect_one_sync()) tma_store_wait_read<1>();  // the bulk store that last read this buffer (two stores ago) is done
       __syncwarp();
     }
 #pragma unroll 1
@@ -625,7 +640,9 @@ __device__ __forceinline__ void epilogue_swiglu_fast(const GemmDev& g, uint32_t 
       tma_store_2d(tma_out, stg, (gc0 + c * 32) >> 1, m0 + q * 32);
       tma_store_commit();
     }
+    turn ^= GEMM_STAGE_OUT;
   }
+  if (lane == 0) *turn_at = turn;
   __syncwarp();
 }
 
@@ -635,7 +652,7 @@ __device__ __forceinline__ void epilogue_swiglu_fast(const GemmDev& g, uint32_t 
 // pace of these products: bf16 7970 x 5152, K 1024: 183.7 us, so 70.7 (1189 TFLOP/s, result 2.3 TB/s); 7970 x 1536, K 512: 63.4, 17.5; tf32 1576 x 3072, K 768: 39.2, 18.9.
 template <int BN>
 __device__ __forceinline__ void epilogue_f32_fast(const GemmDev& g, uint32_t tmem_acc, int m0, int n0, int q, int half, int lane,
-                                                  uint64_t* tfull_bar, uint32_t tfull_phase, uint32_t tmem_empty_bar, uint8_t* stage,
+                                                  uint64_t* tfull_bar, uint32_t tfull_phase, uint32_t tmem_empty_bar, uint8_t* stage, uint32_t* turn_at,
                                                   const CUtensorMap* tma_out) {
   constexpr int WC = BN >= 64 ? BN / 2 : BN;
   constexpr int NCH = WC / 32;
@@ -649,6 +666,7 @@ __device__ __forceinline__ void epilogue_f32_fast(const GemmDev& g, uint32_t tme
   const int gc0 = n0 + wcol0;
   const float scale = g.out_scale == 0.f ? 1.f : g.out_scale;
   const int sw = (lane >> 1) & 3;
+  uint32_t turn = *turn_at;
   const long long arow = g.addend && grow < g.M ? remap_add_row(g, grow) * g.ld_addend + gc0 : -1;
   float add[32];
   const auto fetch = [&](int c) {  // the row operand of chunk c; a row's last columns one by one
@@ -683,7 +701,7 @@ __device__ __forceinline__ void epilogue_f32_fast(const GemmDev& g, uint32_t tme
     for (int h = 0; h < 2; ++h) {
       const int col0 = gc0 + c * 32 + h * 16;
       if (col0 >= g.N) continue;
-      uint8_t* srow = stage + h * GEMM_STAGE_OUT + lane * 64;
+      uint8_t* srow = stage + turn + lane * 64;
       if (elect_one_sync()) tma_store_wait_read<1>();  // the store before the last, out of this buffer, has been read
       __syncwarp();
 #pragma unroll
@@ -711,12 +729,14 @@ __device__ __forceinline__ void epilogue_f32_fast(const GemmDev& g, uint32_t tme
       fence_proxy_async_smem();
       __syncwarp();
       if (elect_one_sync()) {
-        tma_store_2d(tma_out, stage + h * GEMM_STAGE_OUT, col0, m0 + q * 32);
+        tma_store_2d(tma_out, stage + turn, col0, m0 + q * 32);
         tma_store_commit();
       }
+      turn ^= GEMM_STAGE_OUT;
     }
     fetch(c + 1);
   }
+  if (lane == 0) *turn_at = turn;
   __syncwarp();
 }
 
@@ -951,6 +971,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   uint64_t* tfull_bar = bars + 2 * STAGES;   // [2]
   uint64_t* tempty_bar = bars + 2 * STAGES + 2;  // [2]
   uint32_t* tmem_ptr_s = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint32_t* turns = tmem_ptr_s + 1;          // [epilogue warps]
 
   // broadcast through a shuffle so that the compiler knows the warp index (and everything derived from it: role, TMEM
   // lane quarter, staging buffer, store coordinates) is warp-uniform and keeps it in uniform registers
@@ -1144,6 +1165,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     const int half = e >> 2;
     const int et = threadIdx.x - GEMM_FIRST_EPI_WARP * 32;
     uint8_t* stage = epi_stage + e * 2 * GEMM_STAGE_OUT;
+    if (lane == 0) turns[e] = 0;
+    __syncwarp();
     // which fused fast epilogue applies (-1: the general one)
     int fast_mode = -1;
     if (g.epi == VY_EPI_LINEAR && !g.transposed_out && g.vec_ok && g.out_dtype == VY_BF16 && !g.addend2 &&
@@ -1174,11 +1197,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       }
       const uint32_t tmem_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       if constexpr (WB == WB_GATED) {
-        epilogue_swiglu_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, &tma_out);
+        epilogue_swiglu_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e, &tma_out);
         continue;
       }
       if constexpr (WB == WB_F32) {
-        epilogue_f32_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, &tma_out);
+        epilogue_f32_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e, &tma_out);
         continue;
       }
       if (g.debug & 1) {
@@ -1195,31 +1218,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
                                 reinterpret_cast<float*>(epi_stage));
       } else if (fast_mode == EPI_PLAIN) {
         if (g.tma_store)
-          epilogue_linear_fast<BN, EPI_PLAIN, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_PLAIN, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                     local, &tma_out, &tma_aux);
         else
-          epilogue_linear_fast<BN, EPI_PLAIN, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_PLAIN, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                      local, &tma_out, &tma_aux);
       } else if (fast_mode == EPI_ADD) {
         if (g.tma_store)
-          epilogue_linear_fast<BN, EPI_ADD, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_ADD, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                     local, &tma_out, &tma_aux);
         else
-          epilogue_linear_fast<BN, EPI_ADD, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_ADD, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                      local, &tma_out, &tma_aux);
       } else if (fast_mode == EPI_GELU) {
         if (g.tma_store)
-          epilogue_linear_fast<BN, EPI_GELU, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_GELU, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                     local, &tma_out, &tma_aux);
         else
-          epilogue_linear_fast<BN, EPI_GELU, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_GELU, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                      local, &tma_out, &tma_aux);
       } else if (fast_mode == EPI_DGELU) {
         if (g.tma_store)
-          epilogue_linear_fast<BN, EPI_DGELU, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_DGELU, true>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                     local, &tma_out, &tma_aux);
         else
-          epilogue_linear_fast<BN, EPI_DGELU, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage,
+          epilogue_linear_fast<BN, EPI_DGELU, false>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e,
                                                      local, &tma_out, &tma_aux);
       } else {
         epilogue_linear_general<BN>(g, tmem_acc, m0, n0, q, half, lane, bs, &tfull_bar[acc], acc_ph, tempty_addr);
