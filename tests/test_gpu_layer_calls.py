@@ -99,3 +99,72 @@ def test_cached_layers_in_one_call_per_sublayer(monkeypatch, dtype, cache, seqs,
     bad = StaticCacheOne(cfg, max_cache_len=before, batch_size=seqs, dtype=cache, is_gqa=True)
     with pytest.raises(ValueError), torch.no_grad():
         layer(token, None, freqs=rope, use_cache=True, kv_cache=bad, start_pos=before)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("forget", [False, True])
+def test_checkpointed_layers_save_the_same_when_computed_again(dtype, forget):
+    """The first layers of a shape go launch by launch, and the last one's backward pass settles the tilings of the others: what a layer saves must not depend on it, or
+    torch.utils.checkpoint refuses the recomputation. Nor on whether tilings have been forgotten in between."""
+    from torch.utils.checkpoint import checkpoint
+    from vyomai_b200 import gemm_tune
+    from vyomai_b200.functional import MaskSpec, RopeTables
+    from vyomai_b200.layers.positional_embeddings import RotaryEmbedding
+    from vyomai_b200.models.encoder import EncoderLayer
+    torch.manual_seed(0)
+    cfg = _config(256, 2)
+    layers, rope, mask = [EncoderLayer(cfg, i, "gqa").to(DEV, dtype).train() for i in range(3)], RopeTables(RotaryEmbedding(cfg)(300)), MaskSpec()
+    x, dy = torch.randn(3, 50, 256, device=DEV, dtype=dtype, requires_grad=True), torch.randn(3, 50, 256, device=DEV, dtype=dtype)
+    params = [p for m in layers for p in m.parameters()]
+
+    def step(again):
+        y = x
+        for m in layers:
+            y = checkpoint(m, y, mask, rope, use_reentrant=False) if again else m(y, mask, rope)
+        if forget and again:
+            gemm_tune.LAYERS.clear()
+        return [y] + list(torch.autograd.grad(y, [x] + params, dy))
+
+    gemm_tune.clear()
+    first, second, plain = step(True), step(True), step(False)
+    for got in (first, second):
+        assert all(torch.equal(a, b) for a, b in zip(got, plain))
+
+
+@pytest.mark.parametrize("forward_by_launch", [False, True])
+def test_directions_that_go_their_own_ways(monkeypatch, forward_by_launch):
+    """One direction as one call, the other launch by launch."""
+    from vyomai_b200 import gemm_tune
+    from vyomai_b200.functional import MaskSpec, RopeTables
+    from vyomai_b200.layers.positional_embeddings import RotaryEmbedding
+    from vyomai_b200.models.encoder import EncoderLayer
+    torch.manual_seed(1)
+    cfg = _config(256, 2)
+    layer, rope = EncoderLayer(cfg, 0, "gqa").to(DEV, torch.bfloat16).train(), RopeTables(RotaryEmbedding(cfg)(300))
+    x, dy = torch.randn(3, 70, 256, device=DEV, dtype=torch.bfloat16, requires_grad=True), torch.randn(3, 70, 256, device=DEV, dtype=torch.bfloat16)
+    params, names = list(layer.parameters()), _calls(monkeypatch)
+
+    def step(between=lambda: None):
+        y = layer(x, MaskSpec(), rope)
+        between()
+        return [y] + list(torch.autograd.grad(y, [x] + params, dy))
+
+    gemm_tune.clear()
+    want = step()
+    step()
+    kept = dict(gemm_tune.LAYERS)
+    assert len(kept) == 4
+
+    def other_way():
+        gemm_tune.LAYERS.clear()
+        gemm_tune.LAYERS.update({k: v for k, v in kept.items() if (k[0] == "backward") == forward_by_launch})
+
+    def back():
+        gemm_tune.LAYERS.update(kept) if forward_by_launch else other_way()
+
+    if forward_by_launch:
+        other_way()
+    names.clear()
+    got = step(back)
+    assert ("vy_attn_block_fwd" in names) != forward_by_launch and ("vy_attn_block_bwd" in names) == forward_by_launch
+    assert all(torch.equal(a, b) for a, b in zip(want, got))

@@ -31,7 +31,7 @@ def attention_block_fn(mod, x2d: torch.Tensor, B: int, S: int, mask: MaskSpec, r
             raise _lib.VyomError("gradients through a kv-cache forward are not supported (use_cache=True is an inference path)")
         from .autograd_train import AttentionBlockFn
         flat = [x2d] + a.ws + [b for b in a.bs if b is not None] + [a.wo] + ([a.bo] if a.bo is not None else []) + [a.gamma, a.beta]
-        return AttentionBlockFn.apply(mod, B, S, mask, rope, start_pos, *flat)
+        return AttentionBlockFn.apply(a, B, S, mask, rope, start_pos, *flat)
     key = block.attention_key(a, x2d, B, S, mask, rope, kv, decode_no_mask, False)
     hints = gemm_tune.LAYERS.get(key)
     if hints is not None:
@@ -87,7 +87,7 @@ def feed_forward_fn(mod, h2d: torch.Tensor, input2d: torch.Tensor) -> torch.Tens
     key = block.ffn_key(mod._act_name, h2d, input2d, w1, b1, w2, b2, ln, gamma, beta, mod.training and m["dropout"].p > 0.0, train)
     if train:
         from .autograd_train import FeedForwardFn
-        return FeedForwardFn.apply(mod._act_name, ln.eps, F.dropout_state(mod, mod.dropout.p), key, h2d, input2d, w1, b1, w2, b2, gamma, beta)
+        return FeedForwardFn.apply(mod._act_name, ln, F.dropout_state(mod, mod.dropout.p), key, h2d, input2d, w1, b1, w2, b2, gamma, beta)
     hints = gemm_tune.LAYERS.get(key)
     if hints is not None:
         return block.ffn_forward(mod._act_name, h2d, input2d, w1, b1, w2, b2, gamma, beta, ln.eps, hints)[0]

@@ -144,13 +144,12 @@ class AttentionBlockFn(torch.autograd.Function):
     projection weights, their biases (if any), dense.weight, [dense.bias], ln.weight, ln.bias."""
 
     @staticmethod
-    def forward(ctx, mod, B, S, mask: MaskSpec, rope, start_pos, x2d, *params):
-        ctx.mod, ctx.B, ctx.S, ctx.mask, ctx.rope, ctx.start_pos = mod, B, S, mask, rope, start_pos
-        parts = block.AttentionParts(mod)
+    def forward(ctx, parts: block.AttentionParts, B, S, mask: MaskSpec, rope, start_pos, x2d, *params):
+        ctx.parts, ctx.B, ctx.S, ctx.mask, ctx.rope, ctx.start_pos, ctx.drop = parts, B, S, mask, rope, start_pos, None
+        mod = parts.mod
         ctx.key = key = block.attention_key(parts, x2d, B, S, mask, rope, None, False, True)
         hints = gemm_tune.LAYERS.get(key)
-        ctx.whole = hints is not None and ("backward", key) in gemm_tune.LAYERS   # both directions as one call each, or neither
-        if ctx.whole:
+        if hints is not None:
             y, scratch = block.attention_forward(parts, x2d, B, S, mask, rope, None, start_pos, key, hints, save=True)
             ctx.save_for_backward(x2d, scratch)
             return y
@@ -162,30 +161,29 @@ class AttentionBlockFn(torch.autograd.Function):
             q, k, v, lse = saved
             ctx.drop = F.dropout_state(mod.out, mod.out.dropout.p)
             y, (s, mean, rstd) = F.self_output(attn, x2d, dense, ln, save=True, dropout=ctx.drop)
-        if key is not None:
+        if key is None:
+            ctx.save_for_backward(x2d, q, k, v, attn, s, lse, mean, rstd)
+        else:   # what the one call leaves
             gemm_tune.keep_layer(key, got, 2)
-        ctx.n_w = len(lin)
-        ctx.has_qkv_bias = lin[0].bias is not None
-        ctx.has_dense_bias = dense.bias is not None
-        ctx.save_for_backward(x2d, q, k, v, attn, lse, s, mean, rstd)
+            ctx.save_for_backward(x2d, block.pack([q, k, v, attn, s, lse, mean, rstd]))
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        if ctx.whole:
-            x2d, scratch = ctx.saved_tensors
-            return (None, None, None, None, None, None, *block.attention_backward(block.AttentionParts(ctx.mod), x2d, scratch, dy.contiguous(), ctx.B, ctx.S, ctx.mask,
-                                                                                  ctx.rope, ctx.start_pos, gemm_tune.LAYERS.get(("backward", ctx.key), (0, 0, 0, 0))))
+        x2d, *saved = ctx.saved_tensors
+        if ctx.key is None:
+            return AttentionBlockFn._launches(ctx, dy, x2d, *saved)
+        parts, hints = ctx.parts, gemm_tune.LAYERS.get(("backward", ctx.key))
+        if hints is not None:
+            return (None, None, None, None, None, None, *block.attention_backward(parts, x2d, *saved, dy.contiguous(), ctx.B, ctx.S, ctx.mask, ctx.rope, ctx.start_pos, hints))
         with gemm_tune.collecting() as got:
-            grads = AttentionBlockFn._launches(ctx, dy)
-        if ctx.key is not None:
-            gemm_tune.keep_layer(("backward", ctx.key), got, 4)
+            grads = AttentionBlockFn._launches(ctx, dy, x2d, *block.attention_saved(*saved, x2d, ctx.B, ctx.S, parts.mod.num_attention_heads, parts.mod._kv_heads))
+        gemm_tune.keep_layer(("backward", ctx.key), got, 4)
         return grads
 
     @staticmethod
-    def _launches(ctx, dy):
-        x2d, q, k, v, attn, lse, s, mean, rstd = ctx.saved_tensors
-        mod, B, S, mask, rope = ctx.mod, ctx.B, ctx.S, ctx.mask, ctx.rope
+    def _launches(ctx, dy, x2d, q, k, v, attn, s, lse, mean, rstd):
+        mod, B, S, mask, rope = ctx.parts.mod, ctx.B, ctx.S, ctx.mask, ctx.rope
         lin = mod._packed()
         dense, ln = mod.out.dense, mod.out.layernorm
         w_qkv, _ = F.pack_linears(lin)
@@ -220,7 +218,7 @@ class AttentionBlockFn(torch.autograd.Function):
                 n = l.weight.shape[0]
                 grads.append(d_wqkv[r:r + n])
                 r += n
-        if ctx.has_qkv_bias:
+        if lin[0].bias is not None:
             gb = _packed_grads([l.bias for l in lin])
             if gb is not None:
                 acc = not all(_overwrite(l.bias) for l in lin)
@@ -239,7 +237,7 @@ class AttentionBlockFn(torch.autograd.Function):
                     grads.append(d_bqkv[r:r + n])
                     r += n
         grads.append(d_wo)
-        if ctx.has_dense_bias:
+        if dense.bias is not None:
             grads.append(d_bo)
         grads += [dgamma, dbeta]
         ops.side_join()
@@ -337,13 +335,12 @@ class FeedForwardFn(torch.autograd.Function):
     """y = LN(W2 act(W1 h + b1) + b2 + input)."""
 
     @staticmethod
-    def forward(ctx, act, eps, dropout, key, h2d, input2d, w1, b1, w2, b2, gamma, beta):
+    def forward(ctx, act, ln, dropout, key, h2d, input2d, w1, b1, w2, b2, gamma, beta):
         ctx.drop = dropout
-        ctx.act, ctx.eps, ctx.key = act, eps, key
+        ctx.act, ctx.ln, ctx.key = act, ln, key
         ctx.params = (w1, b1, w2, b2, gamma, beta)  # the Parameter objects (direct-gradient attributes live on them)
-        hints = gemm_tune.LAYERS.get(key)
-        ctx.whole = hints is not None and ("backward", key) in gemm_tune.LAYERS
-        if ctx.whole:
+        eps, hints = ln.eps, gemm_tune.LAYERS.get(key)
+        if hints is not None:
             y, scratch = block.ffn_forward(act, h2d, input2d, w1, b1, w2, b2, gamma, beta, eps, hints, save=True)
             ctx.save_for_backward(h2d, scratch)
             return y
@@ -356,26 +353,30 @@ class FeedForwardFn(torch.autograd.Function):
             else:
                 y, s, mean, rstd = ops.add_layernorm(F._lin(a, w2, b2), input2d.contiguous(), gamma, beta, eps, save_stats=True,
                                                      save_sum=True, dropout=dropout)
-        if key is not None:
+        if key is None:
+            ctx.save_for_backward(h2d, z, a, s, mean, rstd)
+        else:   # what the one call leaves
             gemm_tune.keep_layer(key, got, 2)
-        ctx.save_for_backward(h2d, z, a, s, mean, rstd)
+            ctx.save_for_backward(h2d, block.pack([z, a, s, mean, rstd]))
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        if ctx.whole:
-            h2d, scratch = ctx.saved_tensors
-            dh, ds, *grads = block.ffn_backward(ctx.act, h2d, scratch, dy.contiguous(), *ctx.params, ctx.eps, gemm_tune.LAYERS.get(("backward", ctx.key), (0, 0, 0, 0)))
+        h2d, *saved = ctx.saved_tensors
+        if ctx.key is None:
+            return FeedForwardFn._launches(ctx, dy, h2d, *saved)
+        w1, b1, w2, b2, gamma, beta = ctx.params
+        hints = gemm_tune.LAYERS.get(("backward", ctx.key))
+        if hints is not None:
+            dh, ds, *grads = block.ffn_backward(ctx.act, h2d, *saved, dy.contiguous(), *ctx.params, ctx.ln.eps, hints)
             return None, None, None, None, dh, ds, *grads
         with gemm_tune.collecting() as got:
-            grads = FeedForwardFn._launches(ctx, dy)
-        if ctx.key is not None:
-            gemm_tune.keep_layer(("backward", ctx.key), got, 4)
+            grads = FeedForwardFn._launches(ctx, dy, h2d, *block.ffn_saved(*saved, h2d, w1.shape[0]))
+        gemm_tune.keep_layer(("backward", ctx.key), got, 4)
         return grads
 
     @staticmethod
-    def _launches(ctx, dy):
-        h2d, z, a, s, mean, rstd = ctx.saved_tensors
+    def _launches(ctx, dy, h2d, z, a, s, mean, rstd):
         w1, b1, w2, b2, gamma, beta = ctx.params
         ds, dgamma, dbeta, d_b2 = _ln_bwd(dy.contiguous(), s, gamma, beta, mean, rstd, bias=b2, dropout=ctx.drop)
         ds, dxo = _split_ds(ds)  # gradient of input_tensor, gradient of the second Linear's output

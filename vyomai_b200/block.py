@@ -3,9 +3,14 @@
 The functions here take over from functional.py / autograd_train.py where a sublayer's tensors are what those calls take: one dtype, contiguous, on the device,
 no dropout, head_dim 64, tilings settled. Everything else, and a sublayer's first call of each shape (whose products time their tilings), goes the
 general way, launch by launch. Nothing is kept from a call but the tilings, by the values that they depend on; addresses are read anew each time.
+
+Where the one call applies, both ways save the same for the backward pass: the input and one buffer as the library lays it out (`pack`, `attention_saved`, `ffn_saved`).
+So either direction goes its own way, and a forward pass that is computed again (torch.utils.checkpoint) saves what the first one did, whatever has been settled in between.
+With the same tilings the two ways give the same results to the bit; tilings are chosen by timing, and another split of a weight gradient's sum rounds otherwise.
 """
 from __future__ import annotations
 
+import math
 from ctypes import byref
 from typing import Optional
 
@@ -49,6 +54,24 @@ def _param(module, name: str):
 
 def _buffer(nbytes: int, like: torch.Tensor) -> torch.Tensor:
     return torch.empty(nbytes, device=like.device, dtype=torch.uint8)
+
+
+def _pieces(buf: torch.Tensor, specs) -> list:
+    """Views of `buf`, one per (shape, dtype), one after the other on boundaries of 256 bytes: the library's layout of what a forward call leaves."""
+    out, at = [], 0
+    for shape, dt in specs:
+        n = math.prod(shape) * dt.itemsize
+        out.append(buf[at:at + n].view(dt).view(shape))
+        at += (n + 255) // 256 * 256
+    return out
+
+
+def pack(ts) -> torch.Tensor:
+    """The buffer that the one call would have left, from the tensors of the general way."""
+    buf = _buffer(sum((t.numel() * t.element_size() + 255) // 256 * 256 for t in ts), ts[0])
+    for view, t in zip(_pieces(buf, [(tuple(t.shape), t.dtype) for t in ts]), ts):
+        view.copy_(t)
+    return buf
 
 
 # ---- attention block ----
@@ -155,6 +178,13 @@ def attention_backward(a: AttentionParts, x2d, scratch, dy, B, S, mask, rope, st
     return grads + [dg, db]
 
 
+def attention_saved(buf, x2d, B, S, heads, kv_heads) -> list:
+    """[q, k, v, attn, s, lse, mean, rstd] of a forward call with `save`."""
+    bf, f32, (rows, H) = torch.bfloat16, torch.float32, x2d.shape
+    return _pieces(buf, [((B, heads, S, 64), bf), ((B, kv_heads, S, 64), bf), ((B, kv_heads, S, 64), bf), ((rows, heads * 64), x2d.dtype), ((rows, H), x2d.dtype),
+                         ((B, heads, S), f32), ((rows,), f32), ((rows,), f32)])
+
+
 # ---- feed-forward block ----
 def ffn_key(act, h2d, input2d, w1, b1, w2, b2, ln, gamma, beta, drops: bool, train: bool) -> Optional[tuple]:
     T = h2d.dtype
@@ -175,6 +205,12 @@ def _ffn_args(act, h2d, input2d, w1, b1, w2, b2, gamma, beta, eps, save: bool):
     return _FFN(rows=h2d.shape[0], width=h2d.shape[1], inner=w1.shape[0], dtype=_DT[h2d.dtype], act=fwd, dact=bwd, h=h2d.data_ptr(),
                 input=input2d.data_ptr() if input2d is not None else h2d.data_ptr(), w1=w1.data_ptr(), b1=ops._ptr(b1), w2=w2.data_ptr(), b2=ops._ptr(b2),
                 gamma=gamma.data_ptr(), beta=beta.data_ptr(), eps=eps, weights_static=0 if torch.is_grad_enabled() else 1, save=int(save), stream=ops._stream())
+
+
+def ffn_saved(buf, h2d, inner: int) -> list:
+    """[z, a, s, mean, rstd] of a forward call with `save`."""
+    (rows, H), T = h2d.shape, h2d.dtype
+    return _pieces(buf, [((rows, inner), T), ((rows, inner), T), ((rows, H), T), ((rows,), torch.float32), ((rows,), torch.float32)])
 
 
 def ffn_forward(act, h2d, input2d, w1, b1, w2, b2, gamma, beta, eps, hints: tuple, save: bool = False):
