@@ -133,7 +133,7 @@ def test_checkpointed_layers_save_the_same_when_computed_again(dtype, forget):
 
 @pytest.mark.parametrize("forward_by_launch", [False, True])
 def test_directions_that_go_their_own_ways(monkeypatch, forward_by_launch):
-    """One direction as one call, the other launch by launch."""
+    """One direction as one call, the other launch by launch; weights that lie elsewhere by the time of the backward pass."""
     from vyomai_b200 import gemm_tune
     from vyomai_b200.functional import MaskSpec, RopeTables
     from vyomai_b200.layers.positional_embeddings import RotaryEmbedding
@@ -168,3 +168,15 @@ def test_directions_that_go_their_own_ways(monkeypatch, forward_by_launch):
     got = step(back)
     assert ("vy_attn_block_fwd" in names) != forward_by_launch and ("vy_attn_block_bwd" in names) == forward_by_launch
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+    gemm_tune.LAYERS.update(kept)
+    spacers = []
+
+    def move():
+        for p in params:
+            spacers.append(torch.empty(1 << 20, device=DEV))
+            p.data = p.data.clone()
+
+    names.clear()
+    got = step(move)
+    assert "vy_attn_block_bwd" in names and all(torch.equal(a, b) for a, b in zip(want, got))

@@ -174,11 +174,13 @@ class AttentionBlockFn(torch.autograd.Function):
         if ctx.key is None:
             return AttentionBlockFn._launches(ctx, dy, x2d, *saved)
         parts, hints = ctx.parts, gemm_tune.LAYERS.get(("backward", ctx.key))
-        if hints is not None:
+        same = block.attention_weights_fit(parts, x2d)
+        if same and hints is not None:
             return (None, None, None, None, None, None, *block.attention_backward(parts, x2d, *saved, dy.contiguous(), ctx.B, ctx.S, ctx.mask, ctx.rope, ctx.start_pos, hints))
         with gemm_tune.collecting() as got:
             grads = AttentionBlockFn._launches(ctx, dy, x2d, *block.attention_saved(*saved, x2d, ctx.B, ctx.S, parts.mod.num_attention_heads, parts.mod._kv_heads))
-        gemm_tune.keep_layer(("backward", ctx.key), got, 4)
+        if same:
+            gemm_tune.keep_layer(("backward", ctx.key), got, 4)
         return grads
 
     @staticmethod
@@ -367,12 +369,14 @@ class FeedForwardFn(torch.autograd.Function):
             return FeedForwardFn._launches(ctx, dy, h2d, *saved)
         w1, b1, w2, b2, gamma, beta = ctx.params
         hints = gemm_tune.LAYERS.get(("backward", ctx.key))
-        if hints is not None:
+        same = block.ffn_weights_fit(h2d, w1, b1, w2, b2, gamma, beta, ctx.key[4])
+        if same and hints is not None:
             dh, ds, *grads = block.ffn_backward(ctx.act, h2d, *saved, dy.contiguous(), *ctx.params, ctx.ln.eps, hints)
             return None, None, None, None, dh, ds, *grads
         with gemm_tune.collecting() as got:
             grads = FeedForwardFn._launches(ctx, dy, h2d, *block.ffn_saved(*saved, h2d, w1.shape[0]))
-        gemm_tune.keep_layer(("backward", ctx.key), got, 4)
+        if same:
+            gemm_tune.keep_layer(("backward", ctx.key), got, 4)
         return grads
 
     @staticmethod

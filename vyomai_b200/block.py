@@ -121,6 +121,20 @@ def attention_key(a: AttentionParts, x2d, B, S, mask, rope, kv, decode_no_mask, 
     return ("attention", train, B, S, H, T, Hq, Hkv, bs[0] is not None, a.bo is not None, rope is not None, kind, gemm_tune.ENABLED, x2d.device)
 
 
+def attention_weights_fit(a: AttentionParts, x2d) -> bool:
+    """Are the parameters still what `attention_key` found? What was put into their `.data` since the forward pass may lie elsewhere or be of another type."""
+    ws, bs, H, n = a.ws, a.bs, x2d.shape[1], (a.mod.num_attention_heads + 2 * a.mod._kv_heads) * 64
+    if not _plain(x2d.dtype, *ws, *bs, a.wo, a.bo, a.gamma, a.beta) or sum([w.numel() for w in ws]) != n * H or a.wo.numel() != a.mod.num_attention_heads * 64 * H:
+        return False
+    if a.gamma.numel() != H or a.beta.numel() != H or (a.bo is not None and a.bo.numel() != H) or (bs[0] is not None and sum([b.numel() for b in bs]) != n):
+        return False
+    stacked = lambda: _stacked(ws) and (bs[0] is None or _stacked(bs))  # noqa: E731
+    if not stacked():
+        pack_linears(a.lin)
+        return stacked()   # the module may hold other parameters by now
+    return True
+
+
 def _attention_args(a: AttentionParts, x2d, B, S, mask, rope, kv, start_pos, kind: int, save: bool):
     mod = a.mod
     st = _ATTN(seqs=B, tokens=S, width=x2d.shape[1], heads=mod.num_attention_heads, kv_heads=mod._kv_heads, dtype=_DT[x2d.dtype], x=x2d.data_ptr(),
@@ -198,6 +212,13 @@ def ffn_key(act, h2d, input2d, w1, b1, w2, b2, ln, gamma, beta, drops: bool, tra
     if train and (H >= 4096 or F >= 4096 or _direct((w1, b1, w2, b2, gamma, beta))):
         return None
     return ("ffn", train, rows, H, F, T, act, b1 is not None, b2 is not None, gemm_tune.ENABLED, h2d.device)
+
+
+def ffn_weights_fit(h2d, w1, b1, w2, b2, gamma, beta, inner: int) -> bool:
+    """As attention_weights_fit."""
+    H = h2d.shape[1]
+    return (_plain(h2d.dtype, w1, b1, w2, b2, gamma, beta) and w1.numel() == w2.numel() == inner * H and gamma.numel() == beta.numel() == H and
+            (b1 is None or b1.numel() == inner) and (b2 is None or b2.numel() == H))
 
 
 def _ffn_args(act, h2d, input2d, w1, b1, w2, b2, gamma, beta, eps, save: bool):
