@@ -68,3 +68,46 @@ def test_rotation_of_four_entries_per_lane(layout, rot, dim, norm, pool):
     else:
         _close(a[1], b[1])
     assert torch.equal(a[2], b[2])
+
+
+def _gates():
+    """Arguments of SiLU and sigmoid over fp32's range, dense where e^-x leaves the range of the approximate reciprocal (2^126: x = -87.3) and of fp32 (-88.7)."""
+    e = torch.tensor([float("inf"), float("-inf"), float("nan"), 0.0, -0.0, 3e38, -3e38, -1e30, 1e-30, -1e-30, -100.0, 100.0], device=DEV)
+    x = torch.cat([e, torch.linspace(-89.0, -87.0, 2036, device=DEV), torch.linspace(-110.0, 110.0, 2048, device=DEV)])
+    return x, {"silu": x.double() * torch.sigmoid(x.double()), "sigmoid": torch.sigmoid(x.double())}
+
+
+def _gate_close(got, want, x, act):
+    """A few roundings, and what fp32 flushes where e^-x is infinite: |x| 2^-128 (sigmoid: 2^-128)."""
+    want = torch.where(x == float("-inf"), torch.full_like(want, float("nan") if act == "silu" else 0.0), want)   # x / (1 + e^-x) is -inf / inf there
+    assert torch.equal(got.isnan(), want.isnan())
+    fine = want.isfinite()
+    assert torch.equal(got.double()[~fine].nan_to_num(1.0), want[~fine].nan_to_num(1.0))
+    room = 2.0 ** -21 * want.abs() + 2.0 ** -128 * (x.abs().double().clamp(max=200.0) if act == "silu" else 1.0)
+    assert bool(((got.double() - want).abs() <= room)[fine].all())
+
+
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+def test_gates_over_the_whole_range(act):
+    from vyomai_b200 import ops
+    x, want = _gates()
+    n = 160   # tokens: enough for the form with four channels per thread
+    batch = ops.PackedBatch(*(torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, n], [0], [0])), n)
+    xs = x.expand(n, -1).contiguous()
+    got = ops.causal_conv(batch, xs, torch.ones(x.numel(), 1, device=DEV), torch.zeros(1, x.numel(), 0, device=DEV), act=act)
+    for row in (got[0], got[-1]):
+        _gate_close(row, want[act], x, act)
+    ones = torch.ones(3, x.numel(), device=DEV)
+    got = ops.rms_norm(ones, None, eps=0.0, gate=xs[:3].contiguous(), gate_act=act)
+    _gate_close(got[2], want[act], x, act)
+    if act == "silu":   # the state-space convolution: x | b | c, one tap; what it gives shows in the read-out of a token with no state before it
+        H, dim, vdim = 8, 16, 64
+        v = x[:512].clone()
+        v[:12] = -88.0
+        xs, b = v.expand(4, -1).contiguous(), torch.full((4, dim), 30.0, device=DEV)   # silu(30) = 30 to 1e-13
+        w = dict(conv_w=torch.ones(512 + 2 * dim, 1, device=DEV), conv_b=None, dt_bias=torch.full((H,), -50.0, device=DEV), a_log=torch.zeros(H, device=DEV), skip=torch.ones(H, device=DEV),
+                 norm=torch.full((512,), 1.0, device=DEV), heads=H, groups=1, dim=dim, vdim=vdim, taps=1, norm_groups=1, norm_eps=1.0, out_dtype=torch.float32)
+        batch = ops.PackedBatch(*(torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, 4], [0], [0])), 4)
+        got = ops.ssd(batch, xs, b, b.clone(), torch.zeros(4, H, device=DEV), None, **w, conv_state=torch.zeros(1, 1, 512 + 2 * dim, device=DEV), state=torch.zeros(1, H, dim, vdim, device=DEV),
+                      tickets=torch.zeros(1, 1, dtype=torch.int32, device=DEV))
+        _gate_close(got[0] if bool(got.isfinite().all()) else got[0] * float("nan"), v.double() * torch.sigmoid(v.double()), v, "silu")

@@ -70,3 +70,17 @@ def test_chunks_of_128_tokens_at_the_ends_of_their_range(what):
     for p, q in zip(a, b):
         assert torch.equal(p.isfinite(), q.isfinite())
         _close(p.nan_to_num(0, 0, 0), q.nan_to_num(0, 0, 0))
+
+
+def test_gates_far_below_zero_and_where_their_exponential_leaves_fp32():
+    """A read-out times silu(gate), entry by entry, against the same read-out times silu(1): gates around -88 (e^88 is past the approximate reciprocal), large negative ones, which give zero."""
+    lengths, pos0 = [256, 130], [0, 0]
+    x, w, conv, state = _inputs(lengths, 4, 1, 32, 64, 5)
+    w["norm_eps"] = 1e12   # the norm behind the gate: a division by 1e6 (the rows' own squares are 1e-8 of it)
+    gate = torch.cat([torch.linspace(-89.0, -87.0, 128), torch.tensor([-1e30, -3e38, -1e3, -100.0]), torch.linspace(-30.0, 80.0, 124)]).to(DEV)
+    x["gate"] = gate.expand(386, -1).contiguous()
+    got = _run(lengths, pos0, x, w, conv, state, False)[0].double() * 1e6
+    x["gate"] = torch.ones_like(x["gate"])
+    y = _run(lengths, pos0, x, w, conv, state, False)[0].double() * 1e6 / torch.sigmoid(torch.tensor(1.0, dtype=torch.float64))
+    want, g = y * gate.double() * torch.sigmoid(gate.double()), gate.double().abs().clamp(max=200.0)
+    assert bool(((got - want).abs() <= 2.0 ** -20 * want.abs() + y.abs() * g * 2.0 ** -128 + 1e6 * 2.0 ** -148).all())

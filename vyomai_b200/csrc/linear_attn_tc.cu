@@ -33,23 +33,23 @@ __device__ __forceinline__ void split_pair(f32x2 v, f32x2 f, f32x2 f_lo, unsigne
   lo = pack_h2(__floats2half2_rn(y.x, y.y));
 }
 // x / (1 + e^-x) of both entries, in a third of the instructions of two exponentials and two divisions: e^-x as 2^t with what rounding t left over brought back, then a reciprocal with
-// a Newton step, whose quotient is corrected once (without it the outputs' error grows by a hundredth). Infinities and NaN give what the division gives; a sum past 2^126 stays there
-__device__ __forceinline__ float min_nan(float a, float b) {
+// a Newton step, whose quotient is corrected once (without it the outputs' error grows by a hundredth); see silu_near. Infinities and NaN give what the division gives
+__device__ __forceinline__ float within_100(float a) {   // NaN stays
   float r;
-  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  asm("min.NaN.f32 %0, %1, 0f42C80000;\n\tmax.NaN.f32 %0, %0, 0fC2C80000;" : "=f"(r) : "f"(a));
   return r;
 }
 __device__ __forceinline__ f32x2 silu_pair(f32x2 x) {
   constexpr float L2E = 1.4426950408889634f, L2E_LO = static_cast<float>(1.4426950408889634 - static_cast<double>(L2E));
   const float2 g = unpair(x);
-  const f32x2 c = pair(min_nan(g.x, 100.f), min_nan(g.y, 100.f)), t = mul2(c, pair(-L2E));
+  const f32x2 c = pair(within_100(g.x), within_100(g.y)), t = mul2(c, pair(-L2E));   // e^100 is infinite
   const f32x2 left = fma2(c, pair(-L2E_LO), fma2(c, pair(-L2E), mul2(t, pair(-1.f))));
   const float2 tt = unpair(t);
-  const float2 y = unpair(add2(mul2(pair(vy_ex2_approx(tt.x), vy_ex2_approx(tt.y)), fma2(left, pair(0.6931471805599453f), pair(1.f))), pair(1.f)));
-  const float y0 = min_nan(y.x, 0x1p126f), y1 = min_nan(y.y, 0x1p126f);
-  const f32x2 minus = pair(-y0, -y1), r0 = pair(vy_rcp_approx(y0), vy_rcp_approx(y1)), r = fma2(r0, fma2(minus, r0, pair(1.f)), r0), q = mul2(x, r);
-  const float2 a = unpair(fma2(fma2(minus, q, x), r, q)), b = unpair(q);
-  return pair(a.x == a.x ? a.x : b.x, a.y == a.y ? a.y : b.y);
+  const f32x2 y = add2(mul2(pair(vy_ex2_approx(tt.x), vy_ex2_approx(tt.y)), fma2(left, pair(0.6931471805599453f), pair(1.f))), pair(1.f));
+  const float2 ys = unpair(mul2(y, pair(RECIP_SCALE)));
+  const f32x2 minus = mul2(y, pair(-1.f)), r0 = mul2(pair(vy_rcp_approx(ys.x), vy_rcp_approx(ys.y)), pair(RECIP_SCALE)), r = fma2(r0, fma2(minus, r0, pair(1.f)), r0), q = mul2(x, r);
+  const float2 a = unpair(fma2(fma2(minus, q, x), r, q)), b = unpair(mul2(x, r0));
+  return pair(a.x == a.x ? a.x : b.x, a.y == a.y ? a.y : b.y);   // infinities
 }
 static __device__ __noinline__ float gate_any(float x, int act) { return apply_uact(x, act); }
 

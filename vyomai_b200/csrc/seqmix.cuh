@@ -21,15 +21,18 @@ __device__ __forceinline__ float apply_uact(float x, int act) {
   }
 }
 // 1 / y for y >= 1 in two Newton steps from the approximate reciprocal (1 / infinity = 0; a NaN stays one), and x / (1 + e^-x) with its quotient corrected once: rounded as a
-// division but for a hair, which with its range checks is twice as many instructions
+// division but for a hair, which with its range checks is twice as many instructions. The approximate reciprocal flushes what is below 2^-126 (x below -87.3): it is taken of 2^-30 y
+constexpr float RECIP_SCALE = 0x1p-30f;
+__device__ __forceinline__ float recip_first(float y) { return vy_rcp_approx(y * RECIP_SCALE) * RECIP_SCALE; }
 __device__ __forceinline__ float recip_near(float y) {
-  float r = vy_rcp_approx(y), n = fmaf(r, fmaf(-y, r, 1.f), r);
+  const float r = recip_first(y);
+  float n = fmaf(r, fmaf(-y, r, 1.f), r);
   n = fmaf(n, fmaf(-y, n, 1.f), n);
   return y < INFINITY ? n : r;
 }
 __device__ __forceinline__ float sigmoid_near(float x) { return recip_near(1.f + expf(-x)); }
 __device__ __forceinline__ float silu_near(float x) {
-  const float y = 1.f + expf(-x), r0 = vy_rcp_approx(y), r = fmaf(r0, fmaf(-y, r0, 1.f), r0), q = x * r, a = fmaf(fmaf(-y, q, x), r, q);
+  const float y = 1.f + expf(-x), r0 = recip_first(y), r = fmaf(r0, fmaf(-y, r0, 1.f), r0), q = x * r, a = fmaf(fmaf(-y, q, x), r, q);
   return a == a ? a : x * r0;   // infinities
 }
 __device__ __forceinline__ float uact_near(float x, int act) {
