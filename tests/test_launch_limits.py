@@ -18,3 +18,24 @@ def test_shared_memory_limits_are_set_per_device():
             assert kept is None or "[dev]" in before, (path, src[m.start():m.start() + 100])
             sets += 1
     assert sets > 0
+
+
+def test_register_shares_that_a_build_does_not_have_choose_another_form():
+    """Kernels whose warps share registers out (setmaxnreg) run only where the compiler gave the count that the shares add up to. Whether it did belongs to the rule that
+    chooses the form - another toolkit's build then takes the forms beside them - and is no error of the call. The build that is here has it."""
+    kernels = {"window_attn_tc": ("window_attn_tc_applies", "TC_REGS", 4, "window_attn_tc_kernel"), "linear_attn_tc": ("linear_attn_tc_applies", "LT_REGS", 1, "la_outputs_tc_kernel")}
+    csrc = os.path.join(ROOT, "vyomai_b200", "csrc")
+    for path in glob.glob(os.path.join(csrc, "*.cu")):
+        if "setmaxnreg" in open(path).read():
+            assert os.path.basename(path)[:-3] in kernels
+    for name, (rule, regs, forms, kernel) in kernels.items():
+        src = open(os.path.join(csrc, name + ".cu")).read()
+        assert "cudaErrorInvalidConfiguration" not in src
+        count = int(re.search(rf"\b{regs} = (\d+)", src).group(1))
+        body = src[src.index(f"bool {rule}("):]
+        body = body[:body.index("\n}")]
+        assert "registers" in body and re.search(r"\) return false;|!enough\) return false;", body)
+        log = os.path.join(csrc, "build", name + ".ptxas.log")
+        if os.path.exists(log):
+            used = re.findall(rf"entry function '[^']*{kernel}[^']*'(?:(?!entry function).)*?Used (\d+) registers", open(log).read(), re.S)
+            assert len(used) == forms and all((int(u) + 7) // 8 * 8 == count for u in used)

@@ -773,6 +773,12 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
 bool linear_attn_tc_applies(const RecDev& d) {
   const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
   if (d.dim > 128 || d.vdim < 32 || d.in_act != VY_UACT_NONE) return false;
+  // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever: what a compiler gives another number does without this form
+  static const bool enough = [] {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, la_outputs_tc_kernel) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == LT_REGS;
+  }();
+  if (!enough) return false;
   return d.out_dt == VY_F32 && quads(d.out, d.ld_out) && (!d.gate || quads(d.gate, d.ld_gate));
 }
 
@@ -820,12 +826,6 @@ cudaError_t launch_la_outputs_tc(const RecDev& d, const LaChunks& w, int hp, int
   static std::atomic<unsigned long long> allowed{0};
   cudaError_t e = allow_smem(la_outputs_tc_kernel, allowed);
   if (e != cudaSuccess) return e;
-  // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever
-  static const bool enough = [] {
-    cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, la_outputs_tc_kernel) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == LT_REGS;
-  }();
-  if (!enough) return cudaErrorInvalidConfiguration;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
   CUtensorMap gate_map, out_map;

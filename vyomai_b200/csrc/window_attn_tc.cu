@@ -545,8 +545,19 @@ long long window_attn_tc_floats(const WinDev& d, int n_seqs, int max_new) {
   return static_cast<long long>(n_seqs) * d.kv_heads * (w.cap * (w.row_bytes / 4 + 2) + 4LL * w.blocks + 4);
 }
 
+// with fewer registers at launch than the warps share out, the first to ask for more would wait for ever: what a compiler gives another number does without this form
+template <int VD, bool SIG>
+static bool tc_registers() {
+  static const bool enough = [] {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, window_attn_tc_kernel<VD, SIG>) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == TC_REGS;
+  }();
+  return enough;
+}
+
 bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new) {
   if (d.dim > 128 || d.vdim > 128) return false;
+  if (!(d.vdim > 64 ? (d.sigmoid ? tc_registers<128, true>() : tc_registers<128, false>()) : d.sigmoid ? tc_registers<64, true>() : tc_registers<64, false>())) return false;
   // tensor-map rows are counted in 32 bits
   if (static_cast<long long>(n_seqs) * d.kv_heads * (split_slots(d, max_new) + 2 * TC_KEYS) > 0x7fffffffLL - 2 * TC_KEYS) return false;
   const int hl = tc_head_bits(d);
@@ -571,12 +582,6 @@ static cudaError_t launch_tc(const CUtensorMap& map, const WinDev& d, const Spli
   static std::atomic<unsigned long long> allowed{0};
   cudaError_t e = allow_smem(window_attn_tc_kernel<VD, SIG>, allowed);
   if (e != cudaSuccess) return e;
-  // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever
-  static const bool enough = [] {
-    cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, window_attn_tc_kernel<VD, SIG>) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == TC_REGS;
-  }();
-  if (!enough) return cudaErrorInvalidConfiguration;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
   return launch_kernel(window_attn_tc_kernel<VD, SIG>, grid, dim3(TC_THREADS), total(), st, map, d, w, geo, poison);
