@@ -43,6 +43,22 @@ def test_convolution_of_four_channels_per_thread(taps, act):
     assert torch.equal(*states)
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+def test_convolutions_keep_infinities_to_the_tokens_that_see_them(taps):
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(taps)
+    C, n = 8192, 160
+    batch = ops.PackedBatch(*(torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, n], [0], [0])), n)
+    x, w = torch.randn(n, C, generator=g, device=DEV), torch.randn(C, taps, generator=g, device=DEV)
+    x[5, 3], x[33, 3], x[33, 8], x[47, 100], x[159, 7] = float("inf"), float("nan"), float("-inf"), float("inf"), float("inf")
+    a, b = (ops.causal_conv(batch, t, w, torch.zeros(1, C, max(taps - 1, 1), device=DEV)[:, :, :taps - 1].contiguous(), act=None) for t in (x, _off(x)))
+    seen = torch.zeros(n, C, dtype=torch.bool, device=DEV)
+    for i, c in (~x.isfinite()).nonzero().tolist():
+        seen[i:i + taps, c] = True
+    assert torch.equal(~a.isfinite(), seen) and torch.equal(a.isnan(), b.isnan())
+    _close(a.nan_to_num(0, 0, 0), b.nan_to_num(0, 0, 0))
+
+
 @pytest.mark.parametrize("layout,rot,dim", [("half", 64, 128), ("half", 24, 48), ("pairs", 6, 20), ("pairs", 128, 128), ("pairs", 0, 128), ("half", 128, 128)])
 @pytest.mark.parametrize("norm,pool", [("weight", torch.float32), ("unit", torch.float32), (None, torch.bfloat16), ("unit", None)])
 def test_rotation_of_four_entries_per_lane(layout, rot, dim, norm, pool):

@@ -600,6 +600,7 @@ __global__ void __launch_bounds__(128) causal_conv_quads_kernel(ConvDev d) {
     float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int t = 0; t < TAPS; ++t) {
+      if (t >= d.taps) break;   // a weight of 0 would bring infinities and NaN of tokens further back along
       const float4 v = x[u + TAPS - 1 - t];
       y = make_float4(fmaf(w[t].x, v.x, y.x), fmaf(w[t].y, v.y, y.y), fmaf(w[t].z, v.z, y.z), fmaf(w[t].w, v.w, y.w));
     }
