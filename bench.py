@@ -1182,7 +1182,7 @@ def measure_latent(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, de
     fl = len(cfgd["layers"]) * tokens * m["heads"] * visible * (m["dim"] + m["rot_dim"] + m["vdim"]) * 2
     ms = sum(z["prefill_kernels"].get(k, {}).get("ms", 0.0) for k in ("window_attn_tc", "window_attn_mma"))
     if ms:
-        z["window_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        z["window_attn_prompt_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     # single-token attention: the bytes of the visible latent rows, read once per (sequence, layer) if the heads share them through L2
     dk = z["decode_kernels_eager"]   # 8 or more heads per latent row: the heads-as-rows kernel and its merge; else the key-parallel kernel
     ms = sum(dk.get(k, {}).get("ms", 0.0) for k in ("window_attn_heads", "window_attn_heads_merge", "window_attn_decode"))
@@ -1210,7 +1210,7 @@ def measure_latent(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, de
     fl = n_par * tokens * par["heads"] * vis * (par["dim"] + par["vdim"]) * 2
     ms = sum(gz["prefill_kernels"].get(k, {}).get("ms", 0.0) for k in ("window_attn_tc", "window_attn_mma"))
     if ms:
-        gz["window_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        gz["window_attn_prompt_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     ms = gz["decode_kernels_eager"].get("window_attn_decode", {}).get("ms")
     if ms:
         by = n_par * batch_decode * (Wg + K) * par["kv_heads"] * (par["dim"] + par["vdim"]) * 4
@@ -1330,7 +1330,7 @@ def measure_talking(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     fl = len(ld["layers"]) * tokens * lm["heads"] * vis * (lm["dim"] + lm["rot_dim"] + lm["vdim"]) * 2
     ms = sum(lz["prefill_kernels"].get(k, {}).get("ms", 0.0) for k in ("window_attn_tc", "window_attn_mma"))
     if ms:
-        lz["window_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        lz["window_attn_prompt_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     dk = lz["decode_kernels_eager"]
     ms = sum(dk.get(k, {}).get("ms", 0.0) for k in ("window_attn_heads", "window_attn_heads_merge", "window_attn_decode"))
     if ms:
@@ -1439,7 +1439,7 @@ def measure_fubinex(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     # recurrences: per (token, head) and state element, gated linear attention does a decay multiply and two multiply-adds (5 flop), the
     # chunked fixed-decay kernel is counted as in --workload hybrid
     z["prefill_roofline"] = {
-        "window_attn_mma": _roof(pk, ("window_attn_tc", "window_attn_mma"), flop=fl_attn, **rf),
+        "window_attn_prompt": _roof(pk, ("window_attn_tc", "window_attn_mma"), flop=fl_attn, **rf),
         "gated_linear_attn (delta_rule kernel, no correction)": _roof(pk, ("delta_rule",), flop=n_par * tokens * rt["heads"] * rt["dim"] * rt["vdim"] * 5, **rf),
         "linear_attn_chunk": _roof(pk, ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), flop=n_ret * tokens * ret["heads"] * (2 * ret["dim"] * ret["vdim"] + 32 * (ret["dim"] + ret["vdim"])) * 2, **rf),
         # row kernels against the copy bandwidth: fp32 in, bf16 out (poly_norm); q / k read and written in fp32, v copied (rotation)
@@ -1483,7 +1483,7 @@ def measure_fubinex(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     vis = sum(min(p + 1, Wg) + (min(K, p + 1 - Wg) if p + 1 > Wg else 0) for p in range(prompt)) / prompt
     gpk, gdk = gz["prefill_kernels"], gz["decode_kernels_eager"]
     gz["prefill_roofline"] = {
-        "window_attn_mma": _roof(gpk, ("window_attn_tc", "window_attn_mma"), flop=g_par * tokens * gl["heads"] * vis * (gl["dim"] + gl["vdim"]) * 2, **rf),
+        "window_attn_prompt": _roof(gpk, ("window_attn_tc", "window_attn_mma"), flop=g_par * tokens * gl["heads"] * vis * (gl["dim"] + gl["vdim"]) * 2, **rf),
         # the delta rule adds the correction's contraction: a decay multiply and three multiply-adds per state element (7 flop)
         "delta_rule": _roof(gpk, ("delta_rule", "delta_chunk", "delta_scan"), flop=g_par * tokens * gr["heads"] * gr["dim"] * gr["vdim"] * 7, **rf),
         "linear_attn_chunk": _roof(gpk, ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), flop=g_lin * tokens * glin["heads"] * (2 * glin["dim"] * glin["vdim"] + 32 * (glin["dim"] + glin["vdim"])) * 2, **rf),
@@ -1576,7 +1576,7 @@ def measure_kifetar(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     chan = 2 * dl["kv_heads"] * dl["dim"] + dl["heads"] * dl["vdim"]
     vis = sum(min(p + 1, W) for p in range(prompt)) / prompt
     z["prefill_roofline"] = {
-        "window_attn_mma": _roof(pk, ("window_attn_tc", "window_attn_mma"), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
+        "window_attn_prompt": _roof(pk, ("window_attn_tc", "window_attn_mma"), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
         # a decay multiply and three multiply-adds per state element and token, as Gelutar's delta rule is counted
         "gd_scan (gated delta rule)": _roof(pk, ("gd_scan",), flop=n_d * tokens * state * 7, **rf),
         # row kernels against the copy bandwidth. gd_prep: projections in, unit vectors / values / records out (fp32)
@@ -1616,7 +1616,7 @@ def measure_kifetar(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     gstate, gchan = gr["heads"] * gr["dim"] * gr["vdim"], 2 * gr["kv_heads"] * gr["dim"] + gr["heads"] * gr["vdim"]
     glin = gd["layers"][0]["mixer"]
     gz["prefill_roofline"] = {
-        "window_attn_mma": _roof(gpk, ("window_attn_tc", "window_attn_mma"), flop=g_par * tokens * gl["heads"] * gvis * (gl["dim"] + gl["vdim"]) * 2, **rf),
+        "window_attn_prompt": _roof(gpk, ("window_attn_tc", "window_attn_mma"), flop=g_par * tokens * gl["heads"] * gvis * (gl["dim"] + gl["vdim"]) * 2, **rf),
         "delta_rule (+ its preparing launch)": _roof(gpk, ("delta_rule", "delta_chunk", "delta_scan"), flop=g_par * tokens * gstate * 7, **rf),
         "causal_conv": _roof(gpk, ("causal_conv",), byts=g_par * tokens * gchan * 8, **rf),
         # layer norms (bf16 out), the parallel layer's q / k norms and its two output norms added into the residual, the recurrences' gated read-outs
@@ -1712,7 +1712,7 @@ def measure_zaparax(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     chosen = top * moe["router"]["experts"] / (moe["router"]["experts"] + moe["router"]["identity"])
     vis = sum(min(p + 1, W) for p in range(prompt)) / prompt
     z["prefill_roofline"] = {
-        "window_attn_mma": _roof(pk, ("window_attn_tc", "window_attn_mma"), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
+        "window_attn_prompt": _roof(pk, ("window_attn_tc", "window_attn_mma"), flop=n_a * tokens * at["heads"] * vis * (at["dim"] + at["vdim"]) * 2, **rf),
         # per token and head: carried state read and updated (dim x vdim each), half a chunk of 64 inside it; counted as the fixed-decay form is
         "linear_attn_chunk (state-space recurrence)": _roof(pk, ("linear_attn_chunk", "la_states", "la_scan", "la_outputs"), flop=n_s * tokens * sm["heads"] *
                                                             (2 * sm["state"] * sm["vdim"] + 32 * (sm["state"] + sm["vdim"])) * 2, **rf),
@@ -1753,7 +1753,7 @@ def measure_zaparax(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     kpk, kdk = kz["prefill_kernels"], kz["decode_kernels_eager"]
     kstate, kchan = dl["heads"] * dl["dim"] * dl["vdim"], 2 * dl["kv_heads"] * dl["dim"] + dl["heads"] * dl["vdim"]
     kz["prefill_roofline"] = {
-        "window_attn_mma": _roof(kpk, ("window_attn_tc", "window_attn_mma"), flop=n_a * tokens * ka["heads"] * vis * (ka["dim"] + ka["vdim"]) * 2, **rf),
+        "window_attn_prompt": _roof(kpk, ("window_attn_tc", "window_attn_mma"), flop=n_a * tokens * ka["heads"] * vis * (ka["dim"] + ka["vdim"]) * 2, **rf),
         "gd_scan (gated delta rule)": _roof(kpk, ("gd_scan",), flop=n_s * tokens * kstate * 7, **rf),
         "gd_prep": _roof(kpk, ("gd_prep",), byts=n_s * tokens * (2 * kchan + 18 * dl["heads"]) * 4, **rf),
         "sandwich_norm": _roof(kpk, ("sandwich_norm",), byts=2 * n_all * tokens * width * 14, **rf),

@@ -58,23 +58,22 @@ constexpr int LU_T = 256, LU_VB = 64 * 2 + 16;   // threads; bytes between rows 
 // ACT: see act_of
 template <bool TD, int ACT>
 __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w, int hp, int vslices, int dim16, bool vec) {
-  constexpr int C = LM_C;
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) unsigned char lu_smem[];
   const int kb = dim16 * 2 + 16;
   unsigned char* Kh = lu_smem;
-  unsigned char* Kl = Kh + C * kb;
-  unsigned char* Wh = Kl + C * kb;
-  unsigned char* Wl = Wh + C * LU_VB;
-  float* es = reinterpret_cast<float*>(Wl + C * LU_VB);   // [64] decay to the chunk's end times write strength
-  float* ku = es + C;                                     // [128], [64]: units of k's channels and of w's columns
+  unsigned char* Kl = Kh + LM_C * kb;
+  unsigned char* Wh = Kl + LM_C * kb;
+  unsigned char* Wl = Wh + LM_C * LU_VB;
+  float* es = reinterpret_cast<float*>(Wl + LM_C * LU_VB);   // [64] decay to the chunk's end times write strength
+  float* ku = es + LM_C;                                     // [128], [64]: units of k's channels and of w's columns
   float* wu = ku + 128;
   Range* range = reinterpret_cast<Range*>(wu + 64);          // [4]: k, q, v, state
   const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
-  const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * C;
+  const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LM_C;
   if (t0 >= n) return;
-  const int nt = min(C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
+  const int nt = min(LM_C, n - t0), t = threadIdx.x, warp = t >> 5, lane = t & 31, gq = lane >> 2, tq = lane & 3;
   const int hq = TD ? h0 / (d.heads / d.kv_heads) : h0, vw = min(64, d.vdim - v0);
   const long long r0 = base + t0, slot = la_slot(d, s, c);
   if (t < 4) range[t] = {0u, RANGE_NONE};
@@ -82,10 +81,10 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
   const bool few = nt < 8;
   {
     const int row = lane >> 2, ch = 16 * warp + 4 * (lane & 3);
-    float4 x[C / 8];
+    float4 x[LM_C / 8];
     const auto read = [&](const void* p, long long ld) {
 #pragma unroll
-      for (int i = 0; i < C / 8; ++i) {
+      for (int i = 0; i < LM_C / 8; ++i) {
         const int r = row + 8 * i;
         x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < nt && ch < d.dim) x[i] = act4<ACT>(load4(p, d.in_dt, vec, (r0 + r) * ld + static_cast<long long>(hq) * d.dim, ch, d.dim), d.in_act);
@@ -94,26 +93,26 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
     Range rk = {0u, RANGE_NONE}, rq = rk;
     if (v0 == 0) {
       read(d.q, d.ldq);
-      look<C / 8, 4>(x, few, d.dim - 16 * warp < 4, rq);
+      look<LM_C / 8, 4>(x, few, d.dim - 16 * warp < 4, rq);
       note_warp(range + 1, rq);
     }
     read(d.k, d.ldk);
-    const uint4 m = look<C / 8, 4>(x, few, d.dim - 16 * warp < 4, rk);
+    const uint4 m = look<LM_C / 8, 4>(x, few, d.dim - 16 * warp < 4, rk);
     note_warp(range, rk);
     const float4 sc = column_scales(m);
     if (row == 0) *reinterpret_cast<float4*>(ku + ch) = column_units(m);
     if (ch < dim16) {
 #pragma unroll
-      for (int i = 0; i < C / 8; ++i) store_split4(Kh, Kl, (row + 8 * i) * kb + ch * 2, x[i], sc);
+      for (int i = 0; i < LM_C / 8; ++i) store_split4(Kh, Kl, (row + 8 * i) * kb + ch * 2, x[i], sc);
     }
   }
   const unsigned ka = smem_addr(Kh) + lane_b(lane, kb) + 16 * warp * 2, wb = smem_addr(Wh) + lane_bt(lane, LU_VB);
   const int row = lane >> 1, vc = 8 * warp + 4 * (lane & 1);
   Range rv = {0u, RANGE_NONE}, rs = rv;   // this thread's share
-  float4 next[C / 16];
+  float4 next[LM_C / 16];
   const auto fetch = [&](int h) {
 #pragma unroll
-    for (int i = 0; i < C / 16; ++i) {
+    for (int i = 0; i < LM_C / 16; ++i) {
       const int r = row + 16 * i;
       next[i] = r < nt ? load4(d.v, d.in_dt, vec, (r0 + r) * d.ldv + static_cast<long long>(h) * d.vdim + v0, vc, vw) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -123,41 +122,41 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
     __syncthreads();   // the previous head's readers of es and W are done
     if constexpr (TD) {
       if (warp == 0) {
-        const float whole = token_decays<C / 32>(d, r0, nt, h, lane, [&](int i, double L, float strength, double end) { es[i] = expf(static_cast<float>(end - L)) * strength; });
+        const float whole = token_decays<LM_C / 32>(d, r0, nt, h, lane, [&](int i, double L, float strength, double end) { es[i] = expf(static_cast<float>(end - L)) * strength; });
         if (lane == 0 && v0 == 0) w.D[slot * d.heads + h] = whole;
       }
-    } else if (t <= C) {
-      if (t < C) es[t] = t < nt ? power(d.decay[h], nt - 1 - t) : 0.f;
+    } else if (t <= LM_C) {
+      if (t < LM_C) es[t] = t < nt ? power(d.decay[h], nt - 1 - t) : 0.f;
       else if (v0 == 0) w.D[slot * d.heads + h] = power(d.decay[h], nt);
     }
     if (t == 0 && v0 == 0) w.top[slot * d.heads + h] = 0u;
-    float4 y[C / 16];
+    float4 y[LM_C / 16];
 #pragma unroll
-    for (int i = 0; i < C / 16; ++i) y[i] = next[i];
+    for (int i = 0; i < LM_C / 16; ++i) y[i] = next[i];
     if (h + 1 < h0 + hp) fetch(h + 1);   // in flight during this head's products
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < C / 16; ++i) {
+    for (int i = 0; i < LM_C / 16; ++i) {
       if (row + 16 * i < nt) y[i] = act4<ACT>(y[i], d.in_act);
     }
-    uint4 m = look<C / 16, 2>(y, few, vw - 8 * warp < 4, rv);
+    uint4 m = look<LM_C / 16, 2>(y, few, vw - 8 * warp < 4, rv);
     {   // the weighted columns' units from a bound, the columns' largest times the largest weight: rows are within 2^20 of one another, and the halves good to 2^24
       unsigned top = 0u;
 #pragma unroll
-      for (int i = lane; i < C; i += 32) top = max(top, abs_bits(es[i]));
+      for (int i = lane; i < LM_C; i += 32) top = max(top, abs_bits(es[i]));
       const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, top));
       const auto times = [most](unsigned b) { return __float_as_uint(__uint_as_float(b) * most); };
       m = make_uint4(times(m.x), times(m.y), times(m.z), times(m.w));
     }
 #pragma unroll
-    for (int i = 0; i < C / 16; ++i) {
+    for (int i = 0; i < LM_C / 16; ++i) {
       const float e = es[row + 16 * i];
       y[i] = make_float4(y[i].x * e, y[i].y * e, y[i].z * e, y[i].w * e);
     }
     const float4 sv = column_scales(m);
     if (row == 0) *reinterpret_cast<float4*>(wu + vc) = column_units(m);
 #pragma unroll
-    for (int i = 0; i < C / 16; ++i) store_split4(Wh, Wl, (row + 16 * i) * LU_VB + vc * 2, y[i], sv);
+    for (int i = 0; i < LM_C / 16; ++i) store_split4(Wh, Wl, (row + 16 * i) * LU_VB + vc * 2, y[i], sv);
     if (c == 0 && d.pos0[s] > 0) {   // the state that is carried in: a thread reads every fourth entry of a column
       const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 + (t & 63);
       unsigned top = 0u;
@@ -177,15 +176,15 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
 #pragma unroll
         for (int k = 0; k < 4; ++k) a[i][k] = b[i][k] = 0.f;
 #pragma unroll
-      for (int k = 0; k < C / 16; ++k) {
+      for (int k = 0; k < LM_C / 16; ++k) {
         unsigned ah[4], al[4];   // k^T: stored [token][channel], read transposed (lane_b's order is what .trans turns into an A operand)
         ldsm_x4_t(ah, ka + 16 * k * kb);
-        ldsm_x4_t(al, ka + C * kb + 16 * k * kb);
+        ldsm_x4_t(al, ka + LM_C * kb + 16 * k * kb);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           unsigned bh[4], bl[4];
           ldsm_x4_t(bh, wb + 16 * k * LU_VB + 32 * j);
-          ldsm_x4_t(bl, wb + C * LU_VB + 16 * k * LU_VB + 32 * j);
+          ldsm_x4_t(bl, wb + LM_C * LU_VB + 16 * k * LU_VB + 32 * j);
           mma_f16(b[2 * j], al, bh[0], bh[1]);
           mma_f16(b[2 * j + 1], al, bh[2], bh[3]);
           mma_f16(a[2 * j], ah, bh[0], bh[1]);
@@ -200,7 +199,7 @@ __global__ void __launch_bounds__(LU_T, 2) la_states_kernel(RecDev d, LaChunks w
         const int i = 16 * warp + gq + 8 * r;
         if (i >= d.dim) continue;
         const float u1 = ku[i];
-        constexpr float cut = (C / 16 + 1) * 0.5f * SPLIT_CUT;
+        constexpr float cut = (LM_C / 16 + 1) * 0.5f * SPLIT_CUT;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int col = 8 * j + 2 * tq;

@@ -1,18 +1,18 @@
 // Prompt-sized windowed attention over pages on tcgen05 (vy_window_attn, long portions, up to 128 channels): the same arithmetic as
 // window_attn_mma.cu - fp32 precision from fp16 halves - with scores, weights and weighted values in tensor memory.
 //
-// A CTA owns 128 rows: 2^hl query heads of one key / value head times 128 / 2^hl queries. Tiles of 128 keys go in turn to two groups of eight
-// warps (tile t to group t % 2), two threads per row, each group with maxima, sums and outputs (in registers) of its own, which meet at the end: while
-// one group turns scores into weights, the tensor pipe works for the other. A row's two threads take turns at runs of 32 keys and half of the output columns each. Per tile
-//   scores:  small products lo hi + hi lo first, then hi hi onto 2^-11 of them (scale-input-d), one accumulator of 128 columns;
-//   weights: two passes over the scores (final score and maximum, written back; then exp, the value row's unit and the split into halves), the
-//            halves written over the scores they came from (16 columns -> 8 of hi, 8 of lo);
-//   values:  the weights as A out of tensor memory, values as B out of shared memory, the tile's own sum; added to the registers when the group
-//            takes up its next tile. (Sums over all tiles in tensor memory would cut off at every step: see SPLIT_CUT.)
+// A CTA owns 128 rows: 2^hl query heads of one key / value head times 128 / 2^hl queries. Tiles of 64 keys go in turn to two groups of four
+// warps (tile t to group t % 2), a thread per row, each group with maxima, sums and outputs (in registers) of its own, which meet at the end: while
+// one group turns scores into weights, the tensor pipe works for the other. Per tile
+//   scores:  two tiles by one product of 128 columns: small products lo hi + hi lo first, then hi hi onto 2^-11 of them (scale-input-d);
+//   weights: a row's 64 scores in registers (final score, maximum, exp, the value row's unit, the split into halves), the halves over the scores
+//            (32 columns of hi, 32 of lo);
+//   values:  the weights as A out of tensor memory, values as B out of shared memory, the tile's own sum; added to the registers once the group
+//            has its next tile's weights. (Sums over all tiles in tensor memory would cut off at every step: see SPLIT_CUT.)
 // Split rows come from a workspace (window_attn_split_kernel, second layout) by tensor maps; K and V tiles have rings of their own.
 //
-// What bounds it: the two softmax groups' own instructions (3400 cycles per pair of tiles, with 24 + 18 products of 128 x 128 or 64 x 16 in 2400 beside them), and
-// 19,000 cycles per CTA before the first and after the last tile. 4 x 2048 tokens, 16 heads of 96 / 64 channels over the whole context: 182 us and 42 for the
+// What bounds it: the two softmax groups' own instructions (3400 cycles per pair of tiles with 96 / 64 channels, 4400 with 128 / 128; the products beside them take 2400), and
+// 16,000 to 22,000 cycles (8 to 11 us) per CTA before the first and after the last tile. 4 x 2048 tokens, 16 heads of 96 / 64 channels over the whole context: 182 us and 42 for the
 // splitting (mma.sync: 545 and 41); 8 heads of 128 over 2, window 512, capped, sloped: 98 and 8 (236 and 8); sigmoid weights 97 and 8 (237 and 8).
 // Tried: 128-key tiles with one buffer of scores per group 284 us, the same with two threads per row 250 (of the first); 64-key scores alone per product 185.
 #include "seqmix.cuh"
@@ -563,7 +563,7 @@ bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new) {
   const int hl = tc_head_bits(d);
   const long long rows = static_cast<long long>(max_new) << hl;
   if (rows < TC_ROWS || rows / TC_ROWS >= 65535) return false;   // the last: a grid's limit
-  // A CTA takes 8 us before its first tile and after its last; with a tile or two between them the 64-row CTAs of window_attn_mma.cu are as good.
+  // A CTA takes 8 to 11 us before its first tile and after its last; with a tile or two between them the 64-row CTAs of window_attn_mma.cu are as good.
   // Splitting and attention, mma.sync / tcgen05, four portions of n tokens from position 0, 8 heads of 128 over 2: n = 64 20.8 / 23.9 us, 128 24.6 / 24.3,
   // 300 41.4 / 28.7; 16 heads of 96 / 64 with keys of their own: 128 22.4 / 23.3, 200 31.7 / 26.9, 1000 201 / 104. Portions of 32 tokens on 2000 cached
   // ones, 8 heads over 2, window 512: 62 / 39
