@@ -1,5 +1,6 @@
-"""-m gpu: state-space prompts in chunks of 128 tokens (csrc/linear_attn_tc.cu) against the form in chunks of 64 that the same call takes where the gate is one element
-off a 16-byte boundary. Either is within about 2^-22 of the result's 2-norm of 64-bit arithmetic: 8 * 2^-24 between them."""
+"""-m gpu: state-space prompts in chunks of 128 tokens (csrc/linear_attn_tc.cu) against a token-by-token walk in 64 bits, and against the form in chunks of 64 that the same
+call takes where the gate is one element off a 16-byte boundary. Either is within about 2^-22 of the result's 2-norm of 64-bit arithmetic (measured 1.4e-7 for outputs, 3.5e-7
+for states): 8 * 2^-24 between them, 16 * 2^-24 from the walk (whose convolution and steps are in 64 bits too)."""
 import pytest
 import torch
 
@@ -39,17 +40,58 @@ def _run(lengths, pos0, x, w, conv, state, off):
     return out, state
 
 
-def _close(a, b):
-    assert a.shape == b.shape and float((a.double() - b.double()).norm()) <= BOUND * float(b.double().norm())
+def _walk(lengths, pos0, x, w, conv, state):
+    """Token by token in 64 bits: (outputs, states)."""
+    H, G, dim, vdim, taps = (w[k] for k in ("heads", "groups", "dim", "vdim", "taps"))
+    f, outs, states, at = (lambda t: t.double()), [], [], 0
+    rate, cw = torch.exp(f(w["a_log"])), f(w["conv_w"])
+    for s, (n, p0) in enumerate(zip(lengths, pos0)):
+        raw = torch.cat([f(x[k][at:at + n]) for k in ("x", "b", "c")], 1)
+        before = torch.stack([f(conv[s, (p0 - lag) % taps]) if p0 - lag >= 0 else torch.zeros_like(raw[0]) for lag in range(taps - 1, 0, -1)])
+        seq = torch.cat([before, raw])
+        z = f(w["conv_b"]) + sum(seq[t:t + n] * cw[:, t] for t in range(taps))
+        z = z * torch.sigmoid(z)
+        xs, b, c = z[:, :H * vdim].view(n, H, vdim), *(z[:, H * vdim + i * G * dim:][:, :G * dim].view(n, G, dim).repeat_interleave(H // G, 1) for i in (0, 1))
+        step = torch.nn.functional.softplus(f(x["dt"][at:at + n]) + f(w["dt_bias"]), threshold=1e9)
+        S, o = f(state[s]).clone() if p0 else torch.zeros_like(f(state[s])), torch.empty(n, H, vdim, device=DEV, dtype=torch.float64)
+        decay = torch.exp(-rate * step)
+        for t in range(n):
+            S = decay[t, :, None, None] * S + (step[t, :, None] * b[t])[:, :, None] * xs[t][:, None, :]
+            o[t] = torch.einsum("hkv,hk->hv", S, c[t])
+        g = f(x["gate"][at:at + n])
+        y = (o + f(w["skip"])[:, None] * xs).reshape(n, -1) * g * torch.sigmoid(g)
+        y = y.view(n, w["norm_groups"], -1)
+        outs.append((y / torch.sqrt(y.square().mean(-1, keepdim=True) + w["norm_eps"])).reshape(n, -1) * f(w["norm"]))
+        states.append(S)
+        at += n
+    return torch.cat(outs), torch.stack(states)
 
 
-@pytest.mark.parametrize("H,G,dim,vdim", [(8, 1, 128, 64), (6, 2, 96, 40), (5, 5, 16, 64), (24, 2, 64, 132), (4, 1, 128, 32), (22, 2, 20, 68)])
+def _close(a, b, bound=BOUND):
+    assert a.shape == b.shape and float((a.double() - b.double()).norm()) <= bound * float(b.double().norm())
+
+
+def _forms(call):
+    """(the call's result, which forms' kernels it launched)"""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        out = call()
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in prof.key_averages())
+    return out, [n for n in ("la_outputs_tc_kernel", "la_outputs_kernel") if n in names]
+
+
+@pytest.mark.parametrize("H,G,dim,vdim", [(8, 1, 128, 64), (6, 2, 96, 40), (5, 5, 16, 64), (14, 2, 64, 132), (4, 1, 128, 32), (22, 2, 20, 68)])
 @pytest.mark.parametrize("lengths,pos0", [([129], [0]), ([1, 127, 128, 129, 300], [7, 0, 3, 0, 1]), ([256, 5, 640], [0, 2, 9])])
 def test_chunks_of_128_tokens(H, G, dim, vdim, lengths, pos0):
+    from vyomai_b200._lib import lib
+    assert lib().vy_linear_attn_workspace_floats(sum(lengths), len(lengths), max(lengths), H, dim, vdim) > 0   # 0: the walk alone, in either call
     args = _inputs(lengths, H, G, dim, vdim, H + dim)
-    a, b = (_run(lengths, pos0, *args, off) for off in (False, True))
-    _close(a[0], b[0])
-    _close(a[1], b[1])
+    (a, ka), (b, kb) = (_forms(lambda: _run(lengths, pos0, *args, off)) for off in (False, True))
+    assert ka == ["la_outputs_tc_kernel"] and kb == ["la_outputs_kernel"]
+    want = _walk(lengths, pos0, *args)
+    for got, other, exact in zip(a, b, want):
+        _close(got, other)
+        _close(got, exact, 2 * BOUND)
 
 
 @pytest.mark.parametrize("what", ["steep decays", "flat decays", "wide rows", "infinite value", "infinite gates"])
@@ -67,6 +109,9 @@ def test_chunks_of_128_tokens_at_the_ends_of_their_range(what):
     if what == "infinite gates":
         x["gate"][5, 3], x["gate"][200, 65], x["gate"][7, 9], x["gate"][8, 9], x["gate"][9, 9] = float("inf"), float("-inf"), float("nan"), 200.0, -200.0
     a, b = (_run(lengths, pos0, x, w, conv, state, off) for off in (False, True))
+    if what.endswith("decays"):
+        for got, exact in zip(a, _walk(lengths, pos0, x, w, conv, state)):
+            _close(got, exact, 2 * BOUND)
     for p, q in zip(a, b):
         assert torch.equal(p.isfinite(), q.isfinite())
         _close(p.nan_to_num(0, 0, 0), q.nan_to_num(0, 0, 0))
