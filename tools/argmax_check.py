@@ -1,5 +1,7 @@
-import torch, sys
-sys.path.insert(0, "/root/repo")
+import os, sys
+
+import torch
+sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from vyomai_b200 import ops
 torch.manual_seed(0)
 ok = True

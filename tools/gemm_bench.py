@@ -1,6 +1,6 @@
 """Per-shape timing of vy_gemm on the GEMMs of one captioner training step (development aid).
 
-    python tools/gemm_bench.py [--iters 20] [--json gpurun_out/gemm_bench.json]
+    python tools/gemm_bench.py [--iters 20] [--json gemm_bench.json]
 
 For every (role, M, N, K, operand majors, epilogue) of the bench workload it prints the CUDA-event
 time of vy_gemm, the TFLOP/s, and the same contraction through torch.matmul (cuBLAS, no epilogue)

@@ -1,6 +1,6 @@
 """Sweep kernel flavour x tile width x K split for every GEMM shape of the captioner step (development aid).
 
-    python tools/gemm_sweep.py [--iters 10] [--json gpurun_out/gemm_sweep.json]
+    python tools/gemm_sweep.py [--iters 10] [--json gemm_sweep.json]
 
 Uses the vy_gemm_tune_override hook to pin (single CTA | CTA pair, BN, splits) in-process, times each with CUDA events
 over L2-exceeding buffer rotations, and prints per shape the automatic choice next to the best measured one — the data

@@ -450,8 +450,7 @@ def main():
         except subprocess.TimeoutExpired:
             results[n] = "timeout"
             print(f"GROUP {n}: TIMEOUT", flush=True)
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(results, open("gpurun_out/selftest.json", "w"), indent=1)
+    json.dump(results, open("selftest.json", "w"), indent=1)
     print("SUMMARY", json.dumps(results))
     sys.exit(0 if all(v == 0 for v in results.values()) else 1)
 

@@ -57,8 +57,8 @@ def fmt(uv):
 def main():
     dst, reps = sys.argv[1], sys.argv[2:]
     lines = ["# ncu --set full summaries", "",
-             "Captured under gpurun with `--clock-control none`; durations are cold-cache, serialised "
-             "(never bench values). Raw reports stay in gpurun_out/ (scratch).", ""]
+             "Captured with `--clock-control none`; durations are cold-cache, serialised "
+             "(never bench values).", ""]
     for rep in reps:
         for k in load(rep):
             name = k.get("Kernel Name", ("", "?"))[1]

@@ -3,7 +3,7 @@
 nn.Linear / F.scaled_dot_product_attention / nn.LayerNorm in eager PyTorch, bf16 autocast, torch.optim.AdamW(fused) +
 clip_grad_norm_(1.0), the notebook's shifted cross-entropy — next to this repo's Trainer on the same batch.
 
-    python tools/ref_gpu_bench.py [--steps 20] [--dropout 0.0]      -> one JSON line (gpurun_out/ref_gpu_bench.json)
+    python tools/ref_gpu_bench.py [--steps 20] [--dropout 0.0]      -> one JSON line (and ref_gpu_bench_p<dropout>.json)
 """
 import argparse
 import io
@@ -105,8 +105,7 @@ def main():
             "reference_gpu": ref, "ours": ours,
             "speedup_vs_reference_gpu": None if ref is None else ref["ms_per_step"] / ours["ms_per_step"]}
     print(json.dumps(line))
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    json.dump(line, open(os.path.join(ROOT, "gpurun_out", f"ref_gpu_bench_p{args.dropout}.json"), "w"), indent=1)
+    json.dump(line, open(os.path.join(os.getcwd(), f"ref_gpu_bench_p{args.dropout}.json"), "w"), indent=1)
 
 
 if __name__ == "__main__":

@@ -1,5 +1,5 @@
 """Summarise an ncu `--metrics gpu__time_duration.sum --csv` launch list: per kernel name launches, total / mean
-device time and share. Usage: python tools/summarize_launches.py gpurun_out/launches.csv [out.md]"""
+device time and share. Usage: python tools/summarize_launches.py launches.csv [out.md]"""
 import csv
 import re
 import sys

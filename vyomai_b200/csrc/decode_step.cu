@@ -99,7 +99,7 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {  // weights / cache
   return v;
 }
 // DRAM -> L2 prefetch. Measured on this part: one dependent round of loads costs ~0.5 us when it hits L2 and 2-2.5 us from
-// DRAM at this working set (tools/microbench/lat_micro.cu) — five stages of two or three dependent rounds per layer is what
+// DRAM at this working set — five stages of two or three dependent rounds per layer is what
 // made the per-op decode step ten times slower than its byte count. Weights and cached keys / values do not depend on the
 // step's activations, so every CTA asks L2 for its share of the NEXT layer's bytes a whole layer ahead, one
 // `prefetch.global.L2` per 128-byte line spread over all threads of the grid (through the load / store unit: bulk prefetches

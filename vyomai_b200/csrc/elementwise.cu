@@ -486,7 +486,7 @@ xent_colsum_kernel(int rows, int V, __nv_bfloat16* logits, long long ld, const l
   int r = blockIdx.x;
   // Rows are asked into L2 two iterations ahead (one 128-byte line per thread, no register and no scoreboard involved), so
   // the register loads of the next row, issued in two batches inside the last pass, find them there (~0.5 us instead of a
-  // 2 us DRAM round, measured in tools/microbench) and anything that has to wait behind them waits that long at most.
+  // 2 us DRAM round, as measured) and anything that has to wait behind them waits that long at most.
   auto ask_l2 = [&](int rr) {
     if (rr < rows) {
       const char* b = reinterpret_cast<const char*>(logits + static_cast<long long>(rr) * ld);
