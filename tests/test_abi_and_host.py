@@ -376,3 +376,30 @@ def test_bench_kernel_families_map_kernel_names_to_their_entry_points():
     assert f("vy::dp_barrier_kernel(...)").startswith("vy_dp_barrier") and f("vy::dp_reduce_kernel(...)") == "vy_dp_reduce_shard"
     assert f("void vy::gemm_kernel<__nv_bfloat16, 256, true, true, true, false>(...)") == "vy_gemm"
     assert f("at::native::vectorized_elementwise_kernel<4, ...>") == "torch_glue"
+
+
+def test_tilings_are_heard_by_the_thread_that_collects_them():
+    """gemm_tune.collecting: nested, per thread, and nothing is left behind (a product looks only whether anybody listens at all)."""
+    import threading
+    from vyomai_b200 import gemm_tune
+    other = []
+
+    def elsewhere():
+        gemm_tune.heard(True, {"hint_bn": 64})
+        with gemm_tune.collecting() as got:
+            gemm_tune.heard(False, {})
+        other.extend(got)
+
+    with gemm_tune.collecting() as outer:
+        gemm_tune.heard(True, {"hint_flavour": 2, "hint_bn": 256, "hint_splits": 3})
+        t = threading.Thread(target=elsewhere)
+        t.start()
+        t.join()
+        try:
+            with gemm_tune.collecting() as inner:
+                gemm_tune.heard(True, {})
+                raise ValueError
+        except ValueError:
+            pass
+        gemm_tune.heard(True, {"hint_bn": 32})
+    assert outer == [2 | 256 << 4 | 3 << 16, 32 << 4] and inner == [0] and other == [None] and not gemm_tune.LISTENERS

@@ -49,29 +49,29 @@ def keep_plan(key: tuple, block: bytes) -> None:
 
 # the tilings of whole sublayers (block.py): by everything that the hints of their products depend on, the products' hints in the order they are made in, packed
 LAYERS: Dict[tuple, tuple] = {}
-_LISTENING = threading.local()
+LISTENERS: Dict[int, list] = {}   # by thread; empty but for a sublayer's launch-by-launch calls, so that a product asks no more than that
 
 
 class collecting:
     """While it is open, the products of this thread leave their hints in the list it gives (None for one that is not settled yet)."""
 
     def __enter__(self) -> list:
-        self.before = getattr(_LISTENING, "got", None)
-        _LISTENING.got = got = []
+        self.thread = threading.get_ident()
+        self.before = LISTENERS.get(self.thread)
+        LISTENERS[self.thread] = got = []
         return got
 
     def __exit__(self, *exc):
-        _LISTENING.got = self.before
+        if self.before is None:
+            del LISTENERS[self.thread]
+        else:
+            LISTENERS[self.thread] = self.before
 
 
 def heard(settled_: bool, hint: Dict[str, int]) -> None:
-    got = getattr(_LISTENING, "got", None)
+    got = LISTENERS.get(threading.get_ident())
     if got is not None:
         got.append((hint.get("hint_flavour", 0) | hint.get("hint_bn", 0) << 4 | hint.get("hint_splits", 0) << 16) if settled_ else None)
-
-
-def listening() -> bool:
-    return getattr(_LISTENING, "got", None) is not None
 
 
 def keep_layer(key: tuple, got: list, products: int) -> None:

@@ -164,7 +164,7 @@ def gemm(
                 st.aux = aux.data_ptr()
             if allow_split_k:
                 st.workspace = _splitk_workspace(a.device).data_ptr()
-            if gemm_tune.listening():
+            if gemm_tune.LISTENERS:
                 gemm_tune.heard(True, {n: getattr(st, n) for n in ("hint_flavour", "hint_bn", "hint_splits")})
             _lib.run("vy_gemm", st)
             return out
@@ -225,7 +225,8 @@ def gemm(
         saves_aux = aux is not None and act in ("gelu", "gelu_tanh", "swiglu", "geglu_tanh")
         kw.update(gemm_tune.hints(key, kw, [("out", out), ("aux", aux if saves_aux else None)], a.device))
         settled = gemm_tune.settled(key)
-    gemm_tune.heard(settled, kw)
+    if gemm_tune.LISTENERS:
+        gemm_tune.heard(settled, kw)
     _lib.call("vy_gemm", "VyGemm", **kw)
     if plan_key is not None and settled:
         gemm_tune.keep_plan(plan_key, bytes(_lib.fill("VyGemm", kw)))
@@ -292,7 +293,8 @@ def qkv_rope_gemm(
                tokens_per_seq, q_out.dtype, k_out.dtype)
         written = ([("q_out", q_out)] if n_q_heads > 0 else []) + ([("k_out", k_out), ("v_out", v_out)] if n_kv_heads > 0 else [])
         kw.update(gemm_tune.hints(key, kw, written, x.device))
-    gemm_tune.heard(not gemm_tune.ENABLED or gemm_tune.settled(key), kw)
+    if gemm_tune.LISTENERS:
+        gemm_tune.heard(not gemm_tune.ENABLED or gemm_tune.settled(key), kw)
     _lib.call("vy_gemm", "VyGemm", **kw)
 
 
