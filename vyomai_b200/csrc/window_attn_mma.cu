@@ -37,9 +37,12 @@ __global__ void __launch_bounds__(WS_T) window_attn_split_kernel(WinDev d, Split
   const int r0 = blockIdx.x * SPLIT_ROWS, sg = s * d.kv_heads + g;
   if (blockIdx.x == 0 && threadIdx.x == 0) w.odd[sg] = 0;
   // zeros behind the list, units too (rows the last tile's box takes in must not hold what their bits happen to say)
-  for (int r = max(r0, count); w.tail > 0 && r < min(r0 + SPLIT_ROWS, count + w.tail) && slot0 + r < (static_cast<long long>(s) * d.kv_heads + g + 1) * w.cap; ++r) {
-    for (int x = threadIdx.x; x < w.row_bytes / 16; x += WS_T) *reinterpret_cast<uint4*>(w.rows + (slot0 + r) * w.row_bytes + 16 * x) = make_uint4(0, 0, 0, 0);
-    if (threadIdx.x < 2) w.unit[(slot0 + r) * w.ustep + threadIdx.x] = 0.f;
+  // all the CTA's at once (a row after the other cost 32 single tokens beside a prompt 20 of 39 us)
+  const int z0 = max(r0, count), zeros = min(min(r0 + SPLIT_ROWS, count + w.tail), static_cast<int>(w.cap)) - z0;
+  if (w.tail > 0 && zeros > 0) {
+    uint4* at = reinterpret_cast<uint4*>(w.rows + (slot0 + z0) * w.row_bytes);
+    for (int x = threadIdx.x; x < zeros * (w.row_bytes / 16); x += WS_T) at[x] = make_uint4(0, 0, 0, 0);
+    for (int x = threadIdx.x; x < zeros * 2; x += WS_T) w.unit[(slot0 + z0) * w.ustep + x] = 0.f;   // ustep is 2 with a tail
   }
   if (r0 >= count) return;
   __shared__ unsigned top_k, top_v, low_v;   // positive numbers order like their bits (and NaN after infinity)
