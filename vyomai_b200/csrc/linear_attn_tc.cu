@@ -192,11 +192,16 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
       if (c == 0 && d.pos0[s] > 0) {   // the state that is carried in: a thread reads every fourth entry of a column
         const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 + (t & 63);
         unsigned top = 0u;
-#pragma unroll 4
-        for (int i = t >> 6; i < d.dim; i += 4) {
-          const unsigned a = (t & 63) < vw ? abs_bits(sp[static_cast<long long>(i) * d.vdim]) : 0u, large = __reduce_max_sync(0xffffffffu, a);
-          top = max(top, a);
-          note(rs, large, true);
+#pragma unroll 1
+        for (int i0 = t >> 6; i0 < d.dim; i0 += 64) {   // sixteen rows in flight: four at a time took 15 us a head
+          unsigned a[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) a[k] = (t & 63) < vw && i0 + 4 * k < d.dim ? abs_bits(sp[static_cast<long long>(i0 + 4 * k) * d.vdim]) : 0u;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            top = max(top, a[k]);
+            note(rs, __reduce_max_sync(0xffffffffu, a[k]), true);   // a row past the last one notes nothing
+          }
         }
         note(rs, top, true);
       }
