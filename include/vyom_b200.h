@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define VY_ABI_VERSION 15
+#define VY_ABI_VERSION 16
 
 #if defined(__GNUC__)
 #define VY_API __attribute__((visibility("default")))
@@ -803,6 +803,7 @@ typedef struct VyWinAttn {
    * or null): s <- s - head_slope[h] * (i - j), the distance between query and key. The sink gets neither. */
   float softcap;
   const float* head_slope;
+  int64_t rows; /* packed rows of the step, by which the form is chosen where portions are uneven; 0: n_seqs * max_new */
 } VyWinAttn;
 VY_API int64_t vy_window_attn_workspace_floats(int32_t n_seqs, int32_t heads, int32_t kv_heads, int32_t vdim);
 VY_API int64_t vy_window_attn_prompt_floats(int32_t n_seqs, int32_t max_new, int32_t table_width, int32_t block_size, int32_t kv_heads, int32_t dim, int32_t vdim,
@@ -824,6 +825,7 @@ typedef struct VyCausalConv {
   int32_t act;
   void* out; int64_t ld_out; int32_t out_dtype;
   void* stream;
+  int64_t rows; /* packed rows of the step, by which the form is chosen where portions are uneven; 0: n_seqs * max_new */
 } VyCausalConv;
 VY_API int vy_causal_conv(const VyCausalConv* p);
 
@@ -1145,6 +1147,7 @@ typedef struct VyRopeKvWrite {
   void* k_out; int64_t ld_k_out;
   const void* q_norm; const void* k_norm; int32_t norm_dtype;
   float q_temp; int32_t q_temp_every;
+  int64_t rows; /* as in VyCausalConv */
 } VyRopeKvWrite;
 VY_API int vy_rope_kv_write(const VyRopeKvWrite* p);
 

@@ -592,8 +592,11 @@ extern "C" int vy_rope_kv_write(const VyRopeKvWrite* p) {
     // prompts 0.23 -> 0.34 ms over 4 launches of 8192 tokens and saved single-token steps 29 -> 21 us)
     const int units = p->heads + p->kv_heads;
     const auto quads = [](const void* t, long long ld) { return t == nullptr || (reinterpret_cast<uintptr_t>(t) % 16 == 0 && ld % 4 == 0); };
-    // rows of four: in a half layout the halves are whole lanes. From some hundred tokens on: few tokens' heads go to several warps each above (80 tokens 5.8 / 6.8 us)
-    const bool rows = p->max_new >= 16 && static_cast<long long>(p->n_seqs) * p->max_new >= 512 && (p->max_new + 7) / 8 <= 65535 * 1024 && d.in_dt == VY_F32 && d.dim <= 128 && d.dim % 4 == 0 && (!g.half_layout || d.rot_dims % 8 == 0) &&
+    // rows of four: in a half layout the halves are whole lanes. From 1200 tokens on, below which a warp per token leaves schedulers without one: 8 + 2 heads of 128 over 512, 1200, 2048
+    // tokens 8.3 / 8.8, 13.7 / 9.5, 16.2 / 9.7 us (a CTA / a warp per token), 32 + 8 of 64 17.1 / 22.9, 31.7 / 25.0, 38.8 / 25.6; or where portions are so uneven that the other form's CTAs
+    // without a token bound it: one of 512 beside 31 single tokens 22.3 / 9.8, 29.8 / 24.7
+    const long long most = static_cast<long long>(p->n_seqs) * p->max_new, tokens = p->rows > 0 ? p->rows : most;
+    const bool rows = p->max_new >= 16 && (tokens >= 1200 || most >= 12288) && (p->max_new + 7) / 8 <= 65535 * 1024 && d.in_dt == VY_F32 && d.dim <= 128 && d.dim % 4 == 0 && (!g.half_layout || d.rot_dims % 8 == 0) &&
                       (d.heads == 0 || quads(d.q, d.ldq)) && (d.kv_heads == 0 || (quads(d.k, d.ldk) && (paged || quads(g.k_out, g.ld_k_out)))) &&
                       (!paged || (quads(d.v, d.ldv) && d.vdim % 4 == 0 && (d.pool_dt != VY_F32 || (quads(d.kp, 0) && quads(d.vp, 0)))));
     if (rows) {

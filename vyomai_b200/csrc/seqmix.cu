@@ -1017,6 +1017,8 @@ extern "C" int vy_window_attn(const VyWinAttn* p) {
   d.softcap = p->softcap; d.head_slope = p->head_slope;
   d.gate = p->gate; d.ld_gate = p->ld_gate; d.gate_dt = p->gate_dtype;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
+  const long long most = static_cast<long long>(p->n_seqs) * p->max_new;
+  d.rows = p->rows > 0 && p->rows < most ? p->rows : most;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   VY_CHECK_ARG(p->dim <= 32 * WA_VR, "vy_window_attn: dim %d > %d", p->dim, 32 * WA_VR);
   if (p->max_new >= WA_TILED_MIN) {   // prompt-sized: tensor-core tiles
@@ -1078,8 +1080,11 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   const auto quads = [](const void* q, int dt, long long ld) { return dt == VY_F32 && reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0; };
-  // from a CTA per SM on: 80 tokens x 512 channels are 7.2 us with a channel per thread, 8.2 with four
-  if (static_cast<long long>(p->n_seqs) * ((p->max_new + CONV_TOK - 1) / CONV_TOK) * ((p->channels + 511) / 512) >= num_sms() && p->taps <= 4 && p->channels % 4 == 0 &&
+  // Four channels per thread from two CTAs per SM on that find tokens: 1024 channels x 1200, 2080, 4160 tokens 8.9 / 10.1, 12.3 / 11.7, 19.7 / 13.9 us (a channel per thread / four);
+  // 3000 x 512, 768 9.6 / 10.7, 11.9 / 10.9; or from ten on that find some or none, which in either form bound uneven portions: one of 300 beside 7 of 20, 1024 channels, 8.2 / 10.3,
+  // one of 512 beside 31 single tokens 11.3 / 9.7 (of which 256 channels 7.8 / 9.5)
+  const long long tiles = static_cast<long long>(p->n_seqs) * ((p->max_new + CONV_TOK - 1) / CONV_TOK), filled = p->rows > 0 ? (p->rows + CONV_TOK - 1) / CONV_TOK : tiles;
+  if ((filled * p->channels >= 2LL * 512 * num_sms() || tiles * p->channels >= 10LL * 512 * num_sms()) && p->taps <= 4 && p->channels % 4 == 0 &&
       p->channels <= 65535 * 512 && quads(d.x, d.x_dt, d.ldx) && quads(d.out, d.out_dt, d.ld_out)) {
     d.first = 0;
     const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, (p->channels + 511) / 512, p->n_seqs);

@@ -136,6 +136,7 @@ struct WinDev {
   int sigmoid;   // the weight of a visible key is sigmoid(score), not normalised over the keys
   const float* head_scale; const float* head_bias;   // score = (q . k) * scale * head_scale[h] + head_bias[h]; null: 1 / 0
   float softcap; const float* head_slope;   // then: cap tanh(score / cap) (cap > 0), minus head_slope[h] * distance (null: 0)
+  long long rows;   // packed rows of the step (host: which prompt form)
 };
 
 __device__ __forceinline__ float head_scale_of(const WinDev& d, int h) { return d.head_scale ? d.scale * d.head_scale[h] : d.scale; }

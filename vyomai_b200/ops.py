@@ -1184,7 +1184,7 @@ def window_attn(batch: PackedBatch, q: torch.Tensor, k_pool: torch.Tensor, v_poo
               gate=_ptr(gate), ld_gate=gate.stride(0) if gate is not None else 0, gate_dtype=_dt(gate) if gate is not None else 0,
               out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out), k_row=int(k_row), v_row=int(v_row), stream=_stream(), chunk=int(chunk), out_scale=float(out_scale),
               weight_kind=ATTN_WEIGHTS[weights], head_scale=_ptr(head_scale), head_bias=_ptr(head_bias), softcap=float(softcap), head_slope=_ptr(head_slope),
-              **batch._kw(pages=True, slots=False))
+              rows=q.shape[0], **batch._kw(pages=True, slots=False))
     return out
 
 
@@ -1354,7 +1354,7 @@ def rope_kv_write(batch: PackedBatch, q: Optional[torch.Tensor], k: Optional[tor
               half_layout=1 if layout == "half" else 0, unit_rms=1 if unit_rms else 0, eps=float(eps), rot_scale=float(rot_scale), q_scale=float(q_scale),
               k_scale=float(k_scale), k_out=_ptr(k_out), ld_k_out=k_out.stride(0) if k_out is not None else 0,
               q_norm=_ptr(q_norm), k_norm=_ptr(k_norm), norm_dtype=_dt(nw) if nw is not None else 0,
-              q_temp=float(q_temp[0]) if q_temp is not None else 0.0, q_temp_every=int(q_temp[1]) if q_temp is not None else 0,
+              q_temp=float(q_temp[0]) if q_temp is not None else 0.0, q_temp_every=int(q_temp[1]) if q_temp is not None else 0, rows=ins[0].shape[0],
               **batch._kw(pages=paged, slots=False))
 
 
@@ -1457,7 +1457,7 @@ def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: tor
     out = torch.empty((x.shape[0], ch), device=x.device, dtype=out_dtype or x.dtype)
     _lib.call("vy_causal_conv", "VyCausalConv", channels=ch, taps=taps, x=x.data_ptr(), ldx=x.stride(0), x_dtype=_dt(x), w=w.data_ptr(),
               w_dtype=_dt(w), state=state.data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
-              stream=_stream(), **batch._kw())
+              stream=_stream(), rows=x.shape[0], **batch._kw())
     return out
 
 
