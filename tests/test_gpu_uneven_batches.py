@@ -34,6 +34,26 @@ def _close(a, b):
     assert a.shape == b.shape and float((a.double() - b.double()).norm()) <= BOUND * float(b.double().norm())
 
 
+@pytest.mark.parametrize("H,G,d,dv,window,tokens,alone,beside", [(16, 16, 96, 64, 64, 512, "tc", "mma"), (8, 2, 128, 128, 512, 2048, "tc", "tc"), (32, 8, 64, 64, 64, 512, "tc", "mma")])
+def test_prompt_attention_beside_single_tokens(H, G, d, dv, window, tokens, alone, beside):
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(d)
+    new, pos0 = [tokens] + [1] * 31, [0] + [700] * 31
+    batch, pages = _batch(new, pos0)
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    q, kp, vp = R(sum(new), H * d), R(pages, 16, G, d), R(pages, 16, G, dv)
+    call = lambda b, q: ops.window_attn(b, q, kp, vp, heads=H, kv_heads=G, dim=d, vdim=dv, scale=d ** -0.5, window=window, keep_first=0, out_dtype=torch.float32)  # noqa: E731
+    both, names = _kernels(lambda: call(batch, q))
+    assert f"window_attn_{beside}_kernel" in names
+    one, _ = _batch(new[:1], pos0[:1])
+    first, names = _kernels(lambda: call(one, q[:tokens]))
+    assert f"window_attn_{alone}_kernel" in names
+    _close(both[:tokens], first)
+    for s in (1, 31):   # a token by itself has its pages elsewhere in the table
+        b1 = ops.PackedBatch(_i32([0, 1]), _i32([700]), _i32([0]), 1, batch.block_table[s:s + 1].contiguous(), 16)
+        _close(both[tokens + s - 1:tokens + s], call(b1, q[tokens + s - 1:tokens + s]))
+
+
 @pytest.mark.parametrize("new,channels,conv,heads,rope", [([300] + [20] * 7, 1024, "causal_conv_kernel", 32, "rope_heads_kernel"), ([512] + [1] * 31, 4096, "causal_conv_quads_kernel", 8, "rope_heads_rows_kernel"),
                                                           ([700, 600], 2048, "causal_conv_quads_kernel", 8, "rope_heads_rows_kernel"), ([700, 400], 1024, "causal_conv_kernel", 8, "rope_heads_kernel")])
 def test_row_kernels_choose_by_the_tokens_that_are_there(new, channels, conv, heads, rope):

@@ -555,6 +555,28 @@ static bool tc_registers() {
   return enough;
 }
 
+// Is this form faster than window_attn_mma.cu's? Microseconds of either, from the CTAs that find rows and those that find none (the grid has the longest portion's for every
+// sequence) and the keys a block of rows sees. Here a CTA has an SM to itself, its fixed time is that of some ten tiles, and a CTA without rows waits for a whole SM too: a prompt
+// beside many single tokens is as slow as its rounds of CTAs. Fitted to batches of 2 to 32 heads of 16 to 128 channels with both forms timed; of 1353 it takes the one slower by more
+// than 4 % in 11 (by 27 % at most). mma.sync / tcgen05, us, splitting included: 4 x 2048 tokens, 16 heads of 96 / 64, whole context 580 / 216; 16 portions of 130, 8 heads of 128 over 2, window 64 28 / 35
+// (160 CTAs: two rounds); one of 512 beside 31 single tokens, window 64, 16 heads of 96 / 64 51 / 85, 12 of 64 39 / 61, window 512, 8 of 128 over 2 78 / 55
+static bool tc_pays(const WinDev& d, int n_seqs, int max_new, int hl) {
+  const double sms = num_sms(), channels = (round_to(d.dim, 16) + round_to(d.vdim, 16)) / 128.0;
+  const long long all = static_cast<long long>(d.tw) * d.bs, blocks_of_heads = d.heads >> hl;
+  const long long band = d.chunk > 0 ? d.chunk : static_cast<long long>(d.window) + d.keep, seen = band + (TC_ROWS >> hl);
+  const double tiles = (d.chunk > 0 || d.window > 0 ? static_cast<double>(seen < all ? seen : all) : 0.6 * all) / TC_KEYS;
+  const auto ctas = [&](int qn, double& idle) {   // that find rows, at most
+    const long long grid = static_cast<long long>(n_seqs) * ((max_new + qn - 1) / qn), most = d.rows / qn + n_seqs, live = grid < most ? grid : most;
+    idle = static_cast<double>(blocks_of_heads * (grid - live));
+    return static_cast<double>(blocks_of_heads * live);
+  };
+  double idle_tc, idle_mma;
+  const double live_tc = ctas(TC_ROWS >> hl, idle_tc), live_mma = ctas(64 >> hl, idle_mma), rounds = ceil(live_tc / sms) + (idle_tc > sms ? 0.4 : 0.0);
+  const double tc = rounds * (d.vdim > 64 ? 13.0 : 10.5) + rounds * (0.1 + 0.15 * channels) * tiles + 0.75 * idle_tc / sms;
+  const double mma = fmax(1.0, live_mma / (2.0 * sms)) * (13.0 + (0.5 + 3.0 * channels) * tiles) + 0.1 * idle_mma / (2.0 * sms);
+  return tc <= mma;
+}
+
 bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new) {
   if (d.dim > 128 || d.vdim > 128) return false;
   if (!(d.vdim > 64 ? (d.sigmoid ? tc_registers<128, true>() : tc_registers<128, false>()) : d.sigmoid ? tc_registers<64, true>() : tc_registers<64, false>())) return false;
@@ -567,7 +589,7 @@ bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new) {
   // Splitting and attention, mma.sync / tcgen05, four portions of n tokens from position 0, 8 heads of 128 over 2: n = 64 20.8 / 23.9 us, 128 24.6 / 24.3,
   // 300 41.4 / 28.7; 16 heads of 96 / 64 with keys of their own: 128 22.4 / 23.3, 200 31.7 / 26.9, 1000 201 / 104. Portions of 32 tokens on 2000 cached
   // ones, 8 heads over 2, window 512: 62 / 39
-  return split_slots(d, max_new) >= (hl > 0 ? 128 : 192);
+  return split_slots(d, max_new) >= (hl > 0 ? 128 : 192) && tc_pays(d, n_seqs, max_new, hl);
 }
 
 template <int VD, bool SIG>
