@@ -80,3 +80,34 @@ def test_row_kernels_choose_by_the_tokens_that_are_there(new, channels, conv, he
     _close(q[:m], q1)
     _close(kp[:rows], kp1[:rows])
     assert torch.equal(vp[:rows], vp1[:rows])
+
+
+@pytest.mark.parametrize("H,G,beside", [(16, 16, "la_outputs_kernel"), (8, 1, "la_outputs_tc_kernel")])
+def test_state_space_beside_single_tokens(H, G, beside):
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(H)
+    new, pos0, dim, vdim = [512] + [1] * 31, [0] + [7] * 31, 64, 64
+    T, n, C, inner = sum(new), len(new), H * vdim + 2 * G * dim, H * vdim
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    x = dict(x=R(T, inner), b=R(T, G * dim), c=R(T, G * dim), dt=R(T, H), gate=R(T, inner))
+    w = dict(conv_w=R(C, 4) * 0.5, conv_b=R(C), dt_bias=R(H) - 1, a_log=R(H) * 0.3, skip=R(H), norm=torch.ones(inner, device=DEV), heads=H, groups=G, dim=dim, vdim=vdim, taps=4, norm_groups=1,
+             norm_eps=1e-6, out_dtype=torch.float32)
+    conv, state = R(n, 4, C), R(n, H, dim, vdim)
+
+    def run(lo, hi, a, b):
+        cu = [0]
+        for m in new[lo:hi]:
+            cu.append(cu[-1] + m)
+        cs, ss = conv[lo:hi].clone(), state[lo:hi].clone()
+        out = ops.ssd(ops.PackedBatch(_i32(cu), _i32(pos0[lo:hi]), _i32(list(range(hi - lo))), max(new[lo:hi])), **{k: t[a:b] for k, t in x.items()}, **w, conv_state=cs, state=ss,
+                      tickets=torch.zeros(hi - lo, 1, dtype=torch.int32, device=DEV))
+        return out, ss
+
+    (out, states), names = _kernels(lambda: run(0, n, 0, T))
+    assert beside in names
+    first, s0 = run(0, 1, 0, 512)
+    _close(out[:512], first)
+    _close(states[:1], s0)
+    last, s1 = run(n - 1, n, T - 1, T)
+    _close(out[-1:], last)
+    _close(states[-1:], s1)

@@ -103,8 +103,7 @@ __device__ __forceinline__ float4 column_scales(uint4 m) {
 
 // linear_attn_tc.cu: states and read-outs of chunks of LT_C tokens (state space, fp32 rows in quads), at most LT_HEADS heads per CTA
 constexpr int LT_HEADS = 8;
-bool linear_attn_tc_applies(const RecDev& d);
-int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long rows, int vslices);   // heads per CTA
+int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long rows, int vslices);   // heads per CTA; 0: not for this step
 cudaError_t launch_la_states_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st);
 cudaError_t launch_la_outputs_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st);
 

@@ -547,12 +547,13 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   w.top = reinterpret_cast<unsigned*>(w.D + slots * d.heads);
   w.odd = reinterpret_cast<int*>(w.top + slots * d.heads);
   const bool quad = d.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(d.state) % 16 == 0 && reinterpret_cast<uintptr_t>(ws) % 16 == 0;
-  const bool tc = TD && vec && quad && linear_attn_tc_applies(d);
+  const int vslices = (d.vdim + 63) / 64, tc_hp = TD && vec && quad ? linear_attn_tc_heads(d, n_seqs, max_new, rows, vslices) : 0;
+  const bool tc = tc_hp > 0;
   const int C = w.chunk = tc ? LT_C : LM_C;
-  const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, vslices = (d.vdim + 63) / 64, chunks = (max_new + C - 1) / C;
+  const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, chunks = (max_new + C - 1) / C;
   // heads per CTA: those that share q and k, fewer while that leaves less than two CTAs per SM
   int hp = TD ? d.heads / d.kv_heads : 1;
-  if (tc) hp = linear_attn_tc_heads(d, n_seqs, max_new, rows, vslices);
+  if (tc) hp = tc_hp;
   else
     while (hp % 2 == 0 && slots * vslices * (d.heads / hp) < 2LL * num_sms()) hp /= 2;
   const dim3 grid(static_cast<unsigned>(chunks) * vslices, d.heads / hp, n_seqs);

@@ -775,7 +775,7 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
 // In place of the 64-token chunks wherever rows come in quads (values and outputs by bulk copies), us of vy_ssd, mma.sync / here, 32 heads of 128 x 64 in groups of 8: one
 // prompt of 200 tokens 63 / 42, 512 69 / 45, 2048 250 / 88, 4096 494 / 142; 16 of 150 453 / 142; 32 heads each with q and k of its own, one of 512 78 / 50, 4096 577 / 320;
 // 24 heads of 64 x 64 over one q and k, 2048 152 / 64; 8 of 128 x 128 in two groups, 2048 135 / 59
-bool linear_attn_tc_applies(const RecDev& d) {
+static bool linear_attn_tc_applies(const RecDev& d) {
   const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
   if (d.dim > 128 || d.vdim < 32 || d.in_act != VY_UACT_NONE) return false;
   // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever: what a compiler gives another number does without this form
@@ -787,8 +787,11 @@ bool linear_attn_tc_applies(const RecDev& d) {
   return d.out_dt == VY_F32 && quads(d.out, d.ld_out) && (!d.gate || quads(d.gate, d.ld_gate));
 }
 
-// A CTA takes about as long before its first head as for two heads (17,000 cycles and 9,500), one CTA per SM at a time
+// A CTA takes about as long before its first head as for two heads (17,000 cycles and 9,500), one CTA per SM at a time. The grid has the longest portion's chunks for every sequence,
+// and a CTA without a chunk waits for a whole SM too: with a head per CTA and more than eight such per SM, chunks of 64 are faster. 16 heads of 64 x 64 with q and k of their own, one prompt
+// beside single tokens, mma.sync / here, us of vy_ssd: 512 beside 31 129 / 145, 2048 beside 31 230 / 265, 1000 beside 15 108 / 115; 200 beside 31 (three per SM) 89 / 73
 int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long rows, int vslices) {
+  if (!linear_attn_tc_applies(d)) return 0;
   const int rep = d.heads / d.kv_heads, sms = num_sms();
   const long long most = static_cast<long long>(n_seqs) * ((max_new + LT_C - 1) / LT_C), chunks = most < rows / LT_C + n_seqs ? most : rows / LT_C + n_seqs;
   int best = 1;
@@ -801,7 +804,7 @@ int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long row
       best = hp;
     }
   }
-  return best;
+  return best == 1 && (most - chunks) * vslices * d.heads > 8LL * sms ? 0 : best;
 }
 
 static bool row_map(CUtensorMap* m, const void* p, long long cols, long long rows, long long ld, int box_rows) {
