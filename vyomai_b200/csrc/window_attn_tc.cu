@@ -558,8 +558,8 @@ static bool tc_registers() {
 // Is this form faster than window_attn_mma.cu's? Microseconds of either, from the CTAs that find rows and those that find none (the grid has the longest portion's for every
 // sequence) and the keys a block of rows sees. Here a CTA has an SM to itself, its fixed time is that of some ten tiles, and a CTA without rows waits for a whole SM too: a prompt
 // beside many single tokens is as slow as its rounds of CTAs. Fitted to batches of 2 to 32 heads of 16 to 128 channels with both forms timed; of 1353 it takes the one slower by more
-// than 4 % in 11 (by 27 % at most). mma.sync / tcgen05, us, splitting included: 4 x 2048 tokens, 16 heads of 96 / 64, whole context 580 / 216; 16 portions of 130, 8 heads of 128 over 2, window 64 28 / 35
-// (160 CTAs: two rounds); one of 512 beside 31 single tokens, window 64, 16 heads of 96 / 64 51 / 85, 12 of 64 39 / 61, window 512, 8 of 128 over 2 78 / 55
+// than 4 % in 11 (by 27 % at most). mma.sync / tcgen05, us, splitting included: 4 x 2048 tokens, 16 heads of 96 / 64, whole context 590 / 231; 16 portions of 130, 8 heads of 128 over 2, window 64 28 / 35
+// (160 CTAs: two rounds); one of 512 beside 31 single tokens, window 64, 16 heads of 96 / 64 51 / 85, 12 of 64 39 / 61, window 512, 8 of 128 over 2 93 / 46
 static bool tc_pays(const WinDev& d, int n_seqs, int max_new, int hl) {
   const double sms = num_sms(), channels = (round_to(d.dim, 16) + round_to(d.vdim, 16)) / 128.0;
   const long long all = static_cast<long long>(d.tw) * d.bs, blocks_of_heads = d.heads >> hl;
@@ -586,9 +586,9 @@ bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new) {
   const long long rows = static_cast<long long>(max_new) << hl;
   if (rows < TC_ROWS || rows / TC_ROWS >= 65535) return false;   // the last: a grid's limit
   // A CTA takes 8 to 11 us before its first tile and after its last; with a tile or two between them the 64-row CTAs of window_attn_mma.cu are as good.
-  // Splitting and attention, mma.sync / tcgen05, four portions of n tokens from position 0, 8 heads of 128 over 2: n = 64 20.8 / 23.9 us, 128 24.6 / 24.3,
-  // 300 41.4 / 28.7; 16 heads of 96 / 64 with keys of their own: 128 22.4 / 23.3, 200 31.7 / 26.9, 1000 201 / 104. Portions of 32 tokens on 2000 cached
-  // ones, 8 heads over 2, window 512: 62 / 39
+  // Splitting and attention, mma.sync / tcgen05, four portions of n tokens from position 0, 8 heads of 128 over 2: n = 128 25.0 / 22.6 us, 300 41.5 / 26.8;
+  // 16 heads of 96 / 64 with keys of their own: 128 22.5 / 22.6, 300 45.5 / 35.3, 1000 200 / 101. Portions of 32 tokens on 2000 cached
+  // ones, 8 heads over 2, window 512: 57 / 31
   return split_slots(d, max_new) >= (hl > 0 ? 128 : 192) && tc_pays(d, n_seqs, max_new, hl);
 }
 
