@@ -25,12 +25,21 @@ def _off(t):
     return v
 
 
+def _ran(call, kernel):
+    """The call's result, made by `kernel`."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        out = call()
+        torch.cuda.synchronize()
+    assert any(kernel in e.key for e in prof.key_averages()), kernel
+    return out
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4])
 @pytest.mark.parametrize("act", ["silu", "sigmoid", None])
 def test_convolution_of_four_channels_per_thread(taps, act):
     from vyomai_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(taps)
-    C, pos0 = 8196, [0, 3, 0, 40, 2]   # enough channels for a CTA per SM
+    C, pos0 = 20004, [0, 3, 0, 40, 2]   # enough channels for two CTAs per SM
     batch = ops.PackedBatch(torch.tensor([0, 1, 16, 32, 49, 119], dtype=torch.int32, device=DEV), torch.tensor(pos0, dtype=torch.int32, device=DEV),
                             torch.tensor([4, 1, 0, 5, 2], dtype=torch.int32, device=DEV), 70)
     x, w, state = torch.randn(119, C, generator=g, device=DEV) * 3, torch.randn(C, taps, generator=g, device=DEV), torch.randn(6, C, max(taps - 1, 1), generator=g, device=DEV)
@@ -38,7 +47,8 @@ def test_convolution_of_four_channels_per_thread(taps, act):
     if taps == 1:
         state = state[:, :, :0].contiguous()
     states = [state.clone(), state.clone()]
-    a, b = (ops.causal_conv(batch, t, w, s, act=act) for t, s in zip((x, _off(x)), states))
+    a = _ran(lambda: ops.causal_conv(batch, x, w, states[0], act=act), "causal_conv_quads_kernel")
+    b = _ran(lambda: ops.causal_conv(batch, _off(x), w, states[1], act=act), "causal_conv_kernel")
     _close(a, b)
     assert torch.equal(*states)
 
@@ -47,11 +57,12 @@ def test_convolution_of_four_channels_per_thread(taps, act):
 def test_convolutions_keep_infinities_to_the_tokens_that_see_them(taps):
     from vyomai_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(taps)
-    C, n = 8192, 160
+    C, n = 16384, 160
     batch = ops.PackedBatch(*(torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, n], [0], [0])), n)
     x, w = torch.randn(n, C, generator=g, device=DEV), torch.randn(C, taps, generator=g, device=DEV)
     x[5, 3], x[33, 3], x[33, 8], x[47, 100], x[159, 7] = float("inf"), float("nan"), float("-inf"), float("inf"), float("inf")
-    a, b = (ops.causal_conv(batch, t, w, torch.zeros(1, C, max(taps - 1, 1), device=DEV)[:, :, :taps - 1].contiguous(), act=None) for t in (x, _off(x)))
+    run = lambda t: ops.causal_conv(batch, t, w, torch.zeros(1, C, max(taps - 1, 1), device=DEV)[:, :, :taps - 1].contiguous(), act=None)  # noqa: E731
+    a, b = _ran(lambda: run(x), "causal_conv_quads_kernel"), _ran(lambda: run(_off(x)), "causal_conv_kernel")
     seen = torch.zeros(n, C, dtype=torch.bool, device=DEV)
     for i, c in (~x.isfinite()).nonzero().tolist():
         seen[i:i + taps, c] = True
@@ -64,9 +75,9 @@ def test_convolutions_keep_infinities_to_the_tokens_that_see_them(taps):
 def test_rotation_of_four_entries_per_lane(layout, rot, dim, norm, pool):
     from vyomai_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(dim + rot)
-    H, G, dv, new, pos0 = 5, 2, 36, [17, 1, 240], [0, 300, 7]
+    H, G, dv, new, pos0 = 5, 2, 36, [170, 1, 1247], [0, 300, 7]
     batch, _, _, blocks, _ = shuffled_batch(new, pos0, 16, DEV, seed=rot)
-    q, k, v = (torch.randn(258, n, generator=g, device=DEV) for n in (H * dim, G * dim, G * dv))
+    q, k, v = (torch.randn(sum(new), n, generator=g, device=DEV) for n in (H * dim, G * dim, G * dv))
     freq = 100.0 ** -(torch.arange(max(rot // 2, 1), device=DEV) / max(rot // 2, 1))
     nw = torch.randn(dim, generator=g, device=DEV) if norm == "weight" else None
 
@@ -77,7 +88,7 @@ def test_rotation_of_four_entries_per_lane(layout, rot, dim, norm, pool):
                           q_scale=0.7, k_scale=1.3, k_out=ko, q_norm=nw, k_norm=nw, q_temp=(0.3, 9) if norm else None)
         return q, (ko if pool is None else kp.float()), (v if pool is None else vp.float())
 
-    a, b = run(q.clone(), k.clone(), v), run(_off(q), _off(k), _off(v))
+    a, b = _ran(lambda: run(q.clone(), k.clone(), v), "rope_heads_rows_kernel"), _ran(lambda: run(_off(q), _off(k), _off(v)), "rope_heads_kernel")
     _close(a[0], b[0])
     if pool == torch.bfloat16:   # one rounding of a key may go the other way
         assert float((a[1] - b[1]).abs().max()) <= 2.0 ** -7 * float(b[1].abs().max())
@@ -107,10 +118,10 @@ def _gate_close(got, want, x, act):
 def test_gates_over_the_whole_range(act):
     from vyomai_b200 import ops
     x, want = _gates()
-    n = 160   # tokens: enough for the form with four channels per thread
+    n = 640   # tokens: enough for the form with four channels per thread
     batch = ops.PackedBatch(*(torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, n], [0], [0])), n)
     xs = x.expand(n, -1).contiguous()
-    got = ops.causal_conv(batch, xs, torch.ones(x.numel(), 1, device=DEV), torch.zeros(1, x.numel(), 0, device=DEV), act=act)
+    got = _ran(lambda: ops.causal_conv(batch, xs, torch.ones(x.numel(), 1, device=DEV), torch.zeros(1, x.numel(), 0, device=DEV), act=act), "causal_conv_quads_kernel")
     for row in (got[0], got[-1]):
         _gate_close(row, want[act], x, act)
     ones = torch.ones(3, x.numel(), device=DEV)
