@@ -65,6 +65,32 @@ def test_delta_rule_sixteen_tokens_at_a_time(monkeypatch, H, G, dk, dv, dtype):
             assert _err(form[s], want[s]) < 4 * BOUND, s   # a recurrence: each of the up to 66 steps carries its rounding on
 
 
+@pytest.mark.parametrize("H,G,dk,dv", [(1, 1, 128, 128), (2, 1, 100, 40), (3, 3, 64, 16), (2, 2, 36, 130), (4, 2, 32, 33), (1, 1, 4, 1)])
+@pytest.mark.parametrize("copies", [1, 40])
+def test_delta_rule_on_aligned_rows(H, G, dk, dv, copies):
+    """Rows that come in quads, few sequences and many (more CTAs than run at once): portions that end on, before and after a chunk's edge, carried on once."""
+    from vyomai_b200 import ops
+    g = torch.Generator().manual_seed(dk + dv)
+    lengths, more = [64, 33, 16, 47], [1, 32, 64, 17]
+    T = [a + b for a, b in zip(lengths, more)]
+    mk = lambda w: [torch.randn(t, w, generator=g) for t in T]  # noqa: E731
+    q, k, v, a, b = mk(G * dk), mk(G * dk), mk(H * dv), mk(H * dk), mk(H)
+    a_log = torch.randn(H, generator=g) - 1.0
+    want = []
+    for s, t in enumerate(T):
+        unit = lambda x: OH.unit(x.double().view(t, G, dk))  # noqa: E731
+        decay = torch.exp(-torch.exp(a_log.double())[None, :, None] * torch.nn.functional.softplus(a[s].double(), threshold=1e9).view(t, H, dk))
+        want.append(OH.gated_delta_rule(unit(q[s]) * dk ** -0.5, unit(k[s]), v[s].double().view(t, H, dv), decay, torch.sigmoid(b[s].double())).reshape(t, -1))
+    n = 4 * copies
+    state, out = torch.full((n, H, dk, dv), float("nan"), device=DEV), []
+    for at, take in (([0] * 4, lengths), (lengths, more)):
+        quads = lambda src: torch.nn.functional.pad(torch.cat([src[s][at[s]:at[s] + take[s]] for s in range(4)] * copies), (0, -src[0].shape[1] % 4)).to(DEV)[:, :src[0].shape[1]]  # noqa: E731
+        batch = ops.PackedBatch(_i32([sum((take * copies)[:i]) for i in range(n + 1)]), _i32(at * copies), _i32(list(range(n))), max(take))
+        out.append(ops.delta_rule(batch, quads(q), quads(k), quads(v), quads(a), quads(b), a_log.to(DEV), state, heads=H, kv_heads=G, dim=dk, vdim=dv, out_dtype=torch.float32).split(take * copies))
+    for i in range(n):
+        assert _err(torch.cat([out[0][i], out[1][i]]), want[i % 4]) < 4 * BOUND, i   # as above
+
+
 def test_delta_rule_keeps_a_bad_value_to_its_column_and_later_tokens():
     from vyomai_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(1)

@@ -4,15 +4,16 @@
 //   u_t + beta_t sum_{s < t} A_ts u_s = beta_t (v_t - S^T (G_t k_t)),      A_ts = k_t . (G_t / G_s k_s)
 //   o_t = S^T (G_t q_t) + sum_{s <= t} B_ts u_s,                           B_ts = q_t . (G_t / G_s k_s)
 //   S <- G_15 S + sum_s (G_15 / G_s k_s) u_s^T
-// The quotients are products of the decays between s and t or exponentials of sums: nothing is divided, no underflow matters. With W the inverse of the
-// triangular 16 x 16 system times diag(beta), u = W v - (W G k) S. Two launches:
-//   delta_chunk_kernel   all chunks in parallel: W, then W v, P = W G k, G q, G_15 / G_s k, B, split into fp16 pairs and stored in the
+// The quotients are products of the decays between s and t or exponentials of sums: nothing is divided, no underflow matters. Solving the triangular 16 x 16 system for
+// the columns of V and of G k at once gives W v and P with u = W v - P S. Two launches:
+//   delta_chunk_kernel   all chunks in parallel: A and B, then W v, P, G q, G_15 / G_s k, split into fp16 pairs and stored in the
 //                        register layout of the second launch's operands
 //   delta_scan_kernel    the walk. It is transposed (S^T: a warp owns 16 value columns and all channels), so that the state in accumulator
 //                        registers is the next product's A operand, the writes likewise, and no warp waits for another one
 // The walk token by token (delta_rule_kernel) is bound by its chain of two reductions per token: 46 + 1013 us with its preparation for 4 x 2048
-// tokens, 8 heads of 128 x 128; here 164 + 236 us. The first launch is bound by instructions (decays, exponentials, sums of pairs of tokens), the
-// second by the latency of one warp's chain, 1.8 us per chunk. Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
+// tokens, 8 heads of 128 x 128; here 120 + 236 us. The first launch is bound by instructions, 85 million of them (decays, exponentials, sums over pairs of tokens; with
+// W made first, a column of it per lane, and channels loaded one by one 126 million, 163 us), the second by the latency of one
+// warp's chain, 1.8 us per chunk. Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 
@@ -21,7 +22,7 @@ namespace {
 
 constexpr int DC_T = 16;            // tokens per chunk
 constexpr int DC_KTOP = 15;         // the decayed unit keys are split in units of 2^-15: their entries are at most 1
-constexpr int DC_NW = 2;            // warps of the walk's CTA: 32 value columns
+constexpr int DC_NW = 2;            // warps of the walk's CTA where each has all channels: 32 value columns
 constexpr int DC_NS = 3;            // chunks in flight per CTA of the walk
 // What the accumulations cut off (split_mma.cuh) is added back: read-outs are off by -5.8e-8 on average without it, -0.4e-8 with it, in the serial walk +0.5e-8
 
@@ -40,14 +41,28 @@ struct DeltaChunks {
 // a sequence's first chunk slot: cu[s] / 16 + s, so that sequences never overlap and rows / 16 + n_seqs slots suffice
 __device__ __forceinline__ long long chunk_slot0(int base, int s) { return base / DC_T + s; }
 
+// log(1 + e^x): with t = e^-|x| and z = t / (2 + t) <= 1/3 the logarithm of 1 + t is 2 artanh(z), whose series is cut off below 2^-29. What rounding 2 + t and z leaves over
+// goes into the small term: off by 0.58 of 2^-24 in the mean square, as a logarithm of 1 + e^x rounded twice
+__device__ __forceinline__ float softplus_near(float x) {
+  const float t = expf(-fabsf(x)), y = 2.f + t, r0 = vy_rcp_approx(y), r = fmaf(r0, fmaf(-y, r0, 1.f), r0), z = t * r, w = z * z;
+  const float left = fmaf(-z, t - (y - 2.f), fmaf(-z, y, t)) * r;
+  float p = fmaf(w, 1.f / 15.f, 1.f / 13.f);
+  p = fmaf(w, p, 1.f / 11.f);
+  p = fmaf(w, p, 1.f / 9.f);
+  p = fmaf(w, p, 1.f / 7.f);
+  p = fmaf(w, p, 1.f / 5.f);
+  p = fmaf(w, p, 1.f / 3.f);
+  return fmaxf(x, 0.f) + (2.f * z + fmaf(2.f * z * w, p, 2.f * left));
+}
+
 template <int DP>
-__global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks w) {
+__global__ void __launch_bounds__(256, 4) delta_chunk_kernel(RecDev d, DeltaChunks w, bool vec) {
   pdl_trigger();
   pdl_wait();
-  constexpr int LD = DP + 8, NP = DC_T * DP / 256, PER = DP / 16;
   using Blob = DcBlob<DP>;
-  __shared__ __align__(16) float ks[DC_T][LD], qs[DC_T][LD], gs[DC_T][LD], xs[DC_T][LD], kb[DC_T][LD];
-  __shared__ float A[DC_T][DC_T + 1], B[DC_T][DC_T + 1], W[DC_T][DC_T + 1], beta[DC_T], scale[3][DC_T];
+  constexpr int LD = DP + 4, LV = 132, LA = DC_T + 4, Q4 = DP / 4, PER = (DC_T * Q4 + 255) / 256;   // Q4 lanes hold a token, four channels each
+  __shared__ __align__(16) float ks[DC_T][LD], qs[DC_T][LD], gs[DC_T][LD], xs[DC_T][LD], vs[DC_T][LV], As[DC_T][LA];   // As: [s][t] -A_ts
+  __shared__ float B[DC_T][DC_T + 1], beta[DC_T], scale[3][DC_T];
   const int s = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * DC_T;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
   if (t0 >= n) return;
@@ -55,153 +70,178 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks 
   const int gq = h / (d.heads / d.kv_heads);
   const long long row0 = base + t0, at = (chunk_slot0(base, s) + blockIdx.x) * d.heads + h;
   unsigned char* blob = w.blobs + at * Blob::bytes;
-  {
-    float rq[NP], rk[NP], ra[NP];
-#pragma unroll
-    for (int u = 0; u < NP; ++u) {
-      const int e = tid + 256 * u, tt = e / DP, i = e % DP;
-      const bool ok = tt < nt && i < d.dim;
-      rq[u] = ok ? ld_as_float(d.q, d.in_dt, (row0 + tt) * d.ldq + static_cast<long long>(gq) * d.dim + i) : 0.f;
-      rk[u] = ok ? ld_as_float(d.k, d.in_dt, (row0 + tt) * d.ldk + static_cast<long long>(gq) * d.dim + i) : 0.f;
-      ra[u] = ok ? ld_as_float(d.a, d.a_dt, (row0 + tt) * d.ld_a + static_cast<long long>(h) * d.dim + i) : 0.f;
-    }
-    const float neg_rate = -expf(ld_as_float(d.a_log, d.a_log_dt, h));
+  {   // unit vectors, decays and what a token reads of itself
+    const int c = 4 * (tid % Q4);
+    const float neg_rate = -expf(ld_as_float(d.a_log, d.a_log_dt, h)), top = 1.f / sqrtf(static_cast<float>(d.dim));
     if (tid < DC_T) beta[tid] = tid < nt ? sigmoidf_(ld_as_float(d.b, d.b_dt, (row0 + tid) * d.ld_b + h)) : 0.f;
+    float4 q[PER], k[PER], a[PER];
 #pragma unroll
-    for (int u = 0; u < NP; ++u) {
-      const int e = tid + 256 * u, tt = e / DP, i = e % DP;
-      qs[tt][i] = rq[u];
-      ks[tt][i] = rk[u];
-      const float x = tt < nt && i < d.dim ? neg_rate * softplusf_(ra[u]) : 0.f;
-      xs[tt][i] = x;
-      gs[tt][i] = expf(x);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {   // unit vectors, two tokens per warp
-    const int tt = 2 * warp + r;
-    float xq[DP / 32], xk[DP / 32], sq = 0.f, sk = 0.f;
-#pragma unroll
-    for (int m = 0; m < DP / 32; ++m) {
-      xq[m] = qs[tt][lane + 32 * m];
-      xk[m] = ks[tt][lane + 32 * m];
-      sq = fmaf(xq[m], xq[m], sq);
-      sk = fmaf(xk[m], xk[m], sk);
-    }
-    sq = warp_sum(sq);
-    sk = warp_sum(sk);
-    const float qn = tt < nt ? 1.f / sqrtf(static_cast<float>(d.dim)) / sqrtf(sq + d.unit_eps) : 0.f, kn = tt < nt ? 1.f / sqrtf(sk + d.unit_eps) : 0.f;
-#pragma unroll
-    for (int m = 0; m < DP / 32; ++m) {
-      qs[tt][lane + 32 * m] = xq[m] * qn;
-      ks[tt][lane + 32 * m] = xk[m] * kn;
-    }
-  }
-  __syncthreads();
-  {   // G_t and G_15 / G_s k_s, a channel per thread, from sums of the decays' logarithms: an fp32 decay near 1 is off by a share of its distance
-      // from 1 that a product over a long memory multiplies
-    const int i = tid & 127;
-    float G[DC_T], x = 0.f;
-    if (i < DP) {
-      if (tid < 128) {
-#pragma unroll
-        for (int t = 0; t < DC_T; ++t) G[t] = expf(x += xs[t][i]);
-      } else {
-#pragma unroll
-        for (int t = DC_T - 1; t >= 0; --t) {
-          kb[t][i] = ks[t][i] * expf(x);
-          x += xs[t][i];
+    for (int u = 0; u < PER; ++u) {
+      const int t = tid / Q4 + 256 / Q4 * u;
+      const long long oq = (row0 + t) * d.ldq + static_cast<long long>(gq) * d.dim, ok = (row0 + t) * d.ldk + static_cast<long long>(gq) * d.dim,
+                      oa = (row0 + t) * d.ld_a + static_cast<long long>(h) * d.dim;
+      q[u] = k[u] = a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < nt && c < d.dim) {
+        if (vec) {
+          q[u] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.q) + oq + c);
+          k[u] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.k) + ok + c);
+          a[u] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.a) + oa + c);
+        } else {
+          q[u] = load4_any(d.q, d.in_dt, oq, c, d.dim);
+          k[u] = load4_any(d.k, d.in_dt, ok, c, d.dim);
+          a[u] = load4_any(d.a, d.a_dt, oa, c, d.dim);
         }
       }
     }
-    __syncthreads();
-    if (tid < DP) {
 #pragma unroll
-      for (int t = 0; t < DC_T; ++t) xs[t][i] = G[t];
-      reinterpret_cast<float*>(blob + Blob::g_at)[i] = G[DC_T - 1];
-    }
-  }
-  {   // A and B: 16 lanes per token s carry G_t / G_s k_s through the tokens t after it
-    const int sl = tid & 15, c = tid >> 4;
-    const auto lane_channels = [&](const float* p, float (&x)[PER]) {
-      if constexpr (PER == 2) {
-        const float2 v = *reinterpret_cast<const float2*>(p + 2 * sl);
-        x[0] = v.x; x[1] = v.y;
-      } else {
+    for (int u = 0; u < PER; ++u) {
+      const int t = tid / Q4 + 256 / Q4 * u;
+      float sq = dot4(q[u], q[u], 0.f), sk = dot4(k[u], k[u], 0.f);
 #pragma unroll
-        for (int m = 0; m < PER / 4; ++m) {
-          const float4 v = f4(p + 64 * m + 4 * sl);
-          x[4 * m] = v.x; x[4 * m + 1] = v.y; x[4 * m + 2] = v.z; x[4 * m + 3] = v.w;
-        }
+      for (int o = 1; o < Q4; o <<= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        sk += __shfl_xor_sync(0xffffffffu, sk, o);
       }
-    };
-    float D[PER];
+      const float qn = t < nt ? top / sqrtf(sq + d.unit_eps) : 0.f, kn = t < nt ? 1.f / sqrtf(sk + d.unit_eps) : 0.f;
+      const float4 uq = make_float4(q[u].x * qn, q[u].y * qn, q[u].z * qn, q[u].w * qn), uk = make_float4(k[u].x * kn, k[u].y * kn, k[u].z * kn, k[u].w * kn);
+      float own = dot4(uq, uk, 0.f);
 #pragma unroll
-    for (int e = 0; e < PER; ++e) D[e] = 0.f;
-    for (int t = 2 * warp; t < DC_T; ++t) {
-      float kt[PER], qt[PER], gt[PER], a = 0.f, b = 0.f;
-      lane_channels(ks[t], kt);
-      lane_channels(qs[t], qt);
-      lane_channels(gs[t], gt);
-#pragma unroll
-      for (int e = 0; e < PER; ++e) {
-        D[e] = t == c ? kt[e] : (t > c ? D[e] * gt[e] : 0.f);
-        a = fmaf(D[e], kt[e], a);
-        b = fmaf(D[e], qt[e], b);
-      }
-#pragma unroll
-      for (int o = 1; o < 16; o <<= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-      }
-      if (sl == 0 && t >= c) {
-        A[t][c] = a;
-        B[t][c] = b;
-      }
+      for (int o = 1; o < Q4; o <<= 1) own += __shfl_xor_sync(0xffffffffu, own, o);
+      if (DC_T * Q4 < 256 && t >= DC_T) continue;
+      if (c == 0) B[t][t] = own;
+      const auto x_of = [&](float v, int i) { return t < nt && c + i < d.dim ? neg_rate * softplus_near(v) : 0.f; };
+      const float4 x = make_float4(x_of(a[u].x, 0), x_of(a[u].y, 1), x_of(a[u].z, 2), x_of(a[u].w, 3));
+      *reinterpret_cast<float4*>(&qs[t][c]) = uq;
+      *reinterpret_cast<float4*>(&ks[t][c]) = uk;
+      *reinterpret_cast<float4*>(&xs[t][c]) = x;
+      *reinterpret_cast<float4*>(&gs[t][c]) = make_float4(expf(x.x), expf(x.y), expf(x.z), expf(x.w));
     }
   }
   __syncthreads();
-  if (tid < DC_T) {   // W, a column per lane
-    float x[DC_T];
+  {   // A and B: sixteen lanes carry G_t / G_s k_s through the tokens t after s, for s = warp and s = 15 - warp
+    constexpr int RP = (DP + 63) / 64;
+    const int l16 = lane & 15, sl = lane & 16 ? 15 - warp : warp, c = DP < 64 ? 4 * (l16 & 7) : 4 * l16;
+    const bool idle = DP < 64 && l16 >= 8;
+    f32x2 D[RP][2];
+#pragma unroll
+    for (int m = 0; m < RP; ++m) {
+      const float4 v = f4(&ks[sl][c + 64 * m]);
+      D[m][0] = idle ? pair(0.f) : pair(v.x, v.y);
+      D[m][1] = idle ? pair(0.f) : pair(v.z, v.w);
+    }
+#pragma unroll 1
+    for (int t = warp + 1; t < DC_T; ++t) {
+      float a = 0.f, b = 0.f;
+      if (t > sl) {
+        f32x2 sa = pair(0.f), sb = pair(0.f);
+#pragma unroll
+        for (int m = 0; m < RP; ++m) {
+          const float4 gt = f4(&gs[t][c + 64 * m]), kt = f4(&ks[t][c + 64 * m]), qt = f4(&qs[t][c + 64 * m]);
+          D[m][0] = mul2(D[m][0], pair(gt.x, gt.y));
+          D[m][1] = mul2(D[m][1], pair(gt.z, gt.w));
+          sa = fma2(D[m][0], pair(kt.x, kt.y), sa);
+          sb = fma2(D[m][0], pair(qt.x, qt.y), sb);
+          sa = fma2(D[m][1], pair(kt.z, kt.w), sa);
+          sb = fma2(D[m][1], pair(qt.z, qt.w), sb);
+        }
+        const float2 ya = unpair(sa), yb = unpair(sb);
+        a = ya.x + ya.y;
+        b = yb.x + yb.y;
+        if (idle) a = b = 0.f;
+      }
+      __syncwarp();
+      const float other = __shfl_xor_sync(0xffffffffu, lane & 8 ? a : b, 8);   // the first eight lanes of sixteen go on with a, the others with b
+      float y = (lane & 8 ? b : a) + other;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+      if (t > sl && (lane & 7) == 0) (lane & 8 ? B[t][sl] : As[sl][t]) = lane & 8 ? y : -y;
+    }
+  }
+  __syncthreads();
+  // The triangular system, a column per thread: those of G k by the first half of the threads, those of V by the other. A later token never enters an earlier one's
+  // sum, not even times zero
+  const auto solve = [&](float (&r)[DC_T]) {   // what the earlier tokens take away is summed by itself: it is small beside most entries, whose rounding would be that of every term
+    float less[DC_T];
+#pragma unroll
+    for (int t = 0; t < DC_T; ++t) less[t] = 0.f;
+#pragma unroll
+    for (int i = 0; i < DC_T; ++i) {
+      const float x = r[i] = fmaf(beta[i], r[i], beta[i] * less[i]);
+#pragma unroll
+      for (int t = i & ~3; t < DC_T; t += 4) {
+        if (t + 3 == i) continue;
+        const float4 m = f4(&As[i][t]);
+        if (t > i) less[t] = fmaf(m.x, x, less[t]);
+        if (t + 1 > i) less[t + 1] = fmaf(m.y, x, less[t + 1]);
+        if (t + 2 > i) less[t + 2] = fmaf(m.z, x, less[t + 2]);
+        less[t + 3] = fmaf(m.w, x, less[t + 3]);
+      }
+    }
+  };
+  // G_t and G_15 / G_s are exponentials of sums of the decays' logarithms: an fp32 decay near 1 is off by a share of its distance from 1 that a product over a long
+  // memory multiplies
+  const int ch = tid & 127;
+  const auto value_column = [&](int c) {   // W v of column c, into vs
+    float r[DC_T];
+#pragma unroll
+    for (int t = 0; t < DC_T; ++t) r[t] = t < nt && c < d.vdim ? ld_as_float(d.v, d.in_dt, (row0 + t) * d.ldv + static_cast<long long>(h) * d.vdim + c) : 0.f;
+    solve(r);
+#pragma unroll
+    for (int t = 0; t < DC_T; ++t) vs[t][c & 127] = r[t];
+  };
+  float r[DC_T];
+  if (tid >= 128) {
+    if (ch < DP) {
+      float x = 0.f;
+#pragma unroll
+      for (int t = DC_T - 1; t >= 0; --t) {
+        gs[t][ch] = ks[t][ch] * expf(x);
+        x += xs[t][ch];
+      }
+    }
+    value_column(ch);
+  } else if (ch < DP) {
+    float x = 0.f;
 #pragma unroll
     for (int t = 0; t < DC_T; ++t) {
-      float r = 0.f;
-#pragma unroll
-      for (int c = 0; c < t; ++c)
-        if (c >= tid) r = fmaf(A[t][c], x[c], r);
-      x[t] = t < tid ? 0.f : (t == tid ? beta[t] : -beta[t] * r);
-      W[t][tid] = x[t];
+      const float G = expf(x += xs[t][ch]);
+      qs[t][ch] *= G;
+      r[t] = ks[t][ch] * G;
+      if (t == DC_T - 1) reinterpret_cast<float*>(blob + Blob::g_at)[ch] = G;
     }
+    solve(r);
   }
   __syncthreads();
-  {   // P = W G k, and G q in place; a later token never enters an earlier one's sum, not even times zero
-    const int i = tid % DP, tp = tid / DP * NP;
-    float kc[DC_T], p[NP];
+  if (tid < DP)
 #pragma unroll
-    for (int t = 0; t < DC_T; ++t) kc[t] = ks[t][i] * xs[t][i];
+    for (int t = 0; t < DC_T; ++t) xs[t][ch] = r[t];   // P
+  const int l4 = lane >> 2, tq = 2 * (lane & 3);
+  const auto store_values = [&](int c0) {   // entry lane of 16 columns holds columns l4, l4 + 8 of tokens tq, tq + 1, tq + 8, tq + 9
+    const int b16 = (c0 >> 4) + warp;
+    if (16 * b16 >= w.vpad) return;
+    float x[8];
 #pragma unroll
-    for (int r = 0; r < NP; ++r) {
-      p[r] = 0.f;
-#pragma unroll
-      for (int c = 0; c < DC_T; ++c)
-        if (c <= tp + r) p[r] = fmaf(W[tp + r][c], kc[c], p[r]);
-    }
+    for (int e = 0; e < 8; ++e) x[e] = vs[tq + 8 * (e >> 2) + (e & 1)][16 * warp + l4 + 8 * ((e >> 1) & 1)];
+    float4* o = reinterpret_cast<float4*>(w.wv + (at * (w.vpad / 16) + b16) * 256 + lane * 8);
+    o[0] = make_float4(x[0], x[1], x[2], x[3]);
+    o[1] = make_float4(x[4], x[5], x[6], x[7]);
+  };
+  store_values(0);
+#pragma unroll 1
+  for (int c0 = 128; c0 < w.vpad; c0 += 128) {
     __syncthreads();
-#pragma unroll
-    for (int r = 0; r < NP; ++r) {
-      ks[tp + r][i] = p[r];
-      qs[tp + r][i] *= xs[tp + r][i];
-    }
+    if (tid < 128) value_column(c0 + ch);
+    __syncthreads();
+    store_values(c0);
   }
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {   // a scale per token for each of P, G q and B
-    const int tt = 2 * warp + r;
+  for (int e = 0; e < 2; ++e) {   // a scale per token for each of P, G q and B
+    const int tt = 2 * warp + e;
     float mp = 0.f, mq = 0.f, mb = lane <= tt ? fabsf(B[tt][min(lane, DC_T - 1)]) : 0.f;
 #pragma unroll
     for (int m = 0; m < DP / 32; ++m) {
-      mp = fmaxf(mp, fabsf(ks[tt][lane + 32 * m]));
+      mp = fmaxf(mp, fabsf(xs[tt][lane + 32 * m]));
       mq = fmaxf(mq, fabsf(qs[tt][lane + 32 * m]));
     }
     const int ep = split_exponent(warp_max(mp)), eq = split_exponent(warp_max(mq)), eb = split_exponent(warp_max(mb));
@@ -216,7 +256,6 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks 
     }
   }
   __syncthreads();
-  const int l4 = lane >> 2, tq = 2 * (lane & 3);
   uint4* out = reinterpret_cast<uint4*>(blob);
 #pragma unroll
   for (int u = 0; u < DP / 64 + (DP < 64); ++u) {
@@ -225,7 +264,7 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks 
       const int t = 8 * ((e >> 5) & 1) + l4, i = 16 * (e >> 6) + tq;
       uint4 x;
       const float sp = scale[0][t], sq = scale[1][t];
-      const float2 p0 = *reinterpret_cast<const float2*>(&ks[t][i]), p1 = *reinterpret_cast<const float2*>(&ks[t][i + 8]);
+      const float2 p0 = *reinterpret_cast<const float2*>(&xs[t][i]), p1 = *reinterpret_cast<const float2*>(&xs[t][i + 8]);
       split2(p0.x * sp, p0.y * sp, x.x, x.z);
       split2(p1.x * sp, p1.y * sp, x.y, x.w);
       out[e] = x;
@@ -235,8 +274,8 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks 
       out[Blob::q_at / 16 + e] = x;
       const int j = 8 * (e >> 5) + l4;   // G_15 / G_s k_s: 16 tokens (k) x 8 channels (n)
       constexpr float one = 1 << DC_KTOP;
-      split2(kb[tq][j] * one, kb[tq + 1][j] * one, x.x, x.z);
-      split2(kb[tq + 8][j] * one, kb[tq + 9][j] * one, x.y, x.w);
+      split2(gs[tq][j] * one, gs[tq + 1][j] * one, x.x, x.z);
+      split2(gs[tq + 8][j] * one, gs[tq + 9][j] * one, x.y, x.w);
       out[Blob::k_at / 16 + e] = x;
     }
   }
@@ -248,28 +287,6 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(RecDev d, DeltaChunks 
     split2(b(tq), b(tq + 1), x.x, x.z);
     split2(b(tq + 8), b(tq + 9), x.y, x.w);
     out[Blob::b_at / 16 + tid] = x;
-  }
-  for (int e = tid; e < w.vpad * 2; e += 256) {   // W v: entry lane of 16 columns holds columns l4, l4 + 8 of tokens tq, tq + 1, tq + 8, tq + 9
-    const int c0 = 16 * (e >> 5) + l4;
-    const bool ok0 = c0 < d.vdim, ok1 = c0 + 8 < d.vdim;
-    float v[2][DC_T], x[8];
-#pragma unroll
-    for (int c = 0; c < DC_T; ++c) {
-      const long long o = (row0 + c) * d.ldv + static_cast<long long>(h) * d.vdim + c0;
-      v[0][c] = c < nt && ok0 ? ld_as_float(d.v, d.in_dt, o) : 0.f;
-      v[1][c] = c < nt && ok1 ? ld_as_float(d.v, d.in_dt, o + 8) : 0.f;
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {   // register r: token half r / 4, column half r / 2 % 2, token r % 2
-      const int t = tq + 8 * (r >> 2) + (r & 1);
-      x[r] = 0.f;
-#pragma unroll
-      for (int c = 0; c < DC_T; ++c)
-        if (c <= t) x[r] = fmaf(W[t][c], v[(r >> 1) & 1][c], x[r]);
-    }
-    float4* o = reinterpret_cast<float4*>(w.wv + (at * (w.vpad / 16) + (e >> 5)) * 256 + lane * 8);
-    o[0] = make_float4(x[0], x[1], x[2], x[3]);
-    o[1] = make_float4(x[4], x[5], x[6], x[7]);
   }
 }
 
@@ -292,6 +309,51 @@ static __device__ __noinline__ void dc_read_serial(float (&o)[2][4], const float
       o[r >> 1][r & 1] = fmaf(x, u0, o[r >> 1][r & 1]);
       o[r >> 1][2 + (r & 1)] = fmaf(x, u1, o[r >> 1][2 + (r & 1)]);
     }
+  }
+}
+
+// One chunk's writes as accumulators, from what the state gives (read-outs of P by `KW` warps, [warp][4][32 lanes] in `part`), and as A operand; m, w: each column's largest write, its unit
+struct DcWrites {
+  float u[2][4], m[2], w[2];
+  unsigned hi[4], lo[4];
+};
+template <int KW>
+__device__ __forceinline__ void dc_writes(DcWrites& x, const float4* part, const float4* wv, const float* unit, int lane) {
+  const int tq = 2 * (lane & 3);
+  x.m[0] = x.m[1] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    float4 z[KW];
+#pragma unroll
+    for (int k = 0; k < KW; ++k) z[k] = part[(4 * k + j) * 32 + lane];
+#pragma unroll
+    for (int k = 1; k < KW; k <<= 1)
+#pragma unroll
+      for (int i = 0; i + k < KW; i += 2 * k) {
+        z[i].x += z[i + k].x; z[i].y += z[i + k].y; z[i].z += z[i + k].z; z[i].w += z[i + k].w;
+      }
+    const float4 y = wv[j];
+    const float2 p = *reinterpret_cast<const float2*>(unit + 8 * j + tq);
+    x.u[j][0] = fmaf(-z[0].x, p.x, y.x);
+    x.u[j][1] = fmaf(-z[0].y, p.y, y.y);
+    x.u[j][2] = fmaf(-z[0].z, p.x, y.z);
+    x.u[j][3] = fmaf(-z[0].w, p.y, y.w);
+    x.m[0] = fmaxf(x.m[0], fmaxf(fabsf(x.u[j][0]), fabsf(x.u[j][1])));
+    x.m[1] = fmaxf(x.m[1], fmaxf(fabsf(x.u[j][2]), fabsf(x.u[j][3])));
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    x.m[0] = fmaxf(x.m[0], __shfl_xor_sync(0xffffffffu, x.m[0], o));
+    x.m[1] = fmaxf(x.m[1], __shfl_xor_sync(0xffffffffu, x.m[1], o));
+  }
+  const int f0 = split_exponent(x.m[0]), f1 = split_exponent(x.m[1]);
+  const float t0 = split_scale(f0), t1 = split_scale(f1);
+  x.w[0] = pow2i(f0 - SPLIT_TOP);
+  x.w[1] = pow2i(f1 - SPLIT_TOP);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    split2(x.u[j][0] * t0, x.u[j][1] * t0, x.hi[2 * j], x.lo[2 * j]);
+    split2(x.u[j][2] * t1, x.u[j][3] * t1, x.hi[2 * j + 1], x.lo[2 * j + 1]);
   }
 }
 
@@ -511,13 +573,15 @@ int round32(int x) { return (x + 31) / 32 * 32; }
 
 template <int DP>
 cudaError_t launch(const RecDev& d, int n_seqs, int max_new, const DeltaChunks& w, cudaStream_t st) {
-  const size_t smem = DC_NS * (DcBlob<DP>::bytes + DC_NW * 1024);
+  constexpr int smem = DC_NS * (DcBlob<DP>::bytes + DC_NW * 1024);
   static std::atomic<unsigned long long> allowed{0};
-  cudaError_t ea = allow_smem(delta_scan_kernel<DP>, allowed);
-  if (ea != cudaSuccess) return ea;
+  cudaError_t e = allow_smem(delta_scan_kernel<DP>, allowed);
+  if (e != cudaSuccess) return e;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
-  cudaError_t e = launch_kernel(delta_chunk_kernel<DP>, dim3((max_new + DC_T - 1) / DC_T, d.heads, n_seqs), dim3(256), 0, st, d, w);
+  const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
+  const bool vec = d.in_dt == VY_F32 && d.a_dt == VY_F32 && d.dim % 4 == 0 && quads(d.q, d.ldq) && quads(d.k, d.ldk) && quads(d.a, d.ld_a);
+  e = launch_kernel(delta_chunk_kernel<DP>, dim3((max_new + DC_T - 1) / DC_T, d.heads, n_seqs), dim3(256), 0, st, d, w, vec);
   if (e != cudaSuccess) return e;
   count_launch();
   return launch_kernel(delta_scan_kernel<DP>, dim3(w.vpad / 32, d.heads, n_seqs), dim3(32 * DC_NW), smem, st, d, w, poison);
