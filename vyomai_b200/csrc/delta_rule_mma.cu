@@ -10,10 +10,11 @@
 //                        register layout of the second launch's operands
 //   delta_scan_kernel    the walk. It is transposed (S^T: a warp owns 16 value columns and all channels), so that the state in accumulator
 //                        registers is the next product's A operand, the writes likewise, and no warp waits for another one
+//   delta_scan_split_kernel   the same with a warp for every 32 channels, whose shares of the read-outs meet in shared memory once per chunk
 // The walk token by token (delta_rule_kernel) is bound by its chain of two reductions per token: 46 + 1013 us with its preparation for 4 x 2048
-// tokens, 8 heads of 128 x 128; here 120 + 236 us. The first launch is bound by instructions, 85 million of them (decays, exponentials, sums over pairs of tokens; with
-// W made first, a column of it per lane, and channels loaded one by one 126 million, 163 us), the second by the latency of one
-// warp's chain, 1.8 us per chunk. Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
+// tokens, 8 heads of 128 x 128; here 120 + 180 us. The first launch is bound by instructions, 85 million of them (decays, exponentials, sums over pairs of tokens; with
+// W made first, a column of it per lane, and channels loaded one by one 126 million, 163 us), the second by the latency of a warp's chain: 1.4 us per chunk, 1.8 where one
+// warp has all channels (236 us). Error against 64 bits at decays near 1: 2e-7 instead of 1.6e-6.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 
@@ -357,6 +358,207 @@ __device__ __forceinline__ void dc_writes(DcWrites& x, const float4* part, const
   }
 }
 
+// A CTA has 16 value columns, KW warps with 32 channels of the state apiece and one warp for the read-outs. Every warp works out the writes for itself: less of a chain, more
+// instructions, and a barrier per chunk
+template <int DP>
+__global__ void __launch_bounds__(32 * (DP / 32 + 1)) delta_scan_split_kernel(RecDev d, DeltaChunks w, PoisonRef poison) {
+  pdl_trigger();
+  pdl_wait();
+  using Blob = DcBlob<DP>;
+  constexpr int KW = DP / 32, STAGE = Blob::bytes + 1024;
+  extern __shared__ __align__(128) unsigned char dc_smem[];
+  __shared__ __align__(8) uint64_t full[DC_NS];
+  __shared__ int issued[DC_NS];   // chunks sent for into a stage
+  const int s = blockIdx.z, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l4 = lane >> 2, tq = 2 * (lane & 3);
+  const int base = d.cu[s], n = d.cu[s + 1] - base;
+  if (n <= 0) return;
+  const int chunks = (n + DC_T - 1) / DC_T;
+  const long long slot0 = chunk_slot0(base, s);
+  const auto fetch = [&](int c, int b) {
+    const long long at = (slot0 + c) * d.heads + h;
+    unsigned char* st = dc_smem + b * STAGE;
+    ++issued[b];
+    mbar_arrive_expect_tx(&full[b], STAGE);
+    bulk_load(st, w.blobs + at * Blob::bytes, Blob::bytes, &full[b]);
+    bulk_load(st + Blob::bytes, w.wv + (at * (w.vpad / 16) + blockIdx.x) * 256, 1024, &full[b]);
+  };
+  const bool sender = threadIdx.x == 32 * KW;   // a lane of the read-out warp
+  if (sender) {
+    for (int b = 0; b < DC_NS; ++b) {
+      mbar_init(&full[b], 1);
+      issued[b] = 0;
+    }
+    fence_mbar_init();
+    for (int b = 0; b < min(DC_NS, chunks); ++b) fetch(b, b);
+  }
+  float4* exchange = reinterpret_cast<float4*>(dc_smem + DC_NS * STAGE);   // [chunk parity][warp][P, P, G q, G q][lane]
+  constexpr int TURN = KW * 128;
+  const int col = 16 * blockIdx.x + l4;
+  const bool ok0 = col < d.vdim, ok1 = col + 8 < d.vdim;
+  bool alive = true;   // no wait of this thread has timed out
+  // a stage is free once every warp has come to the barrier of the chunk after it
+  const auto refill = [&](int c) {
+    if (c > 0 && alive && c - 1 + DC_NS < chunks) {
+      fence_proxy_async_smem();
+      fetch(c - 1 + DC_NS, (c - 1) % DC_NS);
+    }
+  };
+  if (warp < KW) {
+    // S^T as accumulators: S[j][e] is column l4 + 8 (e / 2), channel 32 warp + 8 j + tq + e % 2
+    float* sp = d.state + ((static_cast<long long>(d.slot[s]) * d.heads + h) * d.dim) * d.vdim + col;
+    const bool carried = d.pos0[s] > 0;
+    float S[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 32 * warp + 8 * j + tq + (e & 1);
+        S[j][e] = carried && i < d.dim && (e < 2 ? ok0 : ok1) ? sp[static_cast<long long>(i) * d.vdim + 8 * (e >> 1)] : 0.f;
+      }
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c % DC_NS;
+      const unsigned char* st = dc_smem + b * STAGE;
+      float4* part = exchange + (c & 1) * TURN;
+      float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        m0 = fmaxf(m0, fmaxf(fabsf(S[j][0]), fabsf(S[j][1])));
+        m1 = fmaxf(m1, fmaxf(fabsf(S[j][2]), fabsf(S[j][3])));
+      }
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+      }
+      const int e0 = split_exponent(m0), e1 = split_exponent(m1);
+      const float s0 = split_scale(e0), s1 = split_scale(e1), n0 = pow2i(e0 - SPLIT_TOP), n1 = pow2i(e1 - SPLIT_TOP);
+      alive = mbar_wait_soft(&full[b], (c / DC_NS) & 1, poison) && alive;
+      const uint4* ops = reinterpret_cast<const uint4*>(st) + lane;
+      const float* unit = reinterpret_cast<const float*>(st + Blob::unit_at);
+      float r[4][4], x[4][4];   // S^T P and S^T G q over this warp's channels: 8 tokens each
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[j][e] = x[j][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        unsigned ah[4], al[4];
+        split2(S[2 * k][0] * s0, S[2 * k][1] * s0, ah[0], al[0]);
+        split2(S[2 * k][2] * s1, S[2 * k][3] * s1, ah[1], al[1]);
+        split2(S[2 * k + 1][0] * s0, S[2 * k + 1][1] * s0, ah[2], al[2]);
+        split2(S[2 * k + 1][2] * s1, S[2 * k + 1][3] * s1, ah[3], al[3]);
+        uint4 f[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = ops[(j >= 2 ? Blob::q_at / 16 : 0) + 32 * (2 * (2 * warp + k) + (j & 1))];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_f16(x[j], al, f[j].x, f[j].y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_f16(r[j], ah, f[j].x, f[j].y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_f16(x[j], ah, f[j].z, f[j].w);
+      }
+      constexpr float cut = 1.5f * SPLIT_CUT;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        part[(4 * warp + j) * 32 + lane] = make_float4(split_sum(r[j][0], x[j][0], cut) * n0, split_sum(r[j][1], x[j][1], cut) * n0,
+                                                     split_sum(r[j][2], x[j][2], cut) * n1, split_sum(r[j][3], x[j][3], cut) * n1);
+        const float2 q = *reinterpret_cast<const float2*>(unit + DC_T + 8 * j + tq);
+        part[(4 * warp + 2 + j) * 32 + lane] = make_float4(split_sum(r[2 + j][0], x[2 + j][0], cut) * (n0 * q.x), split_sum(r[2 + j][1], x[2 + j][1], cut) * (n0 * q.y),
+                                                         split_sum(r[2 + j][2], x[2 + j][2], cut) * (n1 * q.x), split_sum(r[2 + j][3], x[2 + j][3], cut) * (n1 * q.y));
+      }
+      __syncthreads();
+      DcWrites u;
+      dc_writes<KW>(u, part, reinterpret_cast<const float4*>(st + Blob::bytes + 32 * lane), unit, lane);
+      // the state
+      const float k0 = u.w[0] * (1.f / (1 << DC_KTOP)), k1 = u.w[1] * (1.f / (1 << DC_KTOP));
+      const float* G = reinterpret_cast<const float*>(st + Blob::g_at) + 32 * warp + tq;
+      float y[4][4], z[4][4];
+      uint4 f[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[j][e] = z[j][e] = 0.f;
+        f[j] = ops[Blob::k_at / 16 + 32 * (4 * warp + j)];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_f16(z[j], u.lo, f[j].x, f[j].y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_f16(y[j], u.hi, f[j].x, f[j].y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma_f16(z[j], u.hi, f[j].z, f[j].w);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 g = *reinterpret_cast<const float2*>(G + 8 * j);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j][e] = fmaf(S[j][e], e & 1 ? g.y : g.x, split_sum(y[j][e], z[j][e], SPLIT_CUT) * (e < 2 ? k0 : k1));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 32 * warp + 8 * j + tq + (e & 1);
+        if (i < d.dim && (e < 2 ? ok0 : ok1)) sp[static_cast<long long>(i) * d.vdim + 8 * (e >> 1)] = S[j][e];
+      }
+  } else {
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c % DC_NS;
+      const unsigned char* st = dc_smem + b * STAGE;
+      const float4* part = exchange + (c & 1) * TURN;
+      alive = mbar_wait_soft(&full[b], (c / DC_NS) & 1, poison) && alive;
+      __syncthreads();
+      if (sender) refill(c);
+      const float* unit = reinterpret_cast<const float*>(st + Blob::unit_at);
+      DcWrites u;
+      dc_writes<KW>(u, part, reinterpret_cast<const float4*>(st + Blob::bytes + 32 * lane), unit, lane);
+      float o[2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float4 x = part[(2 + j) * 32 + lane];
+#pragma unroll
+        for (int k = 1; k < KW; ++k) {
+          const float4 y = part[(4 * k + 2 + j) * 32 + lane];
+          x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+        }
+        o[j][0] = x.x; o[j][1] = x.y; o[j][2] = x.z; o[j][3] = x.w;
+      }
+      const float a0 = DC_APART * u.m[0], a1 = DC_APART * u.m[1];
+      bool together = u.m[0] < INFINITY && u.m[1] < INFINITY;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) together = together && fabsf(u.u[j][e]) >= (e < 2 ? a0 : a1);   // false for NaN
+      if (__all_sync(0xffffffffu, together)) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
+          const uint4 f = (reinterpret_cast<const uint4*>(st) + lane)[Blob::b_at / 16 + 32 * j];
+          const float2 p = *reinterpret_cast<const float2*>(unit + 2 * DC_T + 8 * j + tq);
+          mma_f16(z, u.lo, f.x, f.y);
+          mma_f16(y, u.hi, f.x, f.y);
+          mma_f16(z, u.hi, f.z, f.w);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[j][e] = fmaf(split_sum(y[e], z[e], SPLIT_CUT) * u.w[e >> 1], e & 1 ? p.y : p.x, o[j][e]);
+        }
+      } else {
+        dc_read_serial(o, u.u, st + Blob::b_at, unit + 2 * DC_T, lane);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = DC_T * c + 8 * j + tq + (e & 1);
+          if (t < n && (e < 2 ? ok0 : ok1))
+            st_from_float(d.out, d.out_dt, static_cast<long long>(base + t) * d.ld_out + static_cast<long long>(h) * d.vdim + col + 8 * (e >> 1), o[j][e]);
+        }
+    }
+  }
+  if (__syncthreads_or(!alive)) mbar_drain(full, issued, DC_NS);
+}
+
 template <int DP>
 __global__ void __launch_bounds__(32 * DC_NW) delta_scan_kernel(RecDev d, DeltaChunks w, PoisonRef poison) {
   pdl_trigger();
@@ -573,9 +775,13 @@ int round32(int x) { return (x + 31) / 32 * 32; }
 
 template <int DP>
 cudaError_t launch(const RecDev& d, int n_seqs, int max_new, const DeltaChunks& w, cudaStream_t st) {
-  constexpr int smem = DC_NS * (DcBlob<DP>::bytes + DC_NW * 1024);
-  static std::atomic<unsigned long long> allowed{0};
-  cudaError_t e = allow_smem(delta_scan_kernel<DP>, allowed);
+  constexpr int split_smem = DC_NS * (DcBlob<DP>::bytes + 1024) + 2 * (DP / 32) * 2048, smem = DC_NS * (DcBlob<DP>::bytes + DC_NW * 1024);
+  // While all CTAs run at once, two per SM, the split walk's shorter chain counts; where they queue up, its instructions. All channels per warp / split, us, heads of 128 x 128:
+  // 8 over 4 x 2048 tokens (256 CTAs) 236 / 180, over one of 500 63 / 40; 16 over one of 2000 231 / 142; 8 over 8 x 1024 (512 CTAs) 125 / 182; 16 over 8 x 1000 243 / 340;
+  // 4 of 64 x 64 over 4 x 300 30 / 22, over 32 x 300 (512 CTAs) 32 / 35
+  const bool split = static_cast<long long>(n_seqs) * d.heads * (w.vpad / 16) <= 2 * num_sms();
+  static std::atomic<unsigned long long> allowed_split{0}, allowed{0};
+  cudaError_t e = split ? allow_smem(delta_scan_split_kernel<DP>, allowed_split) : allow_smem(delta_scan_kernel<DP>, allowed);
   if (e != cudaSuccess) return e;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
@@ -584,6 +790,7 @@ cudaError_t launch(const RecDev& d, int n_seqs, int max_new, const DeltaChunks& 
   e = launch_kernel(delta_chunk_kernel<DP>, dim3((max_new + DC_T - 1) / DC_T, d.heads, n_seqs), dim3(256), 0, st, d, w, vec);
   if (e != cudaSuccess) return e;
   count_launch();
+  if (split) return launch_kernel(delta_scan_split_kernel<DP>, dim3(w.vpad / 16, d.heads, n_seqs), dim3(32 * (DP / 32 + 1)), split_smem, st, d, w, poison);
   return launch_kernel(delta_scan_kernel<DP>, dim3(w.vpad / 32, d.heads, n_seqs), dim3(32 * DC_NW), smem, st, d, w, poison);
 }
 
