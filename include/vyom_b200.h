@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define VY_ABI_VERSION 16
+#define VY_ABI_VERSION 17
 
 #if defined(__GNUC__)
 #define VY_API __attribute__((visibility("default")))
@@ -646,9 +646,10 @@ typedef struct VyLinear {
   float scale;
   void* out; int64_t ld_out; int32_t out_dtype;
   /* batch > 1: `batch` independent products in one launch (one per attention head, say); product b reads A + b * a_batch,
-   * W + b * w_batch and writes out + b * out_batch (strides in elements; bias and addend must be null). 0 = 1. */
+   * W + b * w_batch and writes out + b * out_batch (strides in elements; addend must be null, bias too unless bias_batch gives its stride). 0 = 1. */
   int32_t batch; int64_t a_batch, w_batch, out_batch;
   void* stream;
+  int64_t bias_batch;
 } VyLinear;
 VY_API int vy_linear_plain(const VyLinear* p);
 
@@ -826,6 +827,10 @@ typedef struct VyCausalConv {
   void* out; int64_t ld_out; int32_t out_dtype;
   void* stream;
   int64_t rows; /* packed rows of the step, by which the form is chosen where portions are uneven; 0: n_seqs * max_new */
+  /* up to two further inputs in the same launch (channels 0: none), with the strides, types, taps and activation of the first; their outputs follow the first's columns in out */
+  int32_t channels2, channels3;
+  const void* x2; const void* w2; float* state2;
+  const void* x3; const void* w3; float* state3;
 } VyCausalConv;
 VY_API int vy_causal_conv(const VyCausalConv* p);
 

@@ -109,6 +109,43 @@ def test_delta_rule_keeps_a_bad_value_to_its_column_and_later_tokens():
         assert float((got - clean)[~hit].abs().max()) < 1e-6
 
 
+@pytest.mark.parametrize("M,N,K", [(33, 256, 1), (64, 257, 7), (65, 512, 16), (129, 514, 17), (300, 1030, 32), (9000, 256, 16)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_thin_products(M, N, K, dtype):
+    """Contractions of up to 32 over many rows, two of them in one call, each with its bias, weights with aligned rows and without."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x = torch.randn(M, 2 * K + 3, generator=g, device=DEV)
+    w, b = torch.randn(2, N, K, generator=g, device=DEV).to(dtype), torch.randn(2, N, generator=g, device=DEV).to(dtype)
+    wide = (N + 7) // 8 * 8
+    out = torch.full((M, 2 * wide), 7.0, device=DEV)
+    ops.head_linear(x, w, out, x_head=K + 3, out_head=wide, bias=b)
+    want = [x[:, i * (K + 3):i * (K + 3) + K].double() @ w[i].double().T + b[i].double() for i in range(2)]
+    for i in range(2):
+        assert _err(out[:, i * wide:i * wide + N], want[i].cpu()) < BOUND
+        assert bool((out[:, i * wide + N:(i + 1) * wide] == 7.0).all())   # columns behind the products
+    one = ops.linear_plain(x[:, :K], w[0], bias=b[0], act="silu", scale=0.5, out_dtype=torch.float32)
+    assert _err(one, 0.5 * torch.nn.functional.silu(want[0]).cpu()) < BOUND
+
+
+@pytest.mark.parametrize("channels", [(64, 64, 128), (5, 64, 33), (260, 512, 4), (128, 384)])
+@pytest.mark.parametrize("tokens", [1, 17, 1500])
+def test_convolutions_in_one_launch(channels, tokens):
+    """The same outputs and states as one call per input, with carried states and without."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    batch = ops.PackedBatch(_i32([0, tokens, 2 * tokens, 2 * tokens + 1]), _i32([0, 9, 3]), _i32([2, 0, 1]), tokens)
+    p = torch.randn(2 * tokens + 1, sum(channels) + 4, generator=g, device=DEV)
+    xs = p[:, :sum(channels)].split(list(channels), 1)
+    ws = [torch.randn(c, 4, generator=g, device=DEV).bfloat16() for c in channels]
+    states = [torch.randn(3, c, 3, generator=g, device=DEV) for c in channels]
+    alone = [s.clone() for s in states]
+    got = ops.causal_convs(batch, xs, ws, states).split(list(channels), 1)
+    for x, w, s, y, t in zip(xs, ws, alone, got, states):
+        want = ops.causal_conv(batch, x, w, s, out_dtype=torch.float32)
+        assert _err(y, want.cpu()) < BOUND and torch.equal(s, t)
+
+
 @pytest.mark.parametrize("H,dk,dv", [(2, 20, 24), (1, 128, 64), (3, 64, 65), (2, 100, 130), (1, 8, 7)])
 def test_linear_attention_all_chunks_at_once(monkeypatch, H, dk, dv):
     """Chunks of 64 tokens: portions of 64 (the walk), 65, 128, 130 and 1 token side by side, then a continuation of 66."""

@@ -1,6 +1,6 @@
 // vy_linear_plain: out = act(A W^T + bias) * scale + addend for any M, N, K and any alignment, fp32 accumulation.
-// Four kernels: for many rows 64 x 64 tiles on the tensor cores in fp32 precision where both operands are fp32, aligned and K is long, else
-// 64 x 64 x 16 shared-memory tiles of FMAs (4 x 4 outputs per thread); a weight-streaming kernel
+// Five kernels: for many rows 64 x 64 tiles on the tensor cores in fp32 precision where both operands are fp32, aligned and K is long, else
+// 64 x 64 x 16 shared-memory tiles of FMAs (4 x 4 outputs per thread) or, for K up to 32, weights in registers; a weight-streaming kernel
 // (one warp per output feature, lanes over K) for at most 8 rows, and a 32-feature tile for 9 .. 32 rows. A call may hold a batch
 // of independent products of one shape (blockIdx z / y picks the product). This is the exact-fp32 arm of every projection of the
 // sequence-mixer models and the bf16 arm of the shapes the tensor-core GEMM does not take (a contraction over a
@@ -30,7 +30,7 @@ struct LinDev {
   const void* addend; long long ld_addend; int addend_dt;
   int act; float scale;
   void* out; long long ld_out; int out_dt;
-  long long a_batch, w_batch, out_batch;   // element strides between the independent products of a batched call
+  long long a_batch, w_batch, out_batch, bias_batch;   // element strides between the independent products of a batched call
 };
 
 // product b of a batched call: the same shapes at shifted base pointers
@@ -39,6 +39,7 @@ __device__ __forceinline__ void lin_select(LinDev& d, int b) {
   d.A = static_cast<const char*>(d.A) + d.a_batch * b * (d.a_dt == VY_F32 ? 4 : 2);
   d.W = static_cast<const char*>(d.W) + d.w_batch * b * (d.w_dt == VY_F32 ? 4 : 2);
   d.out = static_cast<char*>(d.out) + d.out_batch * b * (d.out_dt == VY_F32 ? 4 : 2);
+  if (d.bias) d.bias = static_cast<const char*>(d.bias) + d.bias_batch * b * (d.bias_dt == VY_F32 ? 4 : 2);
 }
 
 __device__ __forceinline__ void lin_store(const LinDev& d, int m, int n, float acc) {
@@ -91,6 +92,66 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(LinDev d) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (m0 + tm + i < d.M && n0 + tn + j < d.N) lin_store(d, m0 + tm + i, n0 + tn + j, acc[i][j]);
+}
+
+// Contractions of up to 32 over many rows: bound by the bytes of the results. A thread keeps the weights of two neighbouring features in registers, rows of A come from shared memory
+// as broadcasts, results leave as pairs. The same sums in the same order as the tiles above. 7970 x 1024, K 16: 16 us, 30 in tiles
+// of 64 x 64 (four results per thread for 32 scalar loads); x 2048 27, 52.
+constexpr int LN_ROWS = 64, LN_K = 32;   // rows per CTA: half as many where CTAs would be too few
+template <int KP>
+__device__ __forceinline__ void thin_weights(const LinDev& d, int n, float (&w)[KP]) {
+  if (d.w_dt == VY_BF16 && d.K == KP && n < d.N && d.ldw % 8 == 0 && reinterpret_cast<uintptr_t>(d.W) % 16 == 0) {
+    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const char*>(d.W) + 2 * static_cast<long long>(n) * d.ldw);
+#pragma unroll
+    for (int i = 0; i < KP / 8; ++i) {
+      const uint4 v = p[i];
+      const unsigned u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        w[8 * i + 2 * j] = __uint_as_float(u[j] << 16);
+        w[8 * i + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < KP; ++k) w[k] = n < d.N && k < d.K ? ld_as_float(d.W, d.w_dt, static_cast<long long>(n) * d.ldw + k) : 0.f;
+}
+template <int KP>
+__global__ void __launch_bounds__(256) linear_thin_kernel(const __grid_constant__ LinDev d0, int per_cta) {
+  pdl_trigger();
+  pdl_wait();
+  LinDev d = d0;
+  lin_select(d, blockIdx.z);
+  __shared__ __align__(16) float as[LN_ROWS][KP];
+  const int m0 = blockIdx.y * per_cta, n = 2 * (blockIdx.x * 256 + threadIdx.x);
+  for (int e = threadIdx.x; e < per_cta * KP; e += 256) {
+    const int r = e / KP, k = e % KP;
+    as[r][k] = m0 + r < d.M && k < d.K ? ld_as_float(d.A, d.a_dt, static_cast<long long>(m0 + r) * d.lda + k) : 0.f;
+  }
+  float w[2][KP];
+  thin_weights(d, n, w[0]);
+  thin_weights(d, n + 1, w[1]);
+  const float b0 = d.bias && n < d.N ? ld_as_float(d.bias, d.bias_dt, n) : 0.f, b1 = d.bias && n + 1 < d.N ? ld_as_float(d.bias, d.bias_dt, n + 1) : 0.f;
+  __syncthreads();
+  if (n >= d.N) return;
+  const int rows = min(per_cta, d.M - m0);
+  float* out = static_cast<float*>(d.out) + static_cast<long long>(m0) * d.ld_out + n;
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r, out += d.ld_out) {
+    float y0 = 0.f, y1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < KP; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(&as[r][k]);
+      y0 = fmaf(x.x, w[0][k], y0); y0 = fmaf(x.y, w[0][k + 1], y0); y0 = fmaf(x.z, w[0][k + 2], y0); y0 = fmaf(x.w, w[0][k + 3], y0);
+      y1 = fmaf(x.x, w[1][k], y1); y1 = fmaf(x.y, w[1][k + 1], y1); y1 = fmaf(x.z, w[1][k + 2], y1); y1 = fmaf(x.w, w[1][k + 3], y1);
+    }
+    if (d.bias) { y0 += b0; y1 += b1; }
+    y0 = uact(y0, d.act) * d.scale;
+    y1 = uact(y1, d.act) * d.scale;
+    if (n + 1 < d.N) *reinterpret_cast<float2*>(out) = make_float2(y0, y1);
+    else *out = y0;
+  }
 }
 
 // One product in fp32 FMAs by a warp (16-byte aligned rows, K a multiple of 4), the sum in every lane
@@ -426,7 +487,7 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
   VY_CHECK_ARG(p->lda >= p->K && p->ldw >= p->K && p->ld_out >= p->N, "vy_linear_plain: leading dimension smaller than the row");
   VY_CHECK_ARG(p->act >= VY_UACT_NONE && p->act <= VY_UACT_GELU_TANH, "vy_linear_plain: bad act %d", p->act);
   const int batch = p->batch > 1 ? p->batch : 1;
-  VY_CHECK_ARG(batch <= 65535 && (batch == 1 || (!p->bias && !p->addend)), "vy_linear_plain: a batched call takes no bias / addend (batch %d)", batch);
+  VY_CHECK_ARG(batch <= 65535 && (batch == 1 || ((!p->bias || p->bias_batch > 0) && !p->addend)), "vy_linear_plain: a batched call takes no addend, a bias with its stride (batch %d)", batch);
   if (p->bias) VY_CHECK_ARG(dtype_ok(p->bias_dtype), "vy_linear_plain: bad bias_dtype");
   if (p->addend) VY_CHECK_ARG(dtype_ok(p->addend_dtype) && p->ld_addend >= p->N, "vy_linear_plain: bad addend");
   LinDev d;
@@ -437,7 +498,7 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
   d.addend = p->addend; d.ld_addend = p->ld_addend; d.addend_dt = p->addend_dtype;
   d.act = p->act; d.scale = p->scale == 0.f ? 1.f : p->scale;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
-  d.a_batch = p->a_batch; d.w_batch = p->w_batch; d.out_batch = p->out_batch;
+  d.a_batch = p->a_batch; d.w_batch = p->w_batch; d.out_batch = p->out_batch; d.bias_batch = p->bias_batch;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   if (p->M <= 8) {
     VY_CUDA_OK(launch_kernel(linear_rows_kernel, dim3((p->N + 7) / 8, batch), dim3(256), 0, st, d));
@@ -452,6 +513,17 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
       static std::atomic<unsigned long long> allowed{0};
       VY_CUDA_OK(allow_smem(linear_split_kernel, allowed));
       VY_CUDA_OK(launch_kernel(linear_split_kernel, dim3((p->N + LT - 1) / LT, (p->M + LT - 1) / LT, batch), dim3(256), 2 * LS_BUF, st, d));
+      VY_LAUNCH_OK();
+      count_launch();
+      return VY_OK;
+    }
+    // K up to 32, fp32 results in pairs. A CTA has 512 features: 128 of them, 7970 rows 7.2 us in tiles, 7.9 here; 512 16.9, 9.7; 33 x 512 5.8, 5.0; 2000 x 2048, K 32 22.3, 14.2
+    if (p->K <= LN_K && p->N >= 256 && !d.addend && d.out_dt == VY_F32 && reinterpret_cast<uintptr_t>(d.out) % 8 == 0 && d.ld_out % 2 == 0 && (batch == 1 || d.out_batch % 2 == 0) &&
+        p->M <= 65535 * (LN_ROWS / 4)) {
+      const long long wide = (p->N + 511LL) / 512 * batch;
+      const int per_cta = wide * (p->M / LN_ROWS) >= num_sms() ? LN_ROWS : wide * (2 * p->M / LN_ROWS) >= num_sms() ? LN_ROWS / 2 : LN_ROWS / 4;
+      const dim3 grid((p->N + 511) / 512, (p->M + per_cta - 1) / per_cta, batch);
+      VY_CUDA_OK(p->K <= 16 ? launch_kernel(linear_thin_kernel<16>, grid, dim3(256), 0, st, d, per_cta) : launch_kernel(linear_thin_kernel<32>, grid, dim3(256), 0, st, d, per_cta));
       VY_LAUNCH_OK();
       count_launch();
       return VY_OK;

@@ -8,6 +8,8 @@
 
 #include <type_traits>
 
+#include <limits.h>
+
 #include "seqmix.cuh"
 
 namespace vy {
@@ -506,6 +508,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_attn_decode_kernel(WinDe
 }
 
 // ---- causal depthwise convolution with carried taps ------------------------------------------------------------------
+struct ConvPart { const void* x; const void* w; float* state; int channels; };
 struct ConvDev {
   const int* cu; const int* pos0; const int* slot;
   int channels, taps;
@@ -515,7 +518,24 @@ struct ConvDev {
   int act;
   void* out; long long ld_out; int out_dt;
   int first;   // first channel of the launch
+  int total;   // channels of all parts; those behind the first part's belong to `more`
+  ConvPart more[2];
 };
+// the part that channel c of the launch belongs to takes the first one's place; c becomes a channel of it
+__device__ __forceinline__ void conv_select(ConvDev& d, const ConvDev& all, int& c) {
+  if (c < d.channels) return;
+  int at = d.channels;
+  const bool last = c - at >= all.more[0].channels;
+  if (last) at += all.more[0].channels;
+  const ConvPart& p = all.more[last];
+  d.x = p.x;
+  d.w = p.w;
+  d.state = p.state;
+  d.channels = p.channels;
+  d.out = static_cast<char*>(d.out) + static_cast<long long>(at) * (d.out_dt == VY_F32 ? 4 : 2);
+  c -= at;
+}
+
 constexpr int CONV_MAX_TAPS = 16;
 constexpr int CONV_TOK = 16;   // at least CONV_MAX_TAPS - 1: only the first CTA row of a sequence reaches back to the slot's taps
 
@@ -539,13 +559,15 @@ __device__ __forceinline__ void conv_new_taps(const ConvDev& d, int c, int base,
 // 8192 tokens x 1024 channels 65.5 / 31.8 us, x 512 40.4 / 17.4 us, 80 tokens x 512 31.1 / 7.3 us. The first CTA column of a sequence, the only
 // one that reads the slot's old taps, writes the new ones (a launch of its own before, 2.2 us). TAPS >= taps
 template <int TAPS>
-__global__ void __launch_bounds__(128) causal_conv_kernel(ConvDev d) {
+__global__ void __launch_bounds__(128) causal_conv_kernel(const __grid_constant__ ConvDev all) {
   pdl_trigger();
   pdl_wait();
-  const int c = d.first + blockIdx.y * blockDim.x + threadIdx.x;
+  ConvDev d = all;
+  int c = d.first + blockIdx.y * blockDim.x + threadIdx.x;
   const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (c >= d.channels || i0 >= n) return;
+  if (c >= d.total || i0 >= n) return;
+  conv_select(d, all, c);
   const bool carried = d.pos0[s] > 0;
   float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
   float x[CONV_TOK + TAPS - 1], w[TAPS];
@@ -575,14 +597,16 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(ConvDev d) {
 
 // The same for four neighbouring channels per thread (fp32 rows on 16-byte boundaries, up to 4 taps): a quarter of the loads, stores and addresses per output,
 // and the SiLU without a division. Bound by the bytes and the exponentials: 7970 tokens x 1024 channels 30.1 us with one channel per thread, 18.1 here; x 512 16.7, 11.6.
-__global__ void __launch_bounds__(128) causal_conv_quads_kernel(ConvDev d) {
+__global__ void __launch_bounds__(128) causal_conv_quads_kernel(const __grid_constant__ ConvDev all) {
   pdl_trigger();
   pdl_wait();
   constexpr int TAPS = 4;
-  const int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+  ConvDev d = all;
+  int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
   const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
   const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (c >= d.channels || i0 >= n) return;
+  if (c >= d.total || i0 >= n) return;
+  conv_select(d, all, c);
   const bool carried = d.pos0[s] > 0;
   float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
   const float* xp = reinterpret_cast<const float*>(d.x) + static_cast<long long>(base) * d.ldx + c;
@@ -1071,6 +1095,9 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   VY_CHECK_ARG(p->x && p->w && p->out && p->x != p->out && (p->state || p->taps == 1) && dtype_ok(p->x_dtype) && dtype_ok(p->w_dtype) &&
                    dtype_ok(p->out_dtype), "vy_causal_conv: bad tensors");
   VY_CHECK_ARG((p->max_new + 31) / 32 <= 65535, "vy_causal_conv: too many tokens per sequence");
+  VY_CHECK_ARG(p->channels2 >= 0 && p->channels3 >= 0 && (p->channels2 > 0 || p->channels3 == 0) && static_cast<long long>(p->channels) + p->channels2 + p->channels3 <= INT_MAX &&
+                   (p->channels2 == 0 || (p->x2 && p->w2 && p->x2 != p->out && (p->state2 || p->taps == 1))) &&
+                   (p->channels3 == 0 || (p->x3 && p->w3 && p->x3 != p->out && (p->state3 || p->taps == 1))), "vy_causal_conv: bad further inputs");
   ConvDev d;
   d.cu = p->cu_tokens; d.pos0 = p->pos0; d.slot = p->slot;
   d.channels = p->channels; d.taps = p->taps;
@@ -1078,22 +1105,27 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   d.w = p->w; d.w_dt = p->w_dtype;
   d.state = p->state; d.act = p->act;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
+  d.more[0] = {p->x2, p->w2, p->state2, p->channels2};
+  d.more[1] = {p->x3, p->w3, p->state3, p->channels3};
+  d.total = p->channels + p->channels2 + p->channels3;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   const auto quads = [](const void* q, int dt, long long ld) { return dt == VY_F32 && reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0; };
   // Four channels per thread from two CTAs per SM on that find tokens: 1024 channels x 1200, 2080, 4160 tokens 8.9 / 10.1, 12.3 / 11.7, 19.7 / 13.9 us (a channel per thread / four);
   // 3000 x 512, 768 9.6 / 10.7, 11.9 / 10.9; or from ten on that find some or none, which in either form bound uneven portions: one of 300 beside 7 of 20, 1024 channels, 8.2 / 10.3,
   // one of 512 beside 31 single tokens 11.3 / 9.7 (of which 256 channels 7.8 / 9.5)
   const long long tiles = static_cast<long long>(p->n_seqs) * ((p->max_new + CONV_TOK - 1) / CONV_TOK), filled = p->rows > 0 ? (p->rows + CONV_TOK - 1) / CONV_TOK : tiles;
-  if ((filled * p->channels >= 2LL * 512 * num_sms() || tiles * p->channels >= 10LL * 512 * num_sms()) && p->taps <= 4 && p->channels % 4 == 0 &&
-      p->channels <= 65535 * 512 && quads(d.x, d.x_dt, d.ldx) && quads(d.out, d.out_dt, d.ld_out)) {
+  // Further inputs count with the first: 512, 512 and 1024 channels of 4 x 2048 tokens one after the other 17.8, 11.8 and 20.8 us, together 39
+  bool aligned = p->taps <= 4 && p->channels % 4 == 0 && quads(d.x, d.x_dt, d.ldx) && quads(d.out, d.out_dt, d.ld_out);
+  for (const ConvPart& m : d.more) aligned = aligned && (m.channels == 0 || (m.channels % 4 == 0 && quads(m.x, d.x_dt, d.ldx)));
+  if ((filled * d.total >= 2LL * 512 * num_sms() || tiles * d.total >= 10LL * 512 * num_sms()) && aligned && d.total <= 65535 * 512) {
     d.first = 0;
-    const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, (p->channels + 511) / 512, p->n_seqs);
+    const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, (d.total + 511) / 512, p->n_seqs);
     VY_CUDA_OK(launch_kernel(causal_conv_quads_kernel, grid, dim3(128), 0, st, d));
     VY_LAUNCH_OK();
     count_launch();
     return VY_OK;
   }
-  const long long blocks = (p->channels + 127LL) / 128;
+  const long long blocks = (d.total + 127LL) / 128;
   for (long long b = 0; b < blocks; b += 65535) {   // one launch, up to 8 million channels
     d.first = static_cast<int>(128 * b);
     const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, static_cast<unsigned>(blocks - b < 65535 ? blocks - b : 65535), p->n_seqs);

@@ -939,18 +939,20 @@ def _rows2d(t: torch.Tensor, what: str) -> None:
         raise _lib.VyomError(f"{what}: expected a 2-d tensor with unit column stride, got shape {tuple(t.shape)} strides {t.stride()}")
 
 
-def head_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, x_head: int, out_head: int) -> torch.Tensor:
+def head_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, x_head: int, out_head: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """One launch of `heads` independent products with fp32 FMA accumulation: w is [heads, N, K]; head h reads x[:, h * x_head : h * x_head + K]
-    and writes out[:, h * out_head : h * out_head + N]."""
-    _need_cuda(x, w, out)
+    and writes out[:, h * out_head : h * out_head + N], plus its row of `bias` [heads, N]."""
+    _need_cuda(x, w, out, bias)
     _rows2d(x, "head_linear x")
     _rows2d(out, "head_linear out")
     heads, N, K = w.shape
     if not w.is_contiguous() or (heads - 1) * x_head + K > x.shape[1] or (heads - 1) * out_head + N > out.shape[1]:
         raise _lib.VyomError("head_linear: weight layout / head strides do not fit the operands")
+    if bias is not None and (bias.shape != (heads, N) or not bias.is_contiguous()):
+        raise _lib.VyomError("head_linear: bias is [heads, N]")
     _lib.call("vy_linear_plain", "VyLinear", M=x.shape[0], N=N, K=K, A=x.data_ptr(), lda=x.stride(0), a_dtype=_dt(x), W=w.data_ptr(), ldw=K,
               w_dtype=_dt(w), act=UACT[None], scale=1.0, out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out), batch=heads, a_batch=x_head,
-              w_batch=N * K, out_batch=out_head, stream=_stream())
+              w_batch=N * K, out_batch=out_head, bias=_ptr(bias), bias_dtype=_dt(bias) if bias is not None else 0, bias_batch=N, stream=_stream())
     return out
 
 
@@ -1458,6 +1460,24 @@ def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: tor
     _lib.call("vy_causal_conv", "VyCausalConv", channels=ch, taps=taps, x=x.data_ptr(), ldx=x.stride(0), x_dtype=_dt(x), w=w.data_ptr(),
               w_dtype=_dt(w), state=state.data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
               stream=_stream(), rows=x.shape[0], **batch._kw())
+    return out
+
+
+def causal_convs(batch: PackedBatch, xs, ws, states, act: Optional[str] = "silu") -> torch.Tensor:
+    """`causal_conv` of two or three inputs in one launch: rows of one stride, one dtype, weights of one dtype and as many taps. The fp32 outputs stand side by side in one tensor."""
+    _need_cuda(*xs, *ws, *states)
+    taps = ws[0].shape[1]
+    for x, w, state in zip(xs, ws, states):
+        _rows2d(x, "causal_convs x")
+        if x.shape != (xs[0].shape[0], w.shape[0]) or w.shape[1] != taps or not w.is_contiguous() or w.dtype != ws[0].dtype or x.dtype != xs[0].dtype or x.stride(0) != xs[0].stride(0) \
+                or state.dtype != torch.float32 or not state.is_contiguous():
+            raise _lib.VyomError("causal_convs: shapes / layout")
+    ch = [w.shape[0] for w in ws]
+    out = torch.empty((xs[0].shape[0], sum(ch)), device=xs[0].device, dtype=torch.float32)
+    third = dict(channels3=ch[2], x3=xs[2].data_ptr(), w3=ws[2].data_ptr(), state3=states[2].data_ptr()) if len(ch) > 2 else {}
+    _lib.call("vy_causal_conv", "VyCausalConv", channels=ch[0], taps=taps, x=xs[0].data_ptr(), ldx=xs[0].stride(0), x_dtype=_dt(xs[0]), w=ws[0].data_ptr(),
+              w_dtype=_dt(ws[0]), state=states[0].data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
+              stream=_stream(), rows=xs[0].shape[0], channels2=ch[1], x2=xs[1].data_ptr(), w2=ws[1].data_ptr(), state2=states[1].data_ptr(), **third, **batch._kw())
     return out
 
 
