@@ -1075,6 +1075,26 @@ typedef struct VyMoeCombine {
 } VyMoeCombine;
 VY_API int vy_moe_combine(const VyMoeCombine* p);
 
+/* The sorted form as one call, for SwiGLU experts in bf16 on the tensor cores, without a host decision: the routed rows are copied together by expert, each expert's rows padded to
+ * whole tiles of 128, and both products run over the tiles of all experts. A shared expert (shared_ff a multiple of ff) is more tiles of the same launches.
+ *   out[row, :] = sum_k weight[row, k] * expert_idx[row, k](h[row, :]) + s * shared(h[row, :]),   s = shared_gate ? sigmoid(shared_gate[row * ld_gate]) : 1
+ * Experts' hidden rows are bf16, their results and the sum (in the order k = 0 .., the shared expert last) fp32. Pairs with idx >= experts are left out (identity experts).
+ * up: [experts * 2 ff + 2 shared_ff, width], gate and up rows interleaved; down: [width, experts * ff + shared_ff]. width and ff are multiples of 8, rows 16-byte aligned.
+ * workspace: 128-byte aligned, vy_moe_grouped_bytes(..) bytes (0: the call does not apply to these shapes). */
+typedef struct VyMoeGrouped {
+  int32_t rows, experts, top, width, ff, shared_ff;
+  const int32_t* idx; const float* weight;
+  const void* h; int64_t ldh;
+  const void* up; int64_t ld_up;
+  const void* down; int64_t ld_down;
+  const float* shared_gate; int64_t ld_gate;
+  float* out; int64_t ld_out;
+  void* workspace; int64_t workspace_bytes;
+  void* stream;
+} VyMoeGrouped;
+VY_API int64_t vy_moe_grouped_bytes(int32_t rows, int32_t experts, int32_t top, int32_t width, int32_t ff, int32_t shared_ff);
+VY_API int vy_moe_grouped(const VyMoeGrouped* p);
+
 /* Gated experts: hidden activations of all experts at once, h [rows, experts * 2 ff + 2 shared_ff], expert e's block being
  * [gate (ff) | up (ff)], the shared expert's [gate (shared_ff) | up (shared_ff)] last:
  *   g = min(gate, limit), u = clamp(up, -limit, limit), y = g * sigmoid(alpha * g) * (u + 1)        (fp32)

@@ -253,6 +253,45 @@ def _experts(f, width, dtype, seed=11, **kw):
     return m, {k: v.double() for k, v in w.items()}
 
 
+@pytest.mark.parametrize("rows,experts,identity,top,ff,shared,width", [(128, 5, 2, 3, 8, 0, 64), (129, 3, 0, 1, 72, 72, 136), (300, 40, 8, 9, 64, 128, 200), (33, 256, 0, 4, 16, 48, 1024),
+                                                                      (1, 2, 0, 2, 128, 0, 8), (700, 2, 1, 2, 136, 272, 264)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_grouped_experts(rows, experts, identity, top, ff, shared, width, gated):
+    """Experts on their own rows in tiles of 128: full tiles and remainders, experts without rows, widths and contractions that no tile divides, a shared expert of one and of several segments."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(rows + ff)
+    bf = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=DEV) * std).bfloat16()  # noqa: E731
+    h, up, down = bf(rows, width), bf(experts * 2 * ff + 2 * shared, width, std=width ** -0.5), bf(width, experts * ff + shared, std=ff ** -0.5)
+    score = torch.rand(rows, experts + identity, generator=g, device=DEV)
+    score[:, 1:2] -= 2.0   # an expert that hardly anyone takes
+    idx = score.topk(top, 1).indices.to(torch.int32)
+    weight = torch.rand(rows, top, generator=g, device=DEV)
+    z = torch.randn(rows, 3, generator=g, device=DEV)[:, 1:2] if gated and shared else None
+    need = ops.moe_grouped_bytes(rows, experts, top, width, ff, shared)
+    run = lambda: ops.moe_grouped(h, idx, weight, up, down, experts=experts, ff=ff, shared_ff=shared, shared_gate=z, workspace=torch.full((need,), 255, dtype=torch.uint8, device=DEV))  # noqa: E731
+    got = run()   # the workspace holds NaN: rows that fill up tiles meet no other row
+    def expert(x, u, w):
+        a = x.double() @ u.double().T
+        hid = (torch.nn.functional.silu(a[:, 0::2]) * a[:, 1::2]).to(torch.bfloat16)
+        return hid.double() @ w.double().T
+    want = torch.zeros(rows, width, dtype=torch.float64, device=DEV)
+    for e in range(experts):
+        r, k = (idx == e).nonzero(as_tuple=True)
+        if len(r):
+            want.index_add_(0, r, weight[r, k].double()[:, None] * expert(h[r], up[e * 2 * ff:(e + 1) * 2 * ff], down[:, e * ff:(e + 1) * ff]))
+    if shared:
+        want += (torch.sigmoid(z.double()) if z is not None else 1.0) * expert(h, up[experts * 2 * ff:], down[:, experts * ff:])
+    # a hidden entry that lies at the middle between two bf16 numbers may round the other way: fp32 sums move one in a few thousand by 2^-8 of itself
+    assert float((got.double() - want).norm() / want.norm()) < 5e-4
+    assert torch.equal(got, run())
+
+
+def test_grouped_experts_refuse_what_they_do_not_take():
+    from vyomai_b200 import ops
+    assert ops.moe_grouped_bytes(128, 4, 2, 64, 12, 0) == 0 and ops.moe_grouped_bytes(128, 4, 2, 60, 16, 0) == 0 and ops.moe_grouped_bytes(128, 4, 2, 64, 16, 24) == 0
+    assert ops.moe_grouped_bytes(128, 257, 2, 64, 16, 0) == 0 and ops.moe_grouped_bytes(1 << 22, 8, 8, 64, 16, 0) == 0 and ops.moe_grouped_bytes(128, 4, 2, 64, 16, 32) > 0
+
+
 @pytest.mark.parametrize("rows", [1, 5, 40, 150])
 @pytest.mark.parametrize("f,width,dtype", [(U.moe(), 40, torch.float32), (U.moe(identity=None, shared=None), 40, torch.float32), (U.moe(experts=1, top=2, identity=1), 24, torch.float32),
                                            (U.moe(ff=64, experts=6, top=3, identity=2, shared=96), 128, torch.bfloat16), (U.moe(ff=20, experts=3, top=2, shared=12), 64, torch.bfloat16)])

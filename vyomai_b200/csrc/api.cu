@@ -219,6 +219,7 @@ int vy_abi_sizeof(const char* name) {
   VY_SZ(VyMoeSort);
   VY_SZ(VyMoeGather);
   VY_SZ(VyMoeCombine);
+  VY_SZ(VyMoeGrouped);
   VY_SZ(VyPolyNorm);
   VY_SZ(VyGatedDelta);
   VY_SZ(VySandwichNorm);

@@ -56,6 +56,11 @@ struct GemmDev {
   float* ws;
   PoisonRef poison;  // raised by a wait that timed out (mbar_wait_soft); the host sees it in vy_gemm / vy_gemm_poison_peek / vy_gemm_poisoned
   int tma_store;  // fast epilogues write back with TMA stores (tma_out / tma_aux of the launch)
+  // products of groups (WB_*_GROUPED): the m-tiles of the launch, {row of A, row of the result, row of B / its first k, segments of k}, their number; a segment's k are seg_k entries of B's
+  // rows and the first seg_k of A's rows, seg_rows further down for each segment
+  const int4* groups;
+  const int* group_count;
+  int seg_k, seg_rows;
   int debug;  // development switches (VY_GEMM_DEBUG): 1 = epilogue drains TMEM only, 2 = producer skips TMA after the first ring fill
 };
 
@@ -941,9 +946,9 @@ __device__ __forceinline__ void epilogue_qkv_rope(const GemmDev& g, uint32_t tme
 // kernel
 // --------------------------------------------------------------------------------------------
 // WB: the write-backs that the kernel holds: WB_ANY all but the two that follow, WB_GATED the staged SwiGLU one alone (epilogue_swiglu_fast),
-// WB_F32 the staged fp32 one alone (epilogue_f32_fast). They are instantiations of their own so that the register allocation of the other
+// WB_F32 the staged fp32 one alone (epilogue_f32_fast), the last two the same for the products of groups (moe_grouped.cu). They are instantiations of their own so that the register allocation of the other
 // epilogues does not change with them (inlined next to them SwiGLU cost the split-K / plain paths a few spills and ~5 % on the weight-gradient GEMMs).
-enum { WB_ANY = 0, WB_GATED = 1, WB_F32 = 2 };
+enum { WB_ANY = 0, WB_GATED = 1, WB_F32 = 2, WB_GATED_GROUPED = 3, WB_F32_GROUPED = 4 };
 template <typename TIn, int BN, bool A_MN, bool B_MN, bool PAIR, int WB = WB_ANY>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -956,6 +961,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   constexpr int STAGES = PAIR ? Cfg::PAIR_STAGES : Cfg::STAGES;
   constexpr int B_BYTES = PAIR ? Cfg::PAIR_B_BYTES : Cfg::B_BYTES;      // this CTA's part of the B tile
   constexpr int STAGE_BYTES = Cfg::A_BYTES + B_BYTES;
+  constexpr bool GROUPED = WB == WB_GATED_GROUPED || WB == WB_F32_GROUPED;
+  static_assert(!GROUPED || (!PAIR && !A_MN && !B_MN), "products of groups: K-major operands, one CTA per tile");
   constexpr int BN_CTA = PAIR ? BN / 2 : BN;                            // B rows (output columns) staged by this CTA
   static_assert(!PAIR || !B_MN || BN_CTA % Cfg::EPB == 0, "an MN-major B half must be whole swizzle boxes");
   static_assert(!PAIR || BN % 16 == 0, "cta_group::2 MMAs take N in steps of 16");
@@ -997,9 +1004,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   const int m_slots = PAIR ? (m_tiles + 1) / 2 : m_tiles;
   const int m_mul = PAIR ? 2 : 1;
   const int n_tiles = (g.N + BN - 1) / BN;
-  const int num_tiles = m_slots * n_tiles;
-  const int num_kb = (g.K + BK - 1) / BK;
-  const int num_units = num_tiles * g.k_splits;
+  int num_tiles = m_slots * n_tiles;
+  const int num_kb = ((GROUPED ? g.seg_k : g.K) + BK - 1) / BK;   // of a segment where there are groups
+  int num_units = num_tiles * g.k_splits;
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tma_a);
@@ -1035,6 +1042,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_s;
   pdl_wait();  // everything above is independent of the predecessor grid's output
+  if constexpr (GROUPED) num_units = num_tiles = *g.group_count * n_tiles;
 
   if (warp == 0) {
     // ===================== TMA producer (whole warp, one elected lane issues) =====================
@@ -1042,6 +1050,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       uint32_t it = 0, s = 0, ph = 0;  // k-blocks issued, ring position and its phase bit
       for (int unit = worker; unit < num_units; unit += nworkers) {
         const int tile = unit % num_tiles;
+        if constexpr (GROUPED) {
+          const int4 grp = g.groups[tile / n_tiles];
+          const int n0 = (tile % n_tiles) * BN;
+          constexpr bool BY_ROW = WB == WB_GATED_GROUPED;   // a group's share of B: rows, or a run of k
+          for (int seg = 0; seg < grp.w; ++seg)
+            for (int kb = 0; kb < num_kb; ++kb, ph ^= (s + 1 == STAGES), s = (s + 1 == STAGES) ? 0 : s + 1) {
+              mbar_wait_soft(&empty_bar[s], ph ^ 1, g.poison);
+              if (elect_one_sync()) {
+                mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
+                tma_load_2d(sA + s * Cfg::A_BYTES, &tma_a, &full_bar[s], kb * BK, grp.x + seg * g.seg_rows);
+                tma_load_2d(sB + s * B_BYTES, &tma_b, &full_bar[s], kb * BK + (BY_ROW ? 0 : grp.z + seg * g.seg_k), n0 + (BY_ROW ? grp.z : 0));
+              }
+              __syncwarp();
+            }
+          continue;
+        }
         const int m0 = ((tile / n_tiles) * m_mul + rank) * BM;  // may lie beyond M for the odd m-tile of the last pair: TMA zero-fills
         const int n0 = (tile % n_tiles) * BN + rank * BN_CTA;   // first B row this CTA stages
         const int kb0 = (unit / num_tiles) * g.kb_per_split;
@@ -1114,7 +1138,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       uint32_t local = 0;
       for (int unit = worker; unit < num_units; unit += nworkers, ++local) {
         const int kb0 = (unit / num_tiles) * g.kb_per_split;
-        const int nkb = min(num_kb, kb0 + g.kb_per_split) - kb0;
+        const int nkb = GROUPED ? g.groups[unit / n_tiles].w * num_kb : min(num_kb, kb0 + g.kb_per_split) - kb0;
         const uint32_t acc = local & 1;
         const uint32_t acc_ph = (local >> 1) & 1;
         VY_TRACE(1, local, 0);
@@ -1182,7 +1206,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       const int tile = unit % num_tiles;
       const uint32_t acc = local & 1;
       const uint32_t acc_ph = (local >> 1) & 1;
-      const int m0 = ((tile / n_tiles) * m_mul + rank) * BM;
+      const int m0 = GROUPED ? g.groups[tile / n_tiles].y : ((tile / n_tiles) * m_mul + rank) * BM;
       const int n0 = (tile % n_tiles) * BN;
       float* bs = bias_s + acc * BN;
       // where this warp announces that it has drained the accumulator: the (leader's) MMA thread waits there
@@ -1196,11 +1220,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         named_bar_sync(1, GEMM_EPI_WARPS * 32);
       }
       const uint32_t tmem_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      if constexpr (WB == WB_GATED) {
+      if constexpr (WB == WB_GATED || WB == WB_GATED_GROUPED) {
         epilogue_swiglu_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e, &tma_out);
         continue;
       }
-      if constexpr (WB == WB_F32) {
+      if constexpr (WB == WB_F32 || WB == WB_F32_GROUPED) {
         epilogue_f32_fast<BN>(g, tmem_acc, m0, n0, q, half, lane, &tfull_bar[acc], acc_ph, tempty_addr, stage, turns + e, &tma_out);
         continue;
       }

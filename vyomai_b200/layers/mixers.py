@@ -782,14 +782,15 @@ class MoEFeedForward:
     interleaved so that the product's epilogue can do it. The shared expert is weighted by sigmoid(w_sg . h) when the
     weights hold `shared.sg`, by 1 otherwise.
 
-    Two exact forms of the same sum. Single tokens and short steps (also every CUDA-graph-captured step: no host decision)
+    Three exact forms of the same sum. Single tokens and short steps (also every CUDA-graph-captured step: no host decision)
     run ALL experts as two products over the concatenated experts, the hidden activations multiplied by each token's routing
     weight (0 for the experts it did not choose) in between: the weights are read once, as a decode step would anyway.
     Prompt-sized steps sort the (token, choice) pairs by expert on the device, gather the rows, run each expert's two products
     on its own rows, and combine per token in choice order (no atomics, so the result does not depend on the batch). The sorted
     form costs two launches per expert and one host read of the experts' row counts, the all-experts form experts / top times
     the multiply-adds: a step of at least `sorted_min_rows` rows takes the sorted form when its estimated time is the smaller one
-    (`force_sorted` skips the estimate)."""
+    (`force_sorted` skips the estimate). SwiGLU experts in bf16 take the grouped form instead from `sorted_min_rows` rows on (from 33 on where the width is 1024 or more): the same
+    rows in five launches for all experts, without the host's read."""
 
     # multiply-add rates the estimate assumes for bf16 tensor-core products, fp32 ones on the tensor cores (vy_linear_plain, contractions of 256 and more) and FMA
     # ones (FLOP/s)
@@ -854,6 +855,17 @@ class MoEFeedForward:
         moved = 3.0 * rows * self.top * width * 4 / 2.0e12   # gather, per-pair results, combine
         return self.top * per_choice + launches * self.LAUNCH_COST + moved < self.experts * per_choice
 
+    def _grouped_workspace(self, h: torch.Tensor, batch) -> Optional[torch.Tensor]:
+        """Scratch for the grouped form, or None where it does not apply or is not the fastest. Device us of all experts / grouped, 28 experts of width / 4 and a shared one of width / 2, top 4:
+        width 512 100 rows 42 / 46, 130 42 / 43, 500 48 / 45, 4000 103 / 91; 1024 40 rows 58 / 47, 500 72 / 54, 4000 210 / 136; 2048 40 rows 99 / 88, 500 142 / 97, 2000 318 / 158."""
+        rows = h.shape[0]
+        enough = rows >= self.sorted_min_rows or (32 < rows and h.shape[1] >= 1024 and self.sorted_min_rows <= 128)
+        if not (self.swiglu and not self.force_sorted and batch.max_new > 1 and enough and h.dtype == torch.bfloat16 and self.act_dtype == torch.bfloat16
+                and self.up_all.tensor_cores and self.down_all.tensor_cores and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0):
+            return None
+        need = ops.moe_grouped_bytes(rows, self.experts, self.top, h.shape[1], self.ff, self.shared_ff)
+        return ops._lend((need + 3) // 4, h.device)
+
     def _hidden(self, proj: Projection, x: torch.Tensor, dense: Optional[torch.Tensor], experts: int, shared_ff: int, sg, wide: bool) -> torch.Tensor:
         """The activated (and, with `dense`, weighted) hidden rows of `experts` experts and / or the shared expert, in the activation dtype."""
         if self.swiglu:
@@ -886,11 +898,14 @@ class MoEFeedForward:
         E, rows = self.experts, h.shape[0]
         z = logits if logits is not None else self.router(h)
         scored = E + self.identity
-        sorted_form = batch.max_new > 1 and rows >= self.sorted_min_rows and (self.force_sorted or self._sorted_is_faster(rows))
-        idx, wt, dense, *rest = ops.moe_route(z, scored, self.top, self.route_scale, dense=not sorted_form, kind=self.router_kind, groups=self.groups,
+        grouped = self._grouped_workspace(h, batch)
+        sorted_form = grouped is None and batch.max_new > 1 and rows >= self.sorted_min_rows and (self.force_sorted or self._sorted_is_faster(rows))
+        idx, wt, dense, *rest = ops.moe_route(z, scored, self.top, self.route_scale, dense=grouped is None and not sorted_form, kind=self.router_kind, groups=self.groups,
                                               keep_groups=self.keep_groups, normalize=self.normalize, correction=self.correction, identity=self.identity)
         ident = rest[0] if rest else None
         sg = z[:, scored:scored + 1] if self.shared_gated else None
+        if grouped is not None:
+            return ops.moe_grouped(h, idx, wt, self.up_all.weight, self.down_all.weight, experts=E, ff=self.ff, shared_ff=self.shared_ff, shared_gate=sg, workspace=grouped), ident
         if not sorted_form:
             # few rows: fp32 hidden activations, weighted, rounded once. Prompt-sized steps write them in the activation dtype from
             # the product's epilogue and weight them in place (half the bytes of the step's largest tensor, one more rounding)

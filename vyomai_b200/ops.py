@@ -1432,6 +1432,32 @@ def moe_gather(x: torch.Tensor, perm: torch.Tensor, top: int, out_dtype: torch.d
     return out
 
 
+def moe_grouped_bytes(rows: int, experts: int, top: int, width: int, ff: int, shared_ff: int) -> int:
+    """Scratch of `moe_grouped` (0: it does not apply to these shapes)."""
+    return int(_lib.lib().vy_moe_grouped_bytes(rows, experts, top, width, ff, shared_ff))
+
+
+def moe_grouped(h: torch.Tensor, idx: torch.Tensor, weight: torch.Tensor, up: torch.Tensor, down: torch.Tensor, *, experts: int, ff: int, shared_ff: int = 0,
+                shared_gate: Optional[torch.Tensor] = None, workspace: torch.Tensor) -> torch.Tensor:
+    """SwiGLU experts on the rows that are routed to them, weighted and summed in fp32, plus the shared expert (times sigmoid(shared_gate)): h [rows, width] bf16, idx / weight [rows, top],
+    up [experts * 2 ff + 2 shared_ff, width] with interleaved gate / up rows, down [width, experts * ff + shared_ff]; pairs with idx >= experts are left out."""
+    _need_cuda(h, idx, weight, up, down, shared_gate, workspace)
+    rows, width = h.shape
+    for t, n in ((h, "h"), (up, "up"), (down, "down")):
+        _rows2d(t, f"moe_grouped {n}")
+    if not (h.dtype == up.dtype == down.dtype == torch.bfloat16) or up.shape != (experts * 2 * ff + 2 * shared_ff, width) or down.shape != (width, experts * ff + shared_ff):
+        raise _lib.VyomError("moe_grouped: operands are bf16, up [experts * 2 ff + 2 shared_ff, width], down [width, experts * ff + shared_ff]")
+    if idx.shape != weight.shape or idx.shape[0] != rows or not idx.is_contiguous() or not weight.is_contiguous() or idx.dtype != torch.int32 or weight.dtype != torch.float32 \
+            or (shared_gate is not None and (shared_gate.dtype != torch.float32 or shared_gate.shape[0] != rows)):
+        raise _lib.VyomError("moe_grouped: idx int32 and weight fp32 [rows, top], shared_gate fp32 [rows, 1]")
+    out = torch.empty((rows, width), device=h.device, dtype=torch.float32)
+    _lib.call("vy_moe_grouped", "VyMoeGrouped", rows=rows, experts=experts, top=idx.shape[1], width=width, ff=ff, shared_ff=shared_ff, idx=idx.data_ptr(), weight=weight.data_ptr(),
+              h=h.data_ptr(), ldh=h.stride(0), up=up.data_ptr(), ld_up=up.stride(0), down=down.data_ptr(), ld_down=down.stride(0), shared_gate=_ptr(shared_gate),
+              ld_gate=shared_gate.stride(0) if shared_gate is not None else 0, out=out.data_ptr(), ld_out=out.stride(0), workspace=workspace.data_ptr(),
+              workspace_bytes=workspace.numel() * workspace.element_size(), stream=_stream())
+    return out
+
+
 def moe_combine(part: torch.Tensor, inv: torch.Tensor, weight: torch.Tensor, addend: Optional[torch.Tensor] = None, idx: Optional[torch.Tensor] = None,
                 routed: int = 0) -> torch.Tensor:
     """out[row] = addend[row] + sum_k weight[row, k] * part[inv[row * top + k]] (fp32); with idx [rows, top] the pairs whose expert is
