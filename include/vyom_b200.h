@@ -650,7 +650,11 @@ typedef struct VyLinear {
   int32_t batch; int64_t a_batch, w_batch, out_batch;
   void* stream;
   int64_t bias_batch;
+  /* optional scratch, 128-byte aligned, of vy_linear_plain_bytes(M, N, K) bytes (0: none needed): one product of fp32 operands with 16-byte aligned rows then has both split into
+   * 16-bit halves once, in place of every tile doing so */
+  void* workspace; int64_t workspace_bytes;
 } VyLinear;
+VY_API int64_t vy_linear_plain_bytes(int32_t M, int32_t N, int32_t K);
 VY_API int vy_linear_plain(const VyLinear* p);
 
 /* Grouped RMS norm with optional weight, gate, row gather and accumulation. Row r = (token r / groups, group r % groups),

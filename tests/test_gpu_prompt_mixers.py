@@ -267,6 +267,36 @@ def test_fp32_products_on_the_tensor_cores(M, N, K, aligned):
     assert torch.equal(torch.isnan(bad), torch.isnan(ref)) and torch.equal(torch.isinf(bad), torch.isinf(ref))
 
 
+@pytest.mark.parametrize("M,N,K", [(33, 9700, 516), (128, 4864, 512), (129, 3300, 580), (700, 2100, 260), (1300, 1000, 320), (9700, 33, 1028)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_fp32_products_split_once(monkeypatch, M, N, K, out_dtype):
+    """Operands split ahead of the product: edges of the 128 x 128 tiles and of the stages of 64, with epilogue, large and small rows, infinities and NaN, and entries far below their rows'
+    largest ones; beside the form that splits in every tile."""
+    from vyomai_b200 import ops
+    assert int(ops._lib.lib().vy_linear_plain_bytes(M, N, K)) > 0
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x, w = (torch.randn(r, K + 4, generator=g, device=DEV)[:, :K] for r in (M, N))
+    bias, addend = torch.randn(N, generator=g, device=DEV), torch.randn(M, N, generator=g, device=DEV)
+    x[1] *= 1e30
+    x[2] *= 1e-30
+    x[3], w[4] = 0.0, 0.0
+    exact = x.double() @ w.double().T
+    for add in (None, addend):
+        want = torch.nn.functional.silu(exact + bias.double()) * 0.5 + (0.0 if add is None else add.double())
+        for got in _both(monkeypatch, "vy_linear_plain_bytes", lambda: ops.linear_plain(x, w, bias=bias, act="silu", scale=0.5, addend=add, out_dtype=out_dtype)):
+            for rows in (slice(0, 1), slice(1, 2), slice(2, 4), slice(4, M)):
+                assert _err(got[rows], want[rows].cpu()) < (2 * BOUND if out_dtype == torch.float32 else 2.0 ** -8)
+    if out_dtype == torch.bfloat16:
+        return
+    x[5, K - 1], x[6, 0], w[0, 3] = float("inf"), float("nan"), 0.0
+    bad, ref = ops.linear_plain(x, w), x.double() @ w.double().T
+    assert torch.equal(torch.isnan(bad), torch.isnan(ref)) and torch.equal(torch.isinf(bad), torch.isinf(ref))
+    for ratio in (2.0 ** 20, 1e12):
+        x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+        x[:, 7::64], w[:, 7::64] = ratio, 0.0
+        assert _err(ops.linear_plain(x, w), (x.double() @ w.double().T).cpu()) < BOUND
+
+
 @pytest.mark.parametrize("ratio", [2.0 ** 16, 2.0 ** 20, 2.0 ** 24, 1e8, 1e12, 1e30])
 def test_fp32_products_of_entries_far_below_their_row_s_largest(ratio):
     """One entry per row is `ratio` times the others and meets a zero: the sums consist of the small ones alone."""

@@ -6,48 +6,9 @@
 // sequence-mixer models and the bf16 arm of the shapes the tensor-core GEMM does not take (a contraction over a
 // low rank, a handful of output features, strides that are not 16-byte multiples). vy_unary and vy_embed_rows live
 // here as well.
-#include "split_mma.cuh"
-#include "vy_common.cuh"
-#include "vy_ptx.cuh"   // warp_sum
+#include "linear_plain.cuh"
 
 namespace vy {
-
-__device__ __forceinline__ float uact(float x, int act) {
-  switch (act) {
-    case VY_UACT_RELU2: { const float r = fmaxf(x, 0.f); return r * r; }
-    case VY_UACT_SILU: return x / (1.f + expf(-x));
-    case VY_UACT_SIGMOID: return 1.f / (1.f + expf(-x));
-    case VY_UACT_GELU_TANH: return 0.5f * x * (1.f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
-    default: return x;
-  }
-}
-
-struct LinDev {
-  int M, N, K;
-  const void* A; long long lda; int a_dt;
-  const void* W; long long ldw; int w_dt;
-  const void* bias; int bias_dt;
-  const void* addend; long long ld_addend; int addend_dt;
-  int act; float scale;
-  void* out; long long ld_out; int out_dt;
-  long long a_batch, w_batch, out_batch, bias_batch;   // element strides between the independent products of a batched call
-};
-
-// product b of a batched call: the same shapes at shifted base pointers
-__device__ __forceinline__ void lin_select(LinDev& d, int b) {
-  if (b == 0) return;
-  d.A = static_cast<const char*>(d.A) + d.a_batch * b * (d.a_dt == VY_F32 ? 4 : 2);
-  d.W = static_cast<const char*>(d.W) + d.w_batch * b * (d.w_dt == VY_F32 ? 4 : 2);
-  d.out = static_cast<char*>(d.out) + d.out_batch * b * (d.out_dt == VY_F32 ? 4 : 2);
-  if (d.bias) d.bias = static_cast<const char*>(d.bias) + d.bias_batch * b * (d.bias_dt == VY_F32 ? 4 : 2);
-}
-
-__device__ __forceinline__ void lin_store(const LinDev& d, int m, int n, float acc) {
-  if (d.bias) acc += ld_as_float(d.bias, d.bias_dt, n);
-  acc = uact(acc, d.act) * d.scale;
-  if (d.addend) acc += ld_as_float(d.addend, d.addend_dt, static_cast<long long>(m) * d.ld_addend + n);
-  st_from_float(d.out, d.out_dt, static_cast<long long>(m) * d.ld_out + n, acc);
-}
 
 constexpr int LT = 64, LK = 16;
 
@@ -153,24 +114,6 @@ __global__ void __launch_bounds__(256) linear_thin_kernel(const __grid_constant_
     else *out = y0;
   }
 }
-
-// One product in fp32 FMAs by a warp (16-byte aligned rows, K a multiple of 4), the sum in every lane
-static __device__ __noinline__ float lin_dot(const float* a, const float* w, int K) {
-  float acc = 0.f;
-  for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
-    const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
-    acc = fmaf(x.x, y.x, acc);
-    acc = fmaf(x.y, y.y, acc);
-    acc = fmaf(x.z, y.z, acc);
-    acc = fmaf(x.w, y.w, acc);
-  }
-  return warp_sum(acc);
-}
-
-// An entry's halves are off by at most 2^-48 of the largest entry of its row and tile (split_mma.cuh), so a product is as good as an fp32 one unless it is
-// this small beside its rows' largest entries: then, as where an infinity or NaN went in (the halves of an infinity would all be NaN), it is computed again
-// in FMAs. At 2^-16 the halves' share is below 2^-25 of the product; of normal numbers' products 2 to 6 in a million are that small
-constexpr float LS_SMALL = 0x1p-16f * (1 << SPLIT_TOP) * (1 << SPLIT_TOP);
 
 // fp32 operands with 16-byte aligned rows: fp32 precision on the tensor cores (split_mma.cuh). 64 rows x 64 features per CTA, a warp 32 x 16.
 // Tiles of 64 k: loaded into registers while the tile before is multiplied, then split, with a scale per row and tile, into one of two buffers; a
@@ -474,6 +417,8 @@ extern "C" int vy_pair_embed(const VyPairEmbed* p) {
   return VY_OK;
 }
 
+extern "C" int64_t vy_linear_plain_bytes(int32_t M, int32_t N, int32_t K) { return vy::linear_split_bytes(M, N, K); }
+
 extern "C" int vy_linear_plain(const VyLinear* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_linear_plain: null params");
@@ -510,6 +455,14 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
     // from K = 256 on: below, a chain of FMAs is at least as exact (all terms positive, K 256: 2.5e-7 by FMAs, 2.1e-7 split; K 64: 1.2e-7, 2.1e-7), and the
     // two cost the same at 64 (9 us for 33 x 64)
     if (p->K >= 256 && p->K % 4 == 0 && rows16(d.A, d.a_dt, d.lda, batch > 1 ? d.a_batch : 0) && rows16(d.W, d.w_dt, d.ldw, batch > 1 ? d.w_batch : 0)) {
+      const long long need = batch == 1 ? linear_split_bytes(p->M, p->N, p->K) : 0;
+      if (need > 0 && p->workspace && reinterpret_cast<uintptr_t>(p->workspace) % 128 == 0 && p->workspace_bytes >= need) {
+        if (poison_raised("vy_linear_plain")) return VY_ERR_CUDA;
+        VY_CUDA_OK(launch_linear_split_tc(d, p->workspace, st));
+        VY_LAUNCH_OK();
+        count_launch(2);
+        return VY_OK;
+      }
       static std::atomic<unsigned long long> allowed{0};
       VY_CUDA_OK(allow_smem(linear_split_kernel, allowed));
       VY_CUDA_OK(launch_kernel(linear_split_kernel, dim3((p->N + LT - 1) / LT, (p->M + LT - 1) / LT, batch), dim3(256), 2 * LS_BUF, st, d));
