@@ -223,6 +223,49 @@ def test_score_exchanging_prompts_on_the_tensor_cores(monkeypatch, H, G, d, dv, 
         assert _err(got, torch.cat(want)) < 4 * BOUND   # mixed scores: each is a sum over H capped ones, and the softmax takes its absolute error
 
 
+@pytest.mark.parametrize("H,G,d,dv,window,cap,new,pos0,form", [
+    (16, 4, 64, 64, 0, 9.0, [130, 17, 1], [0, 48, 200], "tc"), (16, 1, 64, 64, 70, 0.0, [129], [63], "tc"), (32, 4, 32, 48, 0, 30.0, [65, 4], [0, 60], "tc"),
+    (32, 2, 7, 5, 3, 0.0, [70], [0], "tc"), (8, 4, 17, 64, 0, 4.0, [64, 128], [0, 1], "tc"), (8, 2, 48, 20, 0, 0.0, [16] * 148, [0, 5] * 74, "tc"),
+    (8, 2, 48, 20, 0, 0.0, [16] * 149, [5] * 149, "mma"), (16, 2, 33, 33, 20, 9.0, [40] * 60, [3] * 60, "mma")])
+@pytest.mark.parametrize("extras", [False, True])
+def test_score_exchanging_on_both_sides_of_the_line(H, G, d, dv, window, cap, new, pos0, form, extras):
+    """Tiles that end on, before and after an edge, few and many sequences; bare, or with bf16 inputs, scores to sink into and gates."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(H + d)
+    bs, io, n = 4, torch.bfloat16 if extras else torch.float32, len(new)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    q, talk = rnd(sum(new), H * d).to(io), torch.eye(H, device=DEV) + 0.3 * rnd(H, H) / H ** 0.5 if not extras or H > 8 else None
+    sink, per_channel = rnd(H) if extras else None, H != 16
+    gate = rnd(sum(new), H * dv if per_channel else H) if extras else None
+    batch, table, _, n_blocks, _ = shuffled_batch(new, pos0, bs, DEV, seed=H)
+    kp, vp = rnd(n_blocks, bs, G, d).to(io), rnd(n_blocks, bs, G, dv).to(io)
+    call = lambda: ops.talk_attn(batch, q, kp, vp, heads=H, kv_heads=G, dim=d, vdim=dv, scale=0.3, softcap=cap, talk=talk, window=window, sink=sink,  # noqa: E731
+                                 gate=gate, gate_per_channel=per_channel and extras, out_dtype=torch.float32)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        got = call().double()
+        torch.cuda.synchronize()
+    assert any(f"talk_attn_{form}_kernel" in e.name for e in prof.events())
+    at = 0
+    for s in range(n):
+        t = pos0[s] + new[s]
+        pages = torch.tensor(table[s][:(t + bs - 1) // bs], device=DEV)
+        k, v = (x[pages].reshape(-1, G, w)[:t].double().repeat_interleave(H // G, 1) for x, w in ((kp, d), (vp, dv)))
+        sc = torch.einsum("qhd,khd->hqk", q[at:at + new[s]].double().view(-1, H, d), k) * 0.3
+        if cap:
+            sc = cap * torch.tanh(sc / cap)
+        if talk is not None:
+            sc = torch.einsum("hb,bqk->hqk", talk.double(), sc)
+        back = torch.arange(pos0[s], t, device=DEV)[:, None] - torch.arange(t, device=DEV)[None, :]
+        sc = sc.masked_fill(~((back >= 0) & (back < window) if window else back >= 0), -float("inf"))
+        if sink is not None:
+            sc = torch.cat([sc, sink.double().view(H, 1, 1).expand(-1, new[s], 1)], -1)
+        want = torch.einsum("hqk,khd->qhd", torch.softmax(sc, -1)[..., :t], v)
+        if gate is not None:
+            want = want * torch.sigmoid(gate[at:at + new[s]].double()).view(new[s], H, -1)
+        assert _err(got[at:at + new[s]], want.reshape(new[s], -1).cpu()) < 4 * BOUND   # as above
+        at += new[s]
+
+
 @pytest.mark.parametrize("taps", [1, 3, 4, 5, 16])
 def test_causal_conv_over_portions_of_every_length(taps):
     """Portions shorter and longer than the taps and the kernel's token block, carried on; the taps that stay behind are the last inputs."""

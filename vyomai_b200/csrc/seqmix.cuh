@@ -239,6 +239,7 @@ long long window_attn_split_floats(const WinDev& d, int n_seqs, int max_new);
 // window_attn_tc.cu: the same rows for tcgen05, and the kernel that reads them (dim, vdim <= 128)
 bool window_attn_tc_applies(const WinDev& d, int n_seqs, int max_new);
 long long window_attn_tc_floats(const WinDev& d, int n_seqs, int max_new);
+SplitKv window_attn_tc_layout(const WinDev& d, int n_seqs, int max_new, float* ws);   // of the second layout, in a workspace of that many floats
 cudaError_t launch_window_attn_tc(const WinDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st);
 // key slots per (sequence, key / value head) that the step's queries can see at most (host-known bounds)
 long long split_slots(const WinDev& d, int max_new);

@@ -33,4 +33,8 @@ __device__ __forceinline__ float gate_of(const TalkDev& d, long long row, int h,
 long long talk_attn_mma_floats(const TalkDev& d, int n_seqs, int max_new);
 cudaError_t launch_talk_attn_mma(const TalkDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st);   // odd: what the fp32 tiles have to do
 
+// talk_attn_tc.cu: the same on tcgen05, from rows in window_attn_tc's layout. Does it pay? Never for more sequences where it does not for fewer
+bool talk_attn_tc_applies(const TalkDev& d, int n_seqs, int max_new);
+cudaError_t launch_talk_attn_tc(const TalkDev& d, const WinDev& keys, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st);
+
 }  // namespace vy

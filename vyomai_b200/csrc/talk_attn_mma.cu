@@ -9,7 +9,8 @@
 //
 // What bounds it: per tile and SM about as many cycles of the tensor pipe as of softmax instructions, and three barriers. The fp32-FMA tiles
 // (talk_attn_tiled_kernel, which stays for other head counts and sizes) spend 62 % of their issue slots on operand reads and the exchange.
-// 2 x 1437 tokens, 16 heads of 64: 805 us by those, 325 us here, 5 for the splitting.
+// 2 x 1437 tokens, 16 heads of 64: 805 us by those, 325 us here, 5 for the splitting. Up to four key / value heads and few or long enough prompts go to talk_attn_tc_kernel, which takes
+// 150 there (talk_attn_tc_applies says which); the others stay here.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 #include "talk_attn.cuh"
@@ -376,7 +377,9 @@ static WinDev talk_keys(const TalkDev& d) {   // the rows a step sees, in the wo
 }
 
 long long talk_attn_mma_floats(const TalkDev& d, int n_seqs, int max_new) {
-  return talk_mma_keys(d) ? window_attn_split_floats(talk_keys(d), n_seqs, max_new) : 0;
+  if (!talk_mma_keys(d)) return 0;
+  const long long a = window_attn_split_floats(talk_keys(d), n_seqs, max_new), b = talk_attn_tc_applies(d, n_seqs, max_new) ? window_attn_tc_floats(talk_keys(d), n_seqs, max_new) : 0;
+  return a > b ? a : b;   // of either layout
 }
 
 template <int HL, int N>
@@ -396,6 +399,7 @@ static cudaError_t launch_talk_mma(const TalkDev& d, const SplitKv& w, int n_seq
 }
 
 cudaError_t launch_talk_attn_mma(const TalkDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st) {
+  if (talk_attn_tc_applies(d, n_seqs, max_new)) return launch_talk_attn_tc(d, talk_keys(d), n_seqs, max_new, ws, odd, st);
   SplitKv w;
   cudaError_t e = launch_window_attn_split(talk_keys(d), n_seqs, max_new, ws, &w, st);
   if (e != cudaSuccess) return e;

@@ -519,7 +519,7 @@ static int tc_head_bits(const WinDev& d) {
   return hl;
 }
 
-static SplitKv tc_layout(const WinDev& d, int n_seqs, int max_new, float* ws) {
+SplitKv window_attn_tc_layout(const WinDev& d, int n_seqs, int max_new, float* ws) {
   const int dim16 = round_to(d.dim, 16), kd = round_to(2 * dim16, 64), vd = round_to(d.vdim, 64);
   SplitKv w = {};
   w.tail = 2 * TC_KEYS;
@@ -541,7 +541,7 @@ static SplitKv tc_layout(const WinDev& d, int n_seqs, int max_new, float* ws) {
 
 long long window_attn_tc_floats(const WinDev& d, int n_seqs, int max_new) {
   if (d.dim > 128 || d.vdim > 128) return 0;
-  const SplitKv w = tc_layout(d, 1, max_new, nullptr);
+  const SplitKv w = window_attn_tc_layout(d, 1, max_new, nullptr);
   return static_cast<long long>(n_seqs) * d.kv_heads * (w.cap * (w.row_bytes / 4 + 2) + 4LL * w.blocks + 4);
 }
 
@@ -610,7 +610,7 @@ static cudaError_t launch_tc(const CUtensorMap& map, const WinDev& d, const Spli
 }
 
 cudaError_t launch_window_attn_tc(const WinDev& d, int n_seqs, int max_new, float* ws, const int** odd, cudaStream_t st) {
-  const SplitKv w = tc_layout(d, n_seqs, max_new, ws);
+  const SplitKv w = window_attn_tc_layout(d, n_seqs, max_new, ws);
   *odd = w.odd;
   cudaError_t e = launch_split_rows(d, n_seqs, w, st);
   if (e != cudaSuccess) return e;
