@@ -907,7 +907,7 @@ def run_ours(args):
 # ------------------------------------------------------------------------------------------------
 # --workload hybrid: the Gelutar hybrid decoder beside DecoderModel at equal width / depth / vocabulary
 # ------------------------------------------------------------------------------------------------
-HYBRID_KERNELS = ("la_states", "la_scan", "la_outputs", "delta_chunk", "delta_scan", "window_attn_tc", "window_attn_mma", "window_attn_split", "linear_split", "linear_attn_chunk", "linear_attn", "delta_rule", "window_attn", "causal_conv", "rms_norm", "kv_page_write", "qk_norm_write",
+HYBRID_KERNELS = ("la_states", "la_scan", "la_outputs", "delta_chunk", "delta_scan", "window_attn_tc", "window_attn_mma", "window_attn_split", "linear_split", "linear_halves", "linear_attn_chunk", "linear_attn", "delta_rule", "window_attn", "causal_conv", "rms_norm", "kv_page_write", "qk_norm_write",
                   "linear_plain", "unary", "embed_rows", "gemm_skinny", "gemm_kernel", "attn_fwd", "attn_decode", "add_layernorm", "argmax")
 
 
@@ -1086,7 +1086,7 @@ def run_hybrid(args):
 # width / depth / vocabulary (both run on HybridBatchEngine's packed step)
 # ------------------------------------------------------------------------------------------------
 LATENT_KERNELS = ("window_attn_tc", "window_attn_mma", "window_attn_split", "la_states", "la_scan", "la_outputs", "delta_chunk", "delta_scan", "linear_split", "window_attn_decode", "window_attn_heads_merge", "window_attn_heads", "window_attn", "latent_kv_write", "rope_split", "moe_route", "moe_scale", "moe_sort",
-                  "moe_gather", "moe_combine", "linear_tile", "linear_rows", "linear_attn_chunk", "linear_attn", "delta_rule", "delta_prep",
+                  "moe_gather", "moe_combine", "linear_halves", "linear_thin", "linear_tile", "linear_rows", "linear_attn_chunk", "linear_attn", "delta_rule", "delta_prep",
                   "causal_conv", "rms_norm", "kv_page_write", "unary", "embed_rows", "gemm_skinny", "gemm_kernel", "argmax")
 
 
@@ -1259,7 +1259,7 @@ def run_latent(args):
 # --workload talking: the Vazepel parallel-layer decoder (score-exchanging attention, gated experts) beside the Zugunex
 # latent-attention decoder at equal width / depth / vocabulary (both run on HybridBatchEngine's packed step)
 # ------------------------------------------------------------------------------------------------
-TALKING_KERNELS = ("talk_attn_mma", "talk_attn_tiled", "talk_attn_rows", "talk_attn_merge", "depth_mix_norm", "moe_glu", "rope_kv_write") + LATENT_KERNELS
+TALKING_KERNELS = ("talk_attn_tc", "talk_attn_mma", "talk_attn_tiled", "talk_attn_rows", "talk_attn_merge", "depth_mix_norm", "moe_glu", "rope_kv_write") + LATENT_KERNELS
 
 
 def talking_config(width, layers=8, vocab=32768):
@@ -1301,9 +1301,9 @@ def measure_talking(dev, width, batch_prefill=4, prompt=2048, batch_decode=32, d
     visible = (prompt + 1) / 2.0
     # prompts: the two contractions (dim + vdim channels per query, key, head) plus the exchange (heads multiply-adds per query, key, head)
     fl = n_layers * tokens * H * visible * (m["dim"] + m["vdim"] + H) * 2
-    ms = z["prefill_kernels"].get("talk_attn_mma", {}).get("ms")
+    ms = sum(z["prefill_kernels"].get(k, {}).get("ms", 0.0) for k in ("talk_attn_tc", "talk_attn_mma"))
     if ms:
-        z["talk_attn_mma_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
+        z["talk_attn_prompt_roofline"] = {"gflop": round(fl / 1e9, 1), "tflops": round(fl / ms / 1e9, 2), "frac_of_fp32_nominal": round(fl / ms / 1e9 / fp32_tflops, 3)}
     dk = z["decode_kernels_eager"]
     ms = sum(dk.get(k, {}).get("ms", 0.0) for k in ("talk_attn_rows", "talk_attn_merge"))
     if ms:

@@ -266,6 +266,37 @@ def test_score_exchanging_on_both_sides_of_the_line(H, G, d, dv, window, cap, ne
         at += new[s]
 
 
+@pytest.mark.parametrize("new,H,dk,dv,carried,form", [
+    ([129], 3, 64, 64, False, "tc"), ([256, 1, 130, 127], 4, 36, 40, True, "tc"), ([300, 128], 2, 100, 132, True, "tc"), ([140] * 5, 5, 128, 96, False, "tc"),
+    ([200, 65], 2, 33, 64, True, "mma"), ([200], 2, 64, 30, False, "mma"), ([200], 2, 32, 64, False, "mma"), ([700] + [2] * 15, 16, 64, 64, True, "mma")])
+def test_linear_attention_of_activated_inputs(new, H, dk, dv, carried, form):
+    """Chunks of 128 tokens with all columns of a head, and what stays with chunks of 64. Decays from 0 and far below one to one; inputs whose exponential overflows."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    T, n = sum(new), len(new)
+    q, k, v = (torch.randn(T, H * w, device=DEV, generator=g) for w in (dk, dk, dv))
+    q[::7, 3], v[::5, 1] = -95.0, -1e4   # silu: below the smallest number, and 0
+    decay = torch.tensor(([1.0, 0.97, 1e-3, 0.5, 0.0, 0.999, 0.9, 0.8] * 2)[:H], device=DEV)
+    S0 = torch.randn(n, H, dk, dv, device=DEV, generator=g) if carried else torch.zeros(n, H, dk, dv, device=DEV)
+    cu = [sum(new[:i]) for i in range(n + 1)]
+    S = S0.clone()
+    batch = ops.PackedBatch(_i32(cu), _i32([9 if carried else 0] * n), _i32(list(range(n))), max(new))
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        got = ops.linear_attn(batch, q, k, v, decay, S, heads=H, dim=dk, vdim=dv, in_act="silu")
+        torch.cuda.synchronize()
+    assert any("la_outputs_tc_kernel" in e.name for e in prof.events()) == (form == "tc")
+    silu, d = torch.nn.functional.silu, decay.double()
+    for s, t in enumerate(new):
+        qq, kk, vv = (silu(x[cu[s]:cu[s + 1]].double()).view(t, H, -1) for x in (q, k, v))
+        i = torch.arange(t, device=DEV)
+        back = i[:, None] - i[None]
+        P = torch.einsum("ihd,jhd->hij", qq, kk) * torch.where(back >= 0, d.view(H, 1, 1) ** back.clamp_min(0), 0.0)
+        want = torch.einsum("hij,jhe->ihe", P, vv) + torch.einsum("ihd,hde->ihe", qq, S0[s].double()) * (d ** (i + 1).view(t, 1)).view(t, H, 1)
+        assert _err(got[cu[s]:cu[s + 1]], want.reshape(t, -1).cpu()) < BOUND
+        want = S0[s].double() * (d ** t).view(H, 1, 1) + torch.einsum("jhd,jhe,hj->hde", kk, vv, d.view(H, 1) ** (t - 1 - i))
+        assert _err(S[s], want.cpu()) < BOUND
+
+
 @pytest.mark.parametrize("taps", [1, 3, 4, 5, 16])
 def test_causal_conv_over_portions_of_every_length(taps):
     """Portions shorter and longer than the taps and the kernel's token block, carried on; the taps that stay behind are the last inputs."""

@@ -17,6 +17,17 @@ struct LaChunks {
 };
 __device__ __forceinline__ long long la_slot(const RecDev& d, int s, int c) { return d.cu[s] / LM_C + s + c; }
 
+// a^n, n <= 128, in eight steps of repeated squaring (double: rounded once, to the fp32 result)
+__device__ __forceinline__ float power(float a, int n) {
+  double x = a, r = 1.0;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if (n >> b & 1) r *= x;
+    x *= x;
+  }
+  return static_cast<float>(r);
+}
+
 // One warp: tokens E lane .. E lane + E - 1 of a chunk of nt (at most 32 E): log decays summed (in double: `each` gets token, sum, write strength and the sum at the
 // chunk's end) as in linear_attn_chunk_kernel. Returns the chunk's whole decay
 template <int E, typename Fn>

@@ -8,7 +8,8 @@
 // The walk this replaces for long portions (linear_attn_chunk_kernel: one CTA per sequence, head and slice of columns goes through the chunks in
 // order, on fp32 FMAs) is as long as the sequence and leaves SMs idle for few sequences; here only the scan is serial, and it is bound by the bytes
 // of the states (dim x vdim x 4 per chunk and head, written twice, read twice). q and k shared by a group of heads (state space: b and c) are
-// split, and their scores computed, once per group. A state-space prompt whose rows come in quads has the first and the third launch on tcgen05 (linear_attn_tc.cu).
+// split, and their scores computed, once per group. Prompts whose rows come in quads, of a state space or with silu of q, k and v, have the
+// first and the third launch on tcgen05 (linear_attn_tc.cu).
 //
 // The fp16 halves are off by at most 2^-49 of the largest entry under their unit, a row of q, k or v or a whole state. la_states looks at the rows (tokens) and
 // columns (channels) of every chunk's q, k and v, as each warp has them, and of the state that is carried in: where the largest entry of one is below 2^-20 of the
@@ -19,17 +20,6 @@
 #include "split_mma.cuh"
 
 namespace vy {
-
-// a^n, n < 128, in seven steps of repeated squaring (double: rounded once, to the fp32 result)
-__device__ __forceinline__ float power(float a, int n) {
-  double x = a, r = 1.0;
-#pragma unroll
-  for (int b = 0; b < 7; ++b) {
-    if (n >> b & 1) r *= x;
-    x *= x;
-  }
-  return static_cast<float>(r);
-}
 
 // four entries of row `row` (element offset o of src) from column c on, zero past `width`
 __device__ __forceinline__ float4 load4(const void* src, int dt, bool vec, long long o, int c, int width) {
@@ -547,7 +537,7 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   w.top = reinterpret_cast<unsigned*>(w.D + slots * d.heads);
   w.odd = reinterpret_cast<int*>(w.top + slots * d.heads);
   const bool quad = d.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(d.state) % 16 == 0 && reinterpret_cast<uintptr_t>(ws) % 16 == 0;
-  const int vslices = (d.vdim + 63) / 64, tc_hp = TD && vec && quad ? linear_attn_tc_heads(d, n_seqs, max_new, rows, vslices) : 0;
+  const int vslices = (d.vdim + 63) / 64, tc_hp = vec && quad ? linear_attn_tc_heads(d, n_seqs, max_new, rows, vslices) : 0;
   const bool tc = tc_hp > 0;
   const int C = w.chunk = tc ? LT_C : LM_C;
   const int dim16 = (d.dim + 15) & ~15, kb = dim16 * 2 + 16, chunks = (max_new + C - 1) / C;
@@ -582,7 +572,7 @@ static cudaError_t launch_la_mma(const RecDev& d, int n_seqs, int max_new, long 
   RecDev r = d;   // the walk, for what is left to it
   r.odd = w.odd;
   r.odd_heads = hp;
-  r.odd_each = vslices;
+  r.odd_each = tc && !TD ? 1 : vslices;   // that form's CTAs have all columns of a head
   r.odd_chunk = C;
   r.first = w.U;
   return TD ? launch_ssd_chunked(r, n_seqs, st) : launch_linear_attn_chunked(r, n_seqs, st);

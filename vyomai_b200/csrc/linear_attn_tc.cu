@@ -1,15 +1,18 @@
-// State-space prompts on tcgen05, chunks of 128 tokens: linear_attn_mma.cu's first and third launch, with fp32 precision from fp16 halves (split_mma.cuh).
+// State-space and linear-attention prompts on tcgen05, chunks of 128 tokens: linear_attn_mma.cu's first and third launch, with fp32 precision from fp16 halves (split_mma.cuh).
 //
 // Read-outs, O = (Q K^T . D) V + diag(decay to i) Q S_before. A CTA owns a chunk, 64 value columns and heads that share q and k. Its scores are made once and stay in
 // tensor memory. Per head eight warps split the values and the state, a head ahead of the sixteen others, which turn scores into weights (by row as fp16
 // halves, into tensor memory; four threads per row, 32 keys each) and bring out the head before: its two products have an accumulator each, since a row's weights have a
 // unit of their own. Small products go first, then hi hi onto 2^-11 of them (scale-input-d). Gates come and outputs leave by bulk copies of 32 columns.
 // A decay from a key to a row further on than the key's run of 32 is a product of two, at the end of the run: one exponential per row and run.
+// Without steps of time (TD false: a fixed decay per head, q, k and v activated as they are read) a head has q and k of its own, and a CTA takes its value columns 64 at a time where it
+// otherwise takes heads; decays come from a table of powers.
 // Loops are kept short: a CTA's code beyond the instruction cache costs as much as its arithmetic.
 //
 // What bounds it: chains of short steps with twenty-four warps to hide them (9,500 cycles per head: 2,500 weights, 1,800 splitting them, 3,500 bringing out) and
 // 17,000 cycles before the first head. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 115 us (mma.sync, chunks of 64: 299). Tried: eight warps for the rows, scores in
 // registers 180; outputs and gates through L1 rather than bulk copies 124; four warps that split, 129; a full division in the gate 138.
+// 4 x 2048 tokens, 8 heads of 128 x 128 with decays by head and silu: 114 here, 93 for the states, 17 for the scan (mma.sync: 332, 140, 39); with divisions in silu 141 and 101.
 #include "linear_attn.cuh"
 #include "split_mma.cuh"
 #include "vy_ptx.cuh"
@@ -39,17 +42,27 @@ __device__ __forceinline__ float within_100(float a) {   // NaN stays
   asm("min.NaN.f32 %0, %1, 0f42C80000;\n\tmax.NaN.f32 %0, %0, 0fC2C80000;" : "=f"(r) : "f"(a));
   return r;
 }
+// EXP: of expf, as good as the division's to the last bit but for rare ones (of q, k and v themselves: by 2^t the outputs' error is a seventh larger)
+template <bool EXP = false>
 __device__ __forceinline__ f32x2 silu_pair(f32x2 x) {
   constexpr float L2E = 1.4426950408889634f, L2E_LO = static_cast<float>(1.4426950408889634 - static_cast<double>(L2E));
   const float2 g = unpair(x);
   const f32x2 c = pair(within_100(g.x), within_100(g.y)), t = mul2(c, pair(-L2E));   // e^100 is infinite
   const f32x2 left = fma2(c, pair(-L2E_LO), fma2(c, pair(-L2E), mul2(t, pair(-1.f))));
-  const float2 tt = unpair(t);
-  const f32x2 y = add2(mul2(pair(vy_ex2_approx(tt.x), vy_ex2_approx(tt.y)), fma2(left, pair(0.6931471805599453f), pair(1.f))), pair(1.f));
+  const float2 tt = unpair(t), cc = unpair(c);
+  const f32x2 y = add2(EXP ? pair(expf(-cc.x), expf(-cc.y)) : mul2(pair(vy_ex2_approx(tt.x), vy_ex2_approx(tt.y)), fma2(left, pair(0.6931471805599453f), pair(1.f))), pair(1.f));
   const float2 ys = unpair(mul2(y, pair(RECIP_SCALE)));
   const f32x2 minus = mul2(y, pair(-1.f)), r0 = mul2(pair(vy_rcp_approx(ys.x), vy_rcp_approx(ys.y)), pair(RECIP_SCALE)), r = fma2(r0, fma2(minus, r0, pair(1.f)), r0), q = mul2(x, r);
   const float2 a = unpair(fma2(fma2(minus, q, x), r, q)), b = unpair(mul2(x, r0));
   return pair(a.x == a.x ? a.x : b.x, a.y == a.y ? a.y : b.y);   // infinities
+}
+template <int ACT>
+__device__ __forceinline__ float4 act_quad(float4 x) {
+  if constexpr (ACT == VY_UACT_SILU) {
+    const float2 a = unpair(silu_pair<true>(two_of(x))), b = unpair(silu_pair<true>(other_two_of(x)));
+    x = make_float4(a.x, a.y, b.x, b.y);
+  }
+  return x;
 }
 static __device__ __noinline__ float gate_any(float x, int act) { return apply_uact(x, act); }
 
@@ -61,6 +74,7 @@ static __device__ __noinline__ float gate_any(float x, int act) { return apply_u
 // What bounds it: 12,000 cycles before the first head, then the splitting's instructions. 4 x 2048 tokens, 32 heads of 128 x 64 in groups of 8: 60 us (mma.sync, chunks of 64: 102;
 // the scan between, of half as many states, 33 for 85).
 constexpr int LTS_THREADS = 544;   // eight warps that split, eight that bring out, one for copies and products
+template <bool TD, int ACT>
 __global__ void __launch_bounds__(LTS_THREADS, 1)
 la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap u_map, const __grid_constant__ RecDev d, const __grid_constant__ LaChunks w, int hp, int vslices,
                     const __grid_constant__ PoisonRef poison) {
@@ -80,10 +94,13 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
   uint32_t* tmem_at = reinterpret_cast<uint32_t*>(bars + 9);
   int* issued = reinterpret_cast<int*>(tmem_at + 1);   // [2] copies of values sent for
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31, t = threadIdx.x;
-  const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
+  const int s = blockIdx.z, c = TD ? blockIdx.x / vslices : blockIdx.x, v0 = TD ? (blockIdx.x % vslices) * 64 : 0, h0 = blockIdx.y * hp;
   const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LT_C;
   if (t0 >= n) return;
-  const int nt = min(LT_C, n - t0), hq = h0 / (d.heads / d.kv_heads), vw = min(64, d.vdim - v0);
+  const int nt = min(LT_C, n - t0), hq = TD ? h0 / (d.heads / d.kv_heads) : h0;
+  const int items = TD ? hp : vslices;   // heads, or 64 columns each of the one head, which then share q and k
+  const auto head_of = [&](int hh) { return TD ? h0 + hh : h0; };
+  const auto col_of = [&](int hh) { return TD ? v0 : 64 * hh; };
   const long long r0 = base + t0, slot = la_slot(d, s, c);
   const bool few = nt < 8;
   bool alive = true;
@@ -91,7 +108,7 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
     const int b = hh & 1;
     ++issued[b];
     mbar_arrive_expect_tx(&vfull[b], 2 * LT_HALF);
-    for (int i = 0; i < 2; ++i) tma_load_2d(Rs + (2 * b + i) * LT_HALF, &v_map, &vfull[b], (h0 + hh) * d.vdim + v0 + 32 * i, static_cast<int>(r0));
+    for (int i = 0; i < 2; ++i) tma_load_2d(Rs + (2 * b + i) * LT_HALF, &v_map, &vfull[b], head_of(hh) * d.vdim + col_of(hh) + 32 * i, static_cast<int>(r0));
   };
   if (t < 4) range[t] = {0u, RANGE_NONE};
   __syncthreads();
@@ -111,13 +128,22 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
     __syncwarp();
     if (elect_one_sync()) {
       load_v(0);
-      if (hp > 1) load_v(1);
+      if (items > 1) load_v(1);
     }
     __syncwarp();
     tmem_alloc(tmem_at, 256);
     tmem_relinquish();
   } else {
-    if (warp >= 8)
+    if (!TD && warp == 8) {
+      const float decay = d.decay[h0];
+#pragma unroll 1
+      for (int i = lane; i < LT_C; i += 32) es[i] = i < nt ? power(decay, nt - 1 - i) : 0.f;
+      if (lane == 0) {
+        w.D[slot * d.heads + h0] = power(decay, nt);
+        w.top[slot * d.heads + h0] = 0u;
+      }
+    }
+    if (TD && warp >= 8)
 #pragma unroll 1
       for (int hh = warp - 8; hh < hp; hh += 8) {   // as token_decays, in short loops: code that a CTA runs once comes cold
         const int h = h0 + hh;
@@ -157,6 +183,10 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
       float4 x[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) x[i] = row + 8 * i < nt && ch < d.dim ? *reinterpret_cast<const float4*>(p + (r0 + row + 8 * i) * ld) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (ACT != VY_UACT_NONE) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = act_quad<ACT>(x[i]);
+      }
       Range rk = {0u, RANGE_NONE};
       const uint4 m = look<16, 4>(x, few, d.dim - 16 * (warp & 7) < 4, rk);
       note_warp(range + isq, rk);
@@ -182,15 +212,15 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
     const int rr = lane >> 1, row = (rr & 8) + 2 * (rr & 3) + (rr >> 2 & 1), vc = 8 * warp + 4 * (lane & 1);
     Range rv = {0u, RANGE_NONE}, rs = rv;   // this thread's share
 #pragma unroll 1
-    for (int hh = 0; hh < hp; ++hh) {
-      const int h = h0 + hh, b = hh & 1;
-      const float* weight = es + hh * LT_C;
+    for (int hh = 0; hh < items; ++hh) {
+      const int h = head_of(hh), b = hh & 1, vw = min(64, d.vdim - col_of(hh));
+      const float* weight = es + (TD ? hh : 0) * LT_C;
       unsigned most_b = 0u;
 #pragma unroll
       for (int i = lane; i < LT_C; i += 32) most_b = max(most_b, abs_bits(weight[i]));
       const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, most_b));
       if (c == 0 && d.pos0[s] > 0) {   // the state that is carried in: a thread reads every fourth entry of a column
-        const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 + (t & 63);
+        const float* sp = d.state + (static_cast<long long>(d.slot[s]) * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + col_of(hh) + (t & 63);
         unsigned top = 0u;
 #pragma unroll 1
         for (int i0 = t >> 6; i0 < d.dim; i0 += 64) {   // sixteen rows in flight: four at a time took 15 us a head
@@ -212,7 +242,7 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
       for (int i = 0; i < 8; ++i) {
         const int r = row + 16 * i;
         const float4 x = *reinterpret_cast<const float4*>(from + r * 128 + (((vc & 31) * 4) ^ ((r & 7) << 4)));
-        y[i] = r < nt && vc < vw ? x : make_float4(0.f, 0.f, 0.f, 0.f);   // other sequences' rows, other heads' columns
+        y[i] = r < nt && vc < vw ? act_quad<ACT>(x) : make_float4(0.f, 0.f, 0.f, 0.f);   // other sequences' rows, other heads' columns
       }
       uint4 m = look<8, 2>(y, few, vw - 8 * warp < 4, rv);
       {   // the weighted columns' units from a bound, the columns' largest times the largest weight: rows are within 2^20 of one another, and the halves good to 2^24
@@ -238,7 +268,7 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
     const uint64_t ka = make_smem_desc_sw128(smem_u32(Ks), LT_ATOM, 1024), wb = make_smem_desc_sw128(smem_u32(Ws), 1024, 1024);
     constexpr uint32_t id = make_idesc(0, LT_C, 64, 1, 1);
 #pragma unroll 1
-    for (int hh = 0; hh < hp; ++hh) {
+    for (int hh = 0; hh < items; ++hh) {
       const int b = hh & 1;
       alive = mbar_wait_soft(wready, hh & 1, poison) && alive;
       if (hh > 1) alive = mbar_wait_soft(&dfree[b], ((hh >> 1) - 1) & 1, poison) && alive;
@@ -258,7 +288,7 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
         }
         umma_commit(wfree);
         umma_commit(&dfull[b]);
-        if (hh + 2 < hp) load_v(hh + 2);   // this head's raw values have been read
+        if (hh + 2 < items) load_v(hh + 2);   // this head's raw values have been read
       }
       __syncwarp();
     }
@@ -270,7 +300,7 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
     const float unit = row < d.dim ? ku[row] : 0.f;
     unsigned char* to = Os + half * LT_HALF + row * 128;
 #pragma unroll 1
-    for (int hh = 0; hh < hp; ++hh) {
+    for (int hh = 0; hh < items; ++hh) {
       const int b = hh & 1;
       alive = mbar_wait_soft(&dfull[b], (hh >> 1) & 1, poison) && alive;
       tc_fence_after();
@@ -298,7 +328,7 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
       if (warp == 8) {
         if (alive && elect_one_sync()) {
           for (int i = 0; i < 2; ++i)
-            if (32 * i < vw) tma_store_2d(&u_map, Os + i * LT_HALF, v0 + 32 * i, static_cast<int>((slot * d.heads + h0 + hh) * d.dim));
+            if (col_of(hh) + 32 * i < d.vdim) tma_store_2d(&u_map, Os + i * LT_HALF, col_of(hh) + 32 * i, static_cast<int>((slot * d.heads + head_of(hh)) * d.dim));
           tma_store_commit();
         }
         __syncwarp();
@@ -314,13 +344,14 @@ la_states_tc_kernel(const __grid_constant__ CUtensorMap v_map, const __grid_cons
     mbar_drain(vfull, issued, 2);
   }
   __syncthreads();
-  if (t == 0) w.odd[(slot * gridDim.y + blockIdx.y) * vslices + blockIdx.x % vslices] = too_wide(range[0]) || too_wide(range[1]) || too_wide(range[2]) || too_wide(range[3]);
+  if (t == 0) w.odd[TD ? (slot * gridDim.y + blockIdx.y) * vslices + blockIdx.x % vslices : slot * gridDim.y + blockIdx.y] = too_wide(range[0]) || too_wide(range[1]) || too_wide(range[2]) || too_wide(range[3]);
   if (warp == 16) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
   }
 }
 
+template <bool TD, int ACT>
 __global__ void __launch_bounds__(LT_THREADS, 1)
 la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_constant__ CUtensorMap out_map, const __grid_constant__ RecDev d, const __grid_constant__ LaChunks w, int hp, int vslices,
                      int dim16, const __grid_constant__ PoisonRef poison) {
@@ -342,10 +373,13 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
   uint32_t* tmem_at = reinterpret_cast<uint32_t*>(bars + 14);
   int* issued = reinterpret_cast<int*>(tmem_at + 1);   // copies of gates sent for
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int s = blockIdx.z, c = blockIdx.x / vslices, v0 = (blockIdx.x % vslices) * 64, h0 = blockIdx.y * hp;
+  const int s = blockIdx.z, c = TD ? blockIdx.x / vslices : blockIdx.x, v0 = TD ? (blockIdx.x % vslices) * 64 : 0, h0 = blockIdx.y * hp;
   const int base = d.cu[s], n = d.cu[s + 1] - base, t0 = c * LT_C;
   if (t0 >= n) return;
-  const int nt = min(LT_C, n - t0), hq = h0 / (d.heads / d.kv_heads), vw = min(64, d.vdim - v0);
+  const int nt = min(LT_C, n - t0), hq = TD ? h0 / (d.heads / d.kv_heads) : h0;
+  const int items = TD ? hp : vslices;   // heads, or 64 columns each of the one head, which then share q and k
+  const auto head_of = [&](int hh) { return TD ? h0 + hh : h0; };
+  const auto col_of = [&](int hh) { return TD ? v0 : 64 * hh; };
   const long long r0 = base + t0, slot = la_slot(d, s, c);
   if (warp == 0) {
     if (lane == 0) {
@@ -372,6 +406,14 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
     const int hh = warp - (LT_WARPS - hp);
     float* mine = decays + hh * 5 * LT_C;
     const int h = h0 + hh;
+    if constexpr (!TD) {
+      const float decay = d.decay[h];   // its powers; up to and with a token
+#pragma unroll 1
+      for (int i = lane; i < LT_C; i += 32) {
+        mine[2 * LT_C + i] = power(decay, i);
+        mine[3 * LT_C + i] = power(decay, i + 1);
+      }
+    } else {
     const float rate = expf(ld_as_float(d.a_log, d.a_log_dt, h)), dt_b = ld_as_float(d.dt_bias, d.a_log_dt, h);
     double before = 0.0;   // log decays summed, as in token_decays; a short loop: code that a CTA runs once comes cold
     float dt = lane < nt ? d.dt[(r0 + lane) * d.ld_dt + h] : 0.f;
@@ -393,6 +435,7 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
       mine[2 * LT_C + i] = strength;
       mine[3 * LT_C + i] = expf(hi);
       mine[4 * LT_C + i] = strength * expf(static_cast<float>(before - L));
+    }
     }
   } else {   // queries, then keys: eight lanes share a row; the next rows are on their way while two are split
     const int l8 = lane & 7, warps = LT_WARPS - hp, first = warp * 4 + (lane >> 3);
@@ -417,7 +460,7 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) x[u][k] = next[u][k];
+        for (int k = 0; k < 4; ++k) x[u][k] = act_quad<ACT>(next[u][k]);
       get(r_0 + 8 * warps);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
@@ -461,27 +504,28 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
     float4 x[4][2];
     unsigned next_top = 0u;
     const auto get = [&](int turn) {
-      const int h = h0 + (turn >> 1);
-      if (h >= h0 + hp) return;
+      const int item = turn >> 1, h = head_of(item), v0 = col_of(item), vw = min(64, d.vdim - v0);
+      if (item >= items) return;
       const bool state = turn & 1;
       const float* p = state ? w.U + (slot * d.heads + h) * static_cast<long long>(d.dim) * d.vdim + v0 : reinterpret_cast<const float*>(d.v) + r0 * d.ldv + static_cast<long long>(h) * d.vdim + v0;
       const long long ld = state ? d.vdim : d.ldv;
       const int rows = state ? d.dim : nt;
       if (state) next_top = w.top[slot * d.heads + h];
       // the next head's on its way to L2: from memory they take longer than half a turn
-      const float* ahead = p + (state ? d.dim * d.vdim : d.vdim);
+      const float* ahead = p + (!TD ? 64 : state ? d.dim * d.vdim : d.vdim);
+      const int ahead_vw = TD ? vw : min(64, d.vdim - v0 - 64);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           const int r = row + 32 * i;
           x[i][k] = r < rows && col + 32 * k < vw ? *reinterpret_cast<const float4*>(p + r * ld + col + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if ((t & 7) == 0 && h + 1 < h0 + hp && r < rows && 32 * k < vw) asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead + r * ld + 32 * k));
+          if ((t & 7) == 0 && item + 1 < items && r < rows && 32 * k < ahead_vw) asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead + r * ld + 32 * k));
         }
     };
     get(0);
 #pragma unroll 1
-    for (int turn = 0; turn < 2 * hp; ++turn) {
+    for (int turn = 0; turn < 2 * items; ++turn) {
       const int hh = turn >> 1, b = hh & 1;
       const bool state = turn & 1;
       float* units = vu + b * LT_C;
@@ -494,7 +538,7 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = row + 32 * i;
-        const float4 u = x[i][0], v = x[i][1];
+        const float4 u = state ? x[i][0] : act_quad<ACT>(x[i][0]), v = state ? x[i][1] : act_quad<ACT>(x[i][1]);
         float f = whole;
         if (!state) {
           float top = fmaxf(fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fmaxf(fabsf(u.z), fabsf(u.w))), fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
@@ -571,29 +615,29 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
     }
     tmem_st_wait();
     unsigned char* half = Os + (j >> 1) * LT_HALF;   // this warp's 16 columns: 16-byte pieces 4 (j & 1) .. of its rows there
-    const bool bulk = vw == 64 && nt == LT_C;        // otherwise a box of outputs would go over other heads' or sequences'
+    const auto bulk_of = [&](int hh) { return d.vdim - col_of(hh) >= 64 && nt == LT_C; };   // otherwise a box of outputs would go over other heads' or sequences'
     const bool copies = quarter == 0 && j == 3;      // another such warp: gates in, outputs out
     const auto gate_in = [&](int hh) {
       if (alive && elect_one_sync()) {
         if (d.gate) {
           ++*issued;
           mbar_arrive_expect_tx(gfull, 2 * LT_HALF);
-          for (int i = 0; i < 2; ++i) tma_load_2d(Os + i * LT_HALF, &gate_map, gfull, (h0 + hh) * d.vdim + v0 + 32 * i, static_cast<int>(r0));
+          for (int i = 0; i < 2; ++i) tma_load_2d(Os + i * LT_HALF, &gate_map, gfull, head_of(hh) * d.vdim + col_of(hh) + 32 * i, static_cast<int>(r0));
         } else mbar_arrive(gfull);
       }
       __syncwarp();
     };
     if (copies) gate_in(0);
-    const auto skip_of = [&](int hh) { return hh < hp ? ld_as_float(d.skip, d.a_log_dt, h0 + hh) : 0.f; };
-    const auto top_of = [&](int hh) { return hh < hp ? w.top[slot * d.heads + h0 + hh] : 0u; };
+    const auto skip_of = [&](int hh) { return TD && hh < hp ? ld_as_float(d.skip, d.a_log_dt, h0 + hh) : 0.f; };
+    const auto top_of = [&](int hh) { return hh < items ? w.top[slot * d.heads + head_of(hh)] : 0u; };
     float skip = skip_of(0);
     unsigned state_top = top_of(0);
     float f_state = 0.f, f_chunk = 0.f;   // of the head whose outputs are to be brought out
 #pragma unroll 1
-    for (int hh = 0; hh <= hp; ++hh) {
-      const int h = h0 + hh, b = hh & 1;
+    for (int hh = 0; hh <= items; ++hh) {
+      const int b = hh & 1;
       float fs = 0.f, fc = 0.f;
-      if (products && hh < hp) {
+      if (products && hh < items) {
         alive = mbar_wait_soft(sready, hh & 1, poison) && alive;
         if (hh > 1) alive = mbar_wait_soft(&ofree[b], ((hh >> 1) - 1) & 1, poison) && alive;   // the outputs of two heads ago have been read
         tc_fence_after();
@@ -610,9 +654,9 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
         }
         __syncwarp();
       }
-      if (hh < hp) {
+      if (hh < items) {
         alive = mbar_wait_soft(&filled[b], (hh >> 1) & 1, poison) && alive;
-        const float* mine = decays + hh * 5 * LT_C;
+        const float* mine = decays + (TD ? hh : 0) * 5 * LT_C;
         const float* units = vu + b * LT_C;
         fs = pow2i(split_exponent(__uint_as_float(state_top)) - SPLIT_TOP) * qunit * mine[3 * LT_C + row];
         float top = 0.f, mul = 1.f;   // mul: what the row's weights of this run still lack
@@ -627,7 +671,14 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
             raw[i + 2] = __float_as_uint(c.x);
             raw[i + 3] = __float_as_uint(c.y);
           };
-          if (j < quarter) {   // the decay from a key to the row in two factors, at the end of the key's run
+          if constexpr (!TD) {
+            const float* powers = mine + 2 * LT_C;
+            const int away = row - 32 * j;
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; i += 4)
+              times(make_float4(powers[max(away - i, 0)], powers[max(away - i - 1, 0)], powers[max(away - i - 2, 0)], powers[max(away - i - 3, 0)]), i);
+          } else if (j < quarter) {   // the decay from a key to the row in two factors, at the end of the key's run
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 32; i += 4) times(*reinterpret_cast<const float4*>(key + 4 * LT_C + i), i);
@@ -694,7 +745,8 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
         }
       }
       if (hh > 0) {   // bring out the head before
-        const int ob = b ^ 1;
+        const int ob = b ^ 1, h = head_of(hh - 1), v0 = col_of(hh - 1), vw = min(64, d.vdim - v0);
+        const bool bulk = bulk_of(hh - 1);
         alive = mbar_wait_soft(&ofull[ob], ((hh - 1) >> 1) & 1, poison) && alive;
         tc_fence_after();
         uint32_t os[16], oc[16];
@@ -737,7 +789,7 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
           for (int k = 0; k < 4; ++k) {
             const int i = quarter * 32 + 8 * k + (lane >> 2);
             const float4 y = *reinterpret_cast<const float4*>(half + i * 128 + (((4 * (j & 1) + tcol) ^ (i & 7)) << 4));
-            if (i < nt && 16 * j + 4 * tcol < vw) *reinterpret_cast<float4*>(reinterpret_cast<float*>(d.out) + (r0 + i) * d.ld_out + static_cast<long long>(h - 1) * d.vdim + v0 + 16 * j + 4 * tcol) = y;
+            if (i < nt && 16 * j + 4 * tcol < vw) *reinterpret_cast<float4*>(reinterpret_cast<float*>(d.out) + (r0 + i) * d.ld_out + static_cast<long long>(h) * d.vdim + v0 + 16 * j + 4 * tcol) = y;
           }
         }
         fence_proxy_async_smem();
@@ -746,12 +798,12 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
         if (copies) {
           alive = mbar_wait_soft(odone, (hh - 1) & 1, poison) && alive;
           if (alive && bulk && elect_one_sync()) {
-            for (int i = 0; i < 2; ++i) tma_store_2d(&out_map, Os + i * LT_HALF, (h - 1) * d.vdim + v0 + 32 * i, static_cast<int>(r0));
+            for (int i = 0; i < 2; ++i) tma_store_2d(&out_map, Os + i * LT_HALF, h * d.vdim + v0 + 32 * i, static_cast<int>(r0));
             tma_store_commit();
             tma_store_wait_read<0>();
           }
           __syncwarp();
-          if (hh < hp) gate_in(hh);
+          if (hh < items) gate_in(hh);
         }
       }
       f_state = fs;
@@ -774,16 +826,22 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
 
 // In place of the 64-token chunks wherever rows come in quads (values and outputs by bulk copies), us of vy_ssd, mma.sync / here, 32 heads of 128 x 64 in groups of 8: one
 // prompt of 200 tokens 63 / 42, 512 69 / 45, 2048 250 / 88, 4096 494 / 142; 16 of 150 453 / 142; 32 heads each with q and k of its own, one of 512 78 / 50, 4096 577 / 320;
-// 24 heads of 64 x 64 over one q and k, 2048 152 / 64; 8 of 128 x 128 in two groups, 2048 135 / 59
-static bool linear_attn_tc_applies(const RecDev& d) {
-  const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
-  if (d.dim > 128 || d.vdim < 32 || d.in_act != VY_UACT_NONE) return false;
-  // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever: what a compiler gives another number does without this form
+// 24 heads of 64 x 64 over one q and k, 2048 152 / 64; 8 of 128 x 128 in two groups, 2048 135 / 59.
+// Decays by head with silu of q, k and v (vy_linear_attn): 4 x 2048 tokens, 16 heads of 128 x 128 1005 / 415; 129 tokens, 4 heads of 64 x 64 62 / 46; 32 x 256, 16 heads of 64 x 64 499 / 286. Not
+// with 32 channels, whose outputs' error would be 1.02 times what it is there (with more it is 0.94 to 1.0), nor without silu: 2 x 1437, 8 heads of 128 x 128 83 / 81, error 1.01
+template <bool TD, int ACT>
+static bool la_registers() {   // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever: what a compiler gives another number does without this form
   static const bool enough = [] {
     cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, la_outputs_tc_kernel) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == LT_REGS;
+    return cudaFuncGetAttributes(&a, la_outputs_tc_kernel<TD, ACT>) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == LT_REGS;
   }();
-  if (!enough) return false;
+  return enough;
+}
+static bool linear_attn_tc_applies(const RecDev& d) {
+  const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
+  const bool silu = d.in_act == VY_UACT_SILU;
+  if (d.dim > 128 || d.vdim < 32 || (d.dt ? d.in_act != VY_UACT_NONE : !silu || d.dim <= 32)) return false;
+  if (!(d.dt ? la_registers<true, VY_UACT_NONE>() : la_registers<false, VY_UACT_SILU>())) return false;
   return d.out_dt == VY_F32 && quads(d.out, d.ld_out) && (!d.gate || quads(d.gate, d.ld_gate));
 }
 
@@ -792,7 +850,7 @@ static bool linear_attn_tc_applies(const RecDev& d) {
 // beside single tokens, mma.sync / here, us of vy_ssd: 512 beside 31 129 / 145, 2048 beside 31 230 / 265, 1000 beside 15 108 / 115; 200 beside 31 (three per SM) 89 / 73
 int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long rows, int vslices) {
   if (!linear_attn_tc_applies(d)) return 0;
-  const int rep = d.heads / d.kv_heads, sms = num_sms();
+  const int rep = d.dt ? d.heads / d.kv_heads : 1, sms = num_sms();
   const long long most = static_cast<long long>(n_seqs) * ((max_new + LT_C - 1) / LT_C), chunks = most < rows / LT_C + n_seqs ? most : rows / LT_C + n_seqs;
   int best = 1;
   long long least = 0;
@@ -804,7 +862,7 @@ int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long row
       best = hp;
     }
   }
-  return best == 1 && (most - chunks) * vslices * d.heads > 8LL * sms ? 0 : best;
+  return best == 1 && (most - chunks) * (d.dt ? vslices : 1) * d.heads > 8LL * sms ? 0 : best;
 }
 
 static bool row_map(CUtensorMap* m, const void* p, long long cols, long long rows, long long ld, int box_rows) {
@@ -813,34 +871,43 @@ static bool row_map(CUtensorMap* m, const void* p, long long cols, long long row
   return get_tensor_map_cached(m, VY_F32, 2, p, dims, strides, box, 1) == VY_OK;
 }
 
-cudaError_t launch_la_states_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
+template <bool TD, int ACT>
+static cudaError_t launch_states(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
   const int vslices = (d.vdim + 63) / 64;
   const size_t smem = static_cast<size_t>(6) * LT_ATOM + static_cast<size_t>(6) * LT_HALF + sizeof(float) * ((LT_HEADS + 1) * LT_C + 4 * 64) + 4 * sizeof(Range) + 128;
   static std::atomic<unsigned long long> allowed{0};
-  cudaError_t e = allow_smem(la_states_tc_kernel, allowed);
+  cudaError_t e = allow_smem(la_states_tc_kernel<TD, ACT>, allowed);
   if (e != cudaSuccess) return e;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
   CUtensorMap v_map, u_map;
   const long long slots = rows / LM_C + n_seqs;
   if (!row_map(&v_map, d.v, static_cast<long long>(d.heads) * d.vdim, rows, d.ldv, LT_C) || !row_map(&u_map, w.U, d.vdim, slots * d.heads * d.dim, d.vdim, d.dim)) return cudaErrorInvalidValue;
-  const dim3 grid(static_cast<unsigned>((max_new + LT_C - 1) / LT_C) * vslices, d.heads / hp, n_seqs);
-  return launch_kernel(la_states_tc_kernel, grid, dim3(LTS_THREADS), smem, st, v_map, u_map, d, w, hp, vslices, poison);
+  const dim3 grid(static_cast<unsigned>((max_new + LT_C - 1) / LT_C) * (TD ? vslices : 1), d.heads / hp, n_seqs);
+  return launch_kernel(la_states_tc_kernel<TD, ACT>, grid, dim3(LTS_THREADS), smem, st, v_map, u_map, d, w, hp, vslices, poison);
 }
 
-cudaError_t launch_la_outputs_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
+template <bool TD, int ACT>
+static cudaError_t launch_outputs(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
   const int dim16 = (d.dim + 15) & ~15, vslices = (d.vdim + 63) / 64;
   const size_t smem = static_cast<size_t>(2 * ((dim16 + 63) / 64) + 4) * LT_ATOM + static_cast<size_t>(2) * dim16 * 128 + 2 * LT_HALF + sizeof(float) * (12 + 5 * LT_HEADS) * LT_C + 128;
   static std::atomic<unsigned long long> allowed{0};
-  cudaError_t e = allow_smem(la_outputs_tc_kernel, allowed);
+  cudaError_t e = allow_smem(la_outputs_tc_kernel<TD, ACT>, allowed);
   if (e != cudaSuccess) return e;
   PoisonRef poison = {};
   if (!poison_ref(&poison)) return cudaErrorMemoryAllocation;
   CUtensorMap gate_map, out_map;
   const long long cols = static_cast<long long>(d.heads) * d.vdim;
   if (!row_map(&out_map, d.out, cols, rows, d.ld_out, LT_C) || !row_map(&gate_map, d.gate ? d.gate : d.out, cols, rows, d.gate ? d.ld_gate : d.ld_out, LT_C)) return cudaErrorInvalidValue;
-  const dim3 grid(static_cast<unsigned>((max_new + LT_C - 1) / LT_C) * vslices, d.heads / hp, n_seqs);
-  return launch_kernel(la_outputs_tc_kernel, grid, dim3(LT_THREADS), smem, st, gate_map, out_map, d, w, hp, vslices, dim16, poison);
+  const dim3 grid(static_cast<unsigned>((max_new + LT_C - 1) / LT_C) * (TD ? vslices : 1), d.heads / hp, n_seqs);
+  return launch_kernel(la_outputs_tc_kernel<TD, ACT>, grid, dim3(LT_THREADS), smem, st, gate_map, out_map, d, w, hp, vslices, dim16, poison);
+}
+
+cudaError_t launch_la_states_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
+  return d.dt ? launch_states<true, VY_UACT_NONE>(d, w, hp, n_seqs, max_new, rows, st) : launch_states<false, VY_UACT_SILU>(d, w, hp, n_seqs, max_new, rows, st);
+}
+cudaError_t launch_la_outputs_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
+  return d.dt ? launch_outputs<true, VY_UACT_NONE>(d, w, hp, n_seqs, max_new, rows, st) : launch_outputs<false, VY_UACT_SILU>(d, w, hp, n_seqs, max_new, rows, st);
 }
 
 }  // namespace vy
