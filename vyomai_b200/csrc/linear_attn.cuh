@@ -118,4 +118,9 @@ int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long row
 cudaError_t launch_la_states_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st);
 cudaError_t launch_la_outputs_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st);
 
+// linear_attn_tc_fixed.cu: the same for decays by head; has the build the registers that its kernels share out?
+bool la_fixed_registers();
+cudaError_t launch_la_states_fixed(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st);
+cudaError_t launch_la_outputs_fixed(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st);
+
 }  // namespace vy

@@ -824,11 +824,6 @@ la_outputs_tc_kernel(const __grid_constant__ CUtensorMap gate_map, const __grid_
   }
 }
 
-// In place of the 64-token chunks wherever rows come in quads (values and outputs by bulk copies), us of vy_ssd, mma.sync / here, 32 heads of 128 x 64 in groups of 8: one
-// prompt of 200 tokens 63 / 42, 512 69 / 45, 2048 250 / 88, 4096 494 / 142; 16 of 150 453 / 142; 32 heads each with q and k of its own, one of 512 78 / 50, 4096 577 / 320;
-// 24 heads of 64 x 64 over one q and k, 2048 152 / 64; 8 of 128 x 128 in two groups, 2048 135 / 59.
-// Decays by head with silu of q, k and v (vy_linear_attn): 4 x 2048 tokens, 16 heads of 128 x 128 1005 / 415; 129 tokens, 4 heads of 64 x 64 62 / 46; 32 x 256, 16 heads of 64 x 64 499 / 286. Not
-// with 32 channels, whose outputs' error would be 1.02 times what it is there (with more it is 0.94 to 1.0), nor without silu: 2 x 1437, 8 heads of 128 x 128 83 / 81, error 1.01
 template <bool TD, int ACT>
 static bool la_registers() {   // with fewer registers at launch than the warps share out, the first to ask for more would wait for ever: what a compiler gives another number does without this form
   static const bool enough = [] {
@@ -836,33 +831,6 @@ static bool la_registers() {   // with fewer registers at launch than the warps 
     return cudaFuncGetAttributes(&a, la_outputs_tc_kernel<TD, ACT>) == cudaSuccess && (a.numRegs + 7) / 8 * 8 == LT_REGS;
   }();
   return enough;
-}
-static bool linear_attn_tc_applies(const RecDev& d) {
-  const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
-  const bool silu = d.in_act == VY_UACT_SILU;
-  if (d.dim > 128 || d.vdim < 32 || (d.dt ? d.in_act != VY_UACT_NONE : !silu || d.dim <= 32)) return false;
-  if (!(d.dt ? la_registers<true, VY_UACT_NONE>() : la_registers<false, VY_UACT_SILU>())) return false;
-  return d.out_dt == VY_F32 && quads(d.out, d.ld_out) && (!d.gate || quads(d.gate, d.ld_gate));
-}
-
-// A CTA takes about as long before its first head as for two heads (17,000 cycles and 9,500), one CTA per SM at a time. The grid has the longest portion's chunks for every sequence,
-// and a CTA without a chunk waits for a whole SM too: with a head per CTA and more than eight such per SM, chunks of 64 are faster. 16 heads of 64 x 64 with q and k of their own, one prompt
-// beside single tokens, mma.sync / here, us of vy_ssd: 512 beside 31 129 / 145, 2048 beside 31 230 / 265, 1000 beside 15 108 / 115; 200 beside 31 (three per SM) 89 / 73
-int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long rows, int vslices) {
-  if (!linear_attn_tc_applies(d)) return 0;
-  const int rep = d.dt ? d.heads / d.kv_heads : 1, sms = num_sms();
-  const long long most = static_cast<long long>(n_seqs) * ((max_new + LT_C - 1) / LT_C), chunks = most < rows / LT_C + n_seqs ? most : rows / LT_C + n_seqs;
-  int best = 1;
-  long long least = 0;
-  for (int hp = 1; hp <= LT_HEADS && hp <= rep; ++hp) {
-    if (rep % hp) continue;
-    const long long time = (chunks * vslices * (d.heads / hp) + sms - 1) / sms * (hp + 2);
-    if (least == 0 || time <= least) {
-      least = time;
-      best = hp;
-    }
-  }
-  return best == 1 && (most - chunks) * (d.dt ? vslices : 1) * d.heads > 8LL * sms ? 0 : best;
 }
 
 static bool row_map(CUtensorMap* m, const void* p, long long cols, long long rows, long long ld, int box_rows) {
@@ -903,11 +871,54 @@ static cudaError_t launch_outputs(const RecDev& d, const LaChunks& w, int hp, in
   return launch_kernel(la_outputs_tc_kernel<TD, ACT>, grid, dim3(LT_THREADS), smem, st, gate_map, out_map, d, w, hp, vslices, dim16, poison);
 }
 
+#ifdef VY_LA_FIXED   // linear_attn_tc_fixed.cu: decays by head, silu
+bool la_fixed_registers() { return la_registers<false, VY_UACT_SILU>(); }
+cudaError_t launch_la_states_fixed(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
+  return launch_states<false, VY_UACT_SILU>(d, w, hp, n_seqs, max_new, rows, st);
+}
+cudaError_t launch_la_outputs_fixed(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
+  return launch_outputs<false, VY_UACT_SILU>(d, w, hp, n_seqs, max_new, rows, st);
+}
+#else
+// In place of the 64-token chunks wherever rows come in quads (values and outputs by bulk copies), us of vy_ssd, mma.sync / here, 32 heads of 128 x 64 in groups of 8: one
+// prompt of 200 tokens 63 / 42, 512 69 / 45, 2048 250 / 88, 4096 494 / 142; 16 of 150 453 / 142; 32 heads each with q and k of its own, one of 512 78 / 50, 4096 577 / 320;
+// 24 heads of 64 x 64 over one q and k, 2048 152 / 64; 8 of 128 x 128 in two groups, 2048 135 / 59.
+// Decays by head with silu of q, k and v (vy_linear_attn): 4 x 2048 tokens, 16 heads of 128 x 128 1005 / 415; 129 tokens, 4 heads of 64 x 64 62 / 46; 32 x 256, 16 heads of 64 x 64 499 / 286. Not
+// with 32 channels, whose outputs' error would be 1.02 times what it is there (with more it is 0.94 to 1.0), nor without silu: 2 x 1437, 8 heads of 128 x 128 83 / 81, error 1.01
+static bool linear_attn_tc_applies(const RecDev& d) {
+  const auto quads = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
+  const bool silu = d.in_act == VY_UACT_SILU;
+  if (d.dim > 128 || d.vdim < 32 || (d.dt ? d.in_act != VY_UACT_NONE : !silu || d.dim <= 32)) return false;
+  if (!(d.dt ? la_registers<true, VY_UACT_NONE>() : la_fixed_registers())) return false;
+  return d.out_dt == VY_F32 && quads(d.out, d.ld_out) && (!d.gate || quads(d.gate, d.ld_gate));
+}
+
+// A CTA takes about as long before its first head as for two heads (17,000 cycles and 9,500), one CTA per SM at a time. The grid has the longest portion's chunks for every sequence,
+// and a CTA without a chunk waits for a whole SM too: with a head per CTA and more than eight such per SM, chunks of 64 are faster. 16 heads of 64 x 64 with q and k of their own, one prompt
+// beside single tokens, mma.sync / here, us of vy_ssd: 512 beside 31 129 / 145, 2048 beside 31 230 / 265, 1000 beside 15 108 / 115; 200 beside 31 (three per SM) 89 / 73
+int linear_attn_tc_heads(const RecDev& d, int n_seqs, int max_new, long long rows, int vslices) {
+  if (!linear_attn_tc_applies(d)) return 0;
+  const int rep = d.dt ? d.heads / d.kv_heads : 1, sms = num_sms();
+  const long long most = static_cast<long long>(n_seqs) * ((max_new + LT_C - 1) / LT_C), chunks = most < rows / LT_C + n_seqs ? most : rows / LT_C + n_seqs;
+  int best = 1;
+  long long least = 0;
+  for (int hp = 1; hp <= LT_HEADS && hp <= rep; ++hp) {
+    if (rep % hp) continue;
+    const long long time = (chunks * vslices * (d.heads / hp) + sms - 1) / sms * (hp + 2);
+    if (least == 0 || time <= least) {
+      least = time;
+      best = hp;
+    }
+  }
+  return best == 1 && (most - chunks) * (d.dt ? vslices : 1) * d.heads > 8LL * sms ? 0 : best;
+}
+
 cudaError_t launch_la_states_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
-  return d.dt ? launch_states<true, VY_UACT_NONE>(d, w, hp, n_seqs, max_new, rows, st) : launch_states<false, VY_UACT_SILU>(d, w, hp, n_seqs, max_new, rows, st);
+  return d.dt ? launch_states<true, VY_UACT_NONE>(d, w, hp, n_seqs, max_new, rows, st) : launch_la_states_fixed(d, w, hp, n_seqs, max_new, rows, st);
 }
 cudaError_t launch_la_outputs_tc(const RecDev& d, const LaChunks& w, int hp, int n_seqs, int max_new, long long rows, cudaStream_t st) {
-  return d.dt ? launch_outputs<true, VY_UACT_NONE>(d, w, hp, n_seqs, max_new, rows, st) : launch_outputs<false, VY_UACT_SILU>(d, w, hp, n_seqs, max_new, rows, st);
+  return d.dt ? launch_outputs<true, VY_UACT_NONE>(d, w, hp, n_seqs, max_new, rows, st) : launch_la_outputs_fixed(d, w, hp, n_seqs, max_new, rows, st);
 }
+#endif
 
 }  // namespace vy
