@@ -464,6 +464,41 @@ def test_score_exchanging_prompts_keep_large_numbers_to_where_they_are_seen(wind
             assert _err(got[rows][..., 5], want[rows][..., 5]) < 4 * BOUND
 
 
+def _exchange_with_one_bad_entry(H, G, cap, window, what, bad):
+    """A prompt of 70 tokens, one of whose query or key entries is `bad`: (this library's output, float64's), [tokens, heads, channels]."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(H)
+    T, d, bs = 70, 32, 16
+    q, talk = torch.randn(T, H, d, generator=g, device=DEV), torch.eye(H, device=DEV) + 0.3 * torch.randn(H, H, generator=g, device=DEV) / H ** 0.5
+    batch, table, _, n_blocks, _ = shuffled_batch([T], [0], bs, DEV, seed=H)
+    kp, vp = torch.randn(n_blocks, bs, G, d, generator=g, device=DEV), torch.randn(n_blocks, bs, G, d, generator=g, device=DEV)
+    if what == "query":
+        q[40, 3, 5] = bad
+    else:
+        kp[table[0][40 // bs], 40 % bs, G - 1, 2] = bad
+    got = ops.talk_attn(batch, q.view(T, -1), kp, vp, heads=H, kv_heads=G, dim=d, vdim=d, scale=0.3, softcap=cap, talk=talk, window=window)
+    pages = torch.tensor(table[0][:(T + bs - 1) // bs], device=DEV)
+    k, v = (x[pages].reshape(-1, G, d)[:T].double().repeat_interleave(H // G, 1) for x in (kp, vp))
+    sc = torch.einsum("qhd,khd->hqk", q.double(), k) * 0.3
+    sc = torch.einsum("hb,bqk->hqk", talk.double(), cap * torch.tanh(sc / cap) if cap else sc)
+    back = torch.arange(T, device=DEV)[:, None] - torch.arange(T, device=DEV)[None, :]
+    seen = (back >= 0) & (back < window) if window else back >= 0
+    p = torch.softmax(sc.masked_fill(~seen, -float("inf")), -1)
+    return got.view(T, H, d), torch.einsum("hqk,khd->qhd", torch.where(seen, p, 0.0), v)
+
+
+@pytest.mark.parametrize("H,G", [(16, 4), (8, 2), (16, 1)])
+@pytest.mark.parametrize("window", [0, 20])
+@pytest.mark.parametrize("cap", [0.0, 9.0])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_score_exchanging_prompts_pass_a_bad_key_on_to_who_sees_it(H, G, window, cap, bad):
+    """NaN under a cap too, which is no score of the cap's size."""
+    got, want = _exchange_with_one_bad_entry(H, G, cap, window, "key", bad)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and bool(torch.isnan(want).any()) == (cap == 0.0 or bad != bad)
+    ok = ~torch.isnan(want)
+    assert _err(got[ok], want[ok].cpu()) < 4 * BOUND   # as above
+
+
 @pytest.mark.parametrize("bad", [1e5, 1e12, float("inf"), float("nan")])
 @pytest.mark.parametrize("where", ["value", "state"])
 def test_linear_attention_keeps_large_numbers_to_their_column(bad, where):

@@ -41,6 +41,12 @@ __device__ __forceinline__ void tt_split(f32x2 v, uint32_t& hi, uint32_t& lo) {
   lo = pack_h2(__floats2half2_rn(y.x, y.y));
 }
 
+__device__ __forceinline__ float at_most_100(float a) {   // NaN stays, as in cap_score; fminf would give the 100, and the score the cap
+  float r;
+  asm("min.NaN.f32 %0, %1, 0f42C80000;" : "=f"(r) : "f"(a));
+  return r;
+}
+
 __global__ void __launch_bounds__(TT_THREADS, 1)
 talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ TalkDev d, const __grid_constant__ SplitKv w, const __grid_constant__ TalkGeo geo,
                     const __grid_constant__ PoisonRef poison) {
@@ -397,7 +403,7 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
             f32x2 x = fma2(y, qhi, mul2(y, qlo));
             if (capped) {   // cap tanh(s / cap) = cap - 2 cap / (1 + e^(2 s / cap)); far out that is cap or -cap
               const float2 e = unpair(x);
-              const f32x2 z = add2(pair(vy_ex2_approx(fminf(e.x, 100.f)), vy_ex2_approx(fminf(e.y, 100.f))), pair(1.f));
+              const f32x2 z = add2(pair(vy_ex2_approx(at_most_100(e.x)), vy_ex2_approx(at_most_100(e.y))), pair(1.f));
               const float2 z2 = unpair(z);
               f32x2 r = pair(vy_rcp_approx(z2.x), vy_rcp_approx(z2.y));
               r = fma2(r, fma2(mul2(z, pair(-1.f)), r, pair(1.f)), r);   // as good as a division: the difference below cancels
