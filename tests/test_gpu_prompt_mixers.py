@@ -499,6 +499,17 @@ def test_score_exchanging_prompts_pass_a_bad_key_on_to_who_sees_it(H, G, window,
     assert _err(got[ok], want[ok].cpu()) < 4 * BOUND   # as above
 
 
+@pytest.mark.parametrize("H,G", [(16, 4), (8, 2), (16, 1)])
+@pytest.mark.parametrize("cap", [0.0, 9.0])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_score_exchanging_prompts_keep_a_bad_query_to_itself(H, G, cap, bad):
+    """128 / H queries share a CTA and its exchange."""
+    got, want = _exchange_with_one_bad_entry(H, G, cap, 0, "query", bad)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and bool(torch.isnan(want).any()) == (cap == 0.0 or bad != bad)
+    ok = ~torch.isnan(want)
+    assert _err(got[ok], want[ok].cpu()) < 4 * BOUND   # as above
+
+
 @pytest.mark.parametrize("bad", [1e5, 1e12, float("inf"), float("nan")])
 @pytest.mark.parametrize("where", ["value", "state"])
 def test_linear_attention_keeps_large_numbers_to_their_column(bad, where):

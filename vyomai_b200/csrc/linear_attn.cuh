@@ -64,7 +64,6 @@ __device__ __forceinline__ void store_split4(unsigned char* hi, unsigned char* l
 // Largest and smallest (but not zero) of rows' and columns' largest entries, as bits: positive numbers order like them, NaN after infinity
 constexpr unsigned RANGE_NONE = 0x7f800000u;   // infinity: no entry yet
 struct Range { unsigned top, low; };
-__device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 __device__ __forceinline__ void note(Range& r, unsigned m, bool few = false) {
   r.top = max(r.top, m);
   if (m) r.low = min(r.low, few ? __float_as_uint(16.f * __uint_as_float(m)) : m);

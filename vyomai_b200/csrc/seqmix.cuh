@@ -45,6 +45,8 @@ __device__ __forceinline__ float cap_score(float s, float cap, float two_over_ca
   return cap > 0.f ? cap * (1.f - __fdividef(2.f, 1.f + expf(s * two_over_cap))) : s;
 }
 
+// |x| as bits, which order as numbers do: those of an infinity are 0x7f800000, a NaN's larger
+__device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 __device__ __forceinline__ float dot4(const float4 a, const float4 b, float acc) {
   acc = fmaf(a.x, b.x, acc);
   acc = fmaf(a.y, b.y, acc);

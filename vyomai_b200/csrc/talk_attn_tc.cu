@@ -161,10 +161,11 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < nq && l16 * 4 < d.dim) x = from(at, l16 * 4);
         *reinterpret_cast<float4*>(Ss + r * 256 + ((l16 ^ (r & 15)) << 4)) = x;
-        float top = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
+        unsigned top = max(max(abs_bits(x.x), abs_bits(x.y)), max(abs_bits(x.z), abs_bits(x.w)));   // bits: a NaN's are the largest
 #pragma unroll
-        for (int k = 1; k < 16; k <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, k));
-        if (l16 == 0) qe[r] = top;
+        for (int k = 1; k < 16; k <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, k));
+        if (l16 == 0) qe[r] = __uint_as_float(top);
+        odd = odd || top >= 0x7f800000u;   // the exchange takes all queries' rows: times zero such a score would still be a NaN in the others'
       }
     };
     if (geo.qvec) fetch([&](long long at, int c) { return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(d.q) + at + c); });
