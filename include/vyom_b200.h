@@ -198,14 +198,15 @@ typedef struct VyGemm {
 VY_API int vy_gemm(const VyGemm* p);
 /* 1 if vy_gemm would serve `p` with the small-batch weight-streaming kernel (tiling hints do not apply to it), else 0 */
 VY_API int vy_gemm_is_small_batch(const VyGemm* p);
-/* Self-check of the barrier protocols of the GEMM, window-attention and delta-rule kernels: a wait inside a kernel that times
+/* Self-check of the barrier protocols of the GEMM and prompt kernels: a wait inside a kernel that times
  * out raises a device flag instead of faulting, and the launch finishes with undefined results. Returns the flag (0 = every
  * launch so far ran its protocol to completion, 1 = some launch did not, -1 = the flag could not be read); a raised flag is
  * lowered by the read. Synchronises the device. */
 VY_API int vy_gemm_poisoned(void);
 /* Same flag without synchronising (a pinned host mirror the kernels write on a timeout): 1 once a kernel on the current
  * device has timed out and nobody has acknowledged it through vy_gemm_poisoned(), else 0. While it is raised every
- * vy_gemm, vy_window_attn and vy_delta_rule call on that device fails with VY_ERR_CUDA, so a corrupted result cannot feed later work silently. */
+ * vy_gemm, vy_window_attn, vy_talk_attn, vy_linear_attn, vy_delta_rule, vy_ssd and vy_moe_grouped call, and every vy_linear_plain that takes its scratch, on that device fails with
+ * VY_ERR_CUDA, so a corrupted result cannot feed later work silently. */
 VY_API int vy_gemm_poison_peek(void);
 /* Raises that mirror from the host, as a kernel would whose wait has timed out: what callers make of it can be tested without one. 0, or -1 without a device */
 VY_API int vy_gemm_poison_raise(void);

@@ -643,6 +643,38 @@ def test_a_wait_that_timed_out_stops_what_would_use_its_results():
     assert lib().vy_gemm_poison_peek() == 0
 
 
+def test_every_op_whose_kernels_wait_looks_at_the_flag():
+    """As above, for the others that launch such kernels: score-exchanging attention, linear attention, state space, grouped experts, products split once."""
+    from vyomai_b200 import ops
+    from vyomai_b200._lib import VyomError, lib
+    x, one = torch.randn(256, 64, device=DEV), torch.ones(1, device=DEV)
+    batch = ops.PackedBatch(_i32([0, 256]), _i32([0]), _i32([0]), 256, _i32([[0]]), 256)
+    pool, h, big = x.view(1, 256, 1, 64), x.bfloat16(), torch.randn(2560, 512, device=DEV)
+    need = ops.moe_grouped_bytes(256, 2, 1, 64, 64, 0)
+    assert int(lib().vy_linear_plain_bytes(2560, 512, 512)) > 0
+    calls = [lambda: ops.talk_attn(batch, x.repeat(1, 8), pool, pool, heads=8, kv_heads=1, dim=64, vdim=64, scale=1.0),
+             lambda: ops.linear_attn(batch, x, x, x, one, torch.zeros(1, 1, 64, 64, device=DEV), heads=1, dim=64, vdim=64, in_act="silu"),
+             lambda: ops.linear_attn(batch, x, x, x, one, torch.zeros(1, 1, 64, 64, device=DEV), heads=1, dim=64, vdim=64),
+             lambda: ops.ssd(batch, x, x, x, x[:, :1], x, conv_w=torch.ones(192, 3, device=DEV), conv_b=None, dt_bias=one, a_log=one, skip=one, norm=torch.ones(64, device=DEV), heads=1, groups=1,
+                             dim=64, vdim=64, taps=3, norm_groups=1, norm_eps=1e-5, conv_state=torch.zeros(1, 3, 192, device=DEV), state=torch.zeros(1, 1, 64, 64, device=DEV),
+                             tickets=torch.zeros(1, 1, dtype=torch.int32, device=DEV)),
+             lambda: ops.moe_grouped(h, torch.zeros(256, 1, dtype=torch.int32, device=DEV), torch.ones(256, 1, device=DEV), h, h[:64].repeat(1, 2), experts=2, ff=64,
+                                     workspace=torch.empty(need, dtype=torch.uint8, device=DEV)),
+             lambda: ops.linear_plain(big, big[:512])]
+    for call in calls:
+        call()
+    assert lib().vy_gemm_poison_raise() == 0
+    try:
+        for call in calls:
+            with pytest.raises(VyomError, match="timed out"):
+                call()
+    finally:
+        assert lib().vy_gemm_poisoned() == 1
+    for call in calls:
+        call()
+    torch.cuda.synchronize()
+
+
 def test_causal_conv_over_very_many_channels():
     """More channels than a launch has blocks of 128 for."""
     from vyomai_b200 import ops

@@ -1165,6 +1165,7 @@ extern "C" int64_t vy_linear_attn_workspace_floats(int64_t rows, int32_t n_seqs,
 extern "C" int vy_linear_attn(const VyLinAttn* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_linear_attn: null params");
+  if (vy_device_ok() && poison_raised("vy_linear_attn")) return VY_ERR_CUDA;
   VY_NEED_DEVICE("vy_linear_attn");
   VY_CHECK_ARG(p->n_seqs > 0 && p->n_seqs <= 65535 && p->cu_tokens && p->pos0 && p->slot, "vy_linear_attn: bad batch");
   VY_CHECK_ARG(p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->dim <= 256 && p->vdim > 0, "vy_linear_attn: heads %d, dim %d (<= 256), vdim %d",

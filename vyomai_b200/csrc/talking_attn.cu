@@ -587,6 +587,7 @@ extern "C" int64_t vy_talk_attn_prompt_floats(int32_t n_seqs, int32_t max_new, i
 extern "C" int vy_talk_attn(const VyTalkAttn* p) {
   using namespace vy;
   VY_CHECK_ARG(p != nullptr, "vy_talk_attn: null params");
+  if (vy_device_ok() && poison_raised("vy_talk_attn")) return VY_ERR_CUDA;
   VY_NEED_DEVICE("vy_talk_attn");
   VY_CHECK_ARG(p->n_seqs > 0 && p->n_seqs <= 65535 && p->max_new > 0 && p->cu_tokens && p->pos0 && p->block_table && p->block_size > 0 &&
                    p->table_width > 0, "vy_talk_attn: bad batch");
