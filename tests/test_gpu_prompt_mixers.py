@@ -510,6 +510,21 @@ def test_score_exchanging_prompts_keep_a_bad_query_to_itself(H, G, cap, bad):
     assert _err(got[ok], want[ok].cpu()) < 4 * BOUND   # as above
 
 
+@pytest.mark.parametrize("small", [2.0 ** -k for k in (40, 28, 27, 26, 25, 24, 20, 10)])
+def test_score_exchanging_prompts_of_scores_far_below_the_cap(small):
+    """What the cap's arithmetic leaves of a score of `small` (up to 2^-23 of the cap, whatever the score) is within the scores' unit."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(12)
+    T, H, d = 70, 16, 64
+    q, kp, vp = torch.randn(T, H * d, generator=g, device=DEV) * small, torch.randn(1, T, 4, d, generator=g, device=DEV), torch.randn(1, T, 4, d, generator=g, device=DEV)
+    batch = ops.PackedBatch(_i32([0, T]), _i32([0]), _i32([0]), T, _i32([[0]]), T)
+    got = ops.talk_attn(batch, q, kp, vp, heads=H, kv_heads=4, dim=d, vdim=d, scale=0.125, softcap=30.0)
+    k, v = (x[0].double().repeat_interleave(H // 4, 1) for x in (kp, vp))
+    sc = 30.0 * torch.tanh(torch.einsum("qhd,khd->hqk", q.double().view(T, H, d), k) * 0.125 / 30.0)
+    p = torch.softmax(sc.masked_fill(torch.ones(T, T, dtype=torch.bool, device=DEV).triu(1), -float("inf")), -1)
+    assert _err(got, torch.einsum("hqk,khd->qhd", p, v).reshape(T, -1).cpu()) < 4 * BOUND   # as above
+
+
 @pytest.mark.parametrize("bad", [1e5, 1e12, float("inf"), float("nan")])
 @pytest.mark.parametrize("where", ["value", "state"])
 def test_linear_attention_keeps_large_numbers_to_their_column(bad, where):

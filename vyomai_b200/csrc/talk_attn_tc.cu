@@ -346,7 +346,7 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
       const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w))));
       largest *= pow2i(split_exponent(__uint_as_float(top)) - SPLIT_TOP) * fabsf(d.scale);
     }
-    if (capped) largest = fminf(largest, d.softcap);
+    if (capped) largest = fmaxf(fminf(largest, d.softcap), d.softcap * 0x1p-20f);   // cap - 2 cap r is off by about 2^-23 cap, whatever the score
     const int es = split_exponent(largest);
     const f32x2 sf = pair(split_scale(es));
     // mixed scores as exponents of 2
