@@ -3,7 +3,7 @@
 //
 // A CTA owns all H heads of 128 / H queries: 128 rows (head, query), a lane of tensor memory each, so that the 32 rows of a warp share a key / value head. Per tile of 64 keys
 //   scores:    all rows times the keys of each key / value head, whose rows alone are kept (the others' lanes are masked out of the product);
-//   exchange:  the capped scores go to shared memory as halves, [row][key]; the rows of `talk` spread over the queries' diagonal (128 x 128, made once) times that are the mixed scores;
+//   exchange:  the capped scores go to shared memory as halves, [query, head][key]; the rows of `talk` spread over the queries' diagonal (128 x 128, made once) times that are the mixed scores;
 //   values:    the weights, written over the mixed scores, times the values of each key / value head, masked in the same way.
 // Queries and the spread `talk` lie in tensor memory too, so that shared memory holds a whole tile's keys and values of four heads ahead. One warp sends off exchanges and
 // values, one the next tile's scores, two bring keys and values, sixteen hold the rows, four threads a row with 16 keys and 16 channels each. A tile's values are added while the next one's
@@ -13,8 +13,9 @@
 // rows when there are four. The rows' own chain - 2000 for caps and halves, 1000 until the exchange is back, 1600 for the softmax - hides behind them or hides them. A CTA's start
 // takes 13000 (queries, `talk` and 64 keys from memory, instructions not yet in the cache). Eight warps of rows with two tiles' scores in tensor memory, products of all scores against all
 // rows: 218 us; masked products by one warp: 193; by two: 150.
-// 2 x 1437 tokens, 16 heads of 64 over 4: 326 us by talk_attn_mma_kernel, 150 here; one of 700, 8 heads: 175 / 58; one of 64: 32 / 17. The cap's tanh divides as exactly as fp32 can,
-// which its cancellation needs: errors are 0.87 to 0.98 of that kernel's.
+// 2 x 1437 tokens, 16 heads of 64 over 4: 326 us by talk_attn_mma_kernel, 150 here; one of 700, 8 heads: 175 / 58; one of 64: 32 / 17. Errors are 0.73 to 0.96 of that kernel's (14 shapes, with caps and
+// without, scores of standard deviation 0.3 to 8): the cap's tanh divides as exactly as fp32 can, which its cancellation needs, the weights' exponents are of differences of scores, and a
+// query's heads meet in one accumulation or two. With the exponents multiplied out before the difference and the contraction in the rows' order they were up to 1.09 of it, at the same time.
 #include "seqmix.cuh"
 #include "split_mma.cuh"
 #include "talk_attn.cuh"
@@ -177,6 +178,9 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
   const uint32_t tmem = *tmem_at, S0 = tmem, X0 = tmem + 64, O0 = tmem + 128, Q0 = tmem + 192, T0 = tmem + 256;   // scores; mixed scores, then weights; weighted values; queries, hi | lo; spread talk, hi | lo
   const int quarter = warp & 3, part = warp >> 2, row = quarter * 32 + lane, h = row >> tqs, q = row & (TQ - 1), g = ((quarter * 32) >> tqs) / geo.per;   // of row warps
   const uint32_t at = static_cast<uint32_t>(quarter * 32) << 16;
+  // The exchange's contraction goes through the scores by query, so that a query's heads come in one step of 16 or two, and steps of others add zeros: an accumulation cuts off. Heads
+  // are turned by the query, for lanes next to one another to write to different banks
+  const int turned = q << (tqs < 3 ? 1 : 0), xrow = q * H + ((h + turned) & (H - 1));
   float qunit = 0.f;
   if (warp < TT_WARPS) {   // the row as halves, and the weights of its query's rows
     {
@@ -198,12 +202,12 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
     }
 #pragma unroll 1
     for (int c0 = part * (128 / TT_PARTS); c0 < (part + 1) * (128 / TT_PARTS); c0 += 16) {   // columns of hi | lo: column c holds rows 2 c and 2 c + 1
-      const uint32_t pick = c0 < 64 ? (q & 1 ? 0x1044u : 0x4410u) : (q & 1 ? 0x3244u : 0x4432u);
       uint32_t w16[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const uint32_t x = __byte_perm(talk[h * H + ((2 * ((c0 + i) & 63)) >> tqs)], 0u, pick);
-        w16[i] = (2 * i & (TQ - 1)) == (q & ~1) ? x : 0u;
+        const int k = 2 * ((c0 + i) & 63), b = k - turned;
+        const uint32_t x = __byte_perm(talk[h * H + (b & (H - 1))], talk[h * H + ((b + 1) & (H - 1))], c0 < 64 ? 0x5410u : 0x7632u);
+        w16[i] = k >> (7 - tqs) == q ? x : 0u;
       }
       tmem_st_x16(T0 + at + c0, w16);
     }
@@ -349,12 +353,13 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
     if (capped) largest = fmaxf(fminf(largest, d.softcap), d.softcap * 0x1p-20f);   // cap - 2 cap r is off by about 2^-23 cap, whatever the score
     const int es = split_exponent(largest);
     const f32x2 sf = pair(split_scale(es));
-    // mixed scores as exponents of 2
-    const float mf = te[h] * pow2i(es - SPLIT_TOP), f1 = mf * L2E;
-    const f32x2 fhi = pair(f1), flo = pair(fmaf(mf, L2E_LO, fmaf(mf, L2E, -f1)));
+    // a power of two for the mixed scores, and what makes a difference of them an exponent of 2: of differences, which are small where they matter, the product's rounding is too. Scores
+    // that are this small are all alike
+    const float mf = fmaxf(te[h] * pow2i(es - SPLIT_TOP), 0x1p-80f), f1 = mf * L2E, f2 = mf * L2E_LO;
+    const f32x2 fhi = pair(f1), flo = pair(f2);
     float sink;
     const bool has = sink_of(d, h, sink);
-    float m = has ? sink * L2E : -INFINITY, l = has && part == 0 ? 1.f : 0.f;
+    float m = has ? sink / mf : -INFINITY, l = has && part == 0 ? 1.f : 0.f;
     const int E = split_exponent(about[3 * g + 2]);
     const float v_unit = pow2i(SPLIT_TOP - E);
     f32x2 o[TT_PER / 2];
@@ -371,7 +376,7 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
         o[i / 2] = add2(o[i / 2], fma2(v, cut, v));
       }
     };
-    const f32x2 cut_s = pair(0.5f * (geo.nks + 1) * 0x1p-25f), cut_x = pair(0.5f * (TT_ROWS / 16 + 1) * 0x1p-25f);
+    const f32x2 cut_s = pair(0.5f * (geo.nks + 1) * 0x1p-25f), cut_x = pair(0.5f * ((H + 15) / 16 + 1) * 0x1p-25f);
     // units: thread i brings those of key i % 64 of key / value head i / 64, a tile ahead
     const bool brings = threadIdx.x < TT_KEYS * G;
     const float2* unit_at = reinterpret_cast<const float2*>(w.unit) + list(brings ? threadIdx.x / TT_KEYS : 0) + threadIdx.x % TT_KEYS;
@@ -413,10 +418,10 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
             tt_split(mul2(x, sf), hi[i + k], lo_[i + k]);
           }
         }
-        unsigned char* to = Ss + row * 128;
+        unsigned char* to = Ss + xrow * 128;
 #pragma unroll
         for (int i = 0; i < TT_PER / 2; i += 4) {
-          const int c = (2 * TT_PER * part + 4 * i) ^ ((row & 7) << 4);
+          const int c = (2 * TT_PER * part + 4 * i) ^ ((xrow & 7) << 4);
           *reinterpret_cast<uint4*>(to + c) = make_uint4(hi[i], hi[i + 1], hi[i + 2], hi[i + 3]);
           *reinterpret_cast<uint4*>(to + TT_ATOM2 + c) = make_uint4(lo_[i], lo_[i + 1], lo_[i + 2], lo_[i + 3]);
         }
@@ -437,8 +442,8 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
       f32x2 x[TT_PER / 2];
 #pragma unroll
       for (int i = 0; i < TT_PER / 2; ++i) {
-        const f32x2 v = pair_bits(raw[2 * i], raw[2 * i + 1]), y = fma2(v, cut_x, v);
-        x[i] = fma2(y, fhi, mul2(y, flo));
+        const f32x2 v = pair_bits(raw[2 * i], raw[2 * i + 1]);
+        x[i] = fma2(v, cut_x, v);
       }
       const int f = lo + t * TT_KEYS + TT_PER * part;   // position of this thread's first key
       if (!(f + TT_PER - 1 <= p_lo && (d.window <= 0 || p_hi - f < d.window))) {
@@ -462,7 +467,7 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
       float mn = share[row];
 #pragma unroll
       for (int k = 1; k < TT_PARTS; ++k) mn = fmaxf(mn, share[k * TT_ROWS + row]);
-      const float cr = mn == -INFINITY ? 1.f : vy_ex2_approx(m - mn);
+      const float cr = mn == -INFINITY ? 1.f : vy_ex2_approx(fmaf(m - mn, f1, (m - mn) * f2));
       m = mn;
       const f32x2 mm = pair(m == -INFINITY ? 0.f : -m);
       f32x2 sum = pair(0.f);
@@ -474,7 +479,8 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
           const float4 v4 = *reinterpret_cast<const float4*>(vu + 2 * i);
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            const float2 z = unpair(add2(x[i + k], mm));
+            const f32x2 less = add2(x[i + k], mm);
+            const float2 z = unpair(fma2(less, fhi, mul2(less, flo)));
             const f32x2 e = pair(vy_ex2_approx(z.x), vy_ex2_approx(z.y));
             sum = add2(sum, e);
             tt_split(mul2(e, mul2(k ? pair(v4.z, v4.w) : pair(v4.x, v4.y), vs)), hi[i + k], lo_[i + k]);
