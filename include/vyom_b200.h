@@ -647,7 +647,7 @@ typedef struct VyLinear {
   float scale;
   void* out; int64_t ld_out; int32_t out_dtype;
   /* batch > 1: `batch` independent products in one launch (one per attention head, say); product b reads A + b * a_batch,
-   * W + b * w_batch and writes out + b * out_batch (strides in elements; addend must be null, bias too unless bias_batch gives its stride). 0 = 1. */
+   * W + b * w_batch and writes out + b * out_batch (strides in elements, of either sign; addend must be null, bias too unless bias_batch gives its stride). 0 = 1. */
   int32_t batch; int64_t a_batch, w_batch, out_batch;
   void* stream;
   int64_t bias_batch;

@@ -128,6 +128,57 @@ def test_thin_products(M, N, K, dtype):
     assert _err(one, 0.5 * torch.nn.functional.silu(want[0]).cpu()) < BOUND
 
 
+def _delta_mixer(W=64, H=2, D=32, rank=16, conv=torch.float32):
+    """(weights, forward(mixer) on the same 200 tokens) of a delta mixer whose input products are made here."""
+    from types import SimpleNamespace
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(1)
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV) / s[-1] ** 0.5  # noqa: E731
+    n = {"q": H * D, "k": H * D, "v": H * D, "b": H, "a1": rank, "g1": rank}
+    w = {**{k: R(v, W) for k, v in n.items()}, "a2": R(H * D, rank), "g2": R(H * D, rank), "dt_bias": R(H * D), "A_log": R(H), "norm": torch.ones(D, device=DEV), "o": R(W, H * D),
+         **{k + ".conv": R(H * D, 4) for k in "qkv"}}
+    w["k.conv"] = w["k.conv"].to(conv)
+    h = R(200, W) * 8
+    packed = torch.cat([torch.nn.functional.pad(h @ w[k].T, (0, -v % 8)) for k, v in n.items()], 1)
+    parts, at = [], 0
+    for v in n.values():
+        parts.append(packed[:, at:at + v])
+        at += v + -v % 8
+    batch = ops.PackedBatch(_i32([0, 130, 200]), _i32([0, 0]), _i32([0, 1]), 130)
+    def forward(mixer, parts=parts):
+        return mixer.forward(parts, batch, SimpleNamespace(states={"S": torch.zeros(2, H, D, D, device=DEV), **{"conv_" + k: torch.zeros(2, H * D, 3, device=DEV) for k in "qkv"}}))
+    return dict(heads=H, kv_heads=H, dim=D, vdim=D, conv=4), w, parts, forward
+
+
+def test_delta_mixer_reads_its_low_rank_weights_where_they_are():
+    """A change of them in place takes effect; blocks of one product and blocks of their own give the same."""
+    from vyomai_b200.layers.mixers import GatedDeltaMixer
+    cfg, w, parts, forward = _delta_mixer()
+    mixer = GatedDeltaMixer(cfg, w, 1e-6, torch.float32, False)
+    first = forward(mixer)
+    for name in ("a2", "g2", "dt_bias"):
+        w[name].mul_(0.25).add_(0.1)
+        after = forward(mixer)
+        assert torch.equal(after, forward(GatedDeltaMixer(cfg, w, 1e-6, torch.float32, False))) and not torch.equal(after, first)
+        first = after
+    apart = parts[:4] + [parts[4].clone(), parts[5].clone()]
+    for other in (apart, parts[:4] + [parts[4].clone(), parts[5]]):   # the last: rows of another stride, a call each
+        assert torch.equal(forward(mixer, other), first)
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 33, 7), (20, 64, 16), (40, 300, 12), (65, 100, 64), (70, 70, 256)])
+def test_two_products_in_one_launch(M, N, K):
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, w, b = torch.randn(2 * M, K, generator=g, device=DEV), torch.randn(2 * N, K, generator=g, device=DEV), torch.randn(2 * N, generator=g, device=DEV)
+    halves = lambda t: (t[:t.shape[0] // 2], t[t.shape[0] // 2:])  # noqa: E731
+    for order in (1, -1):   # the second operand behind the first one, and before it
+        args = [halves(t)[::order] for t in (x, w, b)]
+        for i, y in enumerate(ops.linear_pair(*args)):
+            assert _err(y, (args[0][i].double() @ args[1][i].double().T + args[2][i].double()).cpu()) < BOUND
+    assert ops.linear_pair(halves(x), (w[:N], w[N:].bfloat16()), halves(b)) is None and ops.linear_pair((x[:M], x[:M]), halves(w), (b[:N], b[:N])) is None
+
+
 @pytest.mark.parametrize("channels", [(64, 64, 128), (5, 64, 33), (260, 512, 4), (128, 384)])
 @pytest.mark.parametrize("tokens", [1, 17, 1500])
 def test_convolutions_in_one_launch(channels, tokens):

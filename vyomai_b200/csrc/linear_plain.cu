@@ -432,7 +432,7 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
   VY_CHECK_ARG(p->lda >= p->K && p->ldw >= p->K && p->ld_out >= p->N, "vy_linear_plain: leading dimension smaller than the row");
   VY_CHECK_ARG(p->act >= VY_UACT_NONE && p->act <= VY_UACT_GELU_TANH, "vy_linear_plain: bad act %d", p->act);
   const int batch = p->batch > 1 ? p->batch : 1;
-  VY_CHECK_ARG(batch <= 65535 && (batch == 1 || ((!p->bias || p->bias_batch > 0) && !p->addend)), "vy_linear_plain: a batched call takes no addend, a bias with its stride (batch %d)", batch);
+  VY_CHECK_ARG(batch <= 65535 && (batch == 1 || ((!p->bias || p->bias_batch != 0) && !p->addend)), "vy_linear_plain: a batched call takes no addend, a bias with its stride (batch %d)", batch);
   if (p->bias) VY_CHECK_ARG(dtype_ok(p->bias_dtype), "vy_linear_plain: bad bias_dtype");
   if (p->addend) VY_CHECK_ARG(dtype_ok(p->addend_dtype) && p->ld_addend >= p->N, "vy_linear_plain: bad addend");
   LinDev d;

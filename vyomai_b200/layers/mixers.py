@@ -217,14 +217,10 @@ class GatedDeltaMixer(Mixer):
         self.eps, self.act_dtype = eps, act_dtype
         self._in = [w["q"], w["k"], w["v"], w["b"], w["a1"], w["g1"]]
         self.conv_w = [w["q.conv"].contiguous(), w["k.conv"].contiguous(), w["v.conv"].contiguous()]
-        # contractions over the low rank: fp32 activations straight from the a1 / g1 blocks; one call for both where their shapes are the same
+        self.a2 = Projection(w["a2"], False)  # contractions over the low rank: fp32 activations straight from the a1 / g1 blocks
+        self.g2 = Projection(w["g2"], False)
         self.dt_bias = w["dt_bias"].contiguous()
-        self.both = None
-        if w["a2"].shape == w["g2"].shape and w["a2"].dtype == w["g2"].dtype:
-            self.both = torch.stack([w["a2"], w["g2"]])
-            self.both_bias = torch.stack([self.dt_bias, torch.zeros_like(self.dt_bias)])
-        else:
-            self.a2, self.g2 = Projection(w["a2"], False), Projection(w["g2"], False)
+        self.no_bias = torch.zeros_like(self.dt_bias)
         self.a_log = w["A_log"].contiguous()
         self.norm = w["norm"].contiguous()
         self.o = Projection(w["o"], tensor_cores)
@@ -239,26 +235,14 @@ class GatedDeltaMixer(Mixer):
             st.update({"conv_q": (qk, self.taps - 1), "conv_k": (qk, self.taps - 1), "conv_v": (vv, self.taps - 1)})
         return {"pages": None, "states": st}
 
-    def low_rank(self, a1, g1):
-        a2, g2 = (self.both[0], self.both[1]) if self.both is not None else (self.a2.weight, self.g2.weight)
-        return (ops.linear_plain(a1, a2, bias=self.dt_bias, out_dtype=torch.float32), ops.linear_plain(g1, g2, out_dtype=torch.float32))
-
     def forward(self, parts, batch, cache):
         q, k, v, b, a1, g1 = parts
         dummy = cache.states["S"]
         qkv = ops.causal_convs(batch, (q, k, v), self.conv_w, [cache.states.get(n, dummy) for n in ("conv_q", "conv_k", "conv_v")])
         qk = self.kv_heads * self.dim
         qc, kc, vc = qkv[:, :qk], qkv[:, qk:2 * qk], qkv[:, 2 * qk:]
-        apart = g1.data_ptr() - a1.data_ptr()
-        if self.both is not None and a1.stride(0) == g1.stride(0) and 0 < apart < a1.stride(0) * a1.element_size():   # both blocks of one product
-            _, N, K = self.both.shape
-            wide = _round_up(N, 8)
-            ag = torch.empty((a1.shape[0], 2 * wide), device=a1.device, dtype=torch.float32)
-            x = a1.as_strided((a1.shape[0], apart // a1.element_size() + K), a1.stride())
-            ops.head_linear(x, self.both, ag, x_head=apart // a1.element_size(), out_head=wide, bias=self.both_bias)
-            a, g = ag[:, :N], ag[:, wide:wide + N]
-        else:
-            a, g = self.low_rank(a1, g1)
+        pair = ops.linear_pair((a1, g1), (self.a2.weight, self.g2.weight), (self.dt_bias, self.no_bias))
+        a, g = pair if pair is not None else (self.a2(a1, bias=self.dt_bias), self.g2(g1))
         o = ops.delta_rule(batch, qc, kc, vc, a, b, self.a_log, cache.states["S"], heads=self.heads, kv_heads=self.kv_heads, dim=self.dim,
                            vdim=self.vdim, unit_eps=1e-6)
         on = ops.rms_norm(o, self.norm, eps=self.eps, w_mode="plain", groups=self.heads, gate=g, gate_act="sigmoid", out_dtype=self.act_dtype)

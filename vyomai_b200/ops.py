@@ -956,6 +956,28 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, x_head: 
     return out
 
 
+def linear_pair(xs, ws, biases):
+    """Two products x W^T + bias in one launch, fp32 results side by side, or None where the two differ in a shape, a type or a row stride. The second one's operands are named by
+    their distance from the first one's, so that both are read where they lie."""
+    (x, y), (w, u), (b, c) = xs, ws, biases
+    _need_cuda(x, y, w, u, b, c)
+    _rows2d(x, "linear_pair x")
+    _rows2d(y, "linear_pair x")
+    (M, K), N = x.shape, w.shape[0]
+    if not (x.shape == y.shape and w.shape == u.shape == (N, K) and b.shape == c.shape == (N,) and x.dtype == y.dtype and w.dtype == u.dtype and b.dtype == c.dtype and x.stride() == y.stride()
+            and w.stride() == u.stride() and w.stride(1) == 1 and b.is_contiguous() and c.is_contiguous() and M > 0):
+        return None
+    apart = [divmod(q.data_ptr() - p.data_ptr(), p.element_size()) for p, q in ((x, y), (w, u), (b, c))]
+    if any(r for _, r in apart) or apart[2][0] == 0:
+        return None
+    wide = (N + 7) // 8 * 8
+    out = torch.empty((M, 2 * wide), device=x.device, dtype=torch.float32)
+    _lib.call("vy_linear_plain", "VyLinear", M=M, N=N, K=K, A=x.data_ptr(), lda=x.stride(0), a_dtype=_dt(x), W=w.data_ptr(), ldw=w.stride(0), w_dtype=_dt(w), act=UACT[None], scale=1.0,
+              out=out.data_ptr(), ld_out=2 * wide, out_dtype=_dt(out), batch=2, a_batch=apart[0][0], w_batch=apart[1][0], out_batch=wide, bias=b.data_ptr(), bias_dtype=_dt(b),
+              bias_batch=apart[2][0], stream=_stream())
+    return out[:, :N], out[:, wide:wide + N]
+
+
 def linear_plain(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = None, act: Optional[str] = None, scale: float = 1.0,
                  addend: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """out = act(x @ w.T + bias) * scale + addend with fp32 FMA accumulation (any shape; x and w may differ in dtype)."""
