@@ -197,6 +197,32 @@ def test_convolutions_in_one_launch(channels, tokens):
         assert _err(y, want.cpu()) < BOUND and torch.equal(s, t)
 
 
+@pytest.mark.parametrize("differ", ["weights", "inputs", "strides", "taps"])
+def test_convolutions_that_no_launch_can_share(differ):
+    """Inputs or weights of different types, strides or taps: what one call each gives."""
+    from vyomai_b200 import ops
+    from vyomai_b200.layers.mixers import GatedDeltaMixer
+    g = torch.Generator(device=DEV).manual_seed(3)
+    channels, tokens = (24, 24, 40), 50
+    batch = ops.PackedBatch(_i32([0, tokens, tokens + 1]), _i32([0, 9]), _i32([1, 0]), tokens)
+    xs = list(torch.randn(tokens + 1, sum(channels), generator=g, device=DEV).split(list(channels), 1))
+    ws = [torch.randn(c, 4 if differ != "taps" or c == 24 else 3, generator=g, device=DEV) for c in channels]
+    if differ == "weights":
+        ws[1] = ws[1].bfloat16()
+    elif differ == "inputs":
+        xs[2] = torch.randn(tokens + 1, sum(channels), generator=g, device=DEV).bfloat16()[:, :40]
+    elif differ == "strides":
+        xs[0] = xs[0].contiguous()
+    states = [torch.randn(2, *w.shape, generator=g, device=DEV)[..., 1:].contiguous() for w in ws]
+    alone = [s.clone() for s in states]
+    got = ops.causal_convs(batch, xs, ws, states).split(list(channels), 1)
+    for x, w, s, y, t in zip(xs, ws, alone, got, states):
+        assert torch.equal(y, ops.causal_conv(batch, x, w, s, out_dtype=torch.float32)) and torch.equal(s, t)
+    if differ == "weights":
+        cfg, w, _, forward = _delta_mixer(conv=torch.bfloat16)
+        assert bool(torch.isfinite(forward(GatedDeltaMixer(cfg, w, 1e-6, torch.float32, False))).all())
+
+
 @pytest.mark.parametrize("H,dk,dv", [(2, 20, 24), (1, 128, 64), (3, 64, 65), (2, 100, 130), (1, 8, 7)])
 def test_linear_attention_all_chunks_at_once(monkeypatch, H, dk, dv):
     """Chunks of 64 tokens: portions of 64 (the walk), 65, 128, 130 and 1 token side by side, then a continuation of 66."""

@@ -1497,16 +1497,21 @@ def moe_combine(part: torch.Tensor, inv: torch.Tensor, weight: torch.Tensor, add
     return out
 
 
-def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, act: Optional[str] = "silu",
-                out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """Depthwise causal convolution over time (w [channels, taps], last column = current token) + activation; `state`
-    [slots, channels, taps - 1] fp32 carries each sequence's last inputs and is advanced."""
+def _conv_operands(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor) -> None:
     _need_cuda(x, w, state)
     _rows2d(x, "causal_conv x")
-    ch, taps = w.shape
-    if x.shape[1] != ch or not w.is_contiguous() or state.dtype != torch.float32 or not state.is_contiguous():
+    if x.shape[1] != w.shape[0] or not w.is_contiguous() or state.dtype != torch.float32 or not state.is_contiguous():
         raise _lib.VyomError("causal_conv: shapes / layout")
-    out = torch.empty((x.shape[0], ch), device=x.device, dtype=out_dtype or x.dtype)
+
+
+def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, act: Optional[str] = "silu",
+                out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Depthwise causal convolution over time (w [channels, taps], last column = current token) + activation; `state`
+    [slots, channels, taps - 1] fp32 carries each sequence's last inputs and is advanced."""
+    _conv_operands(x, w, state)
+    ch, taps = w.shape
+    if out is None:
+        out = torch.empty((x.shape[0], ch), device=x.device, dtype=out_dtype or x.dtype)
     _lib.call("vy_causal_conv", "VyCausalConv", channels=ch, taps=taps, x=x.data_ptr(), ldx=x.stride(0), x_dtype=_dt(x), w=w.data_ptr(),
               w_dtype=_dt(w), state=state.data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
               stream=_stream(), rows=x.shape[0], **batch._kw())
@@ -1514,20 +1519,25 @@ def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: tor
 
 
 def causal_convs(batch: PackedBatch, xs, ws, states, act: Optional[str] = "silu") -> torch.Tensor:
-    """`causal_conv` of two or three inputs in one launch: rows of one stride, one dtype, weights of one dtype and as many taps. The fp32 outputs stand side by side in one tensor."""
-    _need_cuda(*xs, *ws, *states)
-    taps = ws[0].shape[1]
+    """`causal_conv` of two or three inputs. Their fp32 outputs stand side by side in one tensor. One launch where the inputs share a type and a row stride and the weights a type and
+    their number of taps, else one each."""
     for x, w, state in zip(xs, ws, states):
-        _rows2d(x, "causal_convs x")
-        if x.shape != (xs[0].shape[0], w.shape[0]) or w.shape[1] != taps or not w.is_contiguous() or w.dtype != ws[0].dtype or x.dtype != xs[0].dtype or x.stride(0) != xs[0].stride(0) \
-                or state.dtype != torch.float32 or not state.is_contiguous():
-            raise _lib.VyomError("causal_convs: shapes / layout")
+        _conv_operands(x, w, state)
     ch = [w.shape[0] for w in ws]
-    out = torch.empty((xs[0].shape[0], sum(ch)), device=xs[0].device, dtype=torch.float32)
+    rows, total = xs[0].shape[0], sum(ch)
+    if any(x.shape[0] != rows for x in xs):
+        raise _lib.VyomError("causal_convs: the inputs are of different lengths")
+    out = torch.empty((rows, total), device=xs[0].device, dtype=torch.float32)
+    if any(x.dtype != xs[0].dtype or x.stride(0) != xs[0].stride(0) or w.dtype != ws[0].dtype or w.shape[1] != ws[0].shape[1] for x, w in zip(xs, ws)):
+        at = 0
+        for x, w, state, c in zip(xs, ws, states, ch):
+            causal_conv(batch, x, w, state, act=act, out=out[:, at:at + c])
+            at += c
+        return out
     third = dict(channels3=ch[2], x3=xs[2].data_ptr(), w3=ws[2].data_ptr(), state3=states[2].data_ptr()) if len(ch) > 2 else {}
-    _lib.call("vy_causal_conv", "VyCausalConv", channels=ch[0], taps=taps, x=xs[0].data_ptr(), ldx=xs[0].stride(0), x_dtype=_dt(xs[0]), w=ws[0].data_ptr(),
+    _lib.call("vy_causal_conv", "VyCausalConv", channels=ch[0], taps=ws[0].shape[1], x=xs[0].data_ptr(), ldx=xs[0].stride(0), x_dtype=_dt(xs[0]), w=ws[0].data_ptr(),
               w_dtype=_dt(ws[0]), state=states[0].data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
-              stream=_stream(), rows=xs[0].shape[0], channels2=ch[1], x2=xs[1].data_ptr(), w2=ws[1].data_ptr(), state2=states[1].data_ptr(), **third, **batch._kw())
+              stream=_stream(), rows=rows, channels2=ch[1], x2=xs[1].data_ptr(), w2=ws[1].data_ptr(), state2=states[1].data_ptr(), **third, **batch._kw())
     return out
 
 
