@@ -197,6 +197,18 @@ def test_convolutions_in_one_launch(channels, tokens):
         assert _err(y, want.cpu()) < BOUND and torch.equal(s, t)
 
 
+@pytest.mark.parametrize("last", [4, 5, 6, 7])
+def test_convolutions_in_one_launch_keep_rows_on_16_bytes(last):
+    """q and k of a delta rule with an odd number of value channels are still read four channels at a time."""
+    from vyomai_b200 import ops
+    batch = ops.PackedBatch(_i32([0, 40]), _i32([0]), _i32([0]), 40)
+    xs, ws = [torch.randn(40, c, device=DEV) for c in (8, 8, last)], [torch.randn(c, 4, device=DEV) for c in (8, 8, last)]
+    xs = list(torch.cat(xs, 1).split([8, 8, last], 1))
+    got = ops.causal_convs(batch, xs, ws, [torch.zeros(1, w.shape[0], 3, device=DEV) for w in ws])
+    assert got.shape == (40, 16 + last) and got.stride(0) % 4 == 0 and got.data_ptr() % 16 == 0
+    assert torch.equal(got[:, 16:], ops.causal_conv(batch, xs[2], ws[2], torch.zeros(1, last, 3, device=DEV), out_dtype=torch.float32))
+
+
 @pytest.mark.parametrize("differ", ["weights", "inputs", "strides", "taps"])
 def test_convolutions_that_no_launch_can_share(differ):
     """Inputs or weights of different types, strides or taps: what one call each gives."""

@@ -1527,7 +1527,7 @@ def causal_convs(batch: PackedBatch, xs, ws, states, act: Optional[str] = "silu"
     rows, total = xs[0].shape[0], sum(ch)
     if any(x.shape[0] != rows for x in xs):
         raise _lib.VyomError("causal_convs: the inputs are of different lengths")
-    out = torch.empty((rows, total), device=xs[0].device, dtype=torch.float32)
+    out = torch.empty((rows, total + -total % 4), device=xs[0].device, dtype=torch.float32)[:, :total]   # rows on 16-byte boundaries, whatever the last input's width: readers take four channels at a time
     if any(x.dtype != xs[0].dtype or x.stride(0) != xs[0].stride(0) or w.dtype != ws[0].dtype or w.shape[1] != ws[0].shape[1] for x, w in zip(xs, ws)):
         at = 0
         for x, w, state, c in zip(xs, ws, states, ch):
