@@ -832,7 +832,8 @@ typedef struct VyCausalConv {
   void* out; int64_t ld_out; int32_t out_dtype;
   void* stream;
   int64_t rows; /* packed rows of the step, by which the form is chosen where portions are uneven; 0: n_seqs * max_new */
-  /* up to two further inputs in the same launch (channels 0: none), with the strides, types, taps and activation of the first; their outputs follow the first's columns in out */
+  /* up to two further inputs in the same launch (channels 0: none), with the strides, types, taps and activation of the first; their outputs follow the first's columns in out,
+   * whose rows hold all of them (ld_out >= channels + channels2 + channels3) */
   int32_t channels2, channels3;
   const void* x2; const void* w2; float* state2;
   const void* x3; const void* w3; float* state3;

@@ -209,6 +209,19 @@ def test_convolutions_in_one_launch_keep_rows_on_16_bytes(last):
     assert torch.equal(got[:, 16:], ops.causal_conv(batch, xs[2], ws[2], torch.zeros(1, last, 3, device=DEV), out_dtype=torch.float32))
 
 
+@pytest.mark.parametrize("short", [dict(ld_out=23), dict(ld_out=8), dict(ldx=7)])
+def test_convolutions_in_one_launch_check_their_rows(monkeypatch, short):
+    """Rows that do not hold what the call writes side by side, or reads, are refused before any launch."""
+    from vyomai_b200 import ops
+    from vyomai_b200._lib import VyomError
+    batch, p = ops.PackedBatch(_i32([0, 40]), _i32([0]), _i32([0]), 40), torch.randn(40, 24, device=DEV)
+    ws, states = [torch.randn(8, 4, device=DEV) for _ in range(3)], [torch.zeros(1, 8, 3, device=DEV) for _ in range(3)]
+    real = ops._lib.call
+    monkeypatch.setattr(ops._lib, "call", lambda fn, st, **kw: real(fn, st, **{**kw, **short}))
+    with pytest.raises(VyomError, match="further inputs"):
+        ops.causal_convs(batch, p.split(8, 1), ws, states)
+
+
 @pytest.mark.parametrize("differ", ["weights", "inputs", "strides", "taps"])
 def test_convolutions_that_no_launch_can_share(differ):
     """Inputs or weights of different types, strides or taps: what one call each gives."""

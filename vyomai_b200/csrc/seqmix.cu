@@ -1098,6 +1098,9 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   VY_CHECK_ARG(p->channels2 >= 0 && p->channels3 >= 0 && (p->channels2 > 0 || p->channels3 == 0) && static_cast<long long>(p->channels) + p->channels2 + p->channels3 <= INT_MAX &&
                    (p->channels2 == 0 || (p->x2 && p->w2 && p->x2 != p->out && (p->state2 || p->taps == 1))) &&
                    (p->channels3 == 0 || (p->x3 && p->w3 && p->x3 != p->out && (p->state3 || p->taps == 1))), "vy_causal_conv: bad further inputs");
+  VY_CHECK_ARG(p->channels2 == 0 || (p->ld_out >= static_cast<long long>(p->channels) + p->channels2 + p->channels3 && p->ldx >= p->channels && p->ldx >= p->channels2 && p->ldx >= p->channels3),
+               "vy_causal_conv: with further inputs a row of out holds all outputs (ld_out %lld, channels %d + %d + %d), a row of x any input's (ldx %lld)", static_cast<long long>(p->ld_out),
+               p->channels, p->channels2, p->channels3, static_cast<long long>(p->ldx));
   ConvDev d;
   d.cu = p->cu_tokens; d.pos0 = p->pos0; d.slot = p->slot;
   d.channels = p->channels; d.taps = p->taps;
