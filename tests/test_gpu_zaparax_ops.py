@@ -286,6 +286,25 @@ def test_grouped_experts(rows, experts, identity, top, ff, shared, width, gated)
     assert torch.equal(got, run())
 
 
+@pytest.mark.parametrize("ff,shared", [(8, 0), (72, 72), (72, 144), (64, 64)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_grouped_experts_keep_bad_weights_to_their_rows(ff, shared, bad):
+    """An expert whose weights are not finite meets the rows that are routed to it and no others, whatever its neighbours' contractions are filled up with."""
+    from vyomai_b200 import ops
+    rows, experts, width = 300, 4, 136
+    g = torch.Generator(device=DEV).manual_seed(ff)
+    bf = lambda *s: (torch.randn(*s, generator=g, device=DEV) * s[-1] ** -0.5).bfloat16()  # noqa: E731
+    h, up, down = bf(rows, width), bf(experts * 2 * ff + 2 * shared, width), bf(width, experts * ff + shared)
+    idx = torch.randint(0, 4, (rows, 1), generator=g, device=DEV, dtype=torch.int32)
+    weight = torch.ones(rows, 1, device=DEV)
+    run = lambda: ops.moe_grouped(h, idx, weight, up, down, experts=experts, ff=ff, shared_ff=shared,  # noqa: E731
+                                  workspace=torch.zeros(ops.moe_grouped_bytes(rows, experts, 1, width, ff, shared), dtype=torch.uint8, device=DEV))
+    clean = run()
+    up[2 * 2 * ff:3 * 2 * ff], down[:, 2 * ff:3 * ff] = bad, bad
+    got, hit = run(), idx[:, 0] == 2
+    assert not bool(torch.isfinite(got[hit]).any()) and torch.equal(got[~hit], clean[~hit])
+
+
 def test_grouped_experts_refuse_what_they_do_not_take():
     from vyomai_b200 import ops
     assert ops.moe_grouped_bytes(128, 4, 2, 64, 12, 0) == 0 and ops.moe_grouped_bytes(128, 4, 2, 60, 16, 0) == 0 and ops.moe_grouped_bytes(128, 4, 2, 64, 16, 24) == 0

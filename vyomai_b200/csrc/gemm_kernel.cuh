@@ -56,8 +56,8 @@ struct GemmDev {
   float* ws;
   PoisonRef poison;  // raised by a wait that timed out (mbar_wait_soft); the host sees it in vy_gemm / vy_gemm_poison_peek / vy_gemm_poisoned
   int tma_store;  // fast epilogues write back with TMA stores (tma_out / tma_aux of the launch)
-  // products of groups (WB_*_GROUPED): the m-tiles of the launch, {row of A, row of the result, row of B / its first k, segments of k}, their number; a segment's k are seg_k entries of B's
-  // rows and the first seg_k of A's rows, seg_rows further down for each segment
+  // products of groups (WB_*_GROUPED): the m-tiles of the launch, {row of A, row of the result, row of B / first run of its k, segments of k}, their number; a segment's k are a run of seg_k
+  // entries of B's rows and the first seg_k of A's rows, seg_rows further down for each segment
   const int4* groups;
   const int* group_count;
   int seg_k, seg_rows;
@@ -1053,14 +1053,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         if constexpr (GROUPED) {
           const int4 grp = g.groups[tile / n_tiles];
           const int n0 = (tile % n_tiles) * BN;
-          constexpr bool BY_ROW = WB == WB_GATED_GROUPED;   // a group's share of B: rows, or a run of k
+          constexpr bool BY_ROW = WB == WB_GATED_GROUPED;   // a group's share of B: rows, or runs of k, as a tensor [row of B][run][seg_k]
           for (int seg = 0; seg < grp.w; ++seg)
             for (int kb = 0; kb < num_kb; ++kb, ph ^= (s + 1 == STAGES), s = (s + 1 == STAGES) ? 0 : s + 1) {
               mbar_wait_soft(&empty_bar[s], ph ^ 1, g.poison);
               if (elect_one_sync()) {
                 mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
                 tma_load_2d(sA + s * Cfg::A_BYTES, &tma_a, &full_bar[s], kb * BK, grp.x + seg * g.seg_rows);
-                tma_load_2d(sB + s * B_BYTES, &tma_b, &full_bar[s], kb * BK + (BY_ROW ? 0 : grp.z + seg * g.seg_k), n0 + (BY_ROW ? grp.z : 0));
+                if constexpr (BY_ROW) tma_load_2d(sB + s * B_BYTES, &tma_b, &full_bar[s], kb * BK, n0 + grp.z);
+                else tma_load_3d(sB + s * B_BYTES, &tma_b, &full_bar[s], kb * BK, grp.z + seg, n0);   // past the run: zeros
               }
               __syncwarp();
             }

@@ -1,7 +1,7 @@
 // Mixture of SwiGLU experts over many rows, each expert on the rows that are routed to it (vy_moe_grouped). Five launches and no host decision:
 //   moe_plan_kernel      one CTA: the pairs (row, choice) placed by expert in row order, every expert's rows padded to whole tiles of 128; the tiles of both products
 //   moe_spread_kernel    a warp per row writes its copies
-//   gemm_kernel          twice, over the tiles of all experts (a tile's rows of A and of the result, its expert's rows or run of k of the weights come from the plan)
+//   gemm_kernel          twice, over the tiles of all experts (a tile's rows of A and of the result, its expert's rows or runs of k of the weights come from the plan)
 //   moe_merge_kernel     a row's results, weighted and summed in the order of its choices
 // A shared expert of m ff hidden columns is m experts that see every row in the first product and one with a contraction of m segments in the second.
 // Rows that fill up tiles are never written: what they hold meets no other row. 4059 rows, 28 experts of 256 and a shared one of 512, top 4 of 32 (4 identity), width 1024: all experts
@@ -108,12 +108,12 @@ __global__ void __launch_bounds__(MG_T) moe_plan_kernel(const __grid_constant__ 
       else hi = mid - 1;
     }
     d.up_tiles[i] = make_int4(i * MG_TILE, i * MG_TILE, lo * 2 * d.ff, 1);
-    d.down_tiles[i] = make_int4(i * MG_TILE, i * MG_TILE, lo * d.ff, 1);
+    d.down_tiles[i] = make_int4(i * MG_TILE, i * MG_TILE, lo, 1);
   }
   if (d.shared > 0) {
     for (int i = t; i < d.shared * per; i += MG_T)
       d.up_tiles[routed + i] = make_int4(d.cap + i % per * MG_TILE, d.cap + i * MG_TILE, (d.experts + i / per) * 2 * d.ff, 1);
-    for (int i = t; i < per; i += MG_T) d.down_tiles[routed + i] = make_int4(d.cap + i * MG_TILE, d.cap + i * MG_TILE, d.experts * d.ff, d.shared);
+    for (int i = t; i < per; i += MG_T) d.down_tiles[routed + i] = make_int4(d.cap + i * MG_TILE, d.cap + i * MG_TILE, d.experts, d.shared);
   }
   if (t == 0) {
     d.counts[0] = routed + d.shared * per;
@@ -211,7 +211,12 @@ int launch_grouped(const GemmDev& g, const void* a, long long a_rows, long long 
   using Cfg = GemmCfg<__nv_bfloat16, BN>;
   CUtensorMap ta, tb, tout;
   int rc = get_tmap_2d(&ta, VY_BF16, a, ka, a_rows, lda * 2, Cfg::BK, Cfg::BM);
-  if (rc == VY_OK) rc = get_tmap_2d(&tb, VY_BF16, b, kb, b_rows, ldb * 2, Cfg::BK, BN);
+  if (rc == VY_OK && WB == WB_GATED_GROUPED) rc = get_tmap_2d(&tb, VY_BF16, b, kb, b_rows, ldb * 2, Cfg::BK, BN);
+  if (rc == VY_OK && WB == WB_F32_GROUPED) {   // [row][expert][ff]: what a contraction reads past an expert's ff is zero, not the next expert's, whose infinity times zero would be a NaN
+    const uint64_t dims[3] = {static_cast<uint64_t>(ka), static_cast<uint64_t>(kb / ka), static_cast<uint64_t>(b_rows)}, strides[3] = {0, static_cast<uint64_t>(ka) * 2, static_cast<uint64_t>(ldb) * 2};
+    const uint32_t box[3] = {Cfg::BK, 1, BN};
+    rc = get_tensor_map_cached(&tb, VY_BF16, 3, b, dims, strides, box, 1);
+  }
   if (rc == VY_OK) rc = WB == WB_F32_GROUPED ? get_tmap_2d(&tout, VY_F32, out, out_cols, out_rows, static_cast<uint64_t>(out_cols) * 4, 16, 32, 3)
                                              : get_tmap_2d(&tout, VY_BF16, out, out_cols, out_rows, static_cast<uint64_t>(out_cols) * 2, 32, 32, 3);
   if (rc != VY_OK) return rc;
