@@ -168,3 +168,16 @@ def test_oracle_router_and_identity_experts():
     assert float((out - h * (2.0 / 3.0)).abs().max()) < 1e-12               # both identity experts, a third of the weight each
     out = O.mixture(h, W, {"router": {"experts": 1, "identity": 2, "top": 3}})
     assert float((out - h * (2.0 / 3.0) - O.silu(h) * h / 3.0).abs().max()) < 1e-12
+
+
+@pytest.mark.parametrize("experts,top,width,ff,shared,identity,rows,every,grouped,by_expert", [
+    (2, 2, 1024, 1024, 0, 0, 500, 27, 33, 59), (2, 2, 1024, 1024, 0, 0, 8000, 109, 152, 213), (4, 4, 1024, 512, 0, 0, 130, 26, 30, 91), (4, 4, 1024, 512, 0, 0, 8000, 109, 176, 375),
+    (4, 2, 1024, 512, 0, 0, 500, 27, 30, 93), (4, 1, 1024, 512, 0, 0, 500, 27, 34, 90), (4, 1, 1024, 512, 0, 0, 8000, 107, 79, 156), (1, 1, 1024, 1024, 0, 0, 2000, 32, 41, 50), (3, 2, 512, 512, 512, 0, 1000, 30, 37, 87),
+    (5, 2, 256, 64, 0, 0, 1000, 19, 33, 91), (8, 2, 256, 128, 128, 2, 1000, 22, 32, 152), (28, 4, 512, 128, 256, 4, 128, 25, 31, 267), (28, 4, 512, 128, 256, 4, 4000, 84, 67, 577),
+    (28, 4, 1024, 256, 512, 4, 40, 43, 35, 312), (28, 4, 1024, 256, 512, 4, 4000, 185, 108, 688), (256, 8, 1024, 128, 0, 0, 128, 124, 103, None), (256, 8, 1024, 128, 0, 0, 4000, 846, 164, None),
+    (256, 8, 2048, 256, 256, 0, 128, 271, 235, None), (64, 6, 1024, 256, 512, 0, 128, 70, 59, None), (8, 2, 4096, 14336, 0, 0, 512, 1258, 691, 861), (8, 2, 4096, 14336, 0, 0, 2048, 4442, 1824, 1647),
+    (8, 2, 4096, 14336, 0, 0, 8192, 21832, 5791, 5080), (16, 4, 2048, 2048, 2048, 0, 8192, 2794, 977, 1353)])
+def test_grouped_experts_are_chosen_where_they_were_measured_to_be_faster(experts, top, width, ff, shared, identity, rows, every, grouped, by_expert):
+    """Device us of the three forms (by_expert: not timed for more than 32 experts, whose launches are far behind)."""
+    from vyomai_b200.layers.mixers import grouped_experts_pay
+    assert grouped_experts_pay(rows, experts, top, width, ff, shared, identity) is (grouped < min(every, by_expert or every))

@@ -752,6 +752,26 @@ class PolyNormMLP:
         return self.down(u, addend=x_residual, out=x_residual)
 
 
+def grouped_experts_pay(rows: int, experts: int, top: int, width: int, ff: int, shared_ff: int, identity: int) -> bool:
+    """Is the grouped form of bf16 SwiGLU experts (ops.moe_grouped) estimated to be faster than all experts over all rows and than the sorted form, a pair of products per expert?
+
+    All experts over all rows leave no multiply-adds out, but their products are one large one each, in the fastest tiles. The grouped form has the chosen experts' alone, in tiles of 128 rows that
+    an expert's last one fills up, copies the rows and writes and reads a row of fp32 results per choice; the sorted form has launches of the host for every expert. Constants fitted to 273 steps of
+    1 to 256 experts, top 1 to 8, widths of 256 to 4096 and 34 to 16000 rows with each form timed (device us; sorted up to 32 experts). Of those the estimate takes the grouped form where another one
+    is faster by more than a hundredth in 4 (by 4 % at most) and another one where the grouped form is faster in 8 (by 7 %, with up to 4 experts by 17 %). All / grouped / sorted: 28 experts of 256 of width 1024 and a shared one of 512, top 4, 40 rows 43 / 35 / 312, 500 57 / 39 / 549, 4000
+    185 / 108 / 688, of 128 of width 512 128 rows 25 / 31 / 267; 2 of 1024, top 2, 2000 rows 44 / 55 / 85; 4 of 512, top 4, 8000 rows 109 / 176 / 375, top 2 108 / 112 / 217, top 1 107 / 79 / 156; 256 of 128,
+    top 8, 128 rows 124 / 103; 8 of 14336 of width 4096, top 2, 512 rows 1258 / 691 / 861, 8192 21832 / 5791 / 5080."""
+    chosen, shared = rows * top * experts / (experts + identity), shared_ff / ff
+    per_row, weights = 6.0 * width * ff, 6.0 * width * ff * experts          # multiply-adds (twice) of an expert's row; bytes of the experts' weights
+    active, blocks = min(experts, chosen), (rows + 127) // 128
+    tiles = active * max(1.0, chosen / experts / 128 + 0.5) + shared * blocks
+    moved = (chosen + (rows if shared_ff else 0)) * 10.0 * width             # copies in bf16, results in fp32, read again
+    every = max(weights * (1 + shared / experts) / 2.3e12, per_row * 128 * blocks * (experts + shared) / 1.45e15) + rows * 4.0 * ff * (experts + shared) / 2.5e12
+    grouped = 5e-6 + max(weights * active / experts / 4e12, per_row * 128 * tiles / 0.95e15) + moved / 4.5e12
+    by_expert = 2.6e-5 * active + max(weights * active / experts / 3e12, per_row * (chosen + shared * rows) / 1.15e15) + chosen * 12.0 * width / 2e12
+    return grouped <= every and grouped <= by_expert and (experts > 4 or rows >= 512)
+
+
 class MoEFeedForward:
     """Mixture of experts with an optional shared expert that runs for every token. Router logits (and the shared gate) are one
     product with fp32 accumulation and an fp32 result (its input is the layer input as the experts read it: bf16-rounded when the
@@ -773,8 +793,8 @@ class MoEFeedForward:
     on its own rows, and combine per token in choice order (no atomics, so the result does not depend on the batch). The sorted
     form costs two launches per expert and one host read of the experts' row counts, the all-experts form experts / top times
     the multiply-adds: a step of at least `sorted_min_rows` rows takes the sorted form when its estimated time is the smaller one
-    (`force_sorted` skips the estimate). SwiGLU experts in bf16 take the grouped form instead from `sorted_min_rows` rows on (from 33 on where the width is 1024 or more): the same
-    rows in five launches for all experts, without the host's read."""
+    (`force_sorted` skips the estimate). SwiGLU experts in bf16 may take the grouped form instead from `sorted_min_rows` rows on (from 33 on where the width is 1024 or more), where
+    its estimated time is the smallest (grouped_experts_pay): the same rows in five launches for all experts, without the host's read."""
 
     # multiply-add rates the estimate assumes for bf16 tensor-core products, fp32 ones on the tensor cores (vy_linear_plain, contractions of 256 and more) and FMA
     # ones (FLOP/s)
@@ -840,12 +860,12 @@ class MoEFeedForward:
         return self.top * per_choice + launches * self.LAUNCH_COST + moved < self.experts * per_choice
 
     def _grouped_workspace(self, h: torch.Tensor, batch) -> Optional[torch.Tensor]:
-        """Scratch for the grouped form, or None where it does not apply or is not the fastest. Device us of all experts / grouped, 28 experts of width / 4 and a shared one of width / 2, top 4:
-        width 512 100 rows 42 / 46, 130 42 / 43, 500 48 / 45, 4000 103 / 91; 1024 40 rows 58 / 47, 500 72 / 54, 4000 210 / 136; 2048 40 rows 99 / 88, 500 142 / 97, 2000 318 / 158."""
+        """Scratch for the grouped form, or None where it does not apply or is not the fastest."""
         rows = h.shape[0]
         enough = rows >= self.sorted_min_rows or (32 < rows and h.shape[1] >= 1024 and self.sorted_min_rows <= 128)
         if not (self.swiglu and not self.force_sorted and batch.max_new > 1 and enough and h.dtype == torch.bfloat16 and self.act_dtype == torch.bfloat16
-                and self.up_all.tensor_cores and self.down_all.tensor_cores and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0):
+                and self.up_all.tensor_cores and self.down_all.tensor_cores and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
+                and grouped_experts_pay(rows, self.experts, self.top, h.shape[1], self.ff, self.shared_ff, self.identity)):
             return None
         need = ops.moe_grouped_bytes(rows, self.experts, self.top, h.shape[1], self.ff, self.shared_ff)
         return ops._lend((need + 3) // 4, h.device)
