@@ -330,6 +330,31 @@ def test_mixture_in_both_forms(rows, f, width, dtype, sort):
     assert HU.rel_err(got, O.mixture(h.double(), W, f)) < (3e-5 if dtype == torch.float32 else 1.5e-2)
 
 
+@pytest.mark.parametrize("rows,experts,identity,top,ff,shared,width,kernel", [
+    (32, 28, 4, 4, 256, 512, 1024, None), (33, 28, 4, 4, 256, 512, 1024, "moe_plan"), (129, 28, 4, 4, 256, 256, 1024, "moe_plan"),
+    (127, 64, 2, 4, 128, 128, 512, None), (128, 64, 2, 4, 128, 128, 512, "moe_plan"), (1030, 12, 0, 2, 256, 0, 512, "moe_plan"), (300, 4, 0, 4, 64, 64, 512, None)])
+def test_experts_of_a_layer_take_the_grouped_form(monkeypatch, rows, experts, identity, top, ff, shared, width, kernel):
+    """The form that a bf16 layer with default settings takes by its rows and shapes: packed weights, the shared expert's gate beside the router's logits, identity experts; and the form
+    that it takes where no scratch can be had."""
+    from vyomai_b200 import ops
+    f = U.moe(ff=ff, experts=experts, top=top, identity=identity or None, shared=shared or None)
+    m, W = _experts(f, width, torch.bfloat16)
+    W = {k: v.bfloat16().double() for k, v in W.items()}   # what the layer holds
+    h = torch.randn(rows, width, generator=_gen(12)).to(torch.bfloat16)
+    batch, x = type("B", (), {"max_new": rows})(), h.to(DEV)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        y, ident = m.forward_parts(x, batch)
+        torch.cuda.synchronize()
+    assert any("moe_plan" in e.name for e in prof.events()) == (kernel is not None)
+    with monkeypatch.context() as mp:
+        mp.setattr(ops, "_lend", lambda floats, device: None)
+        other, ident2 = m.forward_parts(x, batch)
+    assert (ident is None) == (identity == 0) and (ident is None or torch.equal(ident, ident2))
+    want = O.mixture(h.double(), W, f)
+    for got in (y, other):
+        assert HU.rel_err(got.cpu().double() + (0.0 if ident is None else ident.cpu().double()[:, None] * h.double()), want) < 1.5e-2
+
+
 @pytest.mark.parametrize("sort", [False, True])
 def test_every_choice_is_an_identity_expert(sort):
     f = U.moe(experts=3, top=2, identity=2, shared=None)
