@@ -368,6 +368,14 @@ def test_score_exchanging_on_both_sides_of_the_line(H, G, d, dv, window, cap, ne
         at += new[s]
 
 
+@pytest.mark.parametrize("H,G,d,dv,window,cap,new,pos0,form", [
+    (16, 4, 48, 40, 0, 9.0, [40] * 40, [300] * 40, "tc"), (16, 4, 48, 40, 0, 9.0, [40] * 40, [200] * 40, "mma"), (16, 4, 48, 40, 256, 0.0, [40] * 40, [300] * 40, "tc"),
+    (16, 4, 48, 40, 255, 0.0, [40] * 40, [300] * 40, "mma"), (8, 1, 16, 16, 0, 9.0, [40] * 60, [300] * 60, "mma"), (8, 2, 64, 64, 0, 9.0, [33] * 60 + [1], [0] * 60 + [400], "tc")])
+def test_score_exchanging_form_by_the_keys_that_are_seen(H, G, d, dv, window, cap, new, pos0, form):
+    """More CTAs than run at once: the line is at 256 keys on average, cached ones among them."""
+    test_score_exchanging_on_both_sides_of_the_line(H, G, d, dv, window, cap, new, pos0, form, False)
+
+
 @pytest.mark.parametrize("new,H,dk,dv,carried,form", [
     ([129], 3, 64, 64, False, "tc"), ([256, 1, 130, 127], 4, 36, 40, True, "tc"), ([300, 128], 2, 100, 132, True, "tc"), ([140] * 5, 5, 128, 96, False, "tc"),
     ([200, 65], 2, 33, 64, True, "mma"), ([200], 2, 64, 30, False, "mma"), ([200], 2, 32, 64, False, "mma"), ([700] + [2] * 15, 16, 64, 64, True, "mma")])

@@ -560,12 +560,14 @@ talk_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
 static int tt_round(int n, int m) { return (n + m - 1) / m * m; }
 
 bool talk_attn_tc_applies(const TalkDev& d, int n_seqs, int max_new) {
-  const int per = d.heads / d.kv_heads, tq = TT_ROWS / d.heads, sees = d.window > 0 && d.window < max_new / 2 ? d.window : max_new / 2;
+  const int per = d.heads / d.kv_heads, tq = TT_ROWS / d.heads;
+  const long long whole = static_cast<long long>(d.tw) * d.bs - max_new / 2, sees = d.window > 0 && d.window < whole ? d.window : whole;   // keys a query of the longest sequence sees on average
   const long long ctas = static_cast<long long>(n_seqs) * ((max_new + tq - 1) / tq);
   // What a CTA costs before its first tile (7 us) is more than that of talk_attn_mma_kernel, several of which share an SM's time better; a tile costs less than half. It pays where all CTAs
   // run at once (64 x 16 tokens, 8 heads: 30 against 38 us) and where a query sees 256 keys on average (2 x 1437: 150 / 326;
   // 6 x 520 tokens, 32 heads: 1.06 to 2 times as fast). Past that: 148 x 16 tokens, 16 heads: 56 / 40; one of 2000 behind a window of 64: 58 / 54; behind one of 128: equal; 32 heads of 32 and
-  // 300 x 100 tokens: 1058 / 853. Beside one long prompt the CTAs of short ones find nothing to do, at 0.7 us each: 1500 and 20 of 3 tokens, 32 heads, 7900 CTAs: 175 / 136.
+  // 300 x 100 tokens: 1058 / 853. What is cached counts: mma.sync / here, 16 heads of 64, 40 x 64 tokens
+  // on 2000 cached ones 1008 / 466, on 500 304 / 157, behind a window of 256 163 / 107; 100 x 32 on 1000 596 / 324; 50 x 100 from position 0 beside one token on 4000 951 / 269. Beside one long prompt the CTAs of short ones find nothing to do, at 0.7 us each: 1500 and 20 of 3 tokens, 32 heads, 7900 CTAs: 175 / 136.
   if (ctas > num_sms() && (ctas > 8 * num_sms() || sees < 256 || d.dim + d.vdim < 64)) return false;   // 8 x 600, 8 heads of 16: 64 / 60
   // the rows of a warp (H / 4 heads) share a key / value head
   return (d.heads == 8 || d.heads == 16 || d.heads == 32) && (d.kv_heads == 1 || d.kv_heads == 2 || d.kv_heads == 4) && per % (d.heads / 4) == 0 && d.dim <= 64 && d.vdim <= 64;
