@@ -403,3 +403,11 @@ def test_tilings_are_heard_by_the_thread_that_collects_them():
             pass
         gemm_tune.heard(True, {"hint_bn": 32})
     assert outer == [2 | 256 << 4 | 3 << 16, 32 << 4] and inner == [0] and other == [None] and not gemm_tune.LISTENERS
+
+
+@pytest.mark.parametrize("shape", [(2000, 32, 64, 16, 4, 16, 16, 64), (700, 11, 64, 16, 4, 64, 64, 0), (2000, 32, 64, 8, 2, 16, 16, 64), (100, 4, 64, 64, 8, 64, 64, 0)])
+def test_scratch_of_score_exchanging_prompts_holds_the_sequences_it_is_asked_for(shape):
+    """vy_talk_attn goes through the sequences as many at a time as fit by what one asks for; whoever lends what n ask for has them all at once."""
+    from vyomai_b200._lib import lib
+    one = lib().vy_talk_attn_prompt_floats(1, *shape)
+    assert one > 0 and all(lib().vy_talk_attn_prompt_floats(n, *shape) == n * one for n in (2, 3, 20, 300))

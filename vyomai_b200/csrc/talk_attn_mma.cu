@@ -378,8 +378,8 @@ static WinDev talk_keys(const TalkDev& d) {   // the rows a step sees, in the wo
 
 long long talk_attn_mma_floats(const TalkDev& d, int n_seqs, int max_new) {
   if (!talk_mma_keys(d)) return 0;
-  const long long a = window_attn_split_floats(talk_keys(d), n_seqs, max_new), b = talk_attn_tc_applies(d, n_seqs, max_new) ? window_attn_tc_floats(talk_keys(d), n_seqs, max_new) : 0;
-  return a > b ? a : b;   // of either layout
+  const long long a = window_attn_split_floats(talk_keys(d), n_seqs, max_new), b = talk_attn_tc_applies(d, 1, max_new) ? window_attn_tc_floats(talk_keys(d), n_seqs, max_new) : 0;
+  return a > b ? a : b;   // of either layout; as many times one sequence's as there are, by which vy_talk_attn reckons how many fit
 }
 
 template <int HL, int N>
