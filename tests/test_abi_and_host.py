@@ -405,7 +405,7 @@ def test_tilings_are_heard_by_the_thread_that_collects_them():
     assert outer == [2 | 256 << 4 | 3 << 16, 32 << 4] and inner == [0] and other == [None] and not gemm_tune.LISTENERS
 
 
-@pytest.mark.parametrize("shape", [(2000, 32, 64, 16, 4, 16, 16, 64), (700, 11, 64, 16, 4, 64, 64, 0), (2000, 32, 64, 8, 2, 16, 16, 64), (100, 4, 64, 64, 8, 64, 64, 0)])
+@pytest.mark.parametrize("shape", [(2000, 32, 64, 16, 4, 16, 16, 64), (700, 11, 64, 16, 4, 64, 64, 0), (2000, 32, 64, 8, 2, 16, 16, 64), (100, 4, 64, 32, 4, 64, 48, 0)])
 def test_scratch_of_score_exchanging_prompts_holds_the_sequences_it_is_asked_for(shape):
     """vy_talk_attn goes through the sequences as many at a time as fit by what one asks for; whoever lends what n ask for has them all at once."""
     from vyomai_b200._lib import lib
