@@ -411,3 +411,13 @@ def test_scratch_of_score_exchanging_prompts_holds_the_sequences_it_is_asked_for
     from vyomai_b200._lib import lib
     one = lib().vy_talk_attn_prompt_floats(1, *shape)
     assert one > 0 and all(lib().vy_talk_attn_prompt_floats(n, *shape) == n * one for n in (2, 3, 20, 300))
+
+
+@pytest.mark.parametrize("M,N,K,tiled,split", [
+    (33, 9700, 516, 25, 22), (129, 3300, 580, 27, 22), (9700, 33, 1028, 43, 38), (10000, 1, 1024, 38, 34), (12000, 40, 1024, 41, 34), (1300, 1000, 256, 23, 20), (600, 1000, 512, 24, 19), (65, 4800, 4096, 143, 80),
+    (8192, 1024, 1024, 281, 82), (22849, 80, 1424, 147, 93), (1000, 1000, 256, 15, 20), (20000, 30, 256, 23, 37), (20000, 16, 512, 36, 37), (40000, 8, 512, 51, 62), (100000, 8, 1024, 201, 245), (40, 16000, 2048, 77, 82),
+    (3300, 129, 580, 30, 34), (9700, 33, 516, 26, 29), (64, 19200, 256, 23, 26), (32, 9700, 1024, 1, 2), (1000, 512, 512, 17, 18)])
+def test_fp32_products_are_split_ahead_where_that_was_measured_to_be_faster(M, N, K, tiled, split):
+    """us of either form (32 rows and fewer have forms of their own)."""
+    from vyomai_b200._lib import lib
+    assert (lib().vy_linear_plain_bytes(M, N, K) > 0) is (split < tiled)

@@ -464,6 +464,10 @@ def test_fp32_products_split_once(monkeypatch, M, N, K, out_dtype):
     x[1] *= 1e30
     x[2] *= 1e-30
     x[3], w[4] = 0.0, 0.0
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.linear_plain(x, w)
+        torch.cuda.synchronize()
+    assert any("linear_split_tc_kernel" in e.name for e in prof.events())
     exact = x.double() @ w.double().T
     for add in (None, addend):
         want = torch.nn.functional.silu(exact + bias.double()) * 0.5 + (0.0 if add is None else add.double())

@@ -262,12 +262,18 @@ int padded(int K) { return (K + ST_K - 1) / ST_K * ST_K; }
 
 }  // namespace
 
-// Where the tiled form (64 x 64, two CTAs per SM) has a CTA for every SM, of short contractions two: below, two launches and a tile's start cost more than the splitting saved. us, tiled / here:
-// K 256 1000 x 1000 (256 CTAs) 15 / 20, 1300 x 1000 23 / 20; 512 600 x 1000 (160) 23 / 22, 2000 x 1000 47 / 24, 1000 x 512 (128) 17 / 18; 1024 600 x 1000 40 / 28, 12000 x 64 44 / 38, 300 x 1024
-// (80) 27 / 23, for which the host's share of a call of two launches is more than that
+// Where the tiled form (64 x 64, two CTAs per SM) has a CTA for every SM and its estimated time (us) is the longer one. Below, two launches and a tile's start cost more than the splitting saved,
+// for the host too: 300 x 1024, K 1024 (80 CTAs) 27 / 23. Splitting ahead pays for results that many tiles of an operand share: it reads and writes both operands, and the tiles read them again, which
+// thin results over many rows do not repay. us, tiled / here: K 256 1000 x 1000 (256 CTAs) 15 / 20, 1300 x 1000 23 / 20, 20000 x 30 23 / 37; 512 600 x 1000 (160) 24 / 19, 2000 x 1000 47 / 24, 1000 x
+// 512 (128) 17 / 18, 20000 x 16 36 / 37, 40000 x 8 51 / 62; 580 129 x 3300 27 / 22, 3300 x 129 (rows of results not on 16 bytes) 30 / 34; 1024 600 x 1000 41 / 25, 33 x 9700 41 / 29, 9700 x 33 43 / 38,
+// 100000 x 8 201 / 245; 2048 40 x 16000 77 / 82; 4096 65 x 4800 143 / 80
 long long linear_split_bytes(int M, int N, int K) {
-  const long long ctas = ((M + 63LL) / 64) * ((N + 63LL) / 64);
-  if (M <= 32 || N <= 0 || K < 256 || ctas <= num_sms() || (K < 512 && ctas <= 2 * num_sms())) return 0;
+  const long long ctas = ((M + 63LL) / 64) * ((N + 63LL) / 64), tiles = ((M + ST_T - 1LL) / ST_T) * ((N + ST_T - 1LL) / ST_T);
+  if (M <= 32 || N <= 0 || K < 256 || ctas <= num_sms()) return 0;
+  const double sms = num_sms(), share = ctas / (2.0 * sms), halves = (static_cast<double>(M) + N) * K * 4.0, rounds = ceil(tiles / sms);
+  const double tiled = (share > 1.0 ? share + 0.4 : 1.0) * (5.5 + 0.0345 * K);
+  const double split = 9.5 + 2.0 * halves / 7e6 + (halves > 1e8 ? halves / 6e6 : 0.0) /* no longer in L2 */ + 3.0 + 0.0094 * K + (rounds - 1.0) * (3.0 + 0.0127 * K) + (N % 4 ? 6.0 : 0.0);
+  if (split >= tiled) return 0;
   const long long rows = static_cast<long long>(M) + N, bytes = (rows * padded(K) * 4 + 127) / 128 * 128 + rows * 4;
   return bytes <= (1LL << 30) ? bytes : 0;
 }

@@ -991,7 +991,7 @@ def linear_plain(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tenso
     if out is None:
         out = torch.empty((M, N), device=x.device, dtype=out_dtype or x.dtype)
     _rows2d(out, "linear_plain out")
-    need = int(_lib.lib().vy_linear_plain_bytes(M, N, K)) if M > 32 and K >= 256 and M * N > 500000 and x.dtype == torch.float32 and w.dtype == torch.float32 else 0
+    need = int(_lib.lib().vy_linear_plain_bytes(M, N, K)) if M > 32 and K >= 256 and x.dtype == torch.float32 and w.dtype == torch.float32 else 0   # none below, whatever N
     ws = _lend((need + 3) // 4, x.device)
     _lib.call("vy_linear_plain", "VyLinear", workspace=_ptr(ws), workspace_bytes=need if ws is not None else 0, M=M, N=N, K=K, A=x.data_ptr(), lda=x.stride(0), a_dtype=_dt(x), W=w.data_ptr(),
               ldw=w.stride(0), w_dtype=_dt(w), bias=_ptr(bias), bias_dtype=_dt(bias) if bias is not None else 0, addend=_ptr(addend),
