@@ -485,6 +485,20 @@ def test_fp32_products_split_once(monkeypatch, M, N, K, out_dtype):
         assert _err(ops.linear_plain(x, w), (x.double() @ w.double().T).cpu()) < BOUND
 
 
+@pytest.mark.parametrize("K", [512, 8192])
+@pytest.mark.parametrize("ratio", [2.0 ** k for k in (12, 16, 18, 20, 21, 22, 24, 40)])
+def test_fp32_products_split_once_beside_one_large_entry_per_row(monkeypatch, K, ratio):
+    """One entry per row, in one stretch of 64, is `ratio` times the others and meets a zero: the unit of a whole row, results on both sides of the line below which they are computed again
+    (about 2^16 sqrt(K) here). No bits fewer than where every tile is split by itself, whose units are its own."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x, w = torch.randn(260, K, generator=g, device=DEV), torch.randn(2600, K, generator=g, device=DEV)
+    x[:, 77], w[:, 77] = ratio, 0.0
+    want = (x.double() @ w.double().T).cpu()
+    ahead, tiles = (_err(y, want) for y in _both(monkeypatch, "vy_linear_plain_bytes", lambda: ops.linear_plain(x, w)))
+    assert ahead < 1.02 * tiles and ahead < BOUND   # 2 %: errors of 676,000 results each
+
+
 @pytest.mark.parametrize("ratio", [2.0 ** 16, 2.0 ** 20, 2.0 ** 24, 1e8, 1e12, 1e30])
 def test_fp32_products_of_entries_far_below_their_row_s_largest(ratio):
     """One entry per row is `ratio` times the others and meets a zero: the sums consist of the small ones alone."""

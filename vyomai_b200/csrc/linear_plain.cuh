@@ -56,9 +56,11 @@ static __device__ __noinline__ float lin_dot(const float* a, const float* w, int
   return warp_sum(acc);
 }
 
-// An entry's halves are off by at most 2^-48 of the largest entry of its row and tile (split_mma.cuh), so a product is as good as an fp32 one unless it is
-// this small beside its rows' largest entries: then, as where an infinity or NaN went in (the halves of an infinity would all be NaN), it is computed again
-// in FMAs. At 2^-16 the halves' share is below 2^-25 of the product; of normal numbers' products 2 to 6 in a million are that small
+// An entry's halves are off by at most 2^-49 of the largest entry under its unit (split_mma.cuh): a row's in a tile of 64 k where tiles are split, a whole row's where operands are split ahead.
+// So a product is as good as an fp32 one unless it is very small beside the product of its rows' largest entries: then, as where an infinity or NaN went in (the halves of an infinity would
+// all be NaN), it is computed again in FMAs. At 2^-16 of it the halves' share of a result is at most K 2^-32 and, signs being random, about sqrt(K) 2^-33: 2^-28 at K 1024, 2^-26 at 16384, where
+// an fp32 sum's rounding is 2^-23. Of normal numbers' products 2 to 6 in a million are that small. One entry of 2^12 to 2^40 per row in one stretch of 64, error against 64 bits of tiles / of
+// operands split ahead: K 1024 1.55 / 1.45e-7 to 1.20 / 1.20e-7, 8192 2.46 / 1.98e-7 to 2.94 / 2.94e-7, never above
 constexpr float LS_SMALL = 0x1p-16f * (1 << SPLIT_TOP) * (1 << SPLIT_TOP);
 
 // linear_split_tc.cu: scratch of the tcgen05 form (0: not for these sizes), and the form itself, two launches
