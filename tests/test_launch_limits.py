@@ -39,3 +39,19 @@ def test_register_shares_that_a_build_does_not_have_choose_another_form():
         if os.path.exists(log):
             used = re.findall(rf"entry function '[^']*{kernel}[^']*'(?:(?!entry function).)*?Used (\d+) registers", open(log).read(), re.S)
             assert len(used) == forms and all((int(u) + 7) // 8 * 8 == count for u in used)
+
+
+def test_register_shares_of_builds_made_by_including_a_file():
+    """linear_attn_tc_fixed.cu builds linear_attn_tc.cu's kernels once more, with registers of its own: its rule asks for the same count, and the build that is here has it."""
+    csrc = os.path.join(ROOT, "vyomai_b200", "csrc")
+    for path in glob.glob(os.path.join(csrc, "*.cu")):   # every file that builds such kernels by including them
+        src = open(path).read()
+        if re.search(r'#include "\w+\.cu"', src):
+            assert os.path.basename(path) == "linear_attn_tc_fixed.cu" and '#include "linear_attn_tc.cu"' in src
+    src = open(os.path.join(csrc, "linear_attn_tc.cu")).read()
+    count = int(re.search(r"\bLT_REGS = (\d+)", src).group(1))
+    assert "la_fixed_registers()" in src[src.index("bool linear_attn_tc_applies("):] and re.search(r"bool la_fixed_registers\(\) \{ return la_registers<false, VY_UACT_SILU>\(\); \}", src)
+    log = os.path.join(csrc, "build", "linear_attn_tc_fixed.ptxas.log")
+    if os.path.exists(log):
+        used = re.findall(r"entry function '[^']*la_outputs_tc_kernel[^']*'(?:(?!entry function).)*?Used (\d+) registers", open(log).read(), re.S)
+        assert len(used) == 1 and (int(used[0]) + 7) // 8 * 8 == count
