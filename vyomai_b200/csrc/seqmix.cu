@@ -518,12 +518,22 @@ struct ConvDev {
   int act;
   void* out; long long ld_out; int out_dt;
   int first;   // first channel of the launch
-  int total;   // channels of all parts; those behind the first part's belong to `more`
+};
+// several inputs: `one`'s, and those of the channels behind. Kernels of their own, since a single input's would be up to a sixth slower with the choice in front (16 sequences of 2063 tokens, 33
+// channels 12.0 us without, 14.2 with it)
+struct ConvMoreDev {
+  ConvDev one;
   ConvPart more[2];
 };
-// the part that channel c of the launch belongs to takes the first one's place; c becomes a channel of it
-__device__ __forceinline__ void conv_select(ConvDev& d, const ConvDev& all, int& c) {
-  if (c < d.channels) return;
+template <bool MORE> struct ConvArgs { using Type = ConvDev; };
+template <> struct ConvArgs<true> { using Type = ConvMoreDev; };
+__device__ __forceinline__ const ConvDev& conv_one(const ConvDev& all) { return all; }
+__device__ __forceinline__ const ConvDev& conv_one(const ConvMoreDev& all) { return all.one; }
+// the part that channel c of the launch belongs to, in the first one's place; c becomes a channel of it (past its last one if there is none)
+__device__ __forceinline__ const ConvDev& conv_part(const ConvDev& all, ConvDev&, int&) { return all; }
+__device__ __forceinline__ const ConvDev& conv_part(const ConvMoreDev& all, ConvDev& d, int& c) {
+  d = all.one;
+  if (c < d.channels) return d;
   int at = d.channels;
   const bool last = c - at >= all.more[0].channels;
   if (last) at += all.more[0].channels;
@@ -534,6 +544,7 @@ __device__ __forceinline__ void conv_select(ConvDev& d, const ConvDev& all, int&
   d.channels = p.channels;
   d.out = static_cast<char*>(d.out) + static_cast<long long>(at) * (d.out_dt == VY_F32 ? 4 : 2);
   c -= at;
+  return d;
 }
 
 constexpr int CONV_MAX_TAPS = 16;
@@ -558,16 +569,16 @@ __device__ __forceinline__ void conv_new_taps(const ConvDev& d, int c, int base,
 // outputs. Bound by instructions (71 to 75 % of the issue slots). fp32, 4 taps, the walk of 32 tokens that loaded an input per tap and output / this:
 // 8192 tokens x 1024 channels 65.5 / 31.8 us, x 512 40.4 / 17.4 us, 80 tokens x 512 31.1 / 7.3 us. The first CTA column of a sequence, the only
 // one that reads the slot's old taps, writes the new ones (a launch of its own before, 2.2 us). TAPS >= taps
-template <int TAPS>
-__global__ void __launch_bounds__(128) causal_conv_kernel(const __grid_constant__ ConvDev all) {
+template <int TAPS, bool MORE>
+__global__ void __launch_bounds__(128) causal_conv_kernel(typename ConvArgs<MORE>::Type all) {
   pdl_trigger();
   pdl_wait();
-  ConvDev d = all;
-  int c = d.first + blockIdx.y * blockDim.x + threadIdx.x;
+  int c = conv_one(all).first + blockIdx.y * blockDim.x + threadIdx.x;
   const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
-  const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (c >= d.total || i0 >= n) return;
-  conv_select(d, all, c);
+  const int base = conv_one(all).cu[s], n = conv_one(all).cu[s + 1] - base;
+  ConvDev of;
+  const ConvDev& d = conv_part(all, of, c);
+  if (c >= d.channels || i0 >= n) return;
   const bool carried = d.pos0[s] > 0;
   float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
   float x[CONV_TOK + TAPS - 1], w[TAPS];
@@ -597,16 +608,17 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const __grid_constant_
 
 // The same for four neighbouring channels per thread (fp32 rows on 16-byte boundaries, up to 4 taps): a quarter of the loads, stores and addresses per output,
 // and the SiLU without a division. Bound by the bytes and the exponentials: 7970 tokens x 1024 channels 30.1 us with one channel per thread, 18.1 here; x 512 16.7, 11.6.
-__global__ void __launch_bounds__(128) causal_conv_quads_kernel(const __grid_constant__ ConvDev all) {
+template <bool MORE>
+__global__ void __launch_bounds__(128) causal_conv_quads_kernel(typename ConvArgs<MORE>::Type all) {
   pdl_trigger();
   pdl_wait();
   constexpr int TAPS = 4;
-  ConvDev d = all;
   int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
   const int s = blockIdx.z, i0 = blockIdx.x * CONV_TOK;
-  const int base = d.cu[s], n = d.cu[s + 1] - base;
-  if (c >= d.total || i0 >= n) return;
-  conv_select(d, all, c);
+  const int base = conv_one(all).cu[s], n = conv_one(all).cu[s + 1] - base;
+  ConvDev of;
+  const ConvDev& d = conv_part(all, of, c);
+  if (c >= d.channels || i0 >= n) return;
   const bool carried = d.pos0[s] > 0;
   float* stp = d.state + (static_cast<long long>(d.slot[s]) * d.channels + c) * (d.taps - 1);
   const float* xp = reinterpret_cast<const float*>(d.x) + static_cast<long long>(base) * d.ldx + c;
@@ -1108,9 +1120,11 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   d.w = p->w; d.w_dt = p->w_dtype;
   d.state = p->state; d.act = p->act;
   d.out = p->out; d.ld_out = p->ld_out; d.out_dt = p->out_dtype;
-  d.more[0] = {p->x2, p->w2, p->state2, p->channels2};
-  d.more[1] = {p->x3, p->w3, p->state3, p->channels3};
-  d.total = p->channels + p->channels2 + p->channels3;
+  ConvMoreDev m;
+  m.more[0] = {p->x2, p->w2, p->state2, p->channels2};
+  m.more[1] = {p->x3, p->w3, p->state3, p->channels3};
+  const int total = p->channels + p->channels2 + p->channels3;
+  const bool more = p->channels2 > 0;
   cudaStream_t st = static_cast<cudaStream_t>(p->stream);
   const auto quads = [](const void* q, int dt, long long ld) { return dt == VY_F32 && reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0; };
   // Four channels per thread from two CTAs per SM on that find tokens: 1024 channels x 1200, 2080, 4160 tokens 8.9 / 10.1, 12.3 / 11.7, 19.7 / 13.9 us (a channel per thread / four);
@@ -1119,20 +1133,23 @@ extern "C" int vy_causal_conv(const VyCausalConv* p) {
   const long long tiles = static_cast<long long>(p->n_seqs) * ((p->max_new + CONV_TOK - 1) / CONV_TOK), filled = p->rows > 0 ? (p->rows + CONV_TOK - 1) / CONV_TOK : tiles;
   // Further inputs count with the first: 512, 512 and 1024 channels of 4 x 2048 tokens one after the other 17.8, 11.8 and 20.8 us, together 39
   bool aligned = p->taps <= 4 && p->channels % 4 == 0 && quads(d.x, d.x_dt, d.ldx) && quads(d.out, d.out_dt, d.ld_out);
-  for (const ConvPart& m : d.more) aligned = aligned && (m.channels == 0 || (m.channels % 4 == 0 && quads(m.x, d.x_dt, d.ldx)));
-  if ((filled * d.total >= 2LL * 512 * num_sms() || tiles * d.total >= 10LL * 512 * num_sms()) && aligned && d.total <= 65535 * 512) {
-    d.first = 0;
-    const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, (d.total + 511) / 512, p->n_seqs);
-    VY_CUDA_OK(launch_kernel(causal_conv_quads_kernel, grid, dim3(128), 0, st, d));
+  for (const ConvPart& q : m.more) aligned = aligned && (q.channels == 0 || (q.channels % 4 == 0 && quads(q.x, d.x_dt, d.ldx)));
+  d.first = 0;
+  if ((filled * total >= 2LL * 512 * num_sms() || tiles * total >= 10LL * 512 * num_sms()) && aligned && total <= 65535 * 512) {
+    const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, (total + 511) / 512, p->n_seqs);
+    m.one = d;
+    VY_CUDA_OK(more ? launch_kernel(causal_conv_quads_kernel<true>, grid, dim3(128), 0, st, m) : launch_kernel(causal_conv_quads_kernel<false>, grid, dim3(128), 0, st, d));
     VY_LAUNCH_OK();
     count_launch();
     return VY_OK;
   }
-  const long long blocks = (d.total + 127LL) / 128;
+  const long long blocks = (total + 127LL) / 128;
   for (long long b = 0; b < blocks; b += 65535) {   // one launch, up to 8 million channels
     d.first = static_cast<int>(128 * b);
     const dim3 grid((p->max_new + CONV_TOK - 1) / CONV_TOK, static_cast<unsigned>(blocks - b < 65535 ? blocks - b : 65535), p->n_seqs);
-    VY_CUDA_OK(p->taps <= 4 ? launch_kernel(causal_conv_kernel<4>, grid, dim3(128), 0, st, d) : launch_kernel(causal_conv_kernel<CONV_MAX_TAPS>, grid, dim3(128), 0, st, d));
+    m.one = d;
+    VY_CUDA_OK(more ? (p->taps <= 4 ? launch_kernel(causal_conv_kernel<4, true>, grid, dim3(128), 0, st, m) : launch_kernel(causal_conv_kernel<CONV_MAX_TAPS, true>, grid, dim3(128), 0, st, m))
+                    : p->taps <= 4 ? launch_kernel(causal_conv_kernel<4, false>, grid, dim3(128), 0, st, d) : launch_kernel(causal_conv_kernel<CONV_MAX_TAPS, false>, grid, dim3(128), 0, st, d));
     VY_LAUNCH_OK();
     count_launch();
   }
