@@ -128,6 +128,18 @@ def test_thin_products(M, N, K, dtype):
     assert _err(one, 0.5 * torch.nn.functional.silu(want[0]).cpu()) < BOUND
 
 
+@pytest.mark.parametrize("M,N,K,thin", [(500, 512, 24, True), (390, 512, 24, False), (300, 1030, 32, True), (60, 1030, 32, False), (40, 256, 16, True), (40, 256, 12, True), (800, 300, 20, True), (40, 254, 12, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_thin_products_on_both_sides_of_the_line(M, N, K, thin, dtype):
+    """Weights that come 16 bytes at a time, contractions that fill up a step of eight or four and not."""
+    from vyomai_b200 import ops
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.linear_plain(torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV).to(dtype), out_dtype=torch.float32)
+        torch.cuda.synchronize()
+    assert any("linear_thin_kernel" in e.name for e in prof.events()) == thin
+    test_thin_products(M, N, K, dtype)
+
+
 def _delta_mixer(W=64, H=2, D=32, rank=16, conv=torch.float32):
     """(weights, forward(mixer) on the same 200 tokens) of a delta mixer whose input products are made here."""
     from types import SimpleNamespace

@@ -61,17 +61,27 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(LinDev d) {
 constexpr int LN_ROWS = 64, LN_K = 32;   // rows per CTA: half as many where CTAs would be too few
 template <int KP>
 __device__ __forceinline__ void thin_weights(const LinDev& d, int n, float (&w)[KP]) {
-  if (d.w_dt == VY_BF16 && d.K == KP && n < d.N && d.ldw % 8 == 0 && reinterpret_cast<uintptr_t>(d.W) % 16 == 0) {
+  const bool al = n < d.N && reinterpret_cast<uintptr_t>(d.W) % 16 == 0;
+  if (al && d.w_dt == VY_BF16 && d.K % 8 == 0 && d.ldw % 8 == 0) {
     const uint4* p = reinterpret_cast<const uint4*>(static_cast<const char*>(d.W) + 2 * static_cast<long long>(n) * d.ldw);
 #pragma unroll
     for (int i = 0; i < KP / 8; ++i) {
-      const uint4 v = p[i];
+      const uint4 v = 8 * i < d.K ? p[i] : make_uint4(0u, 0u, 0u, 0u);
       const unsigned u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         w[8 * i + 2 * j] = __uint_as_float(u[j] << 16);
         w[8 * i + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
       }
+    }
+    return;
+  }
+  if (al && d.w_dt == VY_F32 && d.K % 4 == 0 && d.ldw % 4 == 0) {
+    const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(d.W) + static_cast<long long>(n) * d.ldw);
+#pragma unroll
+    for (int i = 0; i < KP / 4; ++i) {
+      const float4 v = 4 * i < d.K ? p[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
     }
     return;
   }
@@ -470,8 +480,9 @@ extern "C" int vy_linear_plain(const VyLinear* p) {
       count_launch();
       return VY_OK;
     }
-    // K up to 32, fp32 results in pairs. A CTA has 512 features: 128 of them, 7970 rows 7.2 us in tiles, 7.9 here; 512 16.9, 9.7; 33 x 512 5.8, 5.0; 2000 x 2048, K 32 22.3, 14.2
-    if (p->K <= LN_K && p->N >= 256 && !d.addend && d.out_dt == VY_F32 && reinterpret_cast<uintptr_t>(d.out) % 8 == 0 && d.ld_out % 2 == 0 && (batch == 1 || d.out_batch % 2 == 0) &&
+    // K up to 32, fp32 results in pairs. A CTA has 512 features: 128 of them, 7970 rows 7.2 us in tiles, 7.9 here; 512 16.9, 9.7; 33 x 512 5.8, 5.0; 2000 x 2048, K 32 22.3, 14.2. Beyond 16
+    // a CTA's weights take longer to come than few rows' tiles: K 24 44 x 4034 7.2, 8.2, 187 x 316 7.6, 8.2, 2061 x 478 8.9, 8.5; 32 81 x 462 7.2, 8.1, 355 x 2830 9.0, 8.3
+    if (p->K <= LN_K && p->N >= 256 && (p->K <= 16 || static_cast<long long>(p->M) * p->N >= 200000) && !d.addend && d.out_dt == VY_F32 && reinterpret_cast<uintptr_t>(d.out) % 8 == 0 && d.ld_out % 2 == 0 && (batch == 1 || d.out_batch % 2 == 0) &&
         p->M <= 65535 * (LN_ROWS / 4)) {
       const long long wide = (p->N + 511LL) / 512 * batch;
       const int per_cta = wide * (p->M / LN_ROWS) >= num_sms() ? LN_ROWS : wide * (2 * p->M / LN_ROWS) >= num_sms() ? LN_ROWS / 2 : LN_ROWS / 4;
