@@ -497,6 +497,21 @@ def test_fp32_products_split_once(monkeypatch, M, N, K, out_dtype):
         assert _err(ops.linear_plain(x, w), (x.double() @ w.double().T).cpu()) < BOUND
 
 
+@pytest.mark.parametrize("M,N,K", [(700, 1600, 512), (1300, 1001, 516)])
+def test_fp32_products_split_once_of_rows_that_hold_nan(M, N, K):
+    """Whole rows of NaN, one NaN in a row of either operand, infinities beside it: what float64 gives, and the other rows as without."""
+    from vyomai_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    clean = ops.linear_plain(x, w)
+    nan, inf = float("nan"), float("inf")
+    x[3:90], x[200, 7], x[201, 5], x[202, 5:9], w[40, 9], w[41, 1], w[42:60] = nan, nan, inf, torch.tensor([inf, nan, 1.0, -inf], device=DEV), nan, -inf, nan
+    got, want = ops.linear_plain(x, w), x.double() @ w.double().T
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want)) and torch.equal(got[torch.isinf(got)].sign(), want[torch.isinf(want)].sign().float())
+    ok = torch.isfinite(got)
+    assert torch.equal(got[ok], clean[ok])
+
+
 @pytest.mark.parametrize("K", [512, 8192])
 @pytest.mark.parametrize("ratio", [2.0 ** k for k in (12, 16, 18, 20, 21, 22, 24, 40)])
 def test_fp32_products_split_once_beside_one_large_entry_per_row(monkeypatch, K, ratio):

@@ -20,7 +20,7 @@ struct HalvesDev {
   const float* A; const float* W; long long lda, ldw;
   int M, N, K, kp;
   __half* a_hi; __half* a_lo; __half* w_hi; __half* w_lo;
-  float* units;   // of A's rows, then of W's: 0 for a row of zeros
+  float* units;   // of A's rows, then of W's: 0 for a row of zeros, NaN for one that holds a NaN
 };
 
 __global__ void __launch_bounds__(256) linear_halves_kernel(const __grid_constant__ HalvesDev d) {
@@ -33,19 +33,20 @@ __global__ void __launch_bounds__(256) linear_halves_kernel(const __grid_constan
   const float* p = isa ? d.A + static_cast<long long>(r) * d.lda : d.W + static_cast<long long>(r) * d.ldw;
   __half* hi = (isa ? d.a_hi : d.w_hi) + static_cast<long long>(r) * d.kp;
   __half* lo = (isa ? d.a_lo : d.w_lo) + static_cast<long long>(r) * d.kp;
-  float m = 0.f;
+  unsigned top = 0u;   // as bits: a NaN's are the largest
   for (int k0 = 4 * lane; k0 < d.K; k0 += 512) {
     float4 x[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       x[u] = k0 + 128 * u < d.K ? *reinterpret_cast<const float4*>(p + k0 + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
+    for (int u = 0; u < 4; ++u)
+      top = max(top, max(max(__float_as_uint(fabsf(x[u].x)), __float_as_uint(fabsf(x[u].y))), max(__float_as_uint(fabsf(x[u].z)), __float_as_uint(fabsf(x[u].w)))));
   }
-  m = warp_max(m);
+  const float m = __uint_as_float(__reduce_max_sync(0xffffffffu, top));
   const int e = split_exponent(m);
   const float sc = split_scale(e);
-  if (lane == 0) d.units[row] = m > 0.f ? pow2i(e - SPLIT_TOP) : 0.f;
+  if (lane == 0) d.units[row] = m != m ? m : m > 0.f ? pow2i(e - SPLIT_TOP) : 0.f;
   for (int k0 = 8 * lane; k0 < d.kp; k0 += 512) {
     float4 x[4];
 #pragma unroll
@@ -68,7 +69,8 @@ __global__ void __launch_bounds__(256) linear_halves_kernel(const __grid_constan
   }
 }
 
-// 32 rows x 16 columns of results that lack their columns' units: those that are too small beside their rows' largest entries computed again, then out. A function, since code that is
+// 32 rows x 16 columns of results that lack their columns' units: those that are too small beside their rows' largest entries, or not finite (but where a row or column has a NaN and its results
+// with it: 40 rows of NaN in 4000 x 1024, K 512, 1020 us otherwise), computed again, then out. A function, since code that is
 // unrolled for every run of columns comes from memory (33 x 64, K 256: 23 us instead of 10)
 static __device__ __noinline__ void finish(const LinDev& d, float* mine, const float* uw, float small, int m0, int n0) {
   const int lane = threadIdx.x & 31;
@@ -82,7 +84,11 @@ static __device__ __noinline__ void finish(const LinDev& d, float* mine, const f
       if (!(fabsf(x[k]) >= small * us[k] && fabsf(x[k]) < INFINITY)) again |= 1u << (i + k);
     *reinterpret_cast<float4*>(mine + lane * ST_LD + i) = make_float4(x[0], x[1], x[2], x[3]);
   }
-  if (m0 + lane >= d.M) again = 0u;
+  if (m0 + lane >= d.M || small != small) again = 0u;
+  if (again)
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+      if (uw[i] != uw[i]) again &= ~(1u << i);
   if (d.N - n0 < 16) again &= d.N > n0 ? (1u << (d.N - n0)) - 1u : 0u;
   for (unsigned rows = __ballot_sync(0xffffffffu, again != 0u); rows; rows &= rows - 1) {
     const int src = __ffs(rows) - 1;
