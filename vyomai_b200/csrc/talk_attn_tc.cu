@@ -9,7 +9,7 @@
 // values, one the next tile's scores, two bring keys and values, sixteen hold the rows, four threads a row with 16 keys and 16 channels each. A tile's values are added while the next one's
 // exchange is under way.
 //
-// What bounds it: 6700 cycles a tile. Products are under way in 5600: 120 of 128 x 64 x 16 at 45 to 60 cycles (the pipe's own counter: active 44 % of the time), where those of a key / value head keep a quarter of their
+// What bounds it: 6700 cycles a tile. Products are under way in 5600: 120 of 128 x 64 x 16 at 45 to 60 cycles (the pipe's own counter: active 47 % of the time), where those of a key / value head keep a quarter of their
 // rows when there are four. The rows' own chain - 2000 for caps and halves, 1000 until the exchange is back, 1600 for the softmax - hides behind them or hides them. A CTA's start
 // takes 13000 (queries, `talk` and 64 keys from memory, instructions not yet in the cache). Eight warps of rows with two tiles' scores in tensor memory, products of all scores against all
 // rows: 218 us; masked products by one warp: 193; by two: 150.
