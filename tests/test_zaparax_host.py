@@ -178,6 +178,7 @@ def test_oracle_router_and_identity_experts():
     (256, 8, 2048, 256, 256, 0, 128, 271, 235, None), (64, 6, 1024, 256, 512, 0, 128, 70, 59, None), (8, 2, 4096, 14336, 0, 0, 512, 1258, 691, 861), (8, 2, 4096, 14336, 0, 0, 2048, 4442, 1824, 1647),
     (8, 2, 4096, 14336, 0, 0, 8192, 21832, 5791, 5080), (16, 4, 2048, 2048, 2048, 0, 8192, 2794, 977, 1353)])
 def test_grouped_experts_are_chosen_where_they_were_measured_to_be_faster(experts, top, width, ff, shared, identity, rows, every, grouped, by_expert):
-    """Device us of the three forms (by_expert: not timed for more than 32 experts, whose launches are far behind)."""
+    """Device us of the three forms (by_expert: not timed for more than 32 experts, whose launches are far behind). Where the device is through before the host the form with fewer launches
+    is the faster one."""
     from vyomai_b200.layers.mixers import grouped_experts_pay
-    assert grouped_experts_pay(rows, experts, top, width, ff, shared, identity) is (grouped < min(every, by_expert or every))
+    assert grouped_experts_pay(rows, experts, top, width, ff, shared, identity) is (grouped < min(every, by_expert or every) or (experts + identity >= 16 and max(every, grouped) < 39))

@@ -11,6 +11,7 @@ convolutions, decays, recurrences, the residual) is fp32, and only a projection'
 """
 from __future__ import annotations
 
+import functools
 from typing import Dict, List, Optional, Tuple
 
 import torch
@@ -752,13 +753,14 @@ class PolyNormMLP:
         return self.down(u, addend=x_residual, out=x_residual)
 
 
+@functools.lru_cache(maxsize=4096)   # of numbers alone; 3 us a call otherwise
 def grouped_experts_pay(rows: int, experts: int, top: int, width: int, ff: int, shared_ff: int, identity: int) -> bool:
     """Is the grouped form of bf16 SwiGLU experts (ops.moe_grouped) estimated to be faster than all experts over all rows and than the sorted form, a pair of products per expert?
 
     All experts over all rows leave no multiply-adds out, but their products are one large one each, in the fastest tiles. The grouped form has the chosen experts' alone, in tiles of 128 rows that
     an expert's last one fills up, copies the rows and writes and reads a row of fp32 results per choice; the sorted form has launches of the host for every expert. Constants fitted to 273 steps of
     1 to 256 experts, top 1 to 8, widths of 256 to 4096 and 34 to 16000 rows with each form timed (device us; sorted up to 32 experts). Of those the estimate takes the grouped form where another one
-    is faster by more than a hundredth in 4 (by 4 % at most) and another one where the grouped form is faster in 8 (by 7 %, with up to 4 experts by 17 %). All / grouped / sorted: 28 experts of 256 of width 1024 and a shared one of 512, top 4, 40 rows 43 / 35 / 312, 500 57 / 39 / 549, 4000
+    is faster by more than a hundredth in 4 (by 4 % at most; more where the host is behind, see below) and another one where the grouped form is faster in 8 (by 7 %, with up to 4 experts by 17 %). All / grouped / sorted: 28 experts of 256 of width 1024 and a shared one of 512, top 4, 40 rows 43 / 35 / 312, 500 57 / 39 / 549, 4000
     185 / 108 / 688, of 128 of width 512 128 rows 25 / 31 / 267; 2 of 1024, top 2, 2000 rows 44 / 55 / 85; 4 of 512, top 4, 8000 rows 109 / 176 / 375, top 2 108 / 112 / 217, top 1 107 / 79 / 156; 256 of 128,
     top 8, 128 rows 124 / 103; 8 of 14336 of width 4096, top 2, 512 rows 1258 / 691 / 861, 8192 21832 / 5791 / 5080."""
     chosen, shared = rows * top * experts / (experts + identity), shared_ff / ff
@@ -769,6 +771,10 @@ def grouped_experts_pay(rows: int, experts: int, top: int, width: int, ff: int, 
     every = max(weights * (1 + shared / experts) / 2.3e12, per_row * 128 * blocks * (experts + shared) / 1.45e15) + rows * 4.0 * ff * (experts + shared) / 2.5e12
     grouped = 5e-6 + max(weights * active / experts / 4e12, per_row * 128 * tiles / 0.95e15) + moved / 4.5e12
     by_expert = 2.6e-5 * active + max(weights * active / experts / 3e12, per_row * (chosen + shared * rows) / 1.15e15) + chosen * 12.0 * width / 2e12
+    # A call's host time is 84 us for all experts, 71 grouped; with the routing (25 us) and the launches' own 20 the device is through before where `every` is below 39 us. Fewer than 16 scores come
+    # from a router in FMAs (70 us more): the device is behind
+    if experts + identity >= 16:
+        every = max(every, 3.9e-5)
     return grouped <= every and grouped <= by_expert and (experts > 4 or rows >= 512)
 
 
