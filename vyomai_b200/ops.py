@@ -963,18 +963,19 @@ def linear_pair(xs, ws, biases):
     _need_cuda(x, y, w, u, b, c)
     _rows2d(x, "linear_pair x")
     _rows2d(y, "linear_pair x")
-    (M, K), N = x.shape, w.shape[0]
-    if not (x.shape == y.shape and w.shape == u.shape == (N, K) and b.shape == c.shape == (N,) and x.dtype == y.dtype and w.dtype == u.dtype and b.dtype == c.dtype and x.stride() == y.stride()
-            and w.stride() == u.stride() and w.stride(1) == 1 and b.is_contiguous() and c.is_contiguous() and M > 0):
+    (M, K), N, lda, ldw = x.shape, w.shape[0], x.stride(0), w.stride(0)
+    xd, wd, bd = x.dtype, w.dtype, b.dtype
+    if M == 0 or y.shape != x.shape or w.shape != (N, K) or u.shape != (N, K) or b.shape != (N,) or c.shape != (N,) or y.dtype != xd or u.dtype != wd or c.dtype != bd or y.stride(0) != lda \
+            or w.stride() != (ldw, 1) or u.stride() != (ldw, 1) or not b.is_contiguous() or not c.is_contiguous():
         return None
-    apart = [divmod(q.data_ptr() - p.data_ptr(), p.element_size()) for p, q in ((x, y), (w, u), (b, c))]
-    if any(r for _, r in apart) or apart[2][0] == 0:
+    A, W, bias = x.data_ptr(), w.data_ptr(), b.data_ptr()
+    (xs_apart, r0), (ws_apart, r1), (bs_apart, r2) = divmod(y.data_ptr() - A, xd.itemsize), divmod(u.data_ptr() - W, wd.itemsize), divmod(c.data_ptr() - bias, bd.itemsize)
+    if r0 or r1 or r2 or bs_apart == 0:
         return None
     wide = (N + 7) // 8 * 8
     out = torch.empty((M, 2 * wide), device=x.device, dtype=torch.float32)
-    _lib.call("vy_linear_plain", "VyLinear", M=M, N=N, K=K, A=x.data_ptr(), lda=x.stride(0), a_dtype=_dt(x), W=w.data_ptr(), ldw=w.stride(0), w_dtype=_dt(w), act=UACT[None], scale=1.0,
-              out=out.data_ptr(), ld_out=2 * wide, out_dtype=_dt(out), batch=2, a_batch=apart[0][0], w_batch=apart[1][0], out_batch=wide, bias=b.data_ptr(), bias_dtype=_dt(b),
-              bias_batch=apart[2][0], stream=_stream())
+    _lib.call("vy_linear_plain", "VyLinear", M=M, N=N, K=K, A=A, lda=lda, a_dtype=_dt(x), W=W, ldw=ldw, w_dtype=_dt(w), act=0, scale=1.0, out=out.data_ptr(), ld_out=2 * wide, out_dtype=_dt(out),
+              batch=2, a_batch=xs_apart, w_batch=ws_apart, out_batch=wide, bias=bias, bias_dtype=_dt(b), bias_batch=bs_apart, stream=_stream())
     return out[:, :N], out[:, wide:wide + N]
 
 
@@ -991,7 +992,9 @@ def linear_plain(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tenso
     if out is None:
         out = torch.empty((M, N), device=x.device, dtype=out_dtype or x.dtype)
     _rows2d(out, "linear_plain out")
-    need = int(_lib.lib().vy_linear_plain_bytes(M, N, K)) if M > 32 and K >= 256 and x.dtype == torch.float32 and w.dtype == torch.float32 else 0   # none below, whatever N
+    need = 0
+    if M > 32 and K >= 256 and ((M + 63) >> 6) * ((N + 63) >> 6) > 128 and x.dtype == torch.float32 and w.dtype == torch.float32:   # below, the answer is 0 from 128 SMs on
+        need = int(_lib.lib().vy_linear_plain_bytes(M, N, K))
     ws = _lend((need + 3) // 4, x.device)
     _lib.call("vy_linear_plain", "VyLinear", workspace=_ptr(ws), workspace_bytes=need if ws is not None else 0, M=M, N=N, K=K, A=x.data_ptr(), lda=x.stride(0), a_dtype=_dt(x), W=w.data_ptr(),
               ldw=w.stride(0), w_dtype=_dt(w), bias=_ptr(bias), bias_dtype=_dt(bias) if bias is not None else 0, addend=_ptr(addend),
@@ -1497,19 +1500,15 @@ def moe_combine(part: torch.Tensor, inv: torch.Tensor, weight: torch.Tensor, add
     return out
 
 
-def _conv_operands(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor) -> None:
-    _need_cuda(x, w, state)
-    _rows2d(x, "causal_conv x")
-    if x.shape[1] != w.shape[0] or not w.is_contiguous() or state.dtype != torch.float32 or not state.is_contiguous():
-        raise _lib.VyomError("causal_conv: shapes / layout")
-
-
 def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, act: Optional[str] = "silu",
                 out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Depthwise causal convolution over time (w [channels, taps], last column = current token) + activation; `state`
     [slots, channels, taps - 1] fp32 carries each sequence's last inputs and is advanced."""
-    _conv_operands(x, w, state)
+    _need_cuda(x, w, state)
+    _rows2d(x, "causal_conv x")
     ch, taps = w.shape
+    if x.shape[1] != ch or not w.is_contiguous() or state.dtype != torch.float32 or not state.is_contiguous():
+        raise _lib.VyomError("causal_conv: shapes / layout")
     if out is None:
         out = torch.empty((x.shape[0], ch), device=x.device, dtype=out_dtype or x.dtype)
     _lib.call("vy_causal_conv", "VyCausalConv", channels=ch, taps=taps, x=x.data_ptr(), ldx=x.stride(0), x_dtype=_dt(x), w=w.data_ptr(),
@@ -1521,22 +1520,27 @@ def causal_conv(batch: PackedBatch, x: torch.Tensor, w: torch.Tensor, state: tor
 def causal_convs(batch: PackedBatch, xs, ws, states, act: Optional[str] = "silu") -> torch.Tensor:
     """`causal_conv` of two or three inputs. Their fp32 outputs stand side by side in one tensor. One launch where the inputs share a type and a row stride and the weights a type and
     their number of taps, else one each."""
+    _need_cuda(*xs, *ws, *states)
+    x0, w0, ch, together = xs[0], ws[0], [], True
+    (rows, _), taps, ld = x0.shape, w0.shape[1], x0.stride(0)
     for x, w, state in zip(xs, ws, states):
-        _conv_operands(x, w, state)
-    ch = [w.shape[0] for w in ws]
-    rows, total = xs[0].shape[0], sum(ch)
-    if any(x.shape[0] != rows for x in xs):
-        raise _lib.VyomError("causal_convs: the inputs are of different lengths")
-    out = torch.empty((rows, total + -total % 4), device=xs[0].device, dtype=torch.float32)[:, :total]   # rows on 16-byte boundaries, whatever the last input's width: readers take four channels at a time
-    if any(x.dtype != xs[0].dtype or x.stride(0) != xs[0].stride(0) or w.dtype != ws[0].dtype or w.shape[1] != ws[0].shape[1] for x, w in zip(xs, ws)):
+        _rows2d(x, "causal_convs x")
+        c, t = w.shape
+        if x.shape != (rows, c) or not w.is_contiguous() or state.dtype != torch.float32 or not state.is_contiguous():
+            raise _lib.VyomError("causal_convs: shapes / layout")
+        ch.append(c)
+        together = together and t == taps and x.stride(0) == ld and x.dtype == x0.dtype and w.dtype == w0.dtype
+    total = sum(ch)
+    out = torch.empty((rows, total + -total % 4), device=x0.device, dtype=torch.float32)[:, :total]   # rows on 16-byte boundaries, whatever the last input's width: readers take four channels at a time
+    if not together:
         at = 0
         for x, w, state, c in zip(xs, ws, states, ch):
             causal_conv(batch, x, w, state, act=act, out=out[:, at:at + c])
             at += c
         return out
     third = dict(channels3=ch[2], x3=xs[2].data_ptr(), w3=ws[2].data_ptr(), state3=states[2].data_ptr()) if len(ch) > 2 else {}
-    _lib.call("vy_causal_conv", "VyCausalConv", channels=ch[0], taps=ws[0].shape[1], x=xs[0].data_ptr(), ldx=xs[0].stride(0), x_dtype=_dt(xs[0]), w=ws[0].data_ptr(),
-              w_dtype=_dt(ws[0]), state=states[0].data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
+    _lib.call("vy_causal_conv", "VyCausalConv", channels=ch[0], taps=taps, x=x0.data_ptr(), ldx=ld, x_dtype=_dt(x0), w=w0.data_ptr(),
+              w_dtype=_dt(w0), state=states[0].data_ptr(), act=UACT[act], out=out.data_ptr(), ld_out=out.stride(0), out_dtype=_dt(out),
               stream=_stream(), rows=rows, channels2=ch[1], x2=xs[1].data_ptr(), w2=ws[1].data_ptr(), state2=states[1].data_ptr(), **third, **batch._kw())
     return out
 
