@@ -355,6 +355,28 @@ def test_experts_of_a_layer_take_the_grouped_form(monkeypatch, rows, experts, id
         assert HU.rel_err(got.cpu().double() + (0.0 if ident is None else ident.cpu().double()[:, None] * h.double()), want) < 1.5e-2
 
 
+def test_a_captured_step_of_experts_makes_no_host_decision(monkeypatch):
+    """A step that would take the sorted form, which reads the experts' row counts on the host, takes the grouped form while it is captured."""
+    from vyomai_b200.layers import mixers
+    m, _ = _experts(U.moe(ff=64, experts=6, top=3, identity=2, shared=128), 128, torch.bfloat16)
+    h, batch = torch.randn(300, 128, generator=_gen(12)).to(DEV, torch.bfloat16), type("B", (), {"max_new": 300})()
+    monkeypatch.setattr(mixers, "grouped_experts_pay", lambda *a: False)
+    monkeypatch.setattr(m, "_sorted_is_faster", lambda rows: True)
+    want, ident = m.forward_parts(h, batch)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        m._grouped_workspace(h, batch, anyway=True)
+        monkeypatch.setattr(mixers, "grouped_experts_pay", lambda *a: True)
+        m.forward_parts(h, batch)   # warm
+        monkeypatch.setattr(mixers, "grouped_experts_pay", lambda *a: False)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        y, i = m.forward_parts(h, batch)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(i, ident) and HU.rel_err(y.cpu().double(), want.cpu().double()) < 1.5e-2
+
+
 @pytest.mark.parametrize("sort", [False, True])
 def test_every_choice_is_an_identity_expert(sort):
     f = U.moe(experts=3, top=2, identity=2, shared=None)

@@ -865,13 +865,13 @@ class MoEFeedForward:
         moved = 3.0 * rows * self.top * width * 4 / 2.0e12   # gather, per-pair results, combine
         return self.top * per_choice + launches * self.LAUNCH_COST + moved < self.experts * per_choice
 
-    def _grouped_workspace(self, h: torch.Tensor, batch) -> Optional[torch.Tensor]:
-        """Scratch for the grouped form, or None where it does not apply or is not the fastest."""
+    def _grouped_workspace(self, h: torch.Tensor, batch, anyway: bool = False) -> Optional[torch.Tensor]:
+        """Scratch for the grouped form, or None where it does not apply or (unless `anyway`) is not the fastest."""
         rows = h.shape[0]
         enough = rows >= self.sorted_min_rows or (32 < rows and h.shape[1] >= 1024 and self.sorted_min_rows <= 128)
         if not (self.swiglu and not self.force_sorted and batch.max_new > 1 and enough and h.dtype == torch.bfloat16 and self.act_dtype == torch.bfloat16
                 and self.up_all.tensor_cores and self.down_all.tensor_cores and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
-                and grouped_experts_pay(rows, self.experts, self.top, h.shape[1], self.ff, self.shared_ff, self.identity)):
+                and (anyway or grouped_experts_pay(rows, self.experts, self.top, h.shape[1], self.ff, self.shared_ff, self.identity))):
             return None
         need = ops.moe_grouped_bytes(rows, self.experts, self.top, h.shape[1], self.ff, self.shared_ff)
         return ops._lend((need + 3) // 4, h.device)
@@ -910,6 +910,9 @@ class MoEFeedForward:
         scored = E + self.identity
         grouped = self._grouped_workspace(h, batch)
         sorted_form = grouped is None and batch.max_new > 1 and rows >= self.sorted_min_rows and (self.force_sorted or self._sorted_is_faster(rows))
+        if sorted_form and torch.cuda.is_current_stream_capturing():   # the sorted form reads the device; the grouped one, where it applies, does not
+            grouped = self._grouped_workspace(h, batch, anyway=True)
+            sorted_form = grouped is None
         idx, wt, dense, *rest = ops.moe_route(z, scored, self.top, self.route_scale, dense=grouped is None and not sorted_form, kind=self.router_kind, groups=self.groups,
                                               keep_groups=self.keep_groups, normalize=self.normalize, correction=self.correction, identity=self.identity)
         ident = rest[0] if rest else None
