@@ -1086,7 +1086,7 @@ def run_hybrid(args):
 # width / depth / vocabulary (both run on HybridBatchEngine's packed step)
 # ------------------------------------------------------------------------------------------------
 LATENT_KERNELS = ("window_attn_tc", "window_attn_mma", "window_attn_split", "la_states", "la_scan", "la_outputs", "delta_chunk", "delta_scan", "linear_split", "window_attn_decode", "window_attn_heads_merge", "window_attn_heads", "window_attn", "latent_kv_write", "rope_split", "moe_route", "moe_scale", "moe_sort",
-                  "moe_gather", "moe_combine", "linear_halves", "linear_thin", "linear_tile", "linear_rows", "linear_attn_chunk", "linear_attn", "delta_rule", "delta_prep",
+                  "moe_gather", "moe_combine", "moe_plan", "moe_spread", "moe_merge", "linear_halves", "linear_thin", "linear_tile", "linear_rows", "linear_attn_chunk", "linear_attn", "delta_rule", "delta_prep",
                   "causal_conv", "rms_norm", "kv_page_write", "unary", "embed_rows", "gemm_skinny", "gemm_kernel", "argmax")
 
 
@@ -1685,6 +1685,9 @@ def _expert_rows_roofline(pk, runs, tokens, width, top, chosen, rf):
         "moe_combine": _roof(pk, ("moe_combine",), byts=runs * tokens * width * 4 * (chosen + 2), **rf),
         "moe_route": _roof(pk, ("moe_route",), byts=runs * tokens * (32 + 2 * top) * 4, **rf),
         "moe_sort": _roof(pk, ("moe_sort",), byts=runs * tokens * top * 12, **rf),
+        # grouped: a row read and written per chosen expert and for the shared one (bf16); their fp32 results read, the sum written
+        "moe_spread": _roof(pk, ("moe_spread",), byts=runs * tokens * width * 2 * (chosen + 2), **rf),
+        "moe_merge": _roof(pk, ("moe_merge",), byts=runs * tokens * width * 4 * (chosen + 2), **rf),
     }
 
 
